@@ -318,6 +318,12 @@ int32_t k2b200_intersect_dense_pruned_search(const k2b200_pruned_args *args, voi
                                              size_t workspace_bytes, void *stream,
                                              int32_t *num_states_out, int32_t *num_arcs_out,
                                              int32_t *arena_full);
+/* The same; layer_bounds (HOST [2], may be NULL) receives the most states of a frame and
+ * the most arcs leaving one, for k2b200_fsa_view::max_layer_states / max_layer_arcs of the
+ * lattice (its frames are layers, all arcs go from one to the next). */
+int32_t k2b200_intersect_dense_pruned_search_bounds(
+    const k2b200_pruned_args *args, void *workspace, size_t workspace_bytes, void *stream,
+    int32_t *num_states_out, int32_t *num_arcs_out, int32_t *arena_full, int32_t *layer_bounds);
 int32_t k2b200_intersect_dense_pruned_emit(const k2b200_pruned_args *args, void *workspace,
                                            size_t workspace_bytes, void *stream,
                                            const k2b200_lattice_out *out);
@@ -379,6 +385,13 @@ int32_t k2b200_online_decode_run(const k2b200_online_args *args, void *workspace
                                  size_t workspace_bytes, void *stream, const float *h_beams_in,
                                  float *h_beams_out, int32_t *h_counts, int32_t *num_states_out,
                                  int32_t *num_arcs_out, int32_t *arena_full);
+/* The same; layer_bounds as in k2b200_intersect_dense_pruned_search_bounds. */
+int32_t k2b200_online_decode_run_bounds(const k2b200_online_args *args, void *workspace,
+                                        size_t workspace_bytes, void *stream,
+                                        const float *h_beams_in, float *h_beams_out,
+                                        int32_t *h_counts, int32_t *num_states_out,
+                                        int32_t *num_arcs_out, int32_t *arena_full,
+                                        int32_t *layer_bounds);
 int32_t k2b200_online_decode_emit(const k2b200_online_args *args, void *workspace,
                                   size_t workspace_bytes, void *stream,
                                   const k2b200_lattice_out *out);
@@ -563,11 +576,18 @@ typedef struct {
   int32_t max_layer_arcs;   /* upper bound on arcs between two layers */
 } k2b200_fsa_view;
 
+/* Incoming-arc index of a strictly layered view (max_layers, max_layer_states set), built
+ * layer by layer in one launch: the same arrays as k2b200_fsa_incoming.  *done = 0 when a
+ * layer is too wide for it; the caller then uses k2b200_fsa_incoming. */
+int32_t k2b200_fsa_incoming_layers(const k2b200_fsa_view *fsas, int32_t *in_splits,
+                                   int32_t *in_arcs, int32_t *in_src, float *in_score,
+                                   int32_t *done, void *stream);
+
 /* scratch (k2b200_fsa_scores_scratch_bytes(fsas) bytes; may be NULL) enables the
- * fastest log-semiring kernel for strictly layered views: it keeps every score
- * as mantissa * 2^exponent so that no exp/log sits on the layer-to-layer
- * dependency chain (the arcs' exp() and the states' log() run in separate fully
- * parallel kernels).  Without scratch a slower kernel gives the same values. */
+ * fastest kernels for strictly layered views: for the log semiring they work on
+ * exp(score) with a power of two shared by a layer, so that no exp/log sits on the
+ * layer-to-layer dependency chain (the arcs' exp() and the states' log() run in separate
+ * fully parallel kernels).  Without scratch a slower kernel gives the same values. */
 size_t k2b200_fsa_scores_scratch_bytes(const k2b200_fsa_view *fsas);
 int32_t k2b200_fsa_scores(const k2b200_fsa_view *fsas, int32_t log_semiring,
                           int32_t use_double, void *forward, void *backward,

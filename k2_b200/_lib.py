@@ -145,6 +145,12 @@ _sig("k2b200_intersect_dense_pruned_workspace_bytes", c_i32,
 _sig("k2b200_intersect_dense_pruned_search", c_i32,
      [ctypes.POINTER(PrunedArgs), c_vp, c_sz, c_vp, ctypes.POINTER(c_i32),
       ctypes.POINTER(c_i32), ctypes.POINTER(c_i32)])
+_sig("k2b200_intersect_dense_pruned_search_bounds", c_i32,
+     [ctypes.POINTER(PrunedArgs), c_vp, c_sz, c_vp, ctypes.POINTER(c_i32),
+      ctypes.POINTER(c_i32), ctypes.POINTER(c_i32), ctypes.POINTER(c_i32)])
+_sig("k2b200_online_decode_run_bounds", c_i32,
+     [ctypes.POINTER(OnlineArgs), c_vp, c_sz, c_vp, c_vp, c_vp, c_vp, ctypes.POINTER(c_i32),
+      ctypes.POINTER(c_i32), ctypes.POINTER(c_i32), ctypes.POINTER(c_i32)])
 _sig("k2b200_intersect_dense_pruned_emit", c_i32,
      [ctypes.POINTER(PrunedArgs), c_vp, c_sz, c_vp, ctypes.POINTER(LatticeOut)])
 _sig("k2b200_exclusive_sum_tmp_bytes", c_sz, [c_i64])
@@ -187,6 +193,8 @@ _sig("k2b200_debug_set_copy_wait_limit", None, [c_i32])
 _sig("k2b200_fsa_levels_tmp_bytes", c_sz, [c_i32])
 _sig("k2b200_fsa_levels", c_i32,
      [c_vp, c_vp, c_vp, c_vp, c_i32, c_i32, c_i32, c_vp, c_vp, c_vp, c_vp, c_vp])
+_sig("k2b200_fsa_incoming_layers", c_i32,
+     [ctypes.POINTER(FsaView), c_vp, c_vp, c_vp, c_vp, ctypes.POINTER(c_i32), c_vp])
 _sig("k2b200_fsa_scores_scratch_bytes", c_sz, [ctypes.POINTER(FsaView)])
 _sig("k2b200_fsa_scores", c_i32,
      [ctypes.POINTER(FsaView), c_i32, c_i32, c_vp, c_vp, c_vp, c_vp, c_sz, c_vp])
@@ -231,7 +239,7 @@ EXPORTED = [
     "k2b200_upload_i32",
     "k2b200_exclusive_sum_tmp_bytes", "k2b200_exclusive_sum",
     "k2b200_exclusive_sum_static_max_len", "k2b200_exclusive_sum_static", "k2b200_fsa_incoming_tmp_bytes",
-    "k2b200_fsa_incoming", "k2b200_intersect_dense_workspace_bytes",
+    "k2b200_fsa_incoming", "k2b200_fsa_incoming_layers", "k2b200_intersect_dense_workspace_bytes",
     "k2b200_intersect_dense_prune", "k2b200_intersect_dense_emit", "k2b200_fsa_scores",
     "k2b200_fsa_scores_scratch_bytes",
     "k2b200_fsa_tot_scores", "k2b200_fsa_arc_post", "k2b200_tot_scores_log_backward",
@@ -245,7 +253,8 @@ EXPORTED = [
     "k2b200_dense_loss_supported", "k2b200_dense_loss_workspace_bytes",
     "k2b200_dense_loss_forward", "k2b200_dense_loss_backward",
     "k2b200_intersect_dense_pruned_workspace_bytes", "k2b200_intersect_dense_pruned_search",
-    "k2b200_intersect_dense_pruned_emit",
+    "k2b200_intersect_dense_pruned_emit", "k2b200_intersect_dense_pruned_search_bounds",
+    "k2b200_online_decode_run_bounds",
     "k2b200_fsa_scores_backprop", "k2b200_fsa_arc_post_backprop",
     "k2b200_dense_loss_backward_log_probs",
     "k2b200_peer_reduce_create", "k2b200_peer_reduce_open", "k2b200_peer_reduce_close",

@@ -393,6 +393,7 @@ def _intersect_dense_pruned_arcs(a: RaggedArc, b: DenseFsaVec, search_beam: floa
     cap_a = max(cap_a, _pruned_capacity.get((str(dev), num_seqs), 0))
     stream = _lib.stream_of(dev)
     i32 = dict(dtype=torch.int32, device=dev)
+    bounds = (ctypes.c_int32 * 2)()
     while True:
         args = _lib.PrunedArgs(
             num_fsas=a.num_fsas, num_states=a.num_states, num_arcs=a.num_elements(),
@@ -409,9 +410,9 @@ def _intersect_dense_pruned_arcs(a: RaggedArc, b: DenseFsaVec, search_beam: floa
         ws = torch.empty(nbytes.value, dtype=torch.uint8, device=dev)
         ns, na, full = ctypes.c_int32(), ctypes.c_int32(), ctypes.c_int32()
         with torch.cuda.device(dev):
-            _lib.check(_lib.lib.k2b200_intersect_dense_pruned_search(
+            _lib.check(_lib.lib.k2b200_intersect_dense_pruned_search_bounds(
                 ctypes.byref(args), _lib.ptr(ws), nbytes.value, stream, ctypes.byref(ns),
-                ctypes.byref(na), ctypes.byref(full)))
+                ctypes.byref(na), ctypes.byref(full), bounds))
         if not full.value:
             _pruned_capacity[(str(dev), num_seqs)] = cap_a
             break
@@ -439,6 +440,8 @@ def _intersect_dense_pruned_arcs(a: RaggedArc, b: DenseFsaVec, search_beam: floa
             ctypes.byref(args), _lib.ptr(ws), nbytes.value, stream, ctypes.byref(out)))
     lattice = RaggedArc(values[:na], row_splits1, row_splits2, row_ids1[:ns], row_ids2[:na])
     lattice._levels = (level_offsets, level_splits)
+    # frames are layers; the search measured the largest of them
+    lattice._layer_bounds = (1, int(np.diff(h_brs).max()) + 2, bounds[0], bounds[1])
     return lattice, arc_map_a[:na], arc_map_b[:na]
 
 

@@ -70,9 +70,11 @@ struct SearchArgs {
   uint8_t *arc_keep;
   unsigned long long *winner;  // [num_seqs * a_states] (shared) or [a_states]
   int32_t *frame_s0, *frame_a0;  // [num_seqs][T + 2]
-  int32_t *seq_out;           // [num_seqs][4]: states, arcs, extra final state, status
+  int32_t *seq_out;           // [num_seqs][kSeqOut]: states, arcs, extra final state, status,
+                              // most states of a frame, most arcs leaving one
 };
 
+constexpr int kSeqOut = 6;
 enum : int32_t { kSeqOk = 0, kSeqOverflow = 1, kSeqManyFinal = 2 };
 
 // The CTAs that work on one sequence: a thread-block cluster (of one CTA when there are
@@ -93,6 +95,7 @@ struct Shared {
   int32_t wbest[kSearchThreads / 32][32], wcnt[kSearchThreads / 32][32];  // per warp
   float cutoff;
   float beam;
+  int32_t most_states, most_arcs;
 };
 
 struct Team {
@@ -756,6 +759,23 @@ __device__ void PruneWindow(const SearchArgs &g, const SeqView &v, const Team &t
   *a_top = wa;
 }
 
+// Largest frame of the finished lattice of a sequence, in states and in arcs, over frames
+// 0 .. frames - 1; by the first CTA of the team, its thread 0 has the result in sh.
+__device__ void LargestFrame(const SeqView &v, const Team &tm, int32_t frames) {
+  Shared *sh = tm.sh;
+  if (tm.rank != 0) return;
+  if (threadIdx.x == 0) sh->most_states = sh->most_arcs = 0;
+  __syncthreads();
+  int32_t ms = 0, ma = 0;
+  for (int32_t t = threadIdx.x; t < frames; t += kSearchThreads) {
+    ms = max(ms, v.frame_s0[t + 1] - v.frame_s0[t]);
+    ma = max(ma, v.frame_a0[t + 1] - v.frame_a0[t]);
+  }
+  if (ms) atomicMax(&sh->most_states, ms);
+  if (ma) atomicMax(&sh->most_arcs, ma);
+  __syncthreads();
+}
+
 // One team per sequence: all frames of the search with the pruning windows in the
 // reference's schedule (:164-199, :213-229).
 __global__ void __launch_bounds__(kSearchThreads, 1) PrunedSearch(const SearchArgs g) {
@@ -818,23 +838,31 @@ __global__ void __launch_bounds__(kSearchThreads, 1) PrunedSearch(const SearchAr
   if (status == kSeqOk) {  // the states of the last frame have no arcs in the lattice
     for (int32_t k = tm.tid; k < ns; k += tm.threads) v.st_arc0[s0 + k] = a_top;
   }
-  if (tm.tid == 0) {
-    int32_t extra = 0;
-    if (status == kSeqOk) {
+  if (status == kSeqOk) {
+    if (tm.tid == 0) {
       v.frame_s0[T + 1] = s_top;  // frame T has no arcs
       v.frame_a0[T + 1] = a_top;
       v.st_arc0[s_top] = a_top;
+    }
+    tm.Sync();
+    LargestFrame(v, tm, T + 1);
+  }
+  if (tm.tid == 0) {
+    int32_t extra = 0;
+    if (status == kSeqOk) {
       // a sequence whose final state did not survive still gets a final state, so
       // that the result is a valid FSA (:519-547)
       const int32_t at_final = v.frame_s0[final_t + 1] - v.frame_s0[final_t];
       if (at_final > 1) status = kSeqManyFinal;
       extra = (g_states > 0) * (1 - min(at_final, 1));
     }
-    int32_t *o = g.seq_out + 4 * seq;
+    int32_t *o = g.seq_out + kSeqOut * seq;
     o[0] = s_top + extra;
     o[1] = a_top;
     o[2] = extra;
     o[3] = status;
+    o[4] = sh.most_states;
+    o[5] = sh.most_arcs;
   }
   tm.Sync();  // no CTA leaves while another may still read its shared memory
 }
@@ -869,10 +897,10 @@ __global__ void FormatPruned(const FormatArgs f) {
   if (t == g.T + 1) {
     // the extra final state, if any, and the end of the row_splits
     if (threadIdx.x == 0) {
-      const int32_t extra = g.seq_out[4 * seq + 2];
+      const int32_t extra = g.seq_out[kSeqOut * seq + 2];
       if (extra) {
         f.row_ids1[sb + s0] = seq;
-        f.row_splits2[sb + s0] = ab + g.seq_out[4 * seq + 1];
+        f.row_splits2[sb + s0] = ab + g.seq_out[kSeqOut * seq + 1];
       }
       if (seq == g.num_seqs - 1) f.row_splits2[f.out_rs1[g.num_seqs]] = f.arc_base[g.num_seqs];
     }
@@ -1065,12 +1093,18 @@ __global__ void __launch_bounds__(kSearchThreads, 1) OnlineChunk(const OnlineArg
       }
     }
   }
+  if (status == kSeqOk) {
+    tm.Sync();
+    LargestFrame(v, tm, end + 1);
+  }
   if (tm.tid == 0) {
-    int32_t *out = g.seq_out + 4 * seq;
+    int32_t *out = g.seq_out + kSeqOut * seq;
     out[0] = s_top;      // states without the final one
     out[1] = a_top;
     out[2] = end;        // frames: the frontier is frame `end`
     out[3] = status;
+    out[4] = sh.most_states;
+    out[5] = sh.most_arcs;
     o.beam_out[seq] = sh.beam;
   }
   tm.Sync();
@@ -1198,7 +1232,7 @@ int32_t MakePrunedLayout(const k2b200_pruned_args *a, char *ws, PrunedLayout *L)
   g.winner = reinterpret_cast<unsigned long long *>(ws + Take(&off, L->winner_bytes));
   g.frame_s0 = i32(n * ((size_t)T + 2));
   g.frame_a0 = i32(n * ((size_t)T + 2));
-  g.seq_out = i32(4 * n);
+  g.seq_out = i32(kSeqOut * n);
   L->out_rs1 = i32(n + 1);
   L->arc_base = i32(n + 1);
   L->bytes = off;
@@ -1308,6 +1342,14 @@ int32_t k2b200_intersect_dense_pruned_search(const k2b200_pruned_args *args, voi
                                              size_t workspace_bytes, void *stream_v,
                                              int32_t *num_states_out, int32_t *num_arcs_out,
                                              int32_t *arena_full) {
+  return k2b200_intersect_dense_pruned_search_bounds(args, workspace, workspace_bytes, stream_v,
+                                                     num_states_out, num_arcs_out, arena_full,
+                                                     nullptr);
+}
+
+int32_t k2b200_intersect_dense_pruned_search_bounds(
+    const k2b200_pruned_args *args, void *workspace, size_t workspace_bytes, void *stream_v,
+    int32_t *num_states_out, int32_t *num_arcs_out, int32_t *arena_full, int32_t *layer_bounds) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
   PrunedLayout L;
   K2B_FORWARD(MakePrunedLayout(args, reinterpret_cast<char *>(workspace), &L));
@@ -1343,7 +1385,7 @@ int32_t k2b200_intersect_dense_pruned_search(const k2b200_pruned_args *args, voi
     NoteLaunch();
   }
   K2B_CUDA_OK(cudaGetLastError());
-  std::vector<int32_t> h(4 * (size_t)n);
+  std::vector<int32_t> h(kSeqOut * (size_t)n);
   K2B_CUDA_OK(cudaMemcpyAsync(h.data(), L.g.seq_out, sizeof(int32_t) * h.size(),
                               cudaMemcpyDeviceToHost, stream));
   K2B_CUDA_OK(cudaStreamSynchronize(stream));
@@ -1352,18 +1394,25 @@ int32_t k2b200_intersect_dense_pruned_search(const k2b200_pruned_args *args, voi
   int64_t ts = 0, ta = 0;
   *arena_full = 0;
   for (int32_t i = 0; i < n; ++i) {
-    if (h[4 * i + 3] == kSeqOverflow) *arena_full = 1;
-    K2B_REQUIRE(h[4 * i + 3] != kSeqManyFinal,
+    if (h[kSeqOut * i + 3] == kSeqOverflow) *arena_full = 1;
+    K2B_REQUIRE(h[kSeqOut * i + 3] != kSeqManyFinal,
                 "sequence %d reaches more than one state on its last frame: arcs with label -1 "
                 "must enter the final state of their graph", i);
     srs[i] = (int32_t)ts;
     ars[i] = (int32_t)ta;
-    ts += h[4 * i + 0];
-    ta += h[4 * i + 1];
+    ts += h[kSeqOut * i];
+    ta += h[kSeqOut * i + 1];
   }
   srs[n] = (int32_t)ts;
   ars[n] = (int32_t)ta;
   *num_states_out = *num_arcs_out = 0;
+  if (layer_bounds != nullptr) {
+    layer_bounds[0] = layer_bounds[1] = 1;
+    for (int32_t i = 0; i < n; ++i) {
+      layer_bounds[0] = std::max(layer_bounds[0], h[kSeqOut * i + 4]);
+      layer_bounds[1] = std::max(layer_bounds[1], h[kSeqOut * i + 5]);
+    }
+  }
   if (*arena_full) return kOk;
   K2B_REQUIRE(ts < INT_MAX && ta < INT_MAX, "the lattice has too many states or arcs for int32");
   // out_rs1 and arc_base are adjacent in the workspace only up to alignment: two uploads
@@ -1447,6 +1496,17 @@ int32_t k2b200_online_decode_run(const k2b200_online_args *args, void *workspace
                                  size_t workspace_bytes, void *stream_v, const float *h_beams_in,
                                  float *h_beams_out, int32_t *h_counts, int32_t *num_states_out,
                                  int32_t *num_arcs_out, int32_t *arena_full) {
+  return k2b200_online_decode_run_bounds(args, workspace, workspace_bytes, stream_v, h_beams_in,
+                                         h_beams_out, h_counts, num_states_out, num_arcs_out,
+                                         arena_full, nullptr);
+}
+
+int32_t k2b200_online_decode_run_bounds(const k2b200_online_args *args, void *workspace,
+                                        size_t workspace_bytes, void *stream_v,
+                                        const float *h_beams_in, float *h_beams_out,
+                                        int32_t *h_counts, int32_t *num_states_out,
+                                        int32_t *num_arcs_out, int32_t *arena_full,
+                                        int32_t *layer_bounds) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
   OnlineLayout L;
   K2B_FORWARD(MakeOnlineLayout(args, reinterpret_cast<char *>(workspace), &L));
@@ -1487,7 +1547,7 @@ int32_t k2b200_online_decode_run(const k2b200_online_args *args, void *workspace
     K2B_CUDA_OK(cudaLaunchKernelEx(&cfg, OnlineChunk, o));
     NoteLaunch();
   }
-  std::vector<int32_t> h(4 * (size_t)n);
+  std::vector<int32_t> h(kSeqOut * (size_t)n);
   K2B_CUDA_OK(cudaMemcpyAsync(h.data(), L.base.g.seq_out, sizeof(int32_t) * h.size(),
                               cudaMemcpyDeviceToHost, stream));
   K2B_CUDA_OK(cudaMemcpyAsync(h_beams_out, L.beam_out, sizeof(float) * n, cudaMemcpyDeviceToHost,
@@ -1498,17 +1558,24 @@ int32_t k2b200_online_decode_run(const k2b200_online_args *args, void *workspace
   int64_t ts = 0, ta = 0;
   *arena_full = 0;
   for (int32_t i = 0; i < n; ++i) {
-    if (h[4 * i + 3] == kSeqOverflow) *arena_full = 1;
-    h_counts[2 * i] = h[4 * i];
-    h_counts[2 * i + 1] = h[4 * i + 1];
+    if (h[kSeqOut * i + 3] == kSeqOverflow) *arena_full = 1;
+    h_counts[2 * i] = h[kSeqOut * i];
+    h_counts[2 * i + 1] = h[kSeqOut * i + 1];
     srs[i] = (int32_t)ts;
     ars[i] = (int32_t)ta;
-    ts += h[4 * i] + 1;  // one final state per stream
-    ta += h[4 * i + 1];
+    ts += h[kSeqOut * i] + 1;  // one final state per stream
+    ta += h[kSeqOut * i + 1];
   }
   srs[n] = (int32_t)ts;
   ars[n] = (int32_t)ta;
   *num_states_out = *num_arcs_out = 0;
+  if (layer_bounds != nullptr) {
+    layer_bounds[0] = layer_bounds[1] = 1;
+    for (int32_t i = 0; i < n; ++i) {
+      layer_bounds[0] = std::max(layer_bounds[0], h[kSeqOut * i + 4]);
+      layer_bounds[1] = std::max(layer_bounds[1], h[kSeqOut * i + 5]);
+    }
+  }
   if (*arena_full) return kOk;
   K2B_REQUIRE(ts < INT_MAX && ta < INT_MAX, "the lattice has too many states or arcs for int32");
   K2B_FORWARD(UploadInts(srs, n + 1, L.base.out_rs1, stream));

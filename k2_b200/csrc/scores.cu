@@ -223,14 +223,13 @@ static int32_t LaunchScores(const k2b200_fsa_view *v, int32_t log_semiring, Real
   if (ndir == 0 || v->num_fsas == 0) return kOk;
   PhaseTimer timer(kPhaseScores, stream);
   bool launched = false;
-  if (log_semiring) {
-    K2B_FORWARD(LaunchProbScores<Real>(v, fwd, bwd, scratch, scratch_bytes, stream, &launched));
-    // if a CTA found the layer bounds violated, redo everything the general way
-    if (launched)
-      return LaunchGeneric<Real>(v, 1, fwd, bwd, nullptr, ProbStatusWord(v, scratch), stream);
-  }
-  K2B_FORWARD(LaunchStagedScores<Real>(v, log_semiring, fwd, bwd, entering, stream, &launched));
-  if (launched) return kOk;
+  K2B_FORWARD(LaunchLayerScores<Real>(v, log_semiring, fwd, bwd, entering, scratch, scratch_bytes,
+                                      stream, &launched));
+  // if a CTA found the layer bounds violated, or values out of range, redo everything the
+  // general way
+  if (launched)
+    return LaunchGeneric<Real>(v, log_semiring, fwd, bwd, entering, LayerStatusWord(v, scratch),
+                               stream);
   return LaunchGeneric<Real>(v, log_semiring, fwd, bwd, entering, nullptr, stream);
 }
 
@@ -289,8 +288,22 @@ int32_t k2b200_fsa_incoming(const int32_t *row_splits1, const int32_t *row_ids1,
                        STREAM(stream));
 }
 
+int32_t k2b200_fsa_incoming_layers(const k2b200_fsa_view *v, int32_t *in_splits,
+                                   int32_t *in_arcs, int32_t *in_src, float *in_score,
+                                   int32_t *done, void *stream) {
+  K2B_REQUIRE(v && in_splits && in_arcs && in_src && in_score && done, "NULL pointer");
+  K2B_REQUIRE(v->row_splits1 && v->row_ids1 && v->row_splits2 && v->level_offsets &&
+                  v->level_splits,
+              "NULL pointer in the FsaVec view");
+  PhaseTimer timer(kPhaseIncoming, STREAM(stream));
+  bool ok = false;
+  K2B_FORWARD(BuildLayerIncoming(v, in_splits, in_arcs, in_src, in_score, STREAM(stream), &ok));
+  *done = ok ? 1 : 0;
+  return kOk;
+}
+
 size_t k2b200_fsa_scores_scratch_bytes(const k2b200_fsa_view *v) {
-  return v ? ProbScratchBytes(v) : 0;
+  return v ? LayerScratchBytes(v) : 0;
 }
 
 int32_t k2b200_fsa_scores(const k2b200_fsa_view *v, int32_t log_semiring, int32_t use_double,

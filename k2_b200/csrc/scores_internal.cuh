@@ -1,4 +1,4 @@
-// Internal declarations shared by scores.cu and scores_staged.cu.
+// Internal declarations shared by scores.cu and layer_scores.cu.
 #pragma once
 #include <cmath>
 
@@ -103,17 +103,17 @@ __device__ void LayeredScoresDevice(const k2b200_fsa_view &v, int32_t i, int32_t
 }
 
 
-// Mantissa/exponent log-semiring recursion (scores_staged.cu).
-size_t ProbScratchBytes(const k2b200_fsa_view *v);
+// Strictly layered FsaVecs (layer_scores.cu).  *launched stays false when the view does not
+// qualify.  A non-zero status word afterwards means that its layer bounds did not hold or its
+// values left the range of the recursion: the results must be recomputed.
+size_t LayerScratchBytes(const k2b200_fsa_view *v);
+int32_t *LayerStatusWord(const k2b200_fsa_view *v, void *scratch);
 template <typename Real>
-int32_t LaunchProbScores(const k2b200_fsa_view *v, Real *fwd, Real *bwd, void *scratch,
-                         size_t scratch_bytes, cudaStream_t stream, bool *launched);
-// Address of the status word inside the scratch: non-zero after LaunchProbScores
-// means the view's layer bounds did not hold and the results must be recomputed.
-int32_t *ProbStatusWord(const k2b200_fsa_view *v, void *scratch);
-
-template <typename Real>
-int32_t LaunchStagedScores(const k2b200_fsa_view *v, int32_t log_semiring, Real *fwd, Real *bwd,
-                           int32_t *entering, cudaStream_t stream, bool *launched);
+int32_t LaunchLayerScores(const k2b200_fsa_view *v, int32_t log_semiring, Real *fwd, Real *bwd,
+                          int32_t *entering, void *scratch, size_t scratch_bytes,
+                          cudaStream_t stream, bool *launched);
+// Incoming-arc index of such an FsaVec; *done stays false when a layer is too wide for it.
+int32_t BuildLayerIncoming(const k2b200_fsa_view *v, int32_t *in_splits, int32_t *in_arcs,
+                           int32_t *in_src, float *in_score, cudaStream_t stream, bool *done);
 
 }  // namespace k2b

@@ -235,7 +235,7 @@ class Fsa(object):
             entering = torch.empty(ns, dtype=torch.int32, device=dev)
         view, keep = arcs.view(want_incoming=want_forward)
         scratch, nscratch = None, 0
-        if log_semiring and arcs._layer_bounds[0]:
+        if arcs._layer_bounds[0]:
             nscratch = _lib.lib.k2b200_fsa_scores_scratch_bytes(ctypes.byref(view))
             scratch = torch.empty(nscratch, dtype=torch.uint8, device=dev)
         with torch.cuda.device(dev):

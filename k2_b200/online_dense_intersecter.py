@@ -99,6 +99,7 @@ class OnlineDenseIntersecter:
         cap_a = max(self._arcs_per_seq, 2 * need_a, 4 * need_s)
         stream = _lib.stream_of(dev)
         i32 = dict(dtype=torch.int32, device=dev)
+        bounds = (ctypes.c_int32 * 2)()
         while True:
             args = _lib.OnlineArgs(
                 num_states=arcs.num_states, num_arcs=arcs.num_elements(),
@@ -121,10 +122,10 @@ class OnlineDenseIntersecter:
                 loads = (_lib.OnlineStream * n)(*[s._c() for s in states])
                 _lib.check(_lib.lib.k2b200_online_decode_load_all(
                     ctypes.byref(args), _lib.ptr(ws), loads, stream))
-                _lib.check(_lib.lib.k2b200_online_decode_run(
+                _lib.check(_lib.lib.k2b200_online_decode_run_bounds(
                     ctypes.byref(args), _lib.ptr(ws), nbytes.value, stream,
                     beams_in.ctypes.data, beams_out.ctypes.data, counts.ctypes.data,
-                    ctypes.byref(ns), ctypes.byref(na), ctypes.byref(full)))
+                    ctypes.byref(ns), ctypes.byref(na), ctypes.byref(full), bounds))
             if not full.value:
                 self._arcs_per_seq = max(self._arcs_per_seq, cap_a)
                 break
@@ -167,6 +168,7 @@ class OnlineDenseIntersecter:
                 ctypes.byref(args), _lib.ptr(ws), stores, stream))
         lattice = RaggedArc(values[:na], row_splits1, row_splits2, row_ids1[:ns], row_ids2[:na])
         lattice._levels = (level_offsets, level_splits)  # frames are layers
+        lattice._layer_bounds = (1, int(h_hist.max()) + chunk + 2, bounds[0], bounds[1])
         arc_map_a = arc_map_a[:na]
         # attributes of the graph follow the arc map, as
         # k2.utils.fsa_from_unary_function_tensor does (k2/python/k2/utils.py)

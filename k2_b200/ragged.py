@@ -9,6 +9,7 @@ A 2-axis Fsa (single FSA) is stored as a 3-axis one with one entry and
 `single=True`, which is how the reference lifts it before every FsaVec
 algorithm (k2/python/csrc/torch/fsa_algo.cu:236-238).
 """
+import ctypes
 from typing import Optional
 
 import numpy as np
@@ -140,6 +141,11 @@ class RaggedArc:
             dev = self.device
             in_splits = torch.empty(ns + 1, dtype=torch.int32, device=dev)
             buf = torch.empty((3, max(na, 1)), dtype=torch.int32, device=dev)
+            if self._layer_bounds[0] and self._incoming_by_layers(in_splits, buf):
+                self._incoming = (in_splits, buf[0, :na], buf[1, :na],
+                                  buf[2, :na].view(torch.float32))
+                self._incoming_key = key
+                return self._incoming
             tmp = torch.empty(_lib.lib.k2b200_fsa_incoming_tmp_bytes(ns, na), dtype=torch.uint8,
                               device=dev)
             with torch.cuda.device(dev):
@@ -152,6 +158,18 @@ class RaggedArc:
                               buf[2, :na].view(torch.float32))
             self._incoming_key = key
         return self._incoming
+
+    def _incoming_by_layers(self, in_splits: torch.Tensor, buf: torch.Tensor) -> bool:
+        """k2b200_fsa_incoming_layers: the incoming-arc index of a lattice, layer by
+        layer.  False when a layer is too wide for it."""
+        view, keep = self.view(want_incoming=False)
+        done = _lib.c_i32()
+        with torch.cuda.device(self.device):
+            _lib.check(_lib.lib.k2b200_fsa_incoming_layers(
+                ctypes.byref(view), in_splits.data_ptr(), buf[0].data_ptr(), buf[1].data_ptr(),
+                buf[2].data_ptr(), ctypes.byref(done), _lib.stream_of(self.device)))
+        del keep
+        return bool(done.value)
 
     def band_tables(self):
         """(band_states, band_arcs, ok): the per-state tables of k2b200_band_tables
@@ -169,7 +187,6 @@ class RaggedArc:
         dev = self.device
         ns = self.num_states
         sb, ab = _lib.c_sz(), _lib.c_sz()
-        import ctypes
         _lib.check(_lib.lib.k2b200_band_tables_bytes(ns, ctypes.byref(sb), ctypes.byref(ab)))
         states = torch.empty(sb.value, dtype=torch.uint8, device=dev)
         arcs = torch.empty(ab.value, dtype=torch.uint8, device=dev)
