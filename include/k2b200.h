@@ -670,6 +670,15 @@ int32_t k2b200_fsa_levels(const int32_t *row_splits1, const int32_t *row_splits2
                           int32_t num_states, int32_t num_arcs, int32_t *level_offsets,
                           int32_t *level_splits, int32_t *status, void *tmp, void *stream);
 
+/* Best paths of a layered view (max_layers set; row_splits1, arcs and the layering are
+ * read) as linear FSAs, in two launches and without a host read: path_splits[num_fsas+1],
+ * row_splits1[num_fsas+1], row_splits2 (room for num_fsas*(max_layers+1)+1), arcs and
+ * best_arcs (arc of the view; room for num_fsas*max_layers). */
+size_t k2b200_best_paths_tmp_bytes(const k2b200_fsa_view *fsas);
+int32_t k2b200_best_paths(const k2b200_fsa_view *fsas, const int32_t *entering_arcs,
+                          int32_t *path_splits, int32_t *row_splits1, int32_t *row_splits2,
+                          void *arcs, int32_t *best_arcs, void *tmp, void *stream);
+
 /* Per-FSA property bits (k2/csrc/fsa.h:75-101) and their AND.
  * Replaces k2::GetFsaVecBasicProperties, k2/csrc/fsa.cu:54-217.  tmp must hold
  * k2b200_fsa_properties_tmp_bytes(...) bytes; properties[num_fsas+1] is written

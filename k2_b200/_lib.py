@@ -220,6 +220,9 @@ _sig("k2b200_dense_fsa_vec_from_logits_backward", c_i32,
      [c_vp, c_vp, c_i64, c_i64, c_i32, c_vp, c_vp, c_i32, c_i32, c_i32, c_vp, c_vp])
 _sig("k2b200_shortest_path_tmp_bytes", c_sz, [c_i32])
 _sig("k2b200_shortest_path", c_i32, [c_vp, c_vp, c_vp, c_i32, c_vp, c_vp, c_vp, c_vp])
+_sig("k2b200_best_paths_tmp_bytes", c_sz, [ctypes.POINTER(FsaView)])
+_sig("k2b200_best_paths", c_i32,
+     [ctypes.POINTER(FsaView), c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp])
 _sig("k2b200_fsa_properties_tmp_bytes", c_sz, [c_i32, c_i32])
 _sig("k2b200_fsa_properties", c_i32,
      [c_vp, c_vp, c_vp, c_vp, c_vp, c_i32, c_i32, c_i32, c_vp, c_vp, c_vp])
@@ -244,7 +247,8 @@ EXPORTED = [
     "k2b200_fsa_scores_scratch_bytes",
     "k2b200_fsa_tot_scores", "k2b200_fsa_arc_post", "k2b200_tot_scores_log_backward",
     "k2b200_tot_scores_tropical_backward", "k2b200_index_add", "k2b200_index_select_i32",
-    "k2b200_shortest_path_tmp_bytes", "k2b200_shortest_path",
+    "k2b200_shortest_path_tmp_bytes", "k2b200_shortest_path", "k2b200_best_paths_tmp_bytes",
+    "k2b200_best_paths",
     "k2b200_dense_fsa_vec_fill", "k2b200_dense_fsa_vec_backward",
     "k2b200_dense_fsa_vec_from_logits", "k2b200_dense_fsa_vec_from_logits_backward",
     "k2b200_ctc_graph_tmp_bytes", "k2b200_ctc_graph",

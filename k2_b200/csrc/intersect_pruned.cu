@@ -877,8 +877,9 @@ struct FormatArgs {
   int32_t *level_offsets, *level_splits;
 };
 
-// Lattice of one (sequence, frame) per CTA (FormatOutput, :474-657): the arenas are
-// already in [sequence][frame][state][arc] order.
+// Lattice of one (sequence, frame) (FormatOutput, :474-657): the arenas are already in
+// [sequence][frame][state][arc] order.  gridDim.z CTAs share the states of a frame: with one
+// of them the widest frame (10^4 states) took as long as all others together.
 __global__ void FormatPruned(const FormatArgs f) {
   const SearchArgs &g = f.g;
   const int32_t seq = blockIdx.y, t = blockIdx.x;  // t in [0, T + 1]
@@ -886,7 +887,8 @@ __global__ void FormatPruned(const FormatArgs f) {
   const int32_t row0 = g.b_rs[seq], final_t = g.b_rs[seq + 1] - row0;
   const int32_t sb = f.out_rs1[seq], ab = f.arc_base[seq];
   const int32_t s0 = v.frame_s0[t], s1 = v.frame_s0[t + 1];
-  if (f.level_splits != nullptr && threadIdx.x == 0) {
+  const bool first = blockIdx.z == 0;
+  if (f.level_splits != nullptr && first && threadIdx.x == 0) {
     f.level_splits[(int64_t)seq * (g.T + 2) + t] = sb + s0;
     if (t == 0) f.level_offsets[seq] = seq * (g.T + 2);
     if (seq == g.num_seqs - 1 && t == g.T + 1) {
@@ -896,7 +898,7 @@ __global__ void FormatPruned(const FormatArgs f) {
   }
   if (t == g.T + 1) {
     // the extra final state, if any, and the end of the row_splits
-    if (threadIdx.x == 0) {
+    if (first && threadIdx.x == 0) {
       const int32_t extra = g.seq_out[kSeqOut * seq + 2];
       if (extra) {
         f.row_ids1[sb + s0] = seq;
@@ -907,7 +909,8 @@ __global__ void FormatPruned(const FormatArgs f) {
     return;
   }
   const int32_t next_s0 = s1;  // the states of frame t + 1 start where frame t ends
-  for (int32_t k = s0 + threadIdx.x; k < s1; k += blockDim.x) {
+  for (int32_t k = s0 + blockIdx.z * blockDim.x + threadIdx.x; k < s1;
+       k += gridDim.z * blockDim.x) {
     const int32_t p0 = v.st_arc0[k], p1 = v.st_arc0[k + 1];
     f.row_ids1[sb + k] = seq;
     f.row_splits2[sb + k] = ab + p0;
@@ -931,6 +934,11 @@ __global__ void FormatPruned(const FormatArgs f) {
   }
 }
 
+
+// CTAs per frame: about 16 per SM in all, however few the frames are.
+unsigned FormatParts(int64_t frames, int64_t seqs) {
+  return (unsigned)std::max<int64_t>(1, std::min<int64_t>(32, 148 * 16 / (frames * seqs)));
+}
 
 // ---------------------------------------------------------------------------
 // Chunk-by-chunk decoding (OnlineDenseIntersecter, k2/csrc/intersect_dense_pruned.cu:
@@ -1120,14 +1128,15 @@ __global__ void FormatOnline(const FormatArgs f, const int32_t *__restrict__ his
   const int32_t end = hist[seq] + chunk;  // the frontier
   if (t > end + 1) return;
   const int32_t sb = f.out_rs1[seq], ab = f.arc_base[seq];
-  if (f.level_splits != nullptr && threadIdx.x == 0) {
+  const bool first = blockIdx.z == 0;
+  if (f.level_splits != nullptr && first && threadIdx.x == 0) {
     // frames are layers; the final state is a layer of its own
     const int32_t lo = f.level_offsets[seq];
     f.level_splits[lo + t] = sb + v.frame_s0[t];
     if (seq == g.num_seqs - 1 && t == end + 1) f.level_splits[lo + t + 1] = f.out_rs1[g.num_seqs];
   }
   if (t == end + 1) {
-    if (threadIdx.x == 0) {
+    if (first && threadIdx.x == 0) {
       const int32_t s_top = v.frame_s0[end + 1];
       f.row_ids1[sb + s_top] = seq;
       f.row_splits2[sb + s_top] = ab + v.frame_a0[end + 1];
@@ -1136,7 +1145,8 @@ __global__ void FormatOnline(const FormatArgs f, const int32_t *__restrict__ his
     return;
   }
   const int32_t s0 = v.frame_s0[t], s1 = v.frame_s0[t + 1];
-  for (int32_t k = s0 + threadIdx.x; k < s1; k += blockDim.x) {
+  for (int32_t k = s0 + blockIdx.z * blockDim.x + threadIdx.x; k < s1;
+       k += gridDim.z * blockDim.x) {
     const int32_t p0 = v.st_arc0[k], p1 = v.st_arc0[k + 1];
     f.row_ids1[sb + k] = seq;
     f.row_splits2[sb + k] = ab + p0;
@@ -1240,8 +1250,9 @@ int32_t MakePrunedLayout(const k2b200_pruned_args *a, char *ws, PrunedLayout *L)
 }
 
 
-// Many small device-to-device copies in one launch (the eight arrays of every stream):
-// one CTA per copy, 4-byte elements.
+// Many device-to-device copies in one launch (the eight arrays of every stream): grid =
+// (copies, parts of a copy), 4-byte elements.  A stream's history runs to millions of arcs;
+// one CTA per copy took 400 us for the arrays of four streams.
 struct CopyJob {
   const int32_t *src;
   int32_t *dst;
@@ -1249,7 +1260,16 @@ struct CopyJob {
 };
 __global__ void CopyMany(const CopyJob *__restrict__ jobs) {
   const CopyJob j = jobs[blockIdx.x];
-  for (int64_t k = threadIdx.x; k < j.count; k += blockDim.x) j.dst[k] = j.src[k];
+  const int64_t step = (int64_t)gridDim.y * blockDim.x;
+  for (int64_t k = (int64_t)blockIdx.y * blockDim.x + threadIdx.x; k < j.count; k += 4 * step) {
+    int32_t x[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (k + u * step < j.count) x[u] = j.src[k + u * step];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (k + u * step < j.count) j.dst[k + u * step] = x[u];
+  }
 }
 
 // The online entry points share the arena layout of the batch search: the frame
@@ -1449,7 +1469,7 @@ int32_t k2b200_intersect_dense_pruned_emit(const k2b200_pruned_args *args, void 
   f.level_splits = out->level_splits;
   K2B_CUDA_OK(cudaMemcpyAsync(out->row_splits1, L.out_rs1, sizeof(int32_t) * (args->num_seqs + 1),
                               cudaMemcpyDeviceToDevice, stream));
-  dim3 grid(L.g.T + 2, args->num_seqs);
+  dim3 grid(L.g.T + 2, args->num_seqs, FormatParts(L.g.T + 2, args->num_seqs));
   { FormatPruned<<<grid, 128, 0, stream>>>(f); NoteLaunch(); }
   K2B_CUDA_OK(cudaGetLastError());
   return kOk;
@@ -1618,7 +1638,7 @@ int32_t k2b200_online_decode_emit(const k2b200_online_args *args, void *workspac
   K2B_CUDA_OK(cudaMemcpyAsync(out->row_splits1, L.base.out_rs1,
                               sizeof(int32_t) * (args->num_seqs + 1), cudaMemcpyDeviceToDevice,
                               stream));
-  dim3 grid(L.base.g.T + 2, args->num_seqs);
+  dim3 grid(L.base.g.T + 2, args->num_seqs, FormatParts(L.base.g.T + 2, args->num_seqs));
   { FormatOnline<<<grid, 128, 0, stream>>>(f, L.hist, L.chunk); NoteLaunch(); }
   K2B_CUDA_OK(cudaGetLastError());
   return kOk;
@@ -1691,7 +1711,12 @@ static int32_t CopyStreams(const k2b200_online_args *args, void *workspace,
   K2B_FORWARD(UploadInts(reinterpret_cast<const int32_t *>(jobs.data()),
                          (int64_t)(jobs.size() * sizeof(CopyJob) / 4),
                          reinterpret_cast<int32_t *>(L.jobs), stream));
-  { CopyMany<<<(unsigned)jobs.size(), 256, 0, stream>>>(L.jobs); NoteLaunch(); }
+  int64_t longest = 1;
+  for (const CopyJob &j : jobs) longest = std::max(longest, j.count);
+  // about 8 CTAs per SM when the copies are long
+  const int32_t parts = (int32_t)std::max<int64_t>(
+      1, std::min<int64_t>(CeilDiv(longest, 1024), 148 * 8 / (int64_t)jobs.size() + 1));
+  { CopyMany<<<dim3((unsigned)jobs.size(), parts), 256, 0, stream>>>(L.jobs); NoteLaunch(); }
   K2B_CUDA_OK(cudaGetLastError());
   return kOk;
 }

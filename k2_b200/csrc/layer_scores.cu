@@ -165,7 +165,8 @@ int32_t BuildLayerIncoming(const k2b200_fsa_view *v, int32_t *in_splits, int32_t
   const int32_t maxw = std::max(v->max_layer_states, 1);
   const int64_t levels = (int64_t)v->max_layers * v->num_fsas;  // at least the true number
   if (!v->strict_layers || levels <= 0 || levels >= ((int64_t)1 << 31)) return kOk;
-  // a warp per layer while layers are small (there are many of them), else four
+  // a warp per layer while layers are small (there are many of them), else four; with fewer
+  // for the widest layers (10^4 states, 4 10^4 arcs) sorting the whole FsaVec is faster
   const bool one = maxw <= 1024 && v->num_arcs / levels <= 1024;
   const size_t smem = sizeof(int32_t) * 4 * (size_t)maxw;
   if (smem > kLayerSmemBudget) return kOk;
@@ -712,19 +713,20 @@ LayerChainWide(k2b200_fsa_view v, const LayerArc *__restrict__ fwd_arcs,
   sc.End(lane, status);
 }
 
-// out[s] = log(m[s]) + scale of its layer * ln 2.  grid = (layer tiles, fsas), a warp per
-// layer.  m and out may be the same array.
+// out[s] = log(m[s]) + scale of its layer * ln 2.  grid = (layer tiles, fsas, parts of a
+// layer), `lanes` threads (a power of two) on a part.  m and out may be the same array.
 template <typename Real>
 __global__ void __launch_bounds__(128)
 FinishLayerScores(k2b200_fsa_view v, const double *m, const int32_t *__restrict__ scale,
-                  int32_t nl_cap, int32_t fsa_base, Real *out) {
-  const int lane = threadIdx.x & 31;
-  const int32_t i = fsa_base + blockIdx.y, l = blockIdx.x * 4 + (threadIdx.x >> 5);
+                  int32_t nl_cap, int32_t fsa_base, int32_t lanes, Real *out) {
+  const int32_t lane = threadIdx.x & (lanes - 1);
+  const int32_t i = fsa_base + blockIdx.y,
+                l = (blockIdx.x * blockDim.x + threadIdx.x) / (unsigned)lanes;
   const int32_t lv = v.level_offsets[i] + l;
   if (l >= nl_cap || lv >= v.level_offsets[i + 1]) return;
   const int32_t b = v.level_splits[lv], e = v.level_splits[lv + 1];
   const double shift = (double)scale[(int64_t)i * nl_cap + l] * 0.69314718055994530942;
-  for (int32_t s = b + lane; s < e; s += 32) {
+  for (int32_t s = b + (int32_t)blockIdx.z * lanes + lane; s < e; s += (int32_t)gridDim.z * lanes) {
     const double x = m[s];
     out[s] = x == 0.0 ? (Real)-INFINITY : (Real)(log(x) + shift);
   }
@@ -836,10 +838,16 @@ int32_t LaunchLayerScores(const k2b200_fsa_view *v, int32_t log_semiring, Real *
       Real *out = dir == 0 ? fwd : bwd;
       if (out == nullptr) continue;
       for (int32_t first = 0; first < v->num_fsas; first += 65535) {
-        dim3 grid(CeilDiv(p.nl_cap, 4), std::min(v->num_fsas - first, 65535));
+        // a few states per thread of a mean layer
+        const int32_t mean_w =
+            (int32_t)(v->num_states / std::max<int64_t>((int64_t)v->num_fsas * p.nl_cap, 1));
+        int32_t lanes = 4;
+        while (lanes < 128 && lanes < mean_w) lanes *= 2;
+        dim3 grid(CeilDiv((int64_t)p.nl_cap * lanes, 128), std::min(v->num_fsas - first, 65535),
+                  std::min(16, 1 + mean_w / 512));
         { FinishLayerScores<Real><<<grid, 128, 0, stream>>>(
             *v, dir == 0 ? vf : vb, c.scale + (int64_t)dir * v->num_fsas * p.nl_cap, p.nl_cap,
-            first, out); NoteLaunch(); }
+            first, lanes, out); NoteLaunch(); }
       }
     }
   } else {

@@ -126,6 +126,121 @@ __global__ void PathFill(const int32_t *__restrict__ row_splits1, const Arc *__r
   }
 }
 
+// ---------------------------------------------------------------------------
+// Best paths of a layered FsaVec (arcs go from one layer to a later one, as in lattices).  The
+// trace back is a chain of dependent loads; read from global memory a step costs two of them,
+// about half a microsecond (800 frames: 430 us, and as much again to fill the paths in once
+// their lengths are known).  Here a CTA per FSA brings the predecessors of a run of layers
+// into shared memory with all its threads, one thread follows the path through them, and
+// all of them write the arcs that it took: best[i * max_layers + k] is the k-th last arc.
+// ---------------------------------------------------------------------------
+constexpr int kTraceStates = 8192;  // predecessors in shared memory
+constexpr int kTraceLayers = 512;   // layers of a run at most, one per thread and trip
+constexpr int kTraceFew = 24;       // runs of fewer layers are followed in global memory: to
+                                    // fetch 8192 predecessors takes as long as 20 steps there
+
+__global__ void __launch_bounds__(512)
+TraceLayers(k2b200_fsa_view v, const int32_t *__restrict__ entering, int32_t *__restrict__ best,
+            int32_t *__restrict__ lengths) {
+  __shared__ int32_t pred[kTraceStates], path[kTraceLayers];
+  __shared__ int32_t cur_sh, steps_sh;
+  const int32_t i = blockIdx.x;
+  const int tid = threadIdx.x;
+  const int32_t s_begin = v.row_splits1[i], s_end = v.row_splits1[i + 1];
+  const Arc *arcs = reinterpret_cast<const Arc *>(v.arcs);
+  int32_t *out = best + (int64_t)i * v.max_layers;
+  int32_t len = 0, cur = s_end - 1, hi = v.level_offsets[i + 1];
+  const int32_t lv0 = v.level_offsets[i];
+  bool alive = s_end > s_begin;
+  while (alive && hi > lv0 && len <= v.max_layers) {
+    // as many layers below `hi` as fit
+    const int32_t top = v.level_splits[hi];
+    const int32_t l = hi - 1 - tid;
+    const int32_t n = __syncthreads_count(l >= lv0 && top - v.level_splits[l] <= kTraceStates);
+    const int32_t lo = hi - max(n, 1), base = v.level_splits[lo];
+    const bool staged = n >= min(kTraceFew, hi - lv0);
+    if (staged)
+      for (int32_t s = base + tid; s < top; s += blockDim.x) {
+        const int32_t a = entering[s];
+        pred[s - base] = a >= 0 ? s_begin + arcs[a].src : -1;
+      }
+    __syncthreads();
+    if (tid == 0) {
+      int32_t k = 0;
+      while (cur >= base && cur < top && k < kTraceLayers && len + k < v.max_layers) {
+        int32_t from;
+        if (staged) {
+          from = pred[cur - base];
+        } else {
+          const int32_t a = entering[cur];
+          from = a >= 0 ? s_begin + arcs[a].src : -1;
+        }
+        if (from < 0) {
+          cur = -1 - cur;  // the path begins at this state
+          break;
+        }
+        path[k++] = cur;
+        cur = from;
+      }
+      cur_sh = cur;
+      steps_sh = k;
+    }
+    __syncthreads();
+    for (int32_t k = tid; k < steps_sh; k += blockDim.x) out[len + k] = entering[path[k]];
+    cur = cur_sh;
+    len += steps_sh;
+    alive = cur >= 0;
+    hi = lo;
+    __syncthreads();
+  }
+  // (a path ends where no arc enters: only at the start state is it complete)
+  if (tid == 0) lengths[i] = cur == -1 - s_begin && s_end > s_begin ? len : 0;
+}
+
+// The paths as linear FSAs: arcs (states renumbered, labels and scores kept), the lattice arc
+// of each, the row splits.  One CTA per FSA.
+__global__ void __launch_bounds__(128)
+WritePaths(const Arc *__restrict__ arcs, const int32_t *__restrict__ traced,
+           const int32_t *__restrict__ lengths, int32_t num_fsas, int32_t max_layers,
+           int32_t *__restrict__ path_splits, int32_t *__restrict__ row_splits1,
+           int32_t *__restrict__ row_splits2, Arc *__restrict__ out, int32_t *__restrict__ best) {
+  __shared__ int32_t arcs_before, paths_before;
+  const int32_t i = blockIdx.x;
+  if (threadIdx.x == 0) arcs_before = paths_before = 0;
+  __syncthreads();
+  int32_t na = 0, np = 0;
+  for (int32_t j = threadIdx.x; j < i; j += blockDim.x) {
+    na += lengths[j];
+    np += lengths[j] > 0;
+  }
+  if (na) {
+    atomicAdd(&arcs_before, na);
+    atomicAdd(&paths_before, np);
+  }
+  __syncthreads();
+  const int32_t p0 = arcs_before, s0 = p0 + paths_before, len = lengths[i];
+  for (int32_t k = threadIdx.x; k < len; k += blockDim.x) {
+    const int32_t a = traced[(int64_t)i * max_layers + (len - 1 - k)];
+    Arc arc = arcs[a];
+    arc.src = k;
+    arc.dest = k + 1;
+    out[p0 + k] = arc;
+    best[p0 + k] = a;
+    row_splits2[s0 + k] = p0 + k;
+  }
+  if (threadIdx.x == 0) {
+    path_splits[i] = p0;
+    row_splits1[i] = s0;
+    if (len > 0) row_splits2[s0 + len] = p0 + len;
+    if (i == num_fsas - 1) {
+      const int32_t s1 = s0 + (len > 0 ? len + 1 : 0);
+      path_splits[num_fsas] = p0 + len;
+      row_splits1[num_fsas] = s1;
+      row_splits2[s1] = p0 + len;
+    }
+  }
+}
+
 constexpr int32_t kAllProps = 0x1FF;
 
 __global__ void PropsInit(int32_t *props, int32_t n_plus_one, char *reach, int64_t nreach) {
@@ -434,6 +549,34 @@ int32_t k2b200_shortest_path(const int32_t *row_splits1, const void *arcs,
   K2B_FORWARD(ExclusiveSum(lengths, path_splits, num_fsas, scan_tmp, STREAM(stream)));
   { PathFill<<<CeilDiv(num_fsas, 64), 64, 0, STREAM(stream)>>>(row_splits1, a, entering_arcs,
                                                             num_fsas, path_splits, best_arcs); NoteLaunch(); }
+  K2B_CUDA_OK(cudaGetLastError());
+  return kOk;
+}
+
+size_t k2b200_best_paths_tmp_bytes(const k2b200_fsa_view *v) {
+  if (v == nullptr) return 0;
+  return AlignUp(sizeof(int32_t) * ((size_t)v->num_fsas + 1)) +
+         AlignUp(sizeof(int32_t) * (size_t)v->num_fsas * (size_t)v->max_layers);
+}
+
+int32_t k2b200_best_paths(const k2b200_fsa_view *v, const int32_t *entering_arcs,
+                          int32_t *path_splits, int32_t *row_splits1, int32_t *row_splits2,
+                          void *arcs, int32_t *best_arcs, void *tmp, void *stream) {
+  K2B_REQUIRE(v && entering_arcs && path_splits && row_splits1 && row_splits2 && arcs &&
+                  best_arcs && tmp,
+              "NULL pointer");
+  K2B_REQUIRE(v->row_splits1 && v->level_offsets && v->level_splits && v->max_layers > 0,
+              "k2b200_best_paths needs a layered view");
+  if (v->num_fsas <= 0) return kOk;
+  int32_t *lengths = reinterpret_cast<int32_t *>(tmp);
+  int32_t *traced = reinterpret_cast<int32_t *>(
+      reinterpret_cast<char *>(tmp) + AlignUp(sizeof(int32_t) * ((size_t)v->num_fsas + 1)));
+  { TraceLayers<<<v->num_fsas, 512, 0, STREAM(stream)>>>(*v, entering_arcs, traced, lengths);
+    NoteLaunch(); }
+  { WritePaths<<<v->num_fsas, 128, 0, STREAM(stream)>>>(
+      reinterpret_cast<const Arc *>(v->arcs), traced, lengths, v->num_fsas, v->max_layers,
+      path_splits, row_splits1, row_splits2, reinterpret_cast<Arc *>(arcs), best_arcs);
+    NoteLaunch(); }
   K2B_CUDA_OK(cudaGetLastError());
   return kOk;
 }

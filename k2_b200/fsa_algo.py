@@ -4,6 +4,7 @@
 k2::ShortestPath, fsa_algo.cu:869-1144)."""
 from typing import List, Optional, Tuple, Union
 
+import ctypes
 import itertools
 
 import numpy as np
@@ -242,10 +243,40 @@ def arc_sort(fsa: Fsa, ret_arc_map: bool = False):
     return (ans, amap) if ret_arc_map else ans
 
 
+def _best_paths(fsa: Fsa, use_double_scores: bool):
+    """(path splits on the host [num_fsas+1], row_splits1, row_splits2, arcs, best arcs) of
+    the best paths of a lattice (k2b200_best_paths); the splits are the only host read."""
+    arcs = fsa.arcs
+    dev = arcs.device
+    entering = fsa._get_entering_arcs(use_double_scores)
+    nf, most = arcs.num_fsas, arcs._layer_bounds[1]
+    view, keep = arcs.view(want_incoming=False)
+    n = nf * most
+    buf = torch.empty(2 * (nf + 1) + n + (n + nf + 1), dtype=torch.int32, device=dev)
+    path_splits, row_splits1 = buf[:nf + 1], buf[nf + 1:2 * nf + 2]
+    best, row_splits2 = buf[2 * nf + 2:2 * nf + 2 + n], buf[2 * nf + 2 + n:]
+    values = torch.empty((n, 4), dtype=torch.int32, device=dev)
+    tmp = torch.empty(_lib.lib.k2b200_best_paths_tmp_bytes(ctypes.byref(view)), dtype=torch.uint8,
+                      device=dev)
+    with torch.cuda.device(dev):
+        _lib.check(_lib.lib.k2b200_best_paths(
+            ctypes.byref(view), _lib.ptr(entering), path_splits.data_ptr(),
+            row_splits1.data_ptr(), row_splits2.data_ptr(), _lib.ptr(values), _lib.ptr(best),
+            _lib.ptr(tmp), _lib.stream_of(dev)))
+    del keep
+    h_splits = path_splits.cpu().numpy()
+    total = int(h_splits[-1])
+    states = total + int(np.count_nonzero(np.diff(h_splits)))
+    return h_splits, row_splits1, row_splits2[:states + 1], values[:total], best[:total]
+
+
 def _shortest_path_arcs(fsa: Fsa, use_double_scores: bool) -> Tuple[torch.Tensor, torch.Tensor]:
     """(path_splits [num_fsas+1], best arc indexes in path order)."""
     arcs = fsa.arcs
     dev = arcs.device
+    if arcs._layer_bounds[0]:
+        h_splits, _, _, _, best = _best_paths(fsa, use_double_scores)
+        return torch.from_numpy(h_splits), best
     entering = fsa._get_entering_arcs(use_double_scores)
     nf = arcs.num_fsas
     path_splits = torch.empty(nf + 1, dtype=torch.int32, device=dev)
@@ -264,6 +295,13 @@ def shortest_path(fsa: Fsa, use_double_scores: bool) -> Fsa:
     between equally good entering arcs go to the one with the higher arc index.
     Per-arc tensor attributes are carried along; `arc_map` of the result is kept
     in the attribute `_best_arc_map`."""
+    if fsa.arcs._layer_bounds[0]:
+        h_splits, rs1, rs2, values, best = _best_paths(fsa, use_double_scores)
+        h_rs1 = h_splits.copy()
+        np.cumsum(np.diff(h_splits) > 0, out=h_rs1[1:])
+        h_rs1 += h_splits
+        return _with_attributes(fsa, RaggedArc(values, rs1, rs2, h_row_splits1=h_rs1,
+                                               h_arc_splits=h_splits), best)
     path_splits, best = _shortest_path_arcs(fsa, use_double_scores)
     dev = fsa.device
     src_vals = fsa.arcs.values()
@@ -287,6 +325,11 @@ def shortest_path(fsa: Fsa, use_double_scores: bool) -> Fsa:
                      torch.from_numpy(rs2.astype(np.int32)).to(dev),
                      h_row_splits1=rs1.astype(np.int32),
                      h_arc_splits=rs2[rs1].astype(np.int32))
+    return _with_attributes(fsa, arcs, best)
+
+
+def _with_attributes(fsa: Fsa, arcs: RaggedArc, best: torch.Tensor) -> Fsa:
+    """The best paths `arcs` with the attributes of `fsa` carried through the arc map."""
     ans = Fsa(arcs, _check=False)
     for name, value in fsa.named_tensor_attr(include_scores=False):
         if name != 'labels':

@@ -96,7 +96,11 @@ class OnlineDenseIntersecter:
         chunk = int(h_brs[1] - h_brs[0]) - 1
         need_a = max(s.arc_graph.numel() for s in states)
         need_s = max(s.astate.numel() for s in states)
-        cap_a = max(self._arcs_per_seq, 2 * need_a, 4 * need_s)
+        # what the chunk may add: every frame the arcs of max_active_states states (a retry
+        # with four times as much costs the whole chunk again)
+        per_frame = self.max_active_states * (arcs.num_elements() // max(arcs.num_states, 1) + 1)
+        grow = min(chunk * min(per_frame, arcs.num_elements()), (1 << 26) // max(n, 1))
+        cap_a = max(self._arcs_per_seq, 2 * need_a, 4 * need_s, need_a + grow)
         stream = _lib.stream_of(dev)
         i32 = dict(dtype=torch.int32, device=dev)
         bounds = (ctypes.c_int32 * 2)()
