@@ -21,7 +21,6 @@
 namespace k2b {
 
 constexpr int kCountThreads = 256;
-constexpr int kWordsPerCtaHost = 4 * 4 * (kCountThreads / 32);  // == kWordsPerCta below
 
 int32_t MakeLayout(const k2b200_intersect_args *a, Layout *L) {
   K2B_REQUIRE(a != nullptr, "args is NULL");
@@ -89,12 +88,14 @@ int32_t MakeLayout(const k2b200_intersect_args *a, Layout *L) {
   L->grid_elems = grid;
   L->total_words = words;
   L->total_levels = levels;
-  // CountKept / EmitLattice run on a (word tiles of the largest pair, pairs) grid
+  // CountKept / EmitLattice run on a (word tiles of the largest pair, pairs) grid.  With many
+  // words, most of them empty, a warp takes 16; with few it takes one, so that all SMs have
+  // warps to run (about 64 per SM until every warp has one word).
   int64_t max_pair_words = 0;
   for (const FsaInfo &f : L->infos)
     max_pair_words = std::max<int64_t>(max_pair_words, (int64_t)(f.tk + 1) * f.words);
-  L->tiles_per_pair = CeilDiv(max_pair_words, kWordsPerCtaHost);
-  L->emit_tiles_per_pair = CeilDiv(max_pair_words, 16 * 8);  // kEmitWordsPerCta
+  L->words_per_warp = (int32_t)std::max<int64_t>(1, std::min<int64_t>(16, words / (148 * 64)));
+  L->tiles_per_pair = CeilDiv(max_pair_words, (int64_t)L->words_per_warp * (kCountThreads / 32));
   L->count_blocks = (int32_t)std::min<int64_t>((int64_t)L->tiles_per_pair * a->num_fsas,
                                                0x7fffffff);
   size_t off = 0;
@@ -228,15 +229,42 @@ __device__ __forceinline__ bool KeepArc(const Arc &arc, float fs, const float *f
   return __fadd_rn(__fadd_rn(fs, sc), bd) > cutoff;
 }
 
-// Each warp handles kWordsPerWarp consecutive 32-state words of the (pair, t, state)
-// grid; the loads of all its words are issued before any is used.  Most words hold
-// no surviving state and cost two loads, a ballot and one 12-byte store.
-constexpr int kWordsPerWarp = 4;
-constexpr int kCountRounds = 4;
-constexpr int kWordsPerCta = kCountRounds * kWordsPerWarp * (kCountThreads / 32);
+// The arcs leaving the states of one 32-state word are taken as one flat range, 32 arcs at a
+// time: a lane finds the state of its arc by a search over the 32 range starts held in
+// registers.  (One lane per state walked its arcs one after the other, three dependent
+// gathers each: on a denominator graph of up to 32 arcs per state the pass over 6.7 M
+// surviving arcs took 267 us, and 846 us with the output.)
+// deg = arcs leaving this lane's state (0: not kept), a0 = the first of them.  visit(valid,
+// j, a, start, first) is called by all lanes for every batch: j = lane that owns arc a,
+// start = this lane's range start, first = range position of the batch.
+template <typename Visit>
+__device__ __forceinline__ void ForArcsOfWord(int lane, int32_t a0, int32_t deg, Visit visit) {
+  constexpr unsigned kAll = 0xffffffffu;
+  int32_t inc = deg;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int32_t o = __shfl_up_sync(kAll, inc, d);
+    if (lane >= d) inc += o;
+  }
+  const int32_t start = inc - deg, total = __shfl_sync(kAll, inc, 31);
+  for (int32_t first = 0; first < total; first += 32) {
+    const int32_t p = first + lane;
+    int32_t j = 0;  // largest lane whose range starts at or before p
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1)
+      if (__shfl_sync(kAll, start, j + step) <= p) j += step;
+    const int32_t js = __shfl_sync(kAll, start, j), ja = __shfl_sync(kAll, a0, j);
+    visit(p < total, j, ja + (p - js), start, first);
+  }
+}
+
+// Each warp handles words_per_warp consecutive 32-state words of the (pair, t, state)
+// grid, up to four at a time so that their loads are issued before any is used.  Most words
+// of a CTC grid hold no surviving state and cost two loads, a ballot and one 12-byte store.
+constexpr int kWordsAtOnce = 4;
 
 __global__ void __launch_bounds__(kCountThreads)
-CountKept(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_words,
+CountKept(const FsaInfo *__restrict__ infos, int32_t words_per_warp,
           const Arc *__restrict__ arcs, const int32_t *__restrict__ a_row_splits2,
           const float *__restrict__ scores, int32_t cols, const float *__restrict__ fwd,
           const float *__restrict__ bwd, const float *__restrict__ cutoffs,
@@ -252,75 +280,68 @@ CountKept(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_words,
   const int32_t S = f.num_states;
   const float cutoff = cutoffs[i];
   const float *fgrid = fwd + f.grid_off, *bgrid = bwd + f.grid_off;
-  int32_t cand = 0;
-  bool any = false;
-  for (int round = 0; round < kCountRounds; ++round) {
-  const int64_t rel0 = (int64_t)blockIdx.x * kWordsPerCta +
-                       ((int64_t)round * (kCountThreads / 32) + warp) * kWordsPerWarp;
-  if (rel0 >= pair_words) break;  // warp-uniform
-  float fs[kWordsPerWarp], bs[kWordsPerWarp];
-  int32_t ts[kWordsPerWarp], ss[kWordsPerWarp];
-  // (level, word) of the warp's first word by one 32-bit division (a pair has fewer than
-  // 2^31 words), of the following ones by stepping
-  int32_t t_run = (int32_t)((uint32_t)rel0 / (uint32_t)f.words);
-  int32_t w_run = (int32_t)((uint32_t)rel0 - (uint32_t)t_run * (uint32_t)f.words);
+  unsigned long long cand = 0;
+  const int64_t warp0 =
+      ((int64_t)blockIdx.x * (kCountThreads / 32) + warp) * (int64_t)words_per_warp;
+  const int64_t warp1 = min(warp0 + words_per_warp, pair_words);
+  for (int64_t rel0 = warp0; rel0 < warp1; rel0 += kWordsAtOnce) {
+    float fs[kWordsAtOnce], bs[kWordsAtOnce];
+    int32_t ts[kWordsAtOnce], ss[kWordsAtOnce];
+    // (level, word) of the first word by one 32-bit division (a pair has fewer than 2^31
+    // words), of the following ones by stepping
+    int32_t t_run = (int32_t)((uint32_t)rel0 / (uint32_t)f.words);
+    int32_t w_run = (int32_t)((uint32_t)rel0 - (uint32_t)t_run * (uint32_t)f.words);
 #pragma unroll
-  for (int u = 0; u < kWordsPerWarp; ++u) {
-    const int64_t rel = rel0 + u;
-    const int32_t t = t_run, s = w_run * 32 + lane;
-    if (++w_run == f.words) {
-      w_run = 0;
-      ++t_run;
-    }
-    ts[u] = t;
-    ss[u] = s;
-    const bool in = rel < pair_words && s < S;
-    fs[u] = in ? fgrid[(int64_t)t * S + s] : -INFINITY;
-    bs[u] = in ? bgrid[(int64_t)t * S + s] : -INFINITY;
-  }
-#pragma unroll
-  for (int u = 0; u < kWordsPerWarp; ++u) {
-    const int64_t rel = rel0 + u;
-    if (rel >= pair_words) break;  // warp-uniform
-    const bool keep = __fadd_rn(fs[u], bs[u]) > cutoff;
-    const uint32_t m = __ballot_sync(0xffffffffu, keep);
-    const int64_t w = f.word_off + rel;
-    if (m == 0) {
-      if (lane == 0) {
-        mask[w] = 0;
-        counts[w] = make_int2(0, 0);
+    for (int u = 0; u < kWordsAtOnce; ++u) {
+      const int32_t t = t_run, s = w_run * 32 + lane;
+      if (++w_run == f.words) {
+        w_run = 0;
+        ++t_run;
       }
-      continue;
+      ts[u] = t;
+      ss[u] = s;
+      const bool in = rel0 + u < warp1 && s < S;
+      fs[u] = in ? fgrid[(int64_t)t * S + s] : -INFINITY;
+      bs[u] = in ? bgrid[(int64_t)t * S + s] : -INFINITY;
     }
-    any = true;
-    int32_t narcs = 0;
-    if (keep) {
-      const int32_t t = ts[u];
-      const int32_t idx01 = f.state_off + ss[u], a0 = a_row_splits2[idx01],
-                    a1 = a_row_splits2[idx01 + 1];
-      cand += a1 - a0;
-      if (t < f.tk) {
-        const float *fwd1 = fgrid + (int64_t)(t + 1) * S, *bwd1 = bgrid + (int64_t)(t + 1) * S;
-        const int64_t row = (int64_t)f.row0 + t;
-        for (int32_t a = a0; a < a1; ++a) {
-          float sc;
-          narcs += KeepArc(arcs[a], fs[u], fwd1, bwd1, scores, row, cols, cutoff, &sc);
+#pragma unroll
+    for (int u = 0; u < kWordsAtOnce; ++u) {
+      const int64_t rel = rel0 + u;
+      if (rel >= warp1) break;  // warp-uniform
+      const bool keep = __fadd_rn(fs[u], bs[u]) > cutoff;
+      const uint32_t m = __ballot_sync(0xffffffffu, keep);
+      const int64_t w = f.word_off + rel;
+      int32_t narcs = 0;
+      if (m != 0) {
+        const int32_t t = ts[u];
+        int32_t a0 = 0, deg = 0;
+        if (keep) {
+          const int32_t idx01 = f.state_off + ss[u];
+          a0 = a_row_splits2[idx01];
+          deg = a_row_splits2[idx01 + 1] - a0;
+          cand += deg;
+        }
+        if (t < f.tk) {
+          const float *fwd1 = fgrid + (int64_t)(t + 1) * S, *bwd1 = bgrid + (int64_t)(t + 1) * S;
+          const int64_t row = (int64_t)f.row0 + t;
+          ForArcsOfWord(lane, a0, deg, [&](bool valid, int32_t j, int32_t a, int32_t, int32_t) {
+            const float fj = __shfl_sync(0xffffffffu, fs[u], j);
+            float sc;
+            const bool kept =
+                valid && KeepArc(arcs[a], fj, fwd1, bwd1, scores, row, cols, cutoff, &sc);
+            narcs += __popc(__ballot_sync(0xffffffffu, kept));
+          });
         }
       }
-    }
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) narcs += __shfl_xor_sync(0xffffffffu, narcs, d);
-    if (lane == 0) {
-      mask[w] = m;
-      counts[w] = make_int2(__popc(m), narcs);
+      if (lane == 0) {
+        mask[w] = m;
+        counts[w] = make_int2(__popc(m), narcs);
+      }
     }
   }
-  }  // rounds
-  if (any) {  // warp-uniform
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) cand += __shfl_xor_sync(0xffffffffu, cand, d);
-    if (lane == 0 && cand) atomicAdd(&cand_smem, (unsigned long long)cand);
-  }
+  for (int d = 16; d > 0; d >>= 1) cand += __shfl_xor_sync(0xffffffffu, cand, d);
+  if (lane == 0 && cand) atomicAdd(&cand_smem, cand);
   __syncthreads();
   if (threadIdx.x == 0)
     block_cand[(size_t)(blockIdx.y + fsa_base) * gridDim.x + blockIdx.x] = cand_smem;
@@ -413,66 +434,64 @@ EmitWord(const FsaInfo &f, int32_t i, int32_t n, int64_t rel, float cutoff, int 
       }
     }
   }
+  if (m == 0) return;
   const bool keep = (m >> lane) & 1u;
   const float *fwd0 = fwd + f.grid_off + (int64_t)t * S, *bwd0 = bwd + f.grid_off + (int64_t)t * S;
   const float *fwd1 = fwd0 + S, *bwd1 = bwd0 + S;
   const int64_t row = (int64_t)f.row0 + t;
-  int32_t a0 = 0, a1 = 0, narcs = 0;
+  int32_t a0 = 0, deg = 0;
   float fs = 0;
-  if (keep) {
+  if (keep && t < f.tk) {
     const int32_t idx01 = f.state_off + s;
     a0 = a_row_splits2[idx01];
-    a1 = a_row_splits2[idx01 + 1];
+    deg = a_row_splits2[idx01 + 1] - a0;
     fs = fwd0[s];
-    if (t < f.tk) {
-      for (int32_t a = a0; a < a1; ++a) {
-        float sc;
-        narcs += KeepArc(arcs[a], fs, fwd1, bwd1, scores, row, cols, cutoff, &sc);
-      }
-    }
   }
-  // exclusive prefix of narcs across the warp
-  int32_t inc = narcs;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    int32_t o = __shfl_up_sync(0xffffffffu, inc, d);
-    if (lane >= d) inc += o;
-  }
-  if (!keep) return;
   const int32_t state_id = base.x + __popc(m & ((1u << lane) - 1u));
-  int32_t pos = base.y + inc - narcs;
-  out.row_splits2[state_id] = pos;
-  out.row_ids1[state_id] = i;
-  if (t >= f.tk || narcs == 0) return;
   const int64_t next_word0 = f.word_off + (int64_t)(t + 1) * f.words;
   Arc *out_arcs = reinterpret_cast<Arc *>(out.arcs);
-  for (int32_t a = a0; a < a1; ++a) {
-    Arc arc = arcs[a];
-    float sc;
-    if (!KeepArc(arc, fs, fwd1, bwd1, scores, row, cols, cutoff, &sc)) continue;
-    const int64_t wd = next_word0 + (arc.dest >> 5);
-    const int32_t dest_id = bases[wd].x + __popc(mask[wd] & ((1u << (arc.dest & 31)) - 1u));
-    Arc o;
-    o.src = state_id - fsa_first_state;
-    o.dest = dest_id - fsa_first_state;
-    o.label = arc.label;
-    o.score = sc;
-    out_arcs[pos] = o;
-    out.row_ids2[pos] = state_id;
-    if (out.arc_map_a) out.arc_map_a[pos] = a + f.arc_out_off;
-    if (out.arc_map_b) out.arc_map_b[pos] = (int32_t)(row * cols + (arc.label + 1));
-    ++pos;
+  int32_t run = base.y;      // output position of the batch's first surviving arc
+  int32_t first_pos = -1;    // of this lane's state
+  ForArcsOfWord(lane, a0, deg, [&](bool valid, int32_t j, int32_t a, int32_t start,
+                                   int32_t first) {
+    const float fj = __shfl_sync(0xffffffffu, fs, j);
+    Arc arc;
+    float sc = 0.0f;
+    bool kept = false;
+    if (valid) {
+      arc = arcs[a];
+      kept = KeepArc(arc, fj, fwd1, bwd1, scores, row, cols, cutoff, &sc);
+    }
+    const uint32_t ballot = __ballot_sync(0xffffffffu, kept);
+    const int32_t at = start - first;
+    if (at >= 0 && at < 32) first_pos = run + __popc(ballot & ((1u << at) - 1u));
+    const int32_t src_id = __shfl_sync(0xffffffffu, state_id, j);
+    if (kept) {
+      const int32_t pos = run + __popc(ballot & ((1u << lane) - 1u));
+      const int64_t wd = next_word0 + (arc.dest >> 5);
+      const int32_t dest_id = bases[wd].x + __popc(mask[wd] & ((1u << (arc.dest & 31)) - 1u));
+      Arc o;
+      o.src = src_id - fsa_first_state;
+      o.dest = dest_id - fsa_first_state;
+      o.label = arc.label;
+      o.score = sc;
+      out_arcs[pos] = o;
+      out.row_ids2[pos] = src_id;
+      if (out.arc_map_a) out.arc_map_a[pos] = a + f.arc_out_off;
+      if (out.arc_map_b) out.arc_map_b[pos] = (int32_t)(row * cols + (arc.label + 1));
+    }
+    run += __popc(ballot);
+  });
+  if (keep) {
+    // (a state whose range starts at the end of the flat range has no batch of its own)
+    out.row_splits2[state_id] = first_pos >= 0 ? first_pos : run;
+    out.row_ids1[state_id] = i;
   }
 }
 
-
-constexpr int kEmitWordsPerWarp = 16;
-constexpr int kEmitWordsPerCta = kEmitWordsPerWarp * 8;
-
-// Each warp walks kEmitWordsPerWarp consecutive words (few, fat CTAs: most words
-// hold nothing and are skipped after one load).
+// Each warp walks words_per_warp consecutive words.
 __global__ void __launch_bounds__(256)
-EmitLattice(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_words,
+EmitLattice(const FsaInfo *__restrict__ infos, int32_t n, int32_t words_per_warp,
             const Arc *__restrict__ arcs, const int32_t *__restrict__ a_row_splits2,
             const float *__restrict__ scores, int32_t cols, const float *__restrict__ fwd,
             const float *__restrict__ bwd, const float *__restrict__ cutoffs,
@@ -483,9 +502,9 @@ EmitLattice(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_words,
   const FsaInfo f = infos[i];
   const float cutoff = cutoffs[i];
   const int64_t pair_words = (int64_t)(f.tk + 1) * f.words;
-  const int64_t rel0 =
-      ((int64_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5)) * kEmitWordsPerWarp;
-  for (int u = 0; u < kEmitWordsPerWarp; ++u) {
+  const int64_t rel0 = ((int64_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5)) *
+                       (int64_t)words_per_warp;
+  for (int u = 0; u < words_per_warp; ++u) {
     const int64_t rel = rel0 + u;
     if (rel >= pair_words) return;
     EmitWord(f, i, n, rel, cutoff, lane, arcs, a_row_splits2, scores, cols, fwd, bwd, mask, bases,
@@ -708,7 +727,7 @@ int32_t PruneLoop(const Layout &L, const k2b200_intersect_args *args, char *ws,
         for (int32_t first = 0; first < args->num_fsas; first += 65535) {
           dim3 grid(L.tiles_per_pair, std::min(args->num_fsas - first, 65535));
           { CountKept<<<grid, kCountThreads, 0, stream>>>(
-              d_infos, args->num_fsas, L.total_words, arcs, args->a_row_splits2, args->scores,
+              d_infos, L.words_per_warp, arcs, args->a_row_splits2, args->scores,
               args->cols, fwd, bwd, cutoffs, mask, counts, block_cand, first); NoteLaunch(); }
         }
       K2B_FORWARD(ExclusiveSum2(counts, counts, L.total_words, scan_tmp, stream));
@@ -804,9 +823,9 @@ int32_t k2b200_intersect_dense_emit(const k2b200_intersect_args *args, void *wor
       reinterpret_cast<const int2 *>(ws + L.off_counts), *out); NoteLaunch(); }
   if (L.total_words > 0)
     for (int32_t first = 0; first < args->num_fsas; first += 65535) {
-      dim3 grid(L.emit_tiles_per_pair, std::min(args->num_fsas - first, 65535));
-      { EmitLattice<<<grid, 256, 0, stream>>>(
-          d_infos, args->num_fsas, L.total_words, reinterpret_cast<const Arc *>(args->a_arcs),
+      dim3 grid(L.tiles_per_pair, std::min(args->num_fsas - first, 65535));
+      { EmitLattice<<<grid, kCountThreads, 0, stream>>>(
+          d_infos, args->num_fsas, L.words_per_warp, reinterpret_cast<const Arc *>(args->a_arcs),
           args->a_row_splits2, args->scores, args->cols,
           reinterpret_cast<const float *>(ws + L.off_fwd),
           reinterpret_cast<const float *>(ws + L.off_bwd),

@@ -36,7 +36,7 @@ struct Layout {
   // graphs with states of more than four arcs, small enough for one CTA: lanes are
   // assigned to states by a plan (viterbi_persistent.cu)
   bool lane_plan = false;
-  int32_t count_blocks, tiles_per_pair, emit_tiles_per_pair;
+  int32_t count_blocks, tiles_per_pair, words_per_warp;
 };
 
 // intersect.cu
