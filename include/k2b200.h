@@ -589,6 +589,10 @@ int32_t k2b200_fsa_incoming_layers(const k2b200_fsa_view *fsas, int32_t *in_spli
  * layer-to-layer dependency chain (the arcs' exp() and the states' log() run in separate
  * fully parallel kernels).  Without scratch a slower kernel gives the same values. */
 size_t k2b200_fsa_scores_scratch_bytes(const k2b200_fsa_view *fsas);
+/* The same for a call that asks for one or two directions; *needs_incoming = 0 when such a call
+ * with scratch does without the view's incoming-arc index (it may then be NULL). */
+size_t k2b200_fsa_scores_dir_scratch_bytes(const k2b200_fsa_view *fsas, int32_t directions,
+                                           int32_t *needs_incoming);
 int32_t k2b200_fsa_scores(const k2b200_fsa_view *fsas, int32_t log_semiring,
                           int32_t use_double, void *forward, void *backward,
                           int32_t *entering_arcs, void *scratch, size_t scratch_bytes,

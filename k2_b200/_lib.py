@@ -196,6 +196,8 @@ _sig("k2b200_fsa_levels", c_i32,
 _sig("k2b200_fsa_incoming_layers", c_i32,
      [ctypes.POINTER(FsaView), c_vp, c_vp, c_vp, c_vp, ctypes.POINTER(c_i32), c_vp])
 _sig("k2b200_fsa_scores_scratch_bytes", c_sz, [ctypes.POINTER(FsaView)])
+_sig("k2b200_fsa_scores_dir_scratch_bytes", c_sz,
+     [ctypes.POINTER(FsaView), c_i32, ctypes.POINTER(c_i32)])
 _sig("k2b200_fsa_scores", c_i32,
      [ctypes.POINTER(FsaView), c_i32, c_i32, c_vp, c_vp, c_vp, c_vp, c_sz, c_vp])
 _sig("k2b200_fsa_tot_scores", c_i32, [c_vp, c_i32, c_i32, c_vp, c_vp, c_vp])
@@ -244,7 +246,7 @@ EXPORTED = [
     "k2b200_exclusive_sum_static_max_len", "k2b200_exclusive_sum_static", "k2b200_fsa_incoming_tmp_bytes",
     "k2b200_fsa_incoming", "k2b200_fsa_incoming_layers", "k2b200_intersect_dense_workspace_bytes",
     "k2b200_intersect_dense_prune", "k2b200_intersect_dense_emit", "k2b200_fsa_scores",
-    "k2b200_fsa_scores_scratch_bytes",
+    "k2b200_fsa_scores_scratch_bytes", "k2b200_fsa_scores_dir_scratch_bytes",
     "k2b200_fsa_tot_scores", "k2b200_fsa_arc_post", "k2b200_tot_scores_log_backward",
     "k2b200_tot_scores_tropical_backward", "k2b200_index_add", "k2b200_index_select_i32",
     "k2b200_shortest_path_tmp_bytes", "k2b200_shortest_path", "k2b200_best_paths_tmp_bytes",

@@ -4,26 +4,21 @@
 //
 // The recursion is a chain of T dependent layers, so what bounds it is the latency of one
 // layer, and the rest of the work is moved off that chain:
-//   * LayerIncoming builds the incoming-arc index layer by layer.  The arcs that enter a
-//     layer are exactly those that leave the layer before, one contiguous range, so the
-//     index is a stable counting sort of that range by destination: no global scan, no
-//     atomics on global memory and one launch (lfmmi lattice of 6.7 M arcs: 283 us by
-//     counting, scanning, filling and sorting the whole FsaVec).
-//   * PackLayerArcs writes one 16-byte record per arc: exp(score) as a double for the log
-//     semiring (the score itself for the tropical one), the state at the other end and the
-//     arc's index.
-//   * LayerChain, one CTA per (FSA, direction), then needs one multiply-add per arc: values
+//   * SliceLayers lays the arcs of every layer out for the chain: one 16-byte record per arc
+//     with exp(score) as a double for the log semiring (the score itself for the tropical
+//     one), dealt out evenly to lanes and stored so that a warp reads a row of 32 records
+//     without conflicts.  The arcs that enter a layer are exactly those that leave the layer
+//     before, so no incoming-arc index of the FsaVec is needed.
+//   * SliceChain, one CTA per (FSA, direction), then needs one multiply-add per arc: values
 //     of a layer are plain doubles that share a power of two, which follows the largest of
 //     them every kRescale layers.  What that cannot hold (arc scores beyond +-kMaxScore,
-//     values more than 2^280 away from it) raises the status word, and the caller's general
-//     kernel, launched behind and otherwise returning at once, redoes the call.
+//     values more than 2^280 away from it) raises the status word, and ExactChain, launched
+//     behind and otherwise returning at once, redoes the call.
 //   * FinishLayerScores takes the logarithms, all states in parallel.
-// A state's arcs are taken by one lane, or by eight when states have many; the few states of
-// many arcs that lattices of the first kind have (hub states of decoding graphs) by a warp.
-// Layers come through a ring in shared memory: a slot holds as many consecutive layers as
-// fit (their records and splits are contiguous), fetched by two bulk copies that one lane of
-// an extra warp issues ahead of the chain.  Lattices with layers too wide for a slot
-// (decoding: thousands of states per frame) go to LayerChainWide, a cluster of CTAs per chain.
+// Layers come through a ring in shared memory, many small ones per slot, each by a bulk copy
+// that an extra warp issues ahead of the chain.  Lattices with layers too wide for a slot
+// (decoding: thousands of states per frame) go to LayerChainWide, a cluster of CTAs per chain,
+// which reads records in incoming / leaving order from L2 (LayerIncoming, PackLayerArcs).
 #include <algorithm>
 
 #include <cooperative_groups.h>
@@ -31,6 +26,7 @@
 #include "../../include/k2b200.h"
 #include "common.cuh"
 #include "cp_async.cuh"
+#include "prob_math.cuh"
 #include "scores_internal.cuh"
 
 namespace k2b {
@@ -42,7 +38,7 @@ constexpr float kMaxScore = 300.0f;   // |arc score|: exp() within 2^+-433
 constexpr int kRangeExp = 280;        // values that are not zero stay within 2^+-280, so that no
                                       // product of one with a factor and a scale underflows
 constexpr int kMaxSlots = 8;
-constexpr int kChunkLayers = 32;      // layers of one slot at most
+constexpr int kSliceMaxStates = 16384;  // states of a sliced layer
 
 struct __align__(16) LayerArc {
   double w;       // exp(score) (log semiring) or the score (tropical)
@@ -206,7 +202,10 @@ __global__ void PackLayerArcs(k2b200_fsa_view v, LayerArc *__restrict__ fwd,
 }
 
 struct ChainPlan {
-  int32_t maxw, nl_cap, cap_arcs, splits_ints, slot_bytes, slots, warps, group_log2;
+  int32_t maxw, nl_cap, warps;
+  // sliced layers
+  int32_t rows, slots, slot_bytes;
+  // wide layers
   int32_t wide, team;
   size_t bytes;
   bool ok;
@@ -218,29 +217,33 @@ static ChainPlan PlanChain(const k2b200_fsa_view *v, int32_t ndir) {
     return p;
   p.maxw = (v->max_layer_states + 3) & ~3;
   p.nl_cap = v->max_layers;
-  const size_t bounds = 2 * sizeof(int32_t) * (size_t)((p.nl_cap + 1 + 3) & ~3);
-  const size_t fixed = bounds + 2 * sizeof(double) * (size_t)p.maxw;
   const int64_t layers = (int64_t)v->num_fsas * v->max_layers;
   const int32_t mean_w = (int32_t)((v->num_states + layers - 1) / layers),
                 mean_a = (int32_t)((v->num_arcs + layers - 1) / layers);
-  // Eight lanes per state when states have many arcs, else one.  A warp costs a layer some
-  // hundred instructions whatever it does, and one that runs alone issues one in about five
-  // cycles: as many warps as a mean layer fills, at most 16.
-  p.group_log2 = mean_a >= 6 * (int64_t)mean_w ? 3 : 0;
-  p.warps = std::max(1, std::min(16, CeilDiv((int64_t)mean_w << p.group_log2, 32)));
-  p.cap_arcs = std::max(v->max_layer_arcs, 512);
-  p.splits_ints = (std::max(p.maxw, 256) + kChunkLayers + 8 + 3) & ~3;
-  p.slot_bytes = p.cap_arcs * (int32_t)sizeof(LayerArc) + p.splits_ints * (int32_t)sizeof(int32_t);
+  // arcs per lane (rows of a block): what most states of a lattice have, or a share of it that
+  // leaves the states of many arcs enough lanes
+  const double mean_deg = (double)v->num_arcs / std::max(v->num_states, 1);
+  p.rows = mean_deg < 1.6 ? 2 : mean_deg < 3.0 ? 3 : mean_deg < 6.0 ? 4 : 8;
+  // Warps: a block of 32 lanes each, for a layer between the mean and the largest (a warp that
+  // runs alone issues an instruction in about five cycles, so more warps than blocks only
+  // add to the barrier).
+  const int32_t blocks = CeilDiv(mean_w + mean_a / p.rows, 32),
+                most = CeilDiv(p.maxw + v->max_layer_arcs / p.rows, 32);
+  p.warps = std::max(1, std::min(16, std::min((blocks + most + 1) / 2, 2 * blocks)));
+  const size_t vals = 2 * sizeof(double) * (size_t)p.maxw;
   // with more CTAs than SMs, two of them should share one
   const size_t budget =
       (int64_t)ndir * v->num_fsas > 148 ? kLayerSmemBudget / 2 : kLayerSmemBudget;
+  // a slot takes the largest layer with a quarter of padding, or several small ones
+  const size_t largest = (size_t)v->max_layer_arcs * 22 + (size_t)p.maxw * 16 + 4096;
   for (size_t limit : {budget, kLayerSmemBudget}) {
-    if (fixed + 3 * (size_t)p.slot_bytes <= limit) {
-      p.slots = (int32_t)std::min<size_t>(4, (limit - fixed) / p.slot_bytes);
-      p.bytes = fixed + (size_t)p.slots * p.slot_bytes;
-      p.ok = true;
-      return p;
-    }
+    if (vals + 2 * largest > limit || p.maxw > kSliceMaxStates) continue;
+    p.slots = (int32_t)std::max<size_t>(2, std::min<size_t>(4, (limit - vals) / (24 * 1024)));
+    while (p.slots > 2 && (limit - vals) / p.slots < largest) --p.slots;
+    p.slot_bytes = (int32_t)(std::min<size_t>((limit - vals) / p.slots, 48 * 1024 + largest) & ~127);
+    p.bytes = vals + (size_t)p.slots * p.slot_bytes;
+    p.ok = true;
+    return p;
   }
   // Layers too wide for that are shared by a cluster of CTAs.
   p.wide = 1;
@@ -249,9 +252,251 @@ static ChainPlan PlanChain(const k2b200_fsa_view *v, int32_t ndir) {
   while (p.team < 8 && (int64_t)ndir * v->num_fsas * p.team * 2 <= 148 &&
          p.team * 32 * p.warps < v->max_layer_states)
     p.team *= 2;
-  p.bytes = bounds;
+  p.bytes = sizeof(int32_t) * (size_t)((p.nl_cap + 1 + 3) & ~3);
   p.ok = p.bytes <= kLayerSmemBudget;
   return p;
+}
+
+// ---------------------------------------------------------------------------
+// Sliced layers: what the chain reads.  A layer's states are dealt out to lanes, a state of d
+// arcs to n = 1, 2, 4 ... 32 of them so that a lane has at most K = ChainPlan::rows arcs, in
+// order of falling n; 32 consecutive lanes are a block.  The r-th arc of a state goes to its
+// lane r mod n, row r / n.  The K rows of a block hold a LayerArc per lane (weight 0 / NaN
+// where there is no arc), so that the chain reads them without bank conflicts, without a
+// search and without a test per arc.  A state of more than 32 K arcs has a block of its own
+// with as many rows as it takes ("tall"), behind all others.
+//   layer region: a word per lane of all blocks: state (index in its layer) | log2 n << 16 |
+//     first lane of the state << 19; a word per tall block: first row | rows << 20; the rows
+// Regions are handed out by an atomic counter; where a layer lies does not change results.
+// ---------------------------------------------------------------------------
+constexpr uint32_t kNoState = 0xffffu, kLaneHead = 1u << 19;
+struct SliceDesc {
+  int32_t at;      // of the region, in units of 16 bytes
+  int32_t size;    // likewise
+  int32_t blocks;  // of K rows; -1: the pool was full, the arcs are read where they are
+  int32_t tall;
+};
+// Of a region in units of 16 bytes: where the rows start.
+__device__ __forceinline__ int32_t SliceRowsAt(int32_t blocks, int32_t tall) {
+  return (blocks + tall) * 8 + (tall + 3) / 4;
+}
+
+// Units of 16 bytes the pool needs: records for uneven lanes, two part-filled blocks per
+// layer, lane words.  (A layer that finds the pool full is read the slow way.)
+static int64_t SlicePoolUnits(const k2b200_fsa_view *v, const ChainPlan &p) {
+  const int64_t layers = (int64_t)v->num_fsas * v->max_layers, k = p.rows;
+  return v->num_arcs + v->num_arcs / 2 + (int64_t)v->num_states * (p.rows < 8 ? k - 1 : k / 2) +
+         layers * (40 * k + 16) + 1024;
+}
+
+// Layer `lv` of direction blockIdx.y + dir_base per team of kWarps warps (kWarps == 1: four
+// layers per CTA).  A region of at most buf_units is put together in shared memory (scattered
+// 16-byte stores to global memory took twice as long).
+template <bool kLog, int kWarps>
+__global__ void __launch_bounds__(128)
+SliceLayers(k2b200_fsa_view v, int32_t dir_base, int32_t K, int32_t maxw, int32_t maxa,
+            int32_t buf_units, int32_t nl_total, int64_t pool_units,
+            unsigned long long *__restrict__ pool_used, uint4 *__restrict__ pool,
+            SliceDesc *__restrict__ descs, int32_t *__restrict__ status) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr int nt = 32 * kWarps;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int tid = kWarps == 1 ? lane : threadIdx.x;
+  const int dir = blockIdx.y + dir_base;
+  const int32_t lv = kWarps == 1 ? blockIdx.x * 4 + warp : blockIdx.x;
+  if (lv >= v.level_offsets[v.num_fsas]) return;
+  auto sync = [&]() { if (kWarps == 1) __syncwarp(); else __syncthreads(); };
+  SliceDesc *desc = descs + (int64_t)dir * nl_total + lv;
+  const int32_t b = v.level_splits[lv], w = v.level_splits[lv + 1] - b;
+  if (w <= 0 || w > maxw) {
+    if (tid == 0) {
+      SliceDesc d = {0, 0, w <= 0 ? 0 : -1, 0};
+      *desc = d;
+      if (w > maxw) atomicOr(status, 1);  // the caller's bounds do not hold
+    }
+    return;
+  }
+  const Arc *arcs = reinterpret_cast<const Arc *>(v.arcs);
+  const int32_t fsa = v.row_ids1[b], s_begin = v.row_splits1[fsa];
+  // the arcs: those that leave the layer before (forward) or this layer (backward), and the
+  // first state of the layer at their other end
+  int32_t a0, a1, ob;
+  if (dir == 0) {
+    ob = lv > v.level_offsets[fsa] ? v.level_splits[lv - 1] : b;
+    a0 = v.row_splits2[ob];
+    a1 = ob < b ? v.row_splits2[b] : a0;
+  } else {
+    ob = b + w;
+    a0 = v.row_splits2[b];
+    a1 = v.row_splits2[b + w];
+  }
+  if (a1 - a0 > maxa) {
+    if (tid == 0) {
+      SliceDesc d = {0, 0, -1, 0};
+      *desc = d;
+      atomicOr(status, 1);
+    }
+    return;
+  }
+  // per team: the region, counters of every warp per state, lanes of every state
+  unsigned char *team = smem_raw + (kWarps == 1 ? warp : 0) *
+                                       ((size_t)buf_units * 16 + 4 * (2 * (size_t)maxw + 32));
+  uint4 *buf = reinterpret_cast<uint4 *>(team);
+  int32_t *cnt = reinterpret_cast<int32_t *>(buf + buf_units);  // [kWarps][maxw]
+  int32_t *place = cnt + kWarps * maxw;                         // [maxw] first lane | log2 n << 24
+  int32_t *head = place + maxw;                                 // [32] buckets and the like
+  for (int32_t k = tid; k < w; k += nt)
+#pragma unroll
+    for (int u = 0; u < kWarps; ++u) cnt[u * maxw + k] = 0;
+  if (tid < 32) head[tid] = 0;
+  sync();
+  const int32_t per = ((a1 - a0 + nt - 1) / nt) * 32;
+  const int32_t c0 = kWarps == 1 ? a0 : min(a0 + warp * per, a1);
+  const int32_t c1 = kWarps == 1 ? a1 : min(c0 + per, a1);
+  int32_t *mine = cnt + (kWarps == 1 ? 0 : warp) * maxw;
+  if (dir == 0) {
+#pragma unroll 4
+    for (int32_t a = c0 + lane; a < c1; a += 32) {
+      const int32_t d = s_begin + arcs[a].dest - b;
+      if ((uint32_t)d < (uint32_t)w) atomicAdd(&mine[d], 1);
+    }
+    sync();
+  }
+  // ---- lanes of every state: buckets 0 .. 5 are n = 32 .. 1, 6 the tall states ----------
+  auto degree = [&](int32_t j) {
+    if (dir != 0) return v.row_splits2[b + j + 1] - v.row_splits2[b + j];
+    int32_t d = 0;
+#pragma unroll
+    for (int u = 0; u < kWarps; ++u) d += cnt[u * maxw + j];
+    return d;
+  };
+  auto bucket_of = [&](int32_t d) {
+    if (d > 32 * K) return 6;
+    int n = 0;
+    while (K << n < d) ++n;
+    return 5 - n;
+  };
+  for (int32_t j = tid; j < w; j += nt) {
+    const int32_t d = degree(j), bk = bucket_of(d);
+    const int32_t rows = bk == 6 ? (d + 31) >> 5 : 0;
+    atomicAdd(&head[bk], bk == 6 ? 32 : 32 >> bk);
+    if (bk == 6) atomicAdd(&head[16], rows);
+    place[j] = d;
+  }
+  sync();
+  int32_t lanes = 0;
+  for (int u = 0; u < 6; ++u) lanes += head[u];
+  const int32_t blocks = (lanes + 31) >> 5, tall = head[6] >> 5;
+  const int32_t rows_at = SliceRowsAt(blocks, tall);
+  const int32_t units = rows_at + (blocks * K + head[16]) * 32;
+  sync();
+  if (tid == 0) {
+    int32_t run = 0;
+    for (int u = 0; u < 6; ++u) {
+      head[8 + u] = run;  // first lane of the bucket
+      run += head[u];
+    }
+    head[14] = blocks * 32;  // ... of the tall states
+    head[17] = blocks * K;   // ... and their first row
+    const unsigned long long at = atomicAdd(pool_used, (unsigned long long)units);
+    SliceDesc d = {(int32_t)at, units, blocks, tall};
+    // (a tall block's word has 12 bits for its rows, 20 for the first of them)
+    if (at + units > (unsigned long long)pool_units || head[16] >= 4096 ||
+        blocks * K + head[16] >= (1 << 20)) {
+      d.at = d.size = d.tall = 0;
+      d.blocks = -1;
+    }
+    *desc = d;
+    head[20] = d.blocks;
+    head[21] = d.at;
+  }
+  sync();
+  if (head[20] < 0) return;
+  uint4 *const final_region = pool + head[21];
+  const bool staged = units <= buf_units;
+  uint4 *region = staged ? buf : final_region;
+  uint32_t *words = reinterpret_cast<uint32_t *>(region);
+  LayerArc *recs = reinterpret_cast<LayerArc *>(region + rows_at);
+  for (int32_t k = lanes + tid; k < blocks * 32; k += nt) words[k] = kNoState;
+  {
+    LayerArc none;
+    none.w = kLog ? 0.0 : nan("");  // (never the larger one)
+    none.other = 0;
+    none.arc = -1;
+    for (int32_t k = tid; k < units - rows_at; k += nt) recs[k] = none;
+  }
+  // every state's lanes, every warp's first arc of it
+  for (int32_t j = tid; j < w; j += nt) {
+    const int32_t d = place[j], bk = bucket_of(d);
+    const int32_t nl = bk == 6 ? 5 : 5 - bk;
+    const int32_t at = atomicAdd(&head[8 + bk], 1 << nl);
+    // the row of its first arc times 32, plus its first lane of the block
+    int32_t first = (at >> 5) * K * 32 + (at & 31);
+    if (bk == 6) {
+      const int32_t rows = (d + 31) >> 5, row = atomicAdd(&head[17], rows);
+      words[(blocks + tall) * 32 + ((at >> 5) - blocks)] = (uint32_t)row | (uint32_t)rows << 20;
+      first = row * 32;
+    }
+    place[j] = first | nl << 27;
+    for (int32_t u = 0; u < 1 << nl; ++u)
+      words[at + u] = (uint32_t)j | (uint32_t)nl << 16 | (u == 0 ? kLaneHead : 0u);
+    if (dir == 0) {
+      int32_t r = 0;
+#pragma unroll
+      for (int u = 0; u < kWarps; ++u) {
+        const int32_t n = cnt[u * maxw + j];
+        cnt[u * maxw + j] = r;
+        r += n;
+      }
+    }
+  }
+  sync();  // (also: the records' padding is written before any arc)
+  auto put = [&](const Arc &arc, int32_t a, int32_t j, int32_t rank, int32_t other) {
+    const int32_t at = place[j] & 0x7ffffff, nl = (int32_t)((uint32_t)place[j] >> 27);
+    LayerArc r;
+    r.w = kLog ? exp((double)arc.score) : (double)arc.score;
+    r.other = other;
+    r.arc = a;
+    recs[at + (rank & ((1 << nl) - 1)) + (rank >> nl) * 32] = r;
+    if (kLog && arc.score != -INFINITY && !(fabsf(arc.score) <= kMaxScore)) atomicOr(status, 4);
+  };
+  if (dir != 0) {
+#pragma unroll 2
+    for (int32_t a = c0 + lane; a < c1; a += 32) {
+      const Arc arc = arcs[a];
+      const int32_t j = s_begin + arc.src - b;
+      put(arc, a, j, a - v.row_splits2[b + j], s_begin + arc.dest - ob);
+    }
+  } else {
+    // two batches of 32 arcs at a time, so that their loads are in flight together
+    for (int32_t a = c0; a < c1; a += 64) {
+      Arc arc[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+        if (a + 32 * u + lane < c1) arc[u] = arcs[a + 32 * u + lane];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        if (a + 32 * u >= c1) break;  // uniform
+        int32_t j = -1 - lane;  // lanes without an arc match nobody
+        if (a + 32 * u + lane < c1) {
+          const int32_t x = s_begin + arc[u].dest - b;
+          if ((uint32_t)x < (uint32_t)w) j = x;
+        }
+        const unsigned same = __match_any_sync(kAll, j);
+        int32_t rank = 0;
+        if (j >= 0) rank = mine[j] + __popc(same & ((1u << lane) - 1u));
+        __syncwarp();
+        if (j >= 0 && lane == 31 - __clz(same)) mine[j] = rank + 1;
+        __syncwarp();
+        if (j >= 0) put(arc[u], a + 32 * u + lane, j, rank, s_begin + arc[u].src - ob);
+      }
+    }
+  }
+  if (staged) {
+    sync();
+    for (int32_t k = tid; k < units; k += nt) final_region[k] = buf[k];
+  }
 }
 
 // The sum over a state's arcs (log) or its best entering arc (tropical).
@@ -371,15 +616,51 @@ struct ChainScale {
   }
 };
 
-// grid = (directions, fsas).  val_fwd / val_bwd: values per state (log: doubles relative to
-// 2^scale[(dir * num_fsas + i) * nl_cap + layer]).  kGroup lanes per state (1 or 8).
-template <typename Val, bool kLog, int kGroup>
+// The sum of state s (layer l of FSA i) when the layer was not sliced: all arcs of the layer
+// are looked through.
+template <typename Val, bool kLog>
+__device__ __noinline__ StateSum<Val, kLog> SumUnsliced(const k2b200_fsa_view &v, int32_t i,
+                                                        int32_t dir, int32_t l, int32_t s,
+                                                        const Val *prev) {
+  const int32_t lv = v.level_offsets[i] + l, s_begin = v.row_splits1[i];
+  const int32_t b = v.level_splits[lv], e = v.level_splits[lv + 1];
+  const Arc *arcs = reinterpret_cast<const Arc *>(v.arcs);
+  const int32_t ob = dir != 0 ? e : l > 0 ? v.level_splits[lv - 1] : b;
+  StateSum<Val, kLog> q;
+  q.Clear();
+  const int32_t a0 = v.row_splits2[dir == 0 ? ob : s],
+                a1 = dir == 0 ? (ob < b ? v.row_splits2[b] : a0) : v.row_splits2[s + 1];
+  for (int32_t a = a0; a < a1; ++a) {
+    const Arc arc = arcs[a];
+    if (dir == 0 && s_begin + arc.dest != s) continue;
+    LayerArc r;
+    r.w = kLog ? exp((double)arc.score) : (double)arc.score;
+    r.other = s_begin + (dir == 0 ? arc.src : arc.dest) - ob;
+    r.arc = a;
+    q.Add(r, prev[r.other]);
+  }
+  return q;
+}
+
+// The walk over sliced layers.  grid = (directions, fsas).  val_fwd / val_bwd: values per
+// state (log: doubles relative to 2^scale[(dir * num_fsas + i) * nl_cap + layer]).  The last
+// warp feeds the ring: its lanes look at the next 32 layers, those that fit a slot go there
+// with a bulk copy each.  A warp sums the blocks b = warp, warp + warps, ... of a layer.
+struct __align__(16) SliceEntry {  // of a layer in a slot
+  int32_t at;  // of the region in shared memory, in units of 16 bytes; -1: read from L2
+  int32_t blocks, tall, first_state;
+};
+
+template <typename Val, bool kLog, int K>
 __global__ void __launch_bounds__(544, 1)
-LayerChain(k2b200_fsa_view v, const LayerArc *__restrict__ fwd_arcs,
-           const LayerArc *__restrict__ bwd_arcs, Val *__restrict__ val_fwd,
-           Val *__restrict__ val_bwd, int32_t *__restrict__ entering, int32_t *__restrict__ scale,
-           int32_t dir_base, int32_t fsa_base, ChainPlan p, int32_t *__restrict__ status) {
+SliceChain(k2b200_fsa_view v, const uint4 *__restrict__ pool, const SliceDesc *__restrict__ descs,
+           Val *__restrict__ val_fwd, Val *__restrict__ val_bwd, int32_t *__restrict__ entering,
+           int32_t *__restrict__ scale, int32_t dir_base, int32_t fsa_base, int32_t nl_total,
+           ChainPlan p, int32_t *__restrict__ status) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ __align__(8) uint64_t full[kMaxSlots], empty[kMaxSlots];
+  __shared__ SliceEntry entries[kMaxSlots][32];
+  __shared__ int32_t slot_layers[kMaxSlots], hi_shared[2];
   constexpr unsigned kAll = 0xffffffffu;
   const int32_t i = fsa_base + blockIdx.y, dir = blockIdx.x + dir_base;
   const int32_t s_begin = v.row_splits1[i], s_end = v.row_splits1[i + 1];
@@ -388,21 +669,10 @@ LayerChain(k2b200_fsa_view v, const LayerArc *__restrict__ fwd_arcs,
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nw = p.warps;
   Val *out = dir == 0 ? val_fwd : val_bwd;
-  const int32_t lvl_ints = (p.nl_cap + 1 + 3) & ~3;
-  // everything in shared memory is addressed by index, so that it stays in that space
-  const LayerArc *recs = reinterpret_cast<const LayerArc *>(smem_raw);
-  int32_t *ints = reinterpret_cast<int32_t *>(smem_raw);
-  const size_t vals_at = (size_t)p.slots * p.slot_bytes;
-  Val *vals = reinterpret_cast<Val *>(smem_raw + vals_at);  // [2][maxw]
-  int32_t *lvl = reinterpret_cast<int32_t *>(smem_raw + vals_at + 16 * (size_t)p.maxw);
-  int32_t *alvl = lvl + lvl_ints;
-  const int32_t *gsplits = dir == 0 ? v.in_splits : v.row_splits2;
-  const LayerArc *garcs = dir == 0 ? fwd_arcs : bwd_arcs;
-  __shared__ __align__(8) uint64_t full[kMaxSlots], empty[kMaxSlots];
-  __shared__ int32_t chunk_layers[kMaxSlots];
-  __shared__ int32_t bad_shared, hi_shared[2];
+  const uint32_t *shared_words = reinterpret_cast<const uint32_t *>(smem_raw);
+  const LayerArc *shared_recs = reinterpret_cast<const LayerArc *>(smem_raw);
+  Val *vals = reinterpret_cast<Val *>(smem_raw + (size_t)p.slots * p.slot_bytes);  // [2][maxw]
   if (tid == 0) {
-    bad_shared = nl > p.nl_cap;
     hi_shared[0] = hi_shared[1] = 0;
     for (int32_t s = 0; s < p.slots; ++s) {
       MbarInit(&full[s], 1);
@@ -410,63 +680,52 @@ LayerChain(k2b200_fsa_view v, const LayerArc *__restrict__ fwd_arcs,
     }
     MbarInitFence();
   }
+  // (padding multiplies a value by zero: it has to be one)
+  for (int32_t k = tid; k < 2 * p.maxw; k += blockDim.x) vals[k] = (Val)0;
   __syncthreads();
-  if (!bad_shared)
-    for (int32_t k = tid; k <= nl; k += blockDim.x) {
-      const int32_t s = v.level_splits[lv0 + k];
-      lvl[k] = s;
-      alvl[k] = gsplits[s];
-    }
-  __syncthreads();
-  if (!bad_shared) {
-    bool bad = false;
-    for (int32_t k = tid; k < nl; k += blockDim.x)
-      bad |= lvl[k + 1] - lvl[k] > p.maxw || alvl[k + 1] - alvl[k] > p.cap_arcs;
-    if (bad) bad_shared = 1;
-  }
-  __syncthreads();
-  if (bad_shared) {  // the caller's bounds do not hold: the general kernel takes the call
+  if (nl > p.nl_cap) {  // the caller's bounds do not hold: the exact kernel takes the call
     if (tid == 0) atomicOr(status, 1);
     return;
   }
-  const int32_t slot_recs = p.slot_bytes >> 4, slot_ints = p.slot_bytes >> 2;
   if (warp == nw) {
-    // ---- the producer: one lane keeps the ring full ---------------------------------
-    if (lane != 0) return;
-    const int32_t splits_end = (v.num_states + 1) & ~3;  // last multiple of 4 in the splits
     int32_t slot = 0, issued = 0;
     unsigned parity = 1;  // a fresh barrier counts as "previous phase complete"
+    const int32_t cap = p.slot_bytes >> 4;
     for (int32_t done = 0; done < nl;) {
-      int32_t lo, hi;  // layers lo .. hi - 1
-      if (dir == 0) {
-        lo = done;
-        hi = lo + 1;
-        while (hi < nl && hi - lo < kChunkLayers && alvl[hi + 1] - alvl[lo] <= p.cap_arcs &&
-               lvl[hi + 1] - lvl[lo] + 8 <= p.splits_ints)
-          ++hi;
-      } else {
-        hi = nl - done;
-        lo = hi - 1;
-        while (lo > 0 && hi - lo < kChunkLayers && alvl[hi] - alvl[lo - 1] <= p.cap_arcs &&
-               lvl[hi] - lvl[lo - 1] + 8 <= p.splits_ints)
-          --lo;
+      const int32_t step = done + lane, l = dir == 0 ? step : nl - 1 - step;
+      SliceDesc d = {0, 0, 0, 0};
+      int32_t first = 0;
+      if (step < nl) {
+        d = descs[(int64_t)dir * nl_total + lv0 + l];
+        first = v.level_splits[lv0 + l];
       }
-      done += hi - lo;
-      if (!MbarWaitBounded(&empty[slot], parity)) {
-        atomicOr(status, 2);
+      const int32_t size = d.size <= cap && d.blocks >= 0 ? d.size : 0;
+      int32_t inc = size;
+#pragma unroll
+      for (int k = 1; k < 32; k <<= 1) {
+        const int32_t o = __shfl_up_sync(kAll, inc, k);
+        if (lane >= k) inc += o;
+      }
+      // (monotone, so the layers that fit are the first ones)
+      const int32_t m = __popc(__ballot_sync(kAll, step < nl && inc <= cap));
+      const int32_t total = __shfl_sync(kAll, inc, m - 1);
+      if (!__all_sync(kAll, MbarWaitBounded(&empty[slot], parity))) {
+        if (lane == 0) atomicOr(status, 2);
         break;
       }
-      const int32_t b = lvl[lo], e = lvl[hi];
-      int32_t *sp = ints + slot * slot_ints + p.cap_arcs * 4;
-      const int32_t c0 = b & ~3, c1 = max(c0, min((e + 1 + 3) & ~3, splits_end));
-      for (int32_t k = c1; k <= e; ++k) sp[k - c0] = gsplits[k];  // at most 3 trailing ints
-      chunk_layers[slot] = hi - lo;
-      const unsigned bytes_s = (unsigned)(c1 - c0) * 4u,
-                     bytes_a = (unsigned)(alvl[hi] - alvl[lo]) * (unsigned)sizeof(LayerArc);
-      MbarArriveExpectTx(&full[slot], bytes_s + bytes_a);
-      if (bytes_s) BulkCopyG2S(sp, gsplits + c0, bytes_s, &full[slot]);
-      if (bytes_a)
-        BulkCopyG2S(smem_raw + (size_t)slot * p.slot_bytes, garcs + alvl[lo], bytes_a, &full[slot]);
+      if (lane < m) {
+        SliceEntry e = {d.size > 0 && size == 0 ? -1 : slot * cap + inc - size, d.blocks, d.tall,
+                        first};
+        entries[slot][lane] = e;
+      }
+      if (lane == 0) slot_layers[slot] = m;
+      __syncwarp();
+      if (lane == 0) MbarArriveExpectTx(&full[slot], (unsigned)total * 16u);
+      __syncwarp();
+      if (lane < m && size > 0)
+        BulkCopyG2S(smem_raw + (size_t)(slot * cap + inc - size) * 16, pool + d.at,
+                    (unsigned)size * 16u, &full[slot]);
+      done += m;
       slot = slot + 1 == p.slots ? 0 : slot + 1;
       parity ^= (slot == 0);
       ++issued;
@@ -477,132 +736,257 @@ LayerChain(k2b200_fsa_view v, const LayerArc *__restrict__ fwd_arcs,
     return;
   }
 
-  // ---- the chain -----------------------------------------------------------------------
   const int32_t root = dir == 0 ? s_begin : s_end - 1, nc = 32 * nw;
-  const int32_t per_trip = nc / kGroup;  // states that one trip of all lanes takes
   int32_t *my_scale = kLog ? scale + ((int64_t)dir * v.num_fsas + i) * p.nl_cap : nullptr;
-  ChainScale<kLog> sc;
   auto layer_sync = [&]() {
     if (nw == 1) __syncwarp();
     else asm volatile("bar.sync 1, %0;" ::"r"(nc) : "memory");
   };
-  // the layer whose splits and first records are fetched, one layer ahead of the chain
-  struct Ahead {
-    int32_t b, e;         // its states
-    int32_t body, splits; // where the records / splits of its chunk start in shared memory
-    int32_t slot;         // >= 0: the chunk ends with this layer
-    int32_t s, k0, k1;    // this lane's state and its arcs
-    LayerArc r0;          // first of them
-  };
-  int32_t slot = p.slots - 1, left = 0, body = 0, splits = 0;
+  ChainScale<kLog> sc;
+  int32_t slot = p.slots - 1, k = 0, m = 0;
   unsigned parity = 1;
-  bool opened = false;  // a chunk was waited for since the last barrier
-  const int32_t mine_at = tid / kGroup;
-  auto fetch = [&](int32_t step, Ahead &f) {
-    const int32_t l = dir == 0 ? step : nl - 1 - step;
-    f.b = lvl[l];
-    f.e = lvl[l + 1];
-    if (left == 0) {
+  int32_t prev = p.maxw, cur = 0;
+  for (int32_t step = 0; step < nl; ++step) {
+    if (k == m) {  // the next slot
       slot = slot + 1 == p.slots ? 0 : slot + 1;
       parity ^= (slot == 0);
       if (!MbarWaitBounded(&full[slot], parity)) {
+        // nothing that the slot holds is looked at; the other warps still need the barriers
         atomicOr(status, 2);
-        *reinterpret_cast<volatile int32_t *>(&bad_shared) = 2;
+        for (; step < nl; ++step) layer_sync();
+        break;
       }
-      opened = true;
-      left = chunk_layers[slot];
-      const int32_t lo = dir == 0 ? l : l - left + 1;
-      body = slot * slot_recs - alvl[lo];
-      splits = slot * slot_ints + p.cap_arcs * 4 - (lvl[lo] & ~3);
+      k = 0;
+      m = slot_layers[slot];
     }
-    --left;
-    f.slot = left == 0 ? slot : -1;
-    f.body = body;
-    f.splits = splits;
-    f.s = f.b + mine_at;
-    f.k0 = f.k1 = 0;
-    if (f.s < f.e) {
-      f.k0 = ints[splits + f.s];
-      f.k1 = ints[splits + f.s + 1];
-      if (kGroup == 1 && f.k0 < f.k1) f.r0 = recs[body + f.k0];
-    }
-  };
-  int32_t prev_at = p.maxw, cur_at = 0, pb = 0;  // values of the layer before, of this layer
-  auto layer = [&](int32_t step, Ahead &now, Ahead &next) -> bool {
-    if (step + 1 < nl) fetch(step + 1, next);
+    const SliceEntry e = entries[slot][k++];
     sc.BeginLayer(step, hi_shared, tid == 0);
-    const int32_t prev = prev_at - pb, cur = cur_at - now.b;
-    int32_t s = now.s, k0 = now.k0, k1 = now.k1;
-    auto rec = [&](int32_t k) { return recs[now.body + k]; };
-    auto val = [&](const LayerArc &r) { return vals[prev + r.other]; };
-    for (int32_t s0 = now.b;;) {
-      StateSum<Val, kLog> q;
-      q.Clear();
-      if (kGroup == 1) {
-        const int32_t deg = k1 - k0;
-        const unsigned heavy = __ballot_sync(kAll, deg > kLight);
-        if (deg > 0 && deg <= kLight) {
-          if (s0 == now.b) {
-            q.Add(now.r0, val(now.r0));
-            ++k0;
-          }
-          for (; k0 < k1; ++k0) {
-            const LayerArc r = rec(k0);
-            q.Add(r, val(r));
-          }
-        }
-        if (heavy) q.Heavy(heavy, lane, k0, k1, rec, val);
+    auto finish = [&](int32_t j, StateSum<Val, kLog> &q) {
+      const int32_t s = e.first_state + j;
+      if (kLog) {
+        q.acc = q.acc * (Val)sc.mul;
+        if (q.acc == (Val)0 && s == root) q.acc = (Val)1;
+        sc.Note((double)q.acc);
       } else {
-        q.Walk(k0 + (lane & (kGroup - 1)), k1, kGroup, rec, val);
-        q.Across(kGroup);
+        if (s == root && q.acc == (Val)-INFINITY) q.acc = (Val)0;
+        if (entering != nullptr && dir == 0) entering[s] = q.best;
       }
-      if (s < now.e && (kGroup == 1 || (lane & (kGroup - 1)) == 0)) {
-        if (kLog) {
-          q.acc = q.acc * (Val)sc.mul;
-          if (q.acc == (Val)0 && s == root) q.acc = (Val)1;
-          sc.Note((double)q.acc);
-        } else {
-          if (q.acc == (Val)-INFINITY && s == root) q.acc = (Val)0;
-          if (entering != nullptr && dir == 0) entering[s] = q.best;
+      vals[cur + j] = q.acc;
+      out[s] = q.acc;
+    };
+    // the lanes of a state bring their sums together
+    auto across = [&](uint32_t word, StateSum<Val, kLog> &q) {
+      const int32_t nlog = (int32_t)(word >> 16) & 7;
+      const int32_t most = __reduce_max_sync(kAll, nlog);
+      for (int32_t d = 0; d < most; ++d) {  // uniform
+        StateSum<Val, kLog> o;
+        o.acc = __shfl_xor_sync(kAll, q.acc, 1 << d);
+        o.best = kLog ? 0 : __shfl_xor_sync(kAll, q.best, 1 << d);
+        if (d < nlog) q.Merge(o);
+      }
+    };
+    if (e.at >= 0) {
+      const int32_t rows_at = e.at + SliceRowsAt(e.blocks, e.tall);
+      for (int32_t blk = warp; blk < e.blocks; blk += nw) {
+        const uint32_t word = shared_words[e.at * 4 + blk * 32 + lane];
+        const LayerArc *r = shared_recs + rows_at + blk * (K * 32) + lane;
+        LayerArc x[K];
+        Val y[K];
+#pragma unroll
+        for (int u = 0; u < K; ++u) x[u] = r[u * 32];
+#pragma unroll
+        for (int u = 0; u < K; ++u) y[u] = vals[prev + x[u].other];
+        StateSum<Val, kLog> q;
+        q.Clear();
+#pragma unroll
+        for (int u = 0; u < K; ++u) q.Add(x[u], y[u]);
+        if (__any_sync(kAll, word & (7u << 16))) across(word, q);
+        if (word & kLaneHead) finish((int32_t)(word & kNoState), q);
+      }
+      for (int32_t t = warp; t < e.tall; t += nw) {
+        const int32_t blk = e.blocks + t;
+        const uint32_t word = shared_words[e.at * 4 + blk * 32 + lane],
+                       tw = shared_words[(e.at + (e.blocks + e.tall) * 8) * 4 + t];
+        const LayerArc *r = shared_recs + rows_at + (int32_t)(tw & 0xfffffu) * 32 + lane;
+        StateSum<Val, kLog> q;
+        q.Clear();
+#pragma unroll 4
+        for (int32_t u = 0; u < (int32_t)(tw >> 20); ++u) {
+          const LayerArc x = r[u * 32];
+          q.Add(x, vals[prev + x.other]);
         }
-        vals[cur + s] = q.acc;
-        out[s] = q.acc;
+        across(word, q);
+        if (word & kLaneHead) finish((int32_t)(word & kNoState), q);
       }
-      s0 += per_trip;
-      if (s0 >= now.e) break;  // uniform
-      s += per_trip;
-      k0 = k1 = 0;
-      if (s < now.e) {
-        k0 = ints[now.splits + s];
-        k1 = ints[now.splits + s + 1];
+    } else if (e.blocks >= 0) {  // too large for a slot: from L2
+      const int32_t l = dir == 0 ? step : nl - 1 - step;
+      const uint4 *region = pool + descs[(int64_t)dir * nl_total + lv0 + l].at;
+      const int32_t rows_at = SliceRowsAt(e.blocks, e.tall);
+      for (int32_t blk = warp; blk < e.blocks + e.tall; blk += nw) {
+        const uint32_t word = reinterpret_cast<const uint32_t *>(region)[blk * 32 + lane];
+        int32_t row = blk * K, rows = K;
+        if (blk >= e.blocks) {
+          const uint32_t tw = reinterpret_cast<const uint32_t *>(
+              region)[(e.blocks + e.tall) * 32 + blk - e.blocks];
+          row = (int32_t)(tw & 0xfffffu);
+          rows = (int32_t)(tw >> 20);
+        }
+        const LayerArc *r = reinterpret_cast<const LayerArc *>(region + rows_at) + row * 32 + lane;
+        StateSum<Val, kLog> q;
+        q.Clear();
+#pragma unroll 4
+        for (int32_t u = 0; u < rows; ++u) {
+          const LayerArc x = r[u * 32];
+          q.Add(x, vals[prev + x.other]);
+        }
+        across(word, q);
+        if (word & kLaneHead) finish((int32_t)(word & kNoState), q);
+      }
+    } else {
+      const int32_t l = dir == 0 ? step : nl - 1 - step;
+      const int32_t w = v.level_splits[lv0 + l + 1] - e.first_state;
+      for (int32_t j = tid; j < w && j < p.maxw; j += nc) {
+        StateSum<Val, kLog> q =
+            SumUnsliced<Val, kLog>(v, i, dir, l, e.first_state + j, vals + prev);
+        finish(j, q);
       }
     }
     sc.EndLayer(step, hi_shared, lane, status);
     if (kLog && tid == 0) my_scale[dir == 0 ? step : nl - 1 - step] = sc.K;
-    if (now.slot >= 0) {  // this warp has read the chunk
+    if (k == m) {  // this warp has read the slot
       __syncwarp();
       if (lane == 0)
-        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(SmemAddr(&empty[now.slot]))
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(SmemAddr(&empty[slot]))
                      : "memory");
     }
-    pb = now.b;
-    const int32_t t = prev_at;
-    prev_at = cur_at;
-    cur_at = t;
+    const int32_t t = prev;
+    prev = cur;
+    cur = t;
     layer_sync();
-    if (opened) {
-      if (*reinterpret_cast<volatile int32_t *>(&bad_shared)) return false;  // uniform
-      opened = false;
-    }
-    return true;
-  };
-  Ahead f0, f1;
-  fetch(0, f0);
-  for (int32_t step = 0; step < nl; step += 2) {
-    if (!layer(step, f0, f1)) break;
-    if (step + 1 < nl && !layer(step + 1, f1, f0)) break;
   }
   sc.End(lane, status);
+}
+
+// The same recursion for whatever left the range of SliceChain, or lost a copy: returns at
+// once unless *status is set.  Log values are (mantissa, exponent) pairs and the factors come
+// from the arcs' scores, so there is no range; everything is read from L2.
+template <typename Real, bool kLog>
+struct ExactSum {
+  double m = 0.0;
+  int32_t e = kZeroExp, best = -1;
+  Real top = -INFINITY;
+  __device__ __forceinline__ void Merge(const ExactSum &o) {
+    if (kLog) {
+      const int32_t En = max(e, o.e);
+      m = ScaleDown(m, e - En) + ScaleDown(o.m, o.e - En);
+      e = En;
+    } else if (o.top > top || (o.top == top && o.best > best)) {
+      top = o.top;
+      best = o.best;
+    }
+  }
+  __device__ __forceinline__ void Across(int lanes_below) {  // over the lanes `lanes_below` off
+    ExactSum o;
+    o.m = __shfl_xor_sync(0xffffffffu, m, lanes_below);
+    o.e = __shfl_xor_sync(0xffffffffu, e, lanes_below);
+    o.best = __shfl_xor_sync(0xffffffffu, best, lanes_below);
+    o.top = __shfl_xor_sync(0xffffffffu, top, lanes_below);
+    Merge(o);
+  }
+};
+
+template <typename Real, bool kLog>
+__global__ void __launch_bounds__(256)
+ExactChain(k2b200_fsa_view v, const uint4 *__restrict__ pool, const SliceDesc *__restrict__ descs,
+           double *mant, int32_t *expo, Real *fwd, Real *bwd, int32_t *__restrict__ entering,
+           int32_t dir_base, int32_t fsa_base, int32_t nl_total, int32_t K,
+           const int32_t *__restrict__ status) {
+  if (*status == 0) return;
+  const int32_t i = fsa_base + blockIdx.y, dir = blockIdx.x + dir_base;
+  const int32_t s_begin = v.row_splits1[i], s_end = v.row_splits1[i + 1];
+  const int32_t lv0 = v.level_offsets[i], nl = v.level_offsets[i + 1] - lv0;
+  const Arc *arcs = reinterpret_cast<const Arc *>(v.arcs);
+  Real *out = dir == 0 ? fwd : bwd;
+  double *m = mant + (int64_t)dir * v.num_states;
+  int32_t *x = expo + (int64_t)dir * v.num_states;
+  const int32_t root = dir == 0 ? s_begin : s_end - 1;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  for (int32_t step = 0; step < nl; ++step) {
+    const int32_t l = dir == 0 ? step : nl - 1 - step;
+    const int32_t b = v.level_splits[lv0 + l], e = v.level_splits[lv0 + l + 1];
+    auto add = [&](ExactSum<Real, kLog> &q, int32_t a) {
+      const Arc arc = arcs[a];
+      const int32_t other = s_begin + (dir == 0 ? arc.src : arc.dest);
+      ExactSum<Real, kLog> o;
+      if (kLog) {
+        int32_t k;
+        ExpToMantExp(arc.score, &o.m, &k);
+        o.m *= m[other];
+        o.e = o.m != 0.0 ? x[other] + k : kZeroExp;
+      } else {
+        o.top = out[other] + (Real)arc.score;
+        o.best = a;
+      }
+      q.Merge(o);
+    };
+    auto finish = [&](int32_t s, const ExactSum<Real, kLog> &q) {
+      if (kLog) {
+        int32_t E = q.e;
+        double mm = Renorm(q.m, &E);
+        if (mm == 0.0 && s == root) {
+          mm = 1.0;
+          E = 0;
+        }
+        m[s] = mm;
+        x[s] = E;
+        out[s] = mm == 0.0 ? (Real)-INFINITY
+                           : (Real)(log(mm) + (double)E * 0.69314718055994530942);
+      } else {
+        out[s] = q.top == (Real)-INFINITY && s == root ? (Real)0 : q.top;
+        if (dir == 0 && entering != nullptr) entering[s] = q.best;
+      }
+    };
+    const SliceDesc d = descs[(int64_t)dir * nl_total + lv0 + l];
+    if (d.blocks >= 0 && (*status & 1) == 0) {
+      const uint4 *region = pool + d.at;
+      const uint32_t *words = reinterpret_cast<const uint32_t *>(region);
+      for (int32_t blk = warp; blk < d.blocks + d.tall; blk += nw) {
+        const uint32_t word = words[blk * 32 + lane];
+        int32_t row = blk * K, rows = K;
+        if (blk >= d.blocks) {
+          const uint32_t tw = words[(d.blocks + d.tall) * 32 + blk - d.blocks];
+          row = (int32_t)(tw & 0xfffffu);
+          rows = (int32_t)(tw >> 20);
+        }
+        const LayerArc *r =
+            reinterpret_cast<const LayerArc *>(region + SliceRowsAt(d.blocks, d.tall)) + row * 32 +
+            lane;
+        ExactSum<Real, kLog> q;
+        for (int32_t u = 0; u < rows; ++u)
+          if (r[u * 32].arc >= 0) add(q, r[u * 32].arc);
+        const int32_t nlog = (int32_t)(word >> 16) & 7;
+        for (int32_t u = 0; u < 5; ++u) {
+          ExactSum<Real, kLog> o = q;
+          o.Across(1 << u);
+          if (u < nlog) q = o;
+        }
+        if (word & kLaneHead) finish(b + (int32_t)(word & kNoState), q);
+      }
+    } else {  // a warp per state looks through the layer's arcs
+      const int32_t ob = l > 0 ? v.level_splits[lv0 + l - 1] : b;
+      const int32_t f0 = v.row_splits2[ob], f1 = ob < b ? v.row_splits2[b] : f0;
+      for (int32_t s = b + warp; s < e; s += nw) {
+        const int32_t a0 = dir == 0 ? f0 : v.row_splits2[s],
+                      a1 = dir == 0 ? f1 : v.row_splits2[s + 1];
+        ExactSum<Real, kLog> q;
+        for (int32_t a = a0 + lane; a < a1; a += 32)
+          if (dir != 0 || s_begin + arcs[a].dest == s) add(q, a);
+        for (int u = 16; u > 0; u >>= 1) q.Across(u);
+        if (lane == 0) finish(s, q);
+      }
+    }
+    __syncthreads();
+  }
 }
 
 // The same for layers too wide for the ring: the CTAs of a cluster share a layer.  grid =
@@ -734,15 +1118,21 @@ FinishLayerScores(k2b200_fsa_view v, const double *m, const int32_t *__restrict_
 
 namespace {
 struct ChainScratch {
-  LayerArc *fwd_arcs, *bwd_arcs;
-  int32_t *scale, *status;  // status and the words of ChainScale are cleared together
-  double *vals;  // [2][num_states], for results in float
+  // cleared together: status, the slice pool's counter, the words of ChainScale
+  int32_t *status, *hi_slots;
+  unsigned long long *pool_used;
+  uint4 *pool;        // sliced layers
+  SliceDesc *descs;   // [2][layers]
+  LayerArc *fwd_arcs, *bwd_arcs;  // wide layers
+  int32_t *scale, *expo;
+  double *vals;  // [2][num_states]
+  int64_t pool_units;
   size_t clear_bytes, bytes;
 };
-}  // namespace
 
-static ChainScratch CarveScratch(const k2b200_fsa_view *v, void *scratch) {
-  ChainScratch c;
+ChainScratch CarveScratch(const k2b200_fsa_view *v, const ChainPlan &p, int32_t ndir,
+                          void *scratch) {
+  ChainScratch c = {};
   char *base = reinterpret_cast<char *>(scratch);
   size_t off = 0;
   auto take = [&](size_t bytes) {
@@ -751,44 +1141,81 @@ static ChainScratch CarveScratch(const k2b200_fsa_view *v, void *scratch) {
     return base + at;
   };
   const size_t na = (size_t)std::max(v->num_arcs, 1), ns = (size_t)std::max(v->num_states, 1);
+  const size_t layers = (size_t)v->num_fsas * (size_t)std::max(v->max_layers, 1);
   c.clear_bytes = sizeof(int32_t) * (4 + 4 * (size_t)v->num_fsas);
   c.status = reinterpret_cast<int32_t *>(take(c.clear_bytes));
-  c.fwd_arcs = reinterpret_cast<LayerArc *>(take(sizeof(LayerArc) * na));
-  c.bwd_arcs = reinterpret_cast<LayerArc *>(take(sizeof(LayerArc) * na));
-  c.scale = reinterpret_cast<int32_t *>(
-      take(sizeof(int32_t) * 2 * (size_t)v->num_fsas * (size_t)std::max(v->max_layers, 1)));
+  c.pool_used = reinterpret_cast<unsigned long long *>(c.status + 2);
+  c.hi_slots = c.status + 4;
+  if (p.wide) {
+    c.fwd_arcs = reinterpret_cast<LayerArc *>(take(sizeof(LayerArc) * na));
+    c.bwd_arcs = reinterpret_cast<LayerArc *>(take(sizeof(LayerArc) * na));
+  } else {
+    c.pool_units = SlicePoolUnits(v, p) * ndir;
+    c.pool = reinterpret_cast<uint4 *>(take(sizeof(uint4) * (size_t)c.pool_units));
+    c.descs = reinterpret_cast<SliceDesc *>(take(sizeof(SliceDesc) * 2 * layers));
+  }
+  c.scale = reinterpret_cast<int32_t *>(take(sizeof(int32_t) * 2 * layers));
+  c.expo = reinterpret_cast<int32_t *>(take(sizeof(int32_t) * 2 * ns));
   c.vals = reinterpret_cast<double *>(take(sizeof(double) * 2 * ns));
   c.bytes = off;
   return c;
 }
+}  // namespace
 
-size_t LayerScratchBytes(const k2b200_fsa_view *v) { return CarveScratch(v, nullptr).bytes; }
+size_t LayerScratchBytes(const k2b200_fsa_view *v, int32_t ndir) {
+  return CarveScratch(v, PlanChain(v, ndir), ndir, nullptr).bytes;
+}
 
-int32_t *LayerStatusWord(const k2b200_fsa_view *v, void *scratch) {
-  return CarveScratch(v, scratch).status;
+bool LayerScoresNeedIncoming(const k2b200_fsa_view *v, int32_t ndir) {
+  const ChainPlan p = PlanChain(v, ndir);
+  return !p.ok || p.wide || v->num_arcs == 0;
 }
 
 template <typename Val, bool kLog>
 static int32_t LaunchChain(const k2b200_fsa_view *v, const ChainScratch &c, const ChainPlan &p,
                            Val *val_fwd, Val *val_bwd, int32_t *entering, cudaStream_t stream) {
   const int32_t ndir = (val_fwd != nullptr) + (val_bwd != nullptr), dir_base = val_fwd ? 0 : 1;
-  if (p.wide)
-    K2B_CUDA_OK(cudaFuncSetAttribute(LayerChainWide<Val, kLog>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
+  const int32_t layers = v->num_fsas * v->max_layers;
+  if (!p.wide) {
+    // a warp per layer while layers are small (there are many of them)
+    const bool one = p.maxw <= 512 && v->num_arcs / std::max(layers, 1) <= 256;
+    const size_t fixed = sizeof(int32_t) * ((one ? 2 : 5) * (size_t)p.maxw + 32);
+    // room for a layer well above the mean, with several CTAs per SM
+    const int64_t mean = (SlicePoolUnits(v, p) - 1024) / std::max(layers, 1);
+    int32_t buf = (int32_t)std::min<int64_t>(2 * mean, one ? 512 : 3072);
+    if (!one) buf = (int32_t)std::min<int64_t>(buf, (int64_t)(kLayerSmemBudget - fixed) / 16);
+    const size_t smem = (one ? 4 : 1) * (fixed + 16 * (size_t)buf);
+    auto slice = one ? SliceLayers<kLog, 1> : SliceLayers<kLog, 4>;
+    K2B_CUDA_OK(cudaFuncSetAttribute(slice, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)kLayerSmemBudget));
-  auto kernel = p.group_log2 ? LayerChain<Val, kLog, 8> : LayerChain<Val, kLog, 1>;
-  K2B_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    { slice<<<dim3(one ? CeilDiv(layers, 4) : layers, ndir), 128, smem, stream>>>(
+        *v, dir_base, p.rows, p.maxw, v->max_layer_arcs, buf, layers, c.pool_units, c.pool_used,
+        c.pool, c.descs, c.status); NoteLaunch(); }
+    auto chain = p.rows == 2   ? SliceChain<Val, kLog, 2>
+                 : p.rows == 3 ? SliceChain<Val, kLog, 3>
+                 : p.rows == 4 ? SliceChain<Val, kLog, 4>
+                               : SliceChain<Val, kLog, 8>;
+    K2B_CUDA_OK(cudaFuncSetAttribute(chain, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)kLayerSmemBudget));
+    for (int32_t first = 0; first < v->num_fsas; first += 65535) {
+      const int32_t n = std::min(v->num_fsas - first, 65535);
+      { chain<<<dim3(ndir, n), 32 * (p.warps + 1), p.bytes, stream>>>(
+          *v, c.pool, c.descs, val_fwd, val_bwd, entering, c.scale, dir_base, first, layers, p,
+          c.status); NoteLaunch(); }
+    }
+    K2B_CUDA_OK(cudaGetLastError());
+    return kOk;
+  }
+  auto pack = kLog ? PackLayerArcs<true> : PackLayerArcs<false>;
+  { pack<<<CeilDiv(v->num_arcs, 256), 256, 0, stream>>>(*v, val_fwd ? c.fwd_arcs : nullptr,
+                                                        val_bwd ? c.bwd_arcs : nullptr, c.status);
+    NoteLaunch(); }
+  K2B_CUDA_OK(cudaFuncSetAttribute(LayerChainWide<Val, kLog>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)kLayerSmemBudget));
   for (int32_t first = 0; first < v->num_fsas; first += 65535) {
-    const int32_t n = std::min(v->num_fsas - first, 65535);
-    if (!p.wide) {
-      { kernel<<<dim3(ndir, n), 32 * (p.warps + 1), p.bytes, stream>>>(
-          *v, c.fwd_arcs, c.bwd_arcs, val_fwd, val_bwd, entering, c.scale, dir_base, first, p,
-          c.status); NoteLaunch(); }
-      continue;
-    }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ndir * p.team, n);
+    cfg.gridDim = dim3(ndir * p.team, std::min(v->num_fsas - first, 65535));
     cfg.blockDim = dim3(32 * p.warps);
     cfg.dynamicSmemBytes = p.bytes;
     cfg.stream = stream;
@@ -801,7 +1228,7 @@ static int32_t LaunchChain(const k2b200_fsa_view *v, const ChainScratch &c, cons
     cfg.numAttrs = 1;
     K2B_CUDA_OK(cudaLaunchKernelEx(&cfg, LayerChainWide<Val, kLog>, *v,
                                    (const LayerArc *)c.fwd_arcs, (const LayerArc *)c.bwd_arcs,
-                                   val_fwd, val_bwd, entering, c.scale, c.status + 4, dir_base,
+                                   val_fwd, val_bwd, entering, c.scale, c.hi_slots, dir_base,
                                    first, p, c.status));
     NoteLaunch();
   }
@@ -812,22 +1239,17 @@ static int32_t LaunchChain(const k2b200_fsa_view *v, const ChainScratch &c, cons
 template <typename Real>
 int32_t LaunchLayerScores(const k2b200_fsa_view *v, int32_t log_semiring, Real *fwd, Real *bwd,
                           int32_t *entering, void *scratch, size_t scratch_bytes,
-                          cudaStream_t stream, bool *launched) {
+                          cudaStream_t stream, bool *launched, const int32_t **redo_if) {
   *launched = false;
-  if (scratch == nullptr || v->num_arcs == 0 || v->row_ids2 == nullptr) return kOk;
-  if (fwd != nullptr && (v->in_src == nullptr || v->in_score == nullptr)) return kOk;
-  const ChainPlan p = PlanChain(v, (fwd != nullptr) + (bwd != nullptr));
-  const ChainScratch c = CarveScratch(v, scratch);
-  if (!p.ok || scratch_bytes < c.bytes) return kOk;
-  // bulk copies need 16-byte aligned sources
-  auto aligned16 = [](const void *ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15) == 0; };
-  if (!aligned16(scratch) || !aligned16(v->row_splits2) || (fwd && !aligned16(v->in_splits)))
+  *redo_if = nullptr;
+  if (scratch == nullptr || v->num_arcs == 0 || v->row_ids1 == nullptr || v->row_ids2 == nullptr)
     return kOk;
+  const int32_t ndir = (fwd != nullptr) + (bwd != nullptr), dir_base = fwd ? 0 : 1;
+  const ChainPlan p = PlanChain(v, ndir);
+  const ChainScratch c = CarveScratch(v, p, ndir, scratch);
+  if (!p.ok || scratch_bytes < c.bytes || (reinterpret_cast<uintptr_t>(scratch) & 15)) return kOk;
+  if (p.wide && fwd != nullptr && (v->in_src == nullptr || v->in_score == nullptr)) return kOk;
   K2B_CUDA_OK(cudaMemsetAsync(c.status, 0, c.clear_bytes, stream));
-  auto pack = log_semiring ? PackLayerArcs<true> : PackLayerArcs<false>;
-  { pack<<<CeilDiv(v->num_arcs, 256), 256, 0, stream>>>(*v, fwd ? c.fwd_arcs : nullptr,
-                                                        bwd ? c.bwd_arcs : nullptr, c.status);
-    NoteLaunch(); }
   if (log_semiring) {
     const bool in_place = sizeof(Real) == sizeof(double);
     double *vf = in_place ? reinterpret_cast<double *>(fwd) : c.vals,
@@ -853,14 +1275,26 @@ int32_t LaunchLayerScores(const k2b200_fsa_view *v, int32_t log_semiring, Real *
   } else {
     K2B_FORWARD((LaunchChain<Real, false>(v, c, p, fwd, bwd, entering, stream)));
   }
+  if (p.wide) {
+    *redo_if = c.status;
+  } else {
+    auto exact = log_semiring ? ExactChain<Real, true> : ExactChain<Real, false>;
+    for (int32_t first = 0; first < v->num_fsas; first += 65535) {
+      { exact<<<dim3(ndir, std::min(v->num_fsas - first, 65535)), 256, 0, stream>>>(
+          *v, c.pool, c.descs, c.vals, c.expo, fwd, bwd, entering, dir_base, first,
+          v->num_fsas * v->max_layers, p.rows, c.status); NoteLaunch(); }
+    }
+  }
   K2B_CUDA_OK(cudaGetLastError());
   *launched = true;
   return kOk;
 }
 
 template int32_t LaunchLayerScores<float>(const k2b200_fsa_view *, int32_t, float *, float *,
-                                          int32_t *, void *, size_t, cudaStream_t, bool *);
+                                          int32_t *, void *, size_t, cudaStream_t, bool *,
+                                          const int32_t **);
 template int32_t LaunchLayerScores<double>(const k2b200_fsa_view *, int32_t, double *, double *,
-                                           int32_t *, void *, size_t, cudaStream_t, bool *);
+                                           int32_t *, void *, size_t, cudaStream_t, bool *,
+                                           const int32_t **);
 
 }  // namespace k2b

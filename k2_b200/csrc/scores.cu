@@ -8,6 +8,7 @@
 // tot_scores; k2/csrc/tensor_ops.cu:304-334 IndexAdd; k2/csrc/fsa_algo.cu:869-1144
 // ShortestPath; k2/csrc/fsa.cu:54-217 properties) but walks the layers inside one
 // persistent kernel per (FSA, direction) instead of launching per state batch.
+#include <algorithm>
 #include <cmath>
 
 #include "scores_internal.cuh"
@@ -338,13 +339,15 @@ static int32_t LaunchScores(const k2b200_fsa_view *v, int32_t log_semiring, Real
   if (ndir == 0 || v->num_fsas == 0) return kOk;
   PhaseTimer timer(kPhaseScores, stream);
   bool launched = false;
+  const int32_t *redo_if = nullptr;
   K2B_FORWARD(LaunchLayerScores<Real>(v, log_semiring, fwd, bwd, entering, scratch, scratch_bytes,
-                                      stream, &launched));
-  // if a CTA found the layer bounds violated, or values out of range, redo everything the
-  // general way
+                                      stream, &launched, &redo_if));
+  if (launched && redo_if == nullptr) return kOk;
+  K2B_REQUIRE(fwd == nullptr || v->num_arcs == 0 || (v->in_splits && v->in_arcs && v->row_ids2),
+              "forward scores need the incoming-arc index and row_ids2");
+  // if the layer bounds were violated, or values out of range, everything is redone
   if (launched)
-    return LaunchGeneric<Real>(v, log_semiring, fwd, bwd, entering, LayerStatusWord(v, scratch),
-                               stream);
+    return LaunchGeneric<Real>(v, log_semiring, fwd, bwd, entering, redo_if, stream);
   return LaunchGeneric<Real>(v, log_semiring, fwd, bwd, entering, nullptr, stream);
 }
 
@@ -418,7 +421,14 @@ int32_t k2b200_fsa_incoming_layers(const k2b200_fsa_view *v, int32_t *in_splits,
 }
 
 size_t k2b200_fsa_scores_scratch_bytes(const k2b200_fsa_view *v) {
-  return v ? LayerScratchBytes(v) : 0;
+  // (two directions need at least what one does)
+  return v ? std::max(LayerScratchBytes(v, 1), LayerScratchBytes(v, 2)) : 0;
+}
+size_t k2b200_fsa_scores_dir_scratch_bytes(const k2b200_fsa_view *v, int32_t directions,
+                                           int32_t *needs_incoming) {
+  if (v == nullptr) return 0;
+  if (needs_incoming) *needs_incoming = LayerScoresNeedIncoming(v, directions) ? 1 : 0;
+  return LayerScratchBytes(v, directions);
 }
 
 int32_t k2b200_fsa_scores(const k2b200_fsa_view *v, int32_t log_semiring, int32_t use_double,
@@ -427,9 +437,6 @@ int32_t k2b200_fsa_scores(const k2b200_fsa_view *v, int32_t log_semiring, int32_
   K2B_REQUIRE(v != nullptr, "NULL view");
   K2B_REQUIRE(v->row_splits1 && v->row_splits2 && v->level_offsets && v->level_splits,
               "NULL pointer in the FsaVec view");
-  K2B_REQUIRE(forward == nullptr || v->num_arcs == 0 ||
-                  (v->in_splits && v->in_arcs && v->row_ids2),
-              "forward scores need the incoming-arc index and row_ids2");
   if (use_double)
     return LaunchScores<double>(v, log_semiring, reinterpret_cast<double *>(forward),
                                 reinterpret_cast<double *>(backward), entering_arcs, scratch,

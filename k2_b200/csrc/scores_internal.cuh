@@ -103,15 +103,15 @@ __device__ void LayeredScoresDevice(const k2b200_fsa_view &v, int32_t i, int32_t
 }
 
 
-// Strictly layered FsaVecs (layer_scores.cu).  *launched stays false when the view does not
-// qualify.  A non-zero status word afterwards means that its layer bounds did not hold or its
-// values left the range of the recursion: the results must be recomputed.
-size_t LayerScratchBytes(const k2b200_fsa_view *v);
-int32_t *LayerStatusWord(const k2b200_fsa_view *v, void *scratch);
+// Strictly layered FsaVecs (layer_scores.cu), ndir of the two directions.  *launched stays
+// false when the view does not qualify.  *redo_if: NULL, or a word that is non-zero afterwards
+// when the results must be recomputed by the general kernel.
+size_t LayerScratchBytes(const k2b200_fsa_view *v, int32_t ndir);
+bool LayerScoresNeedIncoming(const k2b200_fsa_view *v, int32_t ndir);
 template <typename Real>
 int32_t LaunchLayerScores(const k2b200_fsa_view *v, int32_t log_semiring, Real *fwd, Real *bwd,
                           int32_t *entering, void *scratch, size_t scratch_bytes,
-                          cudaStream_t stream, bool *launched);
+                          cudaStream_t stream, bool *launched, const int32_t **redo_if);
 // Incoming-arc index of such an FsaVec; *done stays false when a layer is too wide for it.
 int32_t BuildLayerIncoming(const k2b200_fsa_view *v, int32_t *in_splits, int32_t *in_arcs,
                            int32_t *in_src, float *in_score, cudaStream_t stream, bool *done);

@@ -233,11 +233,16 @@ class Fsa(object):
         entering = None
         if want_forward and not log_semiring:
             entering = torch.empty(ns, dtype=torch.int32, device=dev)
-        view, keep = arcs.view(want_incoming=want_forward)
         scratch, nscratch = None, 0
+        need_incoming = ctypes.c_int32(1)
+        view, keep = arcs.view(want_incoming=False)
         if arcs._layer_bounds[0]:
-            nscratch = _lib.lib.k2b200_fsa_scores_scratch_bytes(ctypes.byref(view))
+            nscratch = _lib.lib.k2b200_fsa_scores_dir_scratch_bytes(
+                ctypes.byref(view), int(want_forward) + int(want_backward),
+                ctypes.byref(need_incoming))
             scratch = torch.empty(nscratch, dtype=torch.uint8, device=dev)
+        if want_forward and need_incoming.value:
+            view, keep = arcs.view(want_incoming=True)
         with torch.cuda.device(dev):
             _lib.check(_lib.lib.k2b200_fsa_scores(
                 ctypes.byref(view), int(log_semiring), int(use_double_scores), _lib.ptr(fwd),
