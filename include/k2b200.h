@@ -75,7 +75,7 @@ int32_t k2b200_row_splits_to_row_ids(const int32_t *row_splits, int32_t num_rows
                                      void *stream);
 
 /* n int32 values from (pageable or pinned) host memory to device memory, passed as
- * kernel parameters in launches of up to 960 values: asynchronous on `stream`, the
+ * kernel parameters in launches of up to 8000 values: asynchronous on `stream`, the
  * host array is free for reuse on return, and the copy engine is not involved.  For
  * the few hundred integers of a batch description (segments, row_splits, symbol
  * lists), where k2 copies through Array1::To (k2/csrc/array.h:234-250). */
@@ -144,6 +144,14 @@ int32_t k2b200_ctc_graph(const int32_t *sym_row_splits, const int32_t *symbols,
                          int32_t num_seqs, int32_t num_symbols, int32_t modified,
                          int32_t *row_splits1, int32_t *row_splits2, void *arcs,
                          int32_t *aux_labels, void *tmp, void *stream);
+/* The same graphs with their band tables (k2b200_band_tables), in one or two launches from host
+ * arrays: h_meta = first symbol of every graph [num_seqs+1], first arc of every graph
+ * [num_seqs+1], symbols[num_symbols]; band_states / band_arcs as sized by
+ * k2b200_band_tables_bytes; meta_tmp: room for the int32 of h_meta (device). */
+int32_t k2b200_ctc_graph_host(const int32_t *h_meta, int32_t num_seqs, int32_t num_symbols,
+                              int32_t modified, int32_t *row_splits1, int32_t *row_splits2,
+                              void *arcs, int32_t *aux_labels, void *band_states, void *band_arcs,
+                              int32_t *meta_tmp, void *stream);
 
 /* ---------------------------------------------------------------------------
  * DenseFsaVec.
@@ -473,8 +481,8 @@ int32_t k2b200_dense_loss_backward_log_probs(const k2b200_intersect_args *args, 
  *     band_arcs: its second) and *status (device int32) bit 0 = some graph is not a band
  *     graph, in which case the tables must not be used.  They depend on the graphs only and
  *     can be kept for as long as the arcs do not change.
- *   k2b200_band_loss_supported: *supported = 0 when the sizes do not fit (more than 512
- *     states in a graph, unaligned rows, frames beyond shared memory);
+ *   k2b200_band_loss_supported: *supported = 0 when the sizes do not fit (more than 1024
+ *     states in a graph, rows or frames beyond shared memory);
  *     k2b200_last_error() says which.  Host-side only.
  *   k2b200_band_loss_forward: tot_scores[num_fsas] (device, float64; -inf for a graph
  *     with no surviving path; NaN if a copy into shared memory timed out, see
@@ -537,6 +545,42 @@ int32_t k2b200_band_loss_backward(const k2b200_band_loss_args *args, void *works
                                   int32_t grad_col_off, void *stream);
 int32_t k2b200_band_loss_status(const k2b200_band_loss_args *args, void *workspace,
                                 size_t workspace_bytes, void *stream, int32_t *status);
+
+/* The pieces of a whole training step, for hosts that want no kernels of their own around them.
+ *   k2b200_band_loss_plan: supported, workspace bytes and, in *exclusive_rows, whether no two
+ *     sequences share rows of the log-probs - one pass over the batch description.
+ *   k2b200_band_loss_forward_reduce: k2b200_band_loss_forward plus the loss of
+ *     k2/python/k2/ctc_loss.py:72-84 (`reduce`, may be NULL).  With reduce->logits the
+ *     log-probs at args->log_probs are written first: log_softmax of the logits, for the rows
+ *     of the sequences.
+ *   k2b200_band_loss_backward_dense (exclusive rows only): WRITES the gradient of the log-probs
+ *     (softmax != 0: of the logits) to every row, rows of no sequence included
+ *     (grad_log_probs may be NULL); grad_a (may be NULL) as in k2b200_band_loss_backward. */
+typedef struct {
+  int32_t mode;        /* 0: totals only, 1: loss = -sum, 2: loss = mean of -tot / length,
+                        * of totals rounded to float32 */
+  int32_t lens_type;   /* of lens[num_fsas] (device): 1 int32, 2 int64, 3 float32, 4 float64 */
+  const void *lens;
+  float *loss;         /* device */
+  const float *logits; /* NULL, or [log_prob_rows, num_classes] (device) */
+} k2b200_band_reduce;
+typedef struct {
+  const void *grad;    /* device: dL/dtot (stride elements apart) or, with stride 0, one value */
+  int32_t is_double;   /* float64, else float32 */
+  int32_t stride;
+  int32_t negate;      /* the totals enter with a minus sign */
+  int32_t lens_type;   /* != 0: divided by (length x number of graphs), as for mode 2 */
+  const void *lens;
+} k2b200_band_upstream;
+int32_t k2b200_band_loss_plan(const k2b200_band_loss_args *args, int32_t *supported,
+                              int32_t *exclusive_rows, size_t *bytes);
+int32_t k2b200_band_loss_forward_reduce(const k2b200_band_loss_args *args, void *workspace,
+                                        size_t workspace_bytes, void *stream, double *tot_scores,
+                                        float *beam_used, const k2b200_band_reduce *reduce);
+int32_t k2b200_band_loss_backward_dense(const k2b200_band_loss_args *args, void *workspace,
+                                        size_t workspace_bytes,
+                                        const k2b200_band_upstream *upstream, float *grad_a,
+                                        float *grad_log_probs, int32_t softmax, void *stream);
 void k2b200_debug_set_copy_wait_limit(int32_t polls);
 
 /* ---------------------------------------------------------------------------

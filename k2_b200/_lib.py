@@ -19,6 +19,13 @@ if not os.path.exists(LIB_PATH):
 
 lib = ctypes.CDLL(LIB_PATH)
 
+try:  # the native host layer (csrc/host/torch_host.cc)
+    from . import _host  # noqa: F401,E402
+except ImportError as e:
+    raise ImportError(
+        f"k2_b200/_host.so could not be loaded ({e}): build it with `python k2_b200/build.py`"
+    ) from e
+
 c_i32 = ctypes.c_int32
 c_i64 = ctypes.c_int64
 c_vp = ctypes.c_void_p
@@ -49,6 +56,16 @@ class BandLossArgs(ctypes.Structure):
         ("output_beam", c_f32), ("max_states", c_i32), ("max_arcs", c_i32),
         ("zero_fill", c_vp), ("zero_fill_bytes", c_sz),
     ]
+
+
+class BandReduce(ctypes.Structure):
+    _fields_ = [("mode", c_i32), ("lens_type", c_i32), ("lens", c_vp), ("loss", c_vp),
+                ("logits", c_vp)]
+
+
+class BandUpstream(ctypes.Structure):
+    _fields_ = [("grad", c_vp), ("is_double", c_i32), ("stride", c_i32), ("negate", c_i32),
+                ("lens_type", c_i32), ("lens", c_vp)]
 
 
 class LatticeOut(ctypes.Structure):
@@ -187,6 +204,15 @@ _sig("k2b200_band_loss_forward", c_i32,
 _sig("k2b200_band_loss_backward", c_i32,
      [ctypes.POINTER(BandLossArgs), c_vp, c_sz, c_vp, c_i32, c_vp, c_vp, c_vp, c_i32, c_i32,
       c_vp])
+_sig("k2b200_band_loss_plan", c_i32,
+     [ctypes.POINTER(BandLossArgs), ctypes.POINTER(c_i32), ctypes.POINTER(c_i32),
+      ctypes.POINTER(c_sz)])
+_sig("k2b200_band_loss_forward_reduce", c_i32,
+     [ctypes.POINTER(BandLossArgs), c_vp, c_sz, c_vp, c_vp, ctypes.POINTER(c_f32),
+      ctypes.POINTER(BandReduce)])
+_sig("k2b200_band_loss_backward_dense", c_i32,
+     [ctypes.POINTER(BandLossArgs), c_vp, c_sz, ctypes.POINTER(BandUpstream), c_vp, c_vp, c_i32,
+      c_vp])
 _sig("k2b200_band_loss_status", c_i32,
      [ctypes.POINTER(BandLossArgs), c_vp, c_sz, c_vp, ctypes.POINTER(c_i32)])
 _sig("k2b200_debug_set_copy_wait_limit", None, [c_i32])
@@ -212,6 +238,8 @@ _sig("k2b200_index_select_i32", c_i32, [c_vp, c_i64, c_vp, c_i32, c_vp, c_vp])
 _sig("k2b200_ctc_graph_tmp_bytes", c_sz, [c_i32])
 _sig("k2b200_ctc_graph", c_i32,
      [c_vp, c_vp, c_i32, c_i32, c_i32, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp])
+_sig("k2b200_ctc_graph_host", c_i32,
+     [c_vp, c_i32, c_i32, c_i32, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp])
 _sig("k2b200_dense_fsa_vec_fill", c_i32,
      [c_vp, c_i64, c_i64, c_i32, c_vp, c_vp, c_i32, c_vp, c_i32, c_vp])
 _sig("k2b200_dense_fsa_vec_backward", c_i32,
@@ -253,7 +281,7 @@ EXPORTED = [
     "k2b200_best_paths",
     "k2b200_dense_fsa_vec_fill", "k2b200_dense_fsa_vec_backward",
     "k2b200_dense_fsa_vec_from_logits", "k2b200_dense_fsa_vec_from_logits_backward",
-    "k2b200_ctc_graph_tmp_bytes", "k2b200_ctc_graph",
+    "k2b200_ctc_graph_tmp_bytes", "k2b200_ctc_graph", "k2b200_ctc_graph_host",
     "k2b200_fsa_properties_tmp_bytes", "k2b200_fsa_properties",
     "k2b200_fsa_levels_tmp_bytes", "k2b200_fsa_levels",
     "k2b200_dense_loss_supported", "k2b200_dense_loss_workspace_bytes",
@@ -270,7 +298,8 @@ EXPORTED = [
     "k2b200_online_decode_load_all", "k2b200_online_decode_store_all",
     "k2b200_band_tables_bytes", "k2b200_band_tables", "k2b200_band_loss_supported",
     "k2b200_band_loss_workspace_bytes", "k2b200_band_loss_forward",
-    "k2b200_band_loss_backward", "k2b200_band_loss_status",
+    "k2b200_band_loss_backward", "k2b200_band_loss_status", "k2b200_band_loss_plan",
+    "k2b200_band_loss_forward_reduce", "k2b200_band_loss_backward_dense",
     "k2b200_debug_set_copy_wait_limit",
 ]
 
@@ -366,6 +395,7 @@ def release_workspaces() -> None:
     """Gives the idle workspaces back to torch's allocator."""
     with _ws_lock:
         _ws_idle.clear()
+    _host.release_workspaces()
 
 
 def upload_i32(arr, device) -> torch.Tensor:

@@ -589,8 +589,8 @@ _band_state = {"status": 0}  # status word of the last verified band-path forwar
 def _band_loss_args(a_fsas: Fsa, b_fsas: DenseFsaVec, a_to_b_map: Optional[torch.Tensor],
                     output_beam: float, max_states: int, max_arcs: int):
     """(args, keep-alive objects, host map) of the k2b200_band_loss_* entry points, or
-    None when they do not apply: `b_fsas` must come from a float32 CUDA log-prob tensor
-    with 16-byte aligned rows and the graphs must be band graphs of at most 512 states."""
+    None when they do not apply: `b_fsas` must come from a float32 CUDA log-prob tensor and
+    the graphs must be band graphs of at most 1024 states."""
     src = b_fsas._source
     a = a_fsas.arcs
     cached = b_fsas._band_args
@@ -622,7 +622,7 @@ def _band_loss_args_uncached(a_fsas: Fsa, b_fsas: DenseFsaVec,
         return None
     lp = src[0]
     if not (lp.is_cuda and lp.dtype == torch.float32 and lp.is_contiguous()
-            and lp.device == a.device and lp.shape[-1] % 4 == 0 and lp.data_ptr() % 16 == 0):
+            and lp.device == a.device):
         return None
     h_map = None
     if a_to_b_map is not None:
@@ -646,7 +646,7 @@ def _band_loss_args_uncached(a_fsas: Fsa, b_fsas: DenseFsaVec,
         host = a._band_host = (states, h_rs1, np.ascontiguousarray(a.h_arc_splits, dtype=np.int32),
                                int(np.diff(h_rs1).max(initial=0)))
     _, h_rs1, h_as, most_states = host
-    if most_states > 512:
+    if most_states > 1024:
         return None
     frames = np.diff(b_fsas.h_row_splits) - 1
     first = src[1]
@@ -739,40 +739,49 @@ class _BandTotScoresFunction(torch.autograd.Function):
         return None, None, None, None, grad_a, grad_b
 
 
-class _BandNegSumFunction(torch.autograd.Function):
-    """`-tot_scores.sum(dtype=torch.float32)` over `_BandTotScoresFunction` as ONE node of
-    the autograd graph (the `reduction="sum"` of k2/python/k2/ctc_loss.py:72-84 on the band
-    path): the same kernels, two nodes less to build in the forward and to run in the
-    backward, on the thread that feeds the GPU."""
-
-    @staticmethod
-    def forward(ctx, a_fsas: Fsa, b_fsas: DenseFsaVec, band, use_double_scores: bool,
-                unused_scores_a: torch.Tensor, unused_scores_b: torch.Tensor) -> torch.Tensor:
-        tot = _BandTotScoresFunction.forward(ctx, a_fsas, b_fsas, band, use_double_scores,
-                                             unused_scores_a, unused_scores_b)
-        ctx.tot_shape = tot.shape
-        # (-1 * tot_scores).to(float32).sum() of the reference: the reduction casts every
-        # element before adding, and negation commutes with rounding, so the bits are the same
-        return -tot.sum(dtype=torch.float32)
-
-    @staticmethod
-    def backward(ctx, loss_grad: torch.Tensor):
-        tot_grad = (-loss_grad).to(torch.float64).expand(ctx.tot_shape)  # stride 0
-        return _BandTotScoresFunction.backward(ctx, tot_grad)
+# what the native band loss makes of the total scores
+_TOTALS, _NEG_SUM, _MEAN = 0, 1, 2
 
 
-def band_ctc_loss_sum(a_fsas: Fsa, b_fsas: DenseFsaVec, output_beam: float,
-                      use_double_scores: bool = True) -> Optional[torch.Tensor]:
-    """`-intersect_dense_tot_scores(...).sum(dtype=torch.float32)` on the band kernels, or
-    None when they do not take these inputs."""
-    args = _band_loss_args(a_fsas, b_fsas, None, output_beam, 15000000, 1073741824)
-    if args is None or BAND_VERIFY:
+def _band_native(a_fsas: Fsa, b_fsas: DenseFsaVec, a_to_b_map: Optional[torch.Tensor],
+                 output_beam: float, max_states: int, max_arcs: int, mode: int,
+                 use_double_scores: bool,
+                 target_lengths: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
+    """Total scores of band graphs, or their negated sum / mean, as ONE node of the autograd
+    graph (csrc/host/torch_host.cc over k2b200_band_loss_*), reading the log-probs or logits
+    that `b_fsas` was made from; None when it does not take these inputs."""
+    src, logits = b_fsas._source, False
+    if src is None:
+        src, logits = b_fsas._logit_source, True
+    if src is None or BAND_VERIFY or not a_fsas.arcs.values().is_cuda:
         return None
-    src = b_fsas._source
-    from_log_probs = src[0].requires_grad and src[0].dtype == torch.float32
-    scores_b = src[0] if (from_log_probs or b_fsas._scores is None) else b_fsas.scores
-    return _BandNegSumFunction.apply(a_fsas, b_fsas, args, use_double_scores, a_fsas.scores,
-                                     scores_b)
+    # without autograd on the log-probs the gradient (if any) is that of the score matrix,
+    # which then exists already
+    if b_fsas._scores is not None and not src[0].requires_grad:
+        return None
+    graph = a_fsas.arcs.band_graph()
+    if graph is None:
+        return None
+    h_map = None
+    if a_to_b_map is not None:
+        assert a_to_b_map.ndim == 1 and a_to_b_map.dtype == torch.int32
+        h_map = np.ascontiguousarray(a_to_b_map.detach().cpu().numpy(), dtype=np.int32)
+        if h_map.shape[0] != a_fsas.arcs.num_fsas:
+            raise RuntimeError(f"a_fsas.Dim0() ({a_fsas.arcs.num_fsas}) != "
+                               f"a_to_b_map.Dim() ({h_map.shape[0]})")
+    return _lib._host.band_loss(graph, a_fsas.scores, src[0], logits, src[1], b_fsas.h_row_splits,
+                                h_map, output_beam, max_states, max_arcs, mode, use_double_scores,
+                                target_lengths)
+
+
+def band_ctc_loss(a_fsas: Fsa, b_fsas: DenseFsaVec, output_beam: float, reduction: str,
+                  use_double_scores: bool,
+                  target_lengths: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+    """The reductions "sum" and "mean" of k2/python/k2/ctc_loss.py:72-84 on the band kernels,
+    or None when they do not take these inputs."""
+    return _band_native(a_fsas, b_fsas, None, output_beam, 15000000, 1073741824,
+                        _NEG_SUM if reduction == "sum" else _MEAN, use_double_scores,
+                        target_lengths)
 
 
 def band_loss_supported(a_fsas: Fsa, b_fsas: DenseFsaVec,
@@ -808,6 +817,11 @@ def intersect_dense_tot_scores(a_fsas: Fsa, b_fsas: DenseFsaVec, output_beam: fl
     directly rather than through the score matrix and the adjoint of its layout.
     Band graphs (CTC) take kernels of their own that read the log-probs in place
     (`band=False` keeps them on the general kernels)."""
+    if band:
+        tot = _band_native(a_fsas, b_fsas, a_to_b_map, output_beam, max_states, max_arcs, _TOTALS,
+                           use_double_scores)
+        if tot is not None:
+            return tot
     src = b_fsas._source
     from_log_probs = src is not None and src[0].requires_grad and src[0].dtype == torch.float32
     args = _band_loss_args(a_fsas, b_fsas, a_to_b_map, output_beam, max_states,

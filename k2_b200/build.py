@@ -1,7 +1,8 @@
-"""Builds k2_b200/libk2b200.so from k2_b200/csrc/*.cu with nvcc for sm_100a.
+"""Builds k2_b200/libk2b200.so from k2_b200/csrc/*.cu with nvcc for sm_100a, and
+k2_b200/_host.so, the torch side of the host layer, from k2_b200/csrc/host/*.cc.
 
-The library is built in-tree (next to this file) so that it travels with a
-snapshot of the repository; nothing is JIT-compiled at import time.
+Both are built in-tree (next to this file) so that they travel with a snapshot of the
+repository; nothing is JIT-compiled at import time.
 """
 import glob
 import os
@@ -34,7 +35,45 @@ def _stale() -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+HOST_PATH = os.path.join(_HERE, "_host.so")
+HOST_SOURCE = os.path.join(CSRC, "host", "torch_host.cc")
+
+
+def _host_stale() -> bool:
+    if not os.path.exists(HOST_PATH):
+        return True
+    t = os.path.getmtime(HOST_PATH)
+    deps = [HOST_SOURCE, os.path.join(_HERE, "..", "include", "k2b200.h"),
+            os.path.abspath(__file__)]
+    return any(os.path.getmtime(d) > t for d in deps)
+
+
+def _host_command():
+    """g++ on the one translation unit that includes torch's headers; libk2b200.so is found
+    next to it, torch's libraries are loaded by `import torch`."""
+    import importlib.util
+    import sysconfig
+    torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
+    cuda = os.path.join(os.path.dirname(os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")), "..")
+    inc = os.path.join(torch_dir, "include")
+    return ["/usr/bin/g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+            "-D_GLIBCXX_USE_CXX11_ABI=1", "-DTORCH_EXTENSION_NAME=_host",
+            "-isystem", inc, "-isystem", os.path.join(inc, "torch", "csrc", "api", "include"),
+            "-isystem", os.path.join(cuda, "include"),
+            "-isystem", sysconfig.get_paths()["include"], HOST_SOURCE, "-o", HOST_PATH,
+            "-L" + _HERE, "-l:libk2b200.so", "-Wl,-rpath,$ORIGIN",
+            "-L" + os.path.join(torch_dir, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu",
+            "-ltorch_cuda", "-ltorch", "-ltorch_python"]
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
+    _build_library(force, verbose)
+    if force or _host_stale():
+        subprocess.check_call(_host_command())
+    return LIB_PATH
+
+
+def _build_library(force: bool, verbose: bool) -> str:
     if not force and not _stale():
         return LIB_PATH
     nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")

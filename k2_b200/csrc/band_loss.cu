@@ -45,16 +45,15 @@
 #include <vector>
 
 #include "../../include/k2b200.h"
+#include "band_tables.cuh"
 #include "common.cuh"
 #include "cp_async.cuh"
 #include "prob_math.cuh"
 
 namespace k2b {
 
-constexpr int32_t kNoLabel = INT32_MIN;
-constexpr int kBandMaxStates = 512;
+constexpr int kBandMaxStates = 1024;
 constexpr int kVitK = 4;              // states per thread of BandViterbi
-constexpr int kPrepK = 16;            // states per lane of BandPrep's row scan
 constexpr int kPrepLevels = 16;       // levels per chunk: their lists share one padded size
 constexpr int kPrepSub = 8;           // levels per warp of BandPrep
 constexpr int kGradLevels = 4;        // levels per warp of BandGrad
@@ -74,21 +73,11 @@ struct BandInfo {
   int32_t frames;      // T
   int32_t lp_row;      // row of the log-prob matrix that holds frame 0
   int32_t level_off;   // sum over earlier pairs of (T + 2)
+  int32_t zero_end;    // rows [lp_row + T, zero_end) belong to no sequence (dense gradient)
+  int32_t pad;
   int64_t grid_off;    // sum over earlier pairs of (T + 2) * pitch
 };
 
-// Per state (idx01): the arcs entering it.  w[d] = score of the arc from state s - d
-// (-inf: no such arc); label = their common label (kNoLabel: no entering arc).
-struct __align__(16) BandState {
-  float w[3];
-  int32_t label;
-};
-// Per (state, d): exp(w[d]) = f * 2^k and the arc's index (idx012), -1 if absent.
-struct __align__(16) BandArc {
-  double f;
-  int32_t k;
-  int32_t arc;
-};
 // Entry of a level's list of surviving states.
 struct __align__(8) BandItem {
   int32_t label;  // of the arcs entering the state
@@ -227,13 +216,13 @@ __global__ void BandTables(const int32_t *__restrict__ row_splits1, int32_t num_
 __device__ __forceinline__ float Max3(float a, float b, float c) { return fmaxf(fmaxf(a, b), c); }
 
 constexpr int kVitMaxBatches = 4;  // batches of rows in flight
-constexpr int kVitMaxWarps = 8;
+constexpr int kVitMaxWarps = 12;
 
 __global__ void __launch_bounds__(32 * kVitMaxWarps)
 BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ tab,
             const float *__restrict__ lp, int32_t C, float *__restrict__ vf,
-            float *__restrict__ vb, int32_t F, int32_t nbatch, int32_t xch_pad,
-            int32_t wait_limit, int32_t *__restrict__ status) {
+            float *__restrict__ vb, int32_t F, int32_t nbatch, int32_t slot_floats,
+            int32_t xch_pad, int32_t wait_limit, int32_t *__restrict__ status) {
   constexpr int K = kVitK;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full[kVitMaxBatches];
@@ -246,8 +235,8 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
   if (S == 0) return;
   const int32_t H = F >> 1;         // lanes that recompute the neighbour's states
   const int32_t own = 32 - H;       // lanes whose states this warp owns
-  float *ring = reinterpret_cast<float *>(smem_raw);                    // [nbatch][F][C]
-  float *xch = ring + (size_t)nbatch * F * C;                           // [2][xch_pad], state s at s + 4H
+  float *ring = reinterpret_cast<float *>(smem_raw);       // [nbatch][slot_floats]: F rows
+  float *xch = ring + (size_t)nbatch * slot_floats;        // [2][xch_pad], state s at s + 4H
   if (tid == 0) {
     for (int st = 0; st < nbatch; ++st) MbarInit(&full[st], 1);
     MbarInitFence();
@@ -257,6 +246,10 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
   __syncthreads();
   const int32_t num_batches = (T + F - 1) / F;
   const float *lp0 = lp + (int64_t)f.lp_row * C;
+  // A row may start anywhere (C need not be a multiple of four): a batch is copied from the
+  // 16-byte boundary at or before its first element to the one at or after its last.
+  const uint32_t lp0_words = (uint32_t)(reinterpret_cast<uintptr_t>(lp0) >> 2);
+  auto words_off = [&](int32_t r) { return (int32_t)((lp0_words + (uint32_t)r * (uint32_t)C) & 3u); };
   int32_t issued = 0;
   auto issue = [&]() {  // thread 0 only: the rows of the next batch into the next slot
     if (issued >= num_batches) return;
@@ -264,10 +257,12 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
     // batch q: forward rows [qF, min((q+1)F, T)); backward rows [max(T-(q+1)F, 0), T-qF)
     const int32_t r0 = dir == 0 ? q * F : max(T - (q + 1) * F, 0);
     const int32_t r1 = dir == 0 ? min((q + 1) * F, T) : T - q * F;
-    const unsigned bytes = (unsigned)(r1 - r0) * 4u * (unsigned)C;
+    const int32_t off = words_off(r0);
+    const unsigned bytes = (((unsigned)(r1 - r0) * (unsigned)C + (unsigned)off + 3u) & ~3u) * 4u;
     const int32_t slot = q % nbatch;
     MbarArriveExpectTx(&full[slot], bytes);
-    BulkCopyG2S(ring + (size_t)slot * F * C, lp0 + (int64_t)r0 * C, bytes, &full[slot]);
+    BulkCopyG2S(ring + (size_t)slot * slot_floats, lp0 + (int64_t)r0 * C - off, bytes,
+                &full[slot]);
     ++issued;
   };
   if (tid == 0)
@@ -330,7 +325,7 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
         if (tid == 0 && !late) issue();  // into the slot batch q - 1 used
       }
       const int32_t nf = min(F, T - q * F);
-      const float *rowbuf = ring + (size_t)slot * F * C;
+      const float *rowbuf = ring + (size_t)slot * slot_floats + words_off(q * F);
 #pragma unroll 4
       for (int32_t r = 0; r < nf; ++r, rowbuf += C) {
         float x[K];
@@ -426,7 +421,8 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
       xpar ^= 1;
       if (q > 0 && tid == 0 && !late) issue();
       const int32_t r1 = T - q * F, r0 = max(T - (q + 1) * F, 0);
-      const float *rowbuf = ring + (size_t)slot * F * C + (size_t)(r1 - 1 - r0) * C;
+      const float *rowbuf =
+          ring + (size_t)slot * slot_floats + words_off(r0) + (size_t)(r1 - 1 - r0) * C;
 #pragma unroll 4
       for (int32_t r = r1 - 1; r >= r0; --r, rowbuf -= C) {  // level r from level r + 1
         float x[K + 2];
@@ -468,9 +464,10 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
 // ---------------------------------------------------------------------------
 // Which states survive (intersect_dense.cu:289-296): state s of level l is kept iff
 // vf[l][s] + vb[l][s] > cutoff.  grid = (level chunks, pairs), a warp per kKeepLevels levels;
-// lane j looks at states K j .. K j + K - 1 (K = 16, or 8 when no graph has more than 256
-// states, which keeps more lanes busy) and writes their keep bits: bit (s & 15) of the 16-bit
-// word keep[(level_off + l) * 32 + s / 16] is the bit of state s.  totals[0] += surviving states, totals[2] += the arcs
+// lane j looks at states K j .. K j + K - 1 (K = 8, 16 or 32 for graphs of up to 256, 512 or
+// 1024 states: the smallest keeps the most lanes busy) and writes their keep bits: the bit of
+// state s is bit (s & 7) of byte s / 8 of the level's row of keep_bytes bytes (64, or 128
+// with more than 512 states).  totals[0] += surviving states, totals[2] += the arcs
 // leaving them: the sizes the beam reduction looks at (intersect_dense.cu:289-320), which
 // the host can read while the kernels behind this one run.
 // ---------------------------------------------------------------------------
@@ -480,9 +477,10 @@ template <int K>
 __global__ void __launch_bounds__(128)
 BandKeep(const BandInfo *__restrict__ infos, const int32_t *__restrict__ a_row_splits2,
          const float *__restrict__ vf, const float *__restrict__ vb, float beam,
-         uint16_t *__restrict__ keep_bits, float *__restrict__ cutoffs,
+         unsigned char *__restrict__ keep_bits, float *__restrict__ cutoffs,
          unsigned long long *__restrict__ totals, int32_t count_arcs) {
-  static_assert(K == 8 || K == 16, "keep bits are stored as bytes or 16-bit words");
+  static_assert(K == 8 || K == 16 || K == 32, "keep bits are stored as bytes or words");
+  constexpr int kRowBytes = K == 32 ? 128 : 64;
   constexpr unsigned kAll = 0xffffffffu;
   const int32_t i = blockIdx.y;
   const BandInfo f = infos[i];
@@ -514,10 +512,12 @@ BandKeep(const BandInfo *__restrict__ infos, const int32_t *__restrict__ a_row_s
       if (__fadd_rn(F.z, B.z) > cutoff) keep |= 4u << (4 * c);
       if (__fadd_rn(F.w, B.w) > cutoff) keep |= 8u << (4 * c);
     }
-    if (K == 16) {
-      keep_bits[(int64_t)(f.level_off + l) * 32 + lane] = (uint16_t)keep;
-    } else {  // the same layout byte by byte; states 256 .. 511 do not exist
-      unsigned char *row = reinterpret_cast<unsigned char *>(keep_bits + (int64_t)(f.level_off + l) * 32);
+    unsigned char *row = keep_bits + (int64_t)(f.level_off + l) * kRowBytes;
+    if (K == 32) {
+      reinterpret_cast<uint32_t *>(row)[lane] = keep;
+    } else if (K == 16) {
+      reinterpret_cast<uint16_t *>(row)[lane] = (uint16_t)keep;
+    } else {  // states 256 .. 511 do not exist
       row[lane] = (unsigned char)keep;
       row[32 + lane] = 0;
     }
@@ -563,15 +563,16 @@ BandKeep(const BandInfo *__restrict__ infos, const int32_t *__restrict__ a_row_s
 constexpr float kMinLeanDense = -60.0f;   // dense score of a surviving arc
 constexpr int32_t kMaxLeanArcExp = 60, kMinLeanArcExp = -90;  // binary exponent of exp(arc score)
 
+// K = 16 or 32 states per lane of the scan (32 when a graph has more than 512 states).
+template <int K>
 __global__ void __launch_bounds__(128)
 BandPrep(const BandInfo *__restrict__ infos, const BandState *__restrict__ tab,
-         const BandArc *__restrict__ tabf, const uint16_t *__restrict__ keep_bits,
+         const BandArc *__restrict__ tabf, const unsigned char *__restrict__ keep_bits,
          const float *__restrict__ lp, int32_t C, const float *__restrict__ vf,
          const float *__restrict__ vb, const float *__restrict__ cutoffs,
          BandItem *__restrict__ items, BandFactor *__restrict__ factors,
          int2 *__restrict__ lists, int32_t *__restrict__ chunk_r, int32_t *__restrict__ unfit,
          int32_t s_pad) {
-  constexpr int K = kPrepK;
   constexpr unsigned kAll = 0xffffffffu;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int32_t i = blockIdx.y;
@@ -587,9 +588,10 @@ BandPrep(const BandInfo *__restrict__ infos, const BandState *__restrict__ tab,
   // per warp: a word per state for the current and the previous level (zero outside the
   // lists), and the two lists
   uint16_t *meta_sm = reinterpret_cast<uint16_t *>(smem_raw) +
-                      (size_t)warp * (4 * s_pad + 32 * (kPrepLevels + 2));  // [2][s_pad]
-  uint16_t *list_sm = meta_sm + 2 * s_pad;                                  // [2][s_pad]
-  uint16_t *keep_sm = list_sm + 2 * s_pad;  // [kPrepLevels + 2][32]: the lanes' keep bits
+                      (size_t)warp * (4 * s_pad + 64 * (kPrepSub + 2));  // [2][s_pad]
+  uint16_t *list_sm = meta_sm + 2 * s_pad;                               // [2][s_pad]
+  // [kPrepSub + 2][32]: the lanes' keep bits
+  uint32_t *keep_sm = reinterpret_cast<uint32_t *>(list_sm + 2 * s_pad);
   for (int32_t k = lane; k < 2 * s_pad; k += 32) meta_sm[k] = 0;
   const float *fg = vf + f.grid_off, *bg = vb + f.grid_off;
   const float cutoff = cutoffs[i];
@@ -604,8 +606,10 @@ BandPrep(const BandInfo *__restrict__ infos, const BandState *__restrict__ tab,
   const int32_t lo = min(first, ca), hi = max(last, cb - 1);
 #pragma unroll 6
   for (int32_t l = lo; l <= hi; ++l) {
-    const uint32_t keep = keep_bits[(int64_t)(f.level_off + l) * 32 + lane];
-    if (l >= first && l <= last) keep_sm[(l - first) * 32 + lane] = (uint16_t)keep;
+    const int64_t word = (int64_t)(f.level_off + l) * 32 + lane;
+    const uint32_t keep = K == 32 ? reinterpret_cast<const uint32_t *>(keep_bits)[word]
+                                  : reinterpret_cast<const uint16_t *>(keep_bits)[word];
+    if (l >= first && l <= last) keep_sm[(l - first) * 32 + lane] = keep;
     const int32_t n = __reduce_add_sync(kAll, __popc(keep));
     if (l >= ca && l < cb) longest = max(longest, n);
   }
@@ -1079,20 +1083,18 @@ BandChainLists(const BandInfo *__restrict__ infos, const BandFactor *__restrict_
 // The same recursion with a (mantissa, exponent) pair per state, for the graphs marked in
 // `unfit`; every other graph returns at once.  exp(dense score) is recomputed from the
 // log-probs, the arc factors come from the graph's tables: no range limit.
-__global__ void __launch_bounds__(32)
-BandChainExact(const BandInfo *__restrict__ infos, const BandArc *__restrict__ tabf,
-               const float *__restrict__ lp, int32_t C, const BandItem *__restrict__ items,
-               const int2 *__restrict__ lists, double *__restrict__ am,
-               int32_t *__restrict__ ae, double *__restrict__ bm, int32_t *__restrict__ be,
-               double *__restrict__ tot, BandTotal *__restrict__ total,
-               const int32_t *__restrict__ unfit, int32_t *__restrict__ status, int32_t st_pad,
-               int32_t lv_pad, int32_t wait_limit) {
+__device__ void
+ExactWalk(const BandInfo *__restrict__ infos, const BandArc *__restrict__ tabf,
+          const float *__restrict__ lp, int32_t C, const BandItem *__restrict__ items,
+          const int2 *__restrict__ lists, double *__restrict__ am, int32_t *__restrict__ ae,
+          double *__restrict__ bm, int32_t *__restrict__ be, double *__restrict__ tot,
+          BandTotal *__restrict__ total, const int32_t *__restrict__ unfit,
+          int32_t *__restrict__ status, int32_t st_pad, int32_t lv_pad, int32_t wait_limit) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full[kChainSlots];
   constexpr unsigned kAll = 0xffffffffu;
   const int dir = blockIdx.x;
   const int32_t i = blockIdx.y;
-  if (unfit[i] == 0) return;  // the lean recursion served this graph
   const BandInfo f = infos[i];
   const int lane = threadIdx.x;
   const int32_t S = f.num_states, T = f.frames, pitch = f.pitch, L = T + 2;
@@ -1220,6 +1222,54 @@ BandChainExact(const BandInfo *__restrict__ infos, const BandArc *__restrict__ t
   if (dir == 0 && lane == 0 && (*status & kStatusLate)) tot[i] = nan("");
 }
 
+// What the caller makes of the totals (k2b200_band_reduce), done by the CTA that finishes
+// last: three launches of elementwise and reduction kernels less.
+struct LossSpec {
+  int32_t mode;       // 0: nothing, 1: -sum, 2: mean of -tot / length; both of float32 values
+  int32_t lens_type;  // of the lengths: 1 int32, 2 int64, 3 float32, 4 float64
+  const void *lens;
+  float *loss;
+};
+__device__ __forceinline__ double LengthOf(const void *lens, int32_t type, int32_t i) {
+  switch (type) {
+    case 1: return (double)reinterpret_cast<const int32_t *>(lens)[i];
+    case 2: return (double)reinterpret_cast<const int64_t *>(lens)[i];
+    case 3: return (double)reinterpret_cast<const float *>(lens)[i];
+    default: return reinterpret_cast<const double *>(lens)[i];
+  }
+}
+
+__global__ void __launch_bounds__(32)
+BandChainExact(const BandInfo *__restrict__ infos, const BandArc *__restrict__ tabf,
+               const float *__restrict__ lp, int32_t C, const BandItem *__restrict__ items,
+               const int2 *__restrict__ lists, double *__restrict__ am,
+               int32_t *__restrict__ ae, double *__restrict__ bm, int32_t *__restrict__ be,
+               double *__restrict__ tot, BandTotal *__restrict__ total,
+               const int32_t *__restrict__ unfit, int32_t *__restrict__ status, int32_t st_pad,
+               int32_t lv_pad, int32_t wait_limit, LossSpec spec, uint32_t *__restrict__ ticket) {
+  if (unfit[blockIdx.y] != 0)
+    ExactWalk(infos, tabf, lp, C, items, lists, am, ae, bm, be, tot, total, unfit, status, st_pad,
+              lv_pad, wait_limit);
+  if (spec.mode == 0) return;
+  const int lane = threadIdx.x;
+  uint32_t t = 0;
+  __syncwarp();
+  if (lane == 0) {
+    __threadfence();
+    t = atomicAdd(ticket, 1u);
+  }
+  if (__shfl_sync(0xffffffffu, t, 0) + 1 != 2 * gridDim.y) return;
+  __threadfence();
+  double sum = 0.0;
+  for (int32_t i = lane; i < (int32_t)gridDim.y; i += 32) {
+    const float x = -(float)__ldcg(tot + i);
+    sum += spec.mode == 2 ? (double)(x / (float)LengthOf(spec.lens, spec.lens_type, i)) : (double)x;
+  }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+  if (lane == 0) *spec.loss = (float)(spec.mode == 2 ? sum / (double)gridDim.y : sum);
+}
+
 // ---------------------------------------------------------------------------
 // Gradients.  grid = (level chunks, pairs), a warp per chunk of kGradLevels levels.
 // posterior(l, s) = alpha_l[s] * beta_l[s] / Z is dL/d(dense score of state s's label on
@@ -1229,6 +1279,22 @@ BandChainExact(const BandInfo *__restrict__ infos, const BandArc *__restrict__ t
 // alpha_{l-1}[src] e^w p_l[dest] beta_l[dest] / Z, is added to grad_a[arc]; the warp keeps
 // alpha of the level before by state number in shared memory for that.
 // ---------------------------------------------------------------------------
+// dL/dtot of a graph: what the caller's upstream gradient says (k2b200_band_upstream).
+struct GradSpec {
+  const void *grad;
+  int32_t is_double, stride, negate;
+  int32_t lens_type;  // != 0: the upstream value is divided by (length of the graph * graphs)
+  const void *lens;
+  int32_t n;
+  __device__ __forceinline__ double Of(int32_t i) const {
+    const int64_t at = (int64_t)i * stride;
+    double g = is_double ? reinterpret_cast<const double *>(grad)[at]
+                         : (double)reinterpret_cast<const float *>(grad)[at];
+    if (lens_type) g /= LengthOf(lens, lens_type, i) * n;
+    return negate ? -g : g;
+  }
+};
+
 template <bool kArcs>
 __global__ void __launch_bounds__(128)
 BandGrad(const BandInfo *__restrict__ infos, const BandArc *__restrict__ tabf,
@@ -1237,8 +1303,8 @@ BandGrad(const BandInfo *__restrict__ infos, const BandArc *__restrict__ tabf,
          const int32_t *__restrict__ ae, const double *__restrict__ bm,
          const int32_t *__restrict__ be, const int32_t *__restrict__ a_scale,
          const int32_t *__restrict__ b_scale, const BandTotal *__restrict__ total,
-         const int32_t *__restrict__ unfit, const double *__restrict__ tot_grad,
-         int32_t tot_grad_stride, float *__restrict__ grad_a, float *__restrict__ grad_b,
+         const int32_t *__restrict__ unfit, const GradSpec upstream,
+         float *__restrict__ grad_a, float *__restrict__ grad_b,
          const int32_t *__restrict__ grad_row0, int32_t grad_pitch, int32_t grad_col_off,
          int32_t C, int32_t st_pad) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1259,11 +1325,12 @@ BandGrad(const BandInfo *__restrict__ infos, const BandArc *__restrict__ tabf,
   const double *am0 = am + f.grid_off, *bm0 = bm + f.grid_off;
   const int32_t *ae0 = ae + f.grid_off, *be0 = be + f.grid_off;
   const int32_t *as0 = a_scale + f.level_off, *bs0 = b_scale + f.level_off;
-  const double tg = tot_grad[(int64_t)i * tot_grad_stride];
+  const double tg = upstream.Of(i);
   const int64_t row0 = grad_row0 != nullptr ? grad_row0[i] : f.lp_row;
   const float *lp0 = lp + (int64_t)f.lp_row * C;
   // this warp's row of sums, one per column of the gradient (all zero between levels)
-  const int32_t cols = C + grad_col_off;
+  // (without a gradient for the dense scores only the arcs are wanted)
+  const int32_t cols = grad_b != nullptr ? C + grad_col_off : 0;
   uint32_t *sums = reinterpret_cast<uint32_t *>(smem_raw) + (size_t)warp * cols;
   for (int32_t k = lane; k < cols; k += 32) sums[k] = 0u;
   __syncwarp();
@@ -1319,7 +1386,7 @@ BandGrad(const BandInfo *__restrict__ infos, const BandArc *__restrict__ tabf,
         if (alm != 0.0 && bem != 0.0) {
           const int32_t ale = exact ? ae0[row + j] : ea_l, bee = exact ? be0[row + j] : eb_l;
           const int32_t col = it.label + grad_col_off;
-          if (it.label != kNoLabel && it.label < C && col >= 0) {
+          if (grad_b != nullptr && it.label != kNoLabel && it.label < C && col >= 0) {
             g = (float)(alm * bem * zinv * Pow2Clamp(ale + bee - z.e));
             key = col;
           }
@@ -1366,14 +1433,166 @@ BandGrad(const BandInfo *__restrict__ infos, const BandArc *__restrict__ tabf,
 }
 
 // ---------------------------------------------------------------------------
+// The same gradient for log-probs (or logits) that no two sequences share, written whole:
+// every element of the rows of a sequence and of the rows up to the next one is stored
+// once, so the caller's buffer needs no clearing (at 128 MB of log-probs the clear and the
+// scattered additions took 29 + 26 us of memory time, this takes 30).  A warp per kDenseRows
+// rows; the row's sums gather in shared memory in fixed point as in BandGrad.  kSoftmax: the
+// rows are log_softmax of the tensor the gradient is for, d = g - softmax * sum(g).
+// ---------------------------------------------------------------------------
+constexpr int kDenseRows = 4;
+
+template <bool kSoftmax>
+__global__ void __launch_bounds__(128)
+BandGradRows(const BandInfo *__restrict__ infos, const float *__restrict__ lp,
+             const BandItem *__restrict__ items, const int2 *__restrict__ lists,
+             const double *__restrict__ am, const int32_t *__restrict__ ae,
+             const double *__restrict__ bm, const int32_t *__restrict__ be,
+             const int32_t *__restrict__ a_scale, const int32_t *__restrict__ b_scale,
+             const BandTotal *__restrict__ total, const int32_t *__restrict__ unfit,
+             const GradSpec upstream, float *__restrict__ grad, int32_t C, int32_t C_pad) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr unsigned kAll = 0xffffffffu;
+  const int32_t i = blockIdx.y;
+  const BandInfo f = infos[i];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int32_t T = f.frames, rows = f.zero_end - f.lp_row;
+  const int32_t r0 = (blockIdx.x * (blockDim.x >> 5) + warp) * kDenseRows;
+  if (r0 >= rows) return;
+  const int32_t r1 = min(r0 + kDenseRows, rows);
+  uint32_t *sums = reinterpret_cast<uint32_t *>(smem_raw) + (size_t)warp * C_pad;
+  for (int32_t k = lane; k < C_pad; k += 32) sums[k] = 0u;
+  const BandTotal z = total[i];
+  const bool dead = z.m == 0.0 || f.num_states == 0;  // no path survives: all zero
+  const double zinv = dead ? 0.0 : 1.0 / z.m;
+  const bool exact = unfit[i] != 0;
+  const double tg = dead ? 0.0 : upstream.Of(i);
+  const int2 *lst = lists + f.level_off + 1;  // row r is level r + 1
+  const BandItem *items0 = items + f.grid_off;
+  const double *am0 = am + f.grid_off, *bm0 = bm + f.grid_off;
+  const int32_t *ae0 = ae + f.grid_off, *be0 = be + f.grid_off;
+  const int32_t *as0 = a_scale + f.level_off + 1, *bs0 = b_scale + f.level_off + 1;
+  // the first 32 entries of the rows are requested together, before any is used
+  int2 ls4[kDenseRows];
+  BandItem it4[kDenseRows];
+  double al4[kDenseRows], be4[kDenseRows];
+#pragma unroll
+  for (int u = 0; u < kDenseRows; ++u) {
+    ls4[u] = !dead && r0 + u < min(r1, T) ? lst[r0 + u] : make_int2(0, 0);
+    al4[u] = be4[u] = 0.0;
+    it4[u].s = 0;
+    it4[u].label = kNoLabel;
+  }
+#pragma unroll
+  for (int u = 0; u < kDenseRows; ++u)
+    if (lane < ls4[u].y) {
+      it4[u] = items0[ls4[u].x + lane];
+      al4[u] = am0[ls4[u].x + lane];
+      be4[u] = bm0[ls4[u].x + lane];
+    }
+  __syncwarp();
+#pragma unroll
+  for (int u = 0; u < kDenseRows; ++u) {
+    const int32_t r = r0 + u;
+    if (r >= r1) break;
+    const int32_t n = ls4[u].y;
+    const int64_t row = ls4[u].x;
+    uint32_t added = 0;
+    if (n > 0) {
+      const int32_t ea_l = as0[r], eb_l = bs0[r];
+      for (int32_t j = lane; j < n; j += 32) {
+        const bool first = j < 32;
+        const BandItem it = first ? it4[u] : items0[row + j];
+        const double alm = first ? al4[u] : am0[row + j], bem = first ? be4[u] : bm0[row + j];
+        if (alm == 0.0 || bem == 0.0 || it.label < 0 || it.label >= C) continue;
+        const int32_t ale = exact ? ae0[row + j] : ea_l, bee = exact ? be0[row + j] : eb_l;
+        const float g = (float)(alm * bem * zinv * Pow2Clamp(ale + bee - z.e));
+        const uint32_t fixed = __float2uint_rn(g * 2147483648.0f);
+        added += fixed;
+        atomicAdd(&sums[it.label], fixed);
+      }
+    }
+    __syncwarp();
+    float *out = grad + (int64_t)(f.lp_row + r) * C;
+    const bool vec = (C & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+    if (n == 0) {
+      if (vec) {
+        for (int32_t c = lane * 4; c < C; c += 128)
+          *reinterpret_cast<float4 *>(out + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      } else {
+        for (int32_t c = lane; c < C; c += 32) out[c] = 0.0f;
+      }
+      continue;
+    }
+    const float tgf = (float)tg;
+    auto value = [&](uint32_t fixed) { return tgf * ((float)fixed * (1.0f / 2147483648.0f)); };
+    if (!kSoftmax) {
+      if (vec) {
+#pragma unroll 4
+        for (int32_t c = lane * 4; c < C; c += 128) {
+          const uint4 x = *reinterpret_cast<const uint4 *>(sums + c);
+          if (x.x | x.y | x.z | x.w) *reinterpret_cast<uint4 *>(sums + c) = make_uint4(0, 0, 0, 0);
+          *reinterpret_cast<float4 *>(out + c) =
+              make_float4(value(x.x), value(x.y), value(x.z), value(x.w));
+        }
+      } else {
+#pragma unroll 4
+        for (int32_t c = lane; c < C; c += 32) {
+          const uint32_t x = sums[c];
+          if (x) sums[c] = 0u;
+          out[c] = value(x);
+        }
+      }
+    } else {
+      // (the sum of a row's posteriors is at most 1, its fixed-point value fits 32 bits)
+      const float total_g = value(__reduce_add_sync(kAll, added));
+      const float *x = lp + (int64_t)(f.lp_row + r) * C;
+#pragma unroll 4
+      for (int32_t c = lane; c < C; c += 32) {
+        const uint32_t y = sums[c];
+        if (y) sums[c] = 0u;
+        out[c] = value(y) - expf(__ldg(x + c)) * total_g;
+      }
+    }
+    __syncwarp();  // the row of sums is zero again
+  }
+}
+
+// log_probs rows of the sequences = log_softmax of the logits rows.  A warp per row; the same
+// expressions as LogSoftmaxFill (dense.cu).
+__global__ void __launch_bounds__(256)
+LogSoftmaxRows(const BandInfo *__restrict__ infos, const float *__restrict__ logits, int32_t C,
+               float *__restrict__ log_probs) {
+  const BandInfo f = infos[blockIdx.y];
+  const int32_t r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= f.frames) return;
+  const float *in = logits + (int64_t)(f.lp_row + r) * C;
+  float *out = log_probs + (int64_t)(f.lp_row + r) * C;
+  float mx = -INFINITY;
+#pragma unroll 4
+  for (int32_t c = lane; c < C; c += 32) mx = fmaxf(mx, __ldg(in + c));
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, d));
+  float sum = 0.0f;
+#pragma unroll 4
+  for (int32_t c = lane; c < C; c += 32) sum += expf(__ldg(in + c) - mx);
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+  const float lse = logf(sum);
+#pragma unroll 4
+  for (int32_t c = lane; c < C; c += 32) out[c] = (__ldg(in + c) - mx) - lse;
+}
+
+// ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
 struct BandLayout {
   std::vector<BandInfo> infos;
   int64_t grid_elems = 0, reachable_states = 0, levels = 0;
   long long arc_frames = 0;
-  int32_t max_states = 0, max_frames = 0;
-  int32_t vit_threads = 32, vit_frames = 0, vit_batches = 0, xch_pad = 0;
+  int32_t max_states = 0, max_frames = 0, max_rows = 0;
+  int32_t vit_threads = 32, vit_frames = 0, vit_batches = 0, vit_slot = 0, xch_pad = 0;
+  int32_t keep_row = 64, first_row = 0;
   int32_t st_pad = 0, lv_pad = 0;
   size_t chain_smem = 0, exact_smem = 0, viterbi_smem = 0, prep_smem = 0;
   size_t off_infos, off_vf, off_vb, off_items, off_factors, off_lists, off_chunk_r, off_keep, off_cutoffs, off_am, off_ae, off_bm,
@@ -1435,37 +1654,53 @@ static int32_t MakeBandLayout(const k2b200_band_loss_args *a, BandLayout *L) {
   }
   L->grid_elems = grid;
   L->levels = levels;
+  {
+    // rows of the log-probs that no sequence covers, each given to the sequence before it
+    std::vector<int32_t> order(a->num_fsas);
+    for (int32_t i = 0; i < a->num_fsas; ++i) order[i] = i;
+    std::sort(order.begin(), order.end(), [&](int32_t x, int32_t y) {
+      return L->infos[x].lp_row < L->infos[y].lp_row;
+    });
+    for (int32_t k = 0; k < a->num_fsas; ++k) {
+      BandInfo &f = L->infos[order[k]];
+      const int64_t end = k + 1 < a->num_fsas ? L->infos[order[k + 1]].lp_row : a->log_prob_rows;
+      f.zero_end = (int32_t)std::min<int64_t>(std::max<int64_t>(end, f.lp_row + f.frames), INT32_MAX);
+      if (end < f.lp_row + f.frames) L->exclusive_rows = false;
+      L->max_rows = std::max(L->max_rows, f.zero_end - f.lp_row);
+      f.pad = 0;
+    }
+    L->first_row = L->infos[order[0]].lp_row;
+    if (a->log_prob_rows >= INT32_MAX) L->exclusive_rows = false;
+  }
   // BandViterbi: frames per batch (even, at most 16) so that at least two batches of rows
   // fit in shared memory, up to three batches within ~100 KB so that two CTAs share an SM
   {
     const size_t row_bytes = sizeof(float) * (size_t)a->num_classes;
     int32_t F = 16;
-    while (F > 2 && 2 * F * row_bytes > kBandSmemBudget - 8192) F >>= 1;
+    while (F > 2 && 2 * F * row_bytes > kBandSmemBudget - 16384) F >>= 1;
     L->vit_frames = F;
+    L->vit_slot = (int32_t)(((size_t)F * a->num_classes + 6 + 3) & ~(size_t)3);
     L->vit_batches = (int32_t)std::max<size_t>(
         2, std::min<size_t>(3, (100 * 1024) / std::max<size_t>(F * row_bytes, 1)));
     const int32_t own_states = (32 - F / 2) * kVitK;
     const int32_t warps = std::max(1, CeilDiv(std::max(L->max_states, 1), own_states));
     L->vit_threads = 32 * warps;
     L->xch_pad = (warps * own_states + 4 * kVitK * (F / 2) + 3) & ~3;
-    L->viterbi_smem = (size_t)L->vit_batches * F * row_bytes + sizeof(float) * 2 * (size_t)L->xch_pad;
-    if (warps > kVitMaxWarps || 2 * F * row_bytes > kBandSmemBudget - 8192) {
+    L->viterbi_smem = sizeof(float) * ((size_t)L->vit_batches * L->vit_slot + 2 * (size_t)L->xch_pad);
+    if (warps > kVitMaxWarps || 2 * F * row_bytes > kBandSmemBudget - 16384) {
       L->ok = false;
       L->why = "too many states or classes for the Viterbi kernel";
     }
   }
   L->st_pad = ((L->max_states + 4) + 15) & ~15;
   L->lv_pad = (L->max_frames + 2 + 3) & ~3;
-  L->prep_smem = (size_t)4 * (8 * L->st_pad + 64 * (kPrepLevels + 2));
+  L->prep_smem = (size_t)4 * (8 * L->st_pad + 128 * (kPrepSub + 2));
   L->exact_smem = sizeof(BandItem) * kChainSlots * kSlotItems + sizeof(int2) * (size_t)L->lv_pad +
                   sizeof(ProbState) * 2 * (size_t)L->st_pad;
   L->chain_smem = sizeof(BandFactor) * kChainSlots * kFacSlot;
   if (L->max_states > kBandMaxStates) {
     L->ok = false;
-    L->why = "a graph has more than 512 states";
-  } else if (a->num_classes % 4 != 0 || (reinterpret_cast<uintptr_t>(a->log_probs) & 15) != 0) {
-    L->ok = false;
-    L->why = "rows of the log-prob matrix are not 16-byte aligned";
+    L->why = "a graph has more than 1024 states";
   } else if (L->chain_smem > kBandSmemBudget || L->exact_smem > kBandSmemBudget) {
     L->ok = false;
     L->why = "too many frames, states or classes for the shared memory of the recursions";
@@ -1488,7 +1723,8 @@ static int32_t MakeBandLayout(const k2b200_band_loss_args *a, BandLayout *L) {
   L->off_items = take(sizeof(BandItem) * (size_t)grid);
   L->off_lists = take(sizeof(int2) * (size_t)levels);
   L->off_chunk_r = take(sizeof(int32_t) * (size_t)levels);
-  L->off_keep = take(sizeof(uint16_t) * 32 * (size_t)levels);
+  L->keep_row = L->max_states > 512 ? 128 : 64;
+  L->off_keep = take((size_t)L->keep_row * (size_t)levels);
   L->off_factors = take(sizeof(BandFactor) * (size_t)grid);
   L->off_cutoffs = take(sizeof(float) * a->num_fsas);
   L->off_am = take(sizeof(double) * (size_t)grid);
@@ -1499,7 +1735,7 @@ static int32_t MakeBandLayout(const k2b200_band_loss_args *a, BandLayout *L) {
   L->off_b_scale = take(sizeof(int32_t) * (size_t)levels);
   L->off_total = take(sizeof(BandTotal) * a->num_fsas);
   L->off_unfit = take(sizeof(int32_t) * a->num_fsas);
-  L->off_totals = take(64);  // five 64-bit totals, then the status word
+  L->off_totals = take(64);  // five 64-bit totals, the status word, the ticket (at 48)
   L->off_status = L->off_totals + 5 * sizeof(long long);
   L->total_bytes = off;
   return kOk;
@@ -1526,7 +1762,7 @@ static bool BandReduceBeam(const k2b200_band_loss_args *a, const long long *h_to
 }
 
 static int32_t LaunchBandChains(const BandLayout &L, const k2b200_band_loss_args *args, char *ws,
-                                double *tot_scores, cudaStream_t stream) {
+                                double *tot_scores, const LossSpec &spec, cudaStream_t stream) {
   K2B_CUDA_OK(cudaFuncSetAttribute(BandChainLists, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)L.chain_smem));
   K2B_CUDA_OK(cudaFuncSetAttribute(BandChainExact, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1549,7 +1785,8 @@ static int32_t LaunchBandChains(const BandLayout &L, const k2b200_band_loss_args
       infos, reinterpret_cast<const BandArc *>(args->band_arcs), args->log_probs,
       args->num_classes, items, lists, am, reinterpret_cast<int32_t *>(ws + L.off_ae), bm,
       reinterpret_cast<int32_t *>(ws + L.off_be), tot_scores, total, unfit, status, L.st_pad,
-      L.lv_pad, CopyWaitLimit()); NoteLaunch(); }
+      L.lv_pad, CopyWaitLimit(), spec, reinterpret_cast<uint32_t *>(ws + L.off_totals + 48));
+    NoteLaunch(); }
   K2B_CUDA_OK(cudaGetLastError());
   return kOk;
 }
@@ -1604,9 +1841,28 @@ int32_t k2b200_band_loss_workspace_bytes(const k2b200_band_loss_args *args, size
   return kOk;
 }
 
+int32_t k2b200_band_loss_plan(const k2b200_band_loss_args *args, int32_t *supported,
+                              int32_t *exclusive_rows, size_t *bytes) {
+  K2B_REQUIRE(supported && exclusive_rows && bytes, "NULL output pointer");
+  BandLayout L;
+  K2B_FORWARD(MakeBandLayout(args, &L));
+  *supported = L.ok ? 1 : 0;
+  *exclusive_rows = L.exclusive_rows ? 1 : 0;
+  *bytes = L.total_bytes;
+  if (!L.ok) SetError("band loss path not applicable: %s", L.why);
+  return kOk;
+}
+
 int32_t k2b200_band_loss_forward(const k2b200_band_loss_args *args, void *workspace,
                                  size_t workspace_bytes, void *stream_v, double *tot_scores,
                                  float *beam_used) {
+  return k2b200_band_loss_forward_reduce(args, workspace, workspace_bytes, stream_v, tot_scores,
+                                         beam_used, nullptr);
+}
+
+int32_t k2b200_band_loss_forward_reduce(const k2b200_band_loss_args *args, void *workspace,
+                                        size_t workspace_bytes, void *stream_v, double *tot_scores,
+                                        float *beam_used, const k2b200_band_reduce *reduce) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
   BandLayout L;
   K2B_FORWARD(MakeBandLayout(args, &L));
@@ -1621,12 +1877,34 @@ int32_t k2b200_band_loss_forward(const k2b200_band_loss_args *args, void *worksp
               "NULL device pointer");
   char *ws = reinterpret_cast<char *>(workspace);
   static_assert(sizeof(BandInfo) % sizeof(int32_t) == 0, "BandInfo is uploaded as int32 words");
-  K2B_FORWARD(UploadInts(reinterpret_cast<const int32_t *>(L.infos.data()),
-                         (int64_t)L.infos.size() * (sizeof(BandInfo) / sizeof(int32_t)),
-                         reinterpret_cast<int32_t *>(ws + L.off_infos), stream));
-  // unfit words, totals and the status word lie one after the other: one clear for the first
-  // pass (a repeated pass clears the first two again, not the status of the Viterbi kernels)
-  K2B_CUDA_OK(cudaMemsetAsync(ws + L.off_unfit, 0, L.off_totals + 64 - L.off_unfit, stream));
+  LossSpec spec = {0, 0, nullptr, nullptr};
+  const float *logits = nullptr;
+  if (reduce != nullptr) {
+    K2B_REQUIRE(reduce->mode >= 0 && reduce->mode <= 2, "bad reduction mode %d", reduce->mode);
+    K2B_REQUIRE(reduce->mode == 0 || reduce->loss != nullptr, "NULL loss pointer");
+    K2B_REQUIRE(reduce->mode != 2 || (reduce->lens != nullptr && reduce->lens_type >= 1 &&
+                                      reduce->lens_type <= 4),
+                "the mean needs lengths");
+    spec.mode = reduce->mode;
+    spec.lens = reduce->lens;
+    spec.lens_type = reduce->lens_type;
+    spec.loss = reduce->loss;
+    logits = reduce->logits;
+  }
+  // unfit words, totals, the status word and the ticket lie one after the other: one clear for
+  // the first pass (a repeated pass clears them again but for the status of the Viterbi kernels)
+  K2B_FORWARD(UploadIntsAndClear(reinterpret_cast<const int32_t *>(L.infos.data()),
+                                 (int64_t)L.infos.size() * (sizeof(BandInfo) / sizeof(int32_t)),
+                                 reinterpret_cast<int32_t *>(ws + L.off_infos),
+                                 reinterpret_cast<int32_t *>(ws + L.off_unfit),
+                                 (int64_t)(L.off_totals + 64 - L.off_unfit) / 4, stream));
+  if (logits != nullptr && L.max_frames > 0) {
+    PhaseTimer timer(kPhaseDense, stream);
+    dim3 grid(CeilDiv(L.max_frames, 8), args->num_fsas);
+    { LogSoftmaxRows<<<grid, 256, 0, stream>>>(
+        reinterpret_cast<const BandInfo *>(ws + L.off_infos), logits, args->num_classes,
+        const_cast<float *>(args->log_probs)); NoteLaunch(); }
+  }
   {
     PhaseTimer timer(kPhaseViterbi, stream);
     NotePhaseKernel(kPhaseViterbi, "BandViterbi");
@@ -1637,7 +1915,8 @@ int32_t k2b200_band_loss_forward(const k2b200_band_loss_args *args, void *worksp
         reinterpret_cast<const BandInfo *>(ws + L.off_infos),
         reinterpret_cast<const BandState *>(args->band_states), args->log_probs,
         args->num_classes, reinterpret_cast<float *>(ws + L.off_vf),
-        reinterpret_cast<float *>(ws + L.off_vb), L.vit_frames, L.vit_batches, L.xch_pad,
+        reinterpret_cast<float *>(ws + L.off_vb), L.vit_frames, L.vit_batches, L.vit_slot,
+        L.xch_pad,
         CopyWaitLimit(), reinterpret_cast<int32_t *>(ws + L.off_status)); NoteLaunch(); }
     K2B_CUDA_OK(cudaGetLastError());
   }
@@ -1658,6 +1937,7 @@ int32_t k2b200_band_loss_forward(const k2b200_band_loss_args *args, void *worksp
     SideReadBackScope readback;
     if (iter > 0) {
       K2B_CUDA_OK(cudaMemsetAsync(ws + L.off_totals, 0, 5 * sizeof(long long), stream));
+      K2B_CUDA_OK(cudaMemsetAsync(ws + L.off_totals + 48, 0, sizeof(uint32_t), stream));
       K2B_CUDA_OK(cudaMemsetAsync(ws + L.off_unfit, 0, sizeof(int32_t) * args->num_fsas, stream));
     }
     cudaStream_t side = nullptr;
@@ -1670,11 +1950,13 @@ int32_t k2b200_band_loss_forward(const k2b200_band_loss_args *args, void *worksp
           reinterpret_cast<const BandInfo *>(ws + L.off_infos), args->a_row_splits2,            \
           reinterpret_cast<const float *>(ws + L.off_vf),                                       \
           reinterpret_cast<const float *>(ws + L.off_vb), beam,                                 \
-          reinterpret_cast<uint16_t *>(ws + L.off_keep),                                        \
+          reinterpret_cast<unsigned char *>(ws + L.off_keep),                                   \
           reinterpret_cast<float *>(ws + L.off_cutoffs),                                        \
           reinterpret_cast<unsigned long long *>(ws + L.off_totals),                            \
           L.arc_frames > args->max_arcs ? 1 : 0); NoteLaunch(); }
-      if (L.max_states <= 256) K2B_BAND_KEEP(8) else K2B_BAND_KEEP(kPrepK)
+      if (L.max_states <= 256) K2B_BAND_KEEP(8)
+      else if (L.max_states <= 512) K2B_BAND_KEEP(16)
+      else K2B_BAND_KEEP(32)
 #undef K2B_BAND_KEEP
       // the host reads the counts behind BandKeep, while what follows runs
       if (need_count) {
@@ -1682,11 +1964,12 @@ int32_t k2b200_band_loss_forward(const k2b200_band_loss_args *args, void *worksp
         K2B_FORWARD(readback.Begin(ws + L.off_totals, sizeof(long long) * 6));
       }
       dim3 grid(CeilDiv(L.max_frames + 2, 4 * kPrepSub), args->num_fsas);
-      { BandPrep<<<grid, 128, L.prep_smem, stream>>>(
+      auto prep = L.max_states <= 512 ? BandPrep<16> : BandPrep<32>;
+      { prep<<<grid, 128, L.prep_smem, stream>>>(
           reinterpret_cast<const BandInfo *>(ws + L.off_infos),
           reinterpret_cast<const BandState *>(args->band_states),
           reinterpret_cast<const BandArc *>(args->band_arcs),
-          reinterpret_cast<const uint16_t *>(ws + L.off_keep), args->log_probs,
+          reinterpret_cast<const unsigned char *>(ws + L.off_keep), args->log_probs,
           args->num_classes, reinterpret_cast<const float *>(ws + L.off_vf),
           reinterpret_cast<const float *>(ws + L.off_vb),
           reinterpret_cast<const float *>(ws + L.off_cutoffs),
@@ -1707,7 +1990,7 @@ int32_t k2b200_band_loss_forward(const k2b200_band_loss_args *args, void *worksp
     {
       PhaseTimer timer(kPhaseChain, stream);
       NotePhaseKernel(kPhaseChain, "BandChainLists");
-      K2B_FORWARD(LaunchBandChains(L, args, ws, tot_scores, stream));
+      K2B_FORWARD(LaunchBandChains(L, args, ws, tot_scores, spec, stream));
     }
     if (!need_count) break;
     long long h_totals[6];
@@ -1722,6 +2005,38 @@ int32_t k2b200_band_loss_forward(const k2b200_band_loss_args *args, void *worksp
     K2B_REQUIRE(iter < 200, "output beam reduction did not converge");
   }
   if (beam_used) *beam_used = beam;
+  return kOk;
+}
+
+static int32_t BandArcsOrScatter(const BandLayout &L, const k2b200_band_loss_args *args, char *ws,
+                                 const GradSpec &upstream, float *grad_a, float *grad_b,
+                                 const int32_t *grad_row0, int32_t grad_pitch,
+                                 int32_t grad_col_off, cudaStream_t stream) {
+  dim3 grid(CeilDiv(L.max_frames + 1, 4 * kGradLevels), args->num_fsas);
+  const size_t sums_bytes =
+      grad_b == nullptr
+          ? 0
+          : (sizeof(uint32_t) * 4 * (size_t)(args->num_classes + grad_col_off) + 15) & ~(size_t)15;
+  const size_t smem = sums_bytes + (grad_a ? sizeof(ProbState) * 4 * (size_t)L.st_pad : 0);
+  K2B_REQUIRE(smem <= kBandSmemBudget, "too many classes for the gradient kernel");
+  auto kernel = grad_a != nullptr ? BandGrad<true> : BandGrad<false>;
+  K2B_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)kBandSmemBudget));
+  { kernel<<<grid, 128, smem, stream>>>(
+      reinterpret_cast<const BandInfo *>(ws + L.off_infos),
+      reinterpret_cast<const BandArc *>(args->band_arcs), args->log_probs,
+      reinterpret_cast<const BandItem *>(ws + L.off_items),
+      reinterpret_cast<const int2 *>(ws + L.off_lists),
+      reinterpret_cast<const double *>(ws + L.off_am),
+      reinterpret_cast<const int32_t *>(ws + L.off_ae),
+      reinterpret_cast<const double *>(ws + L.off_bm),
+      reinterpret_cast<const int32_t *>(ws + L.off_be),
+      reinterpret_cast<const int32_t *>(ws + L.off_a_scale),
+      reinterpret_cast<const int32_t *>(ws + L.off_b_scale),
+      reinterpret_cast<const BandTotal *>(ws + L.off_total),
+      reinterpret_cast<const int32_t *>(ws + L.off_unfit), upstream, grad_a, grad_b, grad_row0,
+      grad_pitch, grad_col_off, args->num_classes, L.st_pad); NoteLaunch(); }
+  K2B_CUDA_OK(cudaGetLastError());
   return kOk;
 }
 
@@ -1741,41 +2056,64 @@ int32_t k2b200_band_loss_backward(const k2b200_band_loss_args *args, void *works
   }
   K2B_REQUIRE(tot_grad && grad_b, "NULL device pointer");
   K2B_REQUIRE(grad_col_off == 0 || grad_col_off == 1, "grad_col_off must be 0 or 1");
-  char *ws = reinterpret_cast<char *>(workspace);
   PhaseTimer timer(kPhaseGrad, stream);
   NotePhaseKernel(kPhaseGrad, "BandGrad");
-  dim3 grid(CeilDiv(L.max_frames + 1, 4 * kGradLevels), args->num_fsas);
-#define K2B_BAND_GRAD(ARCS, SMEM)                                                             \
-  { BandGrad<ARCS><<<grid, 128, SMEM, stream>>>(                                              \
-      reinterpret_cast<const BandInfo *>(ws + L.off_infos),                                   \
-      reinterpret_cast<const BandArc *>(args->band_arcs), args->log_probs,                    \
-      reinterpret_cast<const BandItem *>(ws + L.off_items),                                   \
-      reinterpret_cast<const int2 *>(ws + L.off_lists),                                       \
-      reinterpret_cast<const double *>(ws + L.off_am),                                        \
-      reinterpret_cast<const int32_t *>(ws + L.off_ae),                                       \
-      reinterpret_cast<const double *>(ws + L.off_bm),                                        \
-      reinterpret_cast<const int32_t *>(ws + L.off_be),                                       \
-      reinterpret_cast<const int32_t *>(ws + L.off_a_scale),                                  \
-      reinterpret_cast<const int32_t *>(ws + L.off_b_scale),                                  \
-      reinterpret_cast<const BandTotal *>(ws + L.off_total),                                  \
-      reinterpret_cast<const int32_t *>(ws + L.off_unfit), tot_grad, tot_grad_stride, grad_a, \
-      grad_b, grad_row0, grad_pitch, grad_col_off, args->num_classes, L.st_pad); NoteLaunch(); }
-  const size_t sums_bytes =
-      (sizeof(uint32_t) * 4 * (size_t)(args->num_classes + grad_col_off) + 15) & ~(size_t)15;
-  K2B_REQUIRE(sums_bytes + sizeof(ProbState) * 4 * (size_t)L.st_pad <= kBandSmemBudget,
-              "too many classes for the gradient kernel");
-  if (grad_a != nullptr) {
-    const size_t smem = sums_bytes + sizeof(ProbState) * 4 * (size_t)L.st_pad;
-    K2B_CUDA_OK(cudaFuncSetAttribute(BandGrad<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)smem));
-    K2B_BAND_GRAD(true, smem)
-  } else {
-    K2B_CUDA_OK(cudaFuncSetAttribute(BandGrad<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)sums_bytes));
-    K2B_BAND_GRAD(false, sums_bytes)
+  const GradSpec upstream = {tot_grad, 1, tot_grad_stride, 0, 0, nullptr, args->num_fsas};
+  return BandArcsOrScatter(L, args, reinterpret_cast<char *>(workspace), upstream, grad_a, grad_b,
+                           grad_row0, grad_pitch, grad_col_off, stream);
+}
+
+int32_t k2b200_band_loss_backward_dense(const k2b200_band_loss_args *args, void *workspace,
+                                        size_t workspace_bytes,
+                                        const k2b200_band_upstream *upstream, float *grad_a,
+                                        float *grad_log_probs, int32_t softmax, void *stream_v) {
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
+  BandLayout L;
+  K2B_FORWARD(MakeBandLayout(args, &L));
+  K2B_REQUIRE(L.ok, "band loss path not applicable: %s", L.why);
+  K2B_REQUIRE(L.exclusive_rows, "sequences share rows of the log-probs");
+  if (workspace == nullptr || workspace_bytes < L.total_bytes) {
+    SetError("workspace of %zu bytes is smaller than the %zu required", workspace_bytes,
+             L.total_bytes);
+    return kWorkspaceTooSmall;
   }
-#undef K2B_BAND_GRAD
-  K2B_CUDA_OK(cudaGetLastError());
+  K2B_REQUIRE(upstream && upstream->grad, "NULL upstream gradient");
+  char *ws = reinterpret_cast<char *>(workspace);
+  PhaseTimer timer(kPhaseGrad, stream);
+  NotePhaseKernel(kPhaseGrad, "BandGradRows");
+  const GradSpec spec = {upstream->grad,      upstream->is_double, upstream->stride,
+                         upstream->negate,    upstream->lens_type, upstream->lens,
+                         args->num_fsas};
+  if (grad_log_probs != nullptr) {
+    const int32_t C = args->num_classes, C_pad = (C + 3) & ~3;
+    if (L.first_row > 0)  // rows before the first sequence
+      K2B_CUDA_OK(cudaMemsetAsync(grad_log_probs, 0, sizeof(float) * (size_t)L.first_row * C, stream));
+    const size_t row_bytes = sizeof(uint32_t) * (size_t)C_pad;
+    K2B_REQUIRE(row_bytes <= kBandSmemBudget, "too many classes for the gradient kernel");
+    // a row of sums per warp in shared memory: fewer warps per CTA when rows are long, so
+    // that a CTA does not hold the SM's memory for one slow warp
+    const int32_t warps = row_bytes * 4 <= 16 * 1024 ? 4 : row_bytes <= 8 * 1024 ? 2 : 1;
+    auto kernel = softmax ? BandGradRows<true> : BandGradRows<false>;
+    K2B_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)kBandSmemBudget));
+    dim3 grid(CeilDiv(std::max(L.max_rows, 1), warps * kDenseRows), args->num_fsas);
+    { kernel<<<grid, 32 * warps, row_bytes * warps, stream>>>(
+        reinterpret_cast<const BandInfo *>(ws + L.off_infos), args->log_probs,
+        reinterpret_cast<const BandItem *>(ws + L.off_items),
+        reinterpret_cast<const int2 *>(ws + L.off_lists),
+        reinterpret_cast<const double *>(ws + L.off_am),
+        reinterpret_cast<const int32_t *>(ws + L.off_ae),
+        reinterpret_cast<const double *>(ws + L.off_bm),
+        reinterpret_cast<const int32_t *>(ws + L.off_be),
+        reinterpret_cast<const int32_t *>(ws + L.off_a_scale),
+        reinterpret_cast<const int32_t *>(ws + L.off_b_scale),
+        reinterpret_cast<const BandTotal *>(ws + L.off_total),
+        reinterpret_cast<const int32_t *>(ws + L.off_unfit), spec, grad_log_probs, C, C_pad);
+      NoteLaunch(); }
+    K2B_CUDA_OK(cudaGetLastError());
+  }
+  if (grad_a != nullptr)
+    K2B_FORWARD(BandArcsOrScatter(L, args, ws, spec, grad_a, nullptr, nullptr, 0, 0, stream));
   return kOk;
 }
 

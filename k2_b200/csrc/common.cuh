@@ -131,8 +131,17 @@ int32_t RowSplitsToRowIds(const int32_t *row_splits, int32_t num_rows,
                           int32_t *row_ids, int32_t num_elems,
                           cudaStream_t stream);
 
+// Host integers as a kernel parameter (at most 32764 bytes of them).
+template <int kInts>
+struct IntChunk {
+  int32_t v[kInts];
+};
+
 // n host integers -> device memory as kernel parameters (no copy engine, no sync).
 int32_t UploadInts(const int32_t *host, int64_t n, int32_t *device_out, cudaStream_t stream);
+// The same; the first launch also clears `clear_words` words at `clear`.
+int32_t UploadIntsAndClear(const int32_t *host, int64_t n, int32_t *device_out, int32_t *clear,
+                           int64_t clear_words, cudaStream_t stream);
 
 // Incoming-arc index of an FsaVec: for every state (idx01) the arcs (idx012) that
 // enter it, in increasing arc order.

@@ -4,6 +4,7 @@
 // (k2/csrc/utils_inl.h:40-90 ExclusiveSum, k2/csrc/utils.cu:75-200
 // RowSplitsToRowIds, k2/csrc/fsa_utils.cu:901-928 GetIncomingArcs).
 #include <nvtx3/nvToolsExt.h>
+#include <algorithm>
 #include <atomic>
 #include <cstring>
 #include <cstdlib>
@@ -241,23 +242,45 @@ SideReadBackScope::~SideReadBackScope() {
 // in torch, and one from pinned memory queues behind whatever large transfer the
 // application has in flight; a launch does neither.
 // ----------------------------------------------------------------------------
-struct IntChunk {
-  int32_t v[960];  // kernel parameters are limited to 4 KB
-};
-__global__ void StoreInts(IntChunk c, int32_t n, int32_t *__restrict__ out) {
+// A launch carries up to 8000 of them (kernel parameters may be 32764 bytes): a batch of long
+// transcripts took a dozen launches of 960.  The whole parameter block is copied at every
+// launch, so short uploads use a short one.
+template <int kInts>
+__global__ void StoreInts(const __grid_constant__ IntChunk<kInts> c, int32_t n,
+                          int32_t *__restrict__ out, int32_t *__restrict__ clear,
+                          int64_t clear_words) {
   const int32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < n) out[k] = c.v[k];
+  for (int64_t j = k; j < clear_words; j += (int64_t)gridDim.x * blockDim.x) clear[j] = 0;
 }
 
-int32_t UploadInts(const int32_t *host, int64_t n, int32_t *device_out, cudaStream_t stream) {
-  IntChunk c;
-  for (int64_t done = 0; done < n; done += 960) {
-    const int32_t m = (int32_t)std::min<int64_t>(960, n - done);
-    memcpy(c.v, host + done, sizeof(int32_t) * m);
-    { StoreInts<<<CeilDiv(m, 256), 256, 0, stream>>>(c, m, device_out + done); NoteLaunch(); }
+template <int kInts>
+static void LaunchStoreInts(const int32_t *host, int32_t n, int32_t *out, int32_t *clear,
+                            int64_t clear_words, cudaStream_t stream) {
+  IntChunk<kInts> c;
+  memcpy(c.v, host, sizeof(int32_t) * n);
+  const int32_t blocks =
+      std::max(1, std::max(CeilDiv(n, 256), (int32_t)std::min<int64_t>(64, CeilDiv(clear_words, 1024))));
+  { StoreInts<kInts><<<blocks, 256, 0, stream>>>(c, n, out, clear, clear_words); NoteLaunch(); }
+}
+
+int32_t UploadIntsAndClear(const int32_t *host, int64_t n, int32_t *device_out, int32_t *clear,
+                           int64_t clear_words, cudaStream_t stream) {
+  constexpr int kShort = 960, kLong = 8000;
+  for (int64_t done = 0; done < n || clear_words > 0;) {
+    const int32_t m = (int32_t)std::min<int64_t>(n - done > kShort ? kLong : kShort, n - done);
+    if (m <= kShort)
+      LaunchStoreInts<kShort>(host + done, m, device_out + done, clear, clear_words, stream);
+    else
+      LaunchStoreInts<kLong>(host + done, m, device_out + done, clear, clear_words, stream);
+    done += m;
+    clear_words = 0;
   }
   K2B_CUDA_OK(cudaGetLastError());
   return kOk;
+}
+int32_t UploadInts(const int32_t *host, int64_t n, int32_t *device_out, cudaStream_t stream) {
+  return UploadIntsAndClear(host, n, device_out, nullptr, 0, stream);
 }
 
 // ----------------------------------------------------------------------------

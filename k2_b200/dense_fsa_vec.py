@@ -95,6 +95,27 @@ class DenseFsaVec(object):
         assert allow_truncate >= 0
 
         N, T, C = log_probs.shape
+        if log_probs.is_cuda:
+            # the layout alone: the score matrix, and the device copy of the row splits, are
+            # made on first use (a loss that reads the log-probs directly,
+            # k2b200_band_loss_*, needs neither).  Two segments that touch the same frame
+            # make the backward of the matrix use atomic adds.
+            row_splits, first, eff, overlapping = _lib._host.dense_layout(
+                supervision_segments, N, T, allow_truncate)
+            fn = _LogSoftmaxDenseFunction if _logits else _DenseFsaVecFunction
+            self._init(None, row_splits, device=log_probs.device, num_cols=C + 1)
+            # (no closure over self: a reference cycle would keep the log-probs and
+            # their gradient alive until the cycle collector runs)
+            self._make_scores = (fn, log_probs, eff, int(row_splits[-1]), overlapping)
+            if not overlapping and N * T < 2**31:
+                # what a loss needs to read `log_probs` in place and to send its gradient
+                # straight to it (k2b200_band_loss_*, k2b200_dense_loss_backward_log_probs):
+                # the tensor and, per sequence, the row of its first frame
+                if _logits:
+                    self._logit_source = (log_probs, first)
+                else:
+                    self._source = (log_probs, first)
+            return
         seg = supervision_segments.numpy()  # int32 [num_segs, 3]: sequence, start, duration
         num_segs = seg.shape[0]
         seq, start = seg[:, 0], seg[:, 1]
@@ -116,49 +137,21 @@ class DenseFsaVec(object):
         rows = int(row_splits[-1])
         device = log_probs.device
 
-        if log_probs.is_cuda:
-            # one kernel writes the whole matrix; two segments that touch the same
-            # frame make the backward use atomic adds
-            first = seq * np.int32(T) + start if N * T < 2**31 else seq.astype(np.int64) * T + start
-            if num_segs == 0 or np.bincount(seq, minlength=N).max() <= 1:
-                overlapping = False  # at most one segment per sequence
-            else:
-                order = np.argsort(first, kind="stable")
-                overlapping = bool(np.any((first + dur)[order][:-1] > first[order][1:]))
-            # (a copy: the caller's tensor may change before the scores are made)
-            eff = seg.copy() if not truncated else \
-                np.stack([seq, start, dur], axis=1).astype(np.int32)
-            fn = _LogSoftmaxDenseFunction if _logits else _DenseFsaVecFunction
-            # The score matrix, and the device copy of the row splits, are made on first
-            # use: a loss that reads the log-probs directly (k2b200_band_loss_*) needs
-            # neither.
-            self._init(None, row_splits, device=device, num_cols=C + 1)
-            # (no closure over self: a reference cycle would keep the log-probs and
-            # their gradient alive until the cycle collector runs)
-            self._make_scores = (fn, log_probs, eff, rows, overlapping)
-            if not _logits and not overlapping:
-                # what a loss needs to read `log_probs` in place and to send its
-                # gradient straight to it (k2b200_band_loss_*,
-                # k2b200_dense_loss_backward_log_probs): the tensor and, per
-                # sequence, the row of its first frame
-                self._source = (log_probs, first.astype(np.int32, copy=False))
-            return
-        else:
-            if _logits:
-                log_probs = torch.log_softmax(log_probs, dim=-1)
-            # host tensors (layout checks, graph preparation): the reference's own
-            # formulation with torch ops
-            last_frame_indexes = (row_splits[1:] - 1).astype(np.int64)
-            index = np.zeros(rows, dtype=np.int64)
-            for k in range(seg.shape[0]):
-                r0 = int(row_splits[k])
-                index[r0:r0 + int(dur[k])] = np.arange(int(seg[k, 1]), int(seg[k, 1]) + int(dur[k])) + \
-                    int(seg[k, 0]) * T
-            scores = torch.empty(rows, C + 1, dtype=log_probs.dtype, device=device)
-            scores[:, 1:] = log_probs.reshape(-1, C).index_select(0, torch.from_numpy(index))
-            scores[:, 0] = float('-inf')
-            scores[torch.from_numpy(last_frame_indexes)] = torch.tensor(
-                [0] + [float('-inf')] * C, dtype=log_probs.dtype)
+        if _logits:
+            log_probs = torch.log_softmax(log_probs, dim=-1)
+        # host tensors (layout checks, graph preparation): the reference's own
+        # formulation with torch ops
+        last_frame_indexes = (row_splits[1:] - 1).astype(np.int64)
+        index = np.zeros(rows, dtype=np.int64)
+        for k in range(seg.shape[0]):
+            r0 = int(row_splits[k])
+            index[r0:r0 + int(dur[k])] = np.arange(int(seg[k, 1]), int(seg[k, 1]) + int(dur[k])) + \
+                int(seg[k, 0]) * T
+        scores = torch.empty(rows, C + 1, dtype=log_probs.dtype, device=device)
+        scores[:, 1:] = log_probs.reshape(-1, C).index_select(0, torch.from_numpy(index))
+        scores[:, 0] = float('-inf')
+        scores[torch.from_numpy(last_frame_indexes)] = torch.tensor(
+            [0] + [float('-inf')] * C, dtype=log_probs.dtype)
         self._init(scores, row_splits)
 
     @classmethod
@@ -174,6 +167,7 @@ class DenseFsaVec(object):
               d_row_splits: torch.Tensor = None, device=None, num_cols: int = 0) -> None:
         assert scores is None or scores.is_contiguous()
         self._source = None
+        self._logit_source = None  # the same for logits, which are not normalised yet
         self._source_rows = {}
         self._make_scores = None
         self._scores = scores  # for back propagation
@@ -210,6 +204,7 @@ class DenseFsaVec(object):
         self._scores = value
         self._make_scores = None
         self._source = None  # no longer the layout of the tensor it was made from
+        self._logit_source = None
         self._source_rows = {}
         self._band_args = None
 

@@ -77,6 +77,17 @@ class Fsa(object):
         if _check and properties is None:
             _ = self.properties  # validity check, as the reference does eagerly
 
+    @classmethod
+    def _of_ctc_graph(cls, arcs: RaggedArc, scores: torch.Tensor, labels: torch.Tensor,
+                      aux_labels: torch.Tensor) -> 'Fsa':
+        """An FsaVec whose attribute tensors exist already (_host.ctc_graph)."""
+        ans = cls.__new__(cls)
+        d = ans.__dict__
+        d['arcs'], d['_properties'] = arcs, None
+        d['_tensor_attr'] = {'scores': scores, 'labels': labels, 'aux_labels': aux_labels}
+        d['_non_tensor_attr'], d['_cache'] = {}, {}
+        return ans
+
     # ------------------------------------------------------------------ attributes
     def __setattr__(self, name: str, value: Any) -> None:
         assert name not in ('_tensor_attr', '_non_tensor_attr', 'arcs', '_cache', '_properties',

@@ -42,6 +42,16 @@ def ctc_graph(symbols: List[List[int]], modified: bool = False,
     same and `modified` is False - an arc that skips the blank.  `aux_labels`
     holds the symbol on the arcs that enter a symbol state (fsa_algo.cu:672-727).
     """
+    dev = torch.device(device)
+    if dev.type == "cuda":
+        parts = _lib._host.ctc_graph(
+            symbols, bool(modified),
+            torch.cuda.current_device() if dev.index is None else dev.index)
+        if parts is not None:
+            values, rs1, rs2, aux, scores, labels, h_rs1, h_arc_splits, band = parts
+            return Fsa._of_ctc_graph(
+                RaggedArc._of_ctc_graph(values, rs1, rs2, h_rs1, h_arc_splits, band), scores,
+                labels, aux)
     n = len(symbols)
     lens = np.fromiter(map(len, symbols), dtype=np.int64, count=n)
     tot = int(lens.sum())

@@ -44,6 +44,26 @@ class RaggedArc:
         # whose arcs all go from one layer to the next, with bounds on layer sizes
         self._layer_bounds = (0, 0, 0, 0)
 
+    @classmethod
+    def _of_ctc_graph(cls, values, row_splits1, row_splits2, h_row_splits1, h_arc_splits,
+                      band_graph) -> "RaggedArc":
+        """The parts that _host.ctc_graph returns, taken as they are (this runs once per
+        training step on the thread that feeds the GPU)."""
+        ans = cls.__new__(cls)
+        ans._values, ans._row_splits1, ans._row_splits2 = values, row_splits1, row_splits2
+        ans._row_ids1 = ans._row_ids2 = None
+        ans.single = False
+        ans._h_row_splits1, ans._h_arc_splits = h_row_splits1, h_arc_splits
+        ans._incoming = ans._incoming_key = ans._levels = None
+        ans._layer_bounds = (0, 0, 0, 0)
+        # CTC graphs are band graphs for as long as nobody edits them, and no state has more
+        # than three arcs on either side
+        key = (values.data_ptr(), values._version)
+        ans._band_by_construction = key
+        ans._band_graph = (key, band_graph)
+        ans._max_degree = 3
+        return ans
+
     # ---- _k2.RaggedArc interface ----------------------------------------
     def values(self) -> torch.Tensor:
         return self._values
@@ -202,6 +222,24 @@ class RaggedArc:
             ok = (int(status.item()) & 1) == 0
         ans = (states, arcs, ok)
         self._band = (key, ans)
+        return ans
+
+    def band_graph(self):
+        """The tables of `band_tables` as the native loss takes them (_host.BandGraph), or
+        None when some graph is not a band graph.  Cached per version of the arc tensor."""
+        vals = self._values
+        key = (vals.data_ptr(), vals._version)
+        cached = getattr(self, "_band_graph", None)
+        if cached is not None and cached[0] == key:
+            return cached[1]
+        states, arcs, ok = self.band_tables()
+        ans = None
+        if ok:
+            ans = _lib._host.BandGraph(
+                self._row_splits2, states, arcs,
+                np.ascontiguousarray(self.h_row_splits1, dtype=np.int32),
+                np.ascontiguousarray(self.h_arc_splits, dtype=np.int32))
+        self._band_graph = (key, ans)
         return ans
 
     def replicated(self, min_bytes: int = 32 << 20) -> bool:
