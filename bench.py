@@ -338,12 +338,11 @@ def implementation_bytes(phase, kernel, frames, N, T, C, A, A_out, S_out, grid_s
     table = {
         # every row by both directions, both grids written
         "BandViterbi": 2 * 4 * R * C + 8 * grid_states,
-        # BandKeep reads both grids and writes 64 bytes of keep bits per level; BandPrep reads
-        # them back, per surviving state two table entries and five grid values, and writes a
-        # list entry (8 bytes) and a factor record (32 bytes) per entry of the padded lists
-        # (at least 32 entries per level)
-        "BandKeep+BandPrep": 8 * grid_states + 128 * (R + 2 * N) + 84 * S_out +
-                             40 * max(S_out, 32 * (R + 2 * N)),
+        # BandPrep reads both grids (the level on either side of a chunk of 16 twice), per
+        # surviving state two table entries and five grid values, and writes a list entry
+        # (8 bytes) and a factor record (32 bytes) per entry of the padded lists (at least 32
+        # entries per level)
+        "BandPrep": 9 * grid_states + 36 * S_out + 40 * max(S_out, 32 * (R + 2 * N)),
         # both directions read the factor records and write a value per padded entry
         "BandChainLists": 2 * 40 * max(S_out, 32 * (R + 2 * N)),
         # list entry, alpha and beta per surviving state, a gradient element per (frame, label)
@@ -704,7 +703,7 @@ def run_ours(args):
 
 
 # ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch on ctc_large (profiles/)
-NCU_TRAFFIC = {"BandViterbi": 289.5e6, "BandKeep+BandPrep": 296.5e6, "BandChainLists": 101.4e6,
+NCU_TRAFFIC = {"BandViterbi": 289.5e6, "BandPrep": 263.7e6, "BandChainLists": 101.4e6,
                "BandGrad": 77.8e6}
 
 

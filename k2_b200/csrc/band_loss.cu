@@ -21,12 +21,12 @@
 //                 the COMPACT list of surviving states with, per state and entering arc, the
 //                 factor exp(arc score) * exp(dense score) if the arc survives and 0 otherwise,
 //                 and the list positions of the states the arcs come from and go to.
-//   BandChainLists  one warp per (graph, direction) walks the levels over the lists only: a lane
+//   BandChainLists  one CTA per (graph, direction) walks the levels over the lists only: a thread
 //                 holds the value of one surviving state, an entry names the list positions of
-//                 its neighbours on the previous level, whose values come by shuffles: three
-//                 multiply-adds per state and level, no exp or log, no test, no shared-memory
-//                 traffic for values.  The lists arrive by bulk copies.  Values of a level
-//                 share a power-of-two scale that follows the data.
+//                 its neighbours on the previous level, whose values are in shared memory:
+//                 three multiply-adds per state and level, no exp or log, no test.  The lists
+//                 arrive by bulk copies.  Values of a level share a power-of-two scale that
+//                 follows the data.
 //   BandChainExact  the same recursion with a (mantissa, exponent) pair per state, by state
 //                 number in shared memory, for the graphs whose scores leave what a double
 //                 with a per-level scale can hold or whose levels are wider than the registers
@@ -55,7 +55,6 @@ namespace k2b {
 constexpr int kBandMaxStates = 1024;
 constexpr int kVitK = 4;              // states per thread of BandViterbi
 constexpr int kPrepLevels = 16;       // levels per chunk: their lists share one padded size
-constexpr int kPrepSub = 8;           // levels per warp of BandPrep
 constexpr int kGradLevels = 4;        // levels per warp of BandGrad
 constexpr int kDrainPolls = 4000000;  // bounded wait for copies in flight when a kernel gives up
 
@@ -96,21 +95,18 @@ constexpr int kOutbByte = 7;
 // The lists of the kPrepLevels levels of a chunk are padded to the same multiple of 32 entries,
 // larger than the longest of them: a padding entry has pw = 0, src = 0 and dst = kNoDst, and
 // kNoDst (lane 31 of the last register) always names a padding entry of the next level.
+// A level of n entries is stored as n x 16 bytes {pw[0], pw[1]} followed by n x 16 bytes
+// {pw[2], src, dst} (byte d = of d, the fourth unused), so that the lanes of a warp read
+// consecutive 16 bytes of shared memory.
 struct __align__(16) BandFactor {
   double pw[3];
-  uint8_t src[4];  // [3] unused
-  uint8_t dst[4];  // [3] unused
+  uint32_t src, dst;
 };
 static_assert(sizeof(BandFactor) == 32, "BandFactor must be 32 bytes");
-constexpr int kDstByte = 28;
 constexpr uint32_t kNoDst = 255;
-constexpr int kMaxRegs = 4;     // values of a level that a lane of the register recursion holds
-constexpr int kMaxListed = 32 * kMaxRegs - 1;  // entries of a level that it handles (one lane is padding)
-// words of BandPrep's per-state scratch: bit 15 = the state survives, bits 0-8 = its
-// position in the level's list, bits 9-11 = entering-arc bits
-constexpr uint32_t kMetaKept = 0x8000u, kMetaPos = 0x1ffu;
-constexpr int kMetaInShift = 9;
-
+constexpr int kMaxRegs = 4;     // warps of the list recursion
+constexpr int kChainThreads = 32 * kMaxRegs;
+constexpr int kMaxListed = 32 * kMaxRegs - 1;  // entries of a level that it handles (one is padding)
 // alpha of the final state on the last level (= Z) of a graph, as m * 2^e
 struct __align__(16) BandTotal {
   double m;
@@ -462,293 +458,316 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
 }
 
 // ---------------------------------------------------------------------------
-// Which states survive (intersect_dense.cu:289-296): state s of level l is kept iff
-// vf[l][s] + vb[l][s] > cutoff.  grid = (level chunks, pairs), a warp per kKeepLevels levels;
-// lane j looks at states K j .. K j + K - 1 (K = 8, 16 or 32 for graphs of up to 256, 512 or
-// 1024 states: the smallest keeps the most lanes busy) and writes their keep bits: the bit of
-// state s is bit (s & 7) of byte s / 8 of the level's row of keep_bytes bytes (64, or 128
-// with more than 512 states).  totals[0] += surviving states, totals[2] += the arcs
-// leaving them: the sizes the beam reduction looks at (intersect_dense.cu:289-320), which
-// the host can read while the kernels behind this one run.
+// Keep tests and lists.  grid = (chunks of kPrepLevels levels, pairs), kPrepWarps warps per CTA,
+// which looks at the chunk's levels and the level on either side of them:
+//   1. a warp per level, four states per lane at a time: state s of level l survives iff
+//      vf[l][s] + vb[l][s] > cutoff (intersect_dense.cu:289-296).  Shared memory keeps, per
+//      four states, their keep bits and the number of surviving states before them (together:
+//      the list position of a state), and the surviving states in order;
+//   2. a warp per 32 entries of a level: the reference's arc tests (intersect_dense.cu:430-471)
+//      against the states of the level before and the dense score of the state's label give
+//      the entering-arc bits, the factors and where the sources are; also (bits only) for the
+//      level behind the chunk;
+//   3. likewise: where the destinations are; an arc leaving an entry is an entering arc of the
+//      next level seen from its source.
+// Per level the result is the compact list of surviving states: a BandItem (label, state,
+// bits) and a BandFactor per entry.  The passes are a few independent loads deep and all of a
+// CTA's levels are in flight together; what bounds them is the latency of those loads where
+// the batch is small and the traffic (the two grids once, 32 + 8 bytes per padded entry)
+// where it is large.  (A warp that went through eight levels one after the other, behind a
+// separate kernel for the keep bits, took 103 + 38 us at 64 x 1000 frames of up to 501 states;
+// this takes 80, 212 MB read and 52 MB written.)
+// totals[0] += surviving states, totals[2] += the arcs leaving them (the
+// sizes the beam reduction looks at, intersect_dense.cu:289-320).  unfit[i] is set when the
+// list recursion cannot take graph i: a score outside its arithmetic, or a level with
+// more than kMaxListed surviving states.
 // ---------------------------------------------------------------------------
-constexpr int kKeepLevels = 8;
+constexpr float kMinLeanDense = -60.0f;   // dense score of a surviving arc
+constexpr int32_t kMaxLeanArcExp = 60, kMinLeanArcExp = -90;  // binary exponent of exp(arc score)
+constexpr int kPrepWarps = 9;             // 18 levels: two each
+constexpr int kPrepSpan = kPrepLevels + 2;
 
-template <int K>
-__global__ void __launch_bounds__(128)
-BandKeep(const BandInfo *__restrict__ infos, const int32_t *__restrict__ a_row_splits2,
-         const float *__restrict__ vf, const float *__restrict__ vb, float beam,
-         unsigned char *__restrict__ keep_bits, float *__restrict__ cutoffs,
-         unsigned long long *__restrict__ totals, int32_t count_arcs) {
-  static_assert(K == 8 || K == 16 || K == 32, "keep bits are stored as bytes or words");
-  constexpr int kRowBytes = K == 32 ? 128 : 64;
+// states of a graph rounded up to whole groups of 128 (four per lane of a warp)
+__host__ __device__ static inline int32_t PrepPad(int32_t states) { return (states + 127) & ~127; }
+static size_t BandPrepSmem(int32_t max_states) {
+  return (size_t)kPrepSpan * (PrepPad(max_states) / 4 * 2 + PrepPad(max_states) * 3);
+}
+
+__global__ void __launch_bounds__(32 * kPrepWarps, 3)
+BandPrep(const BandInfo *__restrict__ infos, const int32_t *__restrict__ a_row_splits2,
+         const BandState *__restrict__ tab, const BandArc *__restrict__ tabf,
+         const float *__restrict__ lp, int32_t C, const float *__restrict__ vf,
+         const float *__restrict__ vb, float beam, BandItem *__restrict__ items,
+         BandFactor *__restrict__ factors, int2 *__restrict__ lists,
+         int32_t *__restrict__ chunk_r, unsigned long long *__restrict__ totals,
+         int32_t *__restrict__ unfit, int32_t count_arcs) {
   constexpr unsigned kAll = 0xffffffffu;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int32_t longest_sh, risky_sh;
+  __shared__ uint32_t counts_sh[2];
+  __shared__ int32_t n_sh[kPrepSpan];
   const int32_t i = blockIdx.y;
   const BandInfo f = infos[i];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int32_t S = f.num_states, T = f.frames, pitch = f.pitch;
-  if (S == 0) return;
-  const int32_t a = (blockIdx.x * 4 + warp) * kKeepLevels;
-  if (a > T + 1) return;
-  const int32_t b = min(a + kKeepLevels, T + 2);
+  const int32_t a = blockIdx.x * kPrepLevels;  // the chunk's levels: a .. b - 1
+  if (S == 0 || a > T + 1) return;
+  const int32_t b = min(a + kPrepLevels, T + 2);
+  const int32_t P = PrepPad(S);
+  // level l of the chunk is row l - a + 1
+  uint16_t *cells = reinterpret_cast<uint16_t *>(smem_raw);            // [span][P / 4]
+  uint16_t *list = cells + kPrepSpan * (P / 4);                        // [span][P]
+  unsigned char *inbs = reinterpret_cast<unsigned char *>(list + kPrepSpan * P);  // likewise
   const float *fg = vf + f.grid_off, *bg = vb + f.grid_off;
+  if (tid == 0) {
+    longest_sh = risky_sh = 0;
+    counts_sh[0] = counts_sh[1] = 0;
+  }
   float cutoff;
   {
     const float start = bg[0], end = fg[(int64_t)(T + 1) * pitch + (S - 1)];
     cutoff = __fsub_rn(start < end ? start : end, beam);
   }
-  if (a == 0 && lane == 0) cutoffs[i] = cutoff;
-  const int32_t s0 = lane * K;
-  uint32_t n_states = 0, n_cand = 0;
-#pragma unroll 4
-  for (int32_t l = a; l < b; ++l) {
-    uint32_t keep = 0;
+  __syncthreads();
+  // ---- 1. surviving states ----------------------------------------------------------------
+  uint32_t n_cand = 0;
+  for (int32_t row = warp; row < kPrepSpan; row += kPrepWarps) {
+    const int32_t l = a - 1 + row;
+    const bool there = l >= 0 && l <= b && l <= T + 1;
+    const float *fr = fg + (int64_t)l * pitch + 4 * lane, *br = bg + (int64_t)l * pitch + 4 * lane;
+    int32_t n = 0;
+    for (int32_t g0 = 0; g0 < P; g0 += 512) {  // up to four groups of 128 states
+      float4 x[4], y[4];
 #pragma unroll
-    for (int c = 0; c < K / 4; ++c) {
-      if (s0 + 4 * c >= S) continue;
-      const float4 F = *reinterpret_cast<const float4 *>(fg + (int64_t)l * pitch + s0 + 4 * c);
-      const float4 B = *reinterpret_cast<const float4 *>(bg + (int64_t)l * pitch + s0 + 4 * c);
-      if (__fadd_rn(F.x, B.x) > cutoff) keep |= 1u << (4 * c);
-      if (__fadd_rn(F.y, B.y) > cutoff) keep |= 2u << (4 * c);
-      if (__fadd_rn(F.z, B.z) > cutoff) keep |= 4u << (4 * c);
-      if (__fadd_rn(F.w, B.w) > cutoff) keep |= 8u << (4 * c);
+      for (int g = 0; g < 4; ++g) {
+        const bool in = there && g0 + 128 * g + 4 * lane < S;  // (pitch covers the four states)
+        x[g] = y[g] = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+        if (in) {
+          x[g] = *reinterpret_cast<const float4 *>(fr + g0 + 128 * g);
+          y[g] = *reinterpret_cast<const float4 *>(br + g0 + 128 * g);
+        }
+      }
+      uint32_t bits = 0, counts = 0;  // byte g: the keep bits of group g, how many they are
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        uint32_t m = 0;
+        if (__fadd_rn(x[g].x, y[g].x) > cutoff) m |= 1u;
+        if (__fadd_rn(x[g].y, y[g].y) > cutoff) m |= 2u;
+        if (__fadd_rn(x[g].z, y[g].z) > cutoff) m |= 4u;
+        if (__fadd_rn(x[g].w, y[g].w) > cutoff) m |= 8u;
+        bits |= m << (8 * g);
+        counts |= __popc(m) << (8 * g);
+      }
+      uint32_t incl = counts;  // at most 128 in a byte
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t o = __shfl_up_sync(kAll, incl, d);
+        if (lane >= d) incl += o;
+      }
+      const uint32_t sums = __shfl_sync(kAll, incl, 31);
+      incl -= counts;
+#pragma unroll
+      for (int g = 0; g < 4; ++g) {
+        if (g0 + 128 * g >= P) break;  // uniform
+        const uint32_t m = (bits >> (8 * g)) & 15u;
+        const int32_t at = n + (int32_t)((incl >> (8 * g)) & 0xffu);
+        const int32_t s = g0 + 128 * g + 4 * lane;
+        cells[(row * P + s) >> 2] = (uint16_t)(at << 4 | m);
+        const int32_t total = (int32_t)((sums >> (8 * g)) & 0xffu);
+        n += total;
+        if (total == 0) continue;  // uniform
+        uint16_t *out = list + row * P + at;
+        if (m & 1u) *out++ = (uint16_t)s;
+        if (m & 2u) *out++ = (uint16_t)(s + 1);
+        if (m & 4u) *out++ = (uint16_t)(s + 2);
+        if (m & 8u) *out++ = (uint16_t)(s + 3);
+        if (count_arcs && l >= a && l < b) {
+          for (uint32_t r = m; r; r &= r - 1) {
+            const int32_t idx = f.state_off + s + __ffs(r) - 1;
+            n_cand += __ldg(a_row_splits2 + idx + 1) - __ldg(a_row_splits2 + idx);
+          }
+        }
+      }
     }
-    unsigned char *row = keep_bits + (int64_t)(f.level_off + l) * kRowBytes;
-    if (K == 32) {
-      reinterpret_cast<uint32_t *>(row)[lane] = keep;
-    } else if (K == 16) {
-      reinterpret_cast<uint16_t *>(row)[lane] = (uint16_t)keep;
-    } else {  // states 256 .. 511 do not exist
-      row[lane] = (unsigned char)keep;
-      row[32 + lane] = 0;
-    }
-    n_states += __popc(keep);
-    if (count_arcs) {  // uniform; the host leaves it out when no count could reach max_arcs
-      for (uint32_t m = keep; m; m &= m - 1) {
-        const int32_t idx = f.state_off + s0 + __ffs(m) - 1;
-        n_cand += __ldg(a_row_splits2 + idx + 1) - __ldg(a_row_splits2 + idx);
+    if (lane == 0) {
+      n_sh[row] = n;
+      if (l >= a && l < b) {
+        atomicMax(&longest_sh, n);
+        atomicAdd(&counts_sh[0], (uint32_t)n);
       }
     }
   }
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) {
-    n_states += __shfl_xor_sync(kAll, n_states, d);
-    n_cand += __shfl_xor_sync(kAll, n_cand, d);
+  if (count_arcs) {  // uniform; the host leaves it out when no count could reach max_arcs
+    n_cand = __reduce_add_sync(kAll, n_cand);
+    if (lane == 0) atomicAdd(&counts_sh[1], n_cand);
   }
-  if (lane == 0 && (n_states | n_cand)) {
-    atomicAdd(&totals[0], (unsigned long long)n_states);
-    atomicAdd(&totals[2], (unsigned long long)n_cand);
+  __syncthreads();
+  // the longest list of the chunk's levels decides how many entries each of them gets
+  // (pitch >= padded), they lie `padded` entries apart from the start of the chunk;
+  // lists[level] = (start, size)
+  const int32_t longest = longest_sh;
+  const int32_t blocks = longest / 32 + 1, padded = 32 * blocks;
+  if (tid == 0) {
+    chunk_r[f.level_off + a] = blocks;
+    if (counts_sh[0]) atomicAdd(&totals[0], (unsigned long long)counts_sh[0]);
+    if (counts_sh[1]) atomicAdd(&totals[2], (unsigned long long)counts_sh[1]);
   }
-}
-
-// ---------------------------------------------------------------------------
-// Keep tests.  grid = (level chunks, pairs), 4 warps per CTA, a warp per chunk of
-// kPrepLevels levels.  Per level the warp
-//   1. scans the two Viterbi rows (a lane reads 16 consecutive states of each; the rows of
-//      the next level are requested before this level is worked on), marks the surviving
-//      states and writes them, in state order, to a list in shared memory;
-//   2. takes the list one state per lane: the reference's arc tests
-//      (intersect_dense.cu:430-471) against the rows of the level before and the dense
-//      score of the state's label give the entering-arc bits, the factors and where in the
-//      previous list the sources are;
-//   3. gives the entries of the level before their leaving-arc bits and destinations, which
-//      are the entering arcs of this level seen from the source.
-// Per level the result is the compact list of surviving states: a BandItem (label, state,
-// bits) and a BandFactor per entry.  A warp writes the complete entries of the levels it
-// owns, so it also runs step 1 for the level before its first and steps 1-2 for the level
-// after its last.  totals[0] += surviving states, totals[2] += the arcs leaving them (the
-// sizes the beam reduction looks at, intersect_dense.cu:289-320).  unfit[i] is set when the
-// register recursion cannot take graph i: a score outside its arithmetic, or a level with
-// more than kMaxListed surviving states.
-// ---------------------------------------------------------------------------
-constexpr float kMinLeanDense = -60.0f;   // dense score of a surviving arc
-constexpr int32_t kMaxLeanArcExp = 60, kMinLeanArcExp = -90;  // binary exponent of exp(arc score)
-
-// K = 16 or 32 states per lane of the scan (32 when a graph has more than 512 states).
-template <int K>
-__global__ void __launch_bounds__(128)
-BandPrep(const BandInfo *__restrict__ infos, const BandState *__restrict__ tab,
-         const BandArc *__restrict__ tabf, const unsigned char *__restrict__ keep_bits,
-         const float *__restrict__ lp, int32_t C, const float *__restrict__ vf,
-         const float *__restrict__ vb, const float *__restrict__ cutoffs,
-         BandItem *__restrict__ items, BandFactor *__restrict__ factors,
-         int2 *__restrict__ lists, int32_t *__restrict__ chunk_r, int32_t *__restrict__ unfit,
-         int32_t s_pad) {
-  constexpr unsigned kAll = 0xffffffffu;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int32_t i = blockIdx.y;
-  const BandInfo f = infos[i];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int32_t S = f.num_states, T = f.frames, pitch = f.pitch;
-  if (S == 0) return;
-  // a warp owns kPrepSub levels a .. b - 1, part of the chunk of kPrepLevels levels ca .. cb - 1
-  const int32_t a = (blockIdx.x * 4 + warp) * kPrepSub;
-  if (a > T + 1) return;
-  const int32_t b = min(a + kPrepSub, T + 2);
-  const int32_t ca = a / kPrepLevels * kPrepLevels, cb = min(ca + kPrepLevels, T + 2);
-  // per warp: a word per state for the current and the previous level (zero outside the
-  // lists), and the two lists
-  uint16_t *meta_sm = reinterpret_cast<uint16_t *>(smem_raw) +
-                      (size_t)warp * (4 * s_pad + 64 * (kPrepSub + 2));  // [2][s_pad]
-  uint16_t *list_sm = meta_sm + 2 * s_pad;                               // [2][s_pad]
-  // [kPrepSub + 2][32]: the lanes' keep bits
-  uint32_t *keep_sm = reinterpret_cast<uint32_t *>(list_sm + 2 * s_pad);
-  for (int32_t k = lane; k < 2 * s_pad; k += 32) meta_sm[k] = 0;
-  const float *fg = vf + f.grid_off, *bg = vb + f.grid_off;
-  const float cutoff = cutoffs[i];
+  if (tid < b - a)
+    lists[f.level_off + a + tid] = make_int2(a * pitch + tid * padded, n_sh[tid + 1]);
+  // position of state s (in 0 .. P - 1) on the level of `row`, -1 if it does not survive there
+  auto position = [&](int32_t row, int32_t s) {
+    const uint32_t cell = cells[(row * P + s) >> 2], bit = 1u << (s & 3);
+    return cell & bit ? (int32_t)((cell >> 4) + __popc(cell & (bit - 1u))) : -1;
+  };
+  // ---- 2. entering arcs -------------------------------------------------------------------
   const float *lp0 = lp + (int64_t)f.lp_row * C;
-  const int32_t s0 = lane * K;
-  const int32_t first = max(a - 1, 0);  // first level looked at (its list only)
-  const int32_t last = min(b, T + 1);   // last level looked at
-  // ---- 0. the keep bits of every level this warp looks at; the longest list of the
-  // CHUNK's levels decides how many entries every level of the chunk gets (every warp of a
-  // chunk finds the same number) ----------------------------------------------------------
-  int32_t longest = 0;
-  const int32_t lo = min(first, ca), hi = max(last, cb - 1);
-#pragma unroll 6
-  for (int32_t l = lo; l <= hi; ++l) {
-    const int64_t word = (int64_t)(f.level_off + l) * 32 + lane;
-    const uint32_t keep = K == 32 ? reinterpret_cast<const uint32_t *>(keep_bits)[word]
-                                  : reinterpret_cast<const uint16_t *>(keep_bits)[word];
-    if (l >= first && l <= last) keep_sm[(l - first) * 32 + lane] = keep;
-    const int32_t n = __reduce_add_sync(kAll, __popc(keep));
-    if (l >= ca && l < cb) longest = max(longest, n);
-  }
-  const int32_t padded = 32 * (longest / 32 + 1);  // entries per level of this chunk
-  if (lane == 0 && a == ca) chunk_r[f.level_off + ca] = padded / 32;
-  int32_t n_prev = 0;
-  // the lists of a warp's levels lie `padded` entries apart from the start of its chunk
-  // (pitch >= padded); lists[level] = (start, size)
-  int32_t run = ca * pitch + (a - ca) * padded, prev_start = 0;
-  bool risky = false;
-  __syncwarp();
-  for (int32_t l = first; l <= last; ++l) {
-    const bool own = l >= a && l < b;
-    uint16_t *cur_list = list_sm + (l & 1) * s_pad, *prev_list = list_sm + ((l & 1) ^ 1) * s_pad;
-    uint16_t *cur_meta = meta_sm + (l & 1) * s_pad, *prev_meta = meta_sm + ((l & 1) ^ 1) * s_pad;
-    // ---- 1. surviving states ------------------------------------------------------
-    const uint32_t keep = keep_sm[(l - first) * 32 + lane];
-    const int32_t mine = __popc(keep);
-    int32_t incl = mine;
+  bool risky = longest > kMaxListed;
+  {
+    // a warp's two levels together, 32 entries of each at a time, for their loads to overlap
+    static_assert(2 * kPrepWarps >= kPrepLevels + 1, "two levels per warp");
+    const float *xrow[2], *brow[2], *frow[2];
+    char *level[2];
+    int32_t n[2], row[2];
+    bool own[2];
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const int32_t o = __shfl_up_sync(kAll, incl, d);
-      if (lane >= d) incl += o;
+    for (int u = 0; u < 2; ++u) {
+      const int32_t k = warp + u * kPrepWarps, l = a + k;
+      row[u] = k + 1;
+      own[u] = l < b;
+      n[u] = k <= b - a && l <= T + 1 ? n_sh[row[u]] : 0;
+      xrow[u] = l >= 1 && l <= T ? lp0 + (int64_t)(l - 1) * C : nullptr;
+      brow[u] = bg + (int64_t)l * pitch;
+      frow[u] = fg + (int64_t)(l - 1) * pitch;
+      level[u] = reinterpret_cast<char *>(factors + f.grid_off + (int64_t)a * pitch + k * padded) +
+                 lane * 16;
     }
-    const int32_t n = __shfl_sync(kAll, incl, 31);
-    {
-      int32_t pos = incl - mine;
-      for (uint32_t m = keep; m; m &= m - 1) {
-        const int32_t s = s0 + __ffs(m) - 1;
-        cur_list[pos] = (uint16_t)s;
-        cur_meta[s] = (uint16_t)(kMetaKept | (uint32_t)pos);
-        ++pos;
+    const BandState *tab_f = tab + f.state_off;
+    // (the level behind the chunk may have more entries than the chunk's)
+    const int32_t upto = max(own[0] ? padded : 0, max(own[1] ? padded : n[1], n[0]));
+    for (int32_t j = lane; j - lane < upto; j += 32) {
+      int32_t s[2];
+      bool in[2];
+      BandState st[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        in[u] = j < n[u];
+        s[u] = in[u] ? list[row[u] * P + j] : 0;
+        if (in[u]) st[u] = tab_f[s[u]];
       }
-    }
-    if (n > kMaxListed) risky = true;
-    __syncwarp();
-    if (l >= a) {
-      // ---- 2. one surviving state per lane ------------------------------------------
-      BandItem *out = items + f.grid_off + run;
-      BandFactor *fout = factors + f.grid_off + run;
-      const float *fprev = fg + (int64_t)(l - 1) * pitch, *bprev = bg + (int64_t)(l - 1) * pitch;
-      const float *bcur = bg + (int64_t)l * pitch;
-      for (int32_t j = lane; j < n; j += 32) {
-        const int32_t s = cur_list[j];
-        const BandState t = tab[f.state_off + s];
-        uint32_t inb = 0;
-        BandFactor fa;
-        fa.pw[0] = fa.pw[1] = fa.pw[2] = 0.0;
-        fa.src[0] = fa.src[1] = fa.src[2] = fa.src[3] = 0;
-        fa.dst[0] = fa.dst[1] = fa.dst[2] = fa.dst[3] = (uint8_t)kNoDst;
-        if (l >= 1) {
-          const float x = BandDense(lp0, C, T, l - 1, t.label);
-          const float bc = bcur[s];
-          const double p = exp((double)x);
+      float x[2], bc[2], sf[2][3];
+      uint32_t src[2], kept[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        kept[u] = src[u] = 0;
+        x[u] = bc[u] = 0.0f;
+        if (in[u] && row[u] + a >= 2) {
+          if (xrow[u] != nullptr)
+            x[u] = st[u].label >= 0 && st[u].label < C ? __ldg(xrow[u] + st[u].label) : -INFINITY;
+          else  // the implied final row
+            x[u] = st[u].label == -1 ? 0.0f : -INFINITY;
+          bc[u] = brow[u][s[u]];
 #pragma unroll
           for (int d = 0; d < 3; ++d) {
-            if (s - d < 0) continue;
-            const float sf = fprev[s - d];
-            const bool kept = __fadd_rn(sf, bprev[s - d]) > cutoff;
-            const float sc = __fadd_rn(t.w[d], x);
-            if (kept && __fadd_rn(__fadd_rn(sf, sc), bc) > cutoff) {
+            const int32_t at = s[u] >= d ? position(row[u] - 1, s[u] - d) : -1;
+            sf[u][d] = -INFINITY;
+            if (at >= 0) {
+              kept[u] |= 1u << d;
+              src[u] |= ((uint32_t)at & 0xffu) << (8 * d);
+              sf[u][d] = frow[u][s[u] - d];
+            }
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        double pw[3] = {0.0, 0.0, 0.0};
+        uint32_t from = 0;
+        if (in[u]) {
+          uint32_t inb = 0;
+#pragma unroll
+          for (int d = 0; d < 3; ++d)
+            if (((kept[u] >> d) & 1u) &&
+                __fadd_rn(__fadd_rn(sf[u][d], __fadd_rn(st[u].w[d], x[u])), bc[u]) > cutoff)
               inb |= 1u << d;
-              if (own) {
-                const BandArc arc = tabf[(int64_t)(f.state_off + s) * 3 + d];
-                fa.pw[d] = arc.f * Pow2Clamp(arc.k) * p;
-                fa.src[d] = (uint8_t)(prev_meta[s - d] & kMetaPos);
-                // outside what doubles with a scale that follows the data every few
-                // levels hold: such graphs go to the (mantissa, exponent) recursion
-                if (!(x >= kMinLeanDense) || arc.k > kMaxLeanArcExp || arc.k < kMinLeanArcExp)
-                  risky = true;
-              }
-            }
-          }
-        }
-        cur_meta[s] = (uint16_t)(cur_meta[s] | (inb << kMetaInShift));
-        if (own) {
-          BandItem it;
-          it.label = t.label;
-          it.s = (uint16_t)s;
-          it.inb = (uint8_t)inb;
-          it.outb = 0;
-          out[j] = it;
-          fout[j] = fa;
-        }
-      }
-      if (own) {
-        BandFactor none;
-        none.pw[0] = none.pw[1] = none.pw[2] = 0.0;
-        none.src[0] = none.src[1] = none.src[2] = none.src[3] = 0;
-        none.dst[0] = none.dst[1] = none.dst[2] = none.dst[3] = (uint8_t)kNoDst;
-        for (int32_t j = n + lane; j < padded; j += 32) fout[j] = none;
-        if (lane == 0) lists[f.level_off + l] = make_int2(run, n);
-      }
-      __syncwarp();
-      // ---- 3. leaving arcs of the level before --------------------------------------------
-      if (l - 1 >= a) {
-        unsigned char *ibytes = reinterpret_cast<unsigned char *>(items + f.grid_off + prev_start);
-        unsigned char *fbytes = reinterpret_cast<unsigned char *>(factors + f.grid_off + prev_start);
-        for (int32_t j = lane; j < n_prev; j += 32) {
-          const int32_t s = prev_list[j];
-          uint32_t ob = 0;
+          inbs[row[u] * P + j] = (unsigned char)inb;
+          if (own[u] && inb) {
+            const double p = exp((double)x[u]);
+            // outside what doubles with a scale that follows the data every few
+            // levels hold: such graphs go to the (mantissa, exponent) recursion
+            if (!(x[u] >= kMinLeanDense)) risky = true;
 #pragma unroll
-          for (int d = 0; d < 3; ++d) {
-            const uint32_t m = cur_meta[s + d];
-            if ((m >> (kMetaInShift + d)) & 1u) {
-              ob |= 1u << d;
-              fbytes[(size_t)j * sizeof(BandFactor) + kDstByte + d] = (unsigned char)(m & kMetaPos);
-            }
+            for (int d = 0; d < 3; ++d)
+              if ((inb >> d) & 1u) {
+                from |= src[u] & (0xffu << (8 * d));
+                pw[d] = p;
+                if (st[u].w[d] != 0.0f) {  // (the factor of a score of zero is one)
+                  const BandArc arc = tabf[(int64_t)(f.state_off + s[u]) * 3 + d];
+                  pw[d] = arc.f * Pow2Clamp(arc.k) * p;
+                  if (arc.k > kMaxLeanArcExp || arc.k < kMinLeanArcExp) risky = true;
+                }
+              }
           }
-          if (ob) ibytes[(size_t)j * sizeof(BandItem) + kOutbByte] = (unsigned char)ob;
         }
+        if (own[u] && j < padded) {
+          *reinterpret_cast<double2 *>(level[u]) = make_double2(pw[0], pw[1]);
+          *reinterpret_cast<double *>(level[u] + padded * 16) = pw[2];
+          *reinterpret_cast<uint32_t *>(level[u] + padded * 16 + 8) = from;
+        }
+        level[u] += 32 * 16;
       }
-    }
-    __syncwarp();
-    // the previous level's words go back to zero for the level after this one
-    for (int32_t j = lane; j < n_prev; j += 32) prev_meta[prev_list[j]] = 0;
-    __syncwarp();
-    n_prev = n;
-    if (l >= a) {
-      prev_start = run;
-      run += padded;
     }
   }
-  if (__any_sync(kAll, risky) && lane == 0) atomicOr(&unfit[i], kUnfitFactors);
+  if (risky) risky_sh = 1;
+  __syncthreads();
+  // ---- 3. leaving arcs --------------------------------------------------------------------
+  for (int32_t k = warp; k < b - a; k += kPrepWarps) {
+    const int32_t row = k + 1, n = n_sh[row];
+    const int64_t at = f.grid_off + (int64_t)a * pitch + k * padded;
+    char *level = reinterpret_cast<char *>(factors + at) + padded * 16 + 12;
+    const bool leaving = a + k <= T;
+#pragma unroll 2
+    for (int32_t j = lane; j < padded; j += 32) {
+      uint32_t dst = kNoDst * 0x010101u;
+      if (j < n) {
+        const int32_t s = list[row * P + j];
+        BandItem it;
+        it.label = tab[f.state_off + s].label;
+        uint32_t outb = 0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          const int32_t to = leaving && s + d < P ? position(row + 1, s + d) : -1;
+          if (to >= 0 && ((inbs[(row + 1) * P + to] >> d) & 1u)) {
+            outb |= 1u << d;
+            dst ^= (kNoDst ^ ((uint32_t)to & 0xffu)) << (8 * d);
+          }
+        }
+        it.s = (uint16_t)s;
+        it.inb = (uint8_t)inbs[row * P + j];
+        it.outb = (uint8_t)outb;
+        items[at + j] = it;
+      }
+      *reinterpret_cast<uint32_t *>(level + j * 16) = dst;
+    }
+  }
+  if (tid == 0 && risky_sh) atomicOr(&unfit[i], kUnfitFactors);
 }
 
 // ---------------------------------------------------------------------------
-// alpha (dir 0) and beta (dir 1) over the lists, in registers.  grid = (2, pairs), one warp
-// per CTA.  Lane j holds the value of entry j (and j + 32, j + 64, j + 96) of the current level's
-// list; an entry says at which POSITIONS of the previous list its neighbours are, so the
-// values it needs come by shuffles from the lanes that hold them:
+// alpha (dir 0) and beta (dir 1) over the lists.  grid = (2, pairs), kMaxRegs warps per CTA:
+// thread j holds entry j of the current level's list, which says at which POSITIONS of the
+// previous list its neighbours are:
 //   alpha_l[j] = sum_d pw_l[j][d] * alpha_{l-1}[src_l[j][d]]
 //   beta_l[j]  = sum_d (pw_{l+1}[.][d] * beta_{l+1}[.]) at position dst_l[j][d]
-// Every level of a chunk of kPrepLevels levels has the same padded number of entries, 32 per
-// register, so inside a chunk every address is a constant: the fifteen levels after a
-// chunk's first are straight-line code, per level two 16-byte loads from shared memory, six
-// shuffles, three multiply-adds and a store per register: no test (an absent neighbour is
-// a padding entry, whose value is 0), no address arithmetic, no synchronisation.  The chunks
-// arrive in a ring in shared memory by one bulk copy each, requested chunks ahead.
+// What bounds it is the latency of a level: the values of two levels are in shared memory, so a
+// level costs one gather of three values, two dependent multiply-adds, a store and a barrier
+// of the warps that the chunk's lists need (none, with lists of up to 31 entries), whatever
+// the width of the lists; an entry's factors are fetched a level ahead.  (One warp with up to
+// four entries per lane and the values in registers took 48 to 150 instructions per level, at
+// one in five cycles: 145 us on ctc_large, 1002 levels; this takes 91.)
+// Every level of a chunk of kPrepLevels levels has the same padded number of entries, so inside a
+// chunk addresses advance by a constant.  No test: an absent neighbour is a padding entry,
+// whose value is 0.  The chunks arrive in a ring in shared memory by one bulk copy each,
+// requested chunks ahead.
 // The values of a level are stored divided by 2^K; K changes every kRescale levels by the
 // exponent of the largest value since the last change.  A value that is not zero and
 // below 2^-900 (or a value above 2^900) marks the graph in `unfit` for BandChainExact,
@@ -797,133 +816,154 @@ struct ChunkRing {
   }
 };
 
-// One level of the walk.  `rec` = this lane's entry of the level's first 32 (in shared
-// memory), `out` = where its value goes; RC registers per lane on this level, RP on the one
-// walked before.  v = values of the level before (forward), pc[d] = the products
-// pw[d] * value of the level before (backward); both are replaced by this level's.
-template <int DIR, int RC, int RP, bool kScaled>
-__device__ __forceinline__ void ChainLevel(const BandFactor *rec, double *__restrict__ out,
-                                           double scale, double (&v)[kMaxRegs],
-                                           double (&pc)[3][kMaxRegs], int32_t &hi_max,
-                                           uint32_t &min_hi) {
-  constexpr unsigned kAll = 0xffffffffu;
-  double nv[RC], pw[RC][3];
-#pragma unroll
-  for (int r = 0; r < RC; ++r) {
-    const double2 p01 = *reinterpret_cast<const double2 *>(rec + 32 * r);
-    const int4 q = *(reinterpret_cast<const int4 *>(rec + 32 * r) + 1);
-    pw[r][0] = p01.x;
-    pw[r][1] = p01.y;
-    pw[r][2] = __hiloint2double(q.y, q.x);
-    const uint32_t word = DIR == 0 ? (uint32_t)q.z : (uint32_t)q.w;
-    double x[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      // a shuffle looks at the low five bits of the lane only
-      const uint32_t pos = RP == 1 ? word >> (8 * d) : (word >> (8 * d)) & 0xffu;
-      x[d] = __shfl_sync(kAll, DIR == 0 ? v[0] : pc[d][0], (int)pos);
-      if (RP > 1) {
-        const double x1 = __shfl_sync(kAll, DIR == 0 ? v[1] : pc[d][1], (int)pos);
-        x[d] = pos >= 32u ? x1 : x[d];
-      }
-      if (RP > 2) {
-        const double x2 = __shfl_sync(kAll, DIR == 0 ? v[2] : pc[d][2], (int)pos);
-        x[d] = pos >= 64u ? x2 : x[d];
-      }
-      if (RP > 3) {
-        const double x3 = __shfl_sync(kAll, DIR == 0 ? v[3] : pc[d][3], (int)pos);
-        x[d] = pos >= 96u ? x3 : x[d];
-      }
-    }
-    double acc;
-    if (DIR == 0) acc = fma(pw[r][0], x[0], fma(pw[r][1], x[1], pw[r][2] * x[2]));
-    else acc = (x[0] + x[1]) + x[2];
-    nv[r] = kScaled ? acc * scale : acc;
-  }
-#pragma unroll
-  for (int r = 0; r < RC; ++r) {
-    out[32 * r] = nv[r];
-    const int32_t hi = __double2hiint(nv[r]);  // values are not negative
-    hi_max = max(hi_max, hi);
-    min_hi = min(min_hi, (uint32_t)hi - 1u);  // a zero does not count
-    v[r] = nv[r];
-    if (DIR == 1) {
-      pc[0][r] = pw[r][0] * nv[r];
-      pc[1][r] = pw[r][1] * nv[r];
-      pc[2][r] = pw[r][2] * nv[r];
-    }
-  }
+// What a thread reads of its entry.
+struct ChainRec {
+  double p0, p1, p2;
+  uint32_t at;  // positions: of the sources (forward) / destinations (backward)
+};
+template <int DIR, int kPer>
+__device__ __forceinline__ ChainRec LoadRec(const char *r) {
+  const double2 p01 = *reinterpret_cast<const double2 *>(r);
+  const int4 q = *reinterpret_cast<const int4 *>(r + 16 * kPer);
+  ChainRec x;
+  x.p0 = p01.x;
+  x.p1 = p01.y;
+  x.p2 = __hiloint2double(q.y, q.x);
+  x.at = DIR == 0 ? (uint32_t)q.z : (uint32_t)q.w;
+  return x;
 }
 
-// The same with the register counts known at run time only.
-template <int DIR>
-__device__ __forceinline__ void ChainLevelAny(int32_t rc, int32_t rp, const BandFactor *rec,
-                                              double *__restrict__ out, double scale,
-                                              double (&v)[kMaxRegs],
-                                              double (&pc)[3][kMaxRegs], int32_t &hi_max,
-                                              uint32_t &min_hi) {
-#define K2B_LEVEL(RC, RP) \
-  case RC * 8 + RP: ChainLevel<DIR, RC, RP, true>(rec, out, scale, v, pc, hi_max, min_hi); break;
-  switch (rc * 8 + rp) {
-    K2B_LEVEL(1, 1) K2B_LEVEL(1, 2) K2B_LEVEL(1, 3) K2B_LEVEL(1, 4)
-    K2B_LEVEL(2, 1) K2B_LEVEL(2, 2) K2B_LEVEL(2, 3) K2B_LEVEL(2, 4)
-    K2B_LEVEL(3, 1) K2B_LEVEL(3, 2) K2B_LEVEL(3, 3) K2B_LEVEL(3, 4)
-    K2B_LEVEL(4, 1) K2B_LEVEL(4, 2) K2B_LEVEL(4, 3)
-    default: ChainLevel<DIR, 4, 4, true>(rec, out, scale, v, pc, hi_max, min_hi); break;
+// Values of two levels, by list position: forward alpha; backward the three products pw[d] *
+// beta, which is what the entries of the level below add up.  Position kNoDst is always zero.
+struct ChainValues {
+  double v[2][3][256];
+};
+
+// One thread's state of the walk.
+struct ChainState {
+  double acc, scale;
+  int32_t Ksh;      // the level's values are stored divided by 2^Ksh
+  int32_t hi_max;   // largest high word since the last change of scale
+  uint32_t min_hi;  // smallest (high word - 1), zeros apart
+};
+
+// One level.  kBuf: the values go to vals.v[kBuf], those of the level before are in the other.
+template <int DIR, int kBuf>
+__device__ __forceinline__ void ChainLevel(const ChainRec &rec, ChainValues &vals, int tid,
+                                           bool first, bool rescaled, ChainState &st,
+                                           double *out) {
+  const char *prev = reinterpret_cast<const char *>(vals.v[kBuf ^ 1][0]);
+  const double x0 = *reinterpret_cast<const double *>(prev + ((rec.at << 3) & 0x7f8u));
+  const double x1 = *reinterpret_cast<const double *>(prev + ((rec.at >> 5) & 0x7f8u) +
+                                                      (DIR == 0 ? 0 : 2048));
+  const double x2 = *reinterpret_cast<const double *>(prev + ((rec.at >> 13) & 0x7f8u) +
+                                                      (DIR == 0 ? 0 : 4096));
+  double acc = DIR == 0 ? fma(rec.p0, x0, fma(rec.p1, x1, rec.p2 * x2)) : (x0 + x1) + x2;
+  if (rescaled) acc *= st.scale;
+  // the first level holds one state, with the value 1: the start state walking forward, the
+  // final state walking backward
+  if (first) acc = tid == 0 ? 1.0 : 0.0;
+  if (DIR == 0) {
+    vals.v[kBuf][0][tid] = acc;
+  } else {
+    vals.v[kBuf][0][tid] = rec.p0 * acc;
+    vals.v[kBuf][1][tid] = rec.p1 * acc;
+    vals.v[kBuf][2][tid] = rec.p2 * acc;
   }
-#undef K2B_LEVEL
+  *out = acc;
+  const int32_t hi = __double2hiint(acc);  // values are not negative
+  st.hi_max = max(st.hi_max, hi);
+  st.min_hi = min(st.min_hi, (uint32_t)hi - 1u);  // a zero does not count
+  st.acc = acc;
 }
 
-// The new scale after kRescale levels: the exponent of the largest value since the last one.
-__device__ __forceinline__ double ChainRescale(int32_t &hi_max, int32_t &Ksh) {
-  const int32_t hm = __reduce_max_sync(0xffffffffu, hi_max);
+// The scale that the values of the next group of levels are multiplied with.
+__device__ __forceinline__ void ChainRescale(int32_t hm, ChainState &st) {
   const int32_t e = hm > 0 ? (hm >> 20) - 1023 : 0;
-  Ksh += e;
-  hi_max = 0;
-  return __longlong_as_double((long long)(1023 - e) << 52);
+  st.Ksh += e;
+  st.scale = __longlong_as_double((long long)(1023 - e) << 52);
 }
 
-// Levels 1 .. 15 (in walking order) of a full chunk with RC registers per lane: seven levels,
-// the level that changes the scale, seven levels.  kChainUnroll levels of straight-line code per
-// loop iteration: a single warp has nobody to hide an instruction-cache miss behind, so the
-// code of a chunk should stay small.
-constexpr int kChainUnroll = 1;  // (fully unrolled: 178 us for ctc_large; 1: 147 us)
+template <int kBuf>
+struct ChainBuf {
+  static constexpr int value = kBuf;
+};
 
-template <int DIR, int RC>
-__device__ __forceinline__ void ChainRest(const BandFactor *base, double *__restrict__ ob,
-                                          int32_t *__restrict__ osc, int lane, double (&v)[kMaxRegs],
-                                          double (&pc)[3][kMaxRegs], int32_t &hi_max, uint32_t &min_hi,
-                                          int32_t &Ksh) {
-  static_assert(kPrepLevels == 2 * kRescale, "a chunk is two groups of kRescale levels");
+template <int kWarps>
+__device__ __forceinline__ void ChainSync() {
+  if (kWarps == 1) __syncwarp();
+  else asm volatile("bar.sync 1, %0;" ::"n"(32 * kWarps) : "memory");
+}
+
+// The nl levels of a chunk; by the kWarps warps that its lists need.  r = this thread's entry
+// of the first level walked, out / osc = where its results go.
+template <int DIR, int kWarps>
+__device__ __forceinline__ void ChainChunk(const char *r, double *out, int32_t *osc,
+                                           int32_t l, int32_t nl, bool first_chunk,
+                                           ChainValues &vals, int32_t *hi_sh, int &group,
+                                           ChainState &st, int32_t *unfit_i) {
+  constexpr unsigned kAll = 0xffffffffu;
   constexpr int kStep = DIR == 0 ? 1 : -1;
-  auto plain = [&](int kk_first) {  // kRescale - 1 levels without a change of scale
-    const int m0 = DIR == 0 ? kk_first : kPrepLevels - 1 - kk_first;
-    const BandFactor *r = base + m0 * 32 * RC;
-    double *o = ob + m0 * 32 * RC;
-    int32_t *sc = osc + m0;
-#pragma unroll kChainUnroll
-    for (int k = 0; k < kRescale - 1; ++k) {
-      ChainLevel<DIR, RC, RC, false>(r, o, 1.0, v, pc, hi_max, min_hi);
-      if (lane == 0) *sc = Ksh;
-      r += kStep * 32 * RC;
-      o += kStep * 32 * RC;
-      sc += kStep;
+  constexpr int kPer = 32 * kWarps;
+  // levels (mod kRescale) that change the scale / end a group / clear the old maximum
+  constexpr int kScales = DIR == 0 ? 0 : kRescale - 1, kEnds = DIR == 0 ? kRescale - 1 : 0,
+                kClears = DIR == 0 ? 2 : kRescale - 3;
+  const int tid = threadIdx.x, lane = tid & 31;
+  ChainRec rec = LoadRec<DIR, kPer>(r);
+  auto level = [&](auto buf, int32_t phase, bool first, bool last, int32_t j) {
+    constexpr int kBuf = decltype(buf)::value;
+    // (the level behind a chunk's last is read and not used: it is inside the ring)
+    const ChainRec next = last ? rec : LoadRec<DIR, kPer>(r + kStep * (j + 1) * kPer * 32);
+    const bool rescaled = phase == kScales && !first;
+    if (rescaled) {
+      ChainRescale(*reinterpret_cast<volatile int32_t *>(&hi_sh[group]), st);
+      group ^= 1;
     }
+    ChainLevel<DIR, kBuf>(rec, vals, tid, first, rescaled, st, out + kStep * j * kPer);
+    if (phase == kEnds) {
+      const int32_t hm = __reduce_max_sync(kAll, st.hi_max);
+      if (lane == 0) {
+        atomicMax(&hi_sh[group], hm);
+        if (hm >= (1023 + 900) << 20) atomicOr(unfit_i, kUnfitRange);
+      }
+      st.hi_max = 0;
+    }
+    if (tid == 0) {
+      osc[kStep * j] = st.Ksh;
+      if (phase == kClears) hi_sh[group ^ 1] = 0;
+    }
+    rec = next;
+    ChainSync<kWarps>();
   };
-  plain(1);
-  {
-    const int m = DIR == 0 ? kRescale : kPrepLevels - 1 - kRescale;
-    const double scale = ChainRescale(hi_max, Ksh);
-    ChainLevel<DIR, RC, RC, true>(base + m * 32 * RC, ob + m * 32 * RC, scale, v, pc, hi_max,
-                                  min_hi);
-    if (lane == 0) osc[m] = Ksh;
+  // level l's values are in buffer l & 1
+  if (!first_chunk && nl == kPrepLevels) {
+    for (int32_t g = 0; g < kPrepLevels / kRescale; ++g) {
+#pragma unroll
+      for (int j = 0; j < kRescale; ++j) {
+        const int phase = DIR == 0 ? j : kRescale - 1 - j;
+        const bool last = j == kRescale - 1 && g == kPrepLevels / kRescale - 1;
+        if (phase & 1) level(ChainBuf<1>{}, phase, false, last, j);
+        else level(ChainBuf<0>{}, phase, false, last, j);
+      }
+      r += kStep * kRescale * kPer * 32;
+      out += kStep * kRescale * kPer;
+      osc += kStep * kRescale;
+    }
+  } else {
+    for (int32_t k = 0; k < nl; ++k, l += kStep) {
+      if (l & 1) level(ChainBuf<1>{}, l & (kRescale - 1), first_chunk && k == 0, k == nl - 1, 0);
+      else level(ChainBuf<0>{}, l & (kRescale - 1), first_chunk && k == 0, k == nl - 1, 0);
+      r += kStep * kPer * 32;
+      out += kStep * kPer;
+      osc += kStep;
+    }
   }
-  plain(kRescale + 1);
 }
 
 template <int DIR>
 __device__ __forceinline__ void ChainWalk(const BandInfo &f, int32_t i, BandFactor *ring,
-                                          unsigned char *crc, uint64_t *full,
+                                          ChainValues &vals, unsigned char *crc, uint64_t *full,
+                                          int32_t *hi_sh,
                                           const BandFactor *__restrict__ factors,
                                           const int32_t *__restrict__ chunk_r,
                                           double *__restrict__ om, int32_t *__restrict__ oscale,
@@ -931,22 +971,24 @@ __device__ __forceinline__ void ChainWalk(const BandInfo &f, int32_t i, BandFact
                                           int32_t *__restrict__ unfit,
                                           int32_t *__restrict__ status, int32_t wait_limit) {
   constexpr unsigned kAll = 0xffffffffu;
-  const int lane = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int32_t T = f.frames, pitch = f.pitch, L = T + 2;
   const int32_t num_chunks = (L + kPrepLevels - 1) / kPrepLevels;
-  for (int32_t c = lane; c < num_chunks; c += 32)
+  for (int32_t c = tid; c < num_chunks; c += kChainThreads)
     crc[c] = (unsigned char)chunk_r[f.level_off + c * kPrepLevels];
-  if (lane == 0) {
+  if (tid < 6) vals.v[tid / 3][tid % 3][kNoDst] = 0.0;
+  if (tid == 0) {
     for (int st = 0; st < kChainSlots; ++st) MbarInit(&full[st], 1);
     MbarInitFence();
+    hi_sh[0] = hi_sh[1] = hi_sh[2] = hi_sh[3] = 0;
   }
-  __syncwarp();
+  __syncthreads();
   const BandFactor *fac0 = factors + f.grid_off;
   om += f.grid_off;
   oscale += f.level_off;
   int32_t issued = 0;
-  // lane 0: the next chunk (in walking order) into the next slot; a chunk is
-  // levels * 32 * registers entries, a multiple of 1 KB
+  // thread 0: the next chunk (in walking order) into the next slot; a chunk is
+  // levels * 32 * (warps it needs) entries, a multiple of 1 KB
   auto issue = [&]() {
     if (issued >= num_chunks) return;
     const int32_t c = DIR == 0 ? issued : num_chunks - 1 - issued, slot = issued % kChainSlots;
@@ -957,99 +999,80 @@ __device__ __forceinline__ void ChainWalk(const BandInfo &f, int32_t i, BandFact
                 &full[slot]);
     ++issued;
   };
-  if (lane == 0)
+  if (tid == 0)
     for (int32_t k = 0; k < kChainSlots; ++k) issue();
-  double v[kMaxRegs], pc[3][kMaxRegs];
-#pragma unroll
-  for (int r = 0; r < kMaxRegs; ++r) v[r] = pc[0][r] = pc[1][r] = pc[2][r] = 0.0;
-  int32_t Ksh = 0;
-  int32_t hi_max = 0;              // largest high word since the last change of scale
-  uint32_t min_hi = 0xffffffffu;   // smallest (high word - 1), zeros apart
-  bool late = false;
-  int32_t rp = 1;
+  ChainState st;
+  st.acc = 0.0;
+  st.scale = 1.0;
+  st.Ksh = 0;
+  st.hi_max = 0;
+  st.min_hi = 0xffffffffu;
+  int group = 0;
+  bool late = false, idle = false;
   for (int32_t q = 0; q < num_chunks; ++q) {
     const int32_t c = DIR == 0 ? q : num_chunks - 1 - q, slot = q % kChainSlots;
     late = !WaitSlot(&full[slot], (unsigned)(q / kChainSlots) & 1u, wait_limit);
-    late = __any_sync(kAll, late);
+    // (also: the chunk before has been read, and its last level's values are there)
+    late = __syncthreads_or(late);
     if (late) break;
+    if (q > 0 && tid == 0) issue();  // into the slot of the chunk before
+    if (idle) {  // what the warps at work kept track of
+      st.Ksh = hi_sh[2];
+      group = hi_sh[3];
+    }
     const int32_t l_lo = c * kPrepLevels, nl = min(l_lo + kPrepLevels, L) - l_lo;
     const int32_t rc = crc[c];
-    const BandFactor *base = ring + (size_t)slot * kFacSlot + lane;
-    double *ob = om + (int64_t)l_lo * pitch + lane;
-    int32_t *osc = oscale + l_lo;
-    // the chunk's first level meets the registers of the chunk before; the levels of a
-    // short chunk (the last of a graph) are taken the same way
-    int32_t kk = 0;
-    do {
-      const int32_t m = DIR == 0 ? kk : nl - 1 - kk, l = l_lo + m;
-      const BandFactor *rec = base + m * 32 * rc;
-      double *out = ob + m * 32 * rc;
-      if (q == 0 && kk == 0) {
-        // the first level holds one state, with the value 1: the start state walking
-        // forward, the final state walking backward
-        v[0] = lane == 0 ? 1.0 : 0.0;
-#pragma unroll
-        for (int r = 1; r < kMaxRegs; ++r) v[r] = 0.0;
-#pragma unroll
-        for (int r = 0; r < kMaxRegs; ++r) {
-          if (r >= rc) break;  // uniform
-          out[32 * r] = v[r];
-          if (DIR == 1) {
-            const BandFactor e = rec[32 * r];
-            pc[0][r] = e.pw[0] * v[r];
-            pc[1][r] = e.pw[1] * v[r];
-            pc[2][r] = e.pw[2] * v[r];
-          }
-        }
-      } else {
-        double scale = 1.0;
-        if ((l & (kRescale - 1)) == (DIR == 0 ? 0 : kRescale - 1)) scale = ChainRescale(hi_max, Ksh);
-        ChainLevelAny<DIR>(rc, kk == 0 ? rp : rc, rec, out, scale, v, pc, hi_max, min_hi);
+    const int32_t l = DIR == 0 ? l_lo : l_lo + nl - 1;
+    idle = warp >= rc;
+    if (!idle) {
+      const int32_t at = (l - l_lo) * 32 * rc + tid;
+      const char *r = reinterpret_cast<const char *>(ring + (size_t)slot * kFacSlot +
+                                                     (l - l_lo) * 32 * rc) + tid * 16;
+      double *out = om + (int64_t)l_lo * pitch + at;
+      int32_t *osc = oscale + l;
+      switch (rc) {
+        case 1: ChainChunk<DIR, 1>(r, out, osc, l, nl, q == 0, vals, hi_sh, group, st, &unfit[i]); break;
+        case 2: ChainChunk<DIR, 2>(r, out, osc, l, nl, q == 0, vals, hi_sh, group, st, &unfit[i]); break;
+        case 3: ChainChunk<DIR, 3>(r, out, osc, l, nl, q == 0, vals, hi_sh, group, st, &unfit[i]); break;
+        default: ChainChunk<DIR, 4>(r, out, osc, l, nl, q == 0, vals, hi_sh, group, st, &unfit[i]); break;
       }
-      if (lane == 0) osc[m] = Ksh;
-      ++kk;
-    } while (kk < nl && nl != kPrepLevels);
-    if (nl == kPrepLevels) {
-      if (rc == 1) ChainRest<DIR, 1>(base, ob, osc, lane, v, pc, hi_max, min_hi, Ksh);
-      else if (rc == 2) ChainRest<DIR, 2>(base, ob, osc, lane, v, pc, hi_max, min_hi, Ksh);
-      else if (rc == 3) ChainRest<DIR, 3>(base, ob, osc, lane, v, pc, hi_max, min_hi, Ksh);
-      else ChainRest<DIR, 4>(base, ob, osc, lane, v, pc, hi_max, min_hi, Ksh);
     }
-    rp = rc;
-    __syncwarp();  // every lane has read the slot
-    if (lane == 0) issue();  // the chunk is done with: its slot takes the next one
+    if (tid == 0) {
+      hi_sh[2] = st.Ksh;
+      hi_sh[3] = group;
+    }
   }
   if (late) {
-    if (lane == 0) {
+    if (tid == 0) {
       atomicOr(status, kStatusLate);
       for (int32_t k = max(0, issued - kChainSlots); k < issued; ++k)
         WaitSlot(&full[k % kChainSlots], (unsigned)(k / kChainSlots) & 1u, kDrainPolls);
     }
-    __syncwarp();
+    __syncthreads();
   }
   {
     // values that are not zero must have kept clear of the ends of a double's range
-    const int32_t hm = __reduce_max_sync(kAll, hi_max);
-    const uint32_t hn = __reduce_min_sync(kAll, min_hi);
+    const int32_t hm = __reduce_max_sync(kAll, st.hi_max);
+    const uint32_t hn = __reduce_min_sync(kAll, st.min_hi);
     if ((hm >= ((1023 + 900) << 20) || hn < (uint32_t)(((1023 - 900) << 20) - 1)) && lane == 0)
       atomicOr(&unfit[i], kUnfitRange);
   }
-  if (DIR == 0 && lane == 0) {
-    const double last = v[0];  // entry 0 of the last level is the final state
+  if (DIR == 0 && tid == 0) {
+    // entry 0 of the last level is the final state
     if (*status & kStatusLate) {
       tot[i] = nan("");
-    } else if (!late && last > 0.0) {
-      tot[i] = log(last) + (double)Ksh * 0.69314718055994530942;
+    } else if (!late && st.acc > 0.0) {
+      tot[i] = log(st.acc) + (double)st.Ksh * 0.69314718055994530942;
       BandTotal z;
-      z.m = last;
-      z.e = Ksh;
+      z.m = st.acc;
+      z.e = st.Ksh;
       z.pad = 0;
       total[i] = z;
     }
   }
 }
 
-__global__ void __launch_bounds__(32)
+__global__ void __launch_bounds__(kChainThreads)
 BandChainLists(const BandInfo *__restrict__ infos, const BandFactor *__restrict__ factors,
                const int32_t *__restrict__ chunk_r, double *__restrict__ am,
                double *__restrict__ bm, int32_t *__restrict__ a_scale,
@@ -1058,6 +1081,8 @@ BandChainLists(const BandInfo *__restrict__ infos, const BandFactor *__restrict_
                int32_t *__restrict__ status, int32_t wait_limit) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full[kChainSlots];
+  __shared__ ChainValues vals;
+  __shared__ int32_t hi_sh[4];
   __shared__ unsigned char crc[kChainMaxChunks];
   const int dir = blockIdx.x;
   const int32_t i = blockIdx.y;
@@ -1073,10 +1098,10 @@ BandChainLists(const BandInfo *__restrict__ infos, const BandFactor *__restrict_
   if (f.num_states == 0 || unfit[i] != 0) return;  // BandChainExact takes the graphs BandPrep marked
   BandFactor *ring = reinterpret_cast<BandFactor *>(smem_raw);  // [slots][kFacSlot]
   if (dir == 0)
-    ChainWalk<0>(f, i, ring, crc, full, factors, chunk_r, am, a_scale, tot, total, unfit, status,
+    ChainWalk<0>(f, i, ring, vals, crc, full, hi_sh, factors, chunk_r, am, a_scale, tot, total, unfit, status,
                  wait_limit);
   else
-    ChainWalk<1>(f, i, ring, crc, full, factors, chunk_r, bm, b_scale, tot, total, unfit, status,
+    ChainWalk<1>(f, i, ring, vals, crc, full, hi_sh, factors, chunk_r, bm, b_scale, tot, total, unfit, status,
                  wait_limit);
 }
 
@@ -1592,11 +1617,11 @@ struct BandLayout {
   long long arc_frames = 0;
   int32_t max_states = 0, max_frames = 0, max_rows = 0;
   int32_t vit_threads = 32, vit_frames = 0, vit_batches = 0, vit_slot = 0, xch_pad = 0;
-  int32_t keep_row = 64, first_row = 0;
+  int32_t first_row = 0;
   int32_t st_pad = 0, lv_pad = 0;
   size_t chain_smem = 0, exact_smem = 0, viterbi_smem = 0, prep_smem = 0;
-  size_t off_infos, off_vf, off_vb, off_items, off_factors, off_lists, off_chunk_r, off_keep, off_cutoffs, off_am, off_ae, off_bm,
-      off_be, off_a_scale, off_b_scale, off_total, off_unfit, off_totals, off_status,
+  size_t off_infos, off_vf, off_vb, off_items, off_factors, off_lists, off_chunk_r, off_am, off_ae,
+      off_bm, off_be, off_a_scale, off_b_scale, off_total, off_unfit, off_totals, off_status,
       total_bytes;  // off_status = off_totals + 40
   bool ok = true;
   const char *why = "";
@@ -1694,7 +1719,7 @@ static int32_t MakeBandLayout(const k2b200_band_loss_args *a, BandLayout *L) {
   }
   L->st_pad = ((L->max_states + 4) + 15) & ~15;
   L->lv_pad = (L->max_frames + 2 + 3) & ~3;
-  L->prep_smem = (size_t)4 * (8 * L->st_pad + 128 * (kPrepSub + 2));
+  L->prep_smem = BandPrepSmem(L->max_states);
   L->exact_smem = sizeof(BandItem) * kChainSlots * kSlotItems + sizeof(int2) * (size_t)L->lv_pad +
                   sizeof(ProbState) * 2 * (size_t)L->st_pad;
   L->chain_smem = sizeof(BandFactor) * kChainSlots * kFacSlot;
@@ -1723,10 +1748,7 @@ static int32_t MakeBandLayout(const k2b200_band_loss_args *a, BandLayout *L) {
   L->off_items = take(sizeof(BandItem) * (size_t)grid);
   L->off_lists = take(sizeof(int2) * (size_t)levels);
   L->off_chunk_r = take(sizeof(int32_t) * (size_t)levels);
-  L->keep_row = L->max_states > 512 ? 128 : 64;
-  L->off_keep = take((size_t)L->keep_row * (size_t)levels);
   L->off_factors = take(sizeof(BandFactor) * (size_t)grid);
-  L->off_cutoffs = take(sizeof(float) * a->num_fsas);
   L->off_am = take(sizeof(double) * (size_t)grid);
   L->off_ae = take(sizeof(int32_t) * (size_t)grid);
   L->off_bm = take(sizeof(double) * (size_t)grid);
@@ -1775,7 +1797,7 @@ static int32_t LaunchBandChains(const BandLayout &L, const k2b200_band_loss_args
   BandTotal *total = reinterpret_cast<BandTotal *>(ws + L.off_total);
   int32_t *unfit = reinterpret_cast<int32_t *>(ws + L.off_unfit);
   int32_t *status = reinterpret_cast<int32_t *>(ws + L.off_status);
-  { BandChainLists<<<grid, 32, L.chain_smem, stream>>>(
+  { BandChainLists<<<grid, kChainThreads, L.chain_smem, stream>>>(
       infos, reinterpret_cast<const BandFactor *>(ws + L.off_factors),
       reinterpret_cast<const int32_t *>(ws + L.off_chunk_r), am, bm,
       reinterpret_cast<int32_t *>(ws + L.off_a_scale),
@@ -1908,6 +1930,8 @@ int32_t k2b200_band_loss_forward_reduce(const k2b200_band_loss_args *args, void 
   {
     PhaseTimer timer(kPhaseViterbi, stream);
     NotePhaseKernel(kPhaseViterbi, "BandViterbi");
+    K2B_CUDA_OK(cudaFuncSetAttribute(BandPrep, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)L.prep_smem));
     K2B_CUDA_OK(cudaFuncSetAttribute(BandViterbi, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)L.viterbi_smem));
     dim3 grid(2, args->num_fsas);
@@ -1943,41 +1967,26 @@ int32_t k2b200_band_loss_forward_reduce(const k2b200_band_loss_args *args, void 
     cudaStream_t side = nullptr;
     {
       PhaseTimer timer(kPhasePrune, stream);
-      NotePhaseKernel(kPhasePrune, "BandKeep+BandPrep");
-      dim3 kgrid(CeilDiv(L.max_frames + 2, 4 * kKeepLevels), args->num_fsas);
-#define K2B_BAND_KEEP(KK)                                                                   \
-      { BandKeep<KK><<<kgrid, 128, 0, stream>>>(                                                \
-          reinterpret_cast<const BandInfo *>(ws + L.off_infos), args->a_row_splits2,            \
-          reinterpret_cast<const float *>(ws + L.off_vf),                                       \
-          reinterpret_cast<const float *>(ws + L.off_vb), beam,                                 \
-          reinterpret_cast<unsigned char *>(ws + L.off_keep),                                   \
-          reinterpret_cast<float *>(ws + L.off_cutoffs),                                        \
-          reinterpret_cast<unsigned long long *>(ws + L.off_totals),                            \
-          L.arc_frames > args->max_arcs ? 1 : 0); NoteLaunch(); }
-      if (L.max_states <= 256) K2B_BAND_KEEP(8)
-      else if (L.max_states <= 512) K2B_BAND_KEEP(16)
-      else K2B_BAND_KEEP(32)
-#undef K2B_BAND_KEEP
-      // the host reads the counts behind BandKeep, while what follows runs
-      if (need_count) {
-        K2B_FORWARD(SideFork(stream, &side));
-        K2B_FORWARD(readback.Begin(ws + L.off_totals, sizeof(long long) * 6));
-      }
-      dim3 grid(CeilDiv(L.max_frames + 2, 4 * kPrepSub), args->num_fsas);
-      auto prep = L.max_states <= 512 ? BandPrep<16> : BandPrep<32>;
-      { prep<<<grid, 128, L.prep_smem, stream>>>(
-          reinterpret_cast<const BandInfo *>(ws + L.off_infos),
+      NotePhaseKernel(kPhasePrune, "BandPrep");
+      dim3 grid(CeilDiv(L.max_frames + 2, kPrepLevels), args->num_fsas);
+      { BandPrep<<<grid, 32 * kPrepWarps, L.prep_smem, stream>>>(
+          reinterpret_cast<const BandInfo *>(ws + L.off_infos), args->a_row_splits2,
           reinterpret_cast<const BandState *>(args->band_states),
-          reinterpret_cast<const BandArc *>(args->band_arcs),
-          reinterpret_cast<const unsigned char *>(ws + L.off_keep), args->log_probs,
+          reinterpret_cast<const BandArc *>(args->band_arcs), args->log_probs,
           args->num_classes, reinterpret_cast<const float *>(ws + L.off_vf),
-          reinterpret_cast<const float *>(ws + L.off_vb),
-          reinterpret_cast<const float *>(ws + L.off_cutoffs),
+          reinterpret_cast<const float *>(ws + L.off_vb), beam,
           reinterpret_cast<BandItem *>(ws + L.off_items),
           reinterpret_cast<BandFactor *>(ws + L.off_factors),
           reinterpret_cast<int2 *>(ws + L.off_lists),
           reinterpret_cast<int32_t *>(ws + L.off_chunk_r),
-          reinterpret_cast<int32_t *>(ws + L.off_unfit), L.st_pad); NoteLaunch(); }
+          reinterpret_cast<unsigned long long *>(ws + L.off_totals),
+          reinterpret_cast<int32_t *>(ws + L.off_unfit),
+          L.arc_frames > args->max_arcs ? 1 : 0); NoteLaunch(); }
+      // the host reads the counts behind BandPrep, while what follows runs
+      if (need_count) {
+        K2B_FORWARD(SideFork(stream, &side));
+        K2B_FORWARD(readback.Begin(ws + L.off_totals, sizeof(long long) * 6));
+      }
       K2B_CUDA_OK(cudaGetLastError());
     }
     if (iter == 0 && args->zero_fill != nullptr && args->zero_fill_bytes > 0) {
