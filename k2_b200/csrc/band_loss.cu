@@ -42,6 +42,7 @@
 // the last frame a state scores 0 if its label is -1 and -inf otherwise.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "../../include/k2b200.h"
@@ -54,6 +55,7 @@ namespace k2b {
 
 constexpr int kBandMaxStates = 1024;
 constexpr int kVitK = 4;              // states per thread of BandViterbi
+constexpr int kVitFramesByState = 8;  // frames between two exchanges of its warps, rows by state
 constexpr int kPrepLevels = 16;       // levels per chunk: their lists share one padded size
 constexpr int kGradLevels = 4;        // levels per warp of BandGrad
 constexpr int kDrainPolls = 4000000;  // bounded wait for copies in flight when a kernel gives up
@@ -205,16 +207,79 @@ __global__ void BandTables(const int32_t *__restrict__ row_splits1, int32_t num_
 // of a batch are contiguous and arrive by ONE bulk copy (TMA, completion on an mbarrier)
 // requested batches ahead, the warps exchange their boundary states through shared memory
 // once per batch, and the frames of a batch run without any wait, barrier or
-// shared-memory store: per frame four shared-memory reads, two shuffles, the adds and
-// maxima, one 16-byte store.  Same fp32 expressions as the reference:
+// shared-memory store: per frame four (backward: six) shared-memory reads, two shuffles, the
+// adds and maxima, one 16-byte store.  Same fp32 expressions as the reference:
 // (prev + arc.score) + dense, then max.
+// Bound by the instructions of a warp per frame, 45 at one in about three cycles: 87 us for
+// 1000 frames x 501 states.  (Two states per thread: 117 us; rows put in the order of the
+// states by further warps: 118; packed additions: the moves into register pairs cost more
+// than they save.)
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float Max3(float a, float b, float c) { return fmaxf(fmaxf(a, b), c); }
 
 constexpr int kVitMaxBatches = 4;  // batches of rows in flight
 constexpr int kVitMaxWarps = 12;
 
-__global__ void __launch_bounds__(32 * kVitMaxWarps)
+// K consecutive values, stored or read as one word.
+template <int K>
+struct VitPack;
+template <>
+struct VitPack<2> {
+  using type = float2;
+};
+template <>
+struct VitPack<4> {
+  using type = float4;
+};
+template <int K>
+__device__ __forceinline__ void VitStore(float *p, const float (&v)[K]) {
+  typename VitPack<K>::type t;
+  memcpy(&t, v, sizeof(t));
+  *reinterpret_cast<typename VitPack<K>::type *>(p) = t;
+}
+template <int K>
+__device__ __forceinline__ void VitLoad(const float *p, float (&v)[K]) {
+  const typename VitPack<K>::type t = *reinterpret_cast<const typename VitPack<K>::type *>(p);
+  memcpy(v, &t, sizeof(t));
+}
+
+// The log-probs of the states' labels, in the layout of the grids: row r of a sequence at row r of
+// its grid, -inf for a label without a column.  Bound by the 32-byte sectors of the log-probs
+// that it touches.
+constexpr int kGatherRows = 16;  // per CTA: two per warp
+__global__ void __launch_bounds__(256)
+BandGather(const BandInfo *__restrict__ infos, const BandState *__restrict__ tab,
+           const float *__restrict__ lp, int32_t C, float *__restrict__ by_state) {
+  __shared__ int32_t label_sh[kBandMaxStates];
+  const BandInfo f = infos[blockIdx.y];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int32_t r0 = blockIdx.x * kGatherRows, r1 = min(r0 + kGatherRows, f.frames), S = f.num_states;
+  if (S == 0 || r0 >= r1) return;
+  for (int32_t s = threadIdx.x; s < S; s += 256) label_sh[s] = tab[f.state_off + s].label;
+  __syncthreads();
+  for (int32_t r = r0 + warp; r < r1; r += 8) {
+    const float *in = lp + (int64_t)(f.lp_row + r) * C;
+    float *out = by_state + f.grid_off + (int64_t)r * f.pitch;
+    for (int32_t s0 = lane; s0 < S; s0 += 256) {
+      float x[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const int32_t s = s0 + 32 * k, label = s < S ? label_sh[s] : -1;
+        x[k] = label >= 0 && label < C ? __ldg(in + label) : -INFINITY;
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (s0 + 32 * k < S) out[s0 + 32 * k] = x[k];
+    }
+  }
+}
+
+// kByState: `lp` holds scores by state (BandGather) in the layout of the grids instead of
+// log-prob rows of C columns: a thread reads its states' scores in one word.  With 5000 columns
+// the copies of whole rows bounded the kernel (170 us for 500 frames); by state it takes 43,
+// and BandGather 36.
+template <bool kByState>
+__global__ void __launch_bounds__(64 * kVitMaxWarps, 1)
 BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ tab,
             const float *__restrict__ lp, int32_t C, float *__restrict__ vf,
             float *__restrict__ vb, int32_t F, int32_t nbatch, int32_t slot_floats,
@@ -229,10 +294,11 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int32_t S = f.num_states, T = f.frames, pitch = f.pitch;
   if (S == 0) return;
-  const int32_t H = F >> 1;         // lanes that recompute the neighbour's states
+  const int32_t H = 2 * F / K;      // lanes that recompute the neighbour's states
   const int32_t own = 32 - H;       // lanes whose states this warp owns
+  const int32_t width = kByState ? pitch : C;              // floats of a row
   float *ring = reinterpret_cast<float *>(smem_raw);       // [nbatch][slot_floats]: F rows
-  float *xch = ring + (size_t)nbatch * slot_floats;        // [2][xch_pad], state s at s + 4H
+  float *xch = ring + (size_t)nbatch * slot_floats;        // [2][xch_pad], state s at s + 2F
   if (tid == 0) {
     for (int st = 0; st < nbatch; ++st) MbarInit(&full[st], 1);
     MbarInitFence();
@@ -241,11 +307,13 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
   for (int32_t k = tid; k < 2 * xch_pad; k += blockDim.x) xch[k] = -INFINITY;
   __syncthreads();
   const int32_t num_batches = (T + F - 1) / F;
-  const float *lp0 = lp + (int64_t)f.lp_row * C;
+  const float *lp0 = kByState ? lp + f.grid_off : lp + (int64_t)f.lp_row * C;
   // A row may start anywhere (C need not be a multiple of four): a batch is copied from the
   // 16-byte boundary at or before its first element to the one at or after its last.
   const uint32_t lp0_words = (uint32_t)(reinterpret_cast<uintptr_t>(lp0) >> 2);
-  auto words_off = [&](int32_t r) { return (int32_t)((lp0_words + (uint32_t)r * (uint32_t)C) & 3u); };
+  auto words_off = [&](int32_t r) {
+    return kByState ? 0 : (int32_t)((lp0_words + (uint32_t)r * (uint32_t)width) & 3u);
+  };
   int32_t issued = 0;
   auto issue = [&]() {  // thread 0 only: the rows of the next batch into the next slot
     if (issued >= num_batches) return;
@@ -254,10 +322,10 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
     const int32_t r0 = dir == 0 ? q * F : max(T - (q + 1) * F, 0);
     const int32_t r1 = dir == 0 ? min((q + 1) * F, T) : T - q * F;
     const int32_t off = words_off(r0);
-    const unsigned bytes = (((unsigned)(r1 - r0) * (unsigned)C + (unsigned)off + 3u) & ~3u) * 4u;
+    const unsigned bytes = (((unsigned)(r1 - r0) * (unsigned)width + (unsigned)off + 3u) & ~3u) * 4u;
     const int32_t slot = q % nbatch;
     MbarArriveExpectTx(&full[slot], bytes);
-    BulkCopyG2S(ring + (size_t)slot * slot_floats, lp0 + (int64_t)r0 * C - off, bytes,
+    BulkCopyG2S(ring + (size_t)slot * slot_floats, lp0 + (int64_t)r0 * width - off, bytes,
                 &full[slot]);
     ++issued;
   };
@@ -270,21 +338,21 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
   const bool stores = mine && s0 < pitch;
   float *grid = (dir == 0 ? vf : vb) + f.grid_off + s0;
   bool late = false;
-  float v[K] = {0.0f, 0.0f, 0.0f, 0.0f};
+  float v[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) v[k] = 0.0f;
   // exchange of boundary states: owners publish, recomputing lanes pick up
+  const int32_t lead = 2 * F;
   auto exchange = [&](int32_t which) {
-    float *x = xch + (size_t)which * xch_pad + 4 * H;
-    if (mine && s0 < xch_pad - 4 * H - 3)
-      *reinterpret_cast<float4 *>(x + s0) = make_float4(v[0], v[1], v[2], v[3]);
+    float *x = xch + (size_t)which * xch_pad + lead;
+    if (mine && s0 < xch_pad - lead - (K - 1)) VitStore<K>(x + s0, v);
     __syncthreads();
-    if (!mine && s0 + 4 * H >= 0 && s0 < xch_pad - 4 * H - 3) {
-      const float4 t = *reinterpret_cast<const float4 *>(x + s0);
-      v[0] = t.x;
-      v[1] = t.y;
-      v[2] = t.z;
-      v[3] = t.w;
-    }
+    if (!mine && s0 + lead >= 0 && s0 < xch_pad - lead - (K - 1)) VitLoad<K>(x + s0, v);
   };
+  // The values next to a lane's states come from its neighbour.  What lane 0 (forward) or 31
+  // (backward) gets instead is not a neighbour's: either it recomputes another warp's states,
+  // of which the outermost two are lost per frame, or there is no such state and every score
+  // into it is -inf.
   if (dir == 0) {
     // ---- forward: state s from s, s - 1, s - 2 ----------------------------------
     float w0[K], w1[K], w2[K];     // on the frames; -inf for a state whose label has no column
@@ -310,7 +378,25 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
       }
       v[k] = s == 0 ? 0.0f : -INFINITY;
     }
-    if (stores) *reinterpret_cast<float4 *>(grid) = make_float4(v[0], v[1], v[2], v[3]);
+    if (kByState) col[0] = min(max(s0, 0), pitch - K);
+    if (stores) VitStore<K>(grid, v);
+    auto step = [&](const float (&a0)[K], const float (&a1)[K], const float (&a2)[K],
+                    const float (&x)[K]) {
+      const float h1 = __shfl_up_sync(kAll, v[K - 1], 1), h2 = __shfl_up_sync(kAll, v[K - 2], 1);
+      float nv[K];
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        const float a = v[k];
+        const float b = k >= 1 ? v[k >= 1 ? k - 1 : 0] : h1;
+        const float c = k >= 2 ? v[k >= 2 ? k - 2 : 0] : (k == 1 ? h1 : h2);
+        nv[k] = __fadd_rn(
+            Max3(__fadd_rn(a, a0[k]), __fadd_rn(b, a1[k]), __fadd_rn(c, a2[k])), x[k]);
+      }
+#pragma unroll
+      for (int k = 0; k < K; ++k) v[k] = nv[k];
+      grid += pitch;
+      if (stores) VitStore<K>(grid, v);
+    };
     int32_t xpar = 0;
     for (int32_t q = 0; q < num_batches; ++q) {
       const int32_t slot = q % nbatch;
@@ -323,43 +409,24 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
       const int32_t nf = min(F, T - q * F);
       const float *rowbuf = ring + (size_t)slot * slot_floats + words_off(q * F);
 #pragma unroll 4
-      for (int32_t r = 0; r < nf; ++r, rowbuf += C) {
+      for (int32_t r = 0; r < nf; ++r, rowbuf += width) {
         float x[K];
+        if (kByState) {
+          VitLoad<K>(rowbuf + col[0], x);
+        } else {
 #pragma unroll
-        for (int k = 0; k < K; ++k) x[k] = rowbuf[col[k]];
-        float h1 = __shfl_up_sync(kAll, v[K - 1], 1), h2 = __shfl_up_sync(kAll, v[K - 2], 1);
-        if (lane == 0) h1 = h2 = -INFINITY;
-        float nv[K];
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-          const float a = v[k];
-          const float b = k >= 1 ? v[k >= 1 ? k - 1 : 0] : h1;
-          const float c = k >= 2 ? v[k >= 2 ? k - 2 : 0] : (k == 1 ? h1 : h2);
-          const float m = Max3(__fadd_rn(a, w0[k]), __fadd_rn(b, w1[k]), __fadd_rn(c, w2[k]));
-          nv[k] = __fadd_rn(m, x[k]);
+          for (int k = 0; k < K; ++k) x[k] = rowbuf[col[k]];
         }
-#pragma unroll
-        for (int k = 0; k < K; ++k) v[k] = nv[k];
-        grid += pitch;
-        if (stores) *reinterpret_cast<float4 *>(grid) = make_float4(v[0], v[1], v[2], v[3]);
+        step(w0, w1, w2, x);
       }
     }
     // the implied final row: level T + 1
     exchange(xpar);
     {
-      float h1 = __shfl_up_sync(kAll, v[K - 1], 1), h2 = __shfl_up_sync(kAll, v[K - 2], 1);
-      if (lane == 0) h1 = h2 = -INFINITY;
-      float nv[K];
+      float x[K];
 #pragma unroll
-      for (int k = 0; k < K; ++k) {
-        const float a = v[k];
-        const float b = k >= 1 ? v[k >= 1 ? k - 1 : 0] : h1;
-        const float c = k >= 2 ? v[k >= 2 ? k - 2 : 0] : (k == 1 ? h1 : h2);
-        const float m = Max3(__fadd_rn(a, f0[k]), __fadd_rn(b, f1[k]), __fadd_rn(c, f2[k]));
-        nv[k] = __fadd_rn(m, 0.0f);
-      }
-      grid += pitch;
-      if (stores) *reinterpret_cast<float4 *>(grid) = make_float4(nv[0], nv[1], nv[2], nv[3]);
+      for (int k = 0; k < K; ++k) x[k] = 0.0f;
+      step(f0, f1, f2, x);
     }
   } else {
     // ---- backward: state s to s, s + 1, s + 2 -----------------------------------
@@ -387,27 +454,37 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
           else if (t.label == -1) fo[k - d >= 0 ? k - d : 0][d] = t.w[d];
         }
     }
+    if (kByState) {  // (states at and behind S score -inf: any column of the row will do)
+      col[0] = min(s0, pitch - K);
+      col[1] = min(s0 + K, pitch - 2);
+    }
 #pragma unroll
     for (int k = 0; k < K; ++k) v[k] = (s0 + k == S - 1) ? 0.0f : -INFINITY;
     grid += (int64_t)(T + 1) * pitch;
-    if (stores) *reinterpret_cast<float4 *>(grid) = make_float4(v[0], v[1], v[2], v[3]);
-    {  // level T from level T + 1 through the implied final row (nothing to exchange yet:
-       // only the final state is not -inf, and every lane knows it)
-      float g1 = __shfl_down_sync(kAll, v[0], 1), g2 = __shfl_down_sync(kAll, v[1], 1);
-      if (lane == 31) g1 = g2 = -INFINITY;
+    if (stores) VitStore<K>(grid, v);
+    auto step = [&](const float (&w)[K][3], const float (&x)[K + 2]) {
+      const float g1 = __shfl_down_sync(kAll, v[0], 1), g2 = __shfl_down_sync(kAll, v[1], 1);
       float nv[K];
 #pragma unroll
       for (int k = 0; k < K; ++k) {
         const float a = v[k];
         const float b = k + 1 < K ? v[k + 1 < K ? k + 1 : 0] : g1;
         const float c = k + 2 < K ? v[k + 2 < K ? k + 2 : 0] : (k + 2 == K ? g1 : g2);
-        nv[k] = Max3(__fadd_rn(__fadd_rn(a, fo[k][0]), 0.0f), __fadd_rn(__fadd_rn(b, fo[k][1]), 0.0f),
-                     __fadd_rn(__fadd_rn(c, fo[k][2]), 0.0f));
+        nv[k] = Max3(__fadd_rn(__fadd_rn(a, w[k][0]), x[k]),
+                     __fadd_rn(__fadd_rn(b, w[k][1]), x[k + 1]),
+                     __fadd_rn(__fadd_rn(c, w[k][2]), x[k + 2]));
       }
 #pragma unroll
       for (int k = 0; k < K; ++k) v[k] = nv[k];
       grid -= pitch;
-      if (stores) *reinterpret_cast<float4 *>(grid) = make_float4(v[0], v[1], v[2], v[3]);
+      if (stores) VitStore<K>(grid, v);
+    };
+    {  // level T from level T + 1 through the implied final row (nothing to exchange yet:
+       // only the final state is not -inf, and every lane knows it)
+      float x[K + 2];
+#pragma unroll
+      for (int k = 0; k < K + 2; ++k) x[k] = 0.0f;
+      step(fo, x);
     }
     int32_t xpar = 0;
     for (int32_t q = 0; q < num_batches; ++q) {
@@ -418,28 +495,23 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
       if (q > 0 && tid == 0 && !late) issue();
       const int32_t r1 = T - q * F, r0 = max(T - (q + 1) * F, 0);
       const float *rowbuf =
-          ring + (size_t)slot * slot_floats + words_off(r0) + (size_t)(r1 - 1 - r0) * C;
+          ring + (size_t)slot * slot_floats + words_off(r0) + (size_t)(r1 - 1 - r0) * width;
 #pragma unroll 4
-      for (int32_t r = r1 - 1; r >= r0; --r, rowbuf -= C) {  // level r from level r + 1
+      for (int32_t r = r1 - 1; r >= r0; --r, rowbuf -= width) {  // level r from level r + 1
         float x[K + 2];
+        if (kByState) {
+          float lo[K], hi[2];
+          VitLoad<K>(rowbuf + col[0], lo);
+          VitLoad<2>(rowbuf + col[1], hi);
 #pragma unroll
-        for (int k = 0; k < K + 2; ++k) x[k] = rowbuf[col[k]];
-        float g1 = __shfl_down_sync(kAll, v[0], 1), g2 = __shfl_down_sync(kAll, v[1], 1);
-        if (lane == 31) g1 = g2 = -INFINITY;
-        float nv[K];
+          for (int k = 0; k < K; ++k) x[k] = lo[k];
+          x[K] = hi[0];
+          x[K + 1] = hi[1];
+        } else {
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-          const float a = v[k];
-          const float b = k + 1 < K ? v[k + 1 < K ? k + 1 : 0] : g1;
-          const float c = k + 2 < K ? v[k + 2 < K ? k + 2 : 0] : (k + 2 == K ? g1 : g2);
-          nv[k] = Max3(__fadd_rn(__fadd_rn(a, wo[k][0]), x[k]),
-                       __fadd_rn(__fadd_rn(b, wo[k][1]), x[k + 1]),
-                       __fadd_rn(__fadd_rn(c, wo[k][2]), x[k + 2]));
+          for (int k = 0; k < K + 2; ++k) x[k] = rowbuf[col[k]];
         }
-#pragma unroll
-        for (int k = 0; k < K; ++k) v[k] = nv[k];
-        grid -= pitch;
-        if (stores) *reinterpret_cast<float4 *>(grid) = make_float4(v[0], v[1], v[2], v[3]);
+        step(wo, x);
       }
     }
   }
@@ -496,8 +568,8 @@ static size_t BandPrepSmem(int32_t max_states) {
 __global__ void __launch_bounds__(32 * kPrepWarps, 3)
 BandPrep(const BandInfo *__restrict__ infos, const int32_t *__restrict__ a_row_splits2,
          const BandState *__restrict__ tab, const BandArc *__restrict__ tabf,
-         const float *__restrict__ lp, int32_t C, const float *__restrict__ vf,
-         const float *__restrict__ vb, float beam, BandItem *__restrict__ items,
+         const float *__restrict__ lp, int32_t C, const float *__restrict__ by_state,
+         const float *__restrict__ vf, const float *__restrict__ vb, float beam, BandItem *__restrict__ items,
          BandFactor *__restrict__ factors, int2 *__restrict__ lists,
          int32_t *__restrict__ chunk_r, unsigned long long *__restrict__ totals,
          int32_t *__restrict__ unfit, int32_t count_arcs) {
@@ -635,7 +707,10 @@ BandPrep(const BandInfo *__restrict__ infos, const int32_t *__restrict__ a_row_s
       row[u] = k + 1;
       own[u] = l < b;
       n[u] = k <= b - a && l <= T + 1 ? n_sh[row[u]] : 0;
-      xrow[u] = l >= 1 && l <= T ? lp0 + (int64_t)(l - 1) * C : nullptr;
+      xrow[u] = nullptr;
+      if (l >= 1 && l <= T)
+        xrow[u] = by_state != nullptr ? by_state + f.grid_off + (int64_t)(l - 1) * pitch
+                                      : lp0 + (int64_t)(l - 1) * C;
       brow[u] = bg + (int64_t)l * pitch;
       frow[u] = fg + (int64_t)(l - 1) * pitch;
       level[u] = reinterpret_cast<char *>(factors + f.grid_off + (int64_t)a * pitch + k * padded) +
@@ -661,10 +736,12 @@ BandPrep(const BandInfo *__restrict__ infos, const int32_t *__restrict__ a_row_s
         kept[u] = src[u] = 0;
         x[u] = bc[u] = 0.0f;
         if (in[u] && row[u] + a >= 2) {
-          if (xrow[u] != nullptr)
-            x[u] = st[u].label >= 0 && st[u].label < C ? __ldg(xrow[u] + st[u].label) : -INFINITY;
-          else  // the implied final row
+          if (xrow[u] == nullptr)  // the implied final row
             x[u] = st[u].label == -1 ? 0.0f : -INFINITY;
+          else if (by_state != nullptr)
+            x[u] = xrow[u][s[u]];
+          else
+            x[u] = st[u].label >= 0 && st[u].label < C ? __ldg(xrow[u] + st[u].label) : -INFINITY;
           bc[u] = brow[u][s[u]];
 #pragma unroll
           for (int d = 0; d < 3; ++d) {
@@ -1617,10 +1694,11 @@ struct BandLayout {
   long long arc_frames = 0;
   int32_t max_states = 0, max_frames = 0, max_rows = 0;
   int32_t vit_threads = 32, vit_frames = 0, vit_batches = 0, vit_slot = 0, xch_pad = 0;
+  bool by_state = false;
   int32_t first_row = 0;
   int32_t st_pad = 0, lv_pad = 0;
   size_t chain_smem = 0, exact_smem = 0, viterbi_smem = 0, prep_smem = 0;
-  size_t off_infos, off_vf, off_vb, off_items, off_factors, off_lists, off_chunk_r, off_am, off_ae,
+  size_t off_infos, off_vf, off_vb, off_by_state, off_items, off_factors, off_lists, off_chunk_r, off_am, off_ae,
       off_bm, off_be, off_a_scale, off_b_scale, off_total, off_unfit, off_totals, off_status,
       total_bytes;  // off_status = off_totals + 40
   bool ok = true;
@@ -1697,24 +1775,32 @@ static int32_t MakeBandLayout(const k2b200_band_loss_args *a, BandLayout *L) {
     L->first_row = L->infos[order[0]].lp_row;
     if (a->log_prob_rows >= INT32_MAX) L->exclusive_rows = false;
   }
-  // BandViterbi: frames per batch (even, at most 16) so that at least two batches of rows
-  // fit in shared memory, up to three batches within ~100 KB so that two CTAs share an SM
+  // BandViterbi: rows by state when the log-prob rows are much wider than the states of a
+  // graph: a CTA takes in 60 bytes per ns, so beyond 1024 columns a row takes longer to arrive
+  // than to walk, and a row by state is read twice instead of the row of the log-probs.  Also
+  // where two batches of two rows do not fit.
+  // Else frames per batch (even, at most 16) so that at least two batches of rows fit in
+  // shared memory, up to three within ~100 KB so that two CTAs share an SM.
   {
-    const size_t row_bytes = sizeof(float) * (size_t)a->num_classes;
-    int32_t F = 16;
+    const size_t max_pitch = 32 * ((size_t)L->max_states / 32 + 1);
+    const size_t C = (size_t)a->num_classes;
+    L->by_state = (C > 1024 && C > 3 * max_pitch) ||
+                  4 * C * sizeof(float) > kBandSmemBudget - 16384;
+    int32_t F = L->by_state ? kVitFramesByState : 16;
+    const size_t row_bytes = sizeof(float) * (L->by_state ? max_pitch : C);
     while (F > 2 && 2 * F * row_bytes > kBandSmemBudget - 16384) F >>= 1;
     L->vit_frames = F;
-    L->vit_slot = (int32_t)(((size_t)F * a->num_classes + 6 + 3) & ~(size_t)3);
+    L->vit_slot = (int32_t)((F * row_bytes / sizeof(float) + 6 + 3) & ~(size_t)3);
     L->vit_batches = (int32_t)std::max<size_t>(
         2, std::min<size_t>(3, (100 * 1024) / std::max<size_t>(F * row_bytes, 1)));
-    const int32_t own_states = (32 - F / 2) * kVitK;
+    const int32_t own_states = (32 - 2 * F / kVitK) * kVitK;
     const int32_t warps = std::max(1, CeilDiv(std::max(L->max_states, 1), own_states));
     L->vit_threads = 32 * warps;
-    L->xch_pad = (warps * own_states + 4 * kVitK * (F / 2) + 3) & ~3;
+    L->xch_pad = (warps * own_states + 8 * F + 3) & ~3;
     L->viterbi_smem = sizeof(float) * ((size_t)L->vit_batches * L->vit_slot + 2 * (size_t)L->xch_pad);
-    if (warps > kVitMaxWarps || 2 * F * row_bytes > kBandSmemBudget - 16384) {
+    if (warps > kVitMaxWarps) {
       L->ok = false;
-      L->why = "too many states or classes for the Viterbi kernel";
+      L->why = "too many states for the Viterbi kernel";
     }
   }
   L->st_pad = ((L->max_states + 4) + 15) & ~15;
@@ -1745,6 +1831,7 @@ static int32_t MakeBandLayout(const k2b200_band_loss_args *a, BandLayout *L) {
   L->off_infos = take(sizeof(BandInfo) * a->num_fsas);
   L->off_vf = take(sizeof(float) * (size_t)grid);
   L->off_vb = take(sizeof(float) * (size_t)grid);
+  L->off_by_state = take(L->by_state ? sizeof(float) * (size_t)grid : 0);
   L->off_items = take(sizeof(BandItem) * (size_t)grid);
   L->off_lists = take(sizeof(int2) * (size_t)levels);
   L->off_chunk_r = take(sizeof(int32_t) * (size_t)levels);
@@ -1932,16 +2019,25 @@ int32_t k2b200_band_loss_forward_reduce(const k2b200_band_loss_args *args, void 
     NotePhaseKernel(kPhaseViterbi, "BandViterbi");
     K2B_CUDA_OK(cudaFuncSetAttribute(BandPrep, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)L.prep_smem));
-    K2B_CUDA_OK(cudaFuncSetAttribute(BandViterbi, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    const BandInfo *infos = reinterpret_cast<const BandInfo *>(ws + L.off_infos);
+    const BandState *tab = reinterpret_cast<const BandState *>(args->band_states);
+    if (L.by_state && L.max_frames > 0) {
+      dim3 grid(CeilDiv(L.max_frames, kGatherRows), args->num_fsas);
+      { BandGather<<<grid, 256, 0, stream>>>(infos, tab, args->log_probs, args->num_classes,
+                                             reinterpret_cast<float *>(ws + L.off_by_state));
+        NoteLaunch(); }
+    }
+    auto kernel = L.by_state ? BandViterbi<true> : BandViterbi<false>;
+    K2B_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)L.viterbi_smem));
     dim3 grid(2, args->num_fsas);
-    { BandViterbi<<<grid, L.vit_threads, L.viterbi_smem, stream>>>(
-        reinterpret_cast<const BandInfo *>(ws + L.off_infos),
-        reinterpret_cast<const BandState *>(args->band_states), args->log_probs,
+    { kernel<<<grid, L.vit_threads, L.viterbi_smem, stream>>>(
+        infos, tab,
+        L.by_state ? reinterpret_cast<const float *>(ws + L.off_by_state) : args->log_probs,
         args->num_classes, reinterpret_cast<float *>(ws + L.off_vf),
         reinterpret_cast<float *>(ws + L.off_vb), L.vit_frames, L.vit_batches, L.vit_slot,
-        L.xch_pad,
-        CopyWaitLimit(), reinterpret_cast<int32_t *>(ws + L.off_status)); NoteLaunch(); }
+        L.xch_pad, CopyWaitLimit(), reinterpret_cast<int32_t *>(ws + L.off_status));
+      NoteLaunch(); }
     K2B_CUDA_OK(cudaGetLastError());
   }
   // The lattice is never built, but its size still decides the beam
@@ -1973,7 +2069,9 @@ int32_t k2b200_band_loss_forward_reduce(const k2b200_band_loss_args *args, void 
           reinterpret_cast<const BandInfo *>(ws + L.off_infos), args->a_row_splits2,
           reinterpret_cast<const BandState *>(args->band_states),
           reinterpret_cast<const BandArc *>(args->band_arcs), args->log_probs,
-          args->num_classes, reinterpret_cast<const float *>(ws + L.off_vf),
+          args->num_classes,
+          L.by_state ? reinterpret_cast<const float *>(ws + L.off_by_state) : nullptr,
+          reinterpret_cast<const float *>(ws + L.off_vf),
           reinterpret_cast<const float *>(ws + L.off_vb), beam,
           reinterpret_cast<BandItem *>(ws + L.off_items),
           reinterpret_cast<BandFactor *>(ws + L.off_factors),
