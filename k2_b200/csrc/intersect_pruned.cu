@@ -19,6 +19,12 @@
 // no kernel waits on another.  States and arcs of all frames of a sequence live in
 // one arena, frame after frame, so the pruned result is already in lattice order and
 // the output pass is a copy.
+//
+// A frame expands five to ten times the arcs that end in a state it creates, so the expanded
+// arcs live in a scratch region at the far end of the arena and only those that enter a state
+// are moved into the frame's part of it.  Every warp of the team owns a contiguous range of
+// the frame's arcs: what it counts and lists stays in order, and one exchange of per-warp
+// sums numbers a whole frame.
 #include <algorithm>
 #include <climits>
 #include <cmath>
@@ -67,9 +73,10 @@ struct SearchArgs {
   float *st_bwd;
   int32_t *arc_aidx, *arc_dest;
   float *arc_ll, *arc_end;
-  uint8_t *arc_keep;
+  int32_t *list_a, *list_b;    // scratch, like the arcs
   unsigned long long *winner;  // [num_seqs * a_states] (shared) or [a_states]
-  int32_t *frame_s0, *frame_a0;  // [num_seqs][T + 2]
+  int32_t *frame_s0, *frame_a0, *frame_n0, *frame_m0;  // [num_seqs][T + 2], the last two scratch
+  int32_t *warp_first;         // [num_seqs][kTeamWarps]
   int32_t *seq_out;           // [num_seqs][kSeqOut]: states, arcs, extra final state, status,
                               // most states of a frame, most arcs leaving one
 };
@@ -79,22 +86,24 @@ enum : int32_t { kSeqOk = 0, kSeqOverflow = 1, kSeqManyFinal = 2 };
 
 // The CTAs that work on one sequence: a thread-block cluster (of one CTA when there are
 // enough sequences to fill the GPU).  Arena data is exchanged through global memory,
-// ordered by the cluster barrier; scan totals and maxima through distributed shared
-// memory.  Item k of a pass is handled by team thread k mod team size, and the CTAs
-// of a cluster are always co-resident, so the barrier cannot wait for an unscheduled
-// CTA.
+// ordered by the cluster barrier; sums and maxima through distributed shared memory: a CTA
+// writes its own to every CTA before the barrier and all are read locally behind it.  The CTAs
+// of a cluster are always co-resident, so the barrier cannot wait for an unscheduled CTA.
+constexpr int kMaxTeam = 8;
+constexpr int kWarps = kSearchThreads / 32;
+constexpr int kTeamWarps = kMaxTeam * kWarps;
+// Slots of exchanged values.  A slot is written again only when another exchange, with its
+// barrier, lies in between: the two slots of the thread scans alternate.
+enum : int32_t { kSlotMax = 0, kSlotNew, kSlotKept, kSlotWindow, kSlotScan, kSlots = kSlotScan + 2 };
+constexpr int kMaxRow = 8192;        // columns of a row of scores that are kept in shared memory
+constexpr int kMarkWords = 8192;     // words of the set of new states: 2^18 graph states
 struct Shared {
-  int32_t scan[65];
-  float fmax[33];
-  unsigned long long scan2[65];
-  unsigned long long team_l[2];
-  int32_t team_i[2];  // this CTA's contribution to the team-wide scan / or
-  float team_f[2];    // ... and to the team-wide max; two slots used alternately
-  int32_t phase_i, phase_f, phase_l;
-  int32_t new_s0[kWindow], new_a0[kWindow];  // used by the first thread of the team only
-  int32_t wbest[kSearchThreads / 32][32], wcnt[kSearchThreads / 32][32];  // per warp
-  float cutoff;
-  float beam;
+  unsigned long long cta_val[kSlots][kMaxTeam];
+  unsigned long long warp_val[kWarps], warp_ex[kWarps];
+  int4 rec[kWarps][32];                           // per warp: the states whose arcs it walks
+  int32_t wbest[kWarps][32], wcnt[kWarps][32];
+  uint32_t mark[kMarkWords];
+  float row[kMaxRow];
   int32_t most_states, most_arcs;
 };
 
@@ -103,144 +112,82 @@ struct Team {
   Shared *sh;
   int32_t rank, size;     // this CTA within the cluster
   int32_t tid, threads;   // this thread within the team
+  int32_t warp, warps;    // this warp within the team
+  mutable int32_t phase;
 
-  __device__ Team(Shared *shared) : cluster(cg::this_cluster()), sh(shared) {
+  __device__ Team(Shared *shared) : cluster(cg::this_cluster()), sh(shared), phase(0) {
     rank = (int32_t)cluster.block_rank();
     size = (int32_t)cluster.num_blocks();
     tid = rank * kSearchThreads + (int32_t)threadIdx.x;
     threads = size * kSearchThreads;
+    warp = tid >> 5;
+    warps = threads >> 5;
   }
   __device__ __forceinline__ void Sync() const {
     if (size == 1) __syncthreads(); else cluster.sync();
   }
 
-  // exclusive scan of one int per team thread; every thread gets the total
-  __device__ int32_t Scan(int32_t v, int32_t *total) const {
-    int32_t *s = sh->scan;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int32_t inc = v;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      int32_t o = __shfl_up_sync(0xffffffffu, inc, d);
-      if (lane >= d) inc += o;
-    }
-    if (lane == 31) s[warp] = inc;
+  // Exclusive sum over the warps of the team of a value per warp (two counts packed into
+  // it must not overflow); the barrier inside also orders the global writes made before.
+  __device__ unsigned long long ScanWarps(int32_t slot, unsigned long long v,
+                                          unsigned long long *total) const {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (lane == 0) sh->warp_val[w] = v;
     __syncthreads();
-    if (warp == 0) {
-      int32_t w = s[lane];
-      int32_t winc = w;
+    if (w == 0) {
+      const unsigned long long x = sh->warp_val[lane];
+      unsigned long long inc = x;
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1) {
-        int32_t o = __shfl_up_sync(0xffffffffu, winc, d);
-        if (lane >= d) winc += o;
+        const unsigned long long o = __shfl_up_sync(0xffffffffu, inc, d);
+        if (lane >= d) inc += o;
       }
-      s[32 + lane] = winc - w;
-      if (lane == 31) s[64] = winc;
+      sh->warp_ex[lane] = inc - x;
+      const unsigned long long all = __shfl_sync(0xffffffffu, inc, 31);
+      if (lane < size) *cluster.map_shared_rank(&sh->cta_val[slot][rank], lane) = all;
     }
-    __syncthreads();
-    int32_t ex = s[32 + warp] + inc - v;
-    int32_t all = s[64];
-    if (size == 1) {
-      __syncthreads();  // s is reused by the next call
-      *total = all;
-      return ex;
-    }
-    // a slot is rewritten two calls later, after a cluster barrier that every CTA
-    // reaches only when it has read the slot
-    const int32_t slot = sh->phase_i & 1;
-    if (threadIdx.x == 0) sh->team_i[slot] = all;
-    cluster.sync();
-    int32_t before = 0, sum = 0;
+    Sync();
+    unsigned long long before = 0, sum = 0;
     for (int32_t r = 0; r < size; ++r) {
-      const int32_t x = *cluster.map_shared_rank(&sh->team_i[slot], r);
+      const unsigned long long x = sh->cta_val[slot][r];
       sum += x;
       if (r < rank) before += x;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) sh->phase_i += 1;
-    __syncthreads();
     *total = sum;
-    return before + ex;
+    return before + sh->warp_ex[w];
   }
 
-  // the same for a pair of counts, both below 2^31 in total, packed into 64 bits
-  __device__ int32_t Scan2(int32_t a, int32_t b, int32_t *ex_b, int32_t *total_a,
-                           int32_t *total_b) const {
-    unsigned long long *s = sh->scan2;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned long long v = (unsigned long long)(uint32_t)a | ((unsigned long long)(uint32_t)b << 32);
-    unsigned long long inc = v;
+  // exclusive scan of one count per team thread; every thread gets the total
+  __device__ int32_t Scan(int32_t v, int32_t *total) const {
+    const int lane = threadIdx.x & 31;
+    int32_t inc = v;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-      unsigned long long o = __shfl_up_sync(0xffffffffu, inc, d);
+      const int32_t o = __shfl_up_sync(0xffffffffu, inc, d);
       if (lane >= d) inc += o;
     }
-    if (lane == 31) s[warp] = inc;
-    __syncthreads();
-    if (warp == 0) {
-      unsigned long long w = s[lane];
-      unsigned long long winc = w;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        unsigned long long o = __shfl_up_sync(0xffffffffu, winc, d);
-        if (lane >= d) winc += o;
-      }
-      s[32 + lane] = winc - w;
-      if (lane == 31) s[64] = winc;
-    }
-    __syncthreads();
-    unsigned long long ex = s[32 + warp] + inc - v;
-    unsigned long long all = s[64];
-    if (size == 1) {
-      __syncthreads();
-    } else {
-      const int32_t slot = sh->phase_l & 1;
-      if (threadIdx.x == 0) sh->team_l[slot] = all;
-      cluster.sync();
-      unsigned long long before = 0, sum = 0;
-      for (int32_t r = 0; r < size; ++r) {
-        const unsigned long long x = *cluster.map_shared_rank(&sh->team_l[slot], r);
-        sum += x;
-        if (r < rank) before += x;
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) sh->phase_l += 1;
-      __syncthreads();
-      ex += before;
-      all = sum;
-    }
-    *ex_b = (int32_t)(ex >> 32);
-    *total_a = (int32_t)(all & 0xffffffffu);
-    *total_b = (int32_t)(all >> 32);
-    return (int32_t)(ex & 0xffffffffu);
+    unsigned long long all;
+    const unsigned long long base = ScanWarps(
+        kSlotScan + (phase++ & 1), (unsigned long long)__shfl_sync(0xffffffffu, inc, 31), &all);
+    *total = (int32_t)all;
+    return (int32_t)base + inc - v;
   }
 
-  __device__ float Max(float v) const {
-    float *s = sh->fmax;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, d));
-    if (lane == 0) s[warp] = v;
+  // largest value of the team; the barrier inside orders global writes likewise
+  __device__ int32_t Max(int32_t v) const {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    v = __reduce_max_sync(0xffffffffu, v);
+    if (lane == 0) sh->warp_val[w] = (unsigned long long)(uint32_t)v;
     __syncthreads();
-    if (warp == 0) {
-      float w = s[lane];
-#pragma unroll
-      for (int d = 16; d > 0; d >>= 1) w = fmaxf(w, __shfl_xor_sync(0xffffffffu, w, d));
-      if (lane == 0) s[32] = w;
+    if (w == 0) {
+      v = __reduce_max_sync(0xffffffffu, (int32_t)(uint32_t)sh->warp_val[lane]);
+      if (lane < size)
+        *cluster.map_shared_rank(&sh->cta_val[kSlotMax][rank], lane) = (unsigned long long)(uint32_t)v;
     }
-    __syncthreads();
-    float r = s[32];
-    const int32_t slot = sh->phase_f & 1;
-    if (threadIdx.x == 0) sh->team_f[slot] = r;
-    Sync();  // also orders the global writes made before the call
-    if (size > 1) {
-      for (int32_t k = 0; k < size; ++k)
-        r = fmaxf(r, *cluster.map_shared_rank(&sh->team_f[slot], k));
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) sh->phase_f += 1;
-    __syncthreads();
-    return r;
+    Sync();
+    v = (int32_t)(uint32_t)sh->cta_val[kSlotMax][0];
+    for (int32_t r = 1; r < size; ++r) v = max(v, (int32_t)(uint32_t)sh->cta_val[kSlotMax][r]);
+    return v;
   }
 
   // true when `v` is non-zero on any thread of the team
@@ -257,9 +204,9 @@ struct SeqView {
   float *st_bwd;
   int32_t *arc_aidx, *arc_dest;
   float *arc_ll, *arc_end;
-  uint8_t *arc_keep;
+  int32_t *list_a, *list_b;
   unsigned long long *winner;
-  int32_t *frame_s0, *frame_a0;
+  int32_t *frame_s0, *frame_a0, *frame_n0, *frame_m0, *warp_first;
 };
 
 __device__ __forceinline__ SeqView ViewOf(const SearchArgs &g, int32_t seq) {
@@ -275,12 +222,16 @@ __device__ __forceinline__ SeqView ViewOf(const SearchArgs &g, int32_t seq) {
   v.arc_dest = g.arc_dest + ao;
   v.arc_ll = g.arc_ll + ao;
   v.arc_end = g.arc_end + ao;
-  v.arc_keep = g.arc_keep + ao;
+  v.list_a = g.list_a + ao;
+  v.list_b = g.list_b + ao;
   // the reference's hash key is dest_state_idx01 + seq * stride with the stride 0
   // for per-sequence graphs (:118-127): the same index works for a direct table
   v.winner = g.winner + (g.a_stride ? 0 : (int64_t)seq * g.a_states);
   v.frame_s0 = g.frame_s0 + (int64_t)seq * (g.T + 2);
   v.frame_a0 = g.frame_a0 + (int64_t)seq * (g.T + 2);
+  v.frame_n0 = g.frame_n0 + (int64_t)seq * (g.T + 2);
+  v.frame_m0 = g.frame_m0 + (int64_t)seq * (g.T + 2);
+  v.warp_first = g.warp_first + (int64_t)seq * kTeamWarps;
   return v;
 }
 
@@ -309,10 +260,7 @@ __device__ float NextBeam(float dyn, float best, int32_t active, int32_t t, int3
   return dyn;
 }
 
-constexpr int kPer = 8;      // consecutive arcs per thread in the compaction pass
-constexpr int kPerScan = 8;  // ... and where the new states are numbered
-constexpr int kBatch = 4;    // arcs whose loads a thread issues together
-constexpr int kExpand = 2;   // ... in the arc expansion
+constexpr int kExpand = 4;   // groups of 32 arcs whose loads a warp issues together
 
 // Entries of the direct table that replaces the reference's hash: the frame in the
 // high word, so that entries of earlier frames lose against any entry of this frame
@@ -326,17 +274,96 @@ __device__ __forceinline__ unsigned long long StateEntry(int32_t t, int32_t j) {
   return ((unsigned long long)(uint32_t)(t + 1) << 32) | 0x80000000u | (uint32_t)j;
 }
 
-// One step of the search (GetArcs + PropagateForward, :778-1153): expands the na arcs
-// leaving the ns states of frame t at [s0, s0 + ns) - their arc ranges (st_arc0,
-// starting at a0) were laid out when the states were created - and creates the states
-// of frame t + 1 behind them, with their arc ranges.  Returns false when an arena is
-// full.  *ns_next / *na_next: states of frame t + 1 and the arcs leaving them.
+// Arcs that a warp of the team owns of a frame that expands `na`: a multiple of 32.
+__device__ __forceinline__ int32_t ArcsPerWarp(int32_t na, const Team &tm) {
+  return ((na + tm.warps - 1) / tm.warps + 31) & ~31;
+}
+// State k expands arcs [f, f + deg): where a warp's range starts among them, the warp's walk
+// over the states starts at k.
+__device__ __forceinline__ void SetWarpFirst(const SeqView &v, int32_t per_warp, int32_t k,
+                                             int32_t f, int32_t deg) {
+  for (int32_t w = (f + per_warp - 1) / per_warp; w * per_warp < f + deg; ++w) v.warp_first[w] = k;
+}
+
+// The scores of a row of the dense matrix into shared memory, when they fit.
+__device__ __forceinline__ void StageRow(const SearchArgs &g, const Team &tm, int32_t row) {
+  if (g.cols > kMaxRow || row >= g.rows) return;
+  const float *in = g.scores + (int64_t)row * g.cols;
+  for (int32_t c = threadIdx.x; c < g.cols; c += kSearchThreads) tm.sh->row[c] = in[c];
+}
+
+// 32 states whose arcs a warp walks as one flat range: lane j has state j's first arc f
+// (`end` where there is no state) and what goes with its arcs.  The records of the states
+// that have arcs go to shared memory in order; the record of arc p is found by counting the
+// states that start at or before it.
+struct ArcWalk {
+  const int4 *rec;
+  int32_t f;
+  bool nonempty;
+  int32_t before;  // states with arcs that start before the next group
+
+  __device__ __forceinline__ void Begin(int4 *recs, int32_t first, int32_t next, int4 mine,
+                                        int32_t start) {
+    const int lane = threadIdx.x & 31;
+    f = first;
+    nonempty = next > first;
+    const uint32_t ne = __ballot_sync(0xffffffffu, nonempty);
+    __syncwarp();  // the records before have been read
+    if (nonempty) recs[__popc(ne & ((1u << lane) - 1u))] = mine;
+    __syncwarp();
+    rec = recs;
+    before = __popc(__ballot_sync(0xffffffffu, nonempty && f < start));
+  }
+  // index of the record of arc pb + lane; groups of 32 arcs in order
+  __device__ __forceinline__ int32_t Next(int32_t pb) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t x = (uint32_t)(f - pb);
+    const uint32_t starts =
+        __reduce_or_sync(0xffffffffu, nonempty && x < 32u ? 1u << x : 0u);
+    const int32_t r = before + __popc(starts & (0xffffffffu >> (31 - lane))) - 1;
+    before += __popc(starts);
+    return r;
+  }
+};
+
+// One step of the search (GetArcs + PropagateForward, :778-1153): expands the na arcs leaving the
+// ns states of frame t at [s0, s0 + ns) - where each state's arcs start among them (st_cnt)
+// and where the warps start (warp_first) was laid out when the states were created - creates
+// the states of frame t + 1 behind them, with the layout of their arcs, and appends the arcs
+// that enter one of them to the arena at a0.  Returns false when an arena is full.
+// *ns_next / *na_next: states of frame t + 1 and the arcs leaving them; *kept: arcs appended.
+// beam: the search beam carried from frame to frame, the same in every thread.
+//
+// Bound by latency and by the rate of scattered accesses (about one per cycle and SM): the only
+// ones left per expanded arc are its graph arc, which arrives with its neighbours', and its
+// score, in shared memory; the table of states is looked at for the arcs above the cutoff, and
+// for those whose destination is in the set of new states.
 __device__ bool SearchStep(const SearchArgs &g, const SeqView &v, const Team &tm, int32_t seq,
                            int32_t t, int32_t final_t, int32_t row0, int32_t s0, int32_t ns,
-                           int32_t a0, int32_t na, int32_t *ns_next, int32_t *na_next) {
+                           int32_t a0, int32_t na, float *beam, int32_t *ns_next,
+                           int32_t *na_next, int32_t *kept) {
   Shared *sh = tm.sh;
+  constexpr unsigned kAll = 0xffffffffu;
   const float kNegInf = -INFINITY;
-  if ((int64_t)a0 + na > g.cap_a) return false;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  *ns_next = *na_next = *kept = 0;
+  if (na == 0) {  // no arc: the search of this sequence has ended, but for its beam
+    float cutoff;
+    *beam = NextBeam(*beam, kNegInf, ns, t, final_t, g, &cutoff);
+    for (int32_t k = tm.tid; k < ns; k += tm.threads) v.st_arc0[s0 + k] = a0;
+    __syncthreads();
+    StageRow(g, tm, row0 + t + 1);
+    tm.Sync();
+    return true;
+  }
+  const int64_t raw = (g.cap_a - na) & ~(int64_t)31;  // the expanded arcs' place
+  if (g.cap_a < na || raw < a0) return false;
+  int32_t *r_aidx = v.arc_aidx + raw, *r_dest = v.arc_dest + raw;
+  float *r_ll = v.arc_ll + raw, *r_end = v.arc_end + raw;
+  const int32_t per_warp = ArcsPerWarp(na, tm);
+  const int32_t lo = (int32_t)min((int64_t)tm.warp * per_warp, (int64_t)na);
+  const int32_t hi = min(lo + per_warp, na);
+  int32_t *list_a = v.list_a + raw + lo, *list_b = v.list_b + raw + lo;
 
   // graph of this sequence: its final state, for allow_partial (:861-871)
   const int32_t gi = seq * g.a_stride;
@@ -352,411 +379,496 @@ __device__ bool SearchStep(const SearchArgs &g, const SeqView &v, const Team &tm
     redirect = !tm.Any(has);
   }
 
-  // arcs: scores, destination (as a graph state) and the best end score (:858-905).
-  // A warp takes 32 consecutive states; its lanes walk the arcs of those states as
-  // one flat range and find the state of an arc by a search over the 32 range
-  // starts held in registers, so the work per lane is even whatever the out-degrees.
+  // ---- 1. arcs: scores, destination (as a graph state) and the best end score (:858-905).
   // (a row past the end is only asked for by a malformed graph whose arcs with
   // label -1 do not end in a state without arcs)
   const bool row_ok = row0 + t < g.rows;
-  const float *row = g.scores + (int64_t)(row_ok ? row0 + t : 0) * g.cols;
-  float best = kNegInf;
+  const bool staged = g.cols <= kMaxRow;
+  const float *row = staged ? sh->row : g.scores + (int64_t)(row_ok ? row0 + t : 0) * g.cols;
+  int32_t best = OrderedInt(kNegInf);
+  const int32_t k_first = lo < hi ? v.warp_first[tm.warp] : ns;
+  for (int32_t k0 = k_first; k0 < ns; k0 += 32) {
+    const int32_t k = k0 + lane;
+    int32_t f = na, as = 0, fwd = 0, ga0 = 0;
+    if (k < ns) {
+      f = v.st_cnt[s0 + k];
+      as = v.st_astate[s0 + k];
+      fwd = v.st_fwd[s0 + k];
+      ga0 = g.a_rs2[as];
+    }
+    int32_t next = __shfl_down_sync(kAll, f, 1);
+    if (lane == 31) next = k + 1 < ns ? v.st_cnt[s0 + k + 1] : na;
+    const int32_t start = max(lo, __shfl_sync(kAll, f, 0));
+    const int32_t chunk_end = __shfl_sync(kAll, next, 31), stop = min(hi, chunk_end);
+    ArcWalk walk;
+    walk.Begin(sh->rec[warp], f, next, make_int4(ga0 - f, as, fwd, 0), start);
+    for (int32_t pb = start; pb < stop; pb += 32 * kExpand) {
+      int4 rec[kExpand];
+      Arc arc[kExpand];
+#pragma unroll
+      for (int i = 0; i < kExpand; ++i) {
+        const int32_t p = pb + 32 * i + lane, r = walk.Next(pb + 32 * i);
+        if (p < stop) {
+          rec[i] = sh->rec[warp][r];
+          arc[i] = g.a_arcs[p + rec[i].x];
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < kExpand; ++i) {
+        const int32_t p = pb + 32 * i + lane;
+        if (p < stop) {
+          const uint32_t col = (uint32_t)(arc[i].label + 1);
+          float acoustic = (row_ok && col < (uint32_t)g.cols) ? row[col] : kNegInf;
+          int32_t dest = rec[i].y + arc[i].dest - arc[i].src;
+          if (redirect) {
+            dest = g_final;
+            acoustic = 0.0f;
+          }
+          const float ll = acoustic + arc[i].score;
+          const float end = OrderedFloat(rec[i].z) + ll;
+          r_aidx[p] = p + rec[i].x;
+          r_ll[p] = ll;
+          r_dest[p] = dest;
+          r_end[p] = end;
+          best = max(best, OrderedInt(end));
+        }
+      }
+    }
+    if (chunk_end >= hi) break;
+  }
   {
-    const int lane = threadIdx.x & 31;
-    const int32_t team_warp = tm.tid >> 5, team_warps = tm.threads >> 5;
-    for (int32_t kb = team_warp * 32; kb < ns; kb += team_warps * 32) {
-      const int32_t k = kb + lane;
-      int32_t as = 0, fwd = 0, p0 = 0x7fffffff, ga0 = 0;
-      if (k < ns) {
-        as = v.st_astate[s0 + k];
-        fwd = v.st_fwd[s0 + k];
-        p0 = v.st_arc0[s0 + k];
-        ga0 = g.a_rs2[as];
+    float cutoff_f;
+    *beam = NextBeam(*beam, OrderedFloat(tm.Max(best)), ns, t, final_t, g, &cutoff_f);
+    // ---- 2. first arc above the cutoff into every destination state (:1005-1028); the warp
+    // lists those arcs and where they go.
+    int32_t above = 0;
+    for (int32_t pb = lo; pb < hi; pb += 32 * kExpand) {
+      float end[kExpand];
+      int32_t dest[kExpand];
+#pragma unroll
+      for (int i = 0; i < kExpand; ++i) {
+        const int32_t p = pb + 32 * i + lane;
+        end[i] = p < hi ? r_end[p] : kNegInf;
       }
-      const int32_t first = __shfl_sync(0xffffffffu, p0, 0);
-      const int32_t last = v.st_arc0[s0 + min(kb + 32, ns)];
-      for (int32_t pb = first; pb < last; pb += 32 * kExpand) {
-        int32_t p[kExpand], j[kExpand], aidx[kExpand];
-        Arc arc[kExpand];
 #pragma unroll
-        for (int i = 0; i < kExpand; ++i) {
-          p[i] = pb + i * 32 + lane;
-          // largest j with p0[j] <= p (p0 is non-decreasing; absent states hold +inf)
-          int32_t lo = 0;
+      for (int i = 0; i < kExpand; ++i)
+        dest[i] = end[i] > cutoff_f ? r_dest[pb + 32 * i + lane] : -1;
 #pragma unroll
-          for (int step = 16; step > 0; step >>= 1) {
-            const int32_t cand = __shfl_sync(0xffffffffu, p0, lo + step);
-            if (cand <= p[i]) lo += step;
-          }
-          j[i] = lo;
-          const int32_t jp0 = __shfl_sync(0xffffffffu, p0, lo);
-          const int32_t jga0 = __shfl_sync(0xffffffffu, ga0, lo);
-          aidx[i] = p[i] < last ? jga0 + (p[i] - jp0) : -1;
+      for (int i = 0; i < kExpand; ++i) {
+        const int32_t p = pb + 32 * i + lane;
+        const bool in = dest[i] >= 0;
+        const uint32_t m = __ballot_sync(kAll, in);
+        if (in) {
+          const int32_t at = above + __popc(m & ((1u << lane) - 1u));
+          list_a[at] = p;
+          list_b[at] = dest[i];
+          atomicMax(&v.winner[dest[i]], ArcEntry(t, p));
         }
-#pragma unroll
-        for (int i = 0; i < kExpand; ++i) {
-          if (aidx[i] >= 0) arc[i] = g.a_arcs[aidx[i]];
-        }
-#pragma unroll
-        for (int i = 0; i < kExpand; ++i) {
-          const int32_t jas = __shfl_sync(0xffffffffu, as, j[i]);
-          const int32_t jfwd = __shfl_sync(0xffffffffu, fwd, j[i]);
-          if (aidx[i] >= 0) {
-            const uint32_t col = (uint32_t)(arc[i].label + 1);
-            float acoustic = (row_ok && col < (uint32_t)g.cols) ? row[col] : kNegInf;
-            int32_t dest = jas + arc[i].dest - arc[i].src;
-            if (redirect) {
-              dest = g_final;
-              acoustic = 0.0f;
-            }
-            const float ll = acoustic + arc[i].score;
-            const float end = OrderedFloat(jfwd) + ll;
-            v.arc_aidx[p[i]] = aidx[i];
-            v.arc_ll[p[i]] = ll;
-            v.arc_dest[p[i]] = dest;
-            v.arc_end[p[i]] = end;
-            best = fmaxf(best, end);
-          }
-        }
+        above += __popc(m);
       }
     }
+    StageRow(g, tm, row0 + t + 1);  // this frame's has been used
+    tm.Sync();
+    // ---- 3. which of them created their destination state, and the arcs that leave it
+    int32_t won = 0;
+    uint32_t degs = 0;
+    for (int32_t i0 = 0; i0 < above; i0 += 64) {
+      int32_t p[2], d[2], deg[2];
+      unsigned long long w[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int32_t at = i0 + 32 * i + lane;
+        p[i] = at < above ? list_a[at] : 0;
+        d[i] = at < above ? list_b[at] : -1;
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        w[i] = 0;
+        deg[i] = 0;
+        if (d[i] >= 0) {
+          w[i] = v.winner[d[i]];
+          deg[i] = g.a_rs2[d[i] + 1] - g.a_rs2[d[i]];
+        }
+      }
+      __syncwarp();  // the lists are rewritten from their start
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const bool in = d[i] >= 0 && w[i] == ArcEntry(t, p[i]);
+        const uint32_t m = __ballot_sync(kAll, in);
+        if (in) {
+          const int32_t at = won + __popc(m & ((1u << lane) - 1u));
+          list_a[at] = d[i];
+          list_b[at] = deg[i];
+          degs += (uint32_t)deg[i];
+        }
+        won += __popc(m);
+      }
+    }
+    degs = __reduce_add_sync(kAll, degs);
+    // ---- 4. the new states in the order of their arcs (:1031-1100), and the layout of the
+    // arcs that will leave them
+    const int32_t s1 = s0 + ns;
+    unsigned long long total;
+    const unsigned long long base = tm.ScanWarps(
+        kSlotNew, (unsigned long long)(uint32_t)won | ((unsigned long long)degs << 32), &total);
+    const int32_t nn = (int32_t)(total & 0xffffffffu), na1 = (int32_t)(total >> 32);
+    if ((int64_t)s1 + nn > g.cap_s || na1 < 0) return false;
+    const int32_t per_warp1 = max(ArcsPerWarp(na1, tm), 32);
+    int32_t j = (int32_t)(base & 0xffffffffu), first = (int32_t)(base >> 32);
+    for (int32_t i0 = 0; i0 < won; i0 += 32) {
+      const bool in = i0 + lane < won;
+      const int32_t d = in ? list_a[i0 + lane] : 0, deg = in ? list_b[i0 + lane] : 0;
+      int32_t inc = deg;
+#pragma unroll
+      for (int x = 1; x < 32; x <<= 1) {
+        const int32_t o = __shfl_up_sync(kAll, inc, x);
+        if (lane >= x) inc += o;
+      }
+      if (in) {
+        const int32_t k = j + lane, f = first + inc - deg;
+        v.st_astate[s1 + k] = d;
+        v.st_fwd[s1 + k] = OrderedInt(kNegInf);
+        v.st_cnt[s1 + k] = f;
+        v.winner[d] = StateEntry(t, k);
+        SetWarpFirst(v, per_warp1, k, f, deg);
+      }
+      j += 32;
+      first += __shfl_sync(kAll, inc, 31);
+    }
+    for (int32_t x = threadIdx.x; x < kMarkWords; x += kSearchThreads) sh->mark[x] = 0u;
+    tm.Sync();
+    *ns_next = nn;
+    *na_next = na1;
   }
-  best = tm.Max(best);  // also makes the arc records visible to the team
-  if (threadIdx.x == 0) sh->beam = NextBeam(sh->beam, best, ns, t, final_t, g, &sh->cutoff);
+  // ---- 5. the arcs that enter a new state, with its number, and the best score into every
+  // new state; an arc below the cutoff still enters a state that another arc created
+  // (:1103-1138).  The set of the new states (of all that share a bit of it, in graphs of
+  // more than 2^18 states) keeps the others from looking at the table.
+  const int32_t s1 = s0 + ns;
+  for (int32_t k = threadIdx.x; k < *ns_next; k += kSearchThreads) {
+    const uint32_t d = (uint32_t)v.st_astate[s1 + k] & (kMarkWords * 32 - 1);
+    atomicOr(&sh->mark[d >> 5], 1u << (d & 31));
+  }
   __syncthreads();
-  const float cutoff = sh->cutoff;
-
-  // first arc above the cutoff into every destination state (:1005-1028)
-  for (int32_t q0 = tm.tid; q0 < na; q0 += kBatch * tm.threads) {
-    float end[kBatch];
-    int32_t dest[kBatch];
+  int32_t entering = 0;
+  for (int32_t pb = lo; pb < hi; pb += 32 * kExpand) {
+    int32_t dest[kExpand];
+    float end[kExpand];
+    unsigned long long w[kExpand];
 #pragma unroll
-    for (int i = 0; i < kBatch; ++i) {
-      const int32_t q = q0 + i * tm.threads;
-      end[i] = q < na ? v.arc_end[a0 + q] : kNegInf;
-      dest[i] = q < na ? v.arc_dest[a0 + q] : 0;
+    for (int i = 0; i < kExpand; ++i) {
+      const int32_t p = pb + 32 * i + lane;
+      dest[i] = p < hi ? r_dest[p] : -1;
     }
 #pragma unroll
-    for (int i = 0; i < kBatch; ++i) {
-      if (end[i] > cutoff) atomicMax(&v.winner[dest[i]], ArcEntry(t, q0 + i * tm.threads));
+    for (int i = 0; i < kExpand; ++i) {
+      const uint32_t x = (uint32_t)dest[i] & (kMarkWords * 32 - 1);
+      w[i] = 0ull;
+      end[i] = 0.0f;
+      if (dest[i] >= 0 && (sh->mark[x >> 5] >> (x & 31) & 1u)) {
+        w[i] = v.winner[dest[i]];
+        end[i] = r_end[pb + 32 * i + lane];
+      }
+    }
+    __syncwarp();  // (r_end and r_dest take the groups' masks from their start)
+#pragma unroll
+    for (int i = 0; i < kExpand; ++i) {
+      const int32_t p = pb + 32 * i + lane;
+      const bool in = (uint32_t)(w[i] >> 32) == (uint32_t)(t + 1) && (w[i] & 0x80000000u);
+      const uint32_t m = __ballot_sync(kAll, in);
+      if (in) {
+        const int32_t idx1 = (int32_t)(w[i] & 0x7fffffffu);
+        atomicMax(&v.st_fwd[s1 + idx1], OrderedInt(end[i]));
+        const int32_t at = entering + __popc(m & ((1u << lane) - 1u));
+        list_a[at] = p;
+        list_b[at] = idx1;
+      }
+      if (lane == 0 && pb + 32 * i < hi) {
+        const int32_t group = (pb - lo) / 32 + i;
+        r_end[lo + group] = __uint_as_float(m);
+        r_dest[lo + group] = entering;
+      }
+      entering += __popc(m);
     }
   }
-  tm.Sync();
-  // which arcs created their destination state, and how many arcs leave it: one
-  // byte per arc (0: none; else out-degree + 1, 255 standing for "254 or more")
-  for (int32_t q0 = tm.tid; q0 < na; q0 += kBatch * tm.threads) {
-    float end[kBatch];
-    int32_t dest[kBatch];
-    unsigned long long w[kBatch];
+  // ---- 6. these arcs go to the arena.  A state's first one is the first of its arcs' among
+  // them: a warp sees to the states whose arcs start behind its own first arc, up to the
+  // start of the next warp's (the first warp: also at its first arc).
+  unsigned long long total;
+  const int32_t base = a0 + (int32_t)tm.ScanWarps(kSlotKept, (unsigned long long)entering, &total);
+  *kept = (int32_t)total;
+  if (a0 + (int64_t)total > raw) return false;
+  for (int32_t i0 = 0; i0 < entering; i0 += 64) {
+    int32_t p[2], idx1[2], aidx[2];
+    float ll[2];
 #pragma unroll
-    for (int i = 0; i < kBatch; ++i) {
-      const int32_t q = q0 + i * tm.threads;
-      end[i] = q < na ? v.arc_end[a0 + q] : kNegInf;
-      dest[i] = q < na ? v.arc_dest[a0 + q] : 0;
+    for (int i = 0; i < 2; ++i) {
+      const int32_t at = i0 + 32 * i + lane;
+      p[i] = at < entering ? list_a[at] : -1;
+      idx1[i] = at < entering ? list_b[at] : 0;
     }
 #pragma unroll
-    for (int i = 0; i < kBatch; ++i) w[i] = end[i] > cutoff ? v.winner[dest[i]] : 0ull;
-#pragma unroll
-    for (int i = 0; i < kBatch; ++i) {
-      const int32_t q = q0 + i * tm.threads;
-      if (q < na) {
-        uint8_t flag = 0;
-        if (end[i] > cutoff && w[i] == ArcEntry(t, q)) {
-          const int32_t deg = g.a_rs2[dest[i] + 1] - g.a_rs2[dest[i]];
-          flag = (uint8_t)(min(deg, 254) + 1);
-        }
-        v.arc_keep[a0 + q] = flag;
+    for (int i = 0; i < 2; ++i)
+      if (p[i] >= 0) {
+        aidx[i] = r_aidx[p[i]];
+        ll[i] = r_ll[p[i]];
       }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      if (p[i] >= 0) {
+        const int32_t at = base + i0 + 32 * i + lane;
+        v.arc_aidx[at] = aidx[i];
+        v.arc_ll[at] = ll[i];
+        v.arc_dest[at] = idx1[i];
+      }
+  }
+  if (lo < hi) {
+    for (int32_t k0 = tm.warp == 0 ? 0 : k_first; k0 < ns; k0 += 32) {
+      const int32_t k = k0 + lane;
+      const int32_t f = k < ns ? v.st_cnt[s0 + k] : 0x7fffffff;
+      if ((f > lo || tm.warp == 0) && f <= hi) {
+        int32_t before = entering;
+        if (f < hi) {
+          const int32_t group = (f - lo) >> 5;
+          const uint32_t m = __float_as_uint(r_end[lo + group]);
+          before = r_dest[lo + group] + __popc(m & ((1u << ((f - lo) & 31)) - 1u));
+        }
+        v.st_arc0[s0 + k] = base + before;
+      }
+      if (__any_sync(kAll, f > hi)) break;
     }
   }
-  tm.Sync();
-  // number the new states in the order of their winning arcs (:1031-1100) and lay
-  // out the arcs that will leave them
-  const int32_t s1 = s0 + ns, a1 = a0 + na;
-  int32_t nn = 0, na1 = 0;
-  for (int32_t base = 0; base < na; base += tm.threads * kPerScan) {
-    const int32_t q0 = base + tm.tid * kPerScan;
-    int32_t deg[kPerScan];
-    int32_t won = 0, degs = 0;  // bit i: arc q0 + i created its destination state
-#pragma unroll
-    for (int i = 0; i < kPerScan; ++i) {
-      deg[i] = 0;
-      const int32_t flag = q0 + i < na ? v.arc_keep[a0 + q0 + i] : 0;
-      if (flag) {
-        won |= 1 << i;
-        deg[i] = flag - 1;
-      }
-    }
-    if (won) {
-#pragma unroll
-      for (int i = 0; i < kPerScan; ++i) {
-        if (deg[i] == 254) {
-          const int32_t d = v.arc_dest[a0 + q0 + i];
-          deg[i] = g.a_rs2[d + 1] - g.a_rs2[d];
-        }
-        degs += deg[i];
-      }
-    }
-    int32_t tot, dtot, arcs_before;
-    int32_t j = nn + tm.Scan2(__popc(won), degs, &arcs_before, &tot, &dtot);
-    arcs_before += na1;
-    if (won) {
-#pragma unroll
-      for (int i = 0; i < kPerScan; ++i) {
-        if (won >> i & 1) {
-          const int32_t d = v.arc_dest[a0 + q0 + i];
-          const int32_t first = a1 + arcs_before;
-          if ((int64_t)s1 + j < g.cap_s && (int64_t)first + deg[i] <= g.cap_a) {
-            v.st_astate[s1 + j] = d;
-            v.st_fwd[s1 + j] = OrderedInt(kNegInf);
-            v.st_arc0[s1 + j] = first;
-            v.winner[d] = StateEntry(t, j);
-          }
-          arcs_before += deg[i];
-          ++j;
-        }
-      }
-    }
-    nn += tot;
-    na1 += dtot;
-  }
-  if ((int64_t)s1 + nn > g.cap_s || (int64_t)a1 + na1 > g.cap_a) return false;
-  if (tm.tid == 0) v.st_arc0[s1 + nn] = a1 + na1;
-  tm.Sync();
-  // destination index of every arc and the best score into every new state; an
-  // arc below the cutoff still enters a state that another arc created (:1103-1138)
-  for (int32_t q0 = tm.tid; q0 < na; q0 += kBatch * tm.threads) {
-    float end[kBatch];
-    int32_t dest[kBatch];
-    unsigned long long w[kBatch];
-#pragma unroll
-    for (int i = 0; i < kBatch; ++i) {
-      const int32_t q = q0 + i * tm.threads;
-      end[i] = q < na ? v.arc_end[a0 + q] : kNegInf;
-      dest[i] = q < na ? v.arc_dest[a0 + q] : -1;
-    }
-#pragma unroll
-    for (int i = 0; i < kBatch; ++i) w[i] = dest[i] >= 0 ? v.winner[dest[i]] : 0ull;
-#pragma unroll
-    for (int i = 0; i < kBatch; ++i) {
-      const int32_t q = q0 + i * tm.threads;
-      if (q < na) {
-        int32_t idx1 = -1;
-        if ((uint32_t)(w[i] >> 32) == (uint32_t)(t + 1) && (w[i] & 0x80000000u)) {
-          idx1 = (int32_t)(w[i] & 0x7fffffffu);
-          atomicMax(&v.st_fwd[s1 + idx1], OrderedInt(end[i]));
-        }
-        v.arc_dest[a0 + q] = idx1;
-      }
-    }
-  }
-  tm.Sync();
-  *ns_next = nn;
-  *na_next = na1;
+  tm.Sync();  // the scratch region is free again
   return true;
 }
 
 // Backward pass over frames [begin, end) with the output beam (PruneTimeRange,
 // :1373-1634, with SetBackwardProbsFinal :1170-1193 and PropagateBackward
-// :1239-1346), then compaction of those frames in place.  On entry the frames up to
-// `end` are complete and frame `end` has its states and the layout of the na_end arcs
-// that will leave them, but not the arcs; on return *s_top / *a_top are the ends of
-// the arenas and the frame tables are updated.
-__device__ void PruneWindow(const SearchArgs &g, const SeqView &v, const Team &tm, int32_t seq,
-                            int32_t begin, int32_t end, int32_t na_end, int32_t *s_top,
-                            int32_t *a_top, bool keep_all_at_begin = true) {
+// :1239-1346), then compaction of those frames.  On entry the frames up to `end` are complete
+// and frame `end` has its states and the layout of the arcs that will leave them, but no
+// arcs; on return *s_top / *a_top are the ends of the arenas and the frame tables are
+// updated.  Returns false when an arena has no room for the survivors twice.
+//
+// One barrier per frame for the backward pass.  The surviving states and arcs of all frames
+// are then numbered by one exchange, gathered at the far end of the arenas and copied back.
+__device__ bool PruneWindow(const SearchArgs &g, const SeqView &v, const Team &tm, int32_t seq,
+                            int32_t begin, int32_t end, int32_t *s_top, int32_t *a_top,
+                            bool keep_all_at_begin = true) {
   Shared *sh = tm.sh;
+  constexpr unsigned kAll = 0xffffffffu;
   const float kNegInf = -INFINITY;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int32_t gi = seq * g.a_stride;
   const int32_t g_final = g.a_rs1[gi + 1] - 1;  // last state of this sequence's graph
   const float beam = g.output_beam;
+  tm.Sync();  // the frame tables
+  const int32_t sb = v.frame_s0[begin], ab = v.frame_a0[begin];
+  const int32_t se = v.frame_s0[end], ns_end = *s_top - se;
 
-  {  // frame `end`: backward score = -forward score, whatever the state
-    const int32_t s0 = v.frame_s0[end], ns = *s_top - s0;
-    for (int32_t k = tm.tid; k < ns; k += tm.threads) {
-      const float fwd = OrderedFloat(v.st_fwd[s0 + k]);
-      v.st_bwd[s0 + k] = (fwd - fwd == 0.0f) ? -fwd : kNegInf;
-    }
+  // frame `end`: backward score = -forward score, whatever the state
+  for (int32_t k = tm.tid; k < ns_end; k += tm.threads) {
+    const float fwd = OrderedFloat(v.st_fwd[se + k]);
+    v.st_bwd[se + k] = (fwd - fwd == 0.0f) ? -fwd : kNegInf;
   }
   tm.Sync();
 
-  // backwards: arc and state survival, backward scores, new state numbers
-  for (int32_t t = end - 1; t >= begin; --t) {
-    const int32_t s0 = v.frame_s0[t], ns = v.frame_s0[t + 1] - s0, s_next = v.frame_s0[t + 1];
-    int32_t kept = 0;
-    for (int32_t base = 0; base < ns; base += tm.threads) {
-      // a warp takes 32 consecutive states and walks their arcs as one flat range
-      // (as in the search step); per-state maxima and counts gather in shared memory
-      const int32_t k = base + tm.tid;
-      const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-      int32_t keep_state = 0, p0 = 0x7fffffff;
-      float fwd = 0.0f;
-      if (k < ns) {
-        fwd = OrderedFloat(v.st_fwd[s0 + k]);
-        p0 = v.st_arc0[s0 + k];
-      }
-      sh->wbest[warp][lane] = OrderedInt(kNegInf);
-      sh->wcnt[warp][lane] = 0;
-      __syncwarp();
-      const int32_t first = __shfl_sync(0xffffffffu, p0, 0);
-      const int32_t last = v.st_arc0[s0 + min(k - lane + 32, ns)];
-      for (int32_t pb = first; pb < last; pb += 32 * kExpand) {
-        int32_t p[kExpand], j[kExpand], d[kExpand];
-        float ll[kExpand], nb[kExpand];
-#pragma unroll
-        for (int i = 0; i < kExpand; ++i) {
-          p[i] = pb + i * 32 + lane;
-          int32_t lo = 0;
-#pragma unroll
-          for (int step = 16; step > 0; step >>= 1) {
-            const int32_t cand = __shfl_sync(0xffffffffu, p0, lo + step);
-            if (cand <= p[i]) lo += step;
-          }
-          j[i] = lo;
-          d[i] = p[i] < last ? v.arc_dest[p[i]] : -1;
-          ll[i] = p[i] < last ? v.arc_ll[p[i]] : 0.0f;
+  // ---- backwards: arc survival, the number of surviving arcs and the backward score of every
+  // state; the destination of a surviving arc becomes its place in the arena, that of
+  // another -1
+  {
+    int32_t s0 = v.frame_s0[end], a1 = v.frame_a0[end];
+    for (int32_t t = end - 1; t >= begin; --t) {
+      const int32_t s_next = s0, a_next = a1;
+      s0 = v.frame_s0[t];
+      a1 = v.frame_a0[t];
+      const int32_t ns = s_next - s0;
+      for (int32_t k0 = tm.warp * 32; k0 < ns; k0 += tm.warps * 32) {
+        const int32_t k = k0 + lane;
+        int32_t f = a_next, fwd = 0, as = 0;
+        if (k < ns) {
+          f = v.st_arc0[s0 + k];
+          fwd = v.st_fwd[s0 + k];
+          as = v.st_astate[s0 + k];
         }
+        int32_t next = __shfl_down_sync(kAll, f, 1);
+        if (lane == 31) next = k + 1 < ns ? v.st_arc0[s0 + k + 1] : a_next;
+        sh->wbest[warp][lane] = OrderedInt(kNegInf);
+        sh->wcnt[warp][lane] = 0;
+        const int32_t start = __shfl_sync(kAll, f, 0), stop = __shfl_sync(kAll, next, 31);
+        ArcWalk walk;
+        walk.Begin(sh->rec[warp], f, next, make_int4(fwd, lane, 0, 0), start);
+        for (int32_t pb = start; pb < stop; pb += 64) {
+          int32_t r[2], d[2];
+          float ll[2], nb[2];
 #pragma unroll
-        for (int i = 0; i < kExpand; ++i) nb[i] = d[i] >= 0 ? v.st_bwd[s_next + d[i]] : kNegInf;
+          for (int i = 0; i < 2; ++i) {
+            const int32_t p = pb + 32 * i + lane;
+            r[i] = walk.Next(pb + 32 * i);
+            d[i] = p < stop ? v.arc_dest[p] : -1;
+            ll[i] = p < stop ? v.arc_ll[p] : 0.0f;
+          }
 #pragma unroll
-        for (int i = 0; i < kExpand; ++i) {
-          const float jfwd = __shfl_sync(0xffffffffu, fwd, j[i]);
-          if (p[i] < last) {
-            uint8_t keep = 0;
-            if (d[i] >= 0) {
+          for (int i = 0; i < 2; ++i) nb[i] = d[i] >= 0 ? v.st_bwd[s_next + d[i]] : kNegInf;
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const int32_t p = pb + 32 * i + lane;
+            if (p < stop) {
+              const int4 rec = sh->rec[warp][r[i]];
               const float bl = ll[i] + nb[i];
-              if (bl + jfwd >= -beam) {
-                keep = 1;
-                atomicMax(&sh->wbest[warp][j[i]], OrderedInt(bl));
-                atomicAdd(&sh->wcnt[warp][j[i]], 1);
+              int32_t to = -1;
+              if (d[i] >= 0 && bl + OrderedFloat(rec.x) >= -beam) {
+                to = s_next + d[i];
+                atomicMax(&sh->wbest[warp][rec.y], OrderedInt(bl));
+                atomicAdd(&sh->wcnt[warp][rec.y], 1);
               }
+              v.arc_dest[p] = to;
             }
-            v.arc_keep[p[i]] = keep;
+          }
+        }
+        __syncwarp();
+        if (k < ns) {
+          v.st_cnt[s0 + k] = sh->wcnt[warp][lane];
+          v.st_bwd[s0 + k] = as == g_final ? -OrderedFloat(fwd) : OrderedFloat(sh->wbest[warp][lane]);
+        }
+        __syncwarp();
+      }
+      tm.Sync();
+    }
+  }
+
+  // ---- new numbers: of a state (st_new) and of its first arc (st_cnt), whether it survives
+  // or not.  A warp takes a contiguous range of the window's states.
+  const int32_t n = se - sb, all_to = keep_all_at_begin ? v.frame_s0[begin + 1] : sb;
+  const int32_t per_warp = ((n + tm.warps - 1) / tm.warps + 31) & ~31;
+  const int32_t lo = sb + (int32_t)min((int64_t)tm.warp * per_warp, (int64_t)n);
+  const int32_t hi = min(lo + per_warp, se);
+  uint32_t states = 0, arcs = 0;
+#pragma unroll 2
+  for (int32_t s = lo + lane; s < hi; s += 32) {
+    states += v.st_bwd[s] != kNegInf || s < all_to;
+    arcs += (uint32_t)v.st_cnt[s];
+  }
+  states = __reduce_add_sync(kAll, states);
+  arcs = __reduce_add_sync(kAll, arcs);
+  unsigned long long total;
+  const unsigned long long base = tm.ScanWarps(
+      kSlotWindow, (unsigned long long)states | ((unsigned long long)arcs << 32), &total);
+  const int32_t ks = (int32_t)(total & 0xffffffffu), ka = (int32_t)(total >> 32);
+  // where the survivors are gathered: the states (and those of frame `end`) and the arcs
+  const int64_t hold_s = g.cap_s - ks - ns_end, hold_a = g.cap_a - ka;
+  if (hold_s < *s_top || hold_a < *a_top) return false;
+  {
+    int32_t j = sb + (int32_t)(base & 0xffffffffu), q = ab + (int32_t)(base >> 32);
+    for (int32_t s0 = lo; s0 < hi; s0 += 32) {
+      const int32_t s = s0 + lane;
+      const bool keep = s < hi && (v.st_bwd[s] != kNegInf || s < all_to);
+      const int32_t cnt = s < hi ? v.st_cnt[s] : 0;
+      const uint32_t m = __ballot_sync(kAll, keep);
+      int32_t inc = cnt;
+#pragma unroll
+      for (int x = 1; x < 32; x <<= 1) {
+        const int32_t o = __shfl_up_sync(kAll, inc, x);
+        if (lane >= x) inc += o;
+      }
+      if (s < hi) {
+        const int32_t at = j + __popc(m & ((1u << lane) - 1u));
+        v.st_new[s] = at;
+        v.st_cnt[s] = q + inc - cnt;
+        if (keep) {
+          const int64_t h = hold_s + (at - sb);
+          v.st_astate[h] = v.st_astate[s];
+          v.st_fwd[h] = v.st_fwd[s];
+          v.st_arc0[h] = q + inc - cnt;
+        }
+      }
+      j += __popc(m);
+      q += __shfl_sync(kAll, inc, 31);
+    }
+    for (int32_t k = tm.tid; k < ns_end; k += tm.threads) {
+      const int64_t h = hold_s + ks + k;
+      v.st_astate[h] = v.st_astate[se + k];
+      v.st_fwd[h] = v.st_fwd[se + k];
+      v.st_new[h] = v.st_cnt[se + k];
+    }
+  }
+  tm.Sync();
+  // ---- the surviving arcs, 32 states of a frame to a warp: their arcs are consecutive, and
+  // so are the places they go to
+  for (int32_t t = begin + tm.tid; t < end; t += tm.threads) {
+    const int32_t s = v.frame_s0[t];
+    v.frame_n0[t] = s < se ? v.st_new[s] : sb + ks;
+    v.frame_m0[t] = s < se ? v.st_cnt[s] : ab + ka;
+  }
+  {
+    int32_t turn = 0;  // units of 32 states so far, modulo the warps
+    int32_t s1 = sb, a1 = ab;
+    for (int32_t t = begin; t < end; ++t) {
+      const int32_t s0 = s1;
+      s1 = v.frame_s0[t + 1];
+      a1 = v.frame_a0[t + 1];
+      const int32_t ns = s1 - s0;
+      // where frame t + 1 will start (the states of frame `end` keep their numbers)
+      const int32_t new_s1 = t + 1 == end ? 0 : (s1 < se ? v.st_new[s1] : sb + ks);
+      int32_t u = tm.warp - turn;
+      if (u < 0) u += tm.warps;
+      for (int32_t k0 = u * 32; k0 < ns; k0 += tm.warps * 32) {
+        const int32_t start = v.st_arc0[s0 + k0];
+        const int32_t stop = k0 + 32 < ns ? v.st_arc0[s0 + k0 + 32] : a1;
+        int64_t h = hold_a + (v.st_cnt[s0 + k0] - ab);
+        for (int32_t pb = start; pb < stop; pb += 64) {
+          int32_t d[2], aidx[2];
+          float ll[2];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const int32_t p = pb + 32 * i + lane;
+            d[i] = p < stop ? v.arc_dest[p] : -1;
+          }
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+            if (d[i] >= 0) {
+              aidx[i] = v.arc_aidx[pb + 32 * i + lane];
+              ll[i] = v.arc_ll[pb + 32 * i + lane];
+              d[i] = t + 1 == end ? d[i] - se : v.st_new[d[i]] - new_s1;
+            }
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const uint32_t m = __ballot_sync(kAll, d[i] >= 0);
+            if (d[i] >= 0) {
+              const int64_t at = h + __popc(m & ((1u << lane) - 1u));
+              v.arc_aidx[at] = aidx[i];
+              v.arc_ll[at] = ll[i];
+              v.arc_dest[at] = d[i];
+            }
+            h += __popc(m);
           }
         }
       }
-      __syncwarp();
-      if (k < ns) {
-        const float best = OrderedFloat(sh->wbest[warp][lane]);
-        v.st_cnt[s0 + k] = sh->wcnt[warp][lane];
-        const float bwd = (v.st_astate[s0 + k] == g_final) ? -fwd : best;
-        v.st_bwd[s0 + k] = bwd;
-        keep_state = (bwd != kNegInf) || (t == begin && keep_all_at_begin);
-      }
-      int32_t tot;
-      const int32_t j = kept + tm.Scan(keep_state, &tot);
-      if (k < ns) v.st_new[s0 + k] = keep_state ? j : -1;
-      kept += tot;
+      turn = (turn + (ns + 31) / 32) % tm.warps;
     }
-    // (the barrier inside the last scan has published this frame's backward scores)
-  }
-
-  // forwards: move the surviving states and arcs down.  Reads of a chunk complete
-  // before its writes (the scans synchronise), and writes never reach past the
-  // chunk being read, so the compaction is done in place.
-  int32_t ws = v.frame_s0[begin], wa = v.frame_a0[begin];
-  int32_t old_s0 = ws, old_a0 = wa;
-  for (int32_t t = begin; t < end; ++t) {
-    const int32_t old_s1 = v.frame_s0[t + 1], old_a1 = v.frame_a0[t + 1];
-    const int32_t ns = old_s1 - old_s0, na = old_a1 - old_a0;
-    int32_t s_run = 0, a_run = 0;
-    for (int32_t base = 0; base < ns; base += tm.threads) {
-      const int32_t k = base + tm.tid;
-      int32_t keep_state = 0, cnt = 0, as = 0, fwd = 0;
-      float bwd = 0.0f;
-      if (k < ns) {
-        keep_state = v.st_new[old_s0 + k] >= 0;
-        as = v.st_astate[old_s0 + k];
-        fwd = v.st_fwd[old_s0 + k];
-        bwd = v.st_bwd[old_s0 + k];
-        cnt = v.st_cnt[old_s0 + k];
-      }
-      int32_t stot, atot, aj;
-      const int32_t sj = s_run + tm.Scan2(keep_state, cnt, &aj, &stot, &atot);
-      aj += a_run;
-      if (keep_state) {
-        v.st_astate[ws + sj] = as;
-        v.st_fwd[ws + sj] = fwd;
-        v.st_bwd[ws + sj] = bwd;
-        v.st_arc0[ws + sj] = wa + aj;
-      }
-      s_run += stot;
-      a_run += atot;
-    }
-    int32_t moved = 0;
-    const bool renumber = t + 1 < end;  // the states of frame `end` keep their numbers
-    for (int32_t base = 0; base < na; base += tm.threads * kPer) {
-      const int32_t q0 = base + tm.tid * kPer;
-      int32_t aidx[kPer], dest[kPer];
-      float ll[kPer];
-      int32_t keep = 0;
-#pragma unroll
-      for (int i = 0; i < kPer; ++i) {
-        if (q0 + i < na && v.arc_keep[old_a0 + q0 + i]) {
-          keep |= 1 << i;
-          aidx[i] = v.arc_aidx[old_a0 + q0 + i];
-          ll[i] = v.arc_ll[old_a0 + q0 + i];
-          dest[i] = v.arc_dest[old_a0 + q0 + i];
-          if (renumber) dest[i] = v.st_new[old_s1 + dest[i]];
-        }
-      }
-      int32_t tot;
-      int32_t j = moved + tm.Scan(__popc(keep), &tot);
-#pragma unroll
-      for (int i = 0; i < kPer; ++i) {
-        if (keep >> i & 1) {
-          v.arc_aidx[wa + j] = aidx[i];
-          v.arc_ll[wa + j] = ll[i];
-          v.arc_dest[wa + j] = dest[i];
-          ++j;
-        }
-      }
-      moved += tot;
-    }
-    // the new offsets go to the frame tables after the loop: a thread that runs
-    // ahead through empty frames must still find the old ones
-    if (tm.tid == 0) {
-      sh->new_s0[t - begin] = ws;
-      sh->new_a0[t - begin] = wa;
-    }
-    ws += s_run;
-    wa += a_run;
-    old_s0 = old_s1;
-    old_a0 = old_a1;
-  }
-  // frame `end`: its states, and the layout of their arcs, follow the compacted frames
-  const int32_t ns_end = *s_top - old_s0;
-  for (int32_t base = 0; base < ns_end; base += tm.threads) {
-    const int32_t k = base + tm.tid;
-    int32_t as = 0, fwd = 0, arc0 = 0;
-    float bwd = 0.0f;
-    if (k < ns_end) {
-      as = v.st_astate[old_s0 + k];
-      fwd = v.st_fwd[old_s0 + k];
-      bwd = v.st_bwd[old_s0 + k];
-      arc0 = v.st_arc0[old_s0 + k];
-    }
-    tm.Sync();
-    if (k < ns_end) {
-      v.st_astate[ws + k] = as;
-      v.st_fwd[ws + k] = fwd;
-      v.st_bwd[ws + k] = bwd;
-      v.st_arc0[ws + k] = arc0 - old_a0 + wa;
-    }
-  }
-  tm.Sync();  // every thread is past the old frame tables
-  if (tm.tid == 0) {
-    for (int32_t t = begin; t < end; ++t) {
-      v.frame_s0[t] = sh->new_s0[t - begin];
-      v.frame_a0[t] = sh->new_a0[t - begin];
-    }
-    v.frame_s0[end] = ws;
-    v.frame_a0[end] = wa;
-    v.st_arc0[ws + ns_end] = wa + na_end;  // closes the last arc range
   }
   tm.Sync();
-  *s_top = ws + ns_end;
-  *a_top = wa;
+  // ---- back to their places
+#pragma unroll 4
+  for (int32_t k = tm.tid; k < ka; k += tm.threads) {
+    v.arc_aidx[ab + k] = v.arc_aidx[hold_a + k];
+    v.arc_ll[ab + k] = v.arc_ll[hold_a + k];
+    v.arc_dest[ab + k] = v.arc_dest[hold_a + k];
+  }
+#pragma unroll 4
+  for (int32_t k = tm.tid; k < ks + ns_end; k += tm.threads) {
+    v.st_astate[sb + k] = v.st_astate[hold_s + k];
+    v.st_fwd[sb + k] = v.st_fwd[hold_s + k];
+    if (k < ks) v.st_arc0[sb + k] = v.st_arc0[hold_s + k];
+    else v.st_cnt[sb + k] = v.st_new[hold_s + k];
+  }
+  for (int32_t t = begin + tm.tid; t <= end; t += tm.threads) {
+    v.frame_s0[t] = t < end ? v.frame_n0[t] : sb + ks;
+    v.frame_a0[t] = t < end ? v.frame_m0[t] : ab + ka;
+  }
+  tm.Sync();
+  *s_top = sb + ks + ns_end;
+  *a_top = ab + ka;
+  return true;
 }
 
 // Largest frame of the finished lattice of a sequence, in states and in arcs, over frames
@@ -779,12 +891,8 @@ __device__ void LargestFrame(const SeqView &v, const Team &tm, int32_t frames) {
 // One team per sequence: all frames of the search with the pruning windows in the
 // reference's schedule (:164-199, :213-229).
 __global__ void __launch_bounds__(kSearchThreads, 1) PrunedSearch(const SearchArgs g) {
-  __shared__ Shared sh;
-  if (threadIdx.x == 0) {
-    sh.phase_i = sh.phase_f = sh.phase_l = 0;
-    sh.beam = g.search_beam;
-  }
-  __syncthreads();
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Shared &sh = *reinterpret_cast<Shared *>(smem_raw);
   const Team tm(&sh);
   const int32_t seq = blockIdx.x / tm.size;
   const SeqView v = ViewOf(g, seq);
@@ -792,6 +900,7 @@ __global__ void __launch_bounds__(kSearchThreads, 1) PrunedSearch(const SearchAr
   const int32_t T = g.T;
   const int32_t gi = seq * g.a_stride;
   const int32_t g_start = g.a_rs1[gi], g_states = g.a_rs1[gi + 1] - g_start;
+  float beam = g.search_beam;
 
   // frame 0: the start state, if the graph has states (:435-472)
   int32_t s0 = 0, ns = g_states > 0 ? 1 : 0, a0 = 0;
@@ -799,37 +908,41 @@ __global__ void __launch_bounds__(kSearchThreads, 1) PrunedSearch(const SearchAr
   if (tm.tid == 0) {
     v.frame_s0[0] = 0;
     v.frame_a0[0] = 0;
-    v.st_arc0[0] = 0;
     if (ns) {
       v.st_astate[0] = g_start;
       v.st_fwd[0] = OrderedInt(0.0f);
-      v.st_arc0[1] = na;
+      v.st_cnt[0] = 0;
+      if (na) SetWarpFirst(v, ArcsPerWarp(na, tm), 0, 0, na);
     }
   }
+  StageRow(g, tm, row0);
   tm.Sync();
   int32_t s_top = ns, a_top = 0;
   int32_t status = kSeqOk;
   int32_t next_end = kWindowShift;  // end of the next pruning window
   for (int32_t t = 0; t < T; ++t) {
-    if (tm.tid == 0) {  // published by the barriers inside the step
-      v.frame_s0[t + 1] = s0 + ns;
-      v.frame_a0[t + 1] = a0 + na;
-    }
-    int32_t nn, na1;
-    if (!SearchStep(g, v, tm, seq, t, final_t, row0, s0, ns, a0, na, &nn, &na1)) {
+    int32_t nn, na1, kept;
+    if (!SearchStep(g, v, tm, seq, t, final_t, row0, s0, ns, a0, na, &beam, &nn, &na1, &kept)) {
       status = kSeqOverflow;
       break;
     }
     s0 += ns;
-    a0 += na;
+    a0 += kept;
     ns = nn;
     na = na1;
     s_top = s0 + ns;
     a_top = a0;
+    if (tm.tid == 0) {  // published by the next barrier
+      v.frame_s0[t + 1] = s0;
+      v.frame_a0[t + 1] = a0;
+    }
     const int32_t this_end = next_end >= T ? T : next_end;
     if (t == this_end - 1) {
       const int32_t begin = max(0, next_end - kWindow);
-      PruneWindow(g, v, tm, seq, begin, this_end, na, &s_top, &a_top);
+      if (!PruneWindow(g, v, tm, seq, begin, this_end, &s_top, &a_top)) {
+        status = kSeqOverflow;
+        break;
+      }
       s0 = s_top - ns;
       a0 = a_top;
       next_end += kWindowShift;
@@ -958,9 +1071,9 @@ struct OnlineArgs {
                            // at their ends, so the pruning window is counted from there)
 };
 
-// Arc ranges of the states of a frame whose arcs are about to be expanded.
+// Layout of the arcs of a frame that are about to be expanded; returns their number.
 __device__ int32_t LayoutFrame(const SearchArgs &g, const SeqView &v, const Team &tm, int32_t s0,
-                               int32_t ns, int32_t a0) {
+                               int32_t ns) {
   int32_t na = 0;
   for (int32_t base = 0; base < ns; base += tm.threads) {
     const int32_t k = base + tm.tid;
@@ -971,10 +1084,17 @@ __device__ int32_t LayoutFrame(const SearchArgs &g, const SeqView &v, const Team
     }
     int32_t tot;
     const int32_t ex = tm.Scan(deg, &tot);
-    if (k < ns) v.st_arc0[s0 + k] = a0 + na + ex;
+    if (k < ns) v.st_cnt[s0 + k] = na + ex;
     na += tot;
   }
-  if (tm.tid == 0) v.st_arc0[s0 + ns] = a0 + na;
+  tm.Sync();
+  if (na > 0) {
+    const int32_t per_warp = ArcsPerWarp(na, tm);
+    for (int32_t k = tm.tid; k < ns; k += tm.threads) {
+      const int32_t f = v.st_cnt[s0 + k];
+      SetWarpFirst(v, per_warp, k, f, (k + 1 < ns ? v.st_cnt[s0 + k + 1] : na) - f);
+    }
+  }
   tm.Sync();
   return na;
 }
@@ -1042,16 +1162,12 @@ __device__ int32_t FinalArcs(const SearchArgs &g, const SeqView &v, const Team &
 }
 
 __global__ void __launch_bounds__(kSearchThreads, 1) OnlineChunk(const OnlineArgs o) {
-  __shared__ Shared sh;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Shared &sh = *reinterpret_cast<Shared *>(smem_raw);
   const SearchArgs &g = o.g;
-  const Team tm0(&sh);
-  const int32_t seq = blockIdx.x / tm0.size;
-  if (threadIdx.x == 0) {
-    sh.phase_i = sh.phase_f = sh.phase_l = 0;
-    sh.beam = o.beam_in[seq];
-  }
-  __syncthreads();
   const Team tm(&sh);
+  const int32_t seq = blockIdx.x / tm.size;
+  float beam = o.beam_in[seq];
   const SeqView v = ViewOf(g, seq);
   const int32_t row0 = g.b_rs[seq];
   const int32_t h = o.hist[seq];
@@ -1059,34 +1175,39 @@ __global__ void __launch_bounds__(kSearchThreads, 1) OnlineChunk(const OnlineArg
   // the frontier: the states of frame h; what was kept of its arcs (the final arcs of
   // the previous chunk) is dropped and they are expanded again (:354-361)
   int32_t s0 = v.frame_s0[h], ns = v.frame_s0[h + 1] - s0, a0 = v.frame_a0[h];
-  int32_t na = LayoutFrame(g, v, tm, s0, ns, a0);
+  tm.Sync();  // the CTAs of the team have started: their shared memory can be written
+  int32_t na = LayoutFrame(g, v, tm, s0, ns);
+  StageRow(g, tm, row0);
+  tm.Sync();
   int32_t s_top = s0 + ns, a_top = a0;
   int32_t status = kSeqOk;
   for (int32_t t = 0; t < o.chunk; ++t) {
-    if (tm.tid == 0) {
-      v.frame_s0[h + t + 1] = s0 + ns;
-      v.frame_a0[h + t + 1] = a0 + na;
-    }
-    int32_t nn, na1;
-    if (!SearchStep(g, v, tm, seq, t, kNoFinalFrame, row0, s0, ns, a0, na, &nn, &na1)) {
+    int32_t nn, na1, kept;
+    if (!SearchStep(g, v, tm, seq, t, kNoFinalFrame, row0, s0, ns, a0, na, &beam, &nn, &na1,
+                    &kept)) {
       status = kSeqOverflow;
       break;
     }
     s0 += ns;
-    a0 += na;
+    a0 += kept;
     ns = nn;
     na = na1;
     s_top = s0 + ns;
     a_top = a0;
+    if (tm.tid == 0) {  // published by the next barrier
+      v.frame_s0[h + t + 1] = s0;
+      v.frame_a0[h + t + 1] = a0;
+    }
   }
   const int32_t end = h + o.chunk;
+  // PruneTimeRange(max(0, T_ - 2), T_ + chunk) in frames counted from the end of the
+  // longest history: a stream with a shorter one starts inside the window, and then
+  // its first frame is not the one whose states are all kept
+  const int32_t begin_aligned = max(0, o.hist_max - 2) - (o.hist_max - h);
+  if (status == kSeqOk &&
+      !PruneWindow(g, v, tm, seq, max(begin_aligned, 0), end, &s_top, &a_top, begin_aligned >= 0))
+    status = kSeqOverflow;
   if (status == kSeqOk) {
-    // PruneTimeRange(max(0, T_ - 2), T_ + chunk) in frames counted from the end of the
-    // longest history: a stream with a shorter one starts inside the window, and then
-    // its first frame is not the one whose states are all kept
-    const int32_t begin_aligned = max(0, o.hist_max - 2) - (o.hist_max - h);
-    PruneWindow(g, v, tm, seq, max(begin_aligned, 0), end, na, &s_top, &a_top,
-                begin_aligned >= 0);
     s0 = s_top - ns;
     a0 = a_top;
     const int32_t nf = FinalArcs(g, v, tm, seq, row0 + o.chunk, s0, ns, a0);
@@ -1113,7 +1234,7 @@ __global__ void __launch_bounds__(kSearchThreads, 1) OnlineChunk(const OnlineArg
     out[3] = status;
     out[4] = sh.most_states;
     out[5] = sh.most_arcs;
-    o.beam_out[seq] = sh.beam;
+    o.beam_out[seq] = beam;
   }
   tm.Sync();
 }
@@ -1236,12 +1357,16 @@ int32_t MakePrunedLayout(const k2b200_pruned_args *a, char *ws, PrunedLayout *L)
   g.arc_dest = i32(na);
   g.arc_ll = f32(na);
   g.arc_end = f32(na);
-  g.arc_keep = reinterpret_cast<uint8_t *>(ws + Take(&off, na));
+  g.list_a = i32(na);
+  g.list_b = i32(na);
   L->winner_bytes = 8 * (g.a_stride ? (size_t)std::max(a->num_states, 1)
                                     : n * (size_t)std::max(a->num_states, 1));
   g.winner = reinterpret_cast<unsigned long long *>(ws + Take(&off, L->winner_bytes));
   g.frame_s0 = i32(n * ((size_t)T + 2));
   g.frame_a0 = i32(n * ((size_t)T + 2));
+  g.frame_n0 = i32(n * ((size_t)T + 2));
+  g.frame_m0 = i32(n * ((size_t)T + 2));
+  g.warp_first = i32(n * kTeamWarps);
   g.seq_out = i32(kSeqOut * n);
   L->out_rs1 = i32(n + 1);
   L->arc_base = i32(n + 1);
@@ -1401,6 +1526,9 @@ int32_t k2b200_intersect_dense_pruned_search_bounds(
     attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
+    cfg.dynamicSmemBytes = sizeof(Shared);
+    K2B_CUDA_OK(cudaFuncSetAttribute(PrunedSearch, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(Shared)));
     K2B_CUDA_OK(cudaLaunchKernelEx(&cfg, PrunedSearch, L.g));
     NoteLaunch();
   }
@@ -1564,6 +1692,9 @@ int32_t k2b200_online_decode_run_bounds(const k2b200_online_args *args, void *wo
     attr.val.clusterDim.z = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
+    cfg.dynamicSmemBytes = sizeof(Shared);
+    K2B_CUDA_OK(cudaFuncSetAttribute(OnlineChunk, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(Shared)));
     K2B_CUDA_OK(cudaLaunchKernelEx(&cfg, OnlineChunk, o));
     NoteLaunch();
   }
