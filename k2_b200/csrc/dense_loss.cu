@@ -1737,7 +1737,7 @@ static int32_t LaunchChainMasked(const LossLayout &LL, const k2b200_intersect_ar
           masks); NoteLaunch(); }                                                              \
     }
     // state pitch of the staged Viterbi scores, in three sizes
-    if (L.max_states <= 192) K2B_ARC_MASKS(192, 32)
+    if (L.max_states <= 192) K2B_ARC_MASKS(192, 56)
     else if (L.max_states <= 384) K2B_ARC_MASKS(384, 32)
     else K2B_ARC_MASKS(768, 16)
 #undef K2B_ARC_MASKS

@@ -354,13 +354,15 @@ int32_t LaunchPlanLanes(const Layout &L, const k2b200_intersect_args *a, char *w
 constexpr int kVitRing = 4;   // slots of the row ring = frames per unrolled group
 constexpr int kVitAhead = 3;  // rows requested ahead of the frame that uses them
 
-// kV: plan lanes per thread.  Thread t of a CTA of kLaneThreads / kV threads works for the
-// plan's lanes t, t + blockDim, ...: a multiple of 32 apart, so the lanes of a plan warp stay
-// the lanes of one warp and the shuffles of a group work as before.  Fewer, fatter warps:
-// the per-frame cost of a warp that does not depend on its arcs (barrier, row ring, loop) is
-// paid fewer times, and the gathers of a thread's lanes are in flight together.
-template <int kDeg, int kV>
-__global__ void __launch_bounds__(kLaneThreads / kV)
+// kPitch: floats of a ring slot, 0: cols_pad of them.  With a constant pitch every access of the
+// frame loop has its slot in the instruction's offset.
+// Bound by the latency of a frame and by the issue of its instructions: one max instead of a
+// comparison and a selection, constant slot offsets, and copies by the warps that hold a
+// column only took 500 frames of 4627 arcs from 246 to 215 us per round of CTAs (one CTA per
+// SM).  40 registers, for two CTAs per SM, leave no room to request a lane's eight scores
+// together: 256 CTAs took 460 us, and 431 with up to 80.
+template <int kDeg, int kPitch>
+__global__ void __launch_bounds__(kLaneThreads, 1)
 LanesViterbi(const FsaInfo *__restrict__ infos, int32_t n, const Arc *__restrict__ arcs,
              const int32_t *__restrict__ a_row_splits2, const int32_t *__restrict__ in_splits,
              const int32_t *__restrict__ in_arcs, const float *__restrict__ scores,
@@ -370,121 +372,121 @@ LanesViterbi(const FsaInfo *__restrict__ infos, int32_t n, const Arc *__restrict
   __shared__ float buf[2][kLaneThreads];
   const int32_t i = blockIdx.y;
   if (unfit[i] & 1) return;
-  const FsaInfo f = infos[i];
   const int dir = blockIdx.x;
-  const int32_t S = f.num_states, Tk = f.tk;
+  const int32_t S = infos[i].num_states, Tk = infos[i].tk;
   if (S == 0) return;
-  const int tid = threadIdx.x, nt = blockDim.x;  // nt == kLaneThreads / kV
-  float *ring = reinterpret_cast<float *>(smem_raw);  // [kVitRing][cols_pad]
-  int32_t s[kV], g[kV], G[kV], g_max[kV], col0[kV];
-  int32_t other[kV][kDeg], col[kV][kDeg];
-  float w[kV][kDeg];
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const int32_t pitch = kPitch ? kPitch : cols_pad;
+  float *ring = reinterpret_cast<float *>(smem_raw);  // [kVitRing][pitch]
+  int32_t s = -1, g = 0, G = 1, col0 = -1;
+  {
+    const int32_t code = plan[((int64_t)dir * n + i) * kLaneThreads + tid];
+    if (code >= 0) {
+      s = code & 0xffff;
+      g = (code >> 16) & 0xff;
+      G = code >> 24;
+    }
+  }
+  // byte offsets of an arc's other end in a buffer and of its column in a row
+  uint32_t other[kDeg], col[kDeg];
+  float w[kDeg];
   bool same = true;
 #pragma unroll
-  for (int v = 0; v < kV; ++v) {
-    s[v] = -1;
-    g[v] = 0;
-    G[v] = 1;
-    col0[v] = -1;
-    const int32_t code = plan[((int64_t)dir * n + i) * kLaneThreads + tid + v * nt];
-    if (code >= 0) {
-      s[v] = code & 0xffff;
-      g[v] = (code >> 16) & 0xff;
-      G[v] = code >> 24;
-    }
+  for (int j = 0; j < kDeg; ++j) {
+    other[j] = 0;
+    col[j] = 0;
+    w[j] = -INFINITY;
+  }
+  if (s >= 0) {
+    const int32_t state_off = infos[i].state_off;
+    const int32_t *splits = dir == 0 ? in_splits : a_row_splits2;
+    const int32_t a0 = splits[state_off + s], a1 = splits[state_off + s + 1];
 #pragma unroll
     for (int j = 0; j < kDeg; ++j) {
-      other[v][j] = 0;
-      col[v][j] = 0;
-      w[v][j] = -INFINITY;
-    }
-    if (s[v] >= 0) {
-      const int32_t *splits = dir == 0 ? in_splits : a_row_splits2;
-      const int32_t a0 = splits[f.state_off + s[v]], a1 = splits[f.state_off + s[v] + 1];
-#pragma unroll
-      for (int j = 0; j < kDeg; ++j) {
-        const int32_t k = a0 + g[v] + j * G[v];
-        if (k < a1) {
-          const Arc arc = arcs[dir == 0 ? in_arcs[k] : k];
-          other[v][j] = dir == 0 ? arc.src : arc.dest;
-          const int32_t c = arc.label + 1;
-          if (c >= 0 && c < cols) {
-            col[v][j] = c;
-            w[v][j] = arc.score;
-            if (col0[v] < 0) col0[v] = c;
-            else if (c != col0[v]) same = false;
-          }
+      const int32_t k = a0 + g + j * G;
+      if (k < a1) {
+        const Arc arc = arcs[dir == 0 ? in_arcs[k] : k];
+        other[j] = 4u * (uint32_t)(dir == 0 ? arc.src : arc.dest);
+        const int32_t c = arc.label + 1;
+        if (c >= 0 && c < cols) {
+          col[j] = 4u * (uint32_t)c;
+          w[j] = arc.score;
+          if (col0 < 0) col0 = c;
+          else if (c != col0) same = false;
         }
       }
     }
-    if (col0[v] < 0) col0[v] = 0;
-    g_max[v] = __reduce_max_sync(0xffffffffu, G[v]);  // widest lane group of this plan warp
   }
+  const uint32_t col0_off = 4u * (uint32_t)max(col0, 0);
+  const int32_t g_max = __reduce_max_sync(0xffffffffu, G);  // widest lane group of this warp
   const bool hoist = __syncthreads_and(same);  // uniform over the CTA
-  // step t (1..Tk) consumes dense row t-1 (forward) or Tk-t (backward)
-  const float *base = scores + (int64_t)f.row0 * cols;
-  auto issue_row = [&](int32_t step, int32_t slot) {
-    if (step <= Tk) {
-      const float *src = base + (int64_t)(dir == 0 ? step - 1 : Tk - step) * cols;
-      float *dst = ring + slot * cols_pad;
-      for (int32_t c = tid; c < cols; c += nt) CpAsync4(dst + c, src + c);
-    }
+  // step t (1..Tk) consumes dense row t-1 (forward) or Tk-t (backward).  The warps that hold
+  // a column copy it; the others neither copy nor wait.
+  const bool copies = (tid & ~31) < cols;
+  const float *src = scores + ((int64_t)infos[i].row0 + (dir == 0 ? 0 : Tk - 1)) * cols;
+  const int64_t src_step = dir == 0 ? cols : -(int64_t)cols;
+  auto issue_row = [&](bool there, int32_t slot) {
+    if (there)
+      for (int32_t c = tid; c < cols; c += nt) CpAsync4(ring + slot * pitch + c, src + c);
     CpAsyncCommit();
+    src += src_step;
   };
-  for (int32_t step = 1; step <= kVitAhead; ++step) issue_row(step, (step - 1) % kVitRing);
-  float *grid = (dir == 0 ? fwd : bwd) + f.grid_off;
-  for (int32_t q = tid; q < S; q += nt) {
-    const float v0 = (dir == 0 ? (q == 0) : (q == S - 1)) ? 0.0f : -INFINITY;
-    buf[0][q] = v0;
-    grid[(int64_t)(dir == 0 ? 0 : Tk) * S + q] = v0;
-  }
+  if (copies)
+    for (int32_t step = 1; step <= kVitAhead; ++step) issue_row(step <= Tk, (step - 1) % kVitRing);
   const int64_t stride = dir == 0 ? (int64_t)S : -(int64_t)S;
-  float *gout = grid + (dir == 0 ? 1 : Tk - 1) * (int64_t)S;
+  const bool store = s >= 0 && g == 0;
+  float *gout;
+  {
+    float *grid = (dir == 0 ? fwd : bwd) + infos[i].grid_off;
+    for (int32_t q = tid; q < S; q += nt) {
+      const float v0 = (dir == 0 ? (q == 0) : (q == S - 1)) ? 0.0f : -INFINITY;
+      buf[0][q] = v0;
+      grid[(int64_t)(dir == 0 ? 0 : Tk) * S + q] = v0;
+    }
+    gout = grid + (dir == 0 ? 1 : Tk - 1) * (int64_t)S + max(s, 0);
+  }
   // the frame loop once per kind of CTA, so that the unrolled code of only one is fetched
   auto frames = [&](auto hoist_tag) {
     constexpr bool kHoist = decltype(hoist_tag)::value;
-  for (int32_t t0 = 1; t0 <= Tk; t0 += kVitRing) {
+    for (int32_t t0 = 1; t0 <= Tk; t0 += kVitRing) {
 #pragma unroll
       for (int u = 0; u < kVitRing; ++u) {
         const int32_t t = t0 + u;
         if (t > Tk) break;
-        CpAsyncWait<kVitAhead - 1>();  // this thread's part of row t has landed
-        __syncthreads();               // ... everyone's has; the scores of step t - 1 are complete
-        issue_row(t + kVitAhead, (u + kVitAhead) % kVitRing);
-        const float *cur = buf[u & 1];  // t0 is odd: (t - 1) & 1 == u & 1
-        const float *row = ring + u * cols_pad;
-        float best[kV];
+        if (copies) CpAsyncWait<kVitAhead - 1>();  // this thread's part of row t has landed
+        __syncthreads();  // ... everyone's has; the scores of step t - 1 are complete
+        if (copies) issue_row(t + kVitAhead <= Tk, (u + kVitAhead) % kVitRing);
+        // t0 is odd: (t - 1) & 1 == u & 1
+        const char *cur = reinterpret_cast<const char *>(buf[u & 1]);
+        const char *row = reinterpret_cast<const char *>(ring + u * pitch);
+        auto at = [](const char *base, uint32_t off) {
+          return *reinterpret_cast<const float *>(base + off);
+        };
+        // (a max of two chains: NaN never wins, as in the reference's comparisons)
+        float best = -INFINITY, best1 = -INFINITY;
 #pragma unroll
-        for (int v = 0; v < kV; ++v) {
-          best[v] = -INFINITY;
-          if (kHoist) {
+        for (int j = 0; j < kDeg; j += 2) {
+          float x = __fadd_rn(at(cur, other[j]), w[j]);
+          float y = __fadd_rn(at(cur, other[j + 1]), w[j + 1]);
+          if (!kHoist) {
+            x = __fadd_rn(x, at(row, col[j]));
+            y = __fadd_rn(y, at(row, col[j + 1]));
+          }
+          best = fmaxf(best, x);
+          best1 = fmaxf(best1, y);
+        }
+        best = fmaxf(best, best1);
 #pragma unroll
-            for (int j = 0; j < kDeg; ++j) {
-              const float x = __fadd_rn(cur[other[v][j]], w[v][j]);
-              best[v] = x > best[v] ? x : best[v];
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < kDeg; ++j) {
-              const float x = __fadd_rn(__fadd_rn(cur[other[v][j]], w[v][j]), row[col[v][j]]);
-              best[v] = x > best[v] ? x : best[v];
-            }
+        for (int32_t d = 16; d > 0; d >>= 1) {
+          if (d < g_max) {  // warp-uniform
+            const float o = __shfl_down_sync(0xffffffffu, best, d);
+            if (g + d < G) best = fmaxf(best, o);
           }
         }
-#pragma unroll
-        for (int v = 0; v < kV; ++v) {
-#pragma unroll
-          for (int32_t d = 16; d > 0; d >>= 1) {
-            if (d < g_max[v]) {  // warp-uniform
-              const float o = __shfl_down_sync(0xffffffffu, best[v], d);
-              if (g[v] + d < G[v]) best[v] = o > best[v] ? o : best[v];
-            }
-          }
-          if (s[v] >= 0 && g[v] == 0) {
-            if (kHoist) best[v] = __fadd_rn(best[v], row[col0[v]]);
-            buf[(u + 1) & 1][s[v]] = best[v];
-            gout[s[v]] = best[v];
-          }
+        if (store) {
+          if (kHoist) best = __fadd_rn(best, at(row, col0_off));
+          buf[(u + 1) & 1][s] = best;
+          *gout = best;
         }
         gout += stride;
       }
@@ -498,17 +500,23 @@ int32_t LaunchLanesViterbi(const Layout &L, const k2b200_intersect_args *a,
                            const FsaInfo *d_infos, float *fwd, float *bwd, const int32_t *plan,
                            const int32_t *unfit, cudaStream_t stream) {
   (void)L;
+  static_assert(kLaneDeg % 2 == 0, "arcs are taken in pairs");
   dim3 grid(2, a->num_fsas);
   const int32_t cols_pad = (a->cols + 3) & ~3;
-  const size_t smem = sizeof(float) * kVitRing * (size_t)cols_pad;
-  K2B_REQUIRE(smem <= 200 * 1024, "too many columns for the lane Viterbi kernel");
-  constexpr int kV = 1;  // plan lanes per thread (2 was slower: 0.39 against 0.30 ms at 500 frames)
-  K2B_CUDA_OK(cudaFuncSetAttribute(LanesViterbi<kLaneDeg, kV>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  { LanesViterbi<kLaneDeg, kV><<<grid, kLaneThreads / kV, smem, stream>>>(
-      d_infos, a->num_fsas, reinterpret_cast<const Arc *>(a->a_arcs), a->a_row_splits2,
-      a->a_in_splits, a->a_in_arcs, a->scores, a->cols, cols_pad, fwd, bwd, plan, unfit);
-    NoteLaunch(); }
+  auto launch = [&](auto kernel, int32_t pitch) -> int32_t {
+    const size_t smem = sizeof(float) * kVitRing * (size_t)pitch;
+    K2B_REQUIRE(smem <= 200 * 1024, "too many columns for the lane Viterbi kernel");
+    K2B_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)smem));
+    kernel<<<grid, kLaneThreads, smem, stream>>>(
+        d_infos, a->num_fsas, reinterpret_cast<const Arc *>(a->a_arcs), a->a_row_splits2,
+        a->a_in_splits, a->a_in_arcs, a->scores, a->cols, cols_pad, fwd, bwd, plan, unfit);
+    NoteLaunch();
+    return kOk;
+  };
+  // graphs over phones have rows of up to 128 columns
+  if (a->cols <= 128) K2B_FORWARD(launch(LanesViterbi<kLaneDeg, 128>, 128));
+  else K2B_FORWARD(launch(LanesViterbi<kLaneDeg, 0>, cols_pad));
   K2B_CUDA_OK(cudaGetLastError());
   return kOk;
 }
