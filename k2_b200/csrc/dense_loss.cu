@@ -421,20 +421,20 @@ GridChainLanes(const FsaInfo *__restrict__ infos, int32_t n, const Arc *__restri
 // is unrolled, so the score of an arc's other end is one load at (byte offset of that state,
 // fixed for the call) + constant.  Walking forward in a graph where every state has one
 // entering label the dense score of a lane's arcs is one load per row.
-template <int kDeg, int kSPad, int kMaskRows>
-__global__ void __launch_bounds__(kLaneThreads)
+template <int kDeg, int kThreads, int kSPad, int kMaskRows>
+__global__ void __launch_bounds__(kThreads)
 ArcMasks(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_levels,
          const Arc *__restrict__ arcs, const int32_t *__restrict__ a_row_splits2,
          const int32_t *__restrict__ in_splits, const int32_t *__restrict__ in_arcs,
          const unsigned char *__restrict__ dense, DensePack dp,
          const float *__restrict__ vfwd, const float *__restrict__ vbwd,
          const float *__restrict__ cutoffs, const int32_t *__restrict__ plan,
-         int32_t *__restrict__ unfit, unsigned char *__restrict__ masks) {
+         int32_t *__restrict__ unfit, unsigned char *__restrict__ masks, int32_t mask_pitch) {
   static_assert(kDeg <= 8, "one byte per lane");
   constexpr int32_t s_pad = kSPad;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int32_t i = blockIdx.y, dir = blockIdx.z;
-  if (unfit[i] & 1) return;
+  if ((unfit[i] & 1) || unfit[n + i] != LaneClass(kThreads)) return;
   const FsaInfo f = infos[i];
   const int32_t S = f.num_states, Tk = f.tk, cols = dp.cols;
   const int32_t r0 = blockIdx.x * kMaskRows + (dir == 0 ? 1 : 0);
@@ -508,7 +508,8 @@ ArcMasks(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_levels,
   const uint32_t col0_off = 4u * (uint32_t)(col0 < 0 ? 0 : col0);
   __syncthreads();
   // (a slot without an arc has w = -inf: it fails the test like any pruned arc)
-  unsigned char *out = masks + ((int64_t)dir * total_levels + f.level_off + r0) * kLaneThreads + tid;
+  unsigned char *out = masks + ((int64_t)dir * total_levels + f.level_off) * mask_pitch +
+                       (int64_t)r0 * kThreads + tid;
   const int32_t s_ld = s >= 0 ? s : 0;
   // dir 0: arcs from level k into level k + 1 (own); dir 1: from level k (own) to k + 1
   const float *own_p = (dir == 0 ? bo + s_pad : fo) + s_ld;
@@ -550,12 +551,12 @@ ArcMasks(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_levels,
           }
         }
       }
-      out[(int64_t)u * kLaneThreads] = (unsigned char)bits;
+      out[(int64_t)u * kThreads] = (unsigned char)bits;
     }
     own_p += kUnroll * s_pad;
     oth_p += kUnroll * 4 * s_pad;
     lp_p += kUnroll * lp_stride;
-    out += (int64_t)kUnroll * kLaneThreads;
+    out += (int64_t)kUnroll * kThreads;
   }
   if (__syncthreads_or(risky) && tid == 0) atomicOr(&unfit[i], 2);
 }
@@ -575,8 +576,8 @@ ArcMasks(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_levels,
 // ---------------------------------------------------------------------------
 constexpr int kMaskedBatches = 3;  // batches of kU frames in the ring
 
-template <int kDeg, int kU>
-__global__ void __launch_bounds__(kLaneThreads)
+template <int kDeg, int kThreads, int kU>
+__global__ void __launch_bounds__(kThreads)
 GridChainMasked(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_levels,
                 const Arc *__restrict__ arcs, const int32_t *__restrict__ a_row_splits2,
                 const int32_t *__restrict__ in_splits, const int32_t *__restrict__ in_arcs,
@@ -585,7 +586,7 @@ GridChainMasked(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_leve
                 const float *__restrict__ vbwd, const float *__restrict__ cutoffs,
                 ProbState *__restrict__ alpha, ProbState *__restrict__ beta,
                 double *__restrict__ tot, const int32_t *__restrict__ plan,
-                int32_t *__restrict__ unfit, int32_t s_pad, int32_t wait_limit) {
+                int32_t *__restrict__ unfit, int32_t mask_pitch, int32_t wait_limit) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full[kMaskedBatches];
   __shared__ int32_t emax;
@@ -593,7 +594,8 @@ GridChainMasked(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_leve
   constexpr int32_t kNone = INT32_MIN;
   const int32_t i = blockIdx.y;
   const int dir = blockIdx.x;
-  if (unfit[i]) return;  // no plan, or outside the limits: the fallback kernel takes it
+  // no plan, or outside the limits: the fallback kernel takes it; or of the other CTA size
+  if (unfit[i] || unfit[n + i] != LaneClass(kThreads)) return;
   const FsaInfo f = infos[i];
   const int32_t S = f.num_states, Tk = f.tk, cols = dp.cols;
   const int tid = threadIdx.x, nt = blockDim.x;
@@ -601,10 +603,9 @@ GridChainMasked(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_leve
     if (dir == 0 && tid == 0) tot[i] = -INFINITY;
     return;
   }
-  (void)s_pad;
-  constexpr int kSPad = kLaneThreads;  // a planned graph has at most that many states
+  constexpr int kSPad = kThreads;  // a planned graph has at most that many states
   // a batch: kU packed dense rows, then kU rows of mask bytes
-  const uint32_t batch_bytes = (uint32_t)kU * ((uint32_t)dp.pitch + (uint32_t)kLaneThreads);
+  const uint32_t batch_bytes = (uint32_t)kU * ((uint32_t)dp.pitch + (uint32_t)kThreads);
   unsigned char *ring = smem_raw;                                  // [kMaskedBatches][batch_bytes]
   double *pv = reinterpret_cast<double *>(ring + (size_t)kMaskedBatches * batch_bytes);  // [2][kSPad]
   int32_t s = -1, g = 0, G = 1;
@@ -679,7 +680,7 @@ GridChainMasked(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_leve
   const int64_t step_stride = dir == 0 ? (int64_t)S : -(int64_t)S;
   const unsigned char *dense_rows = dense + (int64_t)f.row0 * dp.pitch;
   const uint32_t row_bytes = (uint32_t)dp.pitch, lp_bytes = 4u * (uint32_t)dp.cols4;
-  const unsigned char *mask0 = masks + ((int64_t)dir * total_levels + f.level_off) * kLaneThreads;
+  const unsigned char *mask0 = masks + ((int64_t)dir * total_levels + f.level_off) * mask_pitch;
   const int32_t num_batches = (Tk + kU - 1) / kU;
   // thread 0: the rows of steps b * kU + 1 .. of batch b, as two copies.  Walking forward the
   // dense rows and the mask rows of consecutive steps ascend, walking backward they descend:
@@ -692,9 +693,9 @@ GridChainMasked(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_leve
     const int64_t r_lo = dir == 0 ? t_first : Tk - t_first - nf + 1;        // mask rows
     const int32_t slot = b % kMaskedBatches;
     unsigned char *dst = ring + (size_t)slot * batch_bytes;
-    MbarArriveExpectTx(&full[slot], (unsigned)nf * (row_bytes + (unsigned)kLaneThreads));
+    MbarArriveExpectTx(&full[slot], (unsigned)nf * (row_bytes + (unsigned)kThreads));
     BulkCopyG2S(dst, dense_rows + row_lo * row_bytes, (unsigned)nf * row_bytes, &full[slot]);
-    BulkCopyG2S(dst + kU * row_bytes, mask0 + r_lo * kLaneThreads, (unsigned)nf * kLaneThreads,
+    BulkCopyG2S(dst + kU * row_bytes, mask0 + r_lo * kThreads, (unsigned)nf * kThreads,
                 &full[slot]);
   };
   if (tid == 0)
@@ -741,7 +742,7 @@ GridChainMasked(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_leve
         double *cur = pv + ((pb + u + 1) & 1) * kSPad;
         const int32_t idx = dir == 0 ? u : nf - 1 - u;
         const unsigned char *prow = base + (uint32_t)idx * row_bytes + lp_bytes;
-        const uint32_t m = (base + kU * row_bytes + (uint32_t)idx * kLaneThreads)[tid];
+        const uint32_t m = (base + kU * row_bytes + (uint32_t)idx * kThreads)[tid];
         auto at = [](const unsigned char *p0, uint32_t off) {
           return *reinterpret_cast<const double *>(p0 + off);
         };
@@ -1194,8 +1195,8 @@ GridGradItems(const FsaInfo *__restrict__ infos, const Arc *__restrict__ arcs,
 // lane walks the chunk's frames over the arcs it holds in registers (leaving
 // order, the plan of the backward recursion) with no further barrier.
 // ---------------------------------------------------------------------------
-template <int kDeg>
-__global__ void __launch_bounds__(kLaneThreads)
+template <int kDeg, int kThreads>
+__global__ void __launch_bounds__(kThreads)
 GridGradLanes(const FsaInfo *__restrict__ infos, int32_t n, const Arc *__restrict__ arcs,
               const int32_t *__restrict__ a_row_splits2, const unsigned char *__restrict__ dense,
               DensePack dp, const unsigned char *__restrict__ masks, int64_t total_levels,
@@ -1203,13 +1204,14 @@ GridGradLanes(const FsaInfo *__restrict__ infos, int32_t n, const Arc *__restric
               const ProbState *__restrict__ beta, const double *__restrict__ tot_grad,
               int32_t tot_grad_stride, float *__restrict__ grad_a, float *__restrict__ grad_b,
               const int32_t *__restrict__ plan, const int32_t *__restrict__ unfit,
-              int32_t frames_per_cta, int32_t sub_frames, int32_t s_pad,
+              int32_t mask_pitch, int32_t frames_per_cta, int32_t sub_frames, int32_t s_pad,
               int32_t exclusive_rows, const int32_t *__restrict__ lp_row, int32_t lp_cols,
               const int32_t *__restrict__ served) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int32_t i = blockIdx.y;
   if (served != nullptr && *served) return;  // GridGradStates wrote the gradients
-  if (unfit[i] & 1) return;  // no plan: the warp-per-frame kernel takes this graph
+  // no plan: the warp-per-frame kernel takes this graph; or of the other CTA size
+  if ((unfit[i] & 1) || unfit[n + i] != LaneClass(kThreads)) return;
   const FsaInfo f = infos[i];
   const int32_t S = f.num_states, Tk = f.tk, cols = dp.cols;
   const int32_t cta_u0 = blockIdx.x * frames_per_cta;
@@ -1228,8 +1230,8 @@ GridGradLanes(const FsaInfo *__restrict__ infos, int32_t n, const Arc *__restric
   // posteriors per (frame, column) in fixed point, 2^-31 units: integer atomics are
   // native in shared memory (float ones are compare-and-swap loops) and make the sum
   // independent of the order of the additions
-  unsigned char *mk = rows + (size_t)sub_frames * dp.pitch;  // [sub_frames][kLaneThreads]
-  uint32_t *gb = reinterpret_cast<uint32_t *>(mk + (size_t)sub_frames * kLaneThreads);
+  unsigned char *mk = rows + (size_t)sub_frames * dp.pitch;  // [sub_frames][kThreads]
+  uint32_t *gb = reinterpret_cast<uint32_t *>(mk + (size_t)sub_frames * kThreads);
   const ProbState *al = alpha + f.grid_off, *be = beta + f.grid_off;
   const ProbState z = al[(int64_t)Tk * S + (S - 1)];
   if (z.m == 0.0) return;  // no path survives: all gradients are zero
@@ -1239,7 +1241,7 @@ GridGradLanes(const FsaInfo *__restrict__ infos, int32_t n, const Arc *__restric
   const float tg = (float)tot_grad[(int64_t)i * tot_grad_stride];
   const int32_t zk = -(z.e + zex);
   // survival bits of the lanes' arcs, one row of bytes per level (ArcMasks, direction 1)
-  const unsigned char *mask0 = masks + (total_levels + f.level_off) * (int64_t)kLaneThreads;
+  const unsigned char *mask0 = masks + (total_levels + f.level_off) * (int64_t)mask_pitch;
   // ---- this lane's arcs --------------------------------------------------------
   int32_t s = -1, g = 0, G = 1;
   {
@@ -1311,16 +1313,16 @@ GridGradLanes(const FsaInfo *__restrict__ infos, int32_t n, const Arc *__restric
     }
     for (int32_t k = tid; k < nf * cols; k += nt) gb[k] = 0u;
     {
-      const uint4 *src = reinterpret_cast<const uint4 *>(mask0 + (int64_t)u0 * kLaneThreads);
+      const uint4 *src = reinterpret_cast<const uint4 *>(mask0 + (int64_t)u0 * kThreads);
       uint4 *dst = reinterpret_cast<uint4 *>(mk);
-      for (int32_t k = tid; k < nf * (kLaneThreads / 16); k += nt) dst[k] = src[k];
+      for (int32_t k = tid; k < nf * (kThreads / 16); k += nt) dst[k] = src[k];
     }
     __syncthreads();
     if (s >= 0) {
       for (int32_t l = 0; l < nf; ++l) {
         const double own_am = st_am[l * s_pad + s];
         if (own_am == 0.0) continue;  // pruned or unreachable
-        const uint32_t m = mk[l * kLaneThreads + tid];
+        const uint32_t m = mk[l * kThreads + tid];
         if (m == 0) continue;
         const int32_t own_ae = st_ae[l * s_pad + s];
         const int32_t nx = (l + 1) * s_pad;
@@ -1648,7 +1650,7 @@ static int32_t MakeLossLayout(const k2b200_intersect_args *a, LossLayout *LL) {
   LL->pack = MakeDensePack(a->cols);
   LL->identity = !LL->base.lane_plan;
   LL->k_deg = LL->identity ? (a->a_max_degree <= 3 ? 3 : 4) : kLaneDeg;
-  LL->threads = LL->identity ? std::max(32, (LL->base.max_states + 31) / 32 * 32) : kLaneThreads;
+  LL->threads = LL->identity ? std::max(32, (LL->base.max_states + 31) / 32 * 32) : LL->base.lane_threads;
   size_t off = AlignUp(LL->base.total_bytes);
   auto take = [&](size_t bytes) {
     size_t o = off;
@@ -1660,7 +1662,7 @@ static int32_t MakeLossLayout(const k2b200_intersect_args *a, LossLayout *LL) {
   LL->off_alpha = take(sizeof(ProbState) * (size_t)LL->base.grid_elems);
   LL->off_beta = take(sizeof(ProbState) * (size_t)LL->base.grid_elems);
   // arc survival bytes, planned graphs only: [2 directions][levels][lanes]
-  LL->off_masks = take(LL->identity ? 0 : (size_t)2 * LL->base.total_levels * kLaneThreads + 16);
+  LL->off_masks = take(LL->identity ? 0 : (size_t)2 * LL->base.total_levels * LL->threads + 16);
   LL->off_flags = take(sizeof(int32_t));
   LL->off_state_label = take(sizeof(int32_t) * (size_t)std::max(a->num_states, 1));
   LL->off_one_label = take(sizeof(int32_t));
@@ -1708,10 +1710,10 @@ static int32_t LaunchChainLanes(const LossLayout &LL, const k2b200_intersect_arg
 }
 
 // Planned graphs: survival masks for all frames, then the mask-driven recursion.
+template <int kThreads>
 static int32_t LaunchChainMasked(const LossLayout &LL, const k2b200_intersect_args *args,
                                  char *ws, double *tot, cudaStream_t stream) {
   const Layout &L = LL.base;
-  const int32_t s_pad = (L.max_states + 3) & ~3;
   const FsaInfo *d_infos = reinterpret_cast<const FsaInfo *>(ws + L.off_infos);
   const Arc *arcs = reinterpret_cast<const Arc *>(args->a_arcs);
   const unsigned char *dense = reinterpret_cast<const unsigned char *>(ws + LL.off_dense);
@@ -1727,42 +1729,43 @@ static int32_t LaunchChainMasked(const LossLayout &LL, const k2b200_intersect_ar
       const size_t smem = sizeof(float) * ((size_t)2 * ((ROWS) + 1) * (SPAD) +                 \
                                            (size_t)(ROWS) * LL.pack.cols4);                    \
       K2B_REQUIRE(smem <= kChainSmemBudget, "too many columns for the fused loss path");       \
-      K2B_CUDA_OK(cudaFuncSetAttribute(ArcMasks<kLaneDeg, SPAD, ROWS>,                         \
+      K2B_CUDA_OK(cudaFuncSetAttribute(ArcMasks<kLaneDeg, kThreads, SPAD, ROWS>,                         \
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,            \
                                        (int)smem));                                            \
       dim3 grid(CeilDiv(L.max_tk + 1, (ROWS)), args->num_fsas, 2);                             \
-      { ArcMasks<kLaneDeg, SPAD, ROWS><<<grid, kLaneThreads, smem, stream>>>(                  \
+      { ArcMasks<kLaneDeg, kThreads, SPAD, ROWS><<<grid, kThreads, smem, stream>>>(                  \
           d_infos, args->num_fsas, L.total_levels, arcs, args->a_row_splits2,                  \
           args->a_in_splits, args->a_in_arcs, dense, LL.pack, fwd, bwd, cutoffs, plan, unfit,  \
-          masks); NoteLaunch(); }                                                              \
+          masks, LL.threads); NoteLaunch(); }                                                  \
     }
     // state pitch of the staged Viterbi scores, in three sizes
     if (L.max_states <= 192) K2B_ARC_MASKS(192, 56)
     else if (L.max_states <= 384) K2B_ARC_MASKS(384, 32)
-    else K2B_ARC_MASKS(768, 16)
+    else if (L.max_states <= 768) K2B_ARC_MASKS(768, 16)
+    else K2B_ARC_MASKS(1024, 16)
 #undef K2B_ARC_MASKS
   }
   {
     dim3 grid(2, args->num_fsas);
 #define K2B_CHAIN_MASKED(KU)                                                                  \
     {                                                                                         \
-      const size_t smem = (size_t)kMaskedBatches * (KU) * ((size_t)LL.pack.pitch + kLaneThreads) + \
-                          sizeof(double) * 2 * kLaneThreads;                                  \
-      K2B_CUDA_OK(cudaFuncSetAttribute(GridChainMasked<kLaneDeg, KU>,                         \
+      const size_t smem = (size_t)kMaskedBatches * (KU) * ((size_t)LL.pack.pitch + kThreads) + \
+                          sizeof(double) * 2 * kThreads;                                  \
+      K2B_CUDA_OK(cudaFuncSetAttribute(GridChainMasked<kLaneDeg, kThreads, KU>,                         \
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,           \
                                        (int)smem));                                           \
-      { GridChainMasked<kLaneDeg, KU><<<grid, kLaneThreads, smem, stream>>>(                  \
+      { GridChainMasked<kLaneDeg, kThreads, KU><<<grid, kThreads, smem, stream>>>(                  \
           d_infos, args->num_fsas, L.total_levels, arcs, args->a_row_splits2,                 \
           args->a_in_splits, args->a_in_arcs, dense, LL.pack, masks, fwd, bwd, cutoffs,       \
           reinterpret_cast<ProbState *>(ws + LL.off_alpha),                                   \
-          reinterpret_cast<ProbState *>(ws + LL.off_beta), tot, plan, unfit, s_pad,           \
+          reinterpret_cast<ProbState *>(ws + LL.off_beta), tot, plan, unfit, LL.threads,                                   \
           CopyWaitLimit());                                                                   \
         NoteLaunch(); }                                                                       \
     }
     // frames per batch (one bulk copy of dense rows and one of mask rows each): as many as
     // three batches of them leave room for in shared memory
-    const size_t per_frame = (size_t)kMaskedBatches * ((size_t)LL.pack.pitch + kLaneThreads);
-    const size_t room = kChainSmemBudget - sizeof(double) * 2 * kLaneThreads;
+    const size_t per_frame = (size_t)kMaskedBatches * ((size_t)LL.pack.pitch + kThreads);
+    const size_t room = kChainSmemBudget - sizeof(double) * 2 * kThreads;
     K2B_REQUIRE(per_frame <= room, "too many columns for the fused loss path");
     if (4 * per_frame <= room) K2B_CHAIN_MASKED(4)
     else if (2 * per_frame <= room) K2B_CHAIN_MASKED(2)
@@ -1859,26 +1862,32 @@ static int32_t LaunchGradLanes(const LossLayout &LL, const k2b200_intersect_args
   const int32_t s_pad = (L.max_states + 3) & ~3;
   auto bytes_for = [&](int32_t frames) {
     return (size_t)24 * (frames + 1) * s_pad + (size_t)frames * LL.pack.pitch +
-           (size_t)frames * kLaneThreads + sizeof(float) * (size_t)frames * args->cols;
+           (size_t)frames * LL.threads + sizeof(float) * (size_t)frames * args->cols;
   };
   int32_t sub = 16;
   while (sub > 1 && bytes_for(sub) > 100 * 1024) sub >>= 1;
   const size_t smem = bytes_for(sub);
   const int32_t frames = 4 * sub;  // per CTA: amortises loading the arcs and adding grad_a
   K2B_REQUIRE(smem <= kChainSmemBudget, "graphs too large for the fused loss path");
-  K2B_CUDA_OK(cudaFuncSetAttribute(GridGradLanes<kLaneDeg>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   dim3 grid(CeilDiv(L.max_tk, frames), args->num_fsas);
-  { GridGradLanes<kLaneDeg><<<grid, kLaneThreads, smem, stream>>>(
-      reinterpret_cast<const FsaInfo *>(ws + L.off_infos), args->num_fsas,
-      reinterpret_cast<const Arc *>(args->a_arcs), args->a_row_splits2,
-      reinterpret_cast<const unsigned char *>(ws + LL.off_dense), LL.pack,
-      reinterpret_cast<const unsigned char *>(ws + LL.off_masks), L.total_levels,
-      reinterpret_cast<const ProbState *>(ws + LL.off_alpha),
-      reinterpret_cast<const ProbState *>(ws + LL.off_beta), tot_grad, stride, grad_a, grad_b,
-      reinterpret_cast<const int32_t *>(ws + L.off_plan),
-      reinterpret_cast<const int32_t *>(ws + L.off_unfit), frames, sub, s_pad,
-      LL.exclusive_rows ? 1 : 0, LL.lp_row, LL.lp_cols, LL.served); NoteLaunch(); }
+#define K2B_GRAD_LANES(THREADS)                                                               \
+  {                                                                                           \
+    K2B_CUDA_OK(cudaFuncSetAttribute(GridGradLanes<kLaneDeg, THREADS>,                        \
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+    GridGradLanes<kLaneDeg, THREADS><<<grid, THREADS, smem, stream>>>(                        \
+        reinterpret_cast<const FsaInfo *>(ws + L.off_infos), args->num_fsas,                  \
+        reinterpret_cast<const Arc *>(args->a_arcs), args->a_row_splits2,                     \
+        reinterpret_cast<const unsigned char *>(ws + LL.off_dense), LL.pack,                  \
+        reinterpret_cast<const unsigned char *>(ws + LL.off_masks), L.total_levels,           \
+        reinterpret_cast<const ProbState *>(ws + LL.off_alpha),                               \
+        reinterpret_cast<const ProbState *>(ws + LL.off_beta), tot_grad, stride, grad_a,      \
+        grad_b, reinterpret_cast<const int32_t *>(ws + L.off_plan),                           \
+        reinterpret_cast<const int32_t *>(ws + L.off_unfit), LL.threads, frames, sub, s_pad,  \
+        LL.exclusive_rows ? 1 : 0, LL.lp_row, LL.lp_cols, LL.served);                         \
+    NoteLaunch();                                                                             \
+  }
+  K2B_LANE_THREADS(LL.threads, K2B_GRAD_LANES);
+#undef K2B_GRAD_LANES
   K2B_CUDA_OK(cudaGetLastError());
   return kOk;
 }
@@ -1997,7 +2006,10 @@ int32_t k2b200_dense_loss_forward(const k2b200_intersect_args *args, void *works
       else if (LL.k_deg == 4 && LL.threads <= 512) K2B_FORWARD(K2B_CHAIN(4, 512));
       else if (LL.k_deg == 4) K2B_FORWARD(K2B_CHAIN(4, 1024));
       else
-        K2B_FORWARD(LaunchChainMasked(LL, args, ws, tot_scores, stream));
+#define K2B_MASKED(THREADS) \
+  K2B_FORWARD(LaunchChainMasked<THREADS>(LL, args, ws, tot_scores, stream));
+        K2B_LANE_THREADS(LL.threads, K2B_MASKED);
+#undef K2B_MASKED
 #undef K2B_CHAIN
     // graphs the lane kernel skipped or gave up on
     K2B_CUDA_OK(cudaFuncSetAttribute(GridChain, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -114,8 +114,9 @@ int32_t MakeLayout(const k2b200_intersect_args *a, Layout *L) {
   L->off_block_cand = take(sizeof(unsigned long long) * (size_t)L->count_blocks);
   L->off_totals = take(64);
   L->lane_plan = LanePlanApplies(*L, a);
+  L->lane_threads = LaneThreads(*L);
   L->off_plan = take(L->lane_plan ? sizeof(int32_t) * 2 * (size_t)a->num_fsas * kLaneThreads : 0);
-  L->off_unfit = take(sizeof(int32_t) * (size_t)a->num_fsas);
+  L->off_unfit = take(sizeof(int32_t) * 2 * (size_t)a->num_fsas);
   // a shared graph too large for the one-CTA kernels: sequences on the lanes of a warp
   L->shared_vit = (a->viterbi_mode == 5 ||
                    (a->viterbi_mode == 0 && !RegisterViterbiFits(*L, a) && !L->lane_plan &&

@@ -36,6 +36,7 @@ struct Layout {
   // graphs with states of more than four arcs, small enough for one CTA: lanes are
   // assigned to states by a plan (viterbi_persistent.cu)
   bool lane_plan = false;
+  int32_t lane_threads = 0;
   int32_t count_blocks, tiles_per_pair, words_per_warp;
 };
 
@@ -67,11 +68,24 @@ int32_t LaunchPersistentViterbi(const Layout &L, const k2b200_intersect_args *a,
                                 const FsaInfo *d_infos, float *fwd, float *bwd,
                                 cudaStream_t stream, const int32_t *only_unfit = nullptr);
 
-// Lane plans: CTA size and arcs per lane of the kernels that use them.
-constexpr int kLaneThreads = 768;
+// Lane plans: the most lanes a graph may need, and arcs per lane.
+constexpr int kLaneThreads = 1024;
 constexpr int kLaneDeg = 8;
+// The kernels that use plans have CTAs of 768 threads, with 80 registers each, and again of 1024
+// with 64 for the graphs that need more lanes: the plan says which (LaneClass).  The second
+// launch is left out when no graph can need it - states + arcs / kLaneDeg, and what packing
+// them into warps leaves unused.  (Without it a denominator graph over 80 to 100 phones
+// fell back to the kernels without plans, at three to four times the time.)
+int32_t LaneThreads(const Layout &L);
+__device__ __forceinline__ int32_t LaneClass(int32_t threads) { return threads > 768 ? 1 : 0; }
+#define K2B_LANE_THREADS(THREADS, CALL) \
+  do {                                  \
+    CALL(768)                           \
+    if ((THREADS) > 768) CALL(1024)     \
+  } while (0)
 bool LanePlanApplies(const Layout &L, const k2b200_intersect_args *a);
-// Clears unfit[] and, when L.lane_plan, writes the plans of both directions.
+// Clears unfit[] and, when L.lane_plan, writes the plans of both directions; unfit[n + i] is the
+// class of graph i.
 int32_t LaunchPlanLanes(const Layout &L, const k2b200_intersect_args *a, char *ws,
                         cudaStream_t stream);
 int32_t LaunchLanesViterbi(const Layout &L, const k2b200_intersect_args *a,

@@ -232,8 +232,7 @@ RegisterViterbi(const FsaInfo *__restrict__ infos, const Arc *__restrict__ arcs,
 // Lane plans.  The recursion kernel keeps the arcs of state s in the registers of
 // G(s) = ceil(degree(s) / kDeg) lanes of one warp, so that a frame costs every lane
 // the same few arcs whatever the degree distribution of the graph is.  PlanLanes
-// lays the lane groups of one graph and direction out over a CTA of kLaneThreads
-// threads: groups sorted by size, largest first (states in increasing order within
+// lays the lane groups of one graph and direction out over the threads of a CTA: groups sorted by size, largest first (states in increasing order within
 // a size), packed next-fit into warps - a group never straddles two warps.
 //   plan[(dir * n + i) * kLaneThreads + thread] = state | lane << 16 | G << 24, or -1
 // bit 0 of unfit[i] is set when graph i needs more lanes than a CTA has (or has more than
@@ -243,7 +242,7 @@ RegisterViterbi(const FsaInfo *__restrict__ infos, const Arc *__restrict__ arcs,
 __global__ void __launch_bounds__(256)
 PlanLanes(const FsaInfo *__restrict__ infos, int32_t n,
           const int32_t *__restrict__ a_row_splits2, const int32_t *__restrict__ in_splits,
-          int32_t k_deg, int32_t *__restrict__ plan, int32_t *__restrict__ unfit) {
+          int32_t k_deg, int32_t threads, int32_t *__restrict__ plan, int32_t *__restrict__ unfit) {
   // per group size G = 1..32: number of states, lanes left in the warp where the
   // size class starts, first lane of that start, first lane of the following warps
   __shared__ int32_t count[33], head_room[33], head_pos[33], body_pos[33];
@@ -255,14 +254,14 @@ PlanLanes(const FsaInfo *__restrict__ infos, int32_t n,
   int32_t *out = plan + ((int64_t)dir * n + i) * kLaneThreads;
   for (int32_t t = tid; t < kLaneThreads; t += nt) out[t] = -1;
   if (tid < 33) count[tid] = 0;
-  if (tid == 0) bad = S > kLaneThreads;
+  if (tid == 0) bad = S > threads;
   __syncthreads();
   const int32_t *splits = (dir == 0 ? in_splits : a_row_splits2) + f.state_off;
   auto lanes_of = [&](int32_t s) {
     const int32_t deg = splits[s + 1] - splits[s];
     return deg <= k_deg ? 1 : (deg + k_deg - 1) / k_deg;
   };
-  if (S <= kLaneThreads)
+  if (S <= threads)
     for (int32_t s = tid; s < S; s += nt) {
       const int32_t G = lanes_of(s);
       if (G > 32) bad = 1; else atomicAdd(&count[G], 1);
@@ -285,8 +284,9 @@ PlanLanes(const FsaInfo *__restrict__ infos, int32_t n,
         body_pos[G] = body;
         pos = body + (rest / per_warp) * 32 + (rest % per_warp) * G;
       }
-      if (pos > kLaneThreads) bad = 1;
+      if (pos > threads) bad = 1;
     }
+    if (!bad && (pos > 768 || S > 768)) atomicOr(&unfit[n + i], 1);
   }
   __syncthreads();
   if (bad) {
@@ -320,6 +320,10 @@ PlanLanes(const FsaInfo *__restrict__ infos, int32_t n,
 }
 
 
+int32_t LaneThreads(const Layout &L) {
+  return L.max_states + L.max_arcs / kLaneDeg <= 736 ? 768 : 1024;
+}
+
 bool LanePlanApplies(const Layout &L, const k2b200_intersect_args *a) {
   const bool register_fit = a->a_max_degree > 0 && a->a_max_degree <= 4 && L.max_states <= 1024;
   return !register_fit && L.max_states <= kLaneThreads && a->num_fsas <= 65535 &&
@@ -329,11 +333,12 @@ bool LanePlanApplies(const Layout &L, const k2b200_intersect_args *a) {
 int32_t LaunchPlanLanes(const Layout &L, const k2b200_intersect_args *a, char *ws,
                         cudaStream_t stream) {
   int32_t *unfit = reinterpret_cast<int32_t *>(ws + L.off_unfit);
-  K2B_CUDA_OK(cudaMemsetAsync(unfit, 0, sizeof(int32_t) * a->num_fsas, stream));
+  K2B_CUDA_OK(cudaMemsetAsync(unfit, 0, sizeof(int32_t) * 2 * a->num_fsas, stream));
   if (!L.lane_plan) return kOk;
   { PlanLanes<<<dim3(2, a->num_fsas), 256, 0, stream>>>(
       reinterpret_cast<const FsaInfo *>(ws + L.off_infos), a->num_fsas, a->a_row_splits2,
-      a->a_in_splits, kLaneDeg, reinterpret_cast<int32_t *>(ws + L.off_plan), unfit);
+      a->a_in_splits, kLaneDeg, L.lane_threads, reinterpret_cast<int32_t *>(ws + L.off_plan),
+      unfit);
     NoteLaunch(); }
   K2B_CUDA_OK(cudaGetLastError());
   return kOk;
@@ -361,17 +366,17 @@ constexpr int kVitAhead = 3;  // rows requested ahead of the frame that uses the
 // column only took 500 frames of 4627 arcs from 246 to 215 us per round of CTAs (one CTA per
 // SM).  40 registers, for two CTAs per SM, leave no room to request a lane's eight scores
 // together: 256 CTAs took 460 us, and 431 with up to 80.
-template <int kDeg, int kPitch>
-__global__ void __launch_bounds__(kLaneThreads, 1)
+template <int kDeg, int kPitch, int kThreads>
+__global__ void __launch_bounds__(kThreads, 1)
 LanesViterbi(const FsaInfo *__restrict__ infos, int32_t n, const Arc *__restrict__ arcs,
              const int32_t *__restrict__ a_row_splits2, const int32_t *__restrict__ in_splits,
              const int32_t *__restrict__ in_arcs, const float *__restrict__ scores,
              int32_t cols, int32_t cols_pad, float *__restrict__ fwd, float *__restrict__ bwd,
              const int32_t *__restrict__ plan, const int32_t *__restrict__ unfit) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ float buf[2][kLaneThreads];
+  __shared__ float buf[2][kThreads];
   const int32_t i = blockIdx.y;
-  if (unfit[i] & 1) return;
+  if ((unfit[i] & 1) || unfit[n + i] != LaneClass(kThreads)) return;
   const int dir = blockIdx.x;
   const int32_t S = infos[i].num_states, Tk = infos[i].tk;
   if (S == 0) return;
@@ -499,24 +504,28 @@ LanesViterbi(const FsaInfo *__restrict__ infos, int32_t n, const Arc *__restrict
 int32_t LaunchLanesViterbi(const Layout &L, const k2b200_intersect_args *a,
                            const FsaInfo *d_infos, float *fwd, float *bwd, const int32_t *plan,
                            const int32_t *unfit, cudaStream_t stream) {
-  (void)L;
   static_assert(kLaneDeg % 2 == 0, "arcs are taken in pairs");
   dim3 grid(2, a->num_fsas);
   const int32_t cols_pad = (a->cols + 3) & ~3;
-  auto launch = [&](auto kernel, int32_t pitch) -> int32_t {
+  auto launch = [&](auto kernel, int32_t threads, int32_t pitch) -> int32_t {
     const size_t smem = sizeof(float) * kVitRing * (size_t)pitch;
     K2B_REQUIRE(smem <= 200 * 1024, "too many columns for the lane Viterbi kernel");
     K2B_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem));
-    kernel<<<grid, kLaneThreads, smem, stream>>>(
+    kernel<<<grid, threads, smem, stream>>>(
         d_infos, a->num_fsas, reinterpret_cast<const Arc *>(a->a_arcs), a->a_row_splits2,
         a->a_in_splits, a->a_in_arcs, a->scores, a->cols, cols_pad, fwd, bwd, plan, unfit);
     NoteLaunch();
     return kOk;
   };
   // graphs over phones have rows of up to 128 columns
-  if (a->cols <= 128) K2B_FORWARD(launch(LanesViterbi<kLaneDeg, 128>, 128));
-  else K2B_FORWARD(launch(LanesViterbi<kLaneDeg, 0>, cols_pad));
+#define K2B_LANES_VITERBI(THREADS)                                                           \
+  {                                                                                          \
+    if (a->cols <= 128) K2B_FORWARD(launch(LanesViterbi<kLaneDeg, 128, THREADS>, THREADS, 128)); \
+    else K2B_FORWARD(launch(LanesViterbi<kLaneDeg, 0, THREADS>, THREADS, cols_pad)); \
+  }
+  K2B_LANE_THREADS(L.lane_threads, K2B_LANES_VITERBI);
+#undef K2B_LANES_VITERBI
   K2B_CUDA_OK(cudaGetLastError());
   return kOk;
 }
