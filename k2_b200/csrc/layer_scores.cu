@@ -32,7 +32,6 @@
 namespace k2b {
 
 constexpr size_t kLayerSmemBudget = 200 * 1024;
-constexpr int kLight = 4;             // arcs that one lane sums by itself
 constexpr int kRescale = 4;           // layers between changes of the shared exponent
 constexpr float kMaxScore = 300.0f;   // |arc score|: exp() within 2^+-433
 constexpr int kRangeExp = 280;        // values that are not zero stay within 2^+-280, so that no
@@ -991,9 +990,12 @@ ExactChain(k2b200_fsa_view v, const uint4 *__restrict__ pool, const SliceDesc *_
 
 // The same for layers too wide for the ring: the CTAs of a cluster share a layer.  grid =
 // (directions x team, fsas).  Splits, records and the values of the layer before come from
-// L2; what does not depend on values is fetched a layer ahead, so that a layer costs one
-// gather and one cluster barrier, a microsecond, whatever its width (up to team x 512 states
-// a trip).
+// L2; what does not depend on values is fetched a layer ahead, the records of up to four arcs
+// per lane among it.  A state has 1, 2, 4 or 8 lanes, as many as the width of the layer leaves
+// it, so that few states have more arcs than that: a layer costs one gather and one
+// cluster barrier, a microsecond each.  (One lane per state with one record ahead, and states
+// of more than four arcs one after the other by a whole warp: 3 us per layer of a
+// lattice of 152 layers, now 2.1.)
 template <typename Val, bool kLog>
 __global__ void __launch_bounds__(512, 1)
 LayerChainWide(k2b200_fsa_view v, const LayerArc *__restrict__ fwd_arcs,
@@ -1029,54 +1031,75 @@ LayerChainWide(k2b200_fsa_view v, const LayerArc *__restrict__ fwd_arcs,
     if (team == 1) __syncthreads(); else cluster.sync();
   };
   auto layer_of = [&](int32_t step) { return dir == 0 ? step : nl - 1 - step; };
+  constexpr int kRecs = 4;
   struct Ahead {
-    int32_t k0, k1;
-    LayerArc r0;
+    int32_t k0, k1, log_lanes;  // of the lane's state; log2 of the lanes of a state
+    LayerArc r[kRecs];
+  };
+  // lanes per state in a layer of `width` states
+  auto log_lanes_of = [&](int32_t width) {
+    int32_t n = 0;
+    while (n < 3 && width << (n + 1) <= nt) ++n;
+    return n;
   };
   auto fetch_splits = [&](int32_t step, Ahead &f) {
-    f.k0 = f.k1 = 0;
+    f.k0 = f.k1 = f.log_lanes = 0;
     if (step >= nl) return;
-    const int32_t l = layer_of(step), s = lvl[l] + at;
-    if (s < lvl[l + 1]) {
+    const int32_t l = layer_of(step), b = lvl[l], e = lvl[l + 1];
+    f.log_lanes = log_lanes_of(e - b);
+    const int32_t s = b + (at >> f.log_lanes);
+    if (s < e) {
       f.k0 = __ldg(gsplits + s);
       f.k1 = __ldg(gsplits + s + 1);
     }
   };
-  auto fetch_record = [&](Ahead &f) {
-    if (f.k0 < f.k1) f.r0 = garcs[f.k0];
+  auto fetch_records = [&](Ahead &f) {
+    const int32_t lanes = 1 << f.log_lanes, k = f.k0 + (lane & (lanes - 1));
+#pragma unroll
+    for (int u = 0; u < kRecs; ++u)
+      if (k + u * lanes < f.k1) f.r[u] = garcs[k + u * lanes];
   };
   auto rec = [&](int32_t k) { return garcs[k]; };
   auto val = [&](const LayerArc &r) { return __ldcg(out + r.other); };
   Ahead now, next, after;
   fetch_splits(0, now);
-  fetch_record(now);
+  fetch_records(now);
   fetch_splits(1, next);
   for (int32_t step = 0; step < nl; ++step) {
-    fetch_record(next);
+    fetch_records(next);
     fetch_splits(step + 2, after);
     const int32_t l = layer_of(step), b = lvl[l], e = lvl[l + 1];
+    const int32_t lanes = 1 << now.log_lanes, g = lane & (lanes - 1);
     sc.BeginLayer(step, my_hi, rank == 0 && tid == 0);
-    for (int32_t s0 = b; s0 < e; s0 += nt) {
-      const int32_t s = s0 + at;
+    for (int32_t s0 = b; s0 < e; s0 += nt) {  // (more than once only with a lane per state)
+      const int32_t s = s0 + (at >> now.log_lanes);
       if (s0 > b) {
         now.k0 = now.k1 = 0;
         if (s < e) {
           now.k0 = __ldg(gsplits + s);
           now.k1 = __ldg(gsplits + s + 1);
         }
-        fetch_record(now);
+        fetch_records(now);
       }
       StateSum<Val, kLog> q;
       q.Clear();
-      int32_t k0 = now.k0;
-      const int32_t k1 = now.k1, deg = k1 - k0;
-      const unsigned heavy = __ballot_sync(kAll, deg > kLight);
-      if (deg > 0 && deg <= kLight) {
-        q.Add(now.r0, val(now.r0));
-        q.Walk(k0 + 1, k1, 1, rec, val);
+      const int32_t k0 = now.k0, k1 = now.k1;
+      // states of many arcs are left to the whole warp
+      const bool many = k1 - k0 > 4 * kRecs * lanes;
+      if (!many) {
+        Val x[kRecs];
+#pragma unroll
+        for (int u = 0; u < kRecs; ++u)
+          if (k0 + g + u * lanes < k1) x[u] = val(now.r[u]);
+#pragma unroll
+        for (int u = 0; u < kRecs; ++u)
+          if (k0 + g + u * lanes < k1) q.Add(now.r[u], x[u]);
+        q.Walk(k0 + g + kRecs * lanes, k1, lanes, rec, val);
       }
+      const unsigned heavy = __ballot_sync(kAll, many && g == 0);
       if (heavy) q.Heavy(heavy, lane, k0, k1, rec, val);
-      if (s < e) {
+      q.Across(lanes);
+      if (s < e && g == 0) {
         if (kLog) {
           q.acc = q.acc * (Val)sc.mul;
           if (q.acc == (Val)0 && s == root) q.acc = (Val)1;
