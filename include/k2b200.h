@@ -563,6 +563,13 @@ typedef struct {
   const void *lens;
   float *loss;         /* device */
   const float *logits; /* NULL, or [log_prob_rows, num_classes] (device) */
+  /* Delay penalty of k2/python/k2/ctc_loss.py:99-136, 0 for none: -delay_penalty x (frame - half
+   * the number of frames) is added to the score of the arcs that survive pruning, but
+   * not where a symbol ends or repeats: arcs whose aux label is 0 or -1 or, with arc_repeat,
+   * whose label is 0 or -1 or that arc_repeat (one byte per arc) marks. */
+  float delay_penalty;
+  const uint8_t *arc_repeat; /* device, one of the two */
+  const int32_t *arc_aux;
 } k2b200_band_reduce;
 typedef struct {
   const void *grad;    /* device: dL/dtot (stride elements apart) or, with stride 0, one value */

@@ -60,7 +60,8 @@ class BandLossArgs(ctypes.Structure):
 
 class BandReduce(ctypes.Structure):
     _fields_ = [("mode", c_i32), ("lens_type", c_i32), ("lens", c_vp), ("loss", c_vp),
-                ("logits", c_vp)]
+                ("logits", c_vp), ("delay_penalty", ctypes.c_float), ("arc_repeat", c_vp),
+                ("arc_aux", c_vp)]
 
 
 class BandUpstream(ctypes.Structure):

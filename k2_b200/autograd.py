@@ -745,8 +745,9 @@ _TOTALS, _NEG_SUM, _MEAN = 0, 1, 2
 
 def _band_native(a_fsas: Fsa, b_fsas: DenseFsaVec, a_to_b_map: Optional[torch.Tensor],
                  output_beam: float, max_states: int, max_arcs: int, mode: int,
-                 use_double_scores: bool,
-                 target_lengths: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
+                 use_double_scores: bool, target_lengths: Optional[torch.Tensor] = None,
+                 delay_penalty: float = 0.0,
+                 symbols: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
     """Total scores of band graphs, or their negated sum / mean, as ONE node of the autograd
     graph (csrc/host/torch_host.cc over k2b200_band_loss_*), reading the log-probs or logits
     that `b_fsas` was made from; None when it does not take these inputs."""
@@ -771,17 +772,24 @@ def _band_native(a_fsas: Fsa, b_fsas: DenseFsaVec, a_to_b_map: Optional[torch.Te
                                f"a_to_b_map.Dim() ({h_map.shape[0]})")
     return _lib._host.band_loss(graph, a_fsas.scores, src[0], logits, src[1], b_fsas.h_row_splits,
                                 h_map, output_beam, max_states, max_arcs, mode, use_double_scores,
-                                target_lengths)
+                                target_lengths, delay_penalty, symbols)
 
 
 def band_ctc_loss(a_fsas: Fsa, b_fsas: DenseFsaVec, output_beam: float, reduction: str,
-                  use_double_scores: bool,
-                  target_lengths: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+                  use_double_scores: bool, target_lengths: Optional[torch.Tensor],
+                  delay_penalty: float = 0.0) -> Optional[torch.Tensor]:
     """The reductions "sum" and "mean" of k2/python/k2/ctc_loss.py:72-84 on the band kernels,
-    or None when they do not take these inputs."""
+    with the delay penalty of :99-136, or None when they do not take these inputs."""
+    symbols = None
+    if delay_penalty > 0.0:
+        symbols = getattr(a_fsas, "_is_repeat_token_", None)
+        if symbols is None:
+            symbols = getattr(a_fsas, "aux_labels", None)
+        if not isinstance(symbols, torch.Tensor):
+            return None
     return _band_native(a_fsas, b_fsas, None, output_beam, 15000000, 1073741824,
                         _NEG_SUM if reduction == "sum" else _MEAN, use_double_scores,
-                        target_lengths)
+                        target_lengths, max(delay_penalty, 0.0), symbols)
 
 
 def band_loss_supported(a_fsas: Fsa, b_fsas: DenseFsaVec,

@@ -530,6 +530,35 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
 }
 
 // ---------------------------------------------------------------------------
+// Delay penalty: what the score of an arc that survives gains on frame t.  flags[arc] says
+// which arcs are penalised.  Pruning does not see it.
+// A path that is n symbols ahead of another has gained n penalties; where posteriors are so flat
+// that such paths share a level for long, the graph goes to the (mantissa, exponent) recursion.
+// ---------------------------------------------------------------------------
+struct DelaySpec {
+  float penalty;
+  const uint8_t *flags;  // [arcs]
+  __device__ __forceinline__ float Of(int32_t t, int32_t frames) const {
+    return -penalty * (float)(t - (frames >> 1));
+  }
+};
+
+__global__ void PenaltyFlags(const BandState *__restrict__ tab, const BandArc *__restrict__ tabf,
+                             int32_t num_states, const uint8_t *__restrict__ repeat,
+                             const int32_t *__restrict__ aux, uint8_t *__restrict__ flags) {
+  const int32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= num_states) return;
+  const int32_t label = tab[idx].label;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const int32_t arc = tabf[(int64_t)idx * 3 + d].arc;
+    if (arc < 0) continue;
+    const int32_t symbol = repeat != nullptr ? (repeat[arc] ? 0 : label) : aux[arc];
+    flags[arc] = symbol != 0 && symbol != -1;
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Keep tests and lists.  grid = (chunks of kPrepLevels levels, pairs), kPrepWarps warps per CTA,
 // which looks at the chunk's levels and the level on either side of them:
 //   1. a warp per level, four states per lane at a time: state s of level l survives iff
@@ -565,6 +594,7 @@ static size_t BandPrepSmem(int32_t max_states) {
   return (size_t)kPrepSpan * (PrepPad(max_states) / 4 * 2 + PrepPad(max_states) * 3);
 }
 
+template <bool kDelay>
 __global__ void __launch_bounds__(32 * kPrepWarps, 3)
 BandPrep(const BandInfo *__restrict__ infos, const int32_t *__restrict__ a_row_splits2,
          const BandState *__restrict__ tab, const BandArc *__restrict__ tabf,
@@ -572,7 +602,7 @@ BandPrep(const BandInfo *__restrict__ infos, const int32_t *__restrict__ a_row_s
          const float *__restrict__ vf, const float *__restrict__ vb, float beam, BandItem *__restrict__ items,
          BandFactor *__restrict__ factors, int2 *__restrict__ lists,
          int32_t *__restrict__ chunk_r, unsigned long long *__restrict__ totals,
-         int32_t *__restrict__ unfit, int32_t count_arcs) {
+         int32_t *__restrict__ unfit, int32_t count_arcs, DelaySpec delay) {
   constexpr unsigned kAll = 0xffffffffu;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int32_t longest_sh, risky_sh;
@@ -777,10 +807,20 @@ BandPrep(const BandInfo *__restrict__ infos, const int32_t *__restrict__ a_row_s
               if ((inb >> d) & 1u) {
                 from |= src[u] & (0xffu << (8 * d));
                 pw[d] = p;
-                if (st[u].w[d] != 0.0f) {  // (the factor of a score of zero is one)
+                // (the factor of a score of zero is one)
+                if (kDelay || st[u].w[d] != 0.0f) {
                   const BandArc arc = tabf[(int64_t)(f.state_off + s[u]) * 3 + d];
                   pw[d] = arc.f * Pow2Clamp(arc.k) * p;
                   if (arc.k > kMaxLeanArcExp || arc.k < kMinLeanArcExp) risky = true;
+                  if (kDelay) {
+                    // the score as the lattice has it, a float
+                    const int32_t l = a + row[u] - 1;
+                    float sc = __fadd_rn(st[u].w[d], x[u]);
+                    if (delay.flags[arc.arc]) sc = __fadd_rn(sc, delay.Of(l - 1, T));
+                    pw[d] = exp((double)sc);
+                    // what the limits above leave of a factor
+                    if (!(pw[d] > 1e-52 && pw[d] < 1e52)) risky = true;
+                  }
                 }
               }
           }
@@ -1182,6 +1222,8 @@ BandChainLists(const BandInfo *__restrict__ infos, const BandFactor *__restrict_
                  wait_limit);
 }
 
+constexpr int kExactThreads = 128;
+
 // The same recursion with a (mantissa, exponent) pair per state, for the graphs marked in
 // `unfit`; every other graph returns at once.  exp(dense score) is recomputed from the
 // log-probs, the arc factors come from the graph's tables: no range limit.
@@ -1191,32 +1233,32 @@ ExactWalk(const BandInfo *__restrict__ infos, const BandArc *__restrict__ tabf,
           const int2 *__restrict__ lists, double *__restrict__ am, int32_t *__restrict__ ae,
           double *__restrict__ bm, int32_t *__restrict__ be, double *__restrict__ tot,
           BandTotal *__restrict__ total, const int32_t *__restrict__ unfit,
-          int32_t *__restrict__ status, int32_t st_pad, int32_t lv_pad, int32_t wait_limit) {
+          int32_t *__restrict__ status, int32_t st_pad, int32_t lv_pad, int32_t wait_limit,
+          const BandState *__restrict__ tab, const DelaySpec &delay) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full[kChainSlots];
-  constexpr unsigned kAll = 0xffffffffu;
   const int dir = blockIdx.x;
   const int32_t i = blockIdx.y;
   const BandInfo f = infos[i];
-  const int lane = threadIdx.x;
+  const int tid = threadIdx.x;
   const int32_t S = f.num_states, T = f.frames, pitch = f.pitch, L = T + 2;
   if (S == 0) return;
   BandItem *ring = reinterpret_cast<BandItem *>(smem_raw);
   int2 *lst = reinterpret_cast<int2 *>(ring + kChainSlots * kSlotItems);
   ProbState *vals = reinterpret_cast<ProbState *>(lst + lv_pad);  // [2][st_pad], state s at s + 2
-  for (int32_t l = lane; l < L; l += 32) lst[l] = lists[f.level_off + l];
-  for (int32_t k = lane; k < 2 * st_pad; k += 32) {
+  for (int32_t l = tid; l < L; l += kExactThreads) lst[l] = lists[f.level_off + l];
+  for (int32_t k = tid; k < 2 * st_pad; k += kExactThreads) {
     ProbState z;
     z.m = 0.0;
     z.e = kZeroExp;
     z.pad = 0;
     vals[k] = z;
   }
-  if (lane == 0) {
+  if (tid == 0) {
     for (int st = 0; st < kChainSlots; ++st) MbarInit(&full[st], 1);
     MbarInitFence();
   }
-  __syncwarp();
+  __syncthreads();
   ChunkRing<BandItem, kSlotItems> rg;
   rg.full = full;
   rg.slots = ring;
@@ -1227,7 +1269,7 @@ ExactWalk(const BandInfo *__restrict__ infos, const BandArc *__restrict__ tabf,
   rg.num_chunks = (L + kPrepLevels - 1) / kPrepLevels;
   rg.dir = dir;
   rg.issued = 0;
-  if (lane == 0)
+  if (tid == 0)
     for (int32_t k = 0; k < kChainSlots; ++k) rg.Issue();
   const float *lp0 = lp + (int64_t)f.lp_row * C;
   const BandArc *my_arcs = tabf + (int64_t)f.state_off * 3;
@@ -1238,7 +1280,7 @@ ExactWalk(const BandInfo *__restrict__ infos, const BandArc *__restrict__ tabf,
   for (int32_t q = 0; q < rg.num_chunks; ++q) {
     const int32_t c = rg.ChunkOf(q), slot = q % kChainSlots;
     if (!late) late = !WaitSlot(&full[slot], (unsigned)(q / kChainSlots) & 1u, wait_limit);
-    late = __any_sync(kAll, late);
+    late = __syncthreads_or(late);
     if (late) break;
     const int32_t chunk_start = c * kPrepLevels * pitch;
     const int32_t l_lo = c * kPrepLevels, nl = min(l_lo + kPrepLevels, L) - l_lo;
@@ -1249,7 +1291,7 @@ ExactWalk(const BandInfo *__restrict__ infos, const BandArc *__restrict__ tabf,
       const int2 ls = lst[l];
       ProbState *cur = vals + (step & 1) * st_pad + 2;
       const ProbState *prv = vals + ((step & 1) ^ 1) * st_pad + 2;
-      for (int32_t j = lane; j < ls.y; j += 32) {
+      for (int32_t j = tid; j < ls.y; j += kExactThreads) {
         const BandItem it = src[ls.x + j];
         const int32_t s = it.s;
         // exp(dense score) of this state's label on frame l - 1
@@ -1274,8 +1316,23 @@ ExactWalk(const BandInfo *__restrict__ infos, const BandArc *__restrict__ tabf,
             if ((bits >> d) & 1u) {  // the bit names an arc of this graph
               const ProbState qs = dir == 0 ? prv[s - d] : prv[s + d];
               const BandArc arc = dir == 0 ? my_arcs[3 * s + d] : my_arcs[3 * (s + d) + d];
-              t[d] = qs.m * arc.f;
-              if (t[d] != 0.0) x[d] = qs.e + arc.k;
+              double am_arc = arc.f;
+              int32_t ak = arc.k;
+              if (delay.penalty != 0.0f && delay.flags[arc.arc]) {
+                const int32_t t_arc = dir == 0 ? l - 1 : l;
+                const float gain = delay.Of(t_arc, T);
+                double pen;
+                int32_t pen_k;
+                ExpToMantExp(gain, &pen, &pen_k);
+                // (and what rounding the score to a float, as the lattice has it, makes of it)
+                const BandState to = tab[f.state_off + (dir == 0 ? s : s + d)];
+                const float x_arc = BandDense(lp0, C, T, t_arc, to.label);
+                const float sc = __fadd_rn(__fadd_rn(to.w[d], x_arc), gain);
+                am_arc *= pen * exp((double)sc - (double)to.w[d] - (double)x_arc - (double)gain);
+                ak += pen_k;
+              }
+              t[d] = qs.m * am_arc;
+              if (t[d] != 0.0) x[d] = qs.e + ak;
             }
           }
           const int32_t E = max(x[0], max(x[1], x[2]));
@@ -1310,18 +1367,18 @@ ExactWalk(const BandInfo *__restrict__ infos, const BandArc *__restrict__ tabf,
         }
         cur[s] = r;
       }
-      __syncwarp();  // the level is complete
+      __syncthreads();  // the level is complete
     }
-    if (lane == 0) rg.Issue();
+    if (tid == 0) rg.Issue();
   }
   if (late) {
-    if (lane == 0) {
+    if (tid == 0) {
       atomicOr(status, kStatusLate);
       rg.Drain();
     }
-    __syncwarp();
+    __syncthreads();
   }
-  if (dir == 0 && lane == 0 && (*status & kStatusLate)) tot[i] = nan("");
+  if (dir == 0 && tid == 0 && (*status & kStatusLate)) tot[i] = nan("");
 }
 
 // What the caller makes of the totals (k2b200_band_reduce), done by the CTA that finishes
@@ -1341,21 +1398,23 @@ __device__ __forceinline__ double LengthOf(const void *lens, int32_t type, int32
   }
 }
 
-__global__ void __launch_bounds__(32)
+__global__ void __launch_bounds__(kExactThreads)
 BandChainExact(const BandInfo *__restrict__ infos, const BandArc *__restrict__ tabf,
                const float *__restrict__ lp, int32_t C, const BandItem *__restrict__ items,
                const int2 *__restrict__ lists, double *__restrict__ am,
                int32_t *__restrict__ ae, double *__restrict__ bm, int32_t *__restrict__ be,
                double *__restrict__ tot, BandTotal *__restrict__ total,
                const int32_t *__restrict__ unfit, int32_t *__restrict__ status, int32_t st_pad,
-               int32_t lv_pad, int32_t wait_limit, LossSpec spec, uint32_t *__restrict__ ticket) {
+               int32_t lv_pad, int32_t wait_limit, LossSpec spec, uint32_t *__restrict__ ticket,
+               const BandState *__restrict__ tab, DelaySpec delay) {
   if (unfit[blockIdx.y] != 0)
     ExactWalk(infos, tabf, lp, C, items, lists, am, ae, bm, be, tot, total, unfit, status, st_pad,
-              lv_pad, wait_limit);
+              lv_pad, wait_limit, tab, delay);
   if (spec.mode == 0) return;
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
   const int lane = threadIdx.x;
   uint32_t t = 0;
-  __syncwarp();
   if (lane == 0) {
     __threadfence();
     t = atomicAdd(ticket, 1u);
@@ -1699,7 +1758,7 @@ struct BandLayout {
   int32_t st_pad = 0, lv_pad = 0;
   size_t chain_smem = 0, exact_smem = 0, viterbi_smem = 0, prep_smem = 0;
   size_t off_infos, off_vf, off_vb, off_by_state, off_items, off_factors, off_lists, off_chunk_r, off_am, off_ae,
-      off_bm, off_be, off_a_scale, off_b_scale, off_total, off_unfit, off_totals, off_status,
+      off_bm, off_be, off_penalty, off_a_scale, off_b_scale, off_total, off_unfit, off_totals, off_status,
       total_bytes;  // off_status = off_totals + 40
   bool ok = true;
   const char *why = "";
@@ -1843,6 +1902,7 @@ static int32_t MakeBandLayout(const k2b200_band_loss_args *a, BandLayout *L) {
   L->off_a_scale = take(sizeof(int32_t) * (size_t)levels);
   L->off_b_scale = take(sizeof(int32_t) * (size_t)levels);
   L->off_total = take(sizeof(BandTotal) * a->num_fsas);
+  L->off_penalty = take((size_t)std::max(a->h_a_arc_splits[a->num_fsas], 1));
   L->off_unfit = take(sizeof(int32_t) * a->num_fsas);
   L->off_totals = take(64);  // five 64-bit totals, the status word, the ticket (at 48)
   L->off_status = L->off_totals + 5 * sizeof(long long);
@@ -1871,7 +1931,8 @@ static bool BandReduceBeam(const k2b200_band_loss_args *a, const long long *h_to
 }
 
 static int32_t LaunchBandChains(const BandLayout &L, const k2b200_band_loss_args *args, char *ws,
-                                double *tot_scores, const LossSpec &spec, cudaStream_t stream) {
+                                double *tot_scores, const LossSpec &spec, const DelaySpec &delay,
+                                cudaStream_t stream) {
   K2B_CUDA_OK(cudaFuncSetAttribute(BandChainLists, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)L.chain_smem));
   K2B_CUDA_OK(cudaFuncSetAttribute(BandChainExact, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1890,11 +1951,12 @@ static int32_t LaunchBandChains(const BandLayout &L, const k2b200_band_loss_args
       reinterpret_cast<int32_t *>(ws + L.off_a_scale),
       reinterpret_cast<int32_t *>(ws + L.off_b_scale), tot_scores, total, unfit, status,
       CopyWaitLimit()); NoteLaunch(); }
-  { BandChainExact<<<grid, 32, L.exact_smem, stream>>>(
+  { BandChainExact<<<grid, kExactThreads, L.exact_smem, stream>>>(
       infos, reinterpret_cast<const BandArc *>(args->band_arcs), args->log_probs,
       args->num_classes, items, lists, am, reinterpret_cast<int32_t *>(ws + L.off_ae), bm,
       reinterpret_cast<int32_t *>(ws + L.off_be), tot_scores, total, unfit, status, L.st_pad,
-      L.lv_pad, CopyWaitLimit(), spec, reinterpret_cast<uint32_t *>(ws + L.off_totals + 48));
+      L.lv_pad, CopyWaitLimit(), spec, reinterpret_cast<uint32_t *>(ws + L.off_totals + 48),
+      reinterpret_cast<const BandState *>(args->band_states), delay);
     NoteLaunch(); }
   K2B_CUDA_OK(cudaGetLastError());
   return kOk;
@@ -1987,6 +2049,7 @@ int32_t k2b200_band_loss_forward_reduce(const k2b200_band_loss_args *args, void 
   char *ws = reinterpret_cast<char *>(workspace);
   static_assert(sizeof(BandInfo) % sizeof(int32_t) == 0, "BandInfo is uploaded as int32 words");
   LossSpec spec = {0, 0, nullptr, nullptr};
+  DelaySpec delay = {0.0f, nullptr};
   const float *logits = nullptr;
   if (reduce != nullptr) {
     K2B_REQUIRE(reduce->mode >= 0 && reduce->mode <= 2, "bad reduction mode %d", reduce->mode);
@@ -1999,6 +2062,12 @@ int32_t k2b200_band_loss_forward_reduce(const k2b200_band_loss_args *args, void 
     spec.lens_type = reduce->lens_type;
     spec.loss = reduce->loss;
     logits = reduce->logits;
+    if (reduce->delay_penalty != 0.0f) {
+      K2B_REQUIRE(reduce->arc_repeat != nullptr || reduce->arc_aux != nullptr,
+                  "a delay penalty needs to know the arcs it applies to");
+      delay.penalty = reduce->delay_penalty;
+      delay.flags = reinterpret_cast<const uint8_t *>(ws + L.off_penalty);
+    }
   }
   // unfit words, totals, the status word and the ticket lie one after the other: one clear for
   // the first pass (a repeated pass clears them again but for the status of the Viterbi kernels)
@@ -2007,6 +2076,11 @@ int32_t k2b200_band_loss_forward_reduce(const k2b200_band_loss_args *args, void 
                                  reinterpret_cast<int32_t *>(ws + L.off_infos),
                                  reinterpret_cast<int32_t *>(ws + L.off_unfit),
                                  (int64_t)(L.off_totals + 64 - L.off_unfit) / 4, stream));
+  if (delay.penalty != 0.0f && args->num_states > 0)
+    { PenaltyFlags<<<CeilDiv(args->num_states, 128), 128, 0, stream>>>(
+        reinterpret_cast<const BandState *>(args->band_states),
+        reinterpret_cast<const BandArc *>(args->band_arcs), args->num_states, reduce->arc_repeat,
+        reduce->arc_aux, const_cast<uint8_t *>(delay.flags)); NoteLaunch(); }
   if (logits != nullptr && L.max_frames > 0) {
     PhaseTimer timer(kPhaseDense, stream);
     dim3 grid(CeilDiv(L.max_frames, 8), args->num_fsas);
@@ -2017,7 +2091,8 @@ int32_t k2b200_band_loss_forward_reduce(const k2b200_band_loss_args *args, void 
   {
     PhaseTimer timer(kPhaseViterbi, stream);
     NotePhaseKernel(kPhaseViterbi, "BandViterbi");
-    K2B_CUDA_OK(cudaFuncSetAttribute(BandPrep, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    K2B_CUDA_OK(cudaFuncSetAttribute(delay.penalty != 0.0f ? BandPrep<true> : BandPrep<false>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)L.prep_smem));
     const BandInfo *infos = reinterpret_cast<const BandInfo *>(ws + L.off_infos);
     const BandState *tab = reinterpret_cast<const BandState *>(args->band_states);
@@ -2065,7 +2140,8 @@ int32_t k2b200_band_loss_forward_reduce(const k2b200_band_loss_args *args, void 
       PhaseTimer timer(kPhasePrune, stream);
       NotePhaseKernel(kPhasePrune, "BandPrep");
       dim3 grid(CeilDiv(L.max_frames + 2, kPrepLevels), args->num_fsas);
-      { BandPrep<<<grid, 32 * kPrepWarps, L.prep_smem, stream>>>(
+      auto prep = delay.penalty != 0.0f ? BandPrep<true> : BandPrep<false>;
+      { prep<<<grid, 32 * kPrepWarps, L.prep_smem, stream>>>(
           reinterpret_cast<const BandInfo *>(ws + L.off_infos), args->a_row_splits2,
           reinterpret_cast<const BandState *>(args->band_states),
           reinterpret_cast<const BandArc *>(args->band_arcs), args->log_probs,
@@ -2079,7 +2155,7 @@ int32_t k2b200_band_loss_forward_reduce(const k2b200_band_loss_args *args, void 
           reinterpret_cast<int32_t *>(ws + L.off_chunk_r),
           reinterpret_cast<unsigned long long *>(ws + L.off_totals),
           reinterpret_cast<int32_t *>(ws + L.off_unfit),
-          L.arc_frames > args->max_arcs ? 1 : 0); NoteLaunch(); }
+          L.arc_frames > args->max_arcs ? 1 : 0, delay); NoteLaunch(); }
       // the host reads the counts behind BandPrep, while what follows runs
       if (need_count) {
         K2B_FORWARD(SideFork(stream, &side));
@@ -2097,7 +2173,7 @@ int32_t k2b200_band_loss_forward_reduce(const k2b200_band_loss_args *args, void 
     {
       PhaseTimer timer(kPhaseChain, stream);
       NotePhaseKernel(kPhaseChain, "BandChainLists");
-      K2B_FORWARD(LaunchBandChains(L, args, ws, tot_scores, spec, stream));
+      K2B_FORWARD(LaunchBandChains(L, args, ws, tot_scores, spec, delay, stream));
     }
     if (!need_count) break;
     long long h_totals[6];

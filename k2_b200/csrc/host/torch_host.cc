@@ -372,7 +372,8 @@ py::object BandLoss(const std::shared_ptr<BandGraph> &graph, const at::Tensor &s
                     const at::Tensor &input, bool logits, const IntArray &first,
                     const IntArray &row_splits, const py::object &a_to_b, double beam,
                     int64_t max_states, int64_t max_arcs, int32_t mode, bool use_double,
-                    const c10::optional<at::Tensor> &lens) {
+                    const c10::optional<at::Tensor> &lens, double delay_penalty,
+                    const c10::optional<at::Tensor> &symbols) {
   if (!input.is_cuda() || input.scalar_type() != at::kFloat || input.dim() != 3 ||
       !input.is_contiguous() || graph->states.device() != input.device())
     return py::none();
@@ -405,6 +406,14 @@ py::object BandLoss(const std::shared_ptr<BandGraph> &graph, const at::Tensor &s
         (lens_type = LensType(*lens)) == 0)
       return py::none();
   }
+  // the gradient of the arc scores does not know of the penalty
+  const bool delayed = delay_penalty > 0.0;
+  if (delayed && (!symbols.has_value() || !symbols->is_cuda() ||
+                  symbols->device() != input.device() || symbols->dim() != 1 ||
+                  !symbols->is_contiguous() || symbols->numel() != graph->h_arc_splits.back() ||
+                  (symbols->scalar_type() != at::kInt && symbols->scalar_type() != at::kBool) ||
+                  torch::autograd::compute_requires_grad(scores_a)))
+    return py::none();
   k2b200_band_loss_args &a = call.args;
   const int64_t classes = input.size(2);
   if (classes > (int64_t)1 << 24) return py::none();
@@ -443,6 +452,13 @@ py::object BandLoss(const std::shared_ptr<BandGraph> &graph, const at::Tensor &s
     reduce.lens_type = lens_type;
     reduce.lens = lens_type ? lens->data_ptr() : nullptr;
     reduce.logits = logits ? input.data_ptr<float>() : nullptr;
+    if (delayed) {
+      reduce.delay_penalty = (float)delay_penalty;
+      if (symbols->scalar_type() == at::kBool)
+        reduce.arc_repeat = reinterpret_cast<const uint8_t *>(symbols->data_ptr<bool>());
+      else
+        reduce.arc_aux = symbols->data_ptr<int32_t>();
+    }
     if (mode != kTotals) {
       out = at::empty({}, On(at::kFloat, device));
       reduce.loss = out.data_ptr<float>();

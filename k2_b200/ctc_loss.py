@@ -10,9 +10,9 @@ from .dense_fsa_vec import DenseFsaVec
 from .fsa import Fsa
 
 
-# With no delay penalty nothing but the total scores of the lattice is used, so they
-# are computed without building it when the graphs allow; set to False to force
-# the reference's intersect_dense + get_tot_scores sequence.
+# Nothing but the total scores of the lattice is used, so they are computed without building
+# it when the graphs allow (with a delay penalty: CTC graphs, on the band kernels); set to
+# False to force the reference's intersect_dense + get_tot_scores sequence.
 FUSED_LOSS = True
 # Outside the band-graph kernels (CTC graphs), the lattice-free path exponentiates
 # every element of the dense matrix and streams whole rows through shared memory; with
@@ -35,9 +35,12 @@ class CtcLoss(nn.Module):
     def forward(self, decoding_graph: Fsa, dense_fsa_vec: DenseFsaVec,
                 delay_penalty: float = 0.0,
                 target_lengths: Optional[torch.Tensor] = None) -> torch.Tensor:
-        if FUSED_LOSS and delay_penalty <= 0.0 and self.reduction != "none":
+        # (with a delay penalty, totals in float32 are the lattice's: its gradients differ from
+        # those of double totals by more than their own rounding)
+        if FUSED_LOSS and self.reduction != "none" and (delay_penalty <= 0.0
+                                                        or self.use_double_scores):
             loss = band_ctc_loss(decoding_graph, dense_fsa_vec, self.output_beam, self.reduction,
-                                 self.use_double_scores, target_lengths)
+                                 self.use_double_scores, target_lengths, delay_penalty)
             if loss is not None:
                 return loss
         if FUSED_LOSS and delay_penalty <= 0.0 and (
