@@ -76,7 +76,7 @@ struct SearchArgs {
   float *st_bwd;
   int32_t *arc_aidx, *arc_dest;
   float *arc_ll, *arc_end;
-  int32_t *list_a, *list_b;    // scratch, like the arcs
+  uint8_t *arc_deg;           // scratch: arcs leaving a new state, 255 for that many or more
   unsigned long long *winner;  // [num_seqs * a_states] (shared) or [a_states]
   int32_t *frame_s0, *frame_a0, *frame_n0, *frame_m0;  // [num_seqs][T + 2], the last two scratch
   int32_t *warp_first;         // [num_seqs][kTeamWarps]
@@ -207,7 +207,7 @@ struct SeqView {
   float *st_bwd;
   int32_t *arc_aidx, *arc_dest;
   float *arc_ll, *arc_end;
-  int32_t *list_a, *list_b;
+  uint8_t *arc_deg;
   unsigned long long *winner;
   int32_t *frame_s0, *frame_a0, *frame_n0, *frame_m0, *warp_first;
 };
@@ -225,8 +225,7 @@ __device__ __forceinline__ SeqView ViewOf(const SearchArgs &g, int32_t seq) {
   v.arc_dest = g.arc_dest + ao;
   v.arc_ll = g.arc_ll + ao;
   v.arc_end = g.arc_end + ao;
-  v.list_a = g.list_a + ao;
-  v.list_b = g.list_b + ao;
+  v.arc_deg = g.arc_deg + ao;
   // the reference's hash key is dest_state_idx01 + seq * stride with the stride 0
   // for per-sequence graphs (:118-127): the same index works for a direct table
   v.winner = g.winner + (g.a_stride ? 0 : (int64_t)seq * g.a_states);
@@ -360,13 +359,17 @@ __device__ bool SearchStep(const SearchArgs &g, const SeqView &v, const Team &tm
     return true;
   }
   const int64_t raw = (g.cap_a - na) & ~(int64_t)31;  // the expanded arcs' place
-  if (g.cap_a < na || raw < a0) return false;
+  // (and as much again in front of it, for the warps' lists, until the arcs that are kept
+  // go there)
+  if (g.cap_a < na || raw - a0 < na) return false;
   int32_t *r_aidx = v.arc_aidx + raw, *r_dest = v.arc_dest + raw;
   float *r_ll = v.arc_ll + raw, *r_end = v.arc_end + raw;
   const int32_t per_warp = ArcsPerWarp(na, tm);
   const int32_t lo = (int32_t)min((int64_t)tm.warp * per_warp, (int64_t)na);
   const int32_t hi = min(lo + per_warp, na);
-  int32_t *list_a = v.list_a + raw + lo, *list_b = v.list_b + raw + lo;
+  int32_t *list = reinterpret_cast<int32_t *>(v.arc_end) + a0 + lo;
+  int32_t *list_dest = v.arc_aidx + a0 + lo;  // until step 6
+  uint8_t *list_deg = v.arc_deg + raw + lo;
 
   // graph of this sequence: its final state, for allow_partial (:861-871)
   const int32_t gi = seq * g.a_stride;
@@ -463,8 +466,8 @@ __device__ bool SearchStep(const SearchArgs &g, const SeqView &v, const Team &tm
         const uint32_t m = __ballot_sync(kAll, in);
         if (in) {
           const int32_t at = above + __popc(m & ((1u << lane) - 1u));
-          list_a[at] = p;
-          list_b[at] = dest[i];
+          list[at] = p;
+          list_dest[at] = dest[i];
           atomicMax(&v.winner[dest[i]], ArcEntry(t, p));
         }
         above += __popc(m);
@@ -481,8 +484,8 @@ __device__ bool SearchStep(const SearchArgs &g, const SeqView &v, const Team &tm
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         const int32_t at = i0 + 32 * i + lane;
-        p[i] = at < above ? list_a[at] : 0;
-        d[i] = at < above ? list_b[at] : -1;
+        p[i] = at < above ? list[at] : 0;
+        d[i] = at < above ? list_dest[at] : -1;
       }
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
@@ -500,8 +503,8 @@ __device__ bool SearchStep(const SearchArgs &g, const SeqView &v, const Team &tm
         const uint32_t m = __ballot_sync(kAll, in);
         if (in) {
           const int32_t at = won + __popc(m & ((1u << lane) - 1u));
-          list_a[at] = d[i];
-          list_b[at] = deg[i];
+          list_dest[at] = d[i];
+          list_deg[at] = (uint8_t)min(deg[i], 255);
           degs += (uint32_t)deg[i];
         }
         won += __popc(m);
@@ -520,7 +523,9 @@ __device__ bool SearchStep(const SearchArgs &g, const SeqView &v, const Team &tm
     int32_t j = (int32_t)(base & 0xffffffffu), first = (int32_t)(base >> 32);
     for (int32_t i0 = 0; i0 < won; i0 += 32) {
       const bool in = i0 + lane < won;
-      const int32_t d = in ? list_a[i0 + lane] : 0, deg = in ? list_b[i0 + lane] : 0;
+      const int32_t d = in ? list_dest[i0 + lane] : 0;
+      int32_t deg = in ? list_deg[i0 + lane] : 0;
+      if (deg == 255) deg = g.a_rs2[d + 1] - g.a_rs2[d];
       int32_t inc = deg;
 #pragma unroll
       for (int x = 1; x < 32; x <<= 1) {
@@ -573,7 +578,7 @@ __device__ bool SearchStep(const SearchArgs &g, const SeqView &v, const Team &tm
         end[i] = r_end[pb + 32 * i + lane];
       }
     }
-    __syncwarp();  // (r_end and r_dest take the groups' masks from their start)
+    __syncwarp();  // (the start of r_end takes the groups' masks, that of r_dest the numbers)
 #pragma unroll
     for (int i = 0; i < kExpand; ++i) {
       const int32_t p = pb + 32 * i + lane;
@@ -583,13 +588,13 @@ __device__ bool SearchStep(const SearchArgs &g, const SeqView &v, const Team &tm
         const int32_t idx1 = (int32_t)(w[i] & 0x7fffffffu);
         atomicMax(&v.st_fwd[s1 + idx1], OrderedInt(end[i]));
         const int32_t at = entering + __popc(m & ((1u << lane) - 1u));
-        list_a[at] = p;
-        list_b[at] = idx1;
+        list[at] = p;
+        r_dest[lo + at] = idx1;
       }
-      if (lane == 0 && pb + 32 * i < hi) {
+      if (lane == 0 && pb + 32 * i < hi && hi - lo > 1) {
         const int32_t group = (pb - lo) / 32 + i;
-        r_end[lo + group] = __uint_as_float(m);
-        r_dest[lo + group] = entering;
+        r_end[lo + 2 * group] = __uint_as_float(m);
+        r_end[lo + 2 * group + 1] = __int_as_float(entering);
       }
       entering += __popc(m);
     }
@@ -607,8 +612,8 @@ __device__ bool SearchStep(const SearchArgs &g, const SeqView &v, const Team &tm
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int32_t at = i0 + 32 * i + lane;
-      p[i] = at < entering ? list_a[at] : -1;
-      idx1[i] = at < entering ? list_b[at] : 0;
+      p[i] = at < entering ? list[at] : -1;
+      idx1[i] = at < entering ? r_dest[lo + at] : 0;
     }
 #pragma unroll
     for (int i = 0; i < 2; ++i)
@@ -631,10 +636,13 @@ __device__ bool SearchStep(const SearchArgs &g, const SeqView &v, const Team &tm
       const int32_t f = k < ns ? v.st_cnt[s0 + k] : 0x7fffffff;
       if ((f > lo || tm.warp == 0) && f <= hi) {
         int32_t before = entering;
-        if (f < hi) {
+        if (f == lo) {
+          before = 0;
+        } else if (f < hi) {
           const int32_t group = (f - lo) >> 5;
-          const uint32_t m = __float_as_uint(r_end[lo + group]);
-          before = r_dest[lo + group] + __popc(m & ((1u << ((f - lo) & 31)) - 1u));
+          const uint32_t m = __float_as_uint(r_end[lo + 2 * group]);
+          before = __float_as_int(r_end[lo + 2 * group + 1]) +
+                   __popc(m & ((1u << ((f - lo) & 31)) - 1u));
         }
         v.st_arc0[s0 + k] = base + before;
       }
@@ -1412,8 +1420,7 @@ int32_t MakePrunedLayout(const k2b200_pruned_args *a, char *ws, PrunedLayout *L)
   g.arc_dest = i32(na);
   g.arc_ll = f32(na);
   g.arc_end = f32(na);
-  g.list_a = i32(na);
-  g.list_b = i32(na);
+  g.arc_deg = reinterpret_cast<uint8_t *>(ws + Take(&off, na));
   L->winner_bytes = 8 * (g.a_stride ? (size_t)std::max(a->num_states, 1)
                                     : n * (size_t)std::max(a->num_states, 1));
   g.winner = reinterpret_cast<unsigned long long *>(ws + Take(&off, L->winner_bytes));
