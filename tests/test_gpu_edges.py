@@ -1,0 +1,195 @@
+"""The kernels at the sizes where they could go wrong: edges of lanes, warps, blocks and slots,
+remainders, the smallest and the largest of a range, each branch of a dispatch.  Against the CPU
+oracle, or against another path of this package that the oracle pins."""
+import sys
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle
+from oracle.common import HostFsaVec, make_arcs
+from pruned_util import decoding_graph
+from util import close, random_dense, same_fsa
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.fixture(scope="module")
+def k2():
+    import k2_b200
+    return k2_b200
+
+
+# --------------------------------------------------------------------------- lattice scores
+def layered_lattice(rng, widths, degree, scale, hub=None):
+    """One FSA whose arcs go from a layer to the next; `degree` arcs into a state on average,
+    `hub` of them into the first state of the middle layer."""
+    first = np.concatenate([[0], np.cumsum(widths)])
+    rows = []
+    for l in range(1, len(widths)):
+        for s in range(widths[l]):
+            d = max(1, int(rng.poisson(degree)))
+            if hub and s == 0 and l == len(widths) // 2:
+                d = hub
+            for src in rng.integers(0, widths[l - 1], size=d):
+                label = -1 if l == len(widths) - 1 else int(rng.integers(0, 9))
+                rows.append((first[l - 1] + src, first[l] + s, label, rng.normal() * scale))
+    rows.sort(key=lambda r: r[0])
+    r = np.array(rows, np.float64)
+    rs2 = np.zeros(first[-1] + 1, np.int64)
+    np.add.at(rs2, r[:, 0].astype(np.int64) + 1, 1)
+    arcs = make_arcs(r[:, 0].astype(np.int32), r[:, 1].astype(np.int32),
+                     r[:, 2].astype(np.int32), r[:, 3].astype(np.float32))
+    host = HostFsaVec(np.array([0, first[-1]], np.int32), np.cumsum(rs2).astype(np.int32), arcs)
+    return host, first
+
+
+@pytest.mark.parametrize("widths,degree,scale,hub", [
+    ([1, 1], 1.0, 1.0, None),                        # one arc
+    ([1, 31, 32, 33, 1], 1.2, 1.0, None),            # two arcs per lane, a warp and its edges
+    ([1] + [40] * 70 + [1], 2.5, 1.0, None),         # three; several slots of 32 layers
+    ([1, 70, 64, 65, 1], 5.0, 1.0, 33),              # four; a state over several lanes
+    ([1, 30, 40, 50, 1], 12.0, 1.0, 300),            # eight; a state of more than 32 x 8 arcs
+    ([1, 600, 700, 600, 1], 3.0, 60.0, None),        # values out of the shared exponent's range
+    ([1, 500, 20000, 4097, 8, 1], 2.0, 1.0, None),   # wide: one to eight lanes per state
+    ([1, 18000, 3, 18000, 1], 2.0, 1.0, 700),        # wide, with a state for the whole warp
+])
+def test_lattice_scores_and_best_path(k2, widths, degree, scale, hub):
+    from gpu_util import host_to_fsa
+    rng = np.random.default_rng(len(widths))
+    host, first = layered_lattice(rng, widths, degree, scale, hub)
+    fsa = host_to_fsa(host)
+    arcs_per_layer = np.diff(host.row_splits2[first])
+    fsa.arcs._levels = (torch.tensor([0, len(widths)], dtype=torch.int32, device=DEV),
+                        torch.from_numpy(first.astype(np.int32)).to(DEV))
+    fsa.arcs._layer_bounds = (1, len(widths), int(max(widths)), int(arcs_per_layer.max()))
+    for log in (True, False):
+        for get, want in ((fsa.get_forward_scores, oracle.forward_scores(host, log)),
+                          (fsa.get_backward_scores, oracle.backward_scores(host, log))):
+            got = get(use_double_scores=True, log_semiring=log).detach().cpu().numpy()
+            assert close(got, want, rtol=1e-10, atol=1e-9)
+    best = k2.shortest_path(fsa, use_double_scores=True)
+    tot = fsa.get_tot_scores(log_semiring=False, use_double_scores=True)
+    assert best.num_arcs == (len(widths) - 1 if torch.isfinite(tot).all() else 0)
+    assert close(best.scores.double().sum().item(), tot[0].item(), rtol=1e-6, atol=1e-5)
+
+
+# --------------------------------------------------------------------------- CTC loss
+def ctc_inputs(rng, n, frames, classes, tokens, gaps):
+    durs = np.sort(rng.integers(max(1, frames // 2), frames + 1, size=n))[::-1]
+    durs[0] = frames
+    x = torch.from_numpy(rng.normal(size=(n, frames + gaps, classes)).astype(np.float32) * 1.5)
+    seg = np.stack([np.arange(n), np.full(n, gaps), durs], 1).astype(np.int32)
+    symbols = [rng.integers(1, classes, size=int(min(rng.integers(1, tokens + 1), d // 3))).tolist()
+               for d in durs]
+    for s in symbols[1::2]:  # repeats
+        s[1:2] = s[:1]
+    symbols[-1] = []
+    return x.to(DEV), torch.from_numpy(seg), symbols
+
+
+@pytest.mark.parametrize("n,frames,classes,tokens,modified,gaps,lens_dtype,logits,delay", [
+    (3, 1, 3, 1, False, 0, torch.int32, False, 0.0),       # one frame
+    (4, 15, 29, 5, False, 1, torch.int64, False, 0.0),     # odd columns, rows of no sequence
+    (3, 17, 501, 6, True, 0, torch.float32, True, 0.0),
+    (2, 33, 1023, 11, False, 3, torch.float64, True, 0.0),
+    (3, 40, 1500, 12, True, 0, torch.int32, False, 0.0),   # rows by state
+    (2, 800, 40, 270, False, 0, torch.int64, False, 0.0),  # more than 512 states
+    (3, 60, 30, 20, False, 2, torch.int32, False, 0.1),
+    (3, 50, 1300, 16, True, 0, torch.int64, True, 0.2),
+    (2, 600, 31, 190, False, 0, torch.int32, False, 0.2),  # the exact recursion
+])
+def test_ctc_loss_on_the_band_kernels(k2, n, frames, classes, tokens, modified, gaps, lens_dtype,
+                                      logits, delay):
+    module = sys.modules["k2_b200.ctc_loss"]
+    rng = np.random.default_rng(frames + classes)
+    x, seg, symbols = ctc_inputs(rng, n, frames, classes, tokens, gaps)
+    if not logits:
+        x = torch.log_softmax(x, -1)
+    make = k2.DenseFsaVec.from_logits if logits else k2.DenseFsaVec
+    lens = torch.tensor([max(1, len(s)) for s in symbols], dtype=lens_dtype, device=DEV)
+    for reduction in ("sum", "mean"):
+        got = []
+        for fused in (True, False):
+            module.FUSED_LOSS = fused
+            try:
+                graphs = k2.ctc_graph(symbols, modified=modified, device=DEV)
+                leaf = x.clone().requires_grad_(True)
+                loss = k2.ctc_loss(graphs, make(leaf, seg), output_beam=10.0, delay_penalty=delay,
+                                   reduction=reduction, target_lengths=lens)
+                loss.backward()
+            finally:
+                module.FUSED_LOSS = True
+            got.append((loss.item(), leaf.grad.cpu().numpy()))
+        assert close(got[0][0], got[1][0], rtol=1e-5, atol=1e-4)
+        assert np.abs(got[0][1] - got[1][1]).max() <= 1e-4
+
+
+@pytest.mark.parametrize("modified", [False, True])
+@pytest.mark.parametrize("lengths", [[0], [1], [0, 3, 0], [31, 32, 33], [500, 0, 511, 512]])
+def test_ctc_graph_on_the_device(k2, lengths, modified):
+    from gpu_util import fsa_to_host
+    rng = np.random.default_rng(len(lengths))
+    symbols = [rng.integers(1, 3, size=k).tolist() for k in lengths]  # many repeats
+    got = k2.ctc_graph(symbols, modified=modified, device=DEV)
+    same_fsa(fsa_to_host(got), oracle.ctc_graphs(symbols, modified), f"{lengths}")
+    cpu = k2.ctc_graph(symbols, modified=modified, device="cpu")
+    assert torch.equal(got.aux_labels.cpu(), cpu.aux_labels)
+
+
+# --------------------------------------------------------------------------- planned lanes
+@pytest.mark.parametrize("phones", [40, 78, 80, 84, 105])  # around 768 and 1024 lanes
+def test_lane_plans(k2, phones):
+    from k2_b200 import synthetic as syn
+    rs2, arcs = syn.den_graph(phones, phones)
+    rng = np.random.default_rng(phones)
+    lp = np.log(rng.dirichlet(np.ones(phones + 1) * 0.3, size=(2, 12))).astype(np.float32)
+    w = syn.Workload("lfmmi", torch.from_numpy(lp), torch.tensor([[0, 0, 12], [1, 0, 9]],
+                                                                dtype=torch.int32), 8.0,
+                     graph_row_splits2=rs2, graph_arcs=arcs, num_symbols=None)
+    graphs = syn.build_graphs(w, DEV)
+    got = []
+    for fused in (True, False):
+        x = w.log_probs.to(DEV).requires_grad_(True)
+        dense = k2.DenseFsaVec(x, w.supervision_segments)
+        if fused:
+            tot = k2.intersect_dense_tot_scores(graphs, dense, 8.0)
+        else:
+            tot = k2.intersect_dense(graphs, dense, 8.0).get_tot_scores(True, True)
+        tot.sum().backward()
+        got.append((tot.detach().cpu().numpy(), x.grad.cpu().numpy()))
+    assert close(got[0][0], got[1][0], rtol=1e-6, atol=1e-5)
+    assert np.abs(got[0][1] - got[1][1]).max() <= 1e-4
+
+
+# --------------------------------------------------------------------------- pruned search
+@pytest.mark.parametrize("states,classes,hub,n,teams", [
+    (50, 5, 0, 1, (0, 1, 2, 8)),       # fewer arcs than a warp has lanes
+    (900, 20, 700, 2, (0, 1)),         # a state of more arcs than a byte counts
+    (400, 9000, 0, 2, (0,)),           # rows of scores that stay in global memory
+    (270000, 30, 0, 1, (0, 1)),        # states that share a bit of the set of new states
+])
+def test_pruned_search(k2, states, classes, hub, n, teams):
+    from gpu_util import dense_from_scores, fsa_to_host, host_to_fsa
+    from k2_b200.autograd import _intersect_dense_pruned_arcs
+    rng = np.random.default_rng(states)
+    g = decoding_graph(rng, states, classes, mean_degree=4.0)
+    if hub:  # the arcs of the start state once more, with other labels
+        s0 = g.row_splits2[1]
+        label = rng.integers(1, classes, size=hub).astype(np.int32)
+        dest = rng.integers(1, states // 2, size=hub).astype(np.int32)
+        extra = make_arcs(np.zeros(hub, np.int32), dest, label,
+                          rng.normal(size=hub).astype(np.float32))
+        arcs = np.concatenate([g.arcs[:s0], extra, g.arcs[s0:]])
+        rs2 = g.row_splits2.copy()
+        rs2[1:] += hub
+        g = HostFsaVec(g.row_splits1, rs2, arcs)
+    scores, brs = random_dense(rng, n, 45, classes, scale=2.0, low_rows=False)
+    params = (14.0, 6.0, 5, 700, False)
+    want = oracle.intersect_dense_pruned(g, scores, brs, *params)
+    a, dense = host_to_fsa(g), dense_from_scores(scores, brs)
+    for team in teams:
+        ragged, ma, mb = _intersect_dense_pruned_arcs(a.arcs, dense, *params, team)
+        same_fsa(fsa_to_host(k2.Fsa(ragged, _check=False), ma, mb), want, f"{team} CTAs")
