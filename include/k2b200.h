@@ -235,7 +235,7 @@ typedef struct {
    * 2 = persistent frame-synchronous kernel (graphs that fit in shared memory),
    * 3 = persistent kernel with the arcs in registers (needs a_max_degree <= 4
    *     and at most 1024 states per graph), 4 = persistent kernel with a lane plan
-   *     (graphs of at most 768 states with states of more than four arcs),
+   *     (graphs of at most 1024 states with states of more than four arcs),
    * 5 = one launch per frame with the sequences on the lanes of a warp (needs a_shared
    *     and at least two sequences; what 0 chooses for a shared graph too large for 2-4) */
   int32_t viterbi_mode;

@@ -32,12 +32,14 @@
 //                 with a per-level scale can hold or whose levels are wider than the registers
 //                 of a warp; it runs after BandChainLists and returns at once for every other
 //                 graph.
-//   BandGrad      all levels in parallel: posterior of (level, state) = alpha * beta / Z is the
-//                 gradient of that state's dense score; optionally arc posteriors for the
+//   BandGradRows  all levels in parallel: posterior of (level, state) = alpha * beta / Z is the
+//                 gradient of that state's dense score; every row of the gradient is written
+//                 whole.
+//   BandGrad      the same added to rows that sequences share, and arc posteriors for the
 //                 gradient of the graph's arc scores.
 //
 // The dense scores are read straight from the log-prob tensor the DenseFsaVec was made from
-// ([rows, C], 16-byte aligned rows): the [rows + N, C + 1] score matrix is not needed.  The extra
+// ([rows, C], any C): the [rows + N, C + 1] score matrix is not needed.  The extra
 // final row of a sequence ([0, -inf, ...], k2/csrc/fsa.h:138-185) is implied: on the level after
 // the last frame a state scores 0 if its label is -1 and -inf otherwise.
 #include <algorithm>
