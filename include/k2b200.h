@@ -533,6 +533,10 @@ int32_t k2b200_band_tables_bytes(int32_t num_states, size_t *states_bytes, size_
 int32_t k2b200_band_tables(const int32_t *row_splits1, int32_t num_fsas,
                            const int32_t *row_splits2, const void *arcs, int32_t num_states,
                            void *band_states, void *band_arcs, int32_t *status, void *stream);
+/* The incoming-arc index (as k2b200_fsa_incoming) of graphs whose band tables exist. */
+int32_t k2b200_band_incoming(const void *band_states, const void *band_arcs,
+                             const int32_t *row_splits2, int32_t num_states, int32_t *in_splits,
+                             int32_t *in_arcs, int32_t *in_src, float *in_score, void *stream);
 int32_t k2b200_band_loss_supported(const k2b200_band_loss_args *args, int32_t *supported);
 int32_t k2b200_band_loss_workspace_bytes(const k2b200_band_loss_args *args, size_t *bytes);
 int32_t k2b200_band_loss_forward(const k2b200_band_loss_args *args, void *workspace,

@@ -196,6 +196,7 @@ _sig("k2b200_dense_loss_backward", c_i32,
      [ctypes.POINTER(IntersectArgs), c_vp, c_sz, c_vp, c_i32, c_vp, c_vp, c_vp])
 _sig("k2b200_band_tables_bytes", c_i32, [c_i32, ctypes.POINTER(c_sz), ctypes.POINTER(c_sz)])
 _sig("k2b200_band_tables", c_i32, [c_vp, c_i32, c_vp, c_vp, c_i32, c_vp, c_vp, c_vp, c_vp])
+_sig("k2b200_band_incoming", c_i32, [c_vp, c_vp, c_vp, c_i32, c_vp, c_vp, c_vp, c_vp, c_vp])
 _sig("k2b200_band_loss_supported", c_i32,
      [ctypes.POINTER(BandLossArgs), ctypes.POINTER(c_i32)])
 _sig("k2b200_band_loss_workspace_bytes", c_i32,
@@ -297,7 +298,8 @@ EXPORTED = [
     "k2b200_online_decode_workspace_bytes", "k2b200_online_decode_load",
     "k2b200_online_decode_run", "k2b200_online_decode_emit", "k2b200_online_decode_store",
     "k2b200_online_decode_load_all", "k2b200_online_decode_store_all",
-    "k2b200_band_tables_bytes", "k2b200_band_tables", "k2b200_band_loss_supported",
+    "k2b200_band_tables_bytes", "k2b200_band_tables", "k2b200_band_incoming",
+    "k2b200_band_loss_supported",
     "k2b200_band_loss_workspace_bytes", "k2b200_band_loss_forward",
     "k2b200_band_loss_backward", "k2b200_band_loss_status", "k2b200_band_loss_plan",
     "k2b200_band_loss_forward_reduce", "k2b200_band_loss_backward_dense",

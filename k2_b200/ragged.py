@@ -161,6 +161,17 @@ class RaggedArc:
             dev = self.device
             in_splits = torch.empty(ns + 1, dtype=torch.int32, device=dev)
             buf = torch.empty((3, max(na, 1)), dtype=torch.int32, device=dev)
+            band = getattr(self, "_band_graph", None)
+            if band is not None and band[0] == key and band[1] is not None:
+                with torch.cuda.device(dev):
+                    _lib.check(_lib.lib.k2b200_band_incoming(
+                        band[1].states_ptr, band[1].arcs_ptr, _lib.ptr(self._row_splits2), ns,
+                        _lib.ptr(in_splits), buf[0].data_ptr(), buf[1].data_ptr(),
+                        buf[2].data_ptr(), _lib.stream_of(dev)))
+                self._incoming = (in_splits, buf[0, :na], buf[1, :na],
+                                  buf[2, :na].view(torch.float32))
+                self._incoming_key = key
+                return self._incoming
             if self._layer_bounds[0] and self._incoming_by_layers(in_splits, buf):
                 self._incoming = (in_splits, buf[0, :na], buf[1, :na],
                                   buf[2, :na].view(torch.float32))

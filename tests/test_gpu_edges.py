@@ -193,3 +193,15 @@ def test_pruned_search(k2, states, classes, hub, n, teams):
     for team in teams:
         ragged, ma, mb = _intersect_dense_pruned_arcs(a.arcs, dense, *params, team)
         same_fsa(fsa_to_host(k2.Fsa(ragged, _check=False), ma, mb), want, f"{team} CTAs")
+
+
+@pytest.mark.parametrize("lengths", [[0], [1, 0], [2, 31, 32], [130, 1, 0, 64]])
+def test_incoming_arcs_of_band_graphs(k2, lengths):
+    rng = np.random.default_rng(sum(lengths))
+    symbols = [rng.integers(1, 3, size=k).tolist() for k in lengths]
+    for modified in (False, True):
+        arcs = k2.ctc_graph(symbols, modified=modified, device=DEV).arcs
+        want = k2.ctc_graph(symbols, modified=modified, device=DEV).arcs
+        want._band_graph = None  # the general index
+        for got, ref in zip(arcs.incoming(), want.incoming()):
+            assert torch.equal(got, ref), (lengths, modified)
