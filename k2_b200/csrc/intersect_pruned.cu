@@ -262,7 +262,9 @@ __device__ float NextBeam(float dyn, float best, int32_t active, int32_t t, int3
   return dyn;
 }
 
-constexpr int kExpand = 4;   // groups of 32 arcs whose loads a warp issues together
+// Groups of 32 arcs whose loads a warp issues together.  A thread has 64 registers: with four
+// the kernel spilled more than the loads in flight gained (54.3 ms, with two 52.8).
+constexpr int kExpand = 2;
 
 // Entries of the direct table that replaces the reference's hash: the frame in the
 // high word, so that entries of earlier frames lose against any entry of this frame
@@ -285,6 +287,17 @@ __device__ __forceinline__ int32_t ArcsPerWarp(int32_t na, const Team &tm) {
 __device__ __forceinline__ void SetWarpFirst(const SeqView &v, int32_t per_warp, int32_t k,
                                              int32_t f, int32_t deg) {
   for (int32_t w = (f + per_warp - 1) / per_warp; w * per_warp < f + deg; ++w) v.warp_first[w] = k;
+}
+
+// A graph arc, read-only for the whole launch.
+__device__ __forceinline__ Arc LoadArc(const Arc *p) {
+  const int4 x = __ldg(reinterpret_cast<const int4 *>(p));
+  Arc arc;
+  arc.src = x.x;
+  arc.dest = x.y;
+  arc.label = x.z;
+  arc.score = __int_as_float(x.w);
+  return arc;
 }
 
 // The scores of a row of the dense matrix into shared memory, when they fit.
@@ -373,7 +386,7 @@ __device__ bool SearchStep(const SearchArgs &g, const SeqView &v, const Team &tm
 
   // graph of this sequence: its final state, for allow_partial (:861-871)
   const int32_t gi = seq * g.a_stride;
-  const int32_t g_final = g.a_rs1[gi + 1] - 1;
+  const int32_t g_start = g.a_rs1[gi], g_final = g.a_rs1[gi + 1] - 1;
   bool redirect = false;
   if (g.allow_partial && t == final_t - 1) {
     // is there any arc with label -1 among the arcs expanded on this frame (:839-857)
@@ -395,28 +408,27 @@ __device__ bool SearchStep(const SearchArgs &g, const SeqView &v, const Team &tm
   const int32_t k_first = lo < hi ? v.warp_first[tm.warp] : ns;
   for (int32_t k0 = k_first; k0 < ns; k0 += 32) {
     const int32_t k = k0 + lane;
-    int32_t f = na, as = 0, fwd = 0, ga0 = 0;
+    int32_t f = na, fwd = 0, ga0 = 0;
     if (k < ns) {
       f = v.st_cnt[s0 + k];
-      as = v.st_astate[s0 + k];
       fwd = v.st_fwd[s0 + k];
-      ga0 = g.a_rs2[as];
+      ga0 = __ldg(g.a_rs2 + v.st_astate[s0 + k]);
     }
     int32_t next = __shfl_down_sync(kAll, f, 1);
     if (lane == 31) next = k + 1 < ns ? v.st_cnt[s0 + k + 1] : na;
     const int32_t start = max(lo, __shfl_sync(kAll, f, 0));
     const int32_t chunk_end = __shfl_sync(kAll, next, 31), stop = min(hi, chunk_end);
     ArcWalk walk;
-    walk.Begin(sh->rec[warp], f, next, make_int4(ga0 - f, as, fwd, 0), start);
+    walk.Begin(sh->rec[warp], f, next, make_int4(ga0 - f, fwd, 0, 0), start);
     for (int32_t pb = start; pb < stop; pb += 32 * kExpand) {
-      int4 rec[kExpand];
+      int2 rec[kExpand];
       Arc arc[kExpand];
 #pragma unroll
       for (int i = 0; i < kExpand; ++i) {
         const int32_t p = pb + 32 * i + lane, r = walk.Next(pb + 32 * i);
         if (p < stop) {
-          rec[i] = sh->rec[warp][r];
-          arc[i] = g.a_arcs[p + rec[i].x];
+          rec[i] = *reinterpret_cast<const int2 *>(&sh->rec[warp][r]);
+          arc[i] = LoadArc(g.a_arcs + (p + rec[i].x));
         }
       }
 #pragma unroll
@@ -425,13 +437,13 @@ __device__ bool SearchStep(const SearchArgs &g, const SeqView &v, const Team &tm
         if (p < stop) {
           const uint32_t col = (uint32_t)(arc[i].label + 1);
           float acoustic = (row_ok && col < (uint32_t)g.cols) ? row[col] : kNegInf;
-          int32_t dest = rec[i].y + arc[i].dest - arc[i].src;
+          int32_t dest = g_start + arc[i].dest;
           if (redirect) {
             dest = g_final;
             acoustic = 0.0f;
           }
           const float ll = acoustic + arc[i].score;
-          const float end = OrderedFloat(rec[i].z) + ll;
+          const float end = OrderedFloat(rec[i].y) + ll;
           r_aidx[p] = p + rec[i].x;
           r_ll[p] = ll;
           r_dest[p] = dest;
