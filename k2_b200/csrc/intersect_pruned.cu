@@ -78,7 +78,7 @@ struct SearchArgs {
   float *arc_ll, *arc_end;
   uint8_t *arc_deg;           // scratch: arcs leaving a new state, 255 for that many or more
   unsigned long long *winner;  // [num_seqs * a_states] (shared) or [a_states]
-  int32_t *frame_s0, *frame_a0, *frame_n0, *frame_m0;  // [num_seqs][T + 2], the last two scratch
+  int32_t *frame_s0, *frame_a0;  // [num_seqs][T + 2]
   int32_t *warp_first;         // [num_seqs][kTeamWarps]
   int32_t *seq_out;           // [num_seqs][kSeqOut]: states, arcs, extra final state, status,
                               // most states of a frame, most arcs leaving one
@@ -104,7 +104,7 @@ struct Shared {
   unsigned long long cta_val[kSlots][kMaxTeam];
   unsigned long long warp_val[kWarps], warp_ex[kWarps];
   int4 rec[kWarps][32];                           // per warp: the states whose arcs it walks
-  int32_t wbest[kWarps][32], wcnt[kWarps][32];
+  int32_t wbest[kWarps][32];
   uint32_t mark[kMarkWords];
   float row[kMaxRow];
   int32_t most_states, most_arcs;
@@ -209,7 +209,7 @@ struct SeqView {
   float *arc_ll, *arc_end;
   uint8_t *arc_deg;
   unsigned long long *winner;
-  int32_t *frame_s0, *frame_a0, *frame_n0, *frame_m0, *warp_first;
+  int32_t *frame_s0, *frame_a0, *warp_first;
 };
 
 __device__ __forceinline__ SeqView ViewOf(const SearchArgs &g, int32_t seq) {
@@ -231,8 +231,6 @@ __device__ __forceinline__ SeqView ViewOf(const SearchArgs &g, int32_t seq) {
   v.winner = g.winner + (g.a_stride ? 0 : (int64_t)seq * g.a_states);
   v.frame_s0 = g.frame_s0 + (int64_t)seq * (g.T + 2);
   v.frame_a0 = g.frame_a0 + (int64_t)seq * (g.T + 2);
-  v.frame_n0 = g.frame_n0 + (int64_t)seq * (g.T + 2);
-  v.frame_m0 = g.frame_m0 + (int64_t)seq * (g.T + 2);
   v.warp_first = g.warp_first + (int64_t)seq * kTeamWarps;
   return v;
 }
@@ -672,8 +670,10 @@ __device__ bool SearchStep(const SearchArgs &g, const SeqView &v, const Team &tm
 // arcs; on return *s_top / *a_top are the ends of the arenas and the frame tables are
 // updated.  Returns false when an arena has no room for the survivors twice.
 //
-// One barrier per frame for the backward pass.  The surviving states and arcs of all frames
-// are then numbered by one exchange, gathered at the far end of the arenas and copied back.
+// One barrier per frame for the backward pass, which leaves a record per 32 states of a frame (a
+// unit): which survive and how many arcs, later the first of either.  One exchange of sums
+// numbers the survivors of all frames; where a state goes follows from its unit's record.  They
+// are gathered at the far end of the arenas and copied back.
 __device__ bool PruneWindow(const SearchArgs &g, const SeqView &v, const Team &tm, int32_t seq,
                             int32_t begin, int32_t end, int32_t *s_top, int32_t *a_top,
                             bool keep_all_at_begin = true) {
@@ -695,18 +695,25 @@ __device__ bool PruneWindow(const SearchArgs &g, const SeqView &v, const Team &t
   }
   tm.Sync();
 
-  // ---- backwards: arc survival, the number of surviving arcs and the backward score of every
-  // state; the destination of a surviving arc becomes its place in the arena, that of
-  // another -1
+  // the records of the units: a frame may leave one number unused behind its own, so that
+  // unit 0 of a frame follows from its first state
+  const int32_t num_units = (se - sb) / 32 + (end - begin);
+  if (3 * (int64_t)num_units > g.cap_s) return false;
+  int32_t *unit_mask = v.st_new, *unit_s = v.st_new + num_units, *unit_a = unit_s + num_units;
+  auto unit0 = [&](int32_t t, int32_t s0) { return (s0 - sb) / 32 + (t - begin); };
+
+  // ---- backwards: arc survival (the destination of another arc becomes -1) and the backward
+  // score of every state
   {
     int32_t s0 = v.frame_s0[end], a1 = v.frame_a0[end];
     for (int32_t t = end - 1; t >= begin; --t) {
       const int32_t s_next = s0, a_next = a1;
       s0 = v.frame_s0[t];
       a1 = v.frame_a0[t];
-      const int32_t ns = s_next - s0;
-      for (int32_t k0 = tm.warp * 32; k0 < ns; k0 += tm.warps * 32) {
-        const int32_t k = k0 + lane;
+      const int32_t ns = s_next - s0, u0 = unit0(t, s0), units = unit0(t + 1, s_next) - u0;
+      const bool keep_all = t == begin && keep_all_at_begin;
+      for (int32_t u = tm.warp; u < units; u += tm.warps) {
+        const int32_t k = u * 32 + lane;
         int32_t f = a_next, fwd = 0, as = 0;
         if (k < ns) {
           f = v.st_arc0[s0 + k];
@@ -716,17 +723,16 @@ __device__ bool PruneWindow(const SearchArgs &g, const SeqView &v, const Team &t
         int32_t next = __shfl_down_sync(kAll, f, 1);
         if (lane == 31) next = k + 1 < ns ? v.st_arc0[s0 + k + 1] : a_next;
         sh->wbest[warp][lane] = OrderedInt(kNegInf);
-        sh->wcnt[warp][lane] = 0;
         const int32_t start = __shfl_sync(kAll, f, 0), stop = __shfl_sync(kAll, next, 31);
+        int32_t arcs = 0;
         ArcWalk walk;
         walk.Begin(sh->rec[warp], f, next, make_int4(fwd, lane, 0, 0), start);
         for (int32_t pb = start; pb < stop; pb += 64) {
-          int32_t r[2], d[2];
+          int32_t d[2];
           float ll[2], nb[2];
 #pragma unroll
           for (int i = 0; i < 2; ++i) {
             const int32_t p = pb + 32 * i + lane;
-            r[i] = walk.Next(pb + 32 * i);
             d[i] = p < stop ? v.arc_dest[p] : -1;
             ll[i] = p < stop ? v.arc_ll[p] : 0.0f;
           }
@@ -734,24 +740,26 @@ __device__ bool PruneWindow(const SearchArgs &g, const SeqView &v, const Team &t
           for (int i = 0; i < 2; ++i) nb[i] = d[i] >= 0 ? v.st_bwd[s_next + d[i]] : kNegInf;
 #pragma unroll
           for (int i = 0; i < 2; ++i) {
-            const int32_t p = pb + 32 * i + lane;
+            const int32_t p = pb + 32 * i + lane, r = walk.Next(pb + 32 * i);
+            bool keep = false;
             if (p < stop) {
-              const int4 rec = sh->rec[warp][r[i]];
+              const int2 rec = *reinterpret_cast<const int2 *>(&sh->rec[warp][r]);
               const float bl = ll[i] + nb[i];
-              int32_t to = -1;
-              if (d[i] >= 0 && bl + OrderedFloat(rec.x) >= -beam) {
-                to = s_next + d[i];
-                atomicMax(&sh->wbest[warp][rec.y], OrderedInt(bl));
-                atomicAdd(&sh->wcnt[warp][rec.y], 1);
-              }
-              v.arc_dest[p] = to;
+              keep = d[i] >= 0 && bl + OrderedFloat(rec.x) >= -beam;
+              if (keep) atomicMax(&sh->wbest[warp][rec.y], OrderedInt(bl));
+              else v.arc_dest[p] = -1;
             }
+            arcs += __popc(__ballot_sync(kAll, keep));
           }
         }
         __syncwarp();
-        if (k < ns) {
-          v.st_cnt[s0 + k] = sh->wcnt[warp][lane];
-          v.st_bwd[s0 + k] = as == g_final ? -OrderedFloat(fwd) : OrderedFloat(sh->wbest[warp][lane]);
+        const float bwd =
+            as == g_final ? -OrderedFloat(fwd) : OrderedFloat(sh->wbest[warp][lane]);
+        if (k < ns) v.st_bwd[s0 + k] = bwd;
+        const uint32_t kept = __ballot_sync(kAll, k < ns && (bwd != kNegInf || keep_all));
+        if (lane == 0) {
+          unit_mask[u0 + u] = (int32_t)kept;
+          unit_a[u0 + u] = arcs;
         }
         __syncwarp();
       }
@@ -759,85 +767,81 @@ __device__ bool PruneWindow(const SearchArgs &g, const SeqView &v, const Team &t
     }
   }
 
-  // ---- new numbers: of a state (st_new) and of its first arc (st_cnt), whether it survives
-  // or not.  A warp takes a contiguous range of the window's states.
-  const int32_t n = se - sb, all_to = keep_all_at_begin ? v.frame_s0[begin + 1] : sb;
-  const int32_t per_warp = ((n + tm.warps - 1) / tm.warps + 31) & ~31;
-  const int32_t lo = sb + (int32_t)min((int64_t)tm.warp * per_warp, (int64_t)n);
-  const int32_t hi = min(lo + per_warp, se);
-  uint32_t states = 0, arcs = 0;
-#pragma unroll 2
-  for (int32_t s = lo + lane; s < hi; s += 32) {
-    states += v.st_bwd[s] != kNegInf || s < all_to;
-    arcs += (uint32_t)v.st_cnt[s];
+  // ---- new numbers: the first surviving state and arc of every unit
+  int32_t ks, ka;
+  {
+    const int32_t per_warp = (num_units + tm.warps - 1) / tm.warps;
+    const int32_t lo = min(tm.warp * per_warp, num_units), hi = min(lo + per_warp, num_units);
+    uint32_t states = 0, arcs = 0;
+    for (int32_t i = lo + lane; i < hi; i += 32) {
+      states += __popc(unit_mask[i]);
+      arcs += (uint32_t)unit_a[i];
+    }
+    states = __reduce_add_sync(kAll, states);
+    arcs = __reduce_add_sync(kAll, arcs);
+    unsigned long long total;
+    const unsigned long long base = tm.ScanWarps(
+        kSlotWindow, (unsigned long long)states | ((unsigned long long)arcs << 32), &total);
+    ks = (int32_t)(total & 0xffffffffu);
+    ka = (int32_t)(total >> 32);
+    int32_t j = sb + (int32_t)(base & 0xffffffffu), q = ab + (int32_t)(base >> 32);
+    for (int32_t i0 = lo; i0 < hi; i0 += 32) {
+      const bool in = i0 + lane < hi;
+      const int32_t n = in ? __popc(unit_mask[i0 + lane]) : 0, a = in ? unit_a[i0 + lane] : 0;
+      int32_t inc_s = n, inc_a = a;
+#pragma unroll
+      for (int x = 1; x < 32; x <<= 1) {
+        const int32_t o = __shfl_up_sync(kAll, inc_s, x), p = __shfl_up_sync(kAll, inc_a, x);
+        if (lane >= x) {
+          inc_s += o;
+          inc_a += p;
+        }
+      }
+      if (in) {
+        unit_s[i0 + lane] = j + inc_s - n;
+        unit_a[i0 + lane] = q + inc_a - a;
+      }
+      j += __shfl_sync(kAll, inc_s, 31);
+      q += __shfl_sync(kAll, inc_a, 31);
+    }
   }
-  states = __reduce_add_sync(kAll, states);
-  arcs = __reduce_add_sync(kAll, arcs);
-  unsigned long long total;
-  const unsigned long long base = tm.ScanWarps(
-      kSlotWindow, (unsigned long long)states | ((unsigned long long)arcs << 32), &total);
-  const int32_t ks = (int32_t)(total & 0xffffffffu), ka = (int32_t)(total >> 32);
   // where the survivors are gathered: the states (and those of frame `end`) and the arcs
   const int64_t hold_s = g.cap_s - ks - ns_end, hold_a = g.cap_a - ka;
   if (hold_s < *s_top || hold_a < *a_top) return false;
-  {
-    int32_t j = sb + (int32_t)(base & 0xffffffffu), q = ab + (int32_t)(base >> 32);
-    for (int32_t s0 = lo; s0 < hi; s0 += 32) {
-      const int32_t s = s0 + lane;
-      const bool keep = s < hi && (v.st_bwd[s] != kNegInf || s < all_to);
-      const int32_t cnt = s < hi ? v.st_cnt[s] : 0;
-      const uint32_t m = __ballot_sync(kAll, keep);
-      int32_t inc = cnt;
-#pragma unroll
-      for (int x = 1; x < 32; x <<= 1) {
-        const int32_t o = __shfl_up_sync(kAll, inc, x);
-        if (lane >= x) inc += o;
-      }
-      if (s < hi) {
-        const int32_t at = j + __popc(m & ((1u << lane) - 1u));
-        v.st_new[s] = at;
-        v.st_cnt[s] = q + inc - cnt;
-        if (keep) {
-          const int64_t h = hold_s + (at - sb);
-          v.st_astate[h] = v.st_astate[s];
-          v.st_fwd[h] = v.st_fwd[s];
-          v.st_arc0[h] = q + inc - cnt;
-        }
-      }
-      j += __popc(m);
-      q += __shfl_sync(kAll, inc, 31);
-    }
-    for (int32_t k = tm.tid; k < ns_end; k += tm.threads) {
-      const int64_t h = hold_s + ks + k;
-      v.st_astate[h] = v.st_astate[se + k];
-      v.st_fwd[h] = v.st_fwd[se + k];
-      v.st_new[h] = v.st_cnt[se + k];
-    }
+  for (int32_t k = tm.tid; k < ns_end; k += tm.threads) {
+    const int64_t h = hold_s + ks + k;
+    v.st_astate[h] = v.st_astate[se + k];
+    v.st_fwd[h] = v.st_fwd[se + k];
+    v.st_cnt[h] = v.st_cnt[se + k];
   }
   tm.Sync();
-  // ---- the surviving arcs, 32 states of a frame to a warp: their arcs are consecutive, and
-  // so are the places they go to
-  for (int32_t t = begin + tm.tid; t < end; t += tm.threads) {
-    const int32_t s = v.frame_s0[t];
-    v.frame_n0[t] = s < se ? v.st_new[s] : sb + ks;
-    v.frame_m0[t] = s < se ? v.st_cnt[s] : ab + ka;
-  }
+  // ---- the survivors: the arcs of a unit are consecutive, and so are the places they go to
   {
-    int32_t turn = 0;  // units of 32 states so far, modulo the warps
+    int32_t turn = 0;  // units so far, modulo the warps
     int32_t s1 = sb, a1 = ab;
     for (int32_t t = begin; t < end; ++t) {
       const int32_t s0 = s1;
       s1 = v.frame_s0[t + 1];
       a1 = v.frame_a0[t + 1];
-      const int32_t ns = s1 - s0;
-      // where frame t + 1 will start (the states of frame `end` keep their numbers)
-      const int32_t new_s1 = t + 1 == end ? 0 : (s1 < se ? v.st_new[s1] : sb + ks);
+      const int32_t ns = s1 - s0, u0 = unit0(t, s0), u1 = unit0(t + 1, s1), units = u1 - u0;
+      const bool last = t + 1 == end;  // the states of frame `end` keep their numbers
+      const int32_t new_s1 = last ? 0 : unit_s[u1];
       int32_t u = tm.warp - turn;
       if (u < 0) u += tm.warps;
-      for (int32_t k0 = u * 32; k0 < ns; k0 += tm.warps * 32) {
-        const int32_t start = v.st_arc0[s0 + k0];
-        const int32_t stop = k0 + 32 < ns ? v.st_arc0[s0 + k0 + 32] : a1;
-        int64_t h = hold_a + (v.st_cnt[s0 + k0] - ab);
+      for (; u < units; u += tm.warps) {
+        const int32_t k = u * 32 + lane;
+        int32_t f = a1, as = 0, fwd = 0;
+        if (k < ns) {
+          f = v.st_arc0[s0 + k];
+          as = v.st_astate[s0 + k];
+          fwd = v.st_fwd[s0 + k];
+        }
+        const uint32_t kept = (uint32_t)unit_mask[u0 + u];
+        const int32_t first_s = unit_s[u0 + u];
+        int32_t q = unit_a[u0 + u];
+        const int32_t start = __shfl_sync(kAll, f, 0);
+        const int32_t stop = u * 32 + 32 < ns ? v.st_arc0[s0 + u * 32 + 32] : a1;
+        int32_t my_q = q;
         for (int32_t pb = start; pb < stop; pb += 64) {
           int32_t d[2], aidx[2];
           float ll[2];
@@ -851,22 +855,35 @@ __device__ bool PruneWindow(const SearchArgs &g, const SeqView &v, const Team &t
             if (d[i] >= 0) {
               aidx[i] = v.arc_aidx[pb + 32 * i + lane];
               ll[i] = v.arc_ll[pb + 32 * i + lane];
-              d[i] = t + 1 == end ? d[i] - se : v.st_new[d[i]] - new_s1;
+              if (!last) {
+                const int32_t to = u1 + (d[i] >> 5);
+                d[i] = unit_s[to] - new_s1 +
+                       __popc((uint32_t)unit_mask[to] & ((1u << (d[i] & 31)) - 1u));
+              }
             }
 #pragma unroll
           for (int i = 0; i < 2; ++i) {
             const uint32_t m = __ballot_sync(kAll, d[i] >= 0);
             if (d[i] >= 0) {
-              const int64_t at = h + __popc(m & ((1u << lane) - 1u));
+              const int64_t at = hold_a + (q - ab) + __popc(m & ((1u << lane) - 1u));
               v.arc_aidx[at] = aidx[i];
               v.arc_ll[at] = ll[i];
               v.arc_dest[at] = d[i];
             }
-            h += __popc(m);
+            const uint32_t x = (uint32_t)(f - (pb + 32 * i));
+            if (x < 32u) my_q = q + __popc(m & ((1u << x) - 1u));
+            q += __popc(m);
           }
         }
+        if (f >= stop) my_q = q;  // no arc at or behind its place
+        if ((kept >> lane) & 1u) {
+          const int64_t h = hold_s + (first_s - sb) + __popc(kept & ((1u << lane) - 1u));
+          v.st_astate[h] = as;
+          v.st_fwd[h] = fwd;
+          v.st_arc0[h] = my_q;
+        }
       }
-      turn = (turn + (ns + 31) / 32) % tm.warps;
+      turn = (turn + units) % tm.warps;
     }
   }
   tm.Sync();
@@ -882,11 +899,13 @@ __device__ bool PruneWindow(const SearchArgs &g, const SeqView &v, const Team &t
     v.st_astate[sb + k] = v.st_astate[hold_s + k];
     v.st_fwd[sb + k] = v.st_fwd[hold_s + k];
     if (k < ks) v.st_arc0[sb + k] = v.st_arc0[hold_s + k];
-    else v.st_cnt[sb + k] = v.st_new[hold_s + k];
+    else v.st_cnt[sb + k] = v.st_cnt[hold_s + k];
   }
+  // (a frame's first unit follows from its old first state, which nobody else reads now)
   for (int32_t t = begin + tm.tid; t <= end; t += tm.threads) {
-    v.frame_s0[t] = t < end ? v.frame_n0[t] : sb + ks;
-    v.frame_a0[t] = t < end ? v.frame_m0[t] : ab + ka;
+    const int32_t u = t < end ? unit0(t, v.frame_s0[t]) : 0;
+    v.frame_s0[t] = t < end ? unit_s[u] : sb + ks;
+    v.frame_a0[t] = t < end ? unit_a[u] : ab + ka;
   }
   tm.Sync();
   *s_top = sb + ks + ns_end;
@@ -1438,8 +1457,6 @@ int32_t MakePrunedLayout(const k2b200_pruned_args *a, char *ws, PrunedLayout *L)
   g.winner = reinterpret_cast<unsigned long long *>(ws + Take(&off, L->winner_bytes));
   g.frame_s0 = i32(n * ((size_t)T + 2));
   g.frame_a0 = i32(n * ((size_t)T + 2));
-  g.frame_n0 = i32(n * ((size_t)T + 2));
-  g.frame_m0 = i32(n * ((size_t)T + 2));
   g.warp_first = i32(n * kTeamWarps);
   g.seq_out = i32(kSeqOut * n);
   L->out_rs1 = i32(n + 1);
