@@ -53,6 +53,8 @@ def layered_lattice(rng, widths, degree, scale, hub=None):
     ([1, 70, 64, 65, 1], 5.0, 1.0, 33),              # four; a state over several lanes
     ([1, 30, 40, 50, 1], 12.0, 1.0, 300),            # eight; a state of more than 32 x 8 arcs
     ([1, 600, 700, 600, 1], 3.0, 60.0, None),        # values out of the shared exponent's range
+    ([1, 1023, 1024, 1000, 1], 2.0, 1.0, 700),       # the widest that eight warps slice
+    ([1, 1025, 1000, 1026, 1], 2.0, 1.0, 700),       # by four warps
     ([1, 500, 20000, 4097, 8, 1], 2.0, 1.0, None),   # wide: one to eight lanes per state
     ([1, 18000, 3, 18000, 1], 2.0, 1.0, 700),        # wide, with a state for the whole warp
 ])
