@@ -131,6 +131,16 @@ int32_t RowSplitsToRowIds(const int32_t *row_splits, int32_t num_rows,
                           int32_t *row_ids, int32_t num_elems,
                           cudaStream_t stream);
 
+// a + b of both halves in one instruction, each rounded as a single addition is.
+__device__ __forceinline__ float2 AddPair(float2 a, float2 b) {
+  float2 r;
+  asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+      "add.rn.f32x2 c, a, b;\n\tmov.b64 {%0, %1}, c;\n\t}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+
 // Host integers as a kernel parameter (at most 32764 bytes of them).
 template <int kInts>
 struct IntChunk {
