@@ -365,7 +365,7 @@ constexpr int kVitAhead = 3;  // rows requested ahead of the frame that uses the
 // comparison and a selection, constant slot offsets, and copies by the warps that hold a
 // column only took 500 frames of 4627 arcs from 246 to 215 us per round of CTAs (one CTA per
 // SM).  40 registers, for two CTAs per SM, leave no room to request a lane's eight scores
-// together: 256 CTAs took 460 us, and 431 with up to 80.
+// together: 256 CTAs took 460 us, and 431 with up to 80 (421 with the additions in pairs).
 template <int kDeg, int kPitch, int kThreads>
 __global__ void __launch_bounds__(kThreads, 1)
 LanesViterbi(const FsaInfo *__restrict__ infos, int32_t n, const Arc *__restrict__ arcs,
@@ -471,14 +471,11 @@ LanesViterbi(const FsaInfo *__restrict__ infos, int32_t n, const Arc *__restrict
         float best = -INFINITY, best1 = -INFINITY;
 #pragma unroll
         for (int j = 0; j < kDeg; j += 2) {
-          float x = __fadd_rn(at(cur, other[j]), w[j]);
-          float y = __fadd_rn(at(cur, other[j + 1]), w[j + 1]);
-          if (!kHoist) {
-            x = __fadd_rn(x, at(row, col[j]));
-            y = __fadd_rn(y, at(row, col[j + 1]));
-          }
-          best = fmaxf(best, x);
-          best1 = fmaxf(best1, y);
+          float2 x = AddPair(make_float2(at(cur, other[j]), at(cur, other[j + 1])),
+                             make_float2(w[j], w[j + 1]));
+          if (!kHoist) x = AddPair(x, make_float2(at(row, col[j]), at(row, col[j + 1])));
+          best = fmaxf(best, x.x);
+          best1 = fmaxf(best1, x.y);
         }
         best = fmaxf(best, best1);
 #pragma unroll
