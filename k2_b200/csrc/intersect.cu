@@ -90,11 +90,16 @@ int32_t MakeLayout(const k2b200_intersect_args *a, Layout *L) {
   L->total_levels = levels;
   // CountKept / EmitLattice run on a (word tiles of the largest pair, pairs) grid.  With many
   // words, most of them empty, a warp takes 16; with few it takes one, so that all SMs have
-  // warps to run (about 64 per SM until every warp has one word).
+  // warps to run (about 64 per SM until every warp has one word).  Words of graphs with many
+  // arcs per state differ in what they cost, by up to the hundreds of arcs of one: shorter runs
+  // of them even out (5 words -> 1 of an LF-MMI denominator, 16 x 300 frames: CountKept 110 ->
+  // 99 us, EmitLattice 174 -> 139; the sparse words of alignment graphs lost by it, 22 -> 35
+  // and 21 -> 29).
   int64_t max_pair_words = 0;
   for (const FsaInfo &f : L->infos)
     max_pair_words = std::max<int64_t>(max_pair_words, (int64_t)(f.tk + 1) * f.words);
-  L->words_per_warp = (int32_t)std::max<int64_t>(1, std::min<int64_t>(16, words / (148 * 64)));
+  const int64_t runs = (int64_t)148 * 64 * (a->num_arcs / 8 >= a->num_states ? 5 : 1);
+  L->words_per_warp = (int32_t)std::max<int64_t>(1, std::min<int64_t>(16, words / runs));
   L->tiles_per_pair = CeilDiv(max_pair_words, (int64_t)L->words_per_warp * (kCountThreads / 32));
   L->count_blocks = (int32_t)std::min<int64_t>((int64_t)L->tiles_per_pair * a->num_fsas,
                                                0x7fffffff);
