@@ -1490,6 +1490,9 @@ struct GradSpec {
   }
 };
 
+// A CTA sees to the `width` columns of the gradient from blockIdx.z * width on, as many as a row
+// of sums per warp leaves room for (one range up to 12 800 columns, 8 640 with the arcs of graphs
+// of 1024 states); the arcs' posteriors go with the first range.
 template <bool kArcs>
 __global__ void __launch_bounds__(128)
 BandGrad(const BandInfo *__restrict__ infos, const BandArc *__restrict__ tabf,
@@ -1501,7 +1504,7 @@ BandGrad(const BandInfo *__restrict__ infos, const BandArc *__restrict__ tabf,
          const int32_t *__restrict__ unfit, const GradSpec upstream,
          float *__restrict__ grad_a, float *__restrict__ grad_b,
          const int32_t *__restrict__ grad_row0, int32_t grad_pitch, int32_t grad_col_off,
-         int32_t C, int32_t st_pad) {
+         int32_t C, int32_t width, int32_t st_pad) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int32_t i = blockIdx.y;
   const BandInfo f = infos[i];
@@ -1525,8 +1528,10 @@ BandGrad(const BandInfo *__restrict__ infos, const BandArc *__restrict__ tabf,
   const float *lp0 = lp + (int64_t)f.lp_row * C;
   // this warp's row of sums, one per column of the gradient (all zero between levels)
   // (without a gradient for the dense scores only the arcs are wanted)
-  const int32_t cols = grad_b != nullptr ? C + grad_col_off : 0;
-  uint32_t *sums = reinterpret_cast<uint32_t *>(smem_raw) + (size_t)warp * cols;
+  const int32_t col0 = blockIdx.z * width;
+  const int32_t cols = grad_b != nullptr ? min(width, C + grad_col_off - col0) : 0;
+  const bool arcs = kArcs && blockIdx.z == 0;
+  uint32_t *sums = reinterpret_cast<uint32_t *>(smem_raw) + (size_t)warp * width;
   for (int32_t k = lane; k < cols; k += 32) sums[k] = 0u;
   __syncwarp();
   ProbState *prev = nullptr;  // alpha of the level before, state s at s + 2
@@ -1541,8 +1546,9 @@ BandGrad(const BandInfo *__restrict__ infos, const BandArc *__restrict__ tabf,
       prev[items0[row + j].s] = q;
     }
   };
-  if (kArcs) {
-    prev = reinterpret_cast<ProbState *>(smem_raw + (((size_t)4 * cols * sizeof(uint32_t) + 15) & ~(size_t)15)) +
+  if (arcs) {
+    prev = reinterpret_cast<ProbState *>(
+               smem_raw + (((size_t)4 * width * sizeof(uint32_t) + 15) & ~(size_t)15)) +
            (size_t)warp * st_pad + 2;
     stage_alpha(a - 1);
     __syncwarp();
@@ -1580,12 +1586,12 @@ BandGrad(const BandInfo *__restrict__ infos, const BandArc *__restrict__ tabf,
         const double alm = j0 == 0 ? al4[u] : am0[row + j], bem = j0 == 0 ? be4[u] : bm0[row + j];
         if (alm != 0.0 && bem != 0.0) {
           const int32_t ale = exact ? ae0[row + j] : ea_l, bee = exact ? be0[row + j] : eb_l;
-          const int32_t col = it.label + grad_col_off;
-          if (grad_b != nullptr && it.label != kNoLabel && it.label < C && col >= 0) {
+          const int32_t col = it.label + grad_col_off - col0;  // of this range
+          if (it.label != kNoLabel && it.label < C && col >= 0 && col < cols) {
             g = (float)(alm * bem * zinv * Pow2Clamp(ale + bee - z.e));
             key = col;
           }
-          if (kArcs) {
+          if (arcs) {
             const int32_t s = it.s;
             double pm;
             int32_t pe;
@@ -1614,12 +1620,12 @@ BandGrad(const BandInfo *__restrict__ infos, const BandArc *__restrict__ tabf,
       if (key >= 0) {
         const uint32_t fixed = atomicExch(&sums[key], 0u);
         if (fixed != 0u)
-          atomicAdd(grad_b + (row0 + l - 1) * grad_pitch + key,
+          atomicAdd(grad_b + (row0 + l - 1) * grad_pitch + col0 + key,
                     (float)tg * ((float)fixed * (1.0f / 2147483648.0f)));
       }
       __syncwarp();
     }
-    if (kArcs) {
+    if (arcs) {
       __syncwarp();  // the level before has been read
       stage_alpha(l);
       __syncwarp();
@@ -1632,10 +1638,16 @@ BandGrad(const BandInfo *__restrict__ infos, const BandArc *__restrict__ tabf,
 // every element of the rows of a sequence and of the rows up to the next one is stored
 // once, so the caller's buffer needs no clearing (at 128 MB of log-probs the clear and the
 // scattered additions took 29 + 26 us of memory time, this takes 30).  A warp per kDenseRows
-// rows; the row's sums gather in shared memory in fixed point as in BandGrad.  kSoftmax: the
-// rows are log_softmax of the tensor the gradient is for, d = g - softmax * sum(g).
+// rows; the row's sums gather in shared memory in fixed point as in BandGrad.  A CTA sees to the
+// `width` columns from blockIdx.z * width on.  kSoftmax: the rows are log_softmax of the tensor
+// the gradient is for, d = g - softmax * sum(g).
 // ---------------------------------------------------------------------------
 constexpr int kDenseRows = 4;
+// Columns of a range.  A warp stores its range alone, so a wide one leaves an SM few warps: 60 000
+// columns x 2400 rows took 288 us (logits 4625) in ranges of 51 200, what fits in shared memory,
+// 139 (678) in ranges of 6400, 139 (320) in ranges of 1600; up to 6400 columns the gradient of
+// log-probs only loses by a second range (5000 x 16 000 rows: 109 us, halved 115).
+constexpr int kGradColumns = 6400;
 
 template <bool kSoftmax>
 __global__ void __launch_bounds__(128)
@@ -1645,7 +1657,7 @@ BandGradRows(const BandInfo *__restrict__ infos, const float *__restrict__ lp,
              const double *__restrict__ bm, const int32_t *__restrict__ be,
              const int32_t *__restrict__ a_scale, const int32_t *__restrict__ b_scale,
              const BandTotal *__restrict__ total, const int32_t *__restrict__ unfit,
-             const GradSpec upstream, float *__restrict__ grad, int32_t C, int32_t C_pad) {
+             const GradSpec upstream, float *__restrict__ grad, int32_t C, int32_t width) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr unsigned kAll = 0xffffffffu;
   const int32_t i = blockIdx.y;
@@ -1655,8 +1667,9 @@ BandGradRows(const BandInfo *__restrict__ infos, const float *__restrict__ lp,
   const int32_t r0 = (blockIdx.x * (blockDim.x >> 5) + warp) * kDenseRows;
   if (r0 >= rows) return;
   const int32_t r1 = min(r0 + kDenseRows, rows);
-  uint32_t *sums = reinterpret_cast<uint32_t *>(smem_raw) + (size_t)warp * C_pad;
-  for (int32_t k = lane; k < C_pad; k += 32) sums[k] = 0u;
+  const int32_t col0 = blockIdx.z * width, cols = min(width, C - col0);
+  uint32_t *sums = reinterpret_cast<uint32_t *>(smem_raw) + (size_t)warp * width;
+  for (int32_t k = lane; k < width; k += 32) sums[k] = 0u;
   const BandTotal z = total[i];
   const bool dead = z.m == 0.0 || f.num_states == 0;  // no path survives: all zero
   const double zinv = dead ? 0.0 : 1.0 / z.m;
@@ -1704,18 +1717,19 @@ BandGradRows(const BandInfo *__restrict__ infos, const float *__restrict__ lp,
         const float g = (float)(alm * bem * zinv * Pow2Clamp(ale + bee - z.e));
         const uint32_t fixed = __float2uint_rn(g * 2147483648.0f);
         added += fixed;
-        atomicAdd(&sums[it.label], fixed);
+        const uint32_t col = (uint32_t)(it.label - col0);
+        if (col < (uint32_t)cols) atomicAdd(&sums[col], fixed);
       }
     }
     __syncwarp();
-    float *out = grad + (int64_t)(f.lp_row + r) * C;
-    const bool vec = (C & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+    float *out = grad + (int64_t)(f.lp_row + r) * C + col0;
+    const bool vec = (cols & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
     if (n == 0) {
       if (vec) {
-        for (int32_t c = lane * 4; c < C; c += 128)
+        for (int32_t c = lane * 4; c < cols; c += 128)
           *reinterpret_cast<float4 *>(out + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       } else {
-        for (int32_t c = lane; c < C; c += 32) out[c] = 0.0f;
+        for (int32_t c = lane; c < cols; c += 32) out[c] = 0.0f;
       }
       continue;
     }
@@ -1724,7 +1738,7 @@ BandGradRows(const BandInfo *__restrict__ infos, const float *__restrict__ lp,
     if (!kSoftmax) {
       if (vec) {
 #pragma unroll 4
-        for (int32_t c = lane * 4; c < C; c += 128) {
+        for (int32_t c = lane * 4; c < cols; c += 128) {
           const uint4 x = *reinterpret_cast<const uint4 *>(sums + c);
           if (x.x | x.y | x.z | x.w) *reinterpret_cast<uint4 *>(sums + c) = make_uint4(0, 0, 0, 0);
           *reinterpret_cast<float4 *>(out + c) =
@@ -1732,7 +1746,7 @@ BandGradRows(const BandInfo *__restrict__ infos, const float *__restrict__ lp,
         }
       } else {
 #pragma unroll 4
-        for (int32_t c = lane; c < C; c += 32) {
+        for (int32_t c = lane; c < cols; c += 32) {
           const uint32_t x = sums[c];
           if (x) sums[c] = 0u;
           out[c] = value(x);
@@ -1741,9 +1755,9 @@ BandGradRows(const BandInfo *__restrict__ infos, const float *__restrict__ lp,
     } else {
       // (the sum of a row's posteriors is at most 1, its fixed-point value fits 32 bits)
       const float total_g = value(__reduce_add_sync(kAll, added));
-      const float *x = lp + (int64_t)(f.lp_row + r) * C;
+      const float *x = lp + (int64_t)(f.lp_row + r) * C + col0;
 #pragma unroll 4
-      for (int32_t c = lane; c < C; c += 32) {
+      for (int32_t c = lane; c < cols; c += 32) {
         const uint32_t y = sums[c];
         if (y) sums[c] = 0u;
         out[c] = value(y) - expf(__ldg(x + c)) * total_g;
@@ -2239,17 +2253,24 @@ int32_t k2b200_band_loss_forward_reduce(const k2b200_band_loss_args *args, void 
   return kOk;
 }
 
+// Columns that a CTA of a gradient kernel sees to: all of them where `most` allows, else equal
+// ranges; a multiple of four.
+static int32_t ColumnRange(int32_t cols, size_t most) {
+  const int32_t ranges = std::max(1, CeilDiv(cols, (int64_t)(most & ~(size_t)3)));
+  return (CeilDiv(cols, ranges) + 3) & ~3;
+}
+
 static int32_t BandArcsOrScatter(const BandLayout &L, const k2b200_band_loss_args *args, char *ws,
                                  const GradSpec &upstream, float *grad_a, float *grad_b,
                                  const int32_t *grad_row0, int32_t grad_pitch,
                                  int32_t grad_col_off, cudaStream_t stream) {
-  dim3 grid(CeilDiv(L.max_frames + 1, 4 * kGradLevels), args->num_fsas);
-  const size_t sums_bytes =
-      grad_b == nullptr
-          ? 0
-          : (sizeof(uint32_t) * 4 * (size_t)(args->num_classes + grad_col_off) + 15) & ~(size_t)15;
-  const size_t smem = sums_bytes + (grad_a ? sizeof(ProbState) * 4 * (size_t)L.st_pad : 0);
-  K2B_REQUIRE(smem <= kBandSmemBudget, "too many classes for the gradient kernel");
+  // columns in ranges that four rows of sums have room for beside the states of the arcs
+  const size_t arc_bytes = grad_a ? sizeof(ProbState) * 4 * (size_t)L.st_pad : 0;
+  const int32_t cols = grad_b == nullptr ? 0 : args->num_classes + grad_col_off;
+  const int32_t width = ColumnRange(cols, (kBandSmemBudget - arc_bytes) / (4 * sizeof(uint32_t)));
+  const size_t smem = sizeof(uint32_t) * 4 * (size_t)width + arc_bytes;
+  dim3 grid(CeilDiv(L.max_frames + 1, 4 * kGradLevels), args->num_fsas,
+            cols > 0 ? CeilDiv(cols, width) : 1);
   auto kernel = grad_a != nullptr ? BandGrad<true> : BandGrad<false>;
   K2B_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)kBandSmemBudget));
@@ -2266,7 +2287,7 @@ static int32_t BandArcsOrScatter(const BandLayout &L, const k2b200_band_loss_arg
       reinterpret_cast<const int32_t *>(ws + L.off_b_scale),
       reinterpret_cast<const BandTotal *>(ws + L.off_total),
       reinterpret_cast<const int32_t *>(ws + L.off_unfit), upstream, grad_a, grad_b, grad_row0,
-      grad_pitch, grad_col_off, args->num_classes, L.st_pad); NoteLaunch(); }
+      grad_pitch, grad_col_off, args->num_classes, width, L.st_pad); NoteLaunch(); }
   K2B_CUDA_OK(cudaGetLastError());
   return kOk;
 }
@@ -2316,18 +2337,19 @@ int32_t k2b200_band_loss_backward_dense(const k2b200_band_loss_args *args, void 
                          upstream->negate,    upstream->lens_type, upstream->lens,
                          args->num_fsas};
   if (grad_log_probs != nullptr) {
-    const int32_t C = args->num_classes, C_pad = (C + 3) & ~3;
+    const int32_t C = args->num_classes;
+    const int32_t width = ColumnRange(C, kGradColumns);
     if (L.first_row > 0)  // rows before the first sequence
       K2B_CUDA_OK(cudaMemsetAsync(grad_log_probs, 0, sizeof(float) * (size_t)L.first_row * C, stream));
-    const size_t row_bytes = sizeof(uint32_t) * (size_t)C_pad;
-    K2B_REQUIRE(row_bytes <= kBandSmemBudget, "too many classes for the gradient kernel");
+    const size_t row_bytes = sizeof(uint32_t) * (size_t)width;
     // a row of sums per warp in shared memory: fewer warps per CTA when rows are long, so
     // that a CTA does not hold the SM's memory for one slow warp
     const int32_t warps = row_bytes * 4 <= 16 * 1024 ? 4 : row_bytes <= 8 * 1024 ? 2 : 1;
     auto kernel = softmax ? BandGradRows<true> : BandGradRows<false>;
     K2B_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)kBandSmemBudget));
-    dim3 grid(CeilDiv(std::max(L.max_rows, 1), warps * kDenseRows), args->num_fsas);
+    dim3 grid(CeilDiv(std::max(L.max_rows, 1), warps * kDenseRows), args->num_fsas,
+              CeilDiv(C, width));
     { kernel<<<grid, 32 * warps, row_bytes * warps, stream>>>(
         reinterpret_cast<const BandInfo *>(ws + L.off_infos), args->log_probs,
         reinterpret_cast<const BandItem *>(ws + L.off_items),
@@ -2339,7 +2361,7 @@ int32_t k2b200_band_loss_backward_dense(const k2b200_band_loss_args *args, void 
         reinterpret_cast<const int32_t *>(ws + L.off_a_scale),
         reinterpret_cast<const int32_t *>(ws + L.off_b_scale),
         reinterpret_cast<const BandTotal *>(ws + L.off_total),
-        reinterpret_cast<const int32_t *>(ws + L.off_unfit), spec, grad_log_probs, C, C_pad);
+        reinterpret_cast<const int32_t *>(ws + L.off_unfit), spec, grad_log_probs, C, width);
       NoteLaunch(); }
     K2B_CUDA_OK(cudaGetLastError());
   }

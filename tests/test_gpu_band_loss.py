@@ -454,3 +454,61 @@ def test_a_wait_that_gives_up_is_reported_and_the_general_kernels_take_over():
     # and with the limit restored the band kernels serve the same call
     tot3, _, _ = run(a, lp, seg, 10.0)
     assert close(tot3, want["tot_scores"], rtol=1e-6, atol=1e-6)
+
+
+@pytest.mark.parametrize("classes,amap,layout", [
+    (12736, [0, 0, 1], "log_probs"),    # sequences that share rows: the most columns of one
+    (12737, [0, 0, 1], "log_probs"),    # range beside the states of the arcs, and two ranges
+    (12799, None, "scores"),            # the score matrix: 12 800 columns, one range without arcs
+    (13001, None, "scores"),
+    (6400, None, "log_probs"),          # rows of their own: the most columns of one range
+    (6401, None, "logits"),
+    (51203, None, "log_probs"),
+    (60004, None, "logits"),
+    (110001, None, "log_probs"),
+])
+def test_wide_vocabularies(classes, amap, layout):
+    """More columns than a row of sums in shared memory has room for.  Gradients within 4e-5: the
+    lattice rounds arc score + dense score (at most 16 in size: 4.8e-7) on each of 12 frames of
+    every path, which moves a posterior by at most twice 12 x 4.8e-7, times the largest upstream
+    gradient of 2.8."""
+    import k2_b200 as k2
+    from gpu_util import host_to_fsa
+    rng = np.random.default_rng(classes)
+    n = 2 if amap is None else len(amap)
+    a = random_band_graphs(rng, n, 10, classes)
+    lp, seg = random_log_probs(rng, 2, 12, classes)
+    scores, brs = host_scores(lp, seg)
+    tot_grad = rng.normal(size=n)
+    want = oracle.loss_path(a, scores, brs, 100.0, amap, tot_grad=tot_grad)
+    want_gb = to_lp_layout(want["grad_b"], tuple(lp.shape), seg)
+    for graph_grad in (True, False):
+        fsa = host_to_fsa(a)
+        fsa.scores.requires_grad_(graph_grad)
+        leaf = lp.to(DEV)
+        if layout == "logits":
+            leaf = leaf + 3.0
+            dense = k2.DenseFsaVec.from_logits(leaf.requires_grad_(True), seg)
+        elif layout == "scores":
+            dense = k2.DenseFsaVec(leaf, seg)
+            leaf = dense.scores.requires_grad_(True)
+        else:
+            dense = k2.DenseFsaVec(leaf.requires_grad_(True), seg)
+        m = None if amap is None else torch.as_tensor(amap, dtype=torch.int32)
+        tot = k2.intersect_dense_tot_scores(fsa, dense, 100.0, a_to_b_map=m)
+        assert type(tot.grad_fn).__name__.startswith("_BandTotScores"), tot.grad_fn
+        live = torch.isfinite(tot)
+        assert live.any()
+        (tot * torch.as_tensor(tot_grad, device=DEV))[live].sum().backward()
+        assert close(tot.detach().cpu().numpy(), want["tot_scores"], rtol=1e-6, atol=1e-6)
+        gb = leaf.grad.cpu().numpy()
+        if layout == "scores":
+            assert np.abs(gb - want["grad_b"]).max() <= 4e-5
+        elif layout == "logits":
+            p = np.exp(lp.numpy().astype(np.float64))
+            ref = want_gb - p * want_gb.sum(-1, dtype=np.float64, keepdims=True)
+            assert np.abs(gb - ref).max() <= 4e-5
+        else:
+            assert np.abs(gb - want_gb).max() <= 4e-5
+        if graph_grad:
+            assert np.abs(fsa.scores.grad.cpu().numpy() - want["grad_a"]).max() <= 1e-4
