@@ -212,7 +212,8 @@ struct ChainPlan {
 
 static ChainPlan PlanChain(const k2b200_fsa_view *v, int32_t ndir) {
   ChainPlan p = {};
-  if (!v->strict_layers || v->max_layer_states <= 0 || v->max_layer_arcs < 0 || v->max_layers <= 0)
+  if (!v->strict_layers || v->max_layer_states <= 0 || v->max_layer_arcs < 0 ||
+      v->max_layers <= 0 || (int64_t)v->num_fsas * v->max_layers > INT32_MAX)
     return p;
   p.maxw = (v->max_layer_states + 3) & ~3;
   p.nl_cap = v->max_layers;
@@ -270,7 +271,7 @@ static ChainPlan PlanChain(const k2b200_fsa_view *v, int32_t ndir) {
 // ---------------------------------------------------------------------------
 constexpr uint32_t kNoState = 0xffffu, kLaneHead = 1u << 19;
 struct SliceDesc {
-  int32_t at;      // of the region, in units of 16 bytes
+  uint32_t at;     // of the region, in units of 16 bytes
   int32_t size;    // likewise
   int32_t blocks;  // of K rows; -1: the pool was full, the arcs are read where they are
   int32_t tall;
@@ -281,11 +282,13 @@ __device__ __forceinline__ int32_t SliceRowsAt(int32_t blocks, int32_t tall) {
 }
 
 // Units of 16 bytes the pool needs: records for uneven lanes, two part-filled blocks per
-// layer, lane words.  (A layer that finds the pool full is read the slow way.)
-static int64_t SlicePoolUnits(const k2b200_fsa_view *v, const ChainPlan &p) {
-  const int64_t layers = (int64_t)v->num_fsas * v->max_layers, k = p.rows;
-  return v->num_arcs + v->num_arcs / 2 + (int64_t)v->num_states * (p.rows < 8 ? k - 1 : k / 2) +
-         layers * (40 * k + 16) + 1024;
+// layer, lane words.  (A layer that finds the pool full is read the slow way; 2^32 - 1 units, what
+// a SliceDesc can name, hold both directions of a lattice of 10^9 arcs.)
+static int64_t SlicePoolUnits(const k2b200_fsa_view *v, const ChainPlan &p, int32_t ndir) {
+  const int64_t layers = (int64_t)v->num_fsas * v->max_layers, arcs = v->num_arcs, k = p.rows;
+  const int64_t units = arcs + arcs / 2 + (int64_t)v->num_states * (p.rows < 8 ? k - 1 : k / 2) +
+                        layers * (40 * k + 16) + 1024;
+  return std::min<int64_t>(units * ndir, UINT32_MAX);
 }
 
 // Layer `lv` of direction blockIdx.y + dir_base per team of kWarps warps (kWarps == 1: four
@@ -401,20 +404,19 @@ SliceLayers(k2b200_fsa_view v, int32_t dir_base, int32_t K, int32_t maxw, int32_
     head[14] = blocks * 32;  // ... of the tall states
     head[17] = blocks * K;   // ... and their first row
     const unsigned long long at = atomicAdd(pool_used, (unsigned long long)units);
-    SliceDesc d = {(int32_t)at, units, blocks, tall};
+    SliceDesc d = {(uint32_t)at, units, blocks, tall};
     // (a tall block's word has 12 bits for its rows, 20 for the first of them)
     if (at + units > (unsigned long long)pool_units || head[16] >= 4096 ||
         blocks * K + head[16] >= (1 << 20)) {
-      d.at = d.size = d.tall = 0;
-      d.blocks = -1;
+      d = SliceDesc{0, 0, -1, 0};
     }
     *desc = d;
     head[20] = d.blocks;
-    head[21] = d.at;
+    head[21] = (int32_t)d.at;
   }
   sync();
   if (head[20] < 0) return;
-  uint4 *const final_region = pool + head[21];
+  uint4 *const final_region = pool + (uint32_t)head[21];
   const bool staged = units <= buf_units;
   uint4 *region = staged ? buf : final_region;
   uint32_t *words = reinterpret_cast<uint32_t *>(region);
@@ -1174,8 +1176,8 @@ ChainScratch CarveScratch(const k2b200_fsa_view *v, const ChainPlan &p, int32_t 
   if (p.wide) {
     c.fwd_arcs = reinterpret_cast<LayerArc *>(take(sizeof(LayerArc) * na));
     c.bwd_arcs = reinterpret_cast<LayerArc *>(take(sizeof(LayerArc) * na));
-  } else {
-    c.pool_units = SlicePoolUnits(v, p) * ndir;
+  } else if (p.ok) {
+    c.pool_units = SlicePoolUnits(v, p, ndir);
     c.pool = reinterpret_cast<uint4 *>(take(sizeof(uint4) * (size_t)c.pool_units));
     c.descs = reinterpret_cast<SliceDesc *>(take(sizeof(SliceDesc) * 2 * layers));
   }
@@ -1208,7 +1210,7 @@ static int32_t LaunchChain(const k2b200_fsa_view *v, const ChainScratch &c, cons
     const int32_t warps = one ? 1 : p.maxw <= 1024 ? 8 : 4;
     const size_t fixed = sizeof(int32_t) * ((warps + 1) * (size_t)p.maxw + 32);
     // room for a layer well above the mean, with several CTAs per SM
-    const int64_t mean = (SlicePoolUnits(v, p) - 1024) / std::max(layers, 1);
+    const int64_t mean = (SlicePoolUnits(v, p, 1) - 1024) / std::max(layers, 1);
     int32_t buf = (int32_t)std::min<int64_t>(2 * mean, one ? 512 : 3072);
     if (!one) buf = (int32_t)std::min<int64_t>(buf, (int64_t)(kLayerSmemBudget - fixed) / 16);
     const size_t smem = (one ? 4 : 1) * (fixed + 16 * (size_t)buf);

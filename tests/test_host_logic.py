@@ -287,3 +287,32 @@ def test_splits_of_the_device_ctc_graphs_match_the_host_builder():
             assert np.array_equal(sym_off[1:], np.cumsum(lens))
             assert np.array_equal(rs1, want_rs1), symbols
             assert np.array_equal(arc_splits, arcs._row_splits2.numpy()[want_rs1]), symbols
+
+
+def test_scratch_of_layer_scores():
+    """The scratch of the layer kernels for sizes that no test allocates."""
+    from k2_b200 import _lib
+
+    def plan(**kw):
+        view = _lib.FsaView(**kw)
+        incoming = ctypes.c_int32()
+        nbytes = [_lib.lib.k2b200_fsa_scores_dir_scratch_bytes(ctypes.byref(view), d,
+                                                               ctypes.byref(incoming))
+                  for d in (1, 2)]
+        return nbytes + [incoming.value]
+
+    # 10^9 arcs: what a slice's descriptor can name is 2^32 - 1 units of 16 bytes, of which both
+    # directions need three quarters
+    layers = dict(strict_layers=1, max_layers=15000, max_layer_states=1000, max_layer_arcs=2000)
+    one, two, incoming = plan(num_fsas=64, num_states=15000000, num_arcs=1 << 30, **layers)
+    assert 16 * (1 << 30) < one < two < 16 * (1 << 32) and not incoming
+    # more than that: the layers that the pool has no room for are read where they are
+    one, two, incoming = plan(num_fsas=64, num_states=15000000, num_arcs=(1 << 31) - 1, **layers)
+    extra = 24 * 2 * 64 * 15000 + 24 * 15000000 + (1 << 20)
+    assert two <= 16 * ((1 << 32) - 1) + extra and not incoming
+    # a number of layers that 32 bits cannot hold, and an FsaVec without strict layers: the general
+    # kernels, which need no scratch to speak of
+    for kw in (dict(layers, max_layers=1 << 20, num_fsas=1 << 12),
+               dict(num_fsas=3, strict_layers=0)):
+        one, two, incoming = plan(num_states=5000, num_arcs=10, **kw)
+        assert incoming and max(one, two) < 1 << 40
