@@ -377,6 +377,8 @@ py::object BandLoss(const std::shared_ptr<BandGraph> &graph, const at::Tensor &s
   if (!input.is_cuda() || input.scalar_type() != at::kFloat || input.dim() != 3 ||
       !input.is_contiguous() || graph->states.device() != input.device())
     return py::none();
+  // forward-mode derivatives are refused, which the Python autograd functions do
+  if (input._fw_grad(0).defined() || scores_a._fw_grad(0).defined()) return py::none();
   const int32_t n = (int32_t)graph->h_row_splits1.size() - 1, seqs = (int32_t)first.size();
   BandCall call;
   call.graph = graph;

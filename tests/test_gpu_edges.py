@@ -207,3 +207,29 @@ def test_incoming_arcs_of_band_graphs(k2, lengths):
         want._band_graph = None  # the general index
         for got, ref in zip(arcs.incoming(), want.incoming()):
             assert torch.equal(got, ref), (lengths, modified)
+
+
+# --------------------------------------------------------------------------- the loss as a node
+def small_loss(k2, leaf, logits, reduction="sum", lens=None):
+    seg = torch.tensor([[0, 0, 30], [1, 2, 20], [2, 0, 15]], dtype=torch.int32)
+    graphs = k2.ctc_graph([[1, 2, 3, 3], [5, 6], [16]], device=DEV)
+    make = k2.DenseFsaVec.from_logits if logits else k2.DenseFsaVec
+    return k2.ctc_loss(graphs, make(leaf, seg), reduction=reduction, target_lengths=lens)
+
+
+def small_input(logits):
+    x = torch.from_numpy(np.random.default_rng(5).normal(size=(3, 30, 17)).astype(np.float32))
+    return (x if logits else torch.log_softmax(x, -1)).to(DEV)
+
+
+@pytest.mark.parametrize("logits", [False, True])
+def test_forward_mode_is_refused(k2, logits):
+    from torch.autograd import forward_ad
+    x = small_input(logits)
+    with forward_ad.dual_level():
+        with pytest.raises(NotImplementedError, match="jvp"):
+            small_loss(k2, forward_ad.make_dual(x, torch.ones_like(x)), logits)
+    for transform in (torch.func.grad, torch.func.vmap):
+        with pytest.raises(RuntimeError):
+            transform(lambda y: small_loss(k2, y, logits))(x if transform is torch.func.grad
+                                                           else x[None])
