@@ -405,7 +405,9 @@ py::object BandLoss(const std::shared_ptr<BandGraph> &graph, const at::Tensor &s
   if (mode == kMean) {
     if (!lens.has_value() || !lens->is_cuda() || lens->device() != input.device() ||
         lens->dim() != 1 || lens->numel() != n || !lens->is_contiguous() ||
-        (lens_type = LensType(*lens)) == 0)
+        (lens_type = LensType(*lens)) == 0 ||
+        // (no derivative with respect to the lengths here)
+        torch::autograd::compute_requires_grad(*lens) || lens->_fw_grad(0).defined())
       return py::none();
   }
   // the gradient of the arc scores does not know of the penalty

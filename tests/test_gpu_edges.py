@@ -233,3 +233,14 @@ def test_forward_mode_is_refused(k2, logits):
         with pytest.raises(RuntimeError):
             transform(lambda y: small_loss(k2, y, logits))(x if transform is torch.func.grad
                                                            else x[None])
+
+
+@pytest.mark.parametrize("logits", [False, True])
+def test_gradient_of_the_target_lengths(k2, logits):
+    """mean(-tot / length): the lengths may want a gradient, too."""
+    x = small_input(logits)
+    lens = torch.tensor([4.0, 2.0, 1.0], device=DEV, requires_grad=True)
+    small_loss(k2, x.clone().requires_grad_(True), logits, "mean", lens).backward()
+    each = small_loss(k2, x, logits, "none")
+    want = (-each / (3 * lens.detach() ** 2)).cpu()
+    assert torch.allclose(lens.grad.cpu(), want, rtol=1e-6)
