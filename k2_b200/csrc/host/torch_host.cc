@@ -11,6 +11,7 @@
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_cpp_function.h>
+#include <torch/csrc/autograd/saved_variable.h>
 #include <pybind11/numpy.h>
 #include <torch/extension.h>
 
@@ -293,7 +294,7 @@ struct BandCall {
 
 struct BandLossNode : public torch::autograd::Node {
   BandCall call;
-  at::Tensor lens;
+  torch::autograd::SavedVariable saved_lens;  // complains if they were changed in the meantime
   std::vector<int64_t> input_sizes;
   int64_t num_arcs = 0;
   int32_t mode = kTotals, lens_type = 0;
@@ -316,6 +317,7 @@ struct BandLossNode : public torch::autograd::Node {
     up.stride = mode == kTotals && g.numel() > 0 ? (int32_t)g.stride(0) : 0;
     up.negate = mode != kTotals;
     up.lens_type = lens_type;
+    const at::Tensor lens = lens_type ? saved_lens.unpack() : at::Tensor();
     up.lens = lens_type ? lens.data_ptr() : nullptr;
     if (task_should_compute_output(0)) out[0] = at::empty(input_sizes, On(at::kFloat, device));
     if (task_should_compute_output(1)) out[1] = at::zeros({num_arcs}, On(at::kFloat, device));
@@ -326,7 +328,10 @@ struct BandLossNode : public torch::autograd::Node {
         c10::cuda::getCurrentCUDAStream(device.index()).stream()));
     return out;
   }
-  void release_variables() override { call.workspace.reset(); }
+  void release_variables() override {
+    call.workspace.reset();
+    saved_lens.reset_data();
+  }
 };
 
 // One class per mode, so that `grad_fn` of a result says in Python what it is.
@@ -481,7 +486,7 @@ py::object BandLoss(const std::shared_ptr<BandGraph> &graph, const at::Tensor &s
     node->num_arcs = scores_a.size(0);
     node->mode = mode;
     node->lens_type = lens_type;
-    if (lens_type) node->lens = *lens;
+    if (lens_type) node->saved_lens = torch::autograd::SavedVariable(*lens, false);
     node->logits = logits;
     node->call = std::move(call);
     // the argument block points into the vectors, which have moved

@@ -244,3 +244,26 @@ def test_gradient_of_the_target_lengths(k2, logits):
     each = small_loss(k2, x, logits, "none")
     want = (-each / (3 * lens.detach() ** 2)).cpu()
     assert torch.allclose(lens.grad.cpu(), want, rtol=1e-6)
+
+
+@pytest.mark.parametrize("logits", [False, True])
+def test_when_the_loss_can_be_differentiated(k2, logits):
+    """Twice with retain_graph and the same bits both times, else once; not when the target lengths
+    changed in between."""
+    x = small_input(logits)
+    for reduction in ("sum", "mean"):
+        leaf = x.clone().requires_grad_(True)
+        lens = torch.tensor([4, 2, 1], device=DEV)
+        loss = small_loss(k2, leaf, logits, reduction, lens)
+        first, = torch.autograd.grad(loss, leaf, retain_graph=True)
+        again, = torch.autograd.grad(loss, leaf, retain_graph=True)
+        assert torch.equal(first, again) and first.abs().max() > 0
+        if reduction == "mean":
+            lens.mul_(2)
+            with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+                torch.autograd.grad(loss, leaf, retain_graph=True)
+            loss = small_loss(k2, leaf, logits, reduction, lens)
+        loss.backward()
+        assert torch.equal(leaf.grad, first if reduction == "sum" else first / 2)
+        with pytest.raises(RuntimeError, match="retain_graph"):
+            loss.backward()
