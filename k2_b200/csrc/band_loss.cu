@@ -1724,7 +1724,7 @@ BandGradRows(const BandInfo *__restrict__ infos, const float *__restrict__ lp,
     __syncwarp();
     float *out = grad + (int64_t)(f.lp_row + r) * C + col0;
     const bool vec = (cols & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
-    if (n == 0) {
+    if (n == 0 && !(kSoftmax && r < T)) {
       if (vec) {
         for (int32_t c = lane * 4; c < cols; c += 128)
           *reinterpret_cast<float4 *>(out + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -1733,8 +1733,12 @@ BandGradRows(const BandInfo *__restrict__ infos, const float *__restrict__ lp,
       }
       continue;
     }
+    // (columns without a posterior are 0 whatever the upstream gradient, infinities and NaN too;
+    // rows whose softmax is NaN give NaN even if no path survives)
     const float tgf = (float)tg;
-    auto value = [&](uint32_t fixed) { return tgf * ((float)fixed * (1.0f / 2147483648.0f)); };
+    auto value = [&](uint32_t fixed) {
+      return fixed ? tgf * ((float)fixed * (1.0f / 2147483648.0f)) : 0.0f;
+    };
     if (!kSoftmax) {
       if (vec) {
 #pragma unroll 4

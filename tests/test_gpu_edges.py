@@ -267,3 +267,28 @@ def test_when_the_loss_can_be_differentiated(k2, logits):
         assert torch.equal(leaf.grad, first if reduction == "sum" else first / 2)
         with pytest.raises(RuntimeError, match="retain_graph"):
             loss.backward()
+
+
+@pytest.mark.parametrize("upstream", [1.0, -2.0, 0.0, float("inf"), float("nan")])
+def test_gradients_that_are_not_finite(k2, upstream):
+    """Against the lattice: an upstream gradient of infinity or NaN (a target length of 0 makes one)
+    reaches the elements that some path uses, no others; log-probs of NaN have a gradient of NaN
+    through the softmax, on every row of an utterance without a path too."""
+    module = sys.modules["k2_b200.ctc_loss"]
+    for logits in (False, True):
+        x = small_input(logits)
+        if logits:
+            x[1, 6, 3] = float("nan")    # a row of NaN
+            x[2] = -float("inf")         # an utterance without a path
+        got = []
+        for fused in (True, False):
+            module.FUSED_LOSS = fused
+            try:
+                leaf = x.clone().requires_grad_(True)
+                small_loss(k2, leaf, logits).backward(torch.tensor(upstream, device=DEV))
+            finally:
+                module.FUSED_LOSS = True
+            got.append(leaf.grad.cpu())
+        # (posteriors to 1e-6, twice for the upstream gradient of -2)
+        assert torch.allclose(got[0], got[1], rtol=0, atol=2e-6, equal_nan=True)
+        assert torch.equal(got[0].isinf(), got[1].isinf())
