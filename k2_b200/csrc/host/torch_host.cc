@@ -164,6 +164,8 @@ bool AppendSymbols(PyObject *items, Py_ssize_t n, int32_t *out) {
 // row_splits2, aux_labels, scores, labels, host row_splits1, host arc splits, BandGraph), or
 // None when the transcripts are not sequences of Python integers.
 py::object CtcGraph(py::handle symbols, bool modified, int device_index) {
+  // (what has no length is refused, iterators among it)
+  if (PyObject_Size(symbols.ptr()) < 0) throw py::error_already_set();
   py::object outer = py::reinterpret_steal<py::object>(
       PySequence_Fast(symbols.ptr(), "symbols must be a list of lists"));
   if (!outer) throw py::error_already_set();
@@ -172,8 +174,10 @@ py::object CtcGraph(py::handle symbols, bool modified, int device_index) {
   std::vector<py::object> rows(n);
   int64_t tot = 0;
   for (Py_ssize_t i = 0; i < n; ++i) {
+    PyObject *row = PySequence_Fast_GET_ITEM(outer.ptr(), i);
+    if (PyObject_Size(row) < 0) throw py::error_already_set();
     rows[i] = py::reinterpret_steal<py::object>(
-        PySequence_Fast(PySequence_Fast_GET_ITEM(outer.ptr(), i), "a transcript must be a list"));
+        PySequence_Fast(row, "a transcript must be a list"));
     if (!rows[i]) throw py::error_already_set();
     tot += PySequence_Fast_GET_SIZE(rows[i].ptr());
   }

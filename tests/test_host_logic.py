@@ -316,3 +316,15 @@ def test_scratch_of_layer_scores():
                dict(num_fsas=3, strict_layers=0)):
         one, two, incoming = plan(num_states=5000, num_arcs=10, **kw)
         assert incoming and max(one, two) < 1 << 40
+
+
+def test_transcripts_have_a_length():
+    """Both ways to a graph take what has a length, and refuse iterators (which a first look at them
+    would use up)."""
+    from k2_b200 import _lib
+    for symbols in (iter([[1, 2]]), ([1] for _ in range(2)), [iter([1, 2])], [1, 2]):
+        with pytest.raises(TypeError, match="has no len"):
+            _lib._host.ctc_graph(symbols, False, 0)
+    for symbols in (iter([[1, 2]]), [iter([1, 2])], [1, 2]):
+        with pytest.raises(TypeError, match="has no len"):
+            k2.ctc_graph(symbols)
