@@ -402,7 +402,7 @@ __device__ bool SearchStep(const SearchArgs &g, const SeqView &v, const Team &tm
   const bool row_ok = row0 + t < g.rows;
   const bool staged = g.cols <= kMaxRow;
   const float *row = staged ? sh->row : g.scores + (int64_t)(row_ok ? row0 + t : 0) * g.cols;
-  int32_t best = OrderedInt(kNegInf);
+  float best = kNegInf;
   const int32_t k_first = lo < hi ? v.warp_first[tm.warp] : ns;
   for (int32_t k0 = k_first; k0 < ns; k0 += 32) {
     const int32_t k = k0 + lane;
@@ -446,7 +446,7 @@ __device__ bool SearchStep(const SearchArgs &g, const SeqView &v, const Team &tm
           r_ll[p] = ll;
           r_dest[p] = dest;
           r_end[p] = end;
-          best = max(best, OrderedInt(end));
+          best = fmaxf(best, end);  // (not a NaN)
         }
       }
     }
@@ -454,7 +454,7 @@ __device__ bool SearchStep(const SearchArgs &g, const SeqView &v, const Team &tm
   }
   {
     float cutoff_f;
-    *beam = NextBeam(*beam, OrderedFloat(tm.Max(best)), ns, t, final_t, g, &cutoff_f);
+    *beam = NextBeam(*beam, OrderedFloat(tm.Max(OrderedInt(best))), ns, t, final_t, g, &cutoff_f);
     // ---- 2. first arc above the cutoff into every destination state (:1005-1028); the warp
     // lists those arcs and where they go.
     int32_t above = 0;

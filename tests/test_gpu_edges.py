@@ -292,3 +292,25 @@ def test_gradients_that_are_not_finite(k2, upstream):
         # (posteriors to 1e-6, twice for the upstream gradient of -2)
         assert torch.allclose(got[0], got[1], rtol=0, atol=2e-6, equal_nan=True)
         assert torch.equal(got[0].isinf(), got[1].isinf())
+
+
+def test_pruned_search_passes_by_scores_that_are_not_numbers(k2):
+    """A NaN among the scores costs the arcs that read it, not the utterance.  (On graphs in which the
+    arcs into a state have one label, so that a state whose arcs are NaN does not come up.)"""
+    from gpu_util import dense_from_scores, fsa_to_host, host_to_fsa
+    from k2_b200.autograd import _intersect_dense_pruned_arcs
+    rng = np.random.default_rng(17)
+    symbols = [rng.integers(1, 9, size=7).tolist() for _ in range(4)]
+    graphs = oracle.ctc_graphs(symbols, False)
+    scores, brs = random_dense(rng, 4, 60, 9, low_rows=False)
+    holes = rng.random(scores.shape) < 0.03
+    holes[:, 0] = holes[:, 1] = False
+    holes[brs[1:] - 1] = False
+    scores[holes] = np.nan
+    params = (20.0, 8.0, 0, 10000, False)
+    want = oracle.intersect_dense_pruned(graphs, scores, brs, *params)
+    assert all(np.diff(want.row_splits2[want.row_splits1])[:3] > 100)  # (the last has 3 frames)
+    for team in (0, 1, 4):
+        ragged, ma, mb = _intersect_dense_pruned_arcs(
+            host_to_fsa(graphs).arcs, dense_from_scores(scores, brs), *params, team)
+        same_fsa(fsa_to_host(k2.Fsa(ragged, _check=False), ma, mb), want, f"{team} CTAs")
