@@ -46,5 +46,5 @@ def get_aux_labels(best_paths: Fsa) -> List[List[int]]:
         values = aux.values.cpu().numpy()
         arc_splits = aux.row_splits().cpu().numpy()[arc_splits]
     else:
-        values = aux.cpu().numpy()
+        values = aux.to(torch.int32).cpu().numpy()
     return [v[v > 0].tolist() for v in np.split(values, arc_splits[1:-1])][:len(arc_splits) - 1]

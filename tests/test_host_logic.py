@@ -328,3 +328,12 @@ def test_transcripts_have_a_length():
     for symbols in (iter([[1, 2]]), [iter([1, 2])], [1, 2]):
         with pytest.raises(TypeError, match="has no len"):
             k2.ctc_graph(symbols)
+
+
+def test_aux_labels_are_integers():
+    for aux in (torch.tensor([3, 0, 5, -1], dtype=torch.int32), torch.tensor([3.0, 0.5, 5.7, -1.0]),
+                torch.tensor([3, 0, 2**32 + 5, -1])):
+        fsa = k2.linear_fsa([1, 2, 3])
+        fsa.aux_labels = aux
+        got = k2.get_aux_labels(fsa)
+        assert got == [[3, 5]] and all(type(x) is int for x in got[0])
