@@ -43,8 +43,8 @@ def _host_stale() -> bool:
     if not os.path.exists(HOST_PATH):
         return True
     t = os.path.getmtime(HOST_PATH)
-    deps = [HOST_SOURCE, os.path.join(_HERE, "..", "include", "k2b200.h"),
-            os.path.abspath(__file__)]
+    deps = glob.glob(os.path.join(CSRC, "host", "*")) + \
+        [os.path.join(_HERE, "..", "include", "k2b200.h"), os.path.abspath(__file__)]
     return any(os.path.getmtime(d) > t for d in deps)
 
 

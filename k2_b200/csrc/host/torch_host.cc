@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "../../../include/k2b200.h"
+#include "python_ints.h"
 
 namespace py = pybind11;
 
@@ -133,33 +134,6 @@ std::shared_ptr<BandGraph> MakeBandGraph(at::Tensor row_splits2, at::Tensor stat
   return g;
 }
 
-// One transcript appended to `out`; false when an element is not a Python int of 32 bits.
-bool AppendSymbols(PyObject *items, Py_ssize_t n, int32_t *out) {
-  PyObject **at = PySequence_Fast_ITEMS(items);
-  for (Py_ssize_t k = 0; k < n; ++k) {
-    PyObject *x = at[k];
-    long v;
-    if (PyLong_CheckExact(x) && PyUnstable_Long_IsCompact(reinterpret_cast<PyLongObject *>(x))) {
-      v = (long)PyUnstable_Long_CompactValue(reinterpret_cast<PyLongObject *>(x));
-    } else {
-      PyObject *index = PyNumber_Index(x);
-      if (index == nullptr) {
-        PyErr_Clear();
-        return false;
-      }
-      v = PyLong_AsLong(index);
-      Py_DECREF(index);
-      if (v == -1 && PyErr_Occurred()) {
-        PyErr_Clear();
-        return false;
-      }
-    }
-    if (v != (int32_t)v) return false;
-    out[k] = (int32_t)v;
-  }
-  return true;
-}
-
 // CTC graphs of a batch of transcripts with their band tables: (values, row_splits1,
 // row_splits2, aux_labels, scores, labels, host row_splits1, host arc splits, BandGraph), or
 // None when the transcripts are not sequences of Python integers.
@@ -192,7 +166,7 @@ py::object CtcGraph(py::handle symbols, bool modified, int device_index) {
   for (Py_ssize_t i = 0; i < n; ++i) {
     const Py_ssize_t len = PySequence_Fast_GET_SIZE(rows[i].ptr());
     int32_t *mine = sym + at;
-    if (!AppendSymbols(rows[i].ptr(), len, mine)) return py::none();
+    if (!Int32sOf(rows[i].ptr(), len, mine)) return py::none();
     first[i] = (int32_t)at;
     arc0[i] = (int32_t)arcs;
     rs1[i] = (int32_t)(2 * at + 2 * i);

@@ -3,6 +3,8 @@ format, sharding, and the C-ABI library's exported symbols."""
 import ctypes
 import os
 import re
+import subprocess
+import sysconfig
 
 import numpy as np
 import pytest
@@ -337,3 +339,30 @@ def test_aux_labels_are_integers():
         fsa.aux_labels = aux
         got = k2.get_aux_labels(fsa)
         assert got == [[3, 5]] and all(type(x) is int for x in got[0])
+
+
+@pytest.mark.parametrize("hex_version", [None, "0x030A00F0"])
+def test_python_integers_of_any_python(tmp_path, hex_version):
+    """csrc/host/python_ints.h with what this Python has, and without what came with 3.12."""
+    source = "#include <Python.h>\n"
+    if hex_version:
+        source += (f"#undef PY_VERSION_HEX\n#define PY_VERSION_HEX {hex_version}\n"
+                   "#undef PyUnstable_Long_IsCompact\n#undef PyUnstable_Long_CompactValue\n"
+                   "#pragma GCC poison PyUnstable_Long_IsCompact PyUnstable_Long_CompactValue\n")
+    source += ('#include "python_ints.h"\n'
+               'extern "C" int ints(PyObject *x, int32_t *out) {\n'
+               "  return Int32sOf(x, PySequence_Fast_GET_SIZE(x), out);\n}\n")
+    (tmp_path / "ints.cc").write_text(source)
+    lib = str(tmp_path / "ints.so")
+    subprocess.check_call(["g++", "-std=c++17", "-Wall", "-Werror", "-fPIC", "-shared",
+                           "-I" + sysconfig.get_paths()["include"],
+                           "-I" + os.path.join(ROOT, "k2_b200", "csrc", "host"),
+                           str(tmp_path / "ints.cc"), "-o", lib])
+    ints = ctypes.PyDLL(lib).ints
+    ints.argtypes = [ctypes.py_object, ctypes.c_void_p]
+    good = [0, -1, 5, 2**29, 2**30, 2**31 - 1, -2**31, True, np.int64(7), np.int16(-3)]
+    out = (ctypes.c_int32 * len(good))()
+    assert ints(good, out) == 1 and list(out) == [int(x) for x in good]
+    assert ints(tuple(good), out) == 1
+    for bad in (2**31, -2**31 - 1, 2**70, 1.0, "1", None):
+        assert ints([1, bad], out) == 0, bad
