@@ -6,8 +6,10 @@ repository; nothing is JIT-compiled at import time.
 """
 import glob
 import os
+import shutil
 import subprocess
 import sys
+import sysconfig
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(_HERE, "csrc")
@@ -39,9 +41,21 @@ HOST_PATH = os.path.join(_HERE, "_host.so")
 HOST_SOURCE = os.path.join(CSRC, "host", "torch_host.cc")
 
 
-def _host_stale() -> bool:
-    if not os.path.exists(HOST_PATH):
+# what _host.so was built for: it works with that Python and that torch only
+HOST_KEY_PATH = os.path.join(_HERE, "_host.built_for")
+
+
+def _host_key(command) -> str:
+    import torch
+    return "\n".join([sys.version, torch.__version__] + command) + "\n"
+
+
+def _host_stale(command) -> bool:
+    if not (os.path.exists(HOST_PATH) and os.path.exists(HOST_KEY_PATH)):
         return True
+    with open(HOST_KEY_PATH) as f:
+        if f.read() != _host_key(command):
+            return True
     t = os.path.getmtime(HOST_PATH)
     deps = glob.glob(os.path.join(CSRC, "host", "*")) + \
         [os.path.join(_HERE, "..", "include", "k2b200.h"), os.path.abspath(__file__)]
@@ -49,15 +63,16 @@ def _host_stale() -> bool:
 
 
 def _host_command():
-    """g++ on the one translation unit that includes torch's headers; libk2b200.so is found
-    next to it, torch's libraries are loaded by `import torch`."""
-    import importlib.util
-    import sysconfig
-    torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
+    """The C++ compiler on the one translation unit that includes torch's headers;
+    libk2b200.so is found next to it, torch's libraries are loaded by `import torch`."""
+    import torch
+    torch_dir = os.path.dirname(torch.__file__)
     cuda = os.path.join(os.path.dirname(os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")), "..")
     inc = os.path.join(torch_dir, "include")
-    return ["/usr/bin/g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
-            "-D_GLIBCXX_USE_CXX11_ABI=1", "-DTORCH_EXTENSION_NAME=_host",
+    return [os.environ.get("CXX") or shutil.which("g++") or "c++", "-O2", "-std=c++17", "-fPIC",
+            "-shared", "-fvisibility=hidden",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            "-DTORCH_EXTENSION_NAME=_host",
             "-isystem", inc, "-isystem", os.path.join(inc, "torch", "csrc", "api", "include"),
             "-isystem", os.path.join(cuda, "include"),
             "-isystem", sysconfig.get_paths()["include"], HOST_SOURCE, "-o", HOST_PATH,
@@ -68,8 +83,11 @@ def _host_command():
 
 def build(force: bool = False, verbose: bool = False) -> str:
     _build_library(force, verbose)
-    if force or _host_stale():
-        subprocess.check_call(_host_command())
+    command = _host_command()
+    if force or _host_stale(command):
+        subprocess.check_call(command)
+        with open(HOST_KEY_PATH, "w") as f:
+            f.write(_host_key(command))
     return LIB_PATH
 
 

@@ -366,3 +366,22 @@ def test_python_integers_of_any_python(tmp_path, hex_version):
     assert ints(tuple(good), out) == 1
     for bad in (2**31, -2**31 - 1, 2**70, 1.0, "1", None):
         assert ints([1, bad], out) == 0, bad
+
+
+def test_host_layer_is_stale_under_another_torch_or_python(monkeypatch):
+    """`python k2_b200/build.py`, which the import error names, builds _host.so anew after torch or
+    Python changed."""
+    import importlib.util
+    spec = importlib.util.spec_from_file_location("_build",
+                                                  os.path.join(ROOT, "k2_b200", "build.py"))
+    build = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(build)
+    command = build._host_command()
+    assert not build._host_stale(command)
+    assert build._host_stale(command + ["-g"])
+    with monkeypatch.context() as m:
+        m.setattr(torch, "__version__", "1.0")
+        assert build._host_stale(command)
+    with monkeypatch.context() as m:
+        m.setattr(build.sys, "version", "3.9")
+        assert build._host_stale(command)
