@@ -473,8 +473,8 @@ int32_t k2b200_dense_loss_backward_log_probs(const k2b200_intersect_args *args, 
  * max_states / max_arcs); sums run in float64 mantissa/exponent arithmetic, so any score
  * range is handled.  The dense scores are read from the log-prob matrix the DenseFsaVec was
  * made from (k2/python/k2/dense_fsa_vec.py:43-145), not from its [rows, C+1] score matrix:
- * log_probs is [log_prob_rows, num_classes] contiguous float32, 16-byte aligned, with
- * num_classes a multiple of 4, and graph i reads rows h_first_row[i] .. + h_frames[i] - 1;
+ * log_probs is [log_prob_rows, num_classes] contiguous float32, of any alignment and any number
+ * of classes; nothing outside it is read.  Graph i reads rows h_first_row[i] .. + h_frames[i] - 1;
  * the extra final row of a sequence is implied.
  *
  *   k2b200_band_tables: per-state tables of a_fsas (band_states: tables_bytes' first size,
@@ -482,8 +482,8 @@ int32_t k2b200_dense_loss_backward_log_probs(const k2b200_intersect_args *args, 
  *     graph, in which case the tables must not be used.  They depend on the graphs only and
  *     can be kept for as long as the arcs do not change.
  *   k2b200_band_loss_supported: *supported = 0 when the sizes do not fit (more than 1024
- *     states in a graph, rows or frames beyond shared memory);
- *     k2b200_last_error() says which.  Host-side only.
+ *     states in a graph, 65 534 frames or 65 535 graphs); k2b200_last_error() says which.
+ *     Host-side only.
  *   k2b200_band_loss_forward: tot_scores[num_fsas] (device, float64; -inf for a graph
  *     with no surviving path; NaN if a copy into shared memory timed out, see
  *     k2b200_band_loss_status).  The workspace keeps what the backward needs.  The call

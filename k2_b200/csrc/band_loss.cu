@@ -315,7 +315,7 @@ BandGather(const BandInfo *__restrict__ infos, const BandState *__restrict__ tab
 template <bool kByState>
 __global__ void __launch_bounds__(64 * kVitMaxWarps, 1)
 BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ tab,
-            const float *__restrict__ lp, int32_t C, float *__restrict__ vf,
+            const float *__restrict__ lp, int64_t lp_rows, int32_t C, float *__restrict__ vf,
             float *__restrict__ vb, int32_t F, int32_t nbatch, int32_t slot_floats,
             int32_t xch_pad, int32_t wait_limit, int32_t *__restrict__ status) {
   constexpr int K = kVitK;
@@ -343,7 +343,8 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
   const int32_t num_batches = (T + F - 1) / F;
   const float *lp0 = kByState ? lp + f.grid_off : lp + (int64_t)f.lp_row * C;
   // A row may start anywhere (C need not be a multiple of four): a batch is copied from the
-  // 16-byte boundary at or before its first element to the one at or after its last.
+  // 16-byte boundary at or before its first element to the one at or after its last.  At the ends
+  // of the matrix that may lie outside it: there the last elements are copied one by one.
   const uint32_t lp0_words = (uint32_t)(reinterpret_cast<uintptr_t>(lp0) >> 2);
   auto words_off = [&](int32_t r) {
     return kByState ? 0 : (int32_t)((lp0_words + (uint32_t)r * (uint32_t)width) & 3u);
@@ -356,11 +357,22 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
     const int32_t r0 = dir == 0 ? q * F : max(T - (q + 1) * F, 0);
     const int32_t r1 = dir == 0 ? min((q + 1) * F, T) : T - q * F;
     const int32_t off = words_off(r0);
-    const unsigned bytes = (((unsigned)(r1 - r0) * (unsigned)width + (unsigned)off + 3u) & ~3u) * 4u;
+    // in floats from the first boundary: the batch is [off, end), [from, to) goes as one copy
+    const int32_t end = (r1 - r0) * width + off;
+    int32_t from = 0, to = (end + 3) & ~3;
     const int32_t slot = q % nbatch;
-    MbarArriveExpectTx(&full[slot], bytes);
-    BulkCopyG2S(ring + (size_t)slot * slot_floats, lp0 + (int64_t)r0 * width - off, bytes,
-                &full[slot]);
+    float *dst = ring + (size_t)slot * slot_floats;
+    const float *src = lp0 + (int64_t)r0 * width - off;
+    if (!kByState && (src < lp || src + to > lp + lp_rows * width)) {
+      if (src < lp) from = 4;
+      if (src + to > lp + lp_rows * width) to = max(to - 4, from);
+      for (int32_t k = off; k < min(from, end); ++k) dst[k] = src[k];
+      for (int32_t k = max(to, off); k < end; ++k) dst[k] = src[k];
+      // (the slot's next batch overwrites them)
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    MbarArriveExpectTx(&full[slot], (unsigned)(to - from) * 4u);
+    if (to > from) BulkCopyG2S(dst + from, src + from, (unsigned)(to - from) * 4u, &full[slot]);
     ++issued;
   };
   if (tid == 0)
@@ -2175,7 +2187,7 @@ int32_t k2b200_band_loss_forward_reduce(const k2b200_band_loss_args *args, void 
     { kernel<<<grid, L.vit_threads, L.viterbi_smem, stream>>>(
         infos, tab,
         L.by_state ? reinterpret_cast<const float *>(ws + L.off_by_state) : args->log_probs,
-        args->num_classes, reinterpret_cast<float *>(ws + L.off_vf),
+        args->log_prob_rows, args->num_classes, reinterpret_cast<float *>(ws + L.off_vf),
         reinterpret_cast<float *>(ws + L.off_vb), L.vit_frames, L.vit_batches, L.vit_slot,
         L.xch_pad, CopyWaitLimit(), reinterpret_cast<int32_t *>(ws + L.off_status));
       NoteLaunch(); }

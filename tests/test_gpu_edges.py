@@ -314,3 +314,27 @@ def test_pruned_search_passes_by_scores_that_are_not_numbers(k2):
         ragged, ma, mb = _intersect_dense_pruned_arcs(
             host_to_fsa(graphs).arcs, dense_from_scores(scores, brs), *params, team)
         same_fsa(fsa_to_host(k2.Fsa(ragged, _check=False), ma, mb), want, f"{team} CTAs")
+
+
+@pytest.mark.parametrize("n,frames,classes", [
+    (1, 1, 1), (1, 1, 2), (1, 1, 5), (1, 2, 1), (2, 3, 5), (1, 17, 7), (3, 33, 29), (2, 16, 500),
+])
+def test_log_probs_of_any_alignment(k2, n, frames, classes):
+    """The same bits wherever the log-probs start, with NaN in front of them and behind."""
+    rng = np.random.default_rng(frames)
+    x = torch.log_softmax(torch.from_numpy(
+        rng.normal(size=(n, frames, classes)).astype(np.float32)), -1).to(DEV)
+    seg = torch.tensor([[i, 0, frames] for i in range(n)], dtype=torch.int32)
+    symbols = [[1] if classes > 1 else [] for _ in range(n)]
+    got = []
+    for offset in range(5):
+        buf = torch.full((x.numel() + 12,), float("nan"), device=DEV)
+        leaf = buf[offset:offset + x.numel()].view(x.shape)
+        leaf.copy_(x)
+        leaf.requires_grad_(True)
+        loss = k2.ctc_loss(k2.ctc_graph(symbols, device=DEV), k2.DenseFsaVec(leaf, seg))
+        loss.backward()
+        got.append((loss.detach(), leaf.grad))
+    assert torch.isfinite(got[0][0]) and torch.isfinite(got[0][1]).all()
+    for loss, grad in got[1:]:
+        assert torch.equal(loss, got[0][0]) and torch.equal(grad, got[0][1])
