@@ -46,7 +46,7 @@ at::TensorOptions On(at::ScalarType type, at::Device device) {
 }
 
 // ---------------------------------------------------------------------------
-// Workspaces.  Those of a loss are up to a gigabyte and live from a forward to its backward.
+// Workspaces.  Those of a loss are a gigabyte or more and live from a forward to its backward.
 // Handed back to torch's caching allocator they get split for smaller tensors, after which the
 // next step needs a fresh cudaMalloc, which waits for the whole device.  So the last few are
 // kept here, per device and stream: what comes back may still be read by kernels queued on
@@ -481,6 +481,13 @@ PYBIND11_MODULE(_host, m) {
   NameNode<BandTotScoresNode>("_BandTotScoresBackward");
   NameNode<BandNegSumNode>("_BandNegSumBackward");
   NameNode<BandMeanNode>("_BandMeanBackward");
+  py::class_<Workspace, std::shared_ptr<Workspace>>(m, "Workspace")
+      .def(py::init([](int64_t bytes, int device_index) {
+        const at::Device device(at::kCUDA, (c10::DeviceIndex)device_index);
+        return std::make_shared<Workspace>(
+            bytes, device, c10::cuda::getCurrentCUDAStream(device.index()).stream());
+      }))
+      .def_readonly("tensor", &Workspace::tensor);
   py::class_<BandGraph, std::shared_ptr<BandGraph>>(m, "BandGraph")
       .def(py::init(&MakeBandGraph))
       .def_property_readonly("states_ptr",

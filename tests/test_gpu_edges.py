@@ -338,3 +338,41 @@ def test_log_probs_of_any_alignment(k2, n, frames, classes):
     assert torch.isfinite(got[0][0]) and torch.isfinite(got[0][1]).all()
     for loss, grad in got[1:]:
         assert torch.equal(loss, got[0][0]) and torch.equal(grad, got[0][1])
+
+
+# --------------------------------------------------------------------------- workspaces
+def test_one_pool_of_workspaces(k2):
+    """Large workspaces come back to the next call on their stream, whichever path makes it; at most
+    three are kept, and given back when asked."""
+    from k2_b200 import _lib
+    k2._lib.release_workspaces()
+    torch.cuda.empty_cache()
+    before = torch.cuda.memory_allocated()
+    mb = 1 << 20
+    first = _lib.workspace(100 * mb, DEV)
+    at = first.tensor.data_ptr()
+    assert first.tensor.numel() >= 100 * mb and first.tensor.device == torch.device(DEV)
+    del first
+    assert _lib.workspace(90 * mb, DEV).tensor.data_ptr() == at     # as large, or half as large
+    with torch.cuda.stream(torch.cuda.Stream()):
+        other = _lib.workspace(90 * mb, DEV)                        # another stream, another one
+    assert other.tensor.data_ptr() != at
+    del other
+    k2._lib.release_workspaces()
+    several = [_lib.workspace(n * 40 * mb, DEV) for n in range(1, 6)]
+    del several
+    kept = torch.cuda.memory_allocated() - before
+    assert (3 + 4 + 5) * 40 * mb <= kept <= 1.2 * (3 + 4 + 5) * 40 * mb
+    small = _lib.workspace(mb, DEV)                                 # not pooled
+    del small
+    # the general kernels and the band kernels of one batch size use one workspace after another
+    k2._lib.release_workspaces()
+    x = torch.log_softmax(torch.randn(16, 400, 60, device=DEV), -1)
+    seg = torch.tensor([[i, 0, 400] for i in range(16)], dtype=torch.int32)
+    graphs = k2.ctc_graph([[1 + i % 50 for i in range(100)]] * 16, device=DEV)
+    for band in (True, False, True, False):
+        k2.intersect_dense_tot_scores(graphs, k2.DenseFsaVec(x, seg), 10.0, band=band)
+    torch.cuda.synchronize()
+    del x, graphs
+    k2._lib.release_workspaces()
+    assert torch.cuda.memory_allocated() <= before + mb
