@@ -6,6 +6,7 @@
 // the functions size and allocate outputs, call the C-ABI (include/k2b200.h) and hand tensors
 // back.  Python keeps k2's names and contracts (k2/python/k2/ctc_loss.py:28-208,
 // k2/python/k2/fsa_algo.py:1160-1249, k2/python/k2/dense_fsa_vec.py:43-145).
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/function.h>
@@ -50,7 +51,8 @@ at::TensorOptions On(at::ScalarType type, at::Device device) {
 // Handed back to torch's caching allocator they get split for smaller tensors, after which the
 // next step needs a fresh cudaMalloc, which waits for the whole device.  So the last few are
 // kept here, per device and stream: what comes back may still be read by kernels queued on
-// that stream, and the next user queues behind them.
+// that stream, and the next user queues behind them.  A call that is captured takes memory of
+// its graph instead, which stays the graph's for every replay.
 // ---------------------------------------------------------------------------
 constexpr int64_t kPoolMinBytes = 32 << 20;  // smaller ones go through torch's allocator
 constexpr size_t kPoolKeep = 3;              // idle workspaces per (device, stream)
@@ -68,7 +70,8 @@ struct Workspace {
   at::Tensor tensor;
   std::pair<int, cudaStream_t> key{-1, nullptr};
   Workspace(int64_t bytes, at::Device device, cudaStream_t stream) {
-    if (bytes < kPoolMinBytes) {
+    if (bytes < kPoolMinBytes ||
+        c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) {
       tensor = at::empty({std::max<int64_t>(bytes, 1)}, On(at::kByte, device));
       return;
     }

@@ -376,3 +376,40 @@ def test_one_pool_of_workspaces(k2):
     del x, graphs
     k2._lib.release_workspaces()
     assert torch.cuda.memory_allocated() <= before + mb
+
+
+def test_captured_calls_keep_off_the_pool(k2):
+    """A loss and its gradient as a CUDA graph: replays give the bits of eager calls whatever became
+    of the pool since, and change nothing that other calls hold."""
+    k2._lib.release_workspaces()
+    n, frames, classes = 16, 400, 60
+    seg = torch.tensor([[i, 0, frames] for i in range(n)], dtype=torch.int32)
+    graphs = k2.ctc_graph([[1 + (3 * i + j) % 50 for i in range(100)] for j in range(n)], device=DEV)
+    gen = torch.Generator(DEV).manual_seed(1)
+    draw = lambda: torch.log_softmax(  # noqa: E731
+        torch.randn(n, frames, classes, device=DEV, generator=gen), -1)
+
+    def step(x):
+        tot = k2.intersect_dense_tot_scores(graphs, k2.DenseFsaVec(x, seg), 10.0)
+        return tot, torch.autograd.grad(tot.sum(), x)[0]
+
+    static = draw().requires_grad_(True)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        for _ in range(2):
+            step(static)
+    torch.cuda.synchronize()
+    captured = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(captured, stream=stream):
+        got = step(static)
+    k2._lib.release_workspaces()
+    held = torch.full((1 << 28,), 3.0, device=DEV)  # where the warm-up's workspace was, among others
+    for _ in range(3):
+        x = draw()
+        with torch.no_grad():
+            static.copy_(x)
+        captured.replay()
+        want = step(x.requires_grad_(True))
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    assert bool((held == 3.0).all())
