@@ -6,7 +6,7 @@
 // the functions size and allocate outputs, call the C-ABI (include/k2b200.h) and hand tensors
 // back.  Python keeps k2's names and contracts (k2/python/k2/ctc_loss.py:28-208,
 // k2/python/k2/fsa_algo.py:1160-1249, k2/python/k2/dense_fsa_vec.py:43-145).
-#include <c10/cuda/CUDAGraphsC10Utils.h>
+#include <c10/cuda/CUDAException.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/function.h>
@@ -70,8 +70,9 @@ struct Workspace {
   at::Tensor tensor;
   std::pair<int, cudaStream_t> key{-1, nullptr};
   Workspace(int64_t bytes, at::Device device, cudaStream_t stream) {
-    if (bytes < kPoolMinBytes ||
-        c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (bytes >= kPoolMinBytes) C10_CUDA_CHECK(cudaStreamIsCapturing(stream, &capture));
+    if (bytes < kPoolMinBytes || capture != cudaStreamCaptureStatusNone) {
       tensor = at::empty({std::max<int64_t>(bytes, 1)}, On(at::kByte, device));
       return;
     }
