@@ -1947,8 +1947,11 @@ int32_t k2b200_dense_loss_forward(const k2b200_intersect_args *args, void *works
               "use intersect_dense + get_tot_scores",
               L.max_states, L.max_arcs, args->cols);
   char *ws = reinterpret_cast<char *>(workspace);
-  K2B_CUDA_OK(cudaMemcpyAsync(ws + L.off_infos, L.infos.data(), sizeof(FsaInfo) * args->num_fsas,
-                              cudaMemcpyHostToDevice, stream));
+  // as kernel parameters: a copy that is captured would read the host's array at every replay
+  static_assert(sizeof(FsaInfo) % sizeof(int32_t) == 0, "FsaInfo is uploaded as int32 words");
+  K2B_FORWARD(UploadInts(reinterpret_cast<const int32_t *>(L.infos.data()),
+                         (int64_t)L.infos.size() * (sizeof(FsaInfo) / sizeof(int32_t)),
+                         reinterpret_cast<int32_t *>(ws + L.off_infos), stream));
   const FsaInfo *d_infos = reinterpret_cast<const FsaInfo *>(ws + L.off_infos);
   unsigned char *dense = reinterpret_cast<unsigned char *>(ws + LL.off_dense);
   int32_t *unfit = reinterpret_cast<int32_t *>(ws + L.off_unfit);

@@ -378,7 +378,8 @@ def test_one_pool_of_workspaces(k2):
     assert torch.cuda.memory_allocated() <= before + mb
 
 
-def test_captured_calls_keep_off_the_pool(k2):
+@pytest.mark.parametrize("band", [True, False])
+def test_captured_calls_keep_off_the_pool(k2, band):
     """A loss and its gradient as a CUDA graph: replays give the bits of eager calls whatever became
     of the pool since, and change nothing that other calls hold."""
     k2._lib.release_workspaces()
@@ -390,7 +391,7 @@ def test_captured_calls_keep_off_the_pool(k2):
         torch.randn(n, frames, classes, device=DEV, generator=gen), -1)
 
     def step(x):
-        tot = k2.intersect_dense_tot_scores(graphs, k2.DenseFsaVec(x, seg), 10.0)
+        tot = k2.intersect_dense_tot_scores(graphs, k2.DenseFsaVec(x, seg), 10.0, band=band)
         return tot, torch.autograd.grad(tot.sum(), x)[0]
 
     static = draw().requires_grad_(True)
