@@ -88,6 +88,9 @@ struct PhaseTimer {  // records start/stop events when profiling is enabled
   int slot_;
 };
 
+// SMs of the current device (148 on a whole B200, which is also the answer without a device).
+int32_t NumSms();
+
 // A second stream per device for kernels that do not depend on what the caller's
 // stream is running (they fill the SMs that a latency-bound recursion leaves mostly
 // idle).  SideFork makes the side stream wait for everything enqueued on `main` so

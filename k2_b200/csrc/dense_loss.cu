@@ -1984,7 +1984,7 @@ int32_t k2b200_dense_loss_forward(const k2b200_intersect_args *args, void *works
   {
     PhaseTimer timer(kPhaseDense, side);  // repacking belongs with the dense matrix
     const int64_t n_dense = (int64_t)args->rows * LL.pack.cols4;
-    { ExpDense<<<(int)std::min<int64_t>(CeilDiv(n_dense, 256), 148 * 8), 256, 0, side>>>(
+    { ExpDense<<<(int)std::min<int64_t>(CeilDiv(n_dense, 256), NumSms() * 8), 256, 0, side>>>(
         args->scores, args->rows, LL.pack, dense, kMinDenseScore,
         reinterpret_cast<int32_t *>(ws + LL.off_flags)); NoteLaunch(); }
   }

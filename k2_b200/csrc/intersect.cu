@@ -98,7 +98,7 @@ int32_t MakeLayout(const k2b200_intersect_args *a, Layout *L) {
   int64_t max_pair_words = 0;
   for (const FsaInfo &f : L->infos)
     max_pair_words = std::max<int64_t>(max_pair_words, (int64_t)(f.tk + 1) * f.words);
-  const int64_t runs = (int64_t)148 * 64 * (a->num_arcs / 8 >= a->num_states ? 5 : 1);
+  const int64_t runs = (int64_t)NumSms() * 64 * (a->num_arcs / 8 >= a->num_states ? 5 : 1);
   L->words_per_warp = (int32_t)std::max<int64_t>(1, std::min<int64_t>(16, words / runs));
   L->tiles_per_pair = CeilDiv(max_pair_words, (int64_t)L->words_per_warp * (kCountThreads / 32));
   L->count_blocks = (int32_t)std::min<int64_t>((int64_t)L->tiles_per_pair * a->num_fsas,

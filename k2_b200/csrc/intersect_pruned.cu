@@ -1092,7 +1092,7 @@ __global__ void FormatPruned(const FormatArgs f) {
 
 // CTAs per frame: about 16 per SM in all, however few the frames are.
 unsigned FormatParts(int64_t frames, int64_t seqs) {
-  return (unsigned)std::max<int64_t>(1, std::min<int64_t>(32, 148 * 16 / (frames * seqs)));
+  return (unsigned)std::max<int64_t>(1, std::min<int64_t>(32, NumSms() * 16 / (frames * seqs)));
 }
 
 // ---------------------------------------------------------------------------
@@ -1893,7 +1893,7 @@ static int32_t CopyStreams(const k2b200_online_args *args, void *workspace,
   for (const CopyJob &j : jobs) longest = std::max(longest, j.count);
   // about 8 CTAs per SM when the copies are long
   const int32_t parts = (int32_t)std::max<int64_t>(
-      1, std::min<int64_t>(CeilDiv(longest, 1024), 148 * 8 / (int64_t)jobs.size() + 1));
+      1, std::min<int64_t>(CeilDiv(longest, 1024), NumSms() * 8 / (int64_t)jobs.size() + 1));
   { CopyMany<<<dim3((unsigned)jobs.size(), parts), 256, 0, stream>>>(L.jobs); NoteLaunch(); }
   K2B_CUDA_OK(cudaGetLastError());
   return kOk;

@@ -233,7 +233,7 @@ static ChainPlan PlanChain(const k2b200_fsa_view *v, int32_t ndir) {
   const size_t vals = 2 * sizeof(double) * (size_t)p.maxw;
   // with more CTAs than SMs, two of them should share one
   const size_t budget =
-      (int64_t)ndir * v->num_fsas > 148 ? kLayerSmemBudget / 2 : kLayerSmemBudget;
+      (int64_t)ndir * v->num_fsas > NumSms() ? kLayerSmemBudget / 2 : kLayerSmemBudget;
   // a slot takes the largest layer with a quarter of padding, or several small ones
   const size_t largest = (size_t)v->max_layer_arcs * 22 + (size_t)p.maxw * 16 + 4096;
   for (size_t limit : {budget, kLayerSmemBudget}) {
@@ -249,7 +249,7 @@ static ChainPlan PlanChain(const k2b200_fsa_view *v, int32_t ndir) {
   p.wide = 1;
   p.warps = 16;
   p.team = 1;
-  while (p.team < 8 && (int64_t)ndir * v->num_fsas * p.team * 2 <= 148 &&
+  while (p.team < 8 && (int64_t)ndir * v->num_fsas * p.team * 2 <= NumSms() &&
          p.team * 32 * p.warps < v->max_layer_states)
     p.team *= 2;
   p.bytes = sizeof(int32_t) * (size_t)((p.nl_cap + 1 + 3) & ~3);

@@ -166,6 +166,16 @@ int32_t SideOfCurrentDevice(SideState **out) {
 }
 }  // namespace
 
+int32_t NumSms() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) {
+    cudaGetLastError();
+    return 148;
+  }
+  return sms;
+}
+
 int32_t SideFork(cudaStream_t main, cudaStream_t *side) {
   std::lock_guard<std::mutex> lock(g_side_mutex);
   SideState *st;
@@ -644,7 +654,7 @@ int32_t BuildIncoming(const int32_t *row_splits1, const int32_t *row_ids1,
     { IncomingSortSmall<<<CeilDiv(num_states, 256), 256, 0, stream>>>(
         in_splits, num_states, unsorted, row_ids2, arcs, in_arcs, in_src, in_score, counts);
       NoteLaunch(); }
-    { IncomingSortLarge<<<148 * 8, 256, 0, stream>>>(in_splits, num_states, unsorted, row_ids2, arcs,
+    { IncomingSortLarge<<<NumSms() * 8, 256, 0, stream>>>(in_splits, num_states, unsorted, row_ids2, arcs,
                                                 in_arcs, in_src, in_score, counts);
       NoteLaunch(); }
   }

@@ -329,7 +329,7 @@ int32_t LaunchSharedViterbi(const Layout &L, const k2b200_intersect_args *a, cha
   float *xt = reinterpret_cast<float *>(region + p.off_xt);
   float *dtf = reinterpret_cast<float *>(region + p.off_dtf);
   float *dtb = reinterpret_cast<float *>(region + p.off_dtb);
-  { SharedDenseTranspose<<<148 * 8, 256, 0, stream>>>(d_infos, a->num_fsas, p.upad, p.tk_max,
+  { SharedDenseTranspose<<<NumSms() * 8, 256, 0, stream>>>(d_infos, a->num_fsas, p.upad, p.tk_max,
                                                        a->scores, a->cols, dtf, dtb);
     NoteLaunch(); }
   { SharedViterbiInit<<<CeilDiv((int64_t)S * p.upad, 256), 256, 0, stream>>>(
