@@ -417,7 +417,7 @@ GridChainLanes(const FsaInfo *__restrict__ infos, int32_t n, const Arc *__restri
 // scores of its rows in shared memory.  Also enforces kMinDenseScore (on every finite
 // element of the rows, a little stricter than on surviving arcs only).
 // ---------------------------------------------------------------------------
-// The state pitch of the staged scores and the rows per CTA are compile-time, and the row loop
+// The state pitch of the staged scores is compile-time, and the row loop
 // is unrolled, so the score of an arc's other end is one load at (byte offset of that state,
 // fixed for the call) + constant.  Walking forward in a graph where every state has one
 // entering label the dense score of a lane's arcs is one load per row.
@@ -425,7 +425,7 @@ GridChainLanes(const FsaInfo *__restrict__ infos, int32_t n, const Arc *__restri
 // direction and additions in pairs: 397 -> 322 us for 128 x 500 frames of 4 627 arcs, both
 // directions (four rows side by side for 16-byte gathers: 373, spills at the 40 registers that
 // let two CTAs share an SM).
-template <int kDeg, int kThreads, int kSPad, int kMaskRows>
+template <int kDeg, int kThreads, int kSPad>
 __global__ void __launch_bounds__(kThreads, 1536 / kThreads)
 ArcMasks(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_levels,
          const Arc *__restrict__ arcs, const int32_t *__restrict__ a_row_splits2,
@@ -433,7 +433,8 @@ ArcMasks(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_levels,
          const unsigned char *__restrict__ dense, DensePack dp,
          const float *__restrict__ vfwd, const float *__restrict__ vbwd,
          const float *__restrict__ cutoffs, const int32_t *__restrict__ plan,
-         int32_t *__restrict__ unfit, unsigned char *__restrict__ masks, int32_t mask_pitch) {
+         int32_t *__restrict__ unfit, unsigned char *__restrict__ masks, int32_t mask_pitch,
+         int32_t mask_rows) {
   static_assert(kDeg <= 8 && kDeg % 2 == 0, "one byte per lane, arcs in pairs");
   constexpr int32_t s_pad = kSPad;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -441,15 +442,15 @@ ArcMasks(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_levels,
   if ((unfit[i] & 1) || unfit[n + i] != LaneClass(kThreads)) return;
   const FsaInfo f = infos[i];
   const int32_t S = f.num_states, Tk = f.tk, cols = dp.cols;
-  const int32_t r0 = blockIdx.x * kMaskRows + (dir == 0 ? 1 : 0);
+  const int32_t r0 = blockIdx.x * mask_rows + (dir == 0 ? 1 : 0);
   const int32_t r_end = dir == 0 ? Tk + 1 : Tk;
   if (S == 0 || r0 >= r_end) return;
-  const int32_t nf = min(kMaskRows, r_end - r0);
+  const int32_t nf = min(mask_rows, r_end - r0);
   const int32_t lb = dir == 0 ? r0 - 1 : r0;  // first staged level and first dense row
   const int tid = threadIdx.x, nt = blockDim.x;
-  float *fo = reinterpret_cast<float *>(smem_raw);  // [kMaskRows + 1][s_pad]
-  float *bo = fo + (kMaskRows + 1) * s_pad;         // [kMaskRows + 1][s_pad]
-  float *lp = bo + (kMaskRows + 1) * s_pad;         // [kMaskRows][cols4]
+  float *fo = reinterpret_cast<float *>(smem_raw);  // [mask_rows + 1][s_pad]
+  float *bo = fo + (mask_rows + 1) * s_pad;         // [mask_rows + 1][s_pad]
+  float *lp = bo + (mask_rows + 1) * s_pad;         // [mask_rows][cols4]
   const float cutoff = cutoffs[i];
   const float *fgrid = vfwd + f.grid_off, *bgrid = vbwd + f.grid_off;
   for (int32_t idx = tid; idx < (nf + 1) * S; idx += nt) {
@@ -524,7 +525,6 @@ ArcMasks(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_levels,
     return *reinterpret_cast<const float *>(base + off);
   };
   constexpr int kUnroll = 4;
-  static_assert(kMaskRows % kUnroll == 0, "rows per CTA");
   // One body per direction and per way to read the dense scores: with the direction tested per
   // arc both orders of the sum were formed and one was selected.
   auto rows = [&](auto forward, auto one_column) {
@@ -1696,6 +1696,20 @@ static bool LossFits(const LossLayout &LL, const k2b200_intersect_args *a, Chain
          a->cols < 32768 && LL.base.max_states < 65536;
 }
 
+// ArcMasks: the state pitch of the staged Viterbi scores, in four sizes, and the rows per CTA (a
+// multiple of four): fewer where the rows of dense scores are long.
+static int32_t MaskPitch(int32_t max_states) {
+  return max_states <= 192 ? 192 : max_states <= 384 ? 384 : max_states <= 768 ? 768 : 1024;
+}
+static size_t MaskSmem(int32_t max_states, int32_t rows, const DensePack &d) {
+  return sizeof(float) * ((size_t)2 * (rows + 1) * MaskPitch(max_states) + (size_t)rows * d.cols4);
+}
+static int32_t MaskRows(int32_t max_states, const DensePack &d) {
+  int32_t rows = max_states <= 192 ? 56 : max_states <= 384 ? 32 : 16;
+  while (rows > 4 && MaskSmem(max_states, rows, d) > kChainSmemBudget) rows -= 4;
+  return rows;
+}
+
 template <int kDeg, int kMaxThreads, int kU>
 static int32_t LaunchChainLanes(const LossLayout &LL, const k2b200_intersect_args *args, char *ws,
                                 const LaneSmem &ls, double *tot, cudaStream_t stream) {
@@ -1733,25 +1747,25 @@ static int32_t LaunchChainMasked(const LossLayout &LL, const k2b200_intersect_ar
   int32_t *unfit = reinterpret_cast<int32_t *>(ws + L.off_unfit);
   unsigned char *masks = reinterpret_cast<unsigned char *>(ws + LL.off_masks);
   {
-#define K2B_ARC_MASKS(SPAD, ROWS)                                                              \
-    {                                                                                          \
-      const size_t smem = sizeof(float) * ((size_t)2 * ((ROWS) + 1) * (SPAD) +                 \
-                                           (size_t)(ROWS) * LL.pack.cols4);                    \
-      K2B_REQUIRE(smem <= kChainSmemBudget, "too many columns for the fused loss path");       \
-      K2B_CUDA_OK(cudaFuncSetAttribute(ArcMasks<kLaneDeg, kThreads, SPAD, ROWS>,                         \
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize,            \
-                                       (int)smem));                                            \
-      dim3 grid(CeilDiv(L.max_tk + 1, (ROWS)), args->num_fsas, 2);                             \
-      { ArcMasks<kLaneDeg, kThreads, SPAD, ROWS><<<grid, kThreads, smem, stream>>>(                  \
-          d_infos, args->num_fsas, L.total_levels, arcs, args->a_row_splits2,                  \
-          args->a_in_splits, args->a_in_arcs, dense, LL.pack, fwd, bwd, cutoffs, plan, unfit,  \
-          masks, LL.threads); NoteLaunch(); }                                                  \
+    const int32_t rows = MaskRows(L.max_states, LL.pack);
+    const size_t smem = MaskSmem(L.max_states, rows, LL.pack);
+    K2B_REQUIRE(smem <= kChainSmemBudget, "too many columns for the fused loss path");
+#define K2B_ARC_MASKS(SPAD)                                                                   \
+    {                                                                                         \
+      K2B_CUDA_OK(cudaFuncSetAttribute(ArcMasks<kLaneDeg, kThreads, SPAD>,                    \
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize,           \
+                                       (int)smem));                                           \
+      dim3 grid(CeilDiv(L.max_tk + 1, rows), args->num_fsas, 2);                              \
+      { ArcMasks<kLaneDeg, kThreads, SPAD><<<grid, kThreads, smem, stream>>>(                 \
+          d_infos, args->num_fsas, L.total_levels, arcs, args->a_row_splits2,                 \
+          args->a_in_splits, args->a_in_arcs, dense, LL.pack, fwd, bwd, cutoffs, plan, unfit, \
+          masks, LL.threads, rows); NoteLaunch(); }                                           \
     }
-    // state pitch of the staged Viterbi scores, in three sizes
-    if (L.max_states <= 192) K2B_ARC_MASKS(192, 56)
-    else if (L.max_states <= 384) K2B_ARC_MASKS(384, 32)
-    else if (L.max_states <= 768) K2B_ARC_MASKS(768, 16)
-    else K2B_ARC_MASKS(1024, 16)
+    const int32_t s_pad = MaskPitch(L.max_states);
+    if (s_pad == 192) K2B_ARC_MASKS(192)
+    else if (s_pad == 384) K2B_ARC_MASKS(384)
+    else if (s_pad == 768) K2B_ARC_MASKS(768)
+    else K2B_ARC_MASKS(1024)
 #undef K2B_ARC_MASKS
   }
   {

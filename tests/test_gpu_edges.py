@@ -166,6 +166,33 @@ def test_lane_plans(k2, phones):
     assert np.abs(got[0][1] - got[1][1]).max() <= 1e-4
 
 
+@pytest.mark.parametrize("classes", [613, 614, 1363, 1364, 2047, 4000])
+def test_lane_plans_with_many_classes(k2, classes):
+    """Rows of dense scores that leave shared memory fewer frames per CTA: 56 up to 614 columns of
+    the score matrix, 32 up to 1364."""
+    from k2_b200 import synthetic as syn
+    rs2, arcs = syn.den_graph(20, 20)
+    rng = np.random.default_rng(classes)
+    lp = torch.log_softmax(torch.from_numpy(
+        rng.normal(size=(2, 70, classes)).astype(np.float32)), -1).to(DEV)
+    seg = torch.tensor([[0, 0, 70], [1, 0, 61]], dtype=torch.int32)
+    graphs = syn.build_graphs(syn.Workload("lfmmi", lp.cpu(), seg, 8.0, graph_row_splits2=rs2,
+                                           graph_arcs=arcs, num_symbols=None), DEV)
+    got = []
+    for fused in (True, False):
+        x = lp.clone().requires_grad_(True)
+        dense = k2.DenseFsaVec(x, seg)
+        assert k2.autograd.dense_loss_supported(graphs, dense)
+        if fused:
+            tot = k2.intersect_dense_tot_scores(graphs, dense, 8.0)
+        else:
+            tot = k2.intersect_dense(graphs, dense, 8.0).get_tot_scores(True, True)
+        tot.sum().backward()
+        got.append((tot.detach().cpu().numpy(), x.grad.cpu().numpy()))
+    assert close(got[0][0], got[1][0], rtol=1e-6, atol=1e-5)
+    assert np.abs(got[0][1] - got[1][1]).max() <= 1e-4
+
+
 # --------------------------------------------------------------------------- pruned search
 @pytest.mark.parametrize("states,classes,hub,n,teams", [
     (50, 5, 0, 1, (0, 1, 2, 8)),       # fewer arcs than a warp has lanes
