@@ -1684,18 +1684,6 @@ static int32_t MakeLossLayout(const k2b200_intersect_args *a, LossLayout *LL) {
   return kOk;
 }
 
-static bool LossFits(const LossLayout &LL, const k2b200_intersect_args *a, ChainPlan *p,
-                     LaneSmem *ls) {
-  *p = PlanChain(LL.base, a, LL.pack);
-  // the deep ring when it fits (identity lanes only), else two slots
-  *ls = PlanLaneSmem(LL.base, LL.pack, kChainGroup);
-  if (!LL.identity || ls->stages == 0) *ls = PlanLaneSmem(LL.base, LL.pack, kChainGroupSmall);
-  const bool lanes_ok = LL.base.lane_plan ||
-                        (a->a_max_degree > 0 && a->a_max_degree <= 4 && LL.base.max_states <= 1024);
-  return lanes_ok && p->stages >= 2 && ls->stages >= 2 && a->num_fsas <= 65535 &&
-         a->cols < 32768 && LL.base.max_states < 65536;
-}
-
 // ArcMasks: the state pitch of the staged Viterbi scores, in four sizes, and the rows per CTA (a
 // multiple of four): fewer where the rows of dense scores are long.
 static int32_t MaskPitch(int32_t max_states) {
@@ -1708,6 +1696,28 @@ static int32_t MaskRows(int32_t max_states, const DensePack &d) {
   int32_t rows = max_states <= 192 ? 56 : max_states <= 384 ? 32 : 16;
   while (rows > 4 && MaskSmem(max_states, rows, d) > kChainSmemBudget) rows -= 4;
   return rows;
+}
+
+// GridChainMasked: the ring of kMaskedBatches batches of `frames` frames and the values.
+static size_t MaskedSmem(const DensePack &d, int32_t threads, int32_t frames) {
+  return (size_t)kMaskedBatches * frames * ((size_t)d.pitch + threads) +
+         sizeof(double) * 2 * (size_t)threads;
+}
+
+static bool LossFits(const LossLayout &LL, const k2b200_intersect_args *a, ChainPlan *p,
+                     LaneSmem *ls) {
+  *p = PlanChain(LL.base, a, LL.pack);
+  // the deep ring when it fits (identity lanes only), else two slots
+  *ls = PlanLaneSmem(LL.base, LL.pack, kChainGroup);
+  if (!LL.identity || ls->stages == 0) *ls = PlanLaneSmem(LL.base, LL.pack, kChainGroupSmall);
+  const bool lanes_ok = LL.base.lane_plan ||
+                        (a->a_max_degree > 0 && a->a_max_degree <= 4 && LL.base.max_states <= 1024);
+  const int32_t states = LL.base.max_states;
+  const bool masks_ok =
+      LL.identity || (MaskSmem(states, MaskRows(states, LL.pack), LL.pack) <= kChainSmemBudget &&
+                      MaskedSmem(LL.pack, LL.threads, 1) <= kChainSmemBudget);
+  return lanes_ok && masks_ok && p->stages >= 2 && ls->stages >= 2 && a->num_fsas <= 65535 &&
+         a->cols < 32768 && states < 65536;
 }
 
 template <int kDeg, int kMaxThreads, int kU>
@@ -1749,7 +1759,6 @@ static int32_t LaunchChainMasked(const LossLayout &LL, const k2b200_intersect_ar
   {
     const int32_t rows = MaskRows(L.max_states, LL.pack);
     const size_t smem = MaskSmem(L.max_states, rows, LL.pack);
-    K2B_REQUIRE(smem <= kChainSmemBudget, "too many columns for the fused loss path");
 #define K2B_ARC_MASKS(SPAD)                                                                   \
     {                                                                                         \
       K2B_CUDA_OK(cudaFuncSetAttribute(ArcMasks<kLaneDeg, kThreads, SPAD>,                    \
@@ -1772,8 +1781,7 @@ static int32_t LaunchChainMasked(const LossLayout &LL, const k2b200_intersect_ar
     dim3 grid(2, args->num_fsas);
 #define K2B_CHAIN_MASKED(KU)                                                                  \
     {                                                                                         \
-      const size_t smem = (size_t)kMaskedBatches * (KU) * ((size_t)LL.pack.pitch + kThreads) + \
-                          sizeof(double) * 2 * kThreads;                                  \
+      const size_t smem = MaskedSmem(LL.pack, kThreads, KU);                                  \
       K2B_CUDA_OK(cudaFuncSetAttribute(GridChainMasked<kLaneDeg, kThreads, KU>,                         \
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,           \
                                        (int)smem));                                           \
@@ -1787,11 +1795,8 @@ static int32_t LaunchChainMasked(const LossLayout &LL, const k2b200_intersect_ar
     }
     // frames per batch (one bulk copy of dense rows and one of mask rows each): as many as
     // three batches of them leave room for in shared memory
-    const size_t per_frame = (size_t)kMaskedBatches * ((size_t)LL.pack.pitch + kThreads);
-    const size_t room = kChainSmemBudget - sizeof(double) * 2 * kThreads;
-    K2B_REQUIRE(per_frame <= room, "too many columns for the fused loss path");
-    if (4 * per_frame <= room) K2B_CHAIN_MASKED(4)
-    else if (2 * per_frame <= room) K2B_CHAIN_MASKED(2)
+    if (MaskedSmem(LL.pack, kThreads, 4) <= kChainSmemBudget) K2B_CHAIN_MASKED(4)
+    else if (MaskedSmem(LL.pack, kThreads, 2) <= kChainSmemBudget) K2B_CHAIN_MASKED(2)
     else K2B_CHAIN_MASKED(1)
 #undef K2B_CHAIN_MASKED
   }
@@ -1809,6 +1814,9 @@ static int32_t LaunchGrad(const LossLayout &LL, const k2b200_intersect_args *arg
   // frames per CTA: the chunk's rows of the dense gradient live in shared memory
   int32_t frames = 32;
   while (frames > kGradWarps && sizeof(float) * (size_t)frames * args->cols > 48 * 1024)
+    frames >>= 1;
+  // (fewer than warps where even those rows are too long)
+  while (frames > 1 && nb_bytes + sizeof(float) * ((size_t)frames * args->cols + 3) > kChainSmemBudget)
     frames >>= 1;
   const size_t gb_bytes = sizeof(float) * (((size_t)frames * args->cols + 3) & ~(size_t)3);
   const size_t ga_bytes = sizeof(float) * (size_t)L.max_arcs;

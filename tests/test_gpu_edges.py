@@ -193,6 +193,46 @@ def test_lane_plans_with_many_classes(k2, classes):
     assert np.abs(got[0][1] - got[1][1]).max() <= 1e-4
 
 
+@pytest.mark.parametrize("states,classes", [(40, 6016), (40, 6017), (40, 9000), (300, 7700)])
+def test_lane_per_state_with_many_classes(k2, states, classes):
+    """Graphs of at most four arcs per state that are no band graphs; rows so long that the kernels of
+    the gradient take fewer of them than they have warps."""
+    from gpu_util import host_to_fsa
+    rng = np.random.default_rng(classes)
+    rows = []
+    for s in range(states - 1):
+        for d in (0, 1, 2):
+            if s + d < states:
+                final = s + d == states - 1
+                rows.append((s, s + d, -1 if final else int(rng.integers(0, classes)), rng.normal()))
+    r = np.array(rows)
+    rs2 = np.zeros(states + 1, np.int64)
+    np.add.at(rs2, r[:, 0].astype(np.int64) + 1, 1)
+    graph = host_to_fsa(HostFsaVec(
+        np.array([0, states], np.int32), np.cumsum(rs2).astype(np.int32),
+        make_arcs(r[:, 0].astype(np.int32), r[:, 1].astype(np.int32), r[:, 2].astype(np.int32),
+                  r[:, 3].astype(np.float32))))
+    frames = states
+    lp = torch.log_softmax(torch.from_numpy(
+        rng.normal(size=(1, frames, classes)).astype(np.float32)), -1).to(DEV)
+    seg = torch.tensor([[0, 0, frames]], dtype=torch.int32)
+    got = []
+    for fused in (True, False):
+        x = lp.clone().requires_grad_(True)
+        dense = k2.DenseFsaVec(x, seg)
+        assert not k2.autograd.band_loss_supported(graph, dense)
+        if fused:
+            tot = k2.intersect_dense_tot_scores(graph, dense, 10.0)
+        else:
+            tot = k2.intersect_dense(graph, dense, 10.0).get_tot_scores(True, True)
+        assert torch.isfinite(tot).all()
+        tot.sum().backward()
+        got.append((tot.detach().cpu().numpy(), x.grad.cpu().numpy()))
+    assert close(got[0][0], got[1][0], rtol=1e-6, atol=1e-5)
+    # (scores of a few hundred: the lattice rounds each arc's to float32)
+    assert np.abs(got[0][1] - got[1][1]).max() <= 1e-4
+
+
 # --------------------------------------------------------------------------- pruned search
 @pytest.mark.parametrize("states,classes,hub,n,teams", [
     (50, 5, 0, 1, (0, 1, 2, 8)),       # fewer arcs than a warp has lanes

@@ -385,3 +385,26 @@ def test_host_layer_is_stale_under_another_torch_or_python(monkeypatch):
     with monkeypatch.context() as m:
         m.setattr(build.sys, "version", "3.9")
         assert build._host_stale(command)
+
+
+@pytest.mark.parametrize("degree,states,arcs,columns,supported", [
+    (50, 144, 600, 1364, True),     # planned lanes
+    (50, 144, 600, 5700, True),     # the most columns of which three rows fit in the ring
+    (50, 144, 600, 5900, False),
+    (50, 1000, 2000, 5000, True),
+    (3, 144, 300, 8700, True),      # a lane per state
+    (3, 144, 300, 8900, False),
+])
+def test_what_the_lattice_free_loss_takes(degree, states, arcs, columns, supported):
+    """k2b200_dense_loss_supported says what the launches can do."""
+    from k2_b200 import _lib
+    rs1, arc_splits = np.array([0, states], np.int32), np.array([0, arcs], np.int32)
+    rows = np.array([0, 11], np.int32)
+    args = _lib.IntersectArgs(
+        num_fsas=1, num_states=states, num_arcs=arcs, h_a_row_splits1=rs1.ctypes.data,
+        h_a_arc_splits=arc_splits.ctypes.data, rows=11, cols=columns, num_seqs=1,
+        h_b_row_splits=rows.ctypes.data, output_beam=8.0, max_states=1 << 30, max_arcs=1 << 30,
+        a_max_degree=degree)
+    got = ctypes.c_int32(-1)
+    _lib.check(_lib.lib.k2b200_dense_loss_supported(ctypes.byref(args), ctypes.byref(got)))
+    assert bool(got.value) == supported
