@@ -324,9 +324,13 @@ int32_t LaneThreads(const Layout &L) {
   return L.max_states + L.max_arcs / kLaneDeg <= 736 ? 768 : 1024;
 }
 
+constexpr int kVitRing = 4;   // slots of LanesViterbi's row ring = frames per unrolled group
+constexpr size_t kVitRingBytes = 200 * 1024;
+
 bool LanePlanApplies(const Layout &L, const k2b200_intersect_args *a) {
   const bool register_fit = a->a_max_degree > 0 && a->a_max_degree <= 4 && L.max_states <= 1024;
   return !register_fit && L.max_states <= kLaneThreads && a->num_fsas <= 65535 &&
+         sizeof(float) * kVitRing * ((size_t)a->cols + 3) <= kVitRingBytes &&
          PersistentViterbiFits(L, a);
 }
 
@@ -356,7 +360,6 @@ int32_t LaunchPlanLanes(const Layout &L, const k2b200_intersect_args *a, char *w
 // monotonic, so max_j fl(y_j + x) = fl(max_j y_j + x), bit for bit.
 // Graphs marked unfit are skipped (PersistentViterbi handles them).
 // ---------------------------------------------------------------------------
-constexpr int kVitRing = 4;   // slots of the row ring = frames per unrolled group
 constexpr int kVitAhead = 3;  // rows requested ahead of the frame that uses them
 
 // kPitch: floats of a ring slot, 0: cols_pad of them.  With a constant pitch every access of the
@@ -506,7 +509,7 @@ int32_t LaunchLanesViterbi(const Layout &L, const k2b200_intersect_args *a,
   const int32_t cols_pad = (a->cols + 3) & ~3;
   auto launch = [&](auto kernel, int32_t threads, int32_t pitch) -> int32_t {
     const size_t smem = sizeof(float) * kVitRing * (size_t)pitch;
-    K2B_REQUIRE(smem <= 200 * 1024, "too many columns for the lane Viterbi kernel");
+    K2B_REQUIRE(smem <= kVitRingBytes, "too many columns for the lane Viterbi kernel");
     K2B_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem));
     kernel<<<grid, threads, smem, stream>>>(

@@ -193,6 +193,21 @@ def test_lane_plans_with_many_classes(k2, classes):
     assert np.abs(got[0][1] - got[1][1]).max() <= 1e-4
 
 
+@pytest.mark.parametrize("classes", [12796, 12800, 20000])
+def test_lattice_of_many_classes(k2, classes):
+    """Around the most columns of which four rows fit in the ring of the lane kernel."""
+    from gpu_util import dense_from_scores, fsa_to_host, host_to_fsa, intersect_raw
+    from k2_b200 import synthetic as syn
+    rs2, arcs = syn.den_graph(8, 8)
+    a = HostFsaVec(np.array([0, len(rs2) - 1], np.int32), rs2, arcs)
+    scores, brs = random_dense(np.random.default_rng(classes), 1, 12, classes)
+    want = oracle.intersect_dense(a, scores, brs, 6.0)
+    fsa = host_to_fsa(a)
+    assert fsa.arcs.max_degree() > 4
+    lattice, ma, mb = intersect_raw(fsa, dense_from_scores(scores, brs), 6.0)
+    same_fsa(fsa_to_host(lattice, ma, mb), want, f"{classes} classes")
+
+
 @pytest.mark.parametrize("states,classes", [(40, 6016), (40, 6017), (40, 9000), (300, 7700)])
 def test_lane_per_state_with_many_classes(k2, states, classes):
     """Graphs of at most four arcs per state that are no band graphs; rows so long that the kernels of
