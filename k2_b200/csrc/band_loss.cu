@@ -1937,7 +1937,7 @@ static int32_t MakeBandLayout(const k2b200_band_loss_args *a, BandLayout *L) {
     L->why = "a graph has more than 1024 states";
   } else if (L->chain_smem > kBandSmemBudget || L->exact_smem > kBandSmemBudget) {
     L->ok = false;
-    L->why = "too many frames, states or classes for the shared memory of the recursions";
+    L->why = "too many frames or states for the shared memory of the recursions";
   } else if (L->max_frames + 2 > kChainMaxChunks * kPrepLevels) {
     L->ok = false;
     L->why = "a sequence has more than 65534 frames";

@@ -94,7 +94,9 @@ int32_t MakeLayout(const k2b200_intersect_args *a, Layout *L) {
   // arcs per state differ in what they cost, by up to the hundreds of arcs of one: shorter runs
   // of them even out (5 words -> 1 of an LF-MMI denominator, 16 x 300 frames: CountKept 110 ->
   // 99 us, EmitLattice 174 -> 139; the sparse words of alignment graphs lost by it, 22 -> 35
-  // and 21 -> 29).
+  // and 21 -> 29).  Both together for random graphs of 4 500 arcs, 16 x 300 frames, long and
+  // short runs: 253 and 233 us at 16 arcs per state, 231 and 220 at 12, 206 and 205 at 9, 192
+  // and 196 at 7, 146 and 157 at 3.4.
   int64_t max_pair_words = 0;
   for (const FsaInfo &f : L->infos)
     max_pair_words = std::max<int64_t>(max_pair_words, (int64_t)(f.tk + 1) * f.words);
