@@ -16,8 +16,8 @@ every rank runs its own batch (weak scaling, utterances are independent) and the
 only collective is one all-reduce of [loss, frames].
 
 --impl reference times the reference's own CPU code for the same path
-(oracle/_ref/libk2ref.so when present, else the C restatement in oracle/) on the
-host cores, single-threaded as the reference is by construction.
+(oracle/_ref/libk2ref.so) on the host cores, single-threaded as the reference is by
+construction; where that library is not built it says so.
 
 Diagnostics of the N > 1 arm (environment): K2B_NCCL_REDUCE=1 exchanges [loss, frames]
 with torch.distributed on a helper thread instead of the peer-memory kernel,
@@ -265,12 +265,20 @@ def cpu_reference_sharded(w, graphs, scores, row_splits, impl_mod, cores, repeat
     return best, len(shards)
 
 
+UNAVAILABLE = {"impl": "reference",
+               "unavailable": "the reference's CPU library (oracle/_ref/libk2ref.so) is not built: "
+                              "it is compiled from the reference's sources"}
+
+
 def run_reference(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return
-    w = make_workload(args, 0)
     impl_mod, kind = pick_cpu_impl()
+    if kind != "reference":
+        print(json.dumps(UNAVAILABLE))
+        return
+    w = make_workload(args, 0)
     graphs, scores, row_splits = host_inputs(w, impl_mod)
     frames = w.num_frames
     # single thread, as the reference runs this path
@@ -601,12 +609,11 @@ def run_ours(args):
         pass
     hbm_peak = float(peaks.get("hbm_gbs", 6650.0))
     peak_src = "measured" if "hbm_gbs" in peaks else "fallback"
-    # the dominant phase of the timed region carries the roofline figure: the path's
-    # algorithmic bytes per launch (one launch of it per step) over its duration
+    # roofline: the path's algorithmic bytes over the time of all its kernels; beside it the
+    # kernel that takes longest, with the bytes it moves by its design
     top = max(phases, key=lambda k: phases[k][0])
-    top_ms, top_n = phases[top]
-    top_avg_ms = top_ms / args.steps
-    achieved = b_alg / (top_avg_ms * 1e-3) / 1e9 if top_avg_ms > 0 else 0.0
+    top_avg_ms = phases[top][0] / args.steps
+    achieved = b_alg / (busy * 1e-3) / 1e9 if busy > 0 else 0.0
     impl_b = implementation_bytes(top, kernels[top], frames, N, T, C, A, A_out, S_out, grid_states)
     # dram read + write of one launch from the ncu capture of this workload (profiles/)
     traffic = None
@@ -655,17 +662,17 @@ def run_ours(args):
                     "grid_states": grid_states},
         "roofline": {"kernel": kernels[top], "bound": "hbm", "achieved": achieved,
                      "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
-                     "peak_source": peak_src, "algorithmic_bytes_per_launch": b_alg,
-                     "avg_launch_ms": top_avg_ms, "traffic": traffic,
+                     "peak_source": peak_src, "algorithmic_bytes_per_step": b_alg,
+                     "kernel_ms_per_step": busy, "avg_launch_ms": top_avg_ms, "traffic": traffic,
                      # what the kernel moves by its design over its time: DRAM utilisation,
                      # not a roofline fraction
                      "dram_utilisation": None if not impl_b or top_avg_ms <= 0 else
                      impl_b / (top_avg_ms * 1e-3) / 1e9 / hbm_peak,
                      "implementation_bytes_per_launch": impl_b,
                      "note": "latency-bound: a chain of T dependent frames per utterance; "
-                             "achieved = the path's algorithmic bytes per step over the "
-                             "dominant kernel's launch; traffic = ncu dram read+write of one "
-                             "launch on this workload (profiles/)"},
+                             "achieved = the path's algorithmic bytes per step over the time of "
+                             "all its kernels; kernel = the one that takes longest, traffic = "
+                             "ncu dram read+write of one launch of it (profiles/)"},
         # value: the copy of step k+1 overlaps step k (k2_b200.parallel.HostPrefetcher), as
         # a training loop feeds the GPU; serial_value: copy, compute and read-back of one
         # step strictly after one another.  The loss (8 bytes) is read back every step;
@@ -728,17 +735,18 @@ def run_decode(args):
               "classes": int(w.log_probs.shape[2]), "graph_states": S,
               "graph_arcs": int(len(w.graph_arcs)), **DECODE_PARAMS}
     if args.impl == "reference":
-        from oracle import oracle, ref
+        from oracle import ref
         from oracle.common import HostFsaVec
-        # the reference's own code when it has been compiled, else its C restatement
-        impl, kind = (ref, "reference") if ref.available() else (oracle, "port")
+        if not ref.available():
+            print(json.dumps(UNAVAILABLE))
+            return
         m = min(n, 2)
         scores, row_splits = host_scores(w)
         rows = int(row_splits[m])
         a = HostFsaVec(np.array([0, S], np.int32), w.graph_row_splits2.astype(np.int32),
                        w.graph_arcs)
         t0 = time.perf_counter()
-        lat = impl.intersect_dense_pruned(a, scores[:rows], row_splits[:m + 1],
+        lat = ref.intersect_dense_pruned(a, scores[:rows], row_splits[:m + 1],
                                           *DECODE_PARAMS.values())
         dt = time.perf_counter() - t0
         print(json.dumps({"metric": "decode_frames_per_sec", "impl": "reference",
@@ -746,7 +754,7 @@ def run_decode(args):
                           "ms_per_step": dt * 1e3 * n / m, "higher_is_better": True,
                           "config": config,
                           "cpu_baseline": {"value": m * t / dt, "unit": "frames/s", "cores": 1,
-                                           "kind": kind,
+                                           "kind": "reference",
                                            "sample": f"{m} of {n} sequences, lattice only "
                                                      f"({lat.num_arcs} arcs)"}}))
         return
