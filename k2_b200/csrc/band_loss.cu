@@ -308,11 +308,30 @@ BandGather(const BandInfo *__restrict__ infos, const BandState *__restrict__ tab
   }
 }
 
+// A batch of rows [off, end), in floats from the 16-byte boundary src.  Where the copy between
+// boundaries would leave the matrix [first, last), up to three elements are copied one by one.
+__device__ __forceinline__ void CopyAtEdge(const float *first, const float *last, const float *src,
+                                        int32_t off, int32_t end, float *dst, uint64_t *bar) {
+  int32_t from = 0, to = (end + 3) & ~3;
+  if (src < first || src + to > last) {
+    if (src < first) from = 4;
+    if (src + to > last) to = max(to - 4, from);
+    for (int32_t k = off; k < min(from, end); ++k) dst[k] = src[k];
+    for (int32_t k = max(to, off); k < end; ++k) dst[k] = src[k];
+    // (the slot's next batch overwrites them)
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  MbarArriveExpectTx(bar, (unsigned)(to - from) * 4u);
+  if (to > from) BulkCopyG2S(dst + from, src + from, (unsigned)(to - from) * 4u, bar);
+}
+
 // kByState: `lp` holds scores by state (BandGather) in the layout of the grids instead of
 // log-prob rows of C columns: a thread reads its states' scores in one word.  With 5000 columns
 // the copies of whole rows bounded the kernel (170 us for 500 frames); by state it takes 43,
 // and BandGather 36.
-template <bool kByState>
+// kEdge: the matrix starts or ends between two 16-byte boundaries.  (An instance of its own: a test
+// per batch in the other one took 5 us of 1000 frames.)
+template <bool kByState, bool kEdge>
 __global__ void __launch_bounds__(64 * kVitMaxWarps, 1)
 BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ tab,
             const float *__restrict__ lp, int64_t lp_rows, int32_t C, float *__restrict__ vf,
@@ -343,8 +362,8 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
   const int32_t num_batches = (T + F - 1) / F;
   const float *lp0 = kByState ? lp + f.grid_off : lp + (int64_t)f.lp_row * C;
   // A row may start anywhere (C need not be a multiple of four): a batch is copied from the
-  // 16-byte boundary at or before its first element to the one at or after its last.  At the ends
-  // of the matrix that may lie outside it: there the last elements are copied one by one.
+  // 16-byte boundary at or before its first element to the one at or after its last (which kEdge
+  // keeps inside the matrix).
   const uint32_t lp0_words = (uint32_t)(reinterpret_cast<uintptr_t>(lp0) >> 2);
   auto words_off = [&](int32_t r) {
     return kByState ? 0 : (int32_t)((lp0_words + (uint32_t)r * (uint32_t)width) & 3u);
@@ -357,22 +376,16 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
     const int32_t r0 = dir == 0 ? q * F : max(T - (q + 1) * F, 0);
     const int32_t r1 = dir == 0 ? min((q + 1) * F, T) : T - q * F;
     const int32_t off = words_off(r0);
-    // in floats from the first boundary: the batch is [off, end), [from, to) goes as one copy
-    const int32_t end = (r1 - r0) * width + off;
-    int32_t from = 0, to = (end + 3) & ~3;
     const int32_t slot = q % nbatch;
-    float *dst = ring + (size_t)slot * slot_floats;
-    const float *src = lp0 + (int64_t)r0 * width - off;
-    if (!kByState && (src < lp || src + to > lp + lp_rows * width)) {
-      if (src < lp) from = 4;
-      if (src + to > lp + lp_rows * width) to = max(to - 4, from);
-      for (int32_t k = off; k < min(from, end); ++k) dst[k] = src[k];
-      for (int32_t k = max(to, off); k < end; ++k) dst[k] = src[k];
-      // (the slot's next batch overwrites them)
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    if (kEdge) {
+      CopyAtEdge(lp, lp + lp_rows * width, lp0 + (int64_t)r0 * width - off, off,
+                 (r1 - r0) * width + off, ring + (size_t)slot * slot_floats, &full[slot]);
+    } else {
+      const unsigned bytes = (((unsigned)(r1 - r0) * (unsigned)width + (unsigned)off + 3u) & ~3u) * 4u;
+      MbarArriveExpectTx(&full[slot], bytes);
+      BulkCopyG2S(ring + (size_t)slot * slot_floats, lp0 + (int64_t)r0 * width - off, bytes,
+                  &full[slot]);
     }
-    MbarArriveExpectTx(&full[slot], (unsigned)(to - from) * 4u);
-    if (to > from) BulkCopyG2S(dst + from, src + from, (unsigned)(to - from) * 4u, &full[slot]);
     ++issued;
   };
   if (tid == 0)
@@ -2180,7 +2193,12 @@ int32_t k2b200_band_loss_forward_reduce(const k2b200_band_loss_args *args, void 
                                              reinterpret_cast<float *>(ws + L.off_by_state));
         NoteLaunch(); }
     }
-    auto kernel = L.by_state ? BandViterbi<true> : BandViterbi<false>;
+    const uintptr_t lp_begin = reinterpret_cast<uintptr_t>(args->log_probs),
+                    lp_end = lp_begin + sizeof(float) * (size_t)args->log_prob_rows *
+                                            (size_t)args->num_classes;
+    auto kernel = L.by_state                  ? BandViterbi<true, false>
+                  : ((lp_begin | lp_end) & 15) ? BandViterbi<false, true>
+                                               : BandViterbi<false, false>;
     K2B_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)L.viterbi_smem));
     dim3 grid(2, args->num_fsas);
