@@ -125,8 +125,11 @@ def test_ctc_loss_on_the_band_kernels(k2, n, frames, classes, tokens, modified, 
             finally:
                 module.FUSED_LOSS = True
             got.append((loss.item(), leaf.grad.cpu().numpy()))
-        assert close(got[0][0], got[1][0], rtol=1e-5, atol=1e-4)
-        assert np.abs(got[0][1] - got[1][1]).max() <= 1e-4
+        # Totals in double, four of them added in float32: 4 x 2^-24.  The lattice adds at most 128
+        # posteriors of a frame and label in float32 (128 x 2^-24); with a penalty it also rounds
+        # the score of every arc.
+        assert close(got[0][0], got[1][0], rtol=1e-4 if delay else 3e-7, atol=1e-6)
+        assert np.abs(got[0][1] - got[1][1]).max() <= (1e-4 if delay else 1e-5)
 
 
 @pytest.mark.parametrize("modified", [False, True])
@@ -496,3 +499,30 @@ def test_captured_calls_keep_off_the_pool(k2, band):
         want = step(x.requires_grad_(True))
         assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
     assert bool((held == 3.0).all())
+
+
+# --------------------------------------------------------------------------- streaming
+def test_chunks_give_the_best_path_of_the_whole(k2):
+    """Streams of 48 frames in chunks of 16 with beams that prune next to nothing: the best path of
+    the last lattice has the score of the best path of the whole utterance."""
+    from gpu_util import host_to_fsa
+    rng = np.random.default_rng(23)
+    graph = host_to_fsa(decoding_graph(rng, 400, 12, mean_degree=3.0))
+    lp = torch.log_softmax(torch.from_numpy(
+        rng.normal(size=(3, 48, 12)).astype(np.float32) * 2.0), -1).to(DEV)
+    beams = (60.0, 50.0, 0, 10000)
+    decoder = k2.OnlineDenseIntersecter(graph, 3, *beams)
+    states = [None] * 3
+    seg = torch.tensor([[i, 0, 16] for i in range(3)], dtype=torch.int32)
+    for c in range(3):
+        chunk = lp[:, 16 * c:16 * (c + 1)].contiguous()
+        lattice, states = decoder.decode(k2.DenseFsaVec(chunk, seg), states)
+    whole = k2.intersect_dense_pruned(
+        graph, k2.DenseFsaVec(lp, torch.tensor([[i, 0, 48] for i in range(3)], dtype=torch.int32)),
+        *beams)
+    got = k2.shortest_path(lattice, use_double_scores=True)
+    want = k2.shortest_path(whole, use_double_scores=True)
+    assert torch.equal(got.arcs._row_splits2, want.arcs._row_splits2)
+    assert torch.equal(got.labels, want.labels)
+    # (arc scores are float32 sums of the same two numbers)
+    assert torch.equal(got.scores, want.scores)
