@@ -658,8 +658,8 @@ __global__ void __launch_bounds__(32 * kPrepWarps, 3)
 BandPrep(const BandInfo *__restrict__ infos, const int32_t *__restrict__ a_row_splits2,
          const BandState *__restrict__ tab, const BandArc *__restrict__ tabf,
          const float *__restrict__ lp, int32_t C, const float *__restrict__ by_state,
-         const float *__restrict__ vf, const float *__restrict__ vb, float beam, BandItem *__restrict__ items,
-         BandFactor *__restrict__ factors, int2 *__restrict__ lists,
+         const float *__restrict__ vf, const float *__restrict__ vb, float beam,
+         BandItem *__restrict__ items, BandFactor *__restrict__ factors, int2 *__restrict__ lists,
          int32_t *__restrict__ chunk_r, unsigned long long *__restrict__ totals,
          int32_t *__restrict__ unfit, int32_t count_arcs, DelaySpec delay) {
   constexpr unsigned kAll = 0xffffffffu;
@@ -1834,9 +1834,9 @@ struct BandLayout {
   int32_t first_row = 0;
   int32_t st_pad = 0, lv_pad = 0;
   size_t chain_smem = 0, exact_smem = 0, viterbi_smem = 0, prep_smem = 0;
-  size_t off_infos, off_vf, off_vb, off_by_state, off_items, off_factors, off_lists, off_chunk_r, off_am, off_ae,
-      off_bm, off_be, off_penalty, off_a_scale, off_b_scale, off_total, off_unfit, off_totals, off_status,
-      total_bytes;  // off_status = off_totals + 40
+  size_t off_infos, off_vf, off_vb, off_by_state, off_items, off_factors, off_lists, off_chunk_r,
+      off_am, off_ae, off_bm, off_be, off_penalty, off_a_scale, off_b_scale, off_total, off_unfit,
+      off_totals, off_status, total_bytes;  // off_status = off_totals + 40
   bool ok = true;
   const char *why = "";
   bool exclusive_rows = true;  // no two graphs on one sequence (they would share gradient rows)
@@ -2260,8 +2260,8 @@ int32_t k2b200_band_loss_forward_reduce(const k2b200_band_loss_args *args, void 
       K2B_CUDA_OK(cudaGetLastError());
     }
     if (iter == 0 && args->zero_fill != nullptr && args->zero_fill_bytes > 0) {
-      // behind BandPrep, beside the recursions (one warp per graph and direction: the SMs
-      // are all but idle); joined below
+      // behind BandPrep, beside the recursions (up to four warps per graph and direction: the
+      // SMs are all but idle); joined below
       K2B_FORWARD(SideFork(stream, &side));
       K2B_CUDA_OK(cudaMemsetAsync(args->zero_fill, 0, args->zero_fill_bytes, side));
       join_side = true;

@@ -143,8 +143,8 @@ constexpr int32_t kMinExponent = -480;     // binary exponent of every non-zero 
 // ---------------------------------------------------------------------------
 // The alpha / beta recursion for graphs whose states have at most four arcs each
 // way (CTC): one thread per state, its arcs in registers.  grid = (2 directions,
-// pairs), one CTA walks all frames of its pair.  Per frame three bulk copies (issued kU - 1 frames ahead by
-// thread 0, completion on one mbarrier) bring the packed dense row and the two
+// pairs), one CTA walks all frames of its pair.  Per frame three bulk copies (issued kU - 1
+// frames ahead by thread 0, completion on one mbarrier) bring the packed dense row and the two
 // Viterbi rows of the level into a shared-memory ring of kU slots; every lane runs
 // the reference's pruning test (intersect_dense.cu:430-470) on its arcs with the
 // same fp32 expressions and adds the survivors' alpha[src] * exp(w) * exp(lp).
@@ -1043,8 +1043,8 @@ GridGradWarp(const FsaInfo *__restrict__ infos, const Arc *__restrict__ arcs,
 // of hundreds).  grid = (frame chunks, pairs).  The CTA first compacts the surviving
 // (frame, state) pairs of its frames into a list in shared memory - a coalesced scan
 // of the Viterbi grids by warps, positions from ballots and one shared counter (the
-// order of the list does not matter: the sums are integers) - and then spreads (survivor, arc) items over all its threads, so that the dependent
-// gathers of an arc (destination scores, beta, factors) of many arcs are in flight
+// order of the list does not matter: the sums are integers) - and then spreads
+// (survivor, arc) items over all its threads, so that the dependent gathers of an arc (destination scores, beta, factors) of many arcs are in flight
 // at once instead of one warp walking one frame.  Same fixed-point sums as
 // GridGradWarp.
 // ---------------------------------------------------------------------------
@@ -1786,14 +1786,14 @@ static int32_t LaunchChainMasked(const LossLayout &LL, const k2b200_intersect_ar
 #define K2B_CHAIN_MASKED(KU)                                                                  \
     {                                                                                         \
       const size_t smem = MaskedSmem(LL.pack, kThreads, KU);                                  \
-      K2B_CUDA_OK(cudaFuncSetAttribute(GridChainMasked<kLaneDeg, kThreads, KU>,                         \
+      K2B_CUDA_OK(cudaFuncSetAttribute(GridChainMasked<kLaneDeg, kThreads, KU>,               \
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,           \
                                        (int)smem));                                           \
-      { GridChainMasked<kLaneDeg, kThreads, KU><<<grid, kThreads, smem, stream>>>(                  \
+      { GridChainMasked<kLaneDeg, kThreads, KU><<<grid, kThreads, smem, stream>>>(            \
           d_infos, args->num_fsas, L.total_levels, arcs, args->a_row_splits2,                 \
           args->a_in_splits, args->a_in_arcs, dense, LL.pack, masks, fwd, bwd, cutoffs,       \
           reinterpret_cast<ProbState *>(ws + LL.off_alpha),                                   \
-          reinterpret_cast<ProbState *>(ws + LL.off_beta), tot, plan, unfit, LL.threads,                                   \
+          reinterpret_cast<ProbState *>(ws + LL.off_beta), tot, plan, unfit, LL.threads,      \
           CopyWaitLimit());                                                                   \
         NoteLaunch(); }                                                                       \
     }

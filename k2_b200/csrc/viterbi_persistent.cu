@@ -232,8 +232,9 @@ RegisterViterbi(const FsaInfo *__restrict__ infos, const Arc *__restrict__ arcs,
 // Lane plans.  The recursion kernel keeps the arcs of state s in the registers of
 // G(s) = ceil(degree(s) / kDeg) lanes of one warp, so that a frame costs every lane
 // the same few arcs whatever the degree distribution of the graph is.  PlanLanes
-// lays the lane groups of one graph and direction out over the threads of a CTA: groups sorted by size, largest first (states in increasing order within
-// a size), packed next-fit into warps - a group never straddles two warps.
+// lays the lane groups of one graph and direction out over the threads of a CTA: groups
+// sorted by size, largest first (states in increasing order within a size), packed
+// next-fit into warps - a group never straddles two warps.
 //   plan[(dir * n + i) * kLaneThreads + thread] = state | lane << 16 | G << 24, or -1
 // bit 0 of unfit[i] is set when graph i needs more lanes than a CTA has (or has more than
 // 32 * kDeg arcs on a state); the shared-memory kernels below take those graphs.

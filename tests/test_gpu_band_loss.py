@@ -512,3 +512,19 @@ def test_wide_vocabularies(classes, amap, layout):
             assert np.abs(gb - want_gb).max() <= 4e-5
         if graph_grad:
             assert np.abs(fsa.scores.grad.cpu().numpy() - want["grad_a"]).max() <= 1e-4
+
+
+def test_shared_rows_without_a_gradient():
+    """Two graphs on every sequence through the native call, which has no gradient for them."""
+    import k2_b200 as k2
+    from gpu_util import host_to_fsa
+    rng = np.random.default_rng(31)
+    a = random_band_graphs(rng, 4, 9, 8)
+    lp, seg = random_log_probs(rng, 2, 12, 8)
+    scores, brs = host_scores(lp, seg)
+    amap = np.array([0, 0, 1, 1], np.int32)
+    want = oracle.loss_path(a, scores, brs, 20.0, amap)["tot_scores"]
+    got = k2.intersect_dense_tot_scores(host_to_fsa(a), k2.DenseFsaVec(lp.to(DEV), seg), 20.0,
+                                        a_to_b_map=torch.from_numpy(amap))
+    assert got.grad_fn is None and np.isfinite(want).any()
+    assert close(got.cpu().numpy(), want, rtol=1e-6, atol=1e-6)

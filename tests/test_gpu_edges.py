@@ -144,6 +144,16 @@ def test_ctc_graph_on_the_device(k2, lengths, modified):
     assert torch.equal(got.aux_labels.cpu(), cpu.aux_labels)
 
 
+def test_ctc_graph_of_symbols_that_are_not_integers(k2):
+    """What the native conversion leaves to numpy: the kernels for symbols on the device."""
+    got = k2.ctc_graph([[1.0, 2.0, 2.0], [3.5], []], device=DEV)
+    want = k2.ctc_graph([[1, 2, 2], [3], []], device=DEV)
+    for a, b in ((got.arcs.values(), want.arcs.values()), (got.aux_labels, want.aux_labels),
+                 (got.arcs._row_splits1, want.arcs._row_splits1),
+                 (got.arcs._row_splits2, want.arcs._row_splits2)):
+        assert torch.equal(a, b)
+
+
 # --------------------------------------------------------------------------- planned lanes
 @pytest.mark.parametrize("phones", [40, 78, 80, 84, 105])  # around 768 and 1024 lanes
 def test_lane_plans(k2, phones):
@@ -213,8 +223,8 @@ def test_lattice_of_many_classes(k2, classes):
 
 @pytest.mark.parametrize("states,classes", [(40, 6016), (40, 6017), (40, 9000), (300, 7700)])
 def test_lane_per_state_with_many_classes(k2, states, classes):
-    """Graphs of at most four arcs per state that are no band graphs; rows so long that the kernels of
-    the gradient take fewer of them than they have warps."""
+    """Graphs of at most four arcs per state that are no band graphs; rows so long that the kernels
+    of the gradient take fewer of them than they have warps."""
     from gpu_util import host_to_fsa
     rng = np.random.default_rng(classes)
     rows = []
@@ -222,7 +232,8 @@ def test_lane_per_state_with_many_classes(k2, states, classes):
         for d in (0, 1, 2):
             if s + d < states:
                 final = s + d == states - 1
-                rows.append((s, s + d, -1 if final else int(rng.integers(0, classes)), rng.normal()))
+                label = -1 if final else int(rng.integers(0, classes))
+                rows.append((s, s + d, label, rng.normal()))
     r = np.array(rows)
     rs2 = np.zeros(states + 1, np.int64)
     np.add.at(rs2, r[:, 0].astype(np.int64) + 1, 1)
@@ -380,8 +391,8 @@ def test_gradients_that_are_not_finite(k2, upstream):
 
 
 def test_pruned_search_passes_by_scores_that_are_not_numbers(k2):
-    """A NaN among the scores costs the arcs that read it, not the utterance.  (On graphs in which the
-    arcs into a state have one label, so that a state whose arcs are NaN does not come up.)"""
+    """A NaN among the scores costs the arcs that read it, not the utterance.  (On graphs in which
+    the arcs into a state have one label, so that a state whose arcs are NaN does not come up.)"""
     from gpu_util import dense_from_scores, fsa_to_host, host_to_fsa
     from k2_b200.autograd import _intersect_dense_pruned_arcs
     rng = np.random.default_rng(17)
