@@ -89,7 +89,7 @@ def _make_intersect_args(a: RaggedArc, b: DenseFsaVec, a_to_b_map: Optional[torc
         a_max_degree=a.max_degree(),
         # one large graph copied once per sequence: read copy 0 only
         a_shared=int(h_map is None and a.replicated(SHARED_GRAPH_MIN_BYTES)))
-    return args, (h_rs1, h_as, h_map, in_splits, in_arcs, scores), dev, h_brs
+    return args, (h_rs1, h_as, h_map, in_splits, in_arcs, scores, h_brs), dev, h_brs
 
 
 def _intersect_dense_arcs(a: RaggedArc, b: DenseFsaVec, a_to_b_map: Optional[torch.Tensor],

@@ -537,3 +537,31 @@ def test_chunks_give_the_best_path_of_the_whole(k2):
     assert torch.equal(got.labels, want.labels)
     # (arc scores are float32 sums of the same two numbers)
     assert torch.equal(got.scores, want.scores)
+
+
+def test_backward_after_the_inputs_are_gone(k2):
+    """A loss keeps the host arrays that its backward reads: the DenseFsaVec and the map are dropped
+    and their memory is written over in between."""
+    from k2_b200 import synthetic as syn
+    rs2, arcs = syn.den_graph(20, 20)
+    seg = torch.tensor([[i, 0, 60 - i] for i in range(16)], dtype=torch.int32)
+    lp = torch.log_softmax(torch.randn(16, 60, 21, device=DEV), -1)
+    graphs = {"den": syn.build_graphs(syn.Workload("x", lp.cpu(), seg, 8.0, graph_row_splits2=rs2,
+                                                   graph_arcs=arcs, num_symbols=None), DEV),
+              "ctc": k2.ctc_graph([[1, 2, 3]] * 16, device=DEV)}
+    for name, graph in graphs.items():
+        for amap in (None, list(range(16))):
+            for band in (True, False):
+                grads = []
+                for drop in (False, True):
+                    x = lp.clone().requires_grad_(True)
+                    dense = k2.DenseFsaVec(x, seg)
+                    m = None if amap is None else torch.tensor(amap, dtype=torch.int32)
+                    tot = k2.intersect_dense_tot_scores(graph, dense, 8.0, a_to_b_map=m, band=band)
+                    if drop:
+                        del dense, m
+                        over = [np.full(n, -1, np.int32) for n in (16, 17) for _ in range(200)]
+                    tot.sum().backward()
+                    grads.append(x.grad)
+                del over
+                assert torch.equal(grads[0], grads[1]), (name, amap is None, band)
