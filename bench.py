@@ -711,8 +711,8 @@ def run_ours(args):
 
 
 # ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch on ctc_large (profiles/)
-NCU_TRAFFIC = {"BandViterbi": 287.8e6, "BandPrep": 259.1e6, "BandChainLists": 87.7e6,
-               "BandGradRows": 103.0e6}
+NCU_TRAFFIC = {"BandViterbi": 288.2e6, "BandPrep": 267.7e6, "BandChainLists": 98.9e6,
+               "BandGradRows": 109.0e6}
 
 
 # --------------------------------------------------------------------------- decoding
