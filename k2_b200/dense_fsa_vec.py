@@ -106,7 +106,8 @@ class DenseFsaVec(object):
             self._init(None, row_splits, device=log_probs.device, num_cols=C + 1)
             # (no closure over self: a reference cycle would keep the log-probs and
             # their gradient alive until the cycle collector runs)
-            self._make_scores = (fn, log_probs, eff, int(row_splits[-1]), overlapping)
+            self._make_scores = (fn, log_probs, eff, int(row_splits[-1]), overlapping,
+                                 torch.is_grad_enabled())
             if not overlapping and N * T < 2**31:
                 # what a loss needs to read `log_probs` in place and to send its gradient
                 # straight to it (k2b200_band_loss_*, k2b200_dense_loss_backward_log_probs):
@@ -192,9 +193,12 @@ class DenseFsaVec(object):
     def scores(self) -> torch.Tensor:
         """The [sum_i (T_i + 1), C + 1] score matrix (k2/csrc/fsa.h:138-185)."""
         if self._scores is None:
-            fn, log_probs, eff, rows, overlapping = self._make_scores
+            fn, log_probs, eff, rows, overlapping, grad = self._make_scores
             segments = _lib.upload_i32(eff.reshape(-1), self._device).view(-1, 3)
-            self._scores = fn.apply(log_probs, segments, self.row_splits, rows, overlapping)
+            # differentiable if it were so made by the constructor: the first use may be inside
+            # a loss, where gradients are off
+            with torch.set_grad_enabled(grad):
+                self._scores = fn.apply(log_probs, segments, self.row_splits, rows, overlapping)
             self._make_scores = None
         return self._scores
 

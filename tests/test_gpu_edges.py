@@ -565,3 +565,31 @@ def test_backward_after_the_inputs_are_gone(k2):
                     grads.append(x.grad)
                 del over
                 assert torch.equal(grads[0], grads[1]), (name, amap is None, band)
+
+
+def test_score_matrix_made_inside_a_loss(k2):
+    """The matrix of a DenseFsaVec is made on first use.  Where that is inside a loss (which takes the
+    gradient past it) or under no_grad, a lattice made from the same DenseFsaVec has its gradient;
+    one made under no_grad has none."""
+    from k2_b200 import synthetic as syn
+    rs2, arcs = syn.den_graph(10, 10)
+    seg = torch.tensor([[0, 0, 20], [1, 0, 18]], dtype=torch.int32)
+    lp = torch.log_softmax(torch.randn(2, 20, 11, device=DEV), -1)
+    graph = syn.build_graphs(syn.Workload("x", lp.cpu(), seg, 8.0, graph_row_splits2=rs2,
+                                          graph_arcs=arcs, num_symbols=None), DEV)
+    grads = []
+    for first_use in ("lattice", "loss", "no_grad"):
+        x = lp.clone().requires_grad_(True)
+        dense = k2.DenseFsaVec(x, seg)
+        if first_use == "loss":
+            k2.intersect_dense_tot_scores(graph, dense, 8.0)
+        elif first_use == "no_grad":
+            with torch.no_grad():
+                dense.scores
+        k2.intersect_dense(graph, dense, 8.0).get_tot_scores(True, True).sum().backward()
+        grads.append(x.grad)
+    for grad in grads[1:]:  # (posteriors, added in any order)
+        assert torch.allclose(grad, grads[0], rtol=0, atol=1e-5) and grad.abs().max() > 0.1
+    with torch.no_grad():
+        dense = k2.DenseFsaVec(lp.clone().requires_grad_(True), seg)
+    assert not dense.scores.requires_grad
