@@ -368,7 +368,7 @@ def test_python_integers_of_any_python(tmp_path, hex_version):
         assert ints([1, bad], out) == 0, bad
 
 
-def test_host_layer_is_stale_under_another_torch_or_python(monkeypatch):
+def test_host_layer_is_stale_under_another_torch_or_python(monkeypatch, tmp_path):
     """`python k2_b200/build.py`, which the import error names, builds _host.so anew after torch or
     Python changed."""
     import importlib.util
@@ -377,6 +377,11 @@ def test_host_layer_is_stale_under_another_torch_or_python(monkeypatch):
     build = importlib.util.module_from_spec(spec)
     spec.loader.exec_module(build)
     command = build._host_command()
+    monkeypatch.setattr(build, "HOST_PATH", str(tmp_path / "_host.so"))
+    monkeypatch.setattr(build, "HOST_KEY_PATH", str(tmp_path / "built_for"))
+    (tmp_path / "_host.so").write_bytes(b"")
+    assert build._host_stale(command)  # nobody knows what it was built for
+    (tmp_path / "built_for").write_text(build._host_key(command))
     assert not build._host_stale(command)
     assert build._host_stale(command + ["-g"])
     with monkeypatch.context() as m:
