@@ -12,8 +12,8 @@
 // hundreds).  The kernels are built on that:
 //
 //   BandViterbi   one small CTA per (graph, direction) walks all frames: a thread owns four
-//                 consecutive states in registers, neighbours come by two shuffles (and a
-//                 two-float hand-over between warps), the log-prob row of the frame arrives in a
+//                 consecutive states in registers, neighbours come by shuffles (and a
+//                 hand-over between warps every few frames), the log-prob row of the frame arrives in a
 //                 shared-memory ring by one bulk copy (TMA, mbarrier) issued many frames ahead.
 //                 Same fp32 expressions as the reference: (prev + arc.score) + dense, then max.
 //   BandPrep      all (graph, frame) levels in parallel: the reference's keep tests
@@ -241,15 +241,32 @@ __global__ void BandIncoming(const BandState *__restrict__ tab, const BandArc *_
 // of a batch are contiguous and arrive by ONE bulk copy (TMA, completion on an mbarrier)
 // requested batches ahead, the warps exchange their boundary states through shared memory
 // once per batch, and the frames of a batch run without any wait, barrier or
-// shared-memory store: per frame four (backward: six) shared-memory reads, two shuffles, the
-// adds and maxima, one 16-byte store.  Same fp32 expressions as the reference:
-// (prev + arc.score) + dense, then max.
-// Bound by the instructions of a warp per frame, 45 at one in about three cycles: 87 us for
-// 1000 frames x 501 states.  (Two states per thread: 117 us; rows put in the order of the
-// states by further warps: 118; packed additions: the moves into register pairs cost more
-// than they save.)
+// shared-memory store.  Same fp32 expressions as the reference: (prev + arc.score) + dense, then
+// max.  A warp of its own requests the rows (the thread that did so beside its states held up all
+// others at every batch).
+// A graph that alternates (VitForm) takes 17 instructions per frame and warp: three shared-memory
+// reads, a shuffle (backward: two), ten adds and maxima, a 16-byte store; any other takes 45.
+// Bound by the latency of a frame where the batch is small (45 ns up to 288 states, 56 with the
+// six warps of 501 states, 73 with nine) and by DRAM where it is large: 64 x 1000 frames of 500
+// classes are 204 MB read and 186 MB written in 75 us.  (All arcs by the general expressions and
+// the rows requested by thread 0: 86 us there, 124 instead of 109 for 16 x 1500 frames of up to 801
+// states.  Two states per thread: slower; eight: 99 us.)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float Max3(float a, float b, float c) { return fmaxf(fmaxf(a, b), c); }
+// The largest of three, NaN apart like fmaxf: one instruction.
+__device__ __forceinline__ float Max3(float a, float b, float c) {
+  float m;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(a), "f"(b), "f"(c));
+  return m;
+}
+
+// Whether a graph alternates, like those of k2.ctc_graph: every state but the final one has a
+// self-loop and an arc from the state before it, all arcs score zero, and the states of even
+// number share one label and have no arc from two states before.  (prev + 0) + dense is
+// prev + dense.
+template <bool kAlternates>
+struct VitForm {
+  static constexpr bool value = kAlternates;
+};
 
 constexpr int kVitMaxBatches = 4;  // batches of rows in flight
 constexpr int kVitMaxWarps = 12;
@@ -325,6 +342,39 @@ __device__ __forceinline__ void CopyAtEdge(const float *first, const float *last
   if (to > from) BulkCopyG2S(dst + from, src + from, (unsigned)(to - from) * 4u, bar);
 }
 
+// The frames of a batch, from row `row` on: `step` consumes the scores that `load` reads, which are
+// read four frames ahead of it, the first ones before the barrier of the exchange.
+template <int kX, typename Load, typename Exchange, typename Step>
+__device__ __forceinline__ void VitFrames(int32_t n, const float *row, int32_t width,
+                                          const Load &load, const Exchange &exchange,
+                                          const Step &step) {
+  constexpr int kAhead = 4, kFull = 16;
+  if (n == kFull) {
+    float x[2][kAhead][kX];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) load(row + u * width, x[0][u]);
+    exchange();
+#pragma unroll
+    for (int g = 0; g < kFull / kAhead; ++g) {
+      row += kAhead * width;
+      if (g + 1 < kFull / kAhead) {
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) load(row + u * width, x[(g + 1) & 1][u]);
+      }
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u) step(x[g & 1][u]);
+    }
+  } else {
+    exchange();
+#pragma unroll 4
+    for (int32_t r = 0; r < n; ++r, row += width) {
+      float x[kX];
+      load(row, x);
+      step(x);
+    }
+  }
+}
+
 // kByState: `lp` holds scores by state (BandGather) in the layout of the grids instead of
 // log-prob rows of C columns: a thread reads its states' scores in one word.  With 5000 columns
 // the copies of whole rows bounded the kernel (170 us for 500 frames); by state it takes 43,
@@ -332,7 +382,7 @@ __device__ __forceinline__ void CopyAtEdge(const float *first, const float *last
 // kEdge: the matrix starts or ends between two 16-byte boundaries.  (An instance of its own: a test
 // per batch in the other one took 5 us of 1000 frames.)
 template <bool kByState, bool kEdge>
-__global__ void __launch_bounds__(64 * kVitMaxWarps, 1)
+__global__ void __launch_bounds__(32 * (kVitMaxWarps + 1), 1)
 BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ tab,
             const float *__restrict__ lp, int64_t lp_rows, int32_t C, float *__restrict__ vf,
             float *__restrict__ vb, int32_t F, int32_t nbatch, int32_t slot_floats,
@@ -369,14 +419,16 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
     return kByState ? 0 : (int32_t)((lp0_words + (uint32_t)r * (uint32_t)width) & 3u);
   };
   int32_t issued = 0;
-  auto issue = [&]() {  // thread 0 only: the rows of the next batch into the next slot
+  int32_t next_slot = 0;
+  auto issue = [&]() {  // one thread only: the rows of the next batch into the next slot
     if (issued >= num_batches) return;
     const int32_t q = issued;
     // batch q: forward rows [qF, min((q+1)F, T)); backward rows [max(T-(q+1)F, 0), T-qF)
     const int32_t r0 = dir == 0 ? q * F : max(T - (q + 1) * F, 0);
     const int32_t r1 = dir == 0 ? min((q + 1) * F, T) : T - q * F;
     const int32_t off = words_off(r0);
-    const int32_t slot = q % nbatch;
+    const int32_t slot = next_slot;
+    next_slot = slot + 1 == nbatch ? 0 : slot + 1;
     if (kEdge) {
       CopyAtEdge(lp, lp + lp_rows * width, lp0 + (int64_t)r0 * width - off, off,
                  (r1 - r0) * width + off, ring + (size_t)slot * slot_floats, &full[slot]);
@@ -388,15 +440,42 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
     }
     ++issued;
   };
-  if (tid == 0)
-    for (int32_t q = 0; q < nbatch; ++q) issue();
+  bool late = false;
+  // The last warp requests the rows; its barriers are those of the walks below: the one before
+  // batch q says that every warp has finished batch q - 1.
+  const bool producer = warp == (int)(blockDim.x >> 5) - 1;
+  // slot and phase of the batch that is waited for
+  int32_t slot = 0;
+  unsigned parity = 0;
+  auto wait = [&]() {
+    if (!late) late = !WaitSlot(&full[slot], parity, wait_limit);
+  };
+  auto next_batch = [&]() {
+    if (++slot == nbatch) {
+      slot = 0;
+      parity ^= 1u;
+    }
+  };
+  if (producer) {
+    if (lane == 0)
+      for (int32_t q = 0; q < nbatch; ++q) issue();
+    __syncthreads_and(1);
+    for (int32_t q = 0; q < num_batches; ++q) {
+      if (q > 0 || dir == 1) __syncthreads();
+      if (q > 0 && lane == 0) {
+        wait();  // batch q - 1 has arrived, as the warps that have finished it know
+        if (!late) issue();  // into its slot
+        next_batch();
+      }
+    }
+    if (dir == 0) __syncthreads();
+  } else {
 
   // first state of this lane: forward, the recomputed states come first; backward, last
   const int32_t s0 = warp * own * K + (dir == 0 ? (lane - H) * K : lane * K);
   const bool mine = dir == 0 ? lane >= H : lane < own;   // a lane that owns its states
   const bool stores = mine && s0 < pitch;
   float *grid = (dir == 0 ? vf : vb) + f.grid_off + s0;
-  bool late = false;
   float v[K];
 #pragma unroll
   for (int k = 0; k < K; ++k) v[k] = 0.0f;
@@ -437,19 +516,28 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
       }
       v[k] = s == 0 ? 0.0f : -INFINITY;
     }
-    if (kByState) col[0] = min(max(s0, 0), pitch - K);
     if (stores) VitStore<K>(grid, v);
-    auto step = [&](const float (&a0)[K], const float (&a1)[K], const float (&a2)[K],
-                    const float (&x)[K]) {
-      const float h1 = __shfl_up_sync(kAll, v[K - 1], 1), h2 = __shfl_up_sync(kAll, v[K - 2], 1);
+    auto step = [&](auto alternates, const float (&a0)[K], const float (&a1)[K],
+                    const float (&a2)[K], const float (&x)[K]) {
+      const float h1 = __shfl_up_sync(kAll, v[K - 1], 1);
       float nv[K];
+      if (alternates.value) {
 #pragma unroll
-      for (int k = 0; k < K; ++k) {
-        const float a = v[k];
-        const float b = k >= 1 ? v[k >= 1 ? k - 1 : 0] : h1;
-        const float c = k >= 2 ? v[k >= 2 ? k - 2 : 0] : (k == 1 ? h1 : h2);
-        nv[k] = __fadd_rn(
-            Max3(__fadd_rn(a, a0[k]), __fadd_rn(b, a1[k]), __fadd_rn(c, a2[k])), x[k]);
+        for (int k = 0; k < K; k += 2) {
+          const float b = k ? v[k ? k - 1 : 0] : h1;  // of the state before these two
+          nv[k] = __fadd_rn(fmaxf(v[k], b), x[k]);
+          nv[k + 1] = __fadd_rn(Max3(v[k + 1], v[k], __fadd_rn(b, a2[k + 1])), x[k + 1]);
+        }
+      } else {
+        const float h2 = __shfl_up_sync(kAll, v[K - 2], 1);
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          const float a = v[k];
+          const float b = k >= 1 ? v[k >= 1 ? k - 1 : 0] : h1;
+          const float c = k >= 2 ? v[k >= 2 ? k - 2 : 0] : (k == 1 ? h1 : h2);
+          nv[k] = __fadd_rn(
+              Max3(__fadd_rn(a, a0[k]), __fadd_rn(b, a1[k]), __fadd_rn(c, a2[k])), x[k]);
+        }
       }
 #pragma unroll
       for (int k = 0; k < K; ++k) v[k] = nv[k];
@@ -457,41 +545,62 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
       if (stores) VitStore<K>(grid, v);
     };
     int32_t xpar = 0;
-    for (int32_t q = 0; q < num_batches; ++q) {
-      const int32_t slot = q % nbatch;
-      if (!late) late = !WaitSlot(&full[slot], (unsigned)(q / nbatch) & 1u, wait_limit);
-      if (q > 0) {
-        exchange(xpar);  // its barrier also says: every warp has finished batch q - 1
-        xpar ^= 1;
-        if (tid == 0 && !late) issue();  // into the slot batch q - 1 used
-      }
-      const int32_t nf = min(F, T - q * F);
-      const float *rowbuf = ring + (size_t)slot * slot_floats + words_off(q * F);
-#pragma unroll 4
-      for (int32_t r = 0; r < nf; ++r, rowbuf += width) {
-        float x[K];
+    auto walk = [&](auto alternates) {
+      auto load = [&](const float *row, float (&x)[K]) {
         if (kByState) {
-          VitLoad<K>(rowbuf + col[0], x);
+          VitLoad<K>(row + col[0], x);
         } else {
 #pragma unroll
-          for (int k = 0; k < K; ++k) x[k] = rowbuf[col[k]];
+          for (int k = 0; k < K; ++k)
+            x[k] = alternates.value && k >= 2 && k % 2 == 0 ? x[0] : row[col[k]];
         }
-        step(w0, w1, w2, x);
+      };
+      for (int32_t q = 0; q < num_batches; ++q) {
+        wait();
+        const int32_t nf = min(F, T - q * F);
+        const float *rowbuf = ring + (size_t)slot * slot_floats + words_off(q * F);
+        next_batch();
+        auto boundary = [&]() {
+          if (q == 0) return;
+          exchange(xpar);  // its barrier also says: every warp has finished batch q - 1
+          xpar ^= 1;
+        };
+        VitFrames<K>(nf, rowbuf, width, load, boundary,
+                     [&](const float (&x)[K]) { step(alternates, w0, w1, w2, x); });
       }
+    };
+    // (what the final state of a graph that alternates is given on the frames, where no arc
+    // enters it, goes to no other state, and the backward score that it is added to is -inf)
+    bool alternates = true;
+    const int32_t even_label = tab[f.state_off].label;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int32_t s = s0 + k;
+      if (s < 0 || s >= S) continue;
+      const bool last = s == S - 1 && w0[k] == -INFINITY && w1[k] == -INFINITY && w2[k] == -INFINITY;
+      const bool plain = w0[k] == 0.0f && (s == 0 || w1[k] == 0.0f) &&
+                         (w2[k] == -INFINITY || (k % 2 == 1 && w2[k] == 0.0f));
+      alternates &= (last || plain) && (k % 2 == 1 || col[k] == even_label);
     }
+    if (kByState) col[0] = min(max(s0, 0), pitch - K);
+    if (__syncthreads_and(alternates)) walk(VitForm<true>{});
+    else walk(VitForm<false>{});
     // the implied final row: level T + 1
     exchange(xpar);
     {
       float x[K];
 #pragma unroll
       for (int k = 0; k < K; ++k) x[k] = 0.0f;
-      step(f0, f1, f2, x);
+      step(VitForm<false>{}, f0, f1, f2, x);
     }
   } else {
     // ---- backward: state s to s, s + 1, s + 2 -----------------------------------
     float wo[K][3];   // score of the arc s -> s + d on the frames (-inf: its label has no column)
     float fo[K][3];   // on the implied final row
     int32_t col[K + 2];   // of states s0 .. s0 + K + 1
+    float skip[K + 2];    // score of the arc that enters the state from two states before
+    bool alternates = true;
+    const int32_t even_label = tab[f.state_off].label;
 #pragma unroll
     for (int k = 0; k < K; ++k)
 #pragma unroll
@@ -506,6 +615,11 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
       if (s < S) t = tab[f.state_off + s];
       const bool frame_label = t.label >= 0 && t.label < C;
       if (frame_label) col[k] = t.label;
+      skip[k] = frame_label ? t.w[2] : -INFINITY;
+      if (s < S && (frame_label || s < S - 1))
+        alternates &= frame_label && t.w[0] == 0.0f && (s == 0 || t.w[1] == 0.0f) &&
+                      (t.w[2] == -INFINITY || (k % 2 == 1 && t.w[2] == 0.0f));
+      if (s < S && k % 2 == 0) alternates &= frame_label && t.label == even_label;
 #pragma unroll
       for (int d = 0; d < 3; ++d)
         if (k - d >= 0 && k - d < K) {
@@ -521,6 +635,22 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
     for (int k = 0; k < K; ++k) v[k] = (s0 + k == S - 1) ? 0.0f : -INFINITY;
     grid += (int64_t)(T + 1) * pitch;
     if (stores) VitStore<K>(grid, v);
+    // A graph that alternates: what a state scores with its label's score is needed once, by it and
+    // by its two predecessors, which get it by shuffles.
+    auto short_step = [&](const float (&x)[K]) {
+      float g[K + 2];
+#pragma unroll
+      for (int k = 0; k < K; ++k) g[k] = __fadd_rn(v[k], x[k]);
+      g[K] = __shfl_down_sync(kAll, g[0], 1);
+      g[K + 1] = __shfl_down_sync(kAll, g[1], 1);
+#pragma unroll
+      for (int k = 0; k < K; k += 2) {
+        v[k] = fmaxf(g[k], g[k + 1]);
+        v[k + 1] = Max3(g[k + 1], g[k + 2], __fadd_rn(g[k + 3], skip[k + 3]));
+      }
+      grid -= pitch;
+      if (stores) VitStore<K>(grid, v);
+    };
     auto step = [&](const float (&w)[K][3], const float (&x)[K + 2]) {
       const float g1 = __shfl_down_sync(kAll, v[0], 1), g2 = __shfl_down_sync(kAll, v[1], 1);
       float nv[K];
@@ -546,40 +676,51 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
       step(fo, x);
     }
     int32_t xpar = 0;
-    for (int32_t q = 0; q < num_batches; ++q) {
-      const int32_t slot = q % nbatch;
-      if (!late) late = !WaitSlot(&full[slot], (unsigned)(q / nbatch) & 1u, wait_limit);
-      exchange(xpar);  // also: every warp has finished batch q - 1
-      xpar ^= 1;
-      if (q > 0 && tid == 0 && !late) issue();
-      const int32_t r1 = T - q * F, r0 = max(T - (q + 1) * F, 0);
-      const float *rowbuf =
-          ring + (size_t)slot * slot_floats + words_off(r0) + (size_t)(r1 - 1 - r0) * width;
-#pragma unroll 4
-      for (int32_t r = r1 - 1; r >= r0; --r, rowbuf -= width) {  // level r from level r + 1
-        float x[K + 2];
+    auto walk = [&](auto alternates) {
+      constexpr int kX = decltype(alternates)::value ? K : K + 2;
+      auto load = [&](const float *row, float (&x)[kX]) {
         if (kByState) {
           float lo[K], hi[2];
-          VitLoad<K>(rowbuf + col[0], lo);
-          VitLoad<2>(rowbuf + col[1], hi);
+          VitLoad<K>(row + col[0], lo);
 #pragma unroll
           for (int k = 0; k < K; ++k) x[k] = lo[k];
-          x[K] = hi[0];
-          x[K + 1] = hi[1];
+          if (kX > K) {
+            VitLoad<2>(row + col[1], hi);
+            x[kX - 2] = hi[0];
+            x[kX - 1] = hi[1];
+          }
         } else {
 #pragma unroll
-          for (int k = 0; k < K + 2; ++k) x[k] = rowbuf[col[k]];
+          for (int k = 0; k < kX; ++k)
+            x[k] = alternates.value && k >= 2 && k % 2 == 0 ? x[0] : row[col[k]];
         }
-        step(wo, x);
+      };
+      for (int32_t q = 0; q < num_batches; ++q) {
+        wait();
+        const int32_t r1 = T - q * F, r0 = max(T - (q + 1) * F, 0);
+        const float *rowbuf =
+            ring + (size_t)slot * slot_floats + words_off(r0) + (size_t)(r1 - 1 - r0) * width;
+        next_batch();
+        auto boundary = [&]() {
+          exchange(xpar);  // also: every warp has finished batch q - 1
+          xpar ^= 1;
+        };
+        VitFrames<kX>(r1 - r0, rowbuf, -width, load, boundary, [&](const float (&x)[kX]) {  // level r
+          if constexpr (decltype(alternates)::value) short_step(x);         // from level r + 1
+          else step(wo, x);
+        });
       }
-    }
+    };
+    if (__syncthreads_and(alternates)) walk(VitForm<true>{});
+    else walk(VitForm<false>{});
   }
+  }  // not the producer
   if (late) any_late = 1;
   __syncthreads();
   if (any_late) {
     // A copy did not arrive in time: the grids hold garbage.  Say so, and let the copies
     // that are still in flight towards this CTA's shared memory land before it retires.
-    if (tid == 0) {
+    if (producer && lane == 0) {
       atomicOr(status, kStatusLate);
       for (int32_t q = max(0, issued - nbatch); q < issued; ++q)
         WaitSlot(&full[q % nbatch], (unsigned)(q / nbatch) & 1u, kDrainPolls);
@@ -1931,7 +2072,7 @@ static int32_t MakeBandLayout(const k2b200_band_loss_args *a, BandLayout *L) {
         2, std::min<size_t>(3, (100 * 1024) / std::max<size_t>(F * row_bytes, 1)));
     const int32_t own_states = (32 - 2 * F / kVitK) * kVitK;
     const int32_t warps = std::max(1, CeilDiv(std::max(L->max_states, 1), own_states));
-    L->vit_threads = 32 * warps;
+    L->vit_threads = 32 * (warps + 1);
     L->xch_pad = (warps * own_states + 8 * F + 3) & ~3;
     L->viterbi_smem = sizeof(float) * ((size_t)L->vit_batches * L->vit_slot + 2 * (size_t)L->xch_pad);
     if (warps > kVitMaxWarps) {

@@ -206,6 +206,37 @@ def test_long_transcripts_sixteen_states_per_lane():
     compare(fsa_to_host(graphs), torch.from_numpy(x), seg, 10.0, tag="long")
 
 
+@pytest.mark.parametrize("tokens,frames,classes", [(1, 17, 5), (47, 65, 29), (48, 64, 29),
+                                                   (48, 79, 1100), (143, 161, 40)])
+@pytest.mark.parametrize("change", ["none", "modified", "score", "label", "skip"])
+def test_graphs_that_alternate_and_graphs_that_nearly_do(tokens, frames, classes, change):
+    # 4, 96, 98 and 288 states (a warp of the Viterbi kernel owns 96), a full last batch of
+    # frames and one of a single frame, rows by state (1100 classes); then the same graph
+    # but for one arc's score, one even state's label or an arc past an even state
+    from k2_b200.fsa_algo import ctc_graph
+    from gpu_util import fsa_to_host
+    rng = np.random.default_rng(tokens + frames)
+    symbols = [rng.integers(1, classes, size=tokens).tolist() for _ in range(2)]
+    a = fsa_to_host(ctc_graph(symbols, modified=change == "modified", device=DEV))
+    arcs, ns = a.arcs.copy(), 2 * tokens + 2
+    in_second = int(a.row_splits2[ns])  # of the two graphs, the second is changed
+    if change == "score":
+        arcs[in_second + 1, 3] = np.float32(-0.25).view(np.int32)
+    elif change == "label":
+        arcs[in_second:, 2][arcs[in_second:, 1] == 2 * (tokens // 2)] = classes - 1
+    elif change == "skip" and tokens > 1:
+        # an arc from the blank in state 0 to the blank in state 2 instead of its own loop
+        assert arcs[in_second, 1] == 0 and arcs[in_second + 1, 1] == 1
+        blank = int(arcs[in_second, 2])
+        arcs[in_second] = arcs[in_second + 1]
+        arcs[in_second + 1] = (0, 2, blank, 0)
+    a = HostFsaVec(a.row_splits1, a.row_splits2, arcs)
+    x = rng.normal(size=(2, frames, classes)) * 1.5
+    lp = torch.from_numpy((x - np.log(np.exp(x).sum(-1, keepdims=True))).astype(np.float32))
+    seg = torch.tensor([[0, 0, frames], [1, 0, max(tokens + 1, frames - 1)]], dtype=torch.int32)
+    compare(a, lp, seg, 8.0, tag=change)
+
+
 def test_summed_ctc_loss_as_one_node_equals_the_composition():
     # ctc_loss(reduction="sum") on the band path is one autograd node; the same numbers
     # and gradients as -tot_scores.sum() composed from its parts, for a loss that is scaled
