@@ -110,6 +110,7 @@ static_assert(sizeof(BandFactor) == 32, "BandFactor must be 32 bytes");
 constexpr uint32_t kNoDst = 255;
 constexpr int kMaxRegs = 4;     // warps of the list recursion
 constexpr int kChainThreads = 32 * kMaxRegs;
+constexpr int kKeepThreads = 128;  // of BandChainLists: they look after what the others leave behind
 constexpr int kMaxListed = 32 * kMaxRegs - 1;  // entries of a level that it handles (one is padding)
 // alpha of the final state on the last level (= Z) of a graph, as m * 2^e
 struct __align__(16) BandTotal {
@@ -1075,18 +1076,20 @@ BandPrep(const BandInfo *__restrict__ infos, const int32_t *__restrict__ a_row_s
 // previous list its neighbours are:
 //   alpha_l[j] = sum_d pw_l[j][d] * alpha_{l-1}[src_l[j][d]]
 //   beta_l[j]  = sum_d (pw_{l+1}[.][d] * beta_{l+1}[.]) at position dst_l[j][d]
-// What bounds it is the latency of a level: the values of two levels are in shared memory, so a
-// level costs one gather of three values, two dependent multiply-adds, a store and a barrier
-// of the warps that the chunk's lists need (none, with lists of up to 31 entries), whatever
-// the width of the lists; an entry's factors are fetched a level ahead.  (One warp with up to
-// four entries per lane and the values in registers took 48 to 150 instructions per level, at
-// one in five cycles: 145 us on ctc_large, 1002 levels; this takes 91.)
+// What bounds it is the latency of a level, in which a warp issues in order: one gather of three
+// values from shared memory, two dependent multiply-adds, a store and a barrier of the warps that
+// the chunk's lists need (none, with lists of up to 31 entries).  So these warps do nothing else,
+// and what is not needed for the next level's values (the store to memory, the offsets and
+// factors of the entries to come) is issued while the three values arrive.  Four more warps, the
+// keepers, request the chunks, wait for them on behalf of all, look at the range of the values
+// and write the exponents, a chunk behind.  A level takes 100 cycles forward, 135 backward:
+// 73 us for 64 x 1000 frames, 99 for 16 x 1500 (91 and 130 with all of that in the same warps).
 // Every level of a chunk of kPrepLevels levels has the same padded number of entries, so inside a
 // chunk addresses advance by a constant.  No test: an absent neighbour is a padding entry,
 // whose value is 0.  The chunks arrive in a ring in shared memory by one bulk copy each,
 // requested chunks ahead.
 // The values of a level are stored divided by 2^K; K changes every kRescale levels by the
-// exponent of the largest value since the last change.  A value that is not zero and
+// exponent of the largest value of the last of them.  A value that is not zero and
 // below 2^-900 (or a value above 2^900) marks the graph in `unfit` for BandChainExact,
 // like the graphs BandPrep marked, which return at once here.
 // Outputs: alpha / beta at the list positions, K per level, tot[i], total[i].
@@ -1160,38 +1163,29 @@ struct ChainValues {
 struct ChainState {
   double acc, scale;
   int32_t Ksh;      // the level's values are stored divided by 2^Ksh
-  int32_t hi_max;   // largest high word since the last change of scale
-  uint32_t min_hi;  // smallest (high word - 1), zeros apart
+  int32_t hm;       // largest high word when it was last asked for, of this warp's values
 };
 
-// One level.  kBuf: the values go to vals.v[kBuf], those of the level before are in the other.
-template <int DIR, int kBuf>
-__device__ __forceinline__ void ChainLevel(const ChainRec &rec, ChainValues &vals, int tid,
-                                           bool first, bool rescaled, ChainState &st,
-                                           double *out) {
-  const char *prev = reinterpret_cast<const char *>(vals.v[kBuf ^ 1][0]);
-  const double x0 = *reinterpret_cast<const double *>(prev + ((rec.at << 3) & 0x7f8u));
-  const double x1 = *reinterpret_cast<const double *>(prev + ((rec.at >> 5) & 0x7f8u) +
-                                                      (DIR == 0 ? 0 : 2048));
-  const double x2 = *reinterpret_cast<const double *>(prev + ((rec.at >> 13) & 0x7f8u) +
-                                                      (DIR == 0 ? 0 : 4096));
-  double acc = DIR == 0 ? fma(rec.p0, x0, fma(rec.p1, x1, rec.p2 * x2)) : (x0 + x1) + x2;
-  if (rescaled) acc *= st.scale;
-  // the first level holds one state, with the value 1: the start state walking forward, the
-  // final state walking backward
-  if (first) acc = tid == 0 ? 1.0 : 0.0;
-  if (DIR == 0) {
-    vals.v[kBuf][0][tid] = acc;
-  } else {
-    vals.v[kBuf][0][tid] = rec.p0 * acc;
-    vals.v[kBuf][1][tid] = rec.p1 * acc;
-    vals.v[kBuf][2][tid] = rec.p2 * acc;
-  }
-  *out = acc;
-  const int32_t hi = __double2hiint(acc);  // values are not negative
-  st.hi_max = max(st.hi_max, hi);
-  st.min_hi = min(st.min_hi, (uint32_t)hi - 1u);  // a zero does not count
-  st.acc = acc;
+// Shared-memory offsets of the values that an entry adds up, in a ChainValues buffer.
+struct ChainFrom {
+  uint32_t at[3];
+};
+template <int DIR>
+__device__ __forceinline__ ChainFrom FromOf(uint32_t at) {
+  ChainFrom a;
+  a.at[0] = (at << 3) & 0x7f8u;
+  a.at[1] = ((at >> 5) & 0x7f8u) + (DIR == 0 ? 0 : 2048);
+  a.at[2] = ((at >> 13) & 0x7f8u) + (DIR == 0 ? 0 : 4096);
+  return a;
+}
+
+__device__ __forceinline__ double LoadValue(unsigned smem) {
+  double x;
+  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(x) : "r"(smem) : "memory");
+  return x;
+}
+__device__ __forceinline__ void StoreValue(unsigned smem, double x) {
+  asm volatile("st.shared.f64 [%0], %1;" ::"r"(smem), "d"(x) : "memory");
 }
 
 // The scale that the values of the next group of levels are multiplied with.
@@ -1213,66 +1207,101 @@ __device__ __forceinline__ void ChainSync() {
 }
 
 // The nl levels of a chunk; by the kWarps warps that its lists need.  r = this thread's entry
-// of the first level walked, out / osc = where its results go.
+// of the first level walked, out = where its results go, half_scale: the exponents of the values of
+// either half of the chunk.
 template <int DIR, int kWarps>
-__device__ __forceinline__ void ChainChunk(const char *r, double *out, int32_t *osc,
+__device__ __forceinline__ void ChainChunk(const char *r, double *out, int32_t *half_scale,
                                            int32_t l, int32_t nl, bool first_chunk,
-                                           ChainValues &vals, int32_t *hi_sh, int &group,
-                                           ChainState &st, int32_t *unfit_i) {
+                                           unsigned vals, int32_t *hi_sh, int &group,
+                                           ChainState &st) {
   constexpr unsigned kAll = 0xffffffffu;
   constexpr int kStep = DIR == 0 ? 1 : -1;
   constexpr int kPer = 32 * kWarps;
+  constexpr unsigned kBufBytes = sizeof(double) * 3 * 256;
   // levels (mod kRescale) that change the scale / end a group / clear the old maximum
   constexpr int kScales = DIR == 0 ? 0 : kRescale - 1, kEnds = DIR == 0 ? kRescale - 1 : 0,
                 kClears = DIR == 0 ? 2 : kRescale - 3;
   const int tid = threadIdx.x, lane = tid & 31;
-  ChainRec rec = LoadRec<DIR, kPer>(r);
-  auto level = [&](auto buf, int32_t phase, bool first, bool last, int32_t j) {
+  const unsigned own = vals + tid * 8;
+  // the entry of the level at hand and of the next one
+  ChainRec rec = LoadRec<DIR, kPer>(r), next = rec;
+  ChainFrom from = FromOf<DIR>(rec.at);
+  if (nl > 1) next = LoadRec<DIR, kPer>(r + kStep * kPer * 32);
+  // One level.  What is not needed for the next level's values is seen to while these three arrive:
+  // where the level before goes (`pending`), the record after next, the next offsets.
+  // tail: the level after next is not of this chunk; half: which half of the chunk it is in.
+  auto level = [&](auto buf, int32_t phase, bool first, bool pending, bool tail, int32_t j,
+                   int32_t half, bool single, bool starts) {
     constexpr int kBuf = decltype(buf)::value;
-    // (the level behind a chunk's last is read and not used: it is inside the ring)
-    const ChainRec next = last ? rec : LoadRec<DIR, kPer>(r + kStep * (j + 1) * kPer * 32);
+    const unsigned prev = vals + (kBuf ^ 1) * kBufBytes;
+    const double x0 = LoadValue(prev + from.at[0]), x1 = LoadValue(prev + from.at[1]),
+                 x2 = LoadValue(prev + from.at[2]);
     const bool rescaled = phase == kScales && !first;
+    if (pending) out[kStep * (j - 1) * kPer] = st.acc;
+    from = FromOf<DIR>(next.at);
+    const ChainRec after = tail ? next : LoadRec<DIR, kPer>(r + kStep * (j + 2) * kPer * 32);
     if (rescaled) {
-      ChainRescale(*reinterpret_cast<volatile int32_t *>(&hi_sh[group]), st);
+      // (one warp knows the maximum of the group before, unless another walked the chunk before)
+      ChainRescale(kWarps == 1 && !starts ? st.hm : *reinterpret_cast<volatile int32_t *>(&hi_sh[group]),
+                   st);
       group ^= 1;
     }
-    ChainLevel<DIR, kBuf>(rec, vals, tid, first, rescaled, st, out + kStep * j * kPer);
-    if (phase == kEnds) {
-      const int32_t hm = __reduce_max_sync(kAll, st.hi_max);
-      if (lane == 0) {
-        atomicMax(&hi_sh[group], hm);
-        if (hm >= (1023 + 900) << 20) atomicOr(unfit_i, kUnfitRange);
+    double acc = DIR == 0 ? fma(rec.p0, x0, fma(rec.p1, x1, rec.p2 * x2)) : (x0 + x1) + x2;
+    if (rescaled) acc *= st.scale;
+    // the first level holds one state, with the value 1: the start state walking forward, the
+    // final state walking backward
+    if (first) acc = tid == 0 ? 1.0 : 0.0;
+    if (DIR == 0) {
+      StoreValue(own + kBuf * kBufBytes, acc);
+    } else {
+      StoreValue(own + kBuf * kBufBytes, rec.p0 * acc);
+      StoreValue(own + kBuf * kBufBytes + 2048, rec.p1 * acc);
+      StoreValue(own + kBuf * kBufBytes + 4096, rec.p2 * acc);
+    }
+    st.acc = acc;
+    if (phase == kEnds) {  // (values are not negative: their order is that of the high words)
+      out[kStep * j * kPer] = acc;
+      st.hm = __reduce_max_sync(kAll, __double2hiint(acc));
+      if (kWarps > 1) {
+        if (lane == 0) atomicMax(&hi_sh[group], st.hm);
+      } else if (tid == 0) {
+        hi_sh[group] = st.hm;
       }
-      st.hi_max = 0;
     }
     if (tid == 0) {
-      osc[kStep * j] = st.Ksh;
+      if (phase == kScales || single) half_scale[half] = st.Ksh;
       if (phase == kClears) hi_sh[group ^ 1] = 0;
     }
     rec = next;
+    next = after;
     ChainSync<kWarps>();
   };
   // level l's values are in buffer l & 1
   if (!first_chunk && nl == kPrepLevels) {
+#pragma unroll
     for (int32_t g = 0; g < kPrepLevels / kRescale; ++g) {
 #pragma unroll
       for (int j = 0; j < kRescale; ++j) {
         const int phase = DIR == 0 ? j : kRescale - 1 - j;
-        const bool last = j == kRescale - 1 && g == kPrepLevels / kRescale - 1;
-        if (phase & 1) level(ChainBuf<1>{}, phase, false, last, j);
-        else level(ChainBuf<0>{}, phase, false, last, j);
+        const bool pending = j > 0;  // (the last level of a group of kRescale leaves nothing)
+        const bool tail = j >= kRescale - 2 && g == kPrepLevels / kRescale - 1;
+        const int32_t half = DIR == 0 ? g : 1 - g;
+        if (phase & 1) level(ChainBuf<1>{}, phase, false, pending, tail, j, half, false, g == 0);
+        else level(ChainBuf<0>{}, phase, false, pending, tail, j, half, false, g == 0);
       }
       r += kStep * kRescale * kPer * 32;
       out += kStep * kRescale * kPer;
-      osc += kStep * kRescale;
     }
   } else {
     for (int32_t k = 0; k < nl; ++k, l += kStep) {
-      if (l & 1) level(ChainBuf<1>{}, l & (kRescale - 1), first_chunk && k == 0, k == nl - 1, 0);
-      else level(ChainBuf<0>{}, l & (kRescale - 1), first_chunk && k == 0, k == nl - 1, 0);
+      const int32_t phase = l & (kRescale - 1);
+      const bool tail = k >= nl - 2;
+      const int32_t half = (l / kRescale) & 1;
+      if (l & 1) level(ChainBuf<1>{}, phase, first_chunk && k == 0, false, tail, 0, half, true, true);
+      else level(ChainBuf<0>{}, phase, first_chunk && k == 0, false, tail, 0, half, true, true);
+      if (phase != kEnds) *out = st.acc;
       r += kStep * kPer * 32;
       out += kStep * kPer;
-      osc += kStep;
     }
   }
 }
@@ -1291,13 +1320,13 @@ __device__ __forceinline__ void ChainWalk(const BandInfo &f, int32_t i, BandFact
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int32_t T = f.frames, pitch = f.pitch, L = T + 2;
   const int32_t num_chunks = (L + kPrepLevels - 1) / kPrepLevels;
-  for (int32_t c = tid; c < num_chunks; c += kChainThreads)
+  for (int32_t c = tid; c < num_chunks; c += kChainThreads + kKeepThreads)
     crc[c] = (unsigned char)chunk_r[f.level_off + c * kPrepLevels];
   if (tid < 6) vals.v[tid / 3][tid % 3][kNoDst] = 0.0;
   if (tid == 0) {
     for (int st = 0; st < kChainSlots; ++st) MbarInit(&full[st], 1);
     MbarInitFence();
-    hi_sh[0] = hi_sh[1] = hi_sh[2] = hi_sh[3] = 0;
+    hi_sh[0] = hi_sh[1] = hi_sh[2] = hi_sh[3] = hi_sh[8] = 0;
   }
   __syncthreads();
   const BandFactor *fac0 = factors + f.grid_off;
@@ -1316,23 +1345,51 @@ __device__ __forceinline__ void ChainWalk(const BandInfo &f, int32_t i, BandFact
                 &full[slot]);
     ++issued;
   };
-  if (tid == 0)
+  const bool keeper = tid >= kChainThreads, issuer = tid == kChainThreads;
+  if (issuer)
     for (int32_t k = 0; k < kChainSlots; ++k) issue();
   ChainState st;
   st.acc = 0.0;
   st.scale = 1.0;
-  st.Ksh = 0;
-  st.hi_max = 0;
-  st.min_hi = 0xffffffffu;
+  st.Ksh = st.hm = 0;
+  int32_t hi_max = 0;             // keepers: largest high word,
+  uint32_t min_hi = 0xffffffffu;  // smallest (high word - 1), zeros apart
+  // the keepers' share: what the walk of chunk q left in memory
+  auto keep = [&](int32_t q) {
+    const int32_t c = DIR == 0 ? q : num_chunks - 1 - q, a = c * kPrepLevels;
+    const int32_t nl = min(kPrepLevels, L - a), me = tid - kChainThreads;
+    const double *v = om + (int64_t)a * pitch;
+    const int32_t n = nl * 32 * crc[c];
+#pragma unroll 4
+    for (int32_t k = me; k < n; k += kKeepThreads) {
+      const int32_t hi = __double2hiint(v[k]);  // values are not negative
+      hi_max = max(hi_max, hi);
+      min_hi = min(min_hi, (uint32_t)hi - 1u);  // a zero does not count
+    }
+    if (me < nl) oscale[a + me] = hi_sh[4 + 2 * (q & 1) + me / kRescale];
+  };
   int group = 0;
   bool late = false, idle = false;
+  int32_t slot = 0;
+  unsigned parity = 0;
   for (int32_t q = 0; q < num_chunks; ++q) {
-    const int32_t c = DIR == 0 ? q : num_chunks - 1 - q, slot = q % kChainSlots;
-    late = !WaitSlot(&full[slot], (unsigned)(q / kChainSlots) & 1u, wait_limit);
-    // (also: the chunk before has been read, and its last level's values are there)
-    late = __syncthreads_or(late);
+    // the issuer's warp has seen chunk q arrive; the chunk before has been read, and its last
+    // level's values are there
+    if (tid / 32 == kChainThreads / 32 && !WaitSlot(&full[slot], parity, wait_limit)) hi_sh[8] = 1;
+    __syncthreads();
+    late = *reinterpret_cast<volatile int32_t *>(&hi_sh[8]);
     if (late) break;
-    if (q > 0 && tid == 0) issue();  // into the slot of the chunk before
+    const int32_t c = DIR == 0 ? q : num_chunks - 1 - q;
+    const BandFactor *mine = ring + (size_t)slot * kFacSlot;
+    if (++slot == kChainSlots) {
+      slot = 0;
+      parity ^= 1u;
+    }
+    if (keeper) {
+      if (q > 0 && issuer) issue();  // into the slot of the chunk before
+      if (q > 0) keep(q - 1);
+      continue;
+    }
     if (idle) {  // what the warps at work kept track of
       st.Ksh = hi_sh[2];
       group = hi_sh[3];
@@ -1343,15 +1400,14 @@ __device__ __forceinline__ void ChainWalk(const BandInfo &f, int32_t i, BandFact
     idle = warp >= rc;
     if (!idle) {
       const int32_t at = (l - l_lo) * 32 * rc + tid;
-      const char *r = reinterpret_cast<const char *>(ring + (size_t)slot * kFacSlot +
-                                                     (l - l_lo) * 32 * rc) + tid * 16;
+      const char *r = reinterpret_cast<const char *>(mine + (l - l_lo) * 32 * rc) + tid * 16;
       double *out = om + (int64_t)l_lo * pitch + at;
-      int32_t *osc = oscale + l;
+      int32_t *half_scale = hi_sh + 4 + 2 * (q & 1);
       switch (rc) {
-        case 1: ChainChunk<DIR, 1>(r, out, osc, l, nl, q == 0, vals, hi_sh, group, st, &unfit[i]); break;
-        case 2: ChainChunk<DIR, 2>(r, out, osc, l, nl, q == 0, vals, hi_sh, group, st, &unfit[i]); break;
-        case 3: ChainChunk<DIR, 3>(r, out, osc, l, nl, q == 0, vals, hi_sh, group, st, &unfit[i]); break;
-        default: ChainChunk<DIR, 4>(r, out, osc, l, nl, q == 0, vals, hi_sh, group, st, &unfit[i]); break;
+        case 1: ChainChunk<DIR, 1>(r, out, half_scale, l, nl, q == 0, SmemAddr(&vals), hi_sh, group, st); break;
+        case 2: ChainChunk<DIR, 2>(r, out, half_scale, l, nl, q == 0, SmemAddr(&vals), hi_sh, group, st); break;
+        case 3: ChainChunk<DIR, 3>(r, out, half_scale, l, nl, q == 0, SmemAddr(&vals), hi_sh, group, st); break;
+        default: ChainChunk<DIR, 4>(r, out, half_scale, l, nl, q == 0, SmemAddr(&vals), hi_sh, group, st); break;
       }
     }
     if (tid == 0) {
@@ -1360,17 +1416,18 @@ __device__ __forceinline__ void ChainWalk(const BandInfo &f, int32_t i, BandFact
     }
   }
   if (late) {
-    if (tid == 0) {
+    if (issuer) {
       atomicOr(status, kStatusLate);
       for (int32_t k = max(0, issued - kChainSlots); k < issued; ++k)
         WaitSlot(&full[k % kChainSlots], (unsigned)(k / kChainSlots) & 1u, kDrainPolls);
     }
-    __syncthreads();
   }
-  {
+  __syncthreads();  // the last chunk's values
+  if (keeper && !late) {
+    keep(num_chunks - 1);
     // values that are not zero must have kept clear of the ends of a double's range
-    const int32_t hm = __reduce_max_sync(kAll, st.hi_max);
-    const uint32_t hn = __reduce_min_sync(kAll, st.min_hi);
+    const int32_t hm = __reduce_max_sync(kAll, hi_max);
+    const uint32_t hn = __reduce_min_sync(kAll, min_hi);
     if ((hm >= ((1023 + 900) << 20) || hn < (uint32_t)(((1023 - 900) << 20) - 1)) && lane == 0)
       atomicOr(&unfit[i], kUnfitRange);
   }
@@ -1389,7 +1446,7 @@ __device__ __forceinline__ void ChainWalk(const BandInfo &f, int32_t i, BandFact
   }
 }
 
-__global__ void __launch_bounds__(kChainThreads)
+__global__ void __launch_bounds__(kChainThreads + kKeepThreads)
 BandChainLists(const BandInfo *__restrict__ infos, const BandFactor *__restrict__ factors,
                const int32_t *__restrict__ chunk_r, double *__restrict__ am,
                double *__restrict__ bm, int32_t *__restrict__ a_scale,
@@ -1399,7 +1456,7 @@ BandChainLists(const BandInfo *__restrict__ infos, const BandFactor *__restrict_
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full[kChainSlots];
   __shared__ ChainValues vals;
-  __shared__ int32_t hi_sh[4];
+  __shared__ int32_t hi_sh[9];
   __shared__ unsigned char crc[kChainMaxChunks];
   const int dir = blockIdx.x;
   const int32_t i = blockIdx.y;
@@ -2163,7 +2220,7 @@ static int32_t LaunchBandChains(const BandLayout &L, const k2b200_band_loss_args
   BandTotal *total = reinterpret_cast<BandTotal *>(ws + L.off_total);
   int32_t *unfit = reinterpret_cast<int32_t *>(ws + L.off_unfit);
   int32_t *status = reinterpret_cast<int32_t *>(ws + L.off_status);
-  { BandChainLists<<<grid, kChainThreads, L.chain_smem, stream>>>(
+  { BandChainLists<<<grid, kChainThreads + kKeepThreads, L.chain_smem, stream>>>(
       infos, reinterpret_cast<const BandFactor *>(ws + L.off_factors),
       reinterpret_cast<const int32_t *>(ws + L.off_chunk_r), am, bm,
       reinterpret_cast<int32_t *>(ws + L.off_a_scale),
