@@ -243,15 +243,16 @@ __global__ void BandIncoming(const BandState *__restrict__ tab, const BandArc *_
 // requested batches ahead, the warps exchange their boundary states through shared memory
 // once per batch, and the frames of a batch run without any wait, barrier or
 // shared-memory store.  Same fp32 expressions as the reference: (prev + arc.score) + dense, then
-// max.  A warp of its own requests the rows (the thread that did so beside its states held up all
-// others at every batch).
+// max.  A warp of its own requests the rows and waits for them; the others learn of it by the
+// barrier that they need anyway (a wait of theirs on the mbarrier cost a tenth of the kernel, the
+// requests by a thread that walks more).
 // A graph that alternates (VitForm) takes 17 instructions per frame and warp: three shared-memory
 // reads, a shuffle (backward: two), ten adds and maxima, a 16-byte store; any other takes 45.
-// Bound by the latency of a frame where the batch is small (45 ns up to 288 states, 56 with the
-// six warps of 501 states, 73 with nine) and by DRAM where it is large: 64 x 1000 frames of 500
-// classes are 204 MB read and 186 MB written in 75 us.  (All arcs by the general expressions and
-// the rows requested by thread 0: 86 us there, 124 instead of 109 for 16 x 1500 frames of up to 801
-// states.  Two states per thread: slower; eight: 99 us.)
+// Bound by the latency of a frame where the batch is small (36 ns with the three warps of 240
+// states, 65 with the nine of 801) and by DRAM where it is large: 64 x 1000 frames of 500 classes
+// are 204 MB read and 186 MB written in 67 us.  (All arcs by the general expressions, rows
+// requested and waited for by the warps that walk: 86 us there, 124 instead of 99 for 16 x 1500
+// frames of up to 801 states.  Two states per thread: slower; eight: 99 us.)
 // ---------------------------------------------------------------------------
 // The largest of three, NaN apart like fmaxf: one instruction.
 __device__ __forceinline__ float Max3(float a, float b, float c) {
@@ -344,17 +345,15 @@ __device__ __forceinline__ void CopyAtEdge(const float *first, const float *last
 }
 
 // The frames of a batch, from row `row` on: `step` consumes the scores that `load` reads, which are
-// read four frames ahead of it, the first ones before the barrier of the exchange.
-template <int kX, typename Load, typename Exchange, typename Step>
+// read four frames ahead of it.
+template <int kX, typename Load, typename Step>
 __device__ __forceinline__ void VitFrames(int32_t n, const float *row, int32_t width,
-                                          const Load &load, const Exchange &exchange,
-                                          const Step &step) {
+                                          const Load &load, const Step &step) {
   constexpr int kAhead = 4, kFull = 16;
   if (n == kFull) {
     float x[2][kAhead][kX];
 #pragma unroll
     for (int u = 0; u < kAhead; ++u) load(row + u * width, x[0][u]);
-    exchange();
 #pragma unroll
     for (int g = 0; g < kFull / kAhead; ++g) {
       row += kAhead * width;
@@ -366,7 +365,6 @@ __device__ __forceinline__ void VitFrames(int32_t n, const float *row, int32_t w
       for (int u = 0; u < kAhead; ++u) step(x[g & 1][u]);
     }
   } else {
-    exchange();
 #pragma unroll 4
     for (int32_t r = 0; r < n; ++r, row += width) {
       float x[kX];
@@ -442,31 +440,22 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
     ++issued;
   };
   bool late = false;
-  // The last warp requests the rows; its barriers are those of the walks below: the one before
-  // batch q says that every warp has finished batch q - 1.
+  // The last warp requests the rows and waits for them on behalf of all: the barrier before batch q
+  // says that its rows are there and that every warp has finished batch q - 1.
   const bool producer = warp == (int)(blockDim.x >> 5) - 1;
-  // slot and phase of the batch that is waited for
-  int32_t slot = 0;
-  unsigned parity = 0;
-  auto wait = [&]() {
-    if (!late) late = !WaitSlot(&full[slot], parity, wait_limit);
-  };
-  auto next_batch = [&]() {
-    if (++slot == nbatch) {
-      slot = 0;
-      parity ^= 1u;
-    }
-  };
   if (producer) {
     if (lane == 0)
       for (int32_t q = 0; q < nbatch; ++q) issue();
     __syncthreads_and(1);
+    int32_t slot = 0;
+    unsigned parity = 0;
     for (int32_t q = 0; q < num_batches; ++q) {
-      if (q > 0 || dir == 1) __syncthreads();
-      if (q > 0 && lane == 0) {
-        wait();  // batch q - 1 has arrived, as the warps that have finished it know
-        if (!late) issue();  // into its slot
-        next_batch();
+      if (!late) late = !WaitSlot(&full[slot], parity, wait_limit);
+      __syncthreads();
+      if (q > 0 && lane == 0 && !late) issue();  // into the slot of batch q - 1
+      if (++slot == nbatch) {
+        slot = 0;
+        parity ^= 1u;
       }
     }
     if (dir == 0) __syncthreads();
@@ -545,7 +534,7 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
       grid += pitch;
       if (stores) VitStore<K>(grid, v);
     };
-    int32_t xpar = 0;
+    int32_t xpar = 0, slot = 0;
     auto walk = [&](auto alternates) {
       auto load = [&](const float *row, float (&x)[K]) {
         if (kByState) {
@@ -557,16 +546,12 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
         }
       };
       for (int32_t q = 0; q < num_batches; ++q) {
-        wait();
+        exchange(xpar);
+        xpar ^= 1;
         const int32_t nf = min(F, T - q * F);
         const float *rowbuf = ring + (size_t)slot * slot_floats + words_off(q * F);
-        next_batch();
-        auto boundary = [&]() {
-          if (q == 0) return;
-          exchange(xpar);  // its barrier also says: every warp has finished batch q - 1
-          xpar ^= 1;
-        };
-        VitFrames<K>(nf, rowbuf, width, load, boundary,
+        if (++slot == nbatch) slot = 0;
+        VitFrames<K>(nf, rowbuf, width, load,
                      [&](const float (&x)[K]) { step(alternates, w0, w1, w2, x); });
       }
     };
@@ -676,7 +661,7 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
       for (int k = 0; k < K + 2; ++k) x[k] = 0.0f;
       step(fo, x);
     }
-    int32_t xpar = 0;
+    int32_t xpar = 0, slot = 0;
     auto walk = [&](auto alternates) {
       constexpr int kX = decltype(alternates)::value ? K : K + 2;
       auto load = [&](const float *row, float (&x)[kX]) {
@@ -697,16 +682,13 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
         }
       };
       for (int32_t q = 0; q < num_batches; ++q) {
-        wait();
+        exchange(xpar);
+        xpar ^= 1;
         const int32_t r1 = T - q * F, r0 = max(T - (q + 1) * F, 0);
         const float *rowbuf =
             ring + (size_t)slot * slot_floats + words_off(r0) + (size_t)(r1 - 1 - r0) * width;
-        next_batch();
-        auto boundary = [&]() {
-          exchange(xpar);  // also: every warp has finished batch q - 1
-          xpar ^= 1;
-        };
-        VitFrames<kX>(r1 - r0, rowbuf, -width, load, boundary, [&](const float (&x)[kX]) {  // level r
+        if (++slot == nbatch) slot = 0;
+        VitFrames<kX>(r1 - r0, rowbuf, -width, load, [&](const float (&x)[kX]) {  // level r
           if constexpr (decltype(alternates)::value) short_step(x);         // from level r + 1
           else step(wo, x);
         });
