@@ -707,7 +707,10 @@ GridChainMasked(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_leve
     BulkCopyG2S(dst + kU * row_bytes, mask0 + r_lo * kThreads, (unsigned)nf * kThreads,
                 &full[slot]);
   };
-  if (tid == 0)
+  // the last warp, whose lanes are the last to be given states, requests the batches and waits for
+  // them on behalf of all (a poll of the mbarrier by every warp took its time)
+  const bool waits = tid >= kThreads - 32, issues = tid == kThreads - 32;
+  if (issues)
     for (int32_t b = 0; b < kMaskedBatches - 1; ++b) issue_batch(b);
   const int32_t g_max = __reduce_max_sync(0xffffffffu, G);  // widest lane group of this warp
   const int32_t s_ld = s >= 0 ? s : 0;
@@ -722,7 +725,7 @@ GridChainMasked(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_leve
       const int32_t slot = b % kMaskedBatches;
       const unsigned parity = (unsigned)(b / kMaskedBatches) & 1u;
       // (the usual limit as a constant: the polling loop the compiler makes of it is the cheaper one)
-      const bool late = !MbarTryWait(&full[slot], parity) &&
+      const bool late = waits && !MbarTryWait(&full[slot], parity) &&
                         !(wait_limit == 4000000 ? MbarWaitBounded(&full[slot], parity)
                                                 : MbarWaitBounded(&full[slot], parity, wait_limit));
       // also: the last frame of the batch before is complete; nobody reads its slot any more
@@ -731,7 +734,7 @@ GridChainMasked(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_leve
         if (tid == 0) t_fail_sm = b;  // shared memory: nothing of it stays live in the loop
         break;
       }
-      if (tid == 0) issue_batch(b + kMaskedBatches - 1);
+      if (issues) issue_batch(b + kMaskedBatches - 1);
       const unsigned char *base = ring + (size_t)slot * batch_bytes;
       const int32_t nf = min(kU, Tk - b * kU);
       const int pb = (kU % 2 == 0) ? 0 : (b & 1);  // parity of the state buffers at the batch's start
