@@ -74,6 +74,45 @@ def test_random_fsa_vecs_bit_exact(k2, mode):
         assert lat.properties == oracle.properties(want)[1]
 
 
+@pytest.mark.parametrize("states,frames", [(2, 1), (5, 13), (33, 40), (520, 560)])
+@pytest.mark.parametrize("form", ["plain", "scores", "labels", "columns", "special"])
+def test_one_gather_per_state_bit_exact(k2, states, frames, form):
+    # arcs s -> s, s + 1, s + 2 that all score zero, one label per destination; then with scores
+    # (walking backward the arcs need their own gathers), with a second label into one state, with
+    # labels that have no column, and with infinite scores and NaN in the dense matrix
+    from gpu_util import dense_from_scores, fsa_to_host, host_to_fsa, intersect_raw
+    from oracle.common import HostFsaVec, make_arcs
+    rng = np.random.default_rng(states + frames)
+    cols = 7
+    label = rng.integers(0, cols - 1 + 3 * (form == "columns"), size=states)
+    label[-1] = -1
+    rows, rs2 = [], [0]
+    for s in range(states - 1):
+        for d in range(3):
+            if s + d < states and (s + d < states - 1 or d > 0):
+                score = float(np.float32(rng.normal())) if form == "scores" else 0.0
+                rows.append([s, s + d, label[s + d], score])
+        rs2.append(len(rows))
+    rs2.append(len(rows))
+    if form == "labels" and states > 2:
+        rows[1][2] = (label[1] + 1) % (cols - 1)
+    r = np.array(rows)
+    a = HostFsaVec(np.array([0, states], np.int32), np.array(rs2, np.int32),
+                   make_arcs(r[:, 0].astype(np.int32), r[:, 1].astype(np.int32),
+                             r[:, 2].astype(np.int32), r[:, 3].astype(np.float32)))
+    scores = rng.normal(size=(frames + 1, cols)).astype(np.float32) * 2
+    scores[:, 0] = -np.inf
+    scores[-1], scores[-1, 0] = -np.inf, 0.0
+    if form == "special":
+        scores[0, 1], scores[frames // 2, 2], scores[frames // 3, 3] = -np.inf, np.nan, -np.inf
+    brs = np.array([0, frames + 1], np.int32)
+    lat, ma, mb = intersect_raw(host_to_fsa(a), dense_from_scores(scores, brs), 6.0, mode=3)
+    want, wa, wb = intersect_raw(host_to_fsa(a), dense_from_scores(scores, brs), 6.0, mode=1)
+    same_fsa(fsa_to_host(lat, ma, mb), fsa_to_host(want, wa, wb), form)
+    if form != "special":
+        same_fsa(fsa_to_host(lat, ma, mb), oracle.intersect_dense(a, scores, brs, 6.0, None), form)
+
+
 def _check_scores(k2, lat, want):
     from gpu_util import fsa_to_host
     for log_semiring in (True, False):
