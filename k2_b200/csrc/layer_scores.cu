@@ -221,9 +221,11 @@ static ChainPlan PlanChain(const k2b200_fsa_view *v, int32_t ndir) {
   const int32_t mean_w = (int32_t)((v->num_states + layers - 1) / layers),
                 mean_a = (int32_t)((v->num_arcs + layers - 1) / layers);
   // arcs per lane (rows of a block): what most states of a lattice have, or a share of it that
-  // leaves the states of many arcs enough lanes
+  // leaves the states of many arcs enough lanes.  Three from 1.2 arcs per state on (alignments
+  // have 1.4, at most three): then no state has two lanes, and the tropical walk is the short one
+  // (239 -> 118 us for 802 layers); two below that (decoding, 1.07).
   const double mean_deg = (double)v->num_arcs / std::max(v->num_states, 1);
-  p.rows = mean_deg < 1.6 ? 2 : mean_deg < 3.0 ? 3 : mean_deg < 6.0 ? 4 : 8;
+  p.rows = mean_deg < 1.2 ? 2 : mean_deg < 3.0 ? 3 : mean_deg < 6.0 ? 4 : 8;
   // Warps: a block of 32 lanes each, for a layer between the mean and the largest (a warp that
   // runs alone issues an instruction in about five cycles, so more warps than blocks only
   // add to the barrier).
@@ -274,10 +276,11 @@ struct SliceDesc {
   uint32_t at;     // of the region, in units of 16 bytes
   int32_t size;    // likewise
   int32_t blocks;  // of K rows; -1: the pool was full, the arcs are read where they are
-  int32_t tall;
+  int32_t tall;    // kSingle: none, and one block with a lane per state
 };
+constexpr int32_t kSingle = -1;
 // Of a region in units of 16 bytes: where the rows start.
-__device__ __forceinline__ int32_t SliceRowsAt(int32_t blocks, int32_t tall) {
+__device__ __forceinline__ constexpr int32_t SliceRowsAt(int32_t blocks, int32_t tall) {
   return (blocks + tall) * 8 + (tall + 3) / 4;
 }
 
@@ -404,7 +407,7 @@ SliceLayers(k2b200_fsa_view v, int32_t dir_base, int32_t K, int32_t maxw, int32_
     head[14] = blocks * 32;  // ... of the tall states
     head[17] = blocks * K;   // ... and their first row
     const unsigned long long at = atomicAdd(pool_used, (unsigned long long)units);
-    SliceDesc d = {(uint32_t)at, units, blocks, tall};
+    SliceDesc d = {(uint32_t)at, units, blocks, head[5] == w && blocks == 1 ? kSingle : tall};
     // (a tall block's word has 12 bits for its rows, 20 for the first of them)
     if (at + units > (unsigned long long)pool_units || head[16] >= 4096 ||
         blocks * K + head[16] >= (1 << 20)) {
@@ -749,6 +752,53 @@ SliceChain(k2b200_fsa_view v, const uint4 *__restrict__ pool, const SliceDesc *_
   int32_t slot = p.slots - 1, k = 0, m = 0;
   unsigned parity = 1;
   int32_t prev = p.maxw, cur = 0;
+  // A layer of one block with a lane per state (alignments), of the tropical semiring, in `now`; the
+  // records of the layer behind it, if it is of the same kind and slot, go to `next` meanwhile.
+  // What a warp that runs alone issues per layer bounds such a walk: 290 cycles, against 590 of the
+  // general loop below.
+  // (Its region then lies right behind: it is read before it is known whether it is of that kind.)
+  constexpr int32_t kSingleUnits = SliceRowsAt(1, 0) + K * 32;
+  struct Single {
+    uint32_t word;
+    int32_t first_state;
+    LayerArc x[K];
+  };
+  const int32_t last_single = p.slots * (p.slot_bytes >> 4) - kSingleUnits;
+  auto read_single = [&](int32_t at, Single &l) {
+    l.word = shared_words[at * 4 + lane];
+    const LayerArc *r = shared_recs + at + SliceRowsAt(1, 0) + lane;
+#pragma unroll
+    for (int u = 0; u < K; ++u) l.x[u] = r[u * 32];
+  };
+  auto single = [&](const Single &now, Single &next, int32_t &at, int32_t step) {
+    Val y[K];
+#pragma unroll
+    for (int u = 0; u < K; ++u) y[u] = vals[prev + now.x[u].other];
+    bool more = false;
+    at += kSingleUnits;
+    if (k < m && at <= last_single) {
+      read_single(at, next);
+      const SliceEntry e = entries[slot][k];
+      next.first_state = e.first_state;
+      more = e.tall == kSingle && e.at == at;
+    }
+    StateSum<Val, kLog> q;
+    q.Clear();
+#pragma unroll
+    for (int u = 0; u < K; ++u) q.Add(now.x[u], y[u]);
+    if (now.word & kLaneHead) {
+      const int32_t j = (int32_t)(now.word & kNoState), s = now.first_state + j;
+      if (step == 0 && s == root && q.acc == (Val)-INFINITY) q.acc = (Val)0;
+      vals[cur + j] = q.acc;
+      out[s] = q.acc;
+      if (entering != nullptr && dir == 0) entering[s] = q.best;
+    }
+    const int32_t t = prev;
+    prev = cur;
+    cur = t;
+    __syncwarp();
+    return more;
+  };
   for (int32_t step = 0; step < nl; ++step) {
     if (k == m) {  // the next slot
       slot = slot + 1 == p.slots ? 0 : slot + 1;
@@ -762,7 +812,27 @@ SliceChain(k2b200_fsa_view v, const uint4 *__restrict__ pool, const SliceDesc *_
       k = 0;
       m = slot_layers[slot];
     }
-    const SliceEntry e = entries[slot][k++];
+    SliceEntry e = entries[slot][k++];
+    if (e.tall == kSingle) {
+      e.tall = 0;
+      if (!kLog && nw == 1 && e.at >= 0) {
+        Single a, b;
+        int32_t at = e.at;
+        read_single(at, a);
+        a.first_state = e.first_state;
+        while (single(a, b, at, step)) {
+          ++step;
+          ++k;
+          if (!single(b, a, at, step)) break;
+          ++step;
+          ++k;
+        }
+        if (k == m && lane == 0)  // this warp has read the slot
+          asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(SmemAddr(&empty[slot]))
+                       : "memory");
+        continue;
+      }
+    }
     sc.BeginLayer(step, hi_shared, tid == 0);
     auto finish = [&](int32_t j, StateSum<Val, kLog> &q) {
       const int32_t s = e.first_state + j;
@@ -949,7 +1019,8 @@ ExactChain(k2b200_fsa_view v, const uint4 *__restrict__ pool, const SliceDesc *_
         if (dir == 0 && entering != nullptr) entering[s] = q.best;
       }
     };
-    const SliceDesc d = descs[(int64_t)dir * nl_total + lv0 + l];
+    SliceDesc d = descs[(int64_t)dir * nl_total + lv0 + l];
+    if (d.tall == kSingle) d.tall = 0;
     if (d.blocks >= 0 && (*status & 1) == 0) {
       const uint4 *region = pool + d.at;
       const uint32_t *words = reinterpret_cast<const uint32_t *>(region);

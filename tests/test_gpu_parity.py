@@ -113,6 +113,58 @@ def test_one_gather_per_state_bit_exact(k2, states, frames, form):
         same_fsa(fsa_to_host(lat, ma, mb), oracle.intersect_dense(a, scores, brs, 6.0, None), form)
 
 
+@pytest.mark.parametrize("most", [3, 4, 9])
+@pytest.mark.parametrize("double", [True, False])
+@pytest.mark.parametrize("wide", [False, True])
+def test_best_paths_through_layers_of_one_lane_per_state(k2, most, double, wide):
+    # layers of 1 to 32 states (a warp walks them) with up to `most` entering arcs each, or among
+    # them layers of 33 and 70 states; scores that are multiples of a quarter: many paths tie
+    from gpu_util import host_to_fsa
+    from oracle.common import HostFsaVec, make_arcs
+    rng = np.random.default_rng(most)
+    rs1, rs2, rows, bounds = [0], [0], [], [1, 0, 0, 0]
+    for fsa in range(4):
+        sizes = [1] + rng.choice([1, 2, 5, 31, 32], size=60).tolist()
+        if wide and fsa % 2:
+            sizes[7], sizes[20], sizes[21] = 33, 70, 33
+        sizes += [3, 1]
+        first = np.concatenate([[0], np.cumsum(sizes)])
+        out = [[] for _ in range(first[-1])]
+        for l in range(1, len(sizes)):
+            for s in range(first[l], first[l + 1]):
+                n = int(rng.integers(1, most + 1))
+                # every state of the layer before has an arc somewhere
+                for src in rng.integers(first[l - 1], first[l], size=n).tolist():
+                    out[src].append(s)
+            for src in range(first[l - 1], first[l]):
+                if not out[src]:
+                    out[src].append(int(rng.integers(first[l], first[l + 1])))
+        final = first[-1] - 1
+        for src, dests in enumerate(out):
+            for dest in sorted(dests):
+                rows.append([src, dest, -1 if dest == final else 1, rng.integers(-8, 8) / 4])
+            rs2.append(len(rows))
+        rs1.append(rs1[-1] + first[-1])
+        arcs = [sum(len(d) for d in out[b:e]) for b, e in zip(first[:-1], first[1:])]
+        bounds = [1, max(bounds[1], len(sizes)), max(bounds[2], *sizes), max(bounds[3], *arcs)]
+    r = np.array(rows)
+    a = HostFsaVec(np.array(rs1, np.int32), np.array(rs2, np.int32),
+                   make_arcs(r[:, 0].astype(np.int32), r[:, 1].astype(np.int32),
+                             r[:, 2].astype(np.int32), r[:, 3].astype(np.float32)))
+    fsa = host_to_fsa(a)
+    # as a lattice says of itself
+    assert fsa.arcs.levels()[0].tolist()[-1] == sum(bounds[1:2] * 4)
+    fsa.arcs._layer_bounds = tuple(int(x) for x in bounds)
+    scores, entering = oracle.forward_scores(a, False, double, want_entering_arcs=True)
+    # (sums of quarters are exact, in float32 too)
+    np.testing.assert_array_equal(fsa.get_forward_scores(double, False).cpu().numpy(), scores)
+    np.testing.assert_array_equal(fsa._get_entering_arcs(double).cpu().numpy(), entering)
+    np.testing.assert_array_equal(fsa.get_backward_scores(double, False).cpu().numpy(),
+                                  oracle.backward_scores(a, False, double))
+    np.testing.assert_array_equal(k2.shortest_path(fsa, double)._best_arc_map.cpu().numpy(),
+                                  oracle.shortest_path(a, entering)[1])
+
+
 def _check_scores(k2, lat, want):
     from gpu_util import fsa_to_host
     for log_semiring in (True, False):
