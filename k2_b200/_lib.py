@@ -3,6 +3,7 @@
 There is no CPU path and no fallback: importing this module fails loudly when the
 CUDA library has not been built.
 """
+import contextlib
 import ctypes
 import os
 
@@ -322,12 +323,13 @@ def ptr(t) -> int:
     buffer (never dereferenced: their size is 0)."""
     if t is None:
         return None
-    if t.numel() == 0:
-        key = str(t.device)
-        if key not in _dummy:
-            _dummy[key] = torch.zeros(64, dtype=torch.int32, device=t.device)
-        return _dummy[key].data_ptr()
-    return t.data_ptr()
+    address = t.data_ptr()
+    if address:
+        return address
+    key = str(t.device)
+    if key not in _dummy:
+        _dummy[key] = torch.zeros(64, dtype=torch.int32, device=t.device)
+    return _dummy[key].data_ptr()
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
@@ -339,6 +341,16 @@ def stream_of(device) -> int:
         idx = device.index if isinstance(device, torch.device) else torch.device(device).index
         return _raw_stream(torch.cuda.current_device() if idx is None else idx)
     return torch.cuda.current_stream(device).cuda_stream
+
+
+_current_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
+_nothing = contextlib.nullcontext()
+
+
+def device_guard(device: torch.device):
+    """torch.cuda.device(device), which costs the host 4 us each time, where that is not the
+    current device already: some ten calls of a lattice's way ask for it."""
+    return _nothing if device.index == _current_device() else torch.cuda.device(device)
 
 
 def workspace(nbytes: int, device) -> "_host.Workspace":
@@ -362,7 +374,7 @@ def upload_i32(arr, device) -> torch.Tensor:
     arr = np.ascontiguousarray(arr, dtype=np.int32).reshape(-1)
     out = torch.empty(arr.shape[0], dtype=torch.int32, device=device)
     if arr.shape[0]:
-        with torch.cuda.device(out.device):
+        with device_guard(out.device):
             check(lib.k2b200_upload_i32(arr.ctypes.data, arr.shape[0], out.data_ptr(),
                                         stream_of(out.device)))
     return out

@@ -26,7 +26,7 @@ def _index_add(index: torch.Tensor, value: torch.Tensor, in_out: torch.Tensor) -
     """in_out[index[k]] += value[k] (k2/python/csrc/torch/index_add.cu:38-71)."""
     assert index.dtype == torch.int32 and in_out.dtype == torch.float32
     value = value.to(torch.float32).contiguous()
-    with torch.cuda.device(in_out.device):
+    with _lib.device_guard(in_out.device):
         _lib.check(_lib.lib.k2b200_index_add(_lib.ptr(index), _lib.ptr(value), index.numel(),
                                               _lib.ptr(in_out), in_out.numel(),
                                               _lib.stream_of(in_out.device)))
@@ -46,7 +46,7 @@ def index_select(src, index: torch.Tensor):
         return ans
     src = src.contiguous()
     out = torch.empty(index.numel(), dtype=torch.int32, device=src.device)
-    with torch.cuda.device(src.device):
+    with _lib.device_guard(src.device):
         _lib.check(_lib.lib.k2b200_index_select_i32(_lib.ptr(src), src.numel(), _lib.ptr(index),
                                                      index.numel(), _lib.ptr(out),
                                                      _lib.stream_of(src.device)))
@@ -108,7 +108,7 @@ def _intersect_dense_arcs(a: RaggedArc, b: DenseFsaVec, a_to_b_map: Optional[tor
     ns, na, beam = ctypes.c_int32(), ctypes.c_int32(), ctypes.c_float()
     max_w, max_a = ctypes.c_int32(), ctypes.c_int32()
     stream = _lib.stream_of(dev)
-    with torch.cuda.device(dev):
+    with _lib.device_guard(dev):
         _lib.check(_lib.lib.k2b200_intersect_dense_prune(ctypes.byref(args), _lib.ptr(ws),
                                                           nbytes.value, stream, ctypes.byref(ns),
                                                           ctypes.byref(na), ctypes.byref(beam),
@@ -174,7 +174,7 @@ class _GetTotScoresFunction(torch.autograd.Function):
         stride = tot_scores_grad.stride(0) if tot_scores_grad.numel() > 0 else 0
         rid1 = arcs.row_ids(1 - arcs.single)
         rid2 = arcs.row_ids(2 - arcs.single)
-        with torch.cuda.device(dev):
+        with _lib.device_guard(dev):
             if log_semiring is False:
                 from .fsa_algo import _shortest_path_arcs
                 _, best_arcs = _shortest_path_arcs(fsas, use_double_scores)
@@ -208,7 +208,7 @@ def _backprop_scores(fsas: Fsa, forward: bool, log_semiring: bool, use_double_sc
         else:
             best_tmp = torch.empty(arcs.num_states, dtype=torch.int32, device=dev)
     view, keep = arcs.view(want_incoming=not forward)
-    with torch.cuda.device(dev):
+    with _lib.device_guard(dev):
         _lib.check(_lib.lib.k2b200_fsa_scores_backprop(
             ctypes.byref(view), int(forward), int(log_semiring), int(use_double_scores),
             _lib.ptr(scores.contiguous()), _lib.ptr(entering), _lib.ptr(state_deriv),
@@ -280,7 +280,7 @@ class _GetArcPostFunction(torch.autograd.Function):
         forward_grad = torch.zeros(arcs.num_states, dtype=dtype, device=dev)
         backward_grad = torch.zeros(arcs.num_states, dtype=dtype, device=dev)
         view, keep = arcs.view(want_incoming=True)
-        with torch.cuda.device(dev):
+        with _lib.device_guard(dev):
             _lib.check(_lib.lib.k2b200_fsa_arc_post_backprop(
                 ctypes.byref(view), int(ctx.use_double_scores), _lib.ptr(arc_scores_grad),
                 _lib.ptr(forward_grad), _lib.ptr(backward_grad), _lib.stream_of(dev)))
@@ -409,7 +409,7 @@ def _intersect_dense_pruned_arcs(a: RaggedArc, b: DenseFsaVec, search_beam: floa
             ctypes.byref(args), ctypes.byref(nbytes), ctypes.byref(levels)))
         ws = torch.empty(nbytes.value, dtype=torch.uint8, device=dev)
         ns, na, full = ctypes.c_int32(), ctypes.c_int32(), ctypes.c_int32()
-        with torch.cuda.device(dev):
+        with _lib.device_guard(dev):
             _lib.check(_lib.lib.k2b200_intersect_dense_pruned_search_bounds(
                 ctypes.byref(args), _lib.ptr(ws), nbytes.value, stream, ctypes.byref(ns),
                 ctypes.byref(na), ctypes.byref(full), bounds))
@@ -421,7 +421,7 @@ def _intersect_dense_pruned_arcs(a: RaggedArc, b: DenseFsaVec, search_beam: floa
         if cap_a >= 1 << 30:
             raise RuntimeError("intersect_dense_pruned: more than 2^30 arcs alive in one sequence")
     ns, na = ns.value, na.value
-    with torch.cuda.device(dev):
+    with _lib.device_guard(dev):
         row_splits1 = torch.empty(num_seqs + 1, **i32)
         row_ids1 = torch.empty(ns + 1, **i32)
         row_splits2 = torch.empty(ns + 1, **i32)
@@ -529,7 +529,7 @@ class _DenseTotScoresFunction(torch.autograd.Function):
         ws = lease.tensor
         tot = torch.empty(a_fsas.arcs.num_fsas, dtype=torch.float64, device=dev)
         beam = ctypes.c_float()
-        with torch.cuda.device(dev):
+        with _lib.device_guard(dev):
             _lib.check(_lib.lib.k2b200_dense_loss_forward(
                 ctypes.byref(args), _lib.ptr(ws), nbytes.value, _lib.stream_of(dev),
                 _lib.ptr(tot), ctypes.byref(beam)))
@@ -563,7 +563,7 @@ class _DenseTotScoresFunction(torch.autograd.Function):
         if ctx.needs_input_grad[7]:
             grad_a = torch.zeros(ctx.shape_a, dtype=torch.float32, device=dev)
         grad_b = torch.zeros(ctx.shape_b, dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
+        with _lib.device_guard(dev):
             if ctx.lp_row is None:
                 _lib.check(_lib.lib.k2b200_dense_loss_backward(
                     ctypes.byref(ctx.args), _lib.ptr(ctx.ws), ctx.ws_bytes, _lib.ptr(tot_grad),
@@ -694,7 +694,7 @@ class _BandTotScoresFunction(torch.autograd.Function):
             ctx.grad_b = torch.empty(unused_scores_b.shape, dtype=torch.float32, device=dev)
             args.zero_fill = ctx.grad_b.data_ptr()
             args.zero_fill_bytes = ctx.grad_b.numel() * 4
-        with torch.cuda.device(dev):
+        with _lib.device_guard(dev):
             _lib.check(_lib.lib.k2b200_band_loss_forward(
                 ctypes.byref(args), _lib.ptr(ws), nbytes.value, _lib.stream_of(dev),
                 _lib.ptr(tot), ctypes.byref(beam)))
@@ -731,7 +731,7 @@ class _BandTotScoresFunction(torch.autograd.Function):
         grad_b, ctx.grad_b = ctx.grad_b, None  # cleared by the forward call; used once
         if grad_b is None:
             grad_b = torch.zeros(ctx.shape_b, dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
+        with _lib.device_guard(dev):
             _lib.check(_lib.lib.k2b200_band_loss_backward(
                 ctypes.byref(ctx.args), _lib.ptr(ctx.ws), ctx.ws_bytes, _lib.ptr(tot_grad),
                 stride, _lib.ptr(grad_a), _lib.ptr(grad_b), _lib.ptr(ctx.grad_rows),

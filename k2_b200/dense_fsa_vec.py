@@ -22,7 +22,7 @@ class _DenseFsaVecFunction(torch.autograd.Function):
         N, T, C = log_probs.shape
         dev = log_probs.device
         scores = torch.empty(rows, C + 1, dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
+        with _lib.device_guard(dev):
             _lib.check(_lib.lib.k2b200_dense_fsa_vec_fill(
                 _lib.ptr(log_probs), N, T, C, _lib.ptr(segments), _lib.ptr(row_splits),
                 segments.shape[0], _lib.ptr(scores), rows, _lib.stream_of(dev)))
@@ -39,7 +39,7 @@ class _DenseFsaVecFunction(torch.autograd.Function):
         grad_scores = grad_scores.contiguous()
         dev = grad_scores.device
         grad = torch.empty(N, T, C, dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
+        with _lib.device_guard(dev):
             _lib.check(_lib.lib.k2b200_dense_fsa_vec_backward(
                 _lib.ptr(grad_scores), N, T, C, _lib.ptr(segments), _lib.ptr(row_splits),
                 segments.shape[0], ctx.rows, int(ctx.overlapping), _lib.ptr(grad),
@@ -58,7 +58,7 @@ class _LogSoftmaxDenseFunction(torch.autograd.Function):
         N, T, C = logits.shape
         dev = logits.device
         scores = torch.empty(rows, C + 1, dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
+        with _lib.device_guard(dev):
             _lib.check(_lib.lib.k2b200_dense_fsa_vec_from_logits(
                 _lib.ptr(logits), N, T, C, _lib.ptr(segments), _lib.ptr(row_splits),
                 segments.shape[0], _lib.ptr(scores), rows, _lib.stream_of(dev)))
@@ -75,7 +75,7 @@ class _LogSoftmaxDenseFunction(torch.autograd.Function):
         grad_scores = grad_scores.contiguous()
         dev = grad_scores.device
         grad = torch.empty(N, T, C, dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
+        with _lib.device_guard(dev):
             _lib.check(_lib.lib.k2b200_dense_fsa_vec_from_logits_backward(
                 _lib.ptr(grad_scores), _lib.ptr(scores), N, T, C, _lib.ptr(segments),
                 _lib.ptr(row_splits), segments.shape[0], ctx.rows, int(ctx.overlapping),

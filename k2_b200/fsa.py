@@ -254,7 +254,7 @@ class Fsa(object):
             scratch = torch.empty(nscratch, dtype=torch.uint8, device=dev)
         if want_forward and need_incoming.value:
             view, keep = arcs.view(want_incoming=True)
-        with torch.cuda.device(dev):
+        with _lib.device_guard(dev):
             _lib.check(_lib.lib.k2b200_fsa_scores(
                 ctypes.byref(view), int(log_semiring), int(use_double_scores), _lib.ptr(fwd),
                 _lib.ptr(bwd), _lib.ptr(entering), _lib.ptr(scratch), nscratch,
@@ -296,7 +296,7 @@ class Fsa(object):
             fwd = self._get_forward_scores(use_double_scores, log_semiring)
             arcs = self.arcs
             tot = torch.empty(arcs.num_fsas, dtype=fwd.dtype, device=fwd.device)
-            with torch.cuda.device(fwd.device):
+            with _lib.device_guard(fwd.device):
                 _lib.check(_lib.lib.k2b200_fsa_tot_scores(
                     _lib.ptr(arcs._row_splits1), arcs.num_fsas, int(use_double_scores),
                     _lib.ptr(fwd), _lib.ptr(tot), _lib.stream_of(fwd.device)))
@@ -310,7 +310,7 @@ class Fsa(object):
             bwd = self._get_backward_scores(use_double_scores, log_semiring)
             arcs = self.arcs
             post = torch.empty(arcs.num_elements(), dtype=fwd.dtype, device=fwd.device)
-            with torch.cuda.device(fwd.device):
+            with _lib.device_guard(fwd.device):
                 _lib.check(_lib.lib.k2b200_fsa_arc_post(
                     _lib.ptr(arcs._row_splits1), _lib.ptr(arcs.row_ids(1 - arcs.single)),
                     _lib.ptr(arcs.row_ids(2 - arcs.single)), _lib.ptr(arcs.values()),
@@ -394,7 +394,7 @@ def _basic_properties(arcs: RaggedArc) -> int:
     props = torch.empty(nf + 1, dtype=torch.int32, device=dev)
     tmp = torch.empty(_lib.lib.k2b200_fsa_properties_tmp_bytes(nf, ns), dtype=torch.uint8,
                       device=dev)
-    with torch.cuda.device(dev):
+    with _lib.device_guard(dev):
         _lib.check(_lib.lib.k2b200_fsa_properties(
             _lib.ptr(arcs._row_splits1), _lib.ptr(arcs.row_ids(1 - arcs.single)),
             _lib.ptr(arcs._row_splits2), _lib.ptr(arcs.row_ids(2 - arcs.single)),

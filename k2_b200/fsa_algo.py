@@ -268,7 +268,7 @@ def _best_paths(fsa: Fsa, use_double_scores: bool):
     values = torch.empty((n, 4), dtype=torch.int32, device=dev)
     tmp = torch.empty(_lib.lib.k2b200_best_paths_tmp_bytes(ctypes.byref(view)), dtype=torch.uint8,
                       device=dev)
-    with torch.cuda.device(dev):
+    with _lib.device_guard(dev):
         _lib.check(_lib.lib.k2b200_best_paths(
             ctypes.byref(view), _lib.ptr(entering), path_splits.data_ptr(),
             row_splits1.data_ptr(), row_splits2.data_ptr(), _lib.ptr(values), _lib.ptr(best),
@@ -292,7 +292,7 @@ def _shortest_path_arcs(fsa: Fsa, use_double_scores: bool) -> Tuple[torch.Tensor
     path_splits = torch.empty(nf + 1, dtype=torch.int32, device=dev)
     best = torch.empty(max(arcs.num_states, 1), dtype=torch.int32, device=dev)
     tmp = torch.empty(_lib.lib.k2b200_shortest_path_tmp_bytes(nf), dtype=torch.uint8, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.device_guard(dev):
         _lib.check(_lib.lib.k2b200_shortest_path(
             _lib.ptr(arcs._row_splits1), _lib.ptr(arcs.values()), _lib.ptr(entering), nf,
             _lib.ptr(path_splits), _lib.ptr(best), _lib.ptr(tmp), _lib.stream_of(dev)))

@@ -122,7 +122,7 @@ class OnlineDenseIntersecter:
             beams_out = np.zeros(n, np.float32)
             counts = np.zeros(2 * n, np.int32)
             ns, na, full = ctypes.c_int32(), ctypes.c_int32(), ctypes.c_int32()
-            with torch.cuda.device(dev):
+            with _lib.device_guard(dev):
                 loads = (_lib.OnlineStream * n)(*[s._c() for s in states])
                 _lib.check(_lib.lib.k2b200_online_decode_load_all(
                     ctypes.byref(args), _lib.ptr(ws), loads, stream))
@@ -139,7 +139,7 @@ class OnlineDenseIntersecter:
                 raise RuntimeError("OnlineDenseIntersecter: more than 2^30 arcs alive in a stream")
         ns, na = ns.value, na.value
         new_states = []
-        with torch.cuda.device(dev):
+        with _lib.device_guard(dev):
             row_splits1 = torch.empty(n + 1, **i32)
             row_ids1 = torch.empty(ns + 1, **i32)
             row_splits2 = torch.empty(ns + 1, **i32)

@@ -163,7 +163,7 @@ class RaggedArc:
             buf = torch.empty((3, max(na, 1)), dtype=torch.int32, device=dev)
             band = getattr(self, "_band_graph", None)
             if band is not None and band[0] == key and band[1] is not None:
-                with torch.cuda.device(dev):
+                with _lib.device_guard(dev):
                     _lib.check(_lib.lib.k2b200_band_incoming(
                         band[1].states_ptr, band[1].arcs_ptr, _lib.ptr(self._row_splits2), ns,
                         _lib.ptr(in_splits), buf[0].data_ptr(), buf[1].data_ptr(),
@@ -179,7 +179,7 @@ class RaggedArc:
                 return self._incoming
             tmp = torch.empty(_lib.lib.k2b200_fsa_incoming_tmp_bytes(ns, na), dtype=torch.uint8,
                               device=dev)
-            with torch.cuda.device(dev):
+            with _lib.device_guard(dev):
                 _lib.check(_lib.lib.k2b200_fsa_incoming(
                     _lib.ptr(self._row_splits1), _lib.ptr(self.row_ids(1 - self.single)),
                     _lib.ptr(self.row_ids(2 - self.single)), _lib.ptr(self._values),
@@ -195,7 +195,7 @@ class RaggedArc:
         layer.  False when a layer is too wide for it."""
         view, keep = self.view(want_incoming=False)
         done = _lib.c_i32()
-        with torch.cuda.device(self.device):
+        with _lib.device_guard(self.device):
             _lib.check(_lib.lib.k2b200_fsa_incoming_layers(
                 ctypes.byref(view), in_splits.data_ptr(), buf[0].data_ptr(), buf[1].data_ptr(),
                 buf[2].data_ptr(), ctypes.byref(done), _lib.stream_of(self.device)))
@@ -222,7 +222,7 @@ class RaggedArc:
         states = torch.empty(sb.value, dtype=torch.uint8, device=dev)
         arcs = torch.empty(ab.value, dtype=torch.uint8, device=dev)
         status = torch.empty(1, dtype=torch.int32, device=dev)
-        with torch.cuda.device(dev):
+        with _lib.device_guard(dev):
             _lib.check(_lib.lib.k2b200_band_tables(
                 _lib.ptr(self._row_splits1), self.num_fsas, _lib.ptr(self._row_splits2),
                 _lib.ptr(vals), ns, _lib.ptr(states), _lib.ptr(arcs), _lib.ptr(status),
@@ -328,7 +328,7 @@ def _row_ids(row_splits: torch.Tensor, num_elems: int) -> torch.Tensor:
     if num_elems == 0:
         return out
     if row_splits.is_cuda:
-        with torch.cuda.device(row_splits.device):
+        with _lib.device_guard(row_splits.device):
             _lib.check(_lib.lib.k2b200_row_splits_to_row_ids(
                 _lib.ptr(row_splits), row_splits.shape[0] - 1, _lib.ptr(out), num_elems,
                 _lib.stream_of(row_splits.device)))
@@ -349,7 +349,7 @@ def _gpu_levels(arcs: RaggedArc):
     tmp = torch.empty(_lib.lib.k2b200_fsa_levels_tmp_bytes(ns), dtype=torch.uint8, device=dev)
     rid2 = arcs.row_ids(2 - arcs.single)
     status = offsets[nf + 1:]
-    with torch.cuda.device(dev):
+    with _lib.device_guard(dev):
         _lib.check(_lib.lib.k2b200_fsa_levels(
             _lib.ptr(arcs._row_splits1), _lib.ptr(arcs._row_splits2), _lib.ptr(rid2),
             _lib.ptr(arcs._values), nf, ns, na, _lib.ptr(offsets), _lib.ptr(splits),

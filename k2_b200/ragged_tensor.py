@@ -124,7 +124,7 @@ def _row_ids(row_splits: torch.Tensor, num_elems: int) -> torch.Tensor:
     if num_elems == 0:
         return out
     if row_splits.is_cuda:
-        with torch.cuda.device(row_splits.device):
+        with _lib.device_guard(row_splits.device):
             _lib.check(_lib.lib.k2b200_row_splits_to_row_ids(
                 _lib.ptr(row_splits), row_splits.shape[0] - 1, _lib.ptr(out), num_elems,
                 _lib.stream_of(row_splits.device)))
