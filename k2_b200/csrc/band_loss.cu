@@ -249,10 +249,11 @@ __global__ void BandIncoming(const BandState *__restrict__ tab, const BandArc *_
 // A graph that alternates (VitForm) takes 17 instructions per frame and warp: three shared-memory
 // reads, a shuffle (backward: two), ten adds and maxima, a 16-byte store; any other takes 45.
 // Bound by the latency of a frame where the batch is small (36 ns with the three warps of 240
-// states, 65 with the nine of 801) and by DRAM where it is large: 64 x 1000 frames of 500 classes
-// are 204 MB read and 186 MB written in 67 us.  (All arcs by the general expressions, rows
-// requested and waited for by the warps that walk: 86 us there, 124 instead of 99 for 16 x 1500
-// frames of up to 801 states.  Two states per thread: slower; eight: 99 us.)
+// states, 53 on average with the nine of 801) and by DRAM where it is large: 64 x 1000 frames of
+// 500 classes are 204 MB read and 140 MB written in 62 us.  Cells that no path can pass, a quarter of
+// these grids, are neither stored nor read, and a warp without others sits out (67 and 99 us for
+// 16 x 1500 frames with all of them; 86 and 124 with all arcs by the general expressions and rows
+// requested and waited for by the warps that walk).  Two states per thread: slower; eight: 99 us.
 // ---------------------------------------------------------------------------
 // The largest of three, NaN apart like fmaxf: one instruction.
 __device__ __forceinline__ float Max3(float a, float b, float c) {
@@ -466,6 +467,18 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
   const bool mine = dir == 0 ? lane >= H : lane < own;   // a lane that owns its states
   const bool stores = mine && s0 < pitch;
   float *grid = (dir == 0 ? vf : vb) + f.grid_off + s0;
+  // What is stored: four states s0 .. s0 + 3 of level l of R = T + 1 where one of them can lie on a
+  // path (arcs advance by at most two states: S - 1 - 2 (R - l) <= s <= 2 l).  BandPrep reads no
+  // others.  `at` is s0 - 2 l less the least that it may be.
+  const int32_t least = S - 1 - 2 * (T + 1) - (K - 1);
+  int32_t at = s0 - least - (dir == 0 ? 0 : 2 * (T + 1));
+  const uint32_t most = stores && least <= 0 ? (uint32_t)-least + 1u : 0u;
+  // Whether a warp has such states on any of the levels l0 .. l1; if not it sits out: its scores
+  // stay -inf, or nobody asks for them any more.
+  const int32_t warp_s0 = s0 - lane * K;
+  auto on_paths = [&](int32_t l0, int32_t l1) {
+    return warp_s0 <= 2 * l1 && warp_s0 + 32 * K - 1 >= S - 1 - 2 * (T + 1 - l0);
+  };
   float v[K];
 #pragma unroll
   for (int k = 0; k < K; ++k) v[k] = 0.0f;
@@ -506,7 +519,7 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
       }
       v[k] = s == 0 ? 0.0f : -INFINITY;
     }
-    if (stores) VitStore<K>(grid, v);
+    if ((uint32_t)at < most) VitStore<K>(grid, v);
     auto step = [&](auto alternates, const float (&a0)[K], const float (&a1)[K],
                     const float (&a2)[K], const float (&x)[K]) {
       const float h1 = __shfl_up_sync(kAll, v[K - 1], 1);
@@ -532,7 +545,8 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
 #pragma unroll
       for (int k = 0; k < K; ++k) v[k] = nv[k];
       grid += pitch;
-      if (stores) VitStore<K>(grid, v);
+      at -= 2;
+      if ((uint32_t)at < most) VitStore<K>(grid, v);
     };
     int32_t xpar = 0, slot = 0;
     auto walk = [&](auto alternates) {
@@ -551,6 +565,11 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
         const int32_t nf = min(F, T - q * F);
         const float *rowbuf = ring + (size_t)slot * slot_floats + words_off(q * F);
         if (++slot == nbatch) slot = 0;
+        if (!on_paths(q * F, q * F + nf)) {
+          grid += (int64_t)nf * pitch;
+          at -= 2 * nf;
+          continue;
+        }
         VitFrames<K>(nf, rowbuf, width, load,
                      [&](const float (&x)[K]) { step(alternates, w0, w1, w2, x); });
       }
@@ -620,7 +639,7 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
 #pragma unroll
     for (int k = 0; k < K; ++k) v[k] = (s0 + k == S - 1) ? 0.0f : -INFINITY;
     grid += (int64_t)(T + 1) * pitch;
-    if (stores) VitStore<K>(grid, v);
+    if ((uint32_t)at < most) VitStore<K>(grid, v);
     // A graph that alternates: what a state scores with its label's score is needed once, by it and
     // by its two predecessors, which get it by shuffles.
     auto short_step = [&](const float (&x)[K]) {
@@ -635,7 +654,8 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
         v[k + 1] = Max3(g[k + 1], g[k + 2], __fadd_rn(g[k + 3], skip[k + 3]));
       }
       grid -= pitch;
-      if (stores) VitStore<K>(grid, v);
+      at += 2;
+      if ((uint32_t)at < most) VitStore<K>(grid, v);
     };
     auto step = [&](const float (&w)[K][3], const float (&x)[K + 2]) {
       const float g1 = __shfl_down_sync(kAll, v[0], 1), g2 = __shfl_down_sync(kAll, v[1], 1);
@@ -652,7 +672,8 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
 #pragma unroll
       for (int k = 0; k < K; ++k) v[k] = nv[k];
       grid -= pitch;
-      if (stores) VitStore<K>(grid, v);
+      at += 2;
+      if ((uint32_t)at < most) VitStore<K>(grid, v);
     };
     {  // level T from level T + 1 through the implied final row (nothing to exchange yet:
        // only the final state is not -inf, and every lane knows it)
@@ -688,6 +709,11 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
         const float *rowbuf =
             ring + (size_t)slot * slot_floats + words_off(r0) + (size_t)(r1 - 1 - r0) * width;
         if (++slot == nbatch) slot = 0;
+        if (!on_paths(r0, r1)) {
+          grid -= (int64_t)(r1 - r0) * pitch;
+          at += 2 * (r1 - r0);
+          continue;
+        }
         VitFrames<kX>(r1 - r0, rowbuf, -width, load, [&](const float (&x)[kX]) {  // level r
           if constexpr (decltype(alternates)::value) short_step(x);         // from level r + 1
           else step(wo, x);
@@ -745,7 +771,8 @@ __global__ void PenaltyFlags(const BandState *__restrict__ tab, const BandArc *_
 // Keep tests and lists.  grid = (chunks of kPrepLevels levels, pairs), kPrepWarps warps per CTA,
 // which looks at the chunk's levels and the level on either side of them:
 //   1. a warp per level, four states per lane at a time: state s of level l survives iff
-//      vf[l][s] + vb[l][s] > cutoff (intersect_dense.cu:289-296).  Shared memory keeps, per
+//      vf[l][s] + vb[l][s] > cutoff (intersect_dense.cu:289-296); none does where BandViterbi stored
+//      nothing.  Shared memory keeps, per
 //      four states, their keep bits and the number of surviving states before them (together:
 //      the list position of a state), and the surviving states in order;
 //   2. a warp per 32 entries of a level: the reference's arc tests (intersect_dense.cu:430-471)
@@ -820,12 +847,15 @@ BandPrep(const BandInfo *__restrict__ infos, const int32_t *__restrict__ a_row_s
     const int32_t l = a - 1 + row;
     const bool there = l >= 0 && l <= b && l <= T + 1;
     const float *fr = fg + (int64_t)l * pitch + 4 * lane, *br = bg + (int64_t)l * pitch + 4 * lane;
+    // the states that BandViterbi stored
+    const int32_t first = S - 1 - 2 * (T + 1 - l) - 3, last = min(2 * l, S - 1);
     int32_t n = 0;
     for (int32_t g0 = 0; g0 < P; g0 += 512) {  // up to four groups of 128 states
       float4 x[4], y[4];
 #pragma unroll
       for (int g = 0; g < 4; ++g) {
-        const bool in = there && g0 + 128 * g + 4 * lane < S;  // (pitch covers the four states)
+        const int32_t s = g0 + 128 * g + 4 * lane;
+        const bool in = there && s >= first && s <= last;  // (pitch covers the four states)
         x[g] = y[g] = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
         if (in) {
           x[g] = *reinterpret_cast<const float4 *>(fr + g0 + 128 * g);
