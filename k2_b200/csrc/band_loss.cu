@@ -1872,12 +1872,17 @@ BandGrad(const BandInfo *__restrict__ infos, const BandArc *__restrict__ tabf,
 // The same gradient for log-probs (or logits) that no two sequences share, written whole:
 // every element of the rows of a sequence and of the rows up to the next one is stored
 // once, so the caller's buffer needs no clearing (at 128 MB of log-probs the clear and the
-// scattered additions took 29 + 26 us of memory time, this takes 30).  A warp per kDenseRows
+// scattered additions took 29 + 26 us of memory time, this takes 36).  A warp per DenseRows
 // rows; the row's sums gather in shared memory in fixed point as in BandGrad.  A CTA sees to the
 // `width` columns from blockIdx.z * width on.  kSoftmax: the rows are log_softmax of the tensor
 // the gradient is for, d = g - softmax * sum(g).
 // ---------------------------------------------------------------------------
-constexpr int kDenseRows = 4;
+// Rows whose entries a warp requests together: two, twelve CTAs to an SM, and one, sixteen, where a
+// row is read as well.  Bound by the chain list -> entries -> sums -> row of a warp beside the
+// stores (the rows alone would take 22 of the 36 us of 64 x 1000 frames, 50 of 62 of 32 x 500 x
+// 5000), so more warps with less each: with four rows and eight CTAs 37, 65 us, and 27 instead of 21
+// from the logits of 32 x 600 x 501.
+__host__ __device__ constexpr int DenseRows(bool softmax) { return softmax ? 1 : 2; }
 // Columns of a range.  A warp stores its range alone, so a wide one leaves an SM few warps: 60 000
 // columns x 2400 rows took 288 us (logits 4625) in ranges of 51 200, what fits in shared memory,
 // 139 (678) in ranges of 6400, 139 (320) in ranges of 1600; up to 6400 columns the gradient of
@@ -1885,7 +1890,7 @@ constexpr int kDenseRows = 4;
 constexpr int kGradColumns = 6400;
 
 template <bool kSoftmax>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, kSoftmax ? 16 : 12)
 BandGradRows(const BandInfo *__restrict__ infos, const float *__restrict__ lp,
              const BandItem *__restrict__ items, const int2 *__restrict__ lists,
              const double *__restrict__ am, const int32_t *__restrict__ ae,
@@ -1895,6 +1900,7 @@ BandGradRows(const BandInfo *__restrict__ infos, const float *__restrict__ lp,
              const GradSpec upstream, float *__restrict__ grad, int32_t C, int32_t width) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr unsigned kAll = 0xffffffffu;
+  constexpr int kDenseRows = DenseRows(kSoftmax);
   const int32_t i = blockIdx.y;
   const BandInfo f = infos[i];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -2592,7 +2598,7 @@ int32_t k2b200_band_loss_backward_dense(const k2b200_band_loss_args *args, void 
     auto kernel = softmax ? BandGradRows<true> : BandGradRows<false>;
     K2B_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)kBandSmemBudget));
-    dim3 grid(CeilDiv(std::max(L.max_rows, 1), warps * kDenseRows), args->num_fsas,
+    dim3 grid(CeilDiv(std::max(L.max_rows, 1), warps * DenseRows(softmax)), args->num_fsas,
               CeilDiv(C, width));
     { kernel<<<grid, 32 * warps, row_bytes * warps, stream>>>(
         reinterpret_cast<const BandInfo *>(ws + L.off_infos), args->log_probs,
