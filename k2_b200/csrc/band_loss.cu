@@ -2013,7 +2013,11 @@ BandGradRows(const BandInfo *__restrict__ infos, const float *__restrict__ lp,
 }
 
 // log_probs rows of the sequences = log_softmax of the logits rows.  A warp per row; the same
-// expressions as LogSoftmaxFill (dense.cu).
+// expressions as LogSoftmaxFill (dense.cu).  kPer: a row of at most 32 * kPer columns is read once and
+// held in registers, 0: it is read three times, from L1 after the first.  Bound by the latency of a
+// row's reads and reductions (32 x 600 x 501: 18 us reading three times, 13 once; 8 would be the
+// memory's).
+template <int kPer>
 __global__ void __launch_bounds__(256)
 LogSoftmaxRows(const BandInfo *__restrict__ infos, const float *__restrict__ logits, int32_t C,
                float *__restrict__ log_probs) {
@@ -2022,19 +2026,37 @@ LogSoftmaxRows(const BandInfo *__restrict__ infos, const float *__restrict__ log
   if (r >= f.frames) return;
   const float *in = logits + (int64_t)(f.lp_row + r) * C;
   float *out = log_probs + (int64_t)(f.lp_row + r) * C;
-  float mx = -INFINITY;
+  float x[kPer > 0 ? kPer : 1], mx = -INFINITY, sum = 0.0f;
+  if (kPer > 0) {
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) x[k] = lane + 32 * k < C ? __ldg(in + lane + 32 * k) : -INFINITY;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) mx = fmaxf(mx, x[k]);
+  } else {
 #pragma unroll 4
-  for (int32_t c = lane; c < C; c += 32) mx = fmaxf(mx, __ldg(in + c));
+    for (int32_t c = lane; c < C; c += 32) mx = fmaxf(mx, __ldg(in + c));
+  }
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, d));
-  float sum = 0.0f;
+  if (kPer > 0) {
+#pragma unroll
+    for (int k = 0; k < kPer; ++k)
+      if (lane + 32 * k < C) sum += expf(x[k] - mx);
+  } else {
 #pragma unroll 4
-  for (int32_t c = lane; c < C; c += 32) sum += expf(__ldg(in + c) - mx);
+    for (int32_t c = lane; c < C; c += 32) sum += expf(__ldg(in + c) - mx);
+  }
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
   const float lse = logf(sum);
+  if (kPer > 0) {
+#pragma unroll
+    for (int k = 0; k < kPer; ++k)
+      if (lane + 32 * k < C) out[lane + 32 * k] = (x[k] - mx) - lse;
+  } else {
 #pragma unroll 4
-  for (int32_t c = lane; c < C; c += 32) out[c] = (__ldg(in + c) - mx) - lse;
+    for (int32_t c = lane; c < C; c += 32) out[c] = (__ldg(in + c) - mx) - lse;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -2391,7 +2413,13 @@ int32_t k2b200_band_loss_forward_reduce(const k2b200_band_loss_args *args, void 
   if (logits != nullptr && L.max_frames > 0) {
     PhaseTimer timer(kPhaseDense, stream);
     dim3 grid(CeilDiv(L.max_frames, 8), args->num_fsas);
-    { LogSoftmaxRows<<<grid, 256, 0, stream>>>(
+    const int32_t C = args->num_classes;
+    auto kernel = C <= 128    ? LogSoftmaxRows<4>
+                  : C <= 256  ? LogSoftmaxRows<8>
+                  : C <= 512  ? LogSoftmaxRows<16>
+                  : C <= 1024 ? LogSoftmaxRows<32>
+                              : LogSoftmaxRows<0>;
+    { kernel<<<grid, 256, 0, stream>>>(
         reinterpret_cast<const BandInfo *>(ws + L.off_infos), logits, args->num_classes,
         const_cast<float *>(args->log_probs)); NoteLaunch(); }
   }

@@ -237,6 +237,25 @@ def test_graphs_that_alternate_and_graphs_that_nearly_do(tokens, frames, classes
     compare(a, lp, seg, 8.0, tag=change)
 
 
+@pytest.mark.parametrize("classes", [3, 128, 129, 256, 257, 512, 513, 1024, 1025])
+def test_logits_rows_at_the_edges_of_what_a_warp_holds(classes):
+    # a row is held in 4, 8, 16 or 32 registers per lane, or read three times.  Both sides round
+    # log-probs of magnitude < 16 to float32 (1e-6), on 24 frames; posteriors follow exp of that
+    import k2_b200 as k2
+    from k2_b200.fsa_algo import ctc_graph
+    rng = np.random.default_rng(classes)
+    x = torch.from_numpy(rng.normal(size=(2, 24, classes)).astype(np.float32) * 2).to(DEV)
+    seg = torch.tensor([[1, 0, 24], [0, 3, 17]], dtype=torch.int32)
+    graphs = ctc_graph([rng.integers(1, classes, size=5).tolist() for _ in range(2)], device=DEV)
+    got, want = x.clone().requires_grad_(True), x.clone().requires_grad_(True)
+    a = k2.ctc_loss(graphs, k2.DenseFsaVec.from_logits(got, seg), 8.0)
+    b = k2.ctc_loss(graphs, k2.DenseFsaVec(torch.log_softmax(want, -1), seg), 8.0)
+    a.backward()
+    b.backward()
+    assert abs(a.item() - b.item()) <= 24 * 2e-6 * 2 + 1e-6 * abs(b.item())
+    assert (got.grad - want.grad).abs().max().item() <= 24 * 2e-6
+
+
 def test_summed_ctc_loss_as_one_node_equals_the_composition():
     # ctc_loss(reduction="sum") on the band path is one autograd node; the same numbers
     # and gradients as -tot_scores.sum() composed from its parts, for a loss that is scaled
