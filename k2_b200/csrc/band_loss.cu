@@ -38,6 +38,12 @@
 //   BandGrad      the same added to rows that sequences share, and arc posteriors for the
 //                 gradient of the graph's arc scores.
 //
+// Each of these kernels waits for the one before it and is set up while that one still runs
+// (LaunchBehind): 5 to 8 us of a pass.  BandViterbi and BandChainLists, whose CTAs are all resident
+// from the start, let the next one start at once, BandPrep does near its end.  BandGather and
+// LogSoftmaxRows do not: BandViterbi's CTAs then took what room there was beside theirs, two to an
+// SM (32 x 500 x 5000: 241 us a pass instead of 225).
+//
 // The dense scores are read straight from the log-prob tensor the DenseFsaVec was made from
 // ([rows, C], any C): the [rows + N, C + 1] score matrix is not needed.  The extra
 // final row of a sequence ([0, -inf, ...], k2/csrc/fsa.h:138-185) is implied: on the level after
@@ -305,6 +311,7 @@ __global__ void __launch_bounds__(256)
 BandGather(const BandInfo *__restrict__ infos, const BandState *__restrict__ tab,
            const float *__restrict__ lp, int32_t C, float *__restrict__ by_state) {
   __shared__ int32_t label_sh[kBandMaxStates];
+  WaitForPrevious();
   const BandInfo f = infos[blockIdx.y];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int32_t r0 = blockIdx.x * kGatherRows, r1 = min(r0 + kGatherRows, f.frames), S = f.num_states;
@@ -393,6 +400,8 @@ BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ ta
   __shared__ int32_t any_late;
   constexpr unsigned kAll = 0xffffffffu;
   const int dir = blockIdx.x;
+  WaitForPrevious();
+  LetNextStart();
   const BandInfo f = infos[blockIdx.y];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int32_t S = f.num_states, T = f.frames, pitch = f.pitch;
@@ -819,6 +828,7 @@ BandPrep(const BandInfo *__restrict__ infos, const int32_t *__restrict__ a_row_s
   __shared__ uint32_t counts_sh[2];
   __shared__ int32_t n_sh[kPrepSpan];
   const int32_t i = blockIdx.y;
+  WaitForPrevious();
   const BandInfo f = infos[i];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int32_t S = f.num_states, T = f.frames, pitch = f.pitch;
@@ -1049,6 +1059,7 @@ BandPrep(const BandInfo *__restrict__ infos, const int32_t *__restrict__ a_row_s
   }
   if (risky) risky_sh = 1;
   __syncthreads();
+  LetNextStart();
   // ---- 3. leaving arcs --------------------------------------------------------------------
   for (int32_t k = warp; k < b - a; k += kPrepWarps) {
     const int32_t row = k + 1, n = n_sh[row];
@@ -1472,6 +1483,8 @@ BandChainLists(const BandInfo *__restrict__ infos, const BandFactor *__restrict_
   __shared__ unsigned char crc[kChainMaxChunks];
   const int dir = blockIdx.x;
   const int32_t i = blockIdx.y;
+  WaitForPrevious();
+  LetNextStart();
   const BandInfo f = infos[i];
   if (dir == 0 && threadIdx.x == 0) {
     tot[i] = -INFINITY;
@@ -1676,6 +1689,7 @@ BandChainExact(const BandInfo *__restrict__ infos, const BandArc *__restrict__ t
                const int32_t *__restrict__ unfit, int32_t *__restrict__ status, int32_t st_pad,
                int32_t lv_pad, int32_t wait_limit, LossSpec spec, uint32_t *__restrict__ ticket,
                const BandState *__restrict__ tab, DelaySpec delay) {
+  WaitForPrevious();
   if (unfit[blockIdx.y] != 0)
     ExactWalk(infos, tabf, lp, C, items, lists, am, ae, bm, be, tot, total, unfit, status, st_pad,
               lv_pad, wait_limit, tab, delay);
@@ -1902,6 +1916,7 @@ BandGradRows(const BandInfo *__restrict__ infos, const float *__restrict__ lp,
   constexpr unsigned kAll = 0xffffffffu;
   constexpr int kDenseRows = DenseRows(kSoftmax);
   const int32_t i = blockIdx.y;
+  WaitForPrevious();
   const BandInfo f = infos[i];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int32_t T = f.frames, rows = f.zero_end - f.lp_row;
@@ -2021,6 +2036,7 @@ template <int kPer>
 __global__ void __launch_bounds__(256)
 LogSoftmaxRows(const BandInfo *__restrict__ infos, const float *__restrict__ logits, int32_t C,
                float *__restrict__ log_probs) {
+  WaitForPrevious();
   const BandInfo f = infos[blockIdx.y];
   const int32_t r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (r >= f.frames) return;
@@ -2260,18 +2276,18 @@ static int32_t LaunchBandChains(const BandLayout &L, const k2b200_band_loss_args
   BandTotal *total = reinterpret_cast<BandTotal *>(ws + L.off_total);
   int32_t *unfit = reinterpret_cast<int32_t *>(ws + L.off_unfit);
   int32_t *status = reinterpret_cast<int32_t *>(ws + L.off_status);
-  { BandChainLists<<<grid, kChainThreads + kKeepThreads, L.chain_smem, stream>>>(
+  { K2B_CUDA_OK(LaunchBehind(BandChainLists, grid, kChainThreads + kKeepThreads, L.chain_smem, stream, 
       infos, reinterpret_cast<const BandFactor *>(ws + L.off_factors),
       reinterpret_cast<const int32_t *>(ws + L.off_chunk_r), am, bm,
       reinterpret_cast<int32_t *>(ws + L.off_a_scale),
       reinterpret_cast<int32_t *>(ws + L.off_b_scale), tot_scores, total, unfit, status,
-      CopyWaitLimit()); NoteLaunch(); }
-  { BandChainExact<<<grid, kExactThreads, L.exact_smem, stream>>>(
+      CopyWaitLimit())); NoteLaunch(); }
+  { K2B_CUDA_OK(LaunchBehind(BandChainExact, grid, kExactThreads, L.exact_smem, stream, 
       infos, reinterpret_cast<const BandArc *>(args->band_arcs), args->log_probs,
       args->num_classes, items, lists, am, reinterpret_cast<int32_t *>(ws + L.off_ae), bm,
       reinterpret_cast<int32_t *>(ws + L.off_be), tot_scores, total, unfit, status, L.st_pad,
       L.lv_pad, CopyWaitLimit(), spec, reinterpret_cast<uint32_t *>(ws + L.off_totals + 48),
-      reinterpret_cast<const BandState *>(args->band_states), delay);
+      reinterpret_cast<const BandState *>(args->band_states), delay));
     NoteLaunch(); }
   K2B_CUDA_OK(cudaGetLastError());
   return kOk;
@@ -2419,9 +2435,9 @@ int32_t k2b200_band_loss_forward_reduce(const k2b200_band_loss_args *args, void 
                   : C <= 512  ? LogSoftmaxRows<16>
                   : C <= 1024 ? LogSoftmaxRows<32>
                               : LogSoftmaxRows<0>;
-    { kernel<<<grid, 256, 0, stream>>>(
+    { K2B_CUDA_OK(LaunchBehind(kernel, grid, 256, 0, stream, 
         reinterpret_cast<const BandInfo *>(ws + L.off_infos), logits, args->num_classes,
-        const_cast<float *>(args->log_probs)); NoteLaunch(); }
+        const_cast<float *>(args->log_probs))); NoteLaunch(); }
   }
   {
     PhaseTimer timer(kPhaseViterbi, stream);
@@ -2433,8 +2449,8 @@ int32_t k2b200_band_loss_forward_reduce(const k2b200_band_loss_args *args, void 
     const BandState *tab = reinterpret_cast<const BandState *>(args->band_states);
     if (L.by_state && L.max_frames > 0) {
       dim3 grid(CeilDiv(L.max_frames, kGatherRows), args->num_fsas);
-      { BandGather<<<grid, 256, 0, stream>>>(infos, tab, args->log_probs, args->num_classes,
-                                             reinterpret_cast<float *>(ws + L.off_by_state));
+      { K2B_CUDA_OK(LaunchBehind(BandGather, grid, 256, 0, stream, infos, tab, args->log_probs, args->num_classes,
+                                             reinterpret_cast<float *>(ws + L.off_by_state)));
         NoteLaunch(); }
     }
     const uintptr_t lp_begin = reinterpret_cast<uintptr_t>(args->log_probs),
@@ -2446,12 +2462,12 @@ int32_t k2b200_band_loss_forward_reduce(const k2b200_band_loss_args *args, void 
     K2B_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)L.viterbi_smem));
     dim3 grid(2, args->num_fsas);
-    { kernel<<<grid, L.vit_threads, L.viterbi_smem, stream>>>(
+    { K2B_CUDA_OK(LaunchBehind(kernel, grid, L.vit_threads, L.viterbi_smem, stream, 
         infos, tab,
         L.by_state ? reinterpret_cast<const float *>(ws + L.off_by_state) : args->log_probs,
         args->log_prob_rows, args->num_classes, reinterpret_cast<float *>(ws + L.off_vf),
         reinterpret_cast<float *>(ws + L.off_vb), L.vit_frames, L.vit_batches, L.vit_slot,
-        L.xch_pad, CopyWaitLimit(), reinterpret_cast<int32_t *>(ws + L.off_status));
+        L.xch_pad, CopyWaitLimit(), reinterpret_cast<int32_t *>(ws + L.off_status)));
       NoteLaunch(); }
     K2B_CUDA_OK(cudaGetLastError());
   }
@@ -2481,7 +2497,7 @@ int32_t k2b200_band_loss_forward_reduce(const k2b200_band_loss_args *args, void 
       NotePhaseKernel(kPhasePrune, "BandPrep");
       dim3 grid(CeilDiv(L.max_frames + 2, kPrepLevels), args->num_fsas);
       auto prep = delay.penalty != 0.0f ? BandPrep<true> : BandPrep<false>;
-      { prep<<<grid, 32 * kPrepWarps, L.prep_smem, stream>>>(
+      { K2B_CUDA_OK(LaunchBehind(prep, grid, 32 * kPrepWarps, L.prep_smem, stream, 
           reinterpret_cast<const BandInfo *>(ws + L.off_infos), args->a_row_splits2,
           reinterpret_cast<const BandState *>(args->band_states),
           reinterpret_cast<const BandArc *>(args->band_arcs), args->log_probs,
@@ -2495,7 +2511,7 @@ int32_t k2b200_band_loss_forward_reduce(const k2b200_band_loss_args *args, void 
           reinterpret_cast<int32_t *>(ws + L.off_chunk_r),
           reinterpret_cast<unsigned long long *>(ws + L.off_totals),
           reinterpret_cast<int32_t *>(ws + L.off_unfit),
-          L.arc_frames > args->max_arcs ? 1 : 0, delay); NoteLaunch(); }
+          L.arc_frames > args->max_arcs ? 1 : 0, delay)); NoteLaunch(); }
       // the host reads the counts behind BandPrep, while what follows runs
       if (need_count) {
         K2B_FORWARD(SideFork(stream, &side));
@@ -2628,7 +2644,7 @@ int32_t k2b200_band_loss_backward_dense(const k2b200_band_loss_args *args, void 
                                      (int)kBandSmemBudget));
     dim3 grid(CeilDiv(std::max(L.max_rows, 1), warps * DenseRows(softmax)), args->num_fsas,
               CeilDiv(C, width));
-    { kernel<<<grid, 32 * warps, row_bytes * warps, stream>>>(
+    { K2B_CUDA_OK(LaunchBehind(kernel, grid, 32 * warps, row_bytes * warps, stream, 
         reinterpret_cast<const BandInfo *>(ws + L.off_infos), args->log_probs,
         reinterpret_cast<const BandItem *>(ws + L.off_items),
         reinterpret_cast<const int2 *>(ws + L.off_lists),
@@ -2639,7 +2655,7 @@ int32_t k2b200_band_loss_backward_dense(const k2b200_band_loss_args *args, void 
         reinterpret_cast<const int32_t *>(ws + L.off_a_scale),
         reinterpret_cast<const int32_t *>(ws + L.off_b_scale),
         reinterpret_cast<const BandTotal *>(ws + L.off_total),
-        reinterpret_cast<const int32_t *>(ws + L.off_unfit), spec, grad_log_probs, C, width);
+        reinterpret_cast<const int32_t *>(ws + L.off_unfit), spec, grad_log_probs, C, width));
       NoteLaunch(); }
     K2B_CUDA_OK(cudaGetLastError());
   }

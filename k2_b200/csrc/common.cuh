@@ -113,6 +113,32 @@ struct SideReadBackScope {
   bool held_ = false;
 };
 
+// Kernels of one stream that follow each other closely: a kernel launched with LaunchBehind may be
+// set up while the one before it still runs, from when all its CTAs have called LetNextStart() (or
+// have ended).  It calls WaitForPrevious() before it touches memory; behind that everything is as if
+// it had been launched in the usual way.
+__device__ __forceinline__ void WaitForPrevious() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void LetNextStart() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename... Params, typename... Args>
+static cudaError_t LaunchBehind(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
+                                cudaStream_t stream, Args &&...args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 static inline size_t AlignUp(size_t x, size_t a = 256) { return (x + a - 1) / a * a; }
 
 static inline int CeilDiv(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
