@@ -678,6 +678,14 @@ int32_t k2b200_tot_scores_log_backward(const int32_t *row_ids1, const int32_t *r
                                        int64_t grad_stride, float *arc_grad,
                                        void *stream);
 
+/* k2b200_fsa_arc_post and k2b200_tot_scores_log_backward in one pass, without the posteriors. */
+int32_t k2b200_tot_scores_log_backward_scores(const int32_t *row_splits1, const int32_t *row_ids1,
+                                              const int32_t *row_ids2, const void *arcs,
+                                              int32_t num_arcs, int32_t use_double,
+                                              const void *forward, const void *backward,
+                                              const void *tot_scores_grad, int64_t grad_stride,
+                                              float *arc_grad, void *stream);
+
 /* grad (zero-filled here) gets tot_scores_grad[fsa] on the arcs of the best
  * paths.  Replaces GetTotScoresTropicalBackward,
  * k2/python/csrc/torch/fsa.cu:493-534. */

@@ -233,6 +233,8 @@ _sig("k2b200_fsa_arc_post", c_i32,
      [c_vp, c_vp, c_vp, c_vp, c_i32, c_i32, c_i32, c_vp, c_vp, c_vp, c_vp])
 _sig("k2b200_tot_scores_log_backward", c_i32,
      [c_vp, c_vp, c_i32, c_i32, c_vp, c_vp, c_i64, c_vp, c_vp])
+_sig("k2b200_tot_scores_log_backward_scores", c_i32,
+     [c_vp, c_vp, c_vp, c_vp, c_i32, c_i32, c_vp, c_vp, c_vp, c_i64, c_vp, c_vp])
 _sig("k2b200_tot_scores_tropical_backward", c_i32,
      [c_vp, c_vp, c_i32, c_vp, c_i32, c_i32, c_vp, c_i64, c_vp, c_vp])
 _sig("k2b200_index_add", c_i32, [c_vp, c_vp, c_i32, c_vp, c_i64, c_vp])
@@ -278,6 +280,7 @@ EXPORTED = [
     "k2b200_intersect_dense_prune", "k2b200_intersect_dense_emit", "k2b200_fsa_scores",
     "k2b200_fsa_scores_scratch_bytes", "k2b200_fsa_scores_dir_scratch_bytes",
     "k2b200_fsa_tot_scores", "k2b200_fsa_arc_post", "k2b200_tot_scores_log_backward",
+    "k2b200_tot_scores_log_backward_scores",
     "k2b200_tot_scores_tropical_backward", "k2b200_index_add", "k2b200_index_select_i32",
     "k2b200_shortest_path_tmp_bytes", "k2b200_shortest_path", "k2b200_best_paths_tmp_bytes",
     "k2b200_best_paths",

@@ -182,6 +182,14 @@ class _GetTotScoresFunction(torch.autograd.Function):
                     _lib.ptr(rid1), _lib.ptr(rid2), na, _lib.ptr(best_arcs), best_arcs.numel(),
                     int(use_double_scores), _lib.ptr(tot_scores_grad), stride,
                     _lib.ptr(scores_grad), _lib.stream_of(dev)))
+            elif fsas._score_key('arc_post', use_double_scores, True) not in fsas._cache:
+                fwd = fsas._get_forward_scores(use_double_scores, log_semiring)
+                bwd = fsas._get_backward_scores(use_double_scores, log_semiring)
+                _lib.check(_lib.lib.k2b200_tot_scores_log_backward_scores(
+                    _lib.ptr(arcs._row_splits1), _lib.ptr(rid1), _lib.ptr(rid2),
+                    _lib.ptr(arcs.values()), na, int(use_double_scores), _lib.ptr(fwd),
+                    _lib.ptr(bwd), _lib.ptr(tot_scores_grad), stride, _lib.ptr(scores_grad),
+                    _lib.stream_of(dev)))
             else:
                 arc_post = fsas._get_arc_post(use_double_scores, log_semiring)
                 _lib.check(_lib.lib.k2b200_tot_scores_log_backward(
@@ -339,12 +347,16 @@ class _IntersectDenseFunction(torch.autograd.Function):
         a_scores, b_scores = ctx.saved_tensors
         arc_map_a = ctx.arc_map_a
         arc_map_b = ctx.arc_map_b
-        grad_a = torch.zeros(a_scores.size(0), dtype=torch.float32, device=a_scores.device,
-                             requires_grad=False)
-        grad_b = torch.zeros(*b_scores.shape, dtype=torch.float32, device=b_scores.device,
-                             requires_grad=False).contiguous()
-        _index_add(arc_map_a, out_fsa_grad, grad_a)
-        _index_add(arc_map_b, out_fsa_grad, grad_b.view(-1))
+        # (graphs without a gradient, a denominator's, need no additions: 33 us of 3.3 M arcs)
+        grad_a = grad_b = None
+        if ctx.needs_input_grad[6]:
+            grad_a = torch.zeros(a_scores.size(0), dtype=torch.float32, device=a_scores.device,
+                                 requires_grad=False)
+            _index_add(arc_map_a, out_fsa_grad, grad_a)
+        if ctx.needs_input_grad[7]:
+            grad_b = torch.zeros(*b_scores.shape, dtype=torch.float32, device=b_scores.device,
+                                 requires_grad=False).contiguous()
+            _index_add(arc_map_b, out_fsa_grad, grad_b.view(-1))
         return (None, None, None, None, None, None, grad_a, grad_b, None, None, None)
 
 

@@ -363,6 +363,39 @@ def test_beam_shrinks_when_limits_hit(k2):
         assert abs(lat.arcs.output_beam_used - want.extra["final_beam"]) < 1e-6
 
 
+@pytest.mark.parametrize("double", [True, False])
+@pytest.mark.parametrize("expanded", [True, False])
+def test_gradient_of_totals_with_and_without_the_posteriors(k2, double, expanded):
+    # one pass over the arcs, or (where the posteriors are there already) two: the same bits; graphs
+    # and scores want a gradient or do not
+    from gpu_util import host_to_fsa
+    rng = np.random.default_rng(7)
+    a = random_fsa_vec(rng, 5, acyclic=True)
+    got = []
+    for first in (False, True):
+        fsa = host_to_fsa(a)
+        fsa.scores.requires_grad_(True)
+        if first:
+            fsa.get_arc_post(double, True)
+        tot = fsa.get_tot_scores(double, True)
+        weight = torch.ones_like(tot) if expanded else torch.arange(5, device="cuda").to(tot)
+        ok = torch.isfinite(tot.detach())
+        (tot.sum() if expanded and bool(ok.all()) else (tot[ok] * weight[ok]).sum()).backward()
+        got.append(fsa.scores.grad)
+    assert torch.equal(got[0].nan_to_num(7.0), got[1].nan_to_num(7.0))
+    scores, brs = random_dense(rng, 5, 10, 5)
+    from gpu_util import dense_from_scores
+    grads = []
+    for graph, dense in ((True, True), (True, False), (False, True)):
+        fsa, b = host_to_fsa(a), dense_from_scores(scores, brs, requires_grad=dense)
+        fsa.scores.requires_grad_(graph)
+        k2.intersect_dense(fsa, b, 10.0).scores.sum().backward()
+        grads.append((fsa.scores.grad, b.scores.grad))
+    assert grads[1][1] is None and grads[2][0] is None
+    torch.testing.assert_close(grads[0][0], grads[1][0], rtol=1e-6, atol=1e-6)
+    torch.testing.assert_close(grads[0][1], grads[2][1], rtol=1e-6, atol=1e-6)
+
+
 def test_generic_ragged_ops(k2):
     import ctypes
     from gpu_util import DEV
