@@ -37,6 +37,8 @@ constexpr float kMaxScore = 300.0f;   // |arc score|: exp() within 2^+-433
 constexpr int kRangeExp = 280;        // values that are not zero stay within 2^+-280, so that no
                                       // product of one with a factor and a scale underflows
 constexpr int kMaxSlots = 8;
+constexpr int kWideTeam = 8, kWideWarps = 16;  // CTAs that share a layer, warps of each
+constexpr int kWideRecs = 2;                   // records of a lane ahead
 constexpr int kSliceMaxStates = 16384;  // states of a sliced layer
 
 struct __align__(16) LayerArc {
@@ -205,7 +207,7 @@ struct ChainPlan {
   // sliced layers
   int32_t rows, slots, slot_bytes;
   // wide layers
-  int32_t wide, team;
+  int32_t wide, team, cells;
   size_t bytes;
   bool ok;
 };
@@ -249,13 +251,19 @@ static ChainPlan PlanChain(const k2b200_fsa_view *v, int32_t ndir) {
   }
   // Layers too wide for that are shared by a cluster of CTAs.
   p.wide = 1;
-  p.warps = 16;
+  p.warps = kWideWarps;
   p.team = 1;
-  while (p.team < 8 && (int64_t)ndir * v->num_fsas * p.team * 2 <= NumSms() &&
+  while (p.team < kWideTeam && (int64_t)ndir * v->num_fsas * p.team * 2 <= NumSms() &&
          p.team * 32 * p.warps < v->max_layer_states)
     p.team *= 2;
-  p.bytes = sizeof(int32_t) * (size_t)((p.nl_cap + 1 + 3) & ~3);
+  p.bytes = sizeof(int32_t) * (size_t)((p.nl_cap + 1 + 3) & ~3) +
+            2 * sizeof(LayerArc) * kWideRecs * 32 * kWideWarps;
   p.ok = p.bytes <= kLayerSmemBudget;
+  if (p.ok) {  // as many states of two layers as there is room for
+    p.cells = (int32_t)std::min<int64_t>(
+        p.maxw, (int64_t)(kLayerSmemBudget - p.bytes) / (2 * sizeof(double)) & ~1);
+    p.bytes += 2 * sizeof(double) * (size_t)p.cells;
+  }
   return p;
 }
 
@@ -546,19 +554,19 @@ struct StateSum {
   // arcs k, k + step, ... below k1; rec(k) and val(record) fetch
   template <typename Rec, typename Value>
   __device__ __forceinline__ void Walk(int32_t k, int32_t k1, int32_t step, Rec rec, Value val) {
-    for (; k + 3 * step < k1; k += 4 * step) {
+#pragma unroll 1
+    for (; k < k1; k += 4 * step) {
       LayerArc r[4];
       Val x[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) r[u] = rec(k + u * step);
+      for (int u = 0; u < 4; ++u)
+        if (k + u * step < k1) r[u] = rec(k + u * step);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) x[u] = val(r[u]);
+      for (int u = 0; u < 4; ++u)
+        if (k + u * step < k1) x[u] = val(r[u]);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) Add(r[u], x[u]);
-    }
-    for (; k < k1; k += step) {
-      const LayerArc r = rec(k);
-      Add(r, val(r));
+      for (int u = 0; u < 4; ++u)
+        if (k + u * step < k1) Add(r[u], x[u]);
     }
   }
   // The states of the lanes in `heavy` (their arcs k0 .. k1 - 1), the whole warp on one at a
@@ -579,7 +587,7 @@ struct StateSum {
 };
 
 // The shared power of two of the log semiring: 2^K, replaced every kRescale layers by the
-// exponent of the largest value since.  hi_slots: two words that the CTAs of a chain share.
+// exponent of the largest value since.  hi_slots: two words that the warps of a CTA share.
 template <bool kLog>
 struct ChainScale {
   double mul = 1.0;
@@ -590,13 +598,22 @@ struct ChainScale {
     mul = 1.0;
     const int at = (step / kRescale) & 1;
     if (step % kRescale == 0 && step > 0) {
-      const int32_t hm = *reinterpret_cast<volatile int32_t *>(&hi_slots[at ^ 1]);
-      const int32_t e = hm > 0 ? (hm >> 20) - 1023 : 0;
-      K += e;
-      mul = __longlong_as_double((long long)(1023 - e) << 52);
+      Rescale(*reinterpret_cast<volatile int32_t *>(&hi_slots[at ^ 1]));
     }
     if (step % kRescale == 1 && first_thread)
       *reinterpret_cast<volatile int32_t *>(&hi_slots[at ^ 1]) = 0;
+  }
+  __device__ __forceinline__ void Rescale(int32_t hm) {
+    const int32_t e = hm > 0 ? (hm >> 20) - 1023 : 0;
+    K += e;
+    mul = __longlong_as_double((long long)(1023 - e) << 52);
+  }
+  // the largest of a warp's values since the last change, and 0 again
+  __device__ __forceinline__ int32_t TakeMax(int lane, int32_t *status) {
+    const int32_t hm = __reduce_max_sync(0xffffffffu, hi_max);
+    if (hm >= (1023 + kRangeExp) << 20 && lane == 0) atomicOr(status, 4);
+    hi_max = 0;
+    return hm;
   }
   __device__ __forceinline__ void Note(double x) {  // x >= 0
     if (!kLog) return;
@@ -607,10 +624,8 @@ struct ChainScale {
   __device__ __forceinline__ void EndLayer(int32_t step, int32_t *hi_slots, int lane,
                                            int32_t *status) {
     if (!kLog || step % kRescale != kRescale - 1) return;
-    const int32_t hm = __reduce_max_sync(0xffffffffu, hi_max);
+    const int32_t hm = TakeMax(lane, status);
     if (lane == 0 && hm > 0) atomicMax(&hi_slots[(step / kRescale) & 1], hm);
-    if (hm >= (1023 + kRangeExp) << 20 && lane == 0) atomicOr(status, 4);
-    hi_max = 0;
   }
   __device__ __forceinline__ void End(int lane, int32_t *status) {
     if (!kLog) return;
@@ -1063,32 +1078,75 @@ ExactChain(k2b200_fsa_view v, const uint4 *__restrict__ pool, const SliceDesc *_
   }
 }
 
+// What the CTAs of a chain hand one another: stores into another CTA's shared memory that count
+// as bytes on its barrier, so that nothing is fenced and nobody waits but the reader.  Addresses
+// are those of the cluster's window.
+__device__ __forceinline__ uint32_t InRank(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void StoreAsync(uint32_t addr, int32_t x, uint32_t bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(
+                   addr),
+               "r"(x), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void StoreAsync(uint32_t addr, float x, uint32_t bar) {
+  StoreAsync(addr, __float_as_int(x), bar);
+}
+__device__ __forceinline__ void StoreAsync(uint32_t addr, double x, uint32_t bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(
+                   addr),
+               "l"(__double_as_longlong(x)), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void ClusterSync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 // The same for layers too wide for the ring: the CTAs of a cluster share a layer.  grid =
-// (directions x team, fsas).  Splits, records and the values of the layer before come from
-// L2; what does not depend on values is fetched a layer ahead, the records of up to four arcs
-// per lane among it.  A state has 1, 2, 4 or 8 lanes, as many as the width of the layer leaves
-// it, so that few states have more arcs than that: a layer costs one gather and one
-// cluster barrier, a microsecond each.  (One lane per state with one record ahead, and states
-// of more than four arcs one after the other by a whole warp: 3 us per layer of a
-// lattice of 152 layers, now 2.1.)
+// (directions x team, fsas).  A state has 1, 2, 4 or 8 lanes, as many as the width of the layer
+// leaves it, so that few states have more arcs than the records, up to two per lane, that are
+// copied to shared memory two layers ahead (as many again are brought to L1).
+//
+// Every CTA has the values of the last two layers in its shared memory: a lane that has a value
+// stores it into all of them, and every warp a word beside it (the largest value it has seen),
+// each layer.  A layer is complete where all its bytes have come, and then everybody is past
+// the layer before, whose place the next one takes.  All else (global stores, records, splits)
+// is between a warp's stores and its wait.  Layers of more than `p.cells` states go through L2, with
+// a barrier of the cluster.
+//
+// Bound by what arrives: about 1.5 cycles per value and CTA, and a microsecond per layer besides.
+// 153 layers of 1 200 states, forward: 341 -> 235 us with the layer before in L2 and a barrier of the
+// cluster per layer (its release alone was 700 cycles); 58 layers of 3 000: 220 -> 190.  Slower:
+// the values where they were made and read from there (281; the barrier again), a bulk copy per
+// CTA pair (300), two states per store (263), teams of four (269; 261 for the 3 000), four
+// records per lane (252).
 template <typename Val, bool kLog>
-__global__ void __launch_bounds__(512, 1)
+__global__ void __launch_bounds__(32 * kWideWarps, 1)
 LayerChainWide(k2b200_fsa_view v, const LayerArc *__restrict__ fwd_arcs,
                const LayerArc *__restrict__ bwd_arcs, Val *val_fwd, Val *val_bwd,
-               int32_t *__restrict__ entering, int32_t *__restrict__ scale, int32_t *hi_slots,
-               int32_t dir_base, int32_t fsa_base, ChainPlan p, int32_t *__restrict__ status) {
+               int32_t *__restrict__ entering, int32_t *__restrict__ scale, int32_t dir_base,
+               int32_t fsa_base, ChainPlan p, int32_t *__restrict__ status) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ __align__(8) uint64_t bars[2];
+  __shared__ int32_t words[2][kWideTeam * kWideWarps];
   constexpr unsigned kAll = 0xffffffffu;
   namespace cg = cooperative_groups;
-  const cg::cluster_group cluster = cg::this_cluster();
-  const int32_t rank = (int32_t)cluster.block_rank(), team = p.team;
+  const int32_t rank = (int32_t)cg::this_cluster().block_rank(), team = p.team;
   const int32_t i = fsa_base + blockIdx.y, dir = (int32_t)blockIdx.x / team + dir_base;
   const int32_t s_begin = v.row_splits1[i], s_end = v.row_splits1[i + 1];
   const int32_t lv0 = v.level_offsets[i], nl = v.level_offsets[i + 1] - lv0;
   if (s_end == s_begin) return;  // uniform over the cluster, as is the next return
   const int tid = threadIdx.x, lane = tid & 31;
   Val *out = dir == 0 ? val_fwd : val_bwd;
-  int32_t *lvl = reinterpret_cast<int32_t *>(smem_raw);
+  Val *vals = reinterpret_cast<Val *>(smem_raw);  // [2][p.cells]
+  constexpr int kRecs = kWideRecs, nc = 32 * kWideWarps;
+  LayerArc *recs = reinterpret_cast<LayerArc *>(smem_raw + 2 * sizeof(double) * (size_t)p.cells) +
+                   tid;  // [2][kRecs][threads]
+  int32_t *lvl = reinterpret_cast<int32_t *>(recs - tid + 2 * kRecs * nc);
   const int32_t *gsplits = dir == 0 ? v.in_splits : v.row_splits2;
   const LayerArc *garcs = dir == 0 ? fwd_arcs : bwd_arcs;
   if (nl > p.nl_cap) {
@@ -1096,30 +1154,28 @@ LayerChainWide(k2b200_fsa_view v, const LayerArc *__restrict__ fwd_arcs,
     return;
   }
   for (int32_t k = tid; k <= nl; k += blockDim.x) lvl[k] = v.level_splits[lv0 + k];
-  int32_t *my_hi = hi_slots + 2 * ((int64_t)dir * v.num_fsas + i);
+  if (tid == 0) {
+    MbarInit(&bars[0], 1);
+    MbarInit(&bars[1], 1);
+    MbarInitFence();
+  }
   __syncthreads();
+  ClusterSync();
   const int32_t root = dir == 0 ? s_begin : s_end - 1;
-  const int32_t nt = team * 512, at = rank * 512 + tid;
+  const int32_t nt = team * nc, at = rank * nc + tid;
   int32_t *my_scale = kLog ? scale + ((int64_t)dir * v.num_fsas + i) * p.nl_cap : nullptr;
   ChainScale<kLog> sc;
-  auto layer_sync = [&]() {
-    if (team == 1) __syncthreads(); else cluster.sync();
-  };
   auto layer_of = [&](int32_t step) { return dir == 0 ? step : nl - 1 - step; };
-  constexpr int kRecs = 4;
-  struct Ahead {
+  struct Splits {
     int32_t k0, k1, log_lanes;  // of the lane's state; log2 of the lanes of a state
-    LayerArc r[kRecs];
   };
   // lanes per state in a layer of `width` states
   auto log_lanes_of = [&](int32_t width) {
-    int32_t n = 0;
-    while (n < 3 && width << (n + 1) <= nt) ++n;
-    return n;
+    return (width << 1 <= nt) + (width << 2 <= nt) + (width << 3 <= nt);
   };
-  auto fetch_splits = [&](int32_t step, Ahead &f) {
-    f.k0 = f.k1 = f.log_lanes = 0;
-    if (step >= nl) return;
+  auto splits_of = [&](int32_t step) {
+    Splits f = {0, 0, 0};
+    if (step >= nl) return f;
     const int32_t l = layer_of(step), b = lvl[l], e = lvl[l + 1];
     f.log_lanes = log_lanes_of(e - b);
     const int32_t s = b + (at >> f.log_lanes);
@@ -1127,36 +1183,103 @@ LayerChainWide(k2b200_fsa_view v, const LayerArc *__restrict__ fwd_arcs,
       f.k0 = __ldg(gsplits + s);
       f.k1 = __ldg(gsplits + s + 1);
     }
+    return f;
   };
-  auto fetch_records = [&](Ahead &f) {
+  auto fetch_records = [&](int32_t step, const Splits &f) {
     const int32_t lanes = 1 << f.log_lanes, k = f.k0 + (lane & (lanes - 1));
+    LayerArc *to = recs + (step & 1) * (kRecs * nc);
 #pragma unroll
     for (int u = 0; u < kRecs; ++u)
-      if (k + u * lanes < f.k1) f.r[u] = garcs[k + u * lanes];
+      if (k + u * lanes < f.k1) CpAsync16(to + u * nc, garcs + k + u * lanes);
+    CpAsyncCommit();
+    if (k + kRecs * lanes < f.k1) {
+#pragma unroll 1
+      for (int32_t t = k + kRecs * lanes; t < min(f.k1, k + 2 * kRecs * lanes); t += lanes) {
+        int32_t unused;
+        asm volatile("ld.global.ca.s32 %0, [%1];" : "=r"(unused) : "l"(&garcs[t].arc));
+      }
+    }
   };
   auto rec = [&](int32_t k) { return garcs[k]; };
-  auto val = [&](const LayerArc &r) { return __ldcg(out + r.other); };
-  Ahead now, next, after;
-  fetch_splits(0, now);
-  fetch_records(now);
-  fetch_splits(1, next);
-  for (int32_t step = 0; step < nl; ++step) {
-    fetch_records(next);
-    fetch_splits(step + 2, after);
-    const int32_t l = layer_of(step), b = lvl[l], e = lvl[l + 1];
-    const int32_t lanes = 1 << now.log_lanes, g = lane & (lanes - 1);
-    sc.BeginLayer(step, my_hi, rank == 0 && tid == 0);
-    for (int32_t s0 = b; s0 < e; s0 += nt) {  // (more than once only with a lane per state)
-      const int32_t s = s0 + (at >> now.log_lanes);
+  // The layer before: its values in shared memory (or not), its first state, its last one's number.
+  const uint32_t vals0 = SmemAddr(vals), bars0 = SmemAddr(bars);
+  uint32_t was_vals = vals0;
+  int32_t was_b = 0, was_last = 0;
+  bool was_far = false;
+  auto find = [&](int32_t other) {  // where the value is: an address, or the state itself
+    return was_far ? other
+                   : (int32_t)(was_vals + min((uint32_t)(other - was_b), (uint32_t)was_last) *
+                                              (uint32_t)sizeof(Val));
+  };
+  auto found = [&](int32_t where) {
+    if (was_far) return __ldcg(out + where);
+    return *reinterpret_cast<const Val *>(__cvta_shared_to_generic((uint32_t)where));
+  };
+  auto val = [&](const LayerArc &r) { return found(find(r.other)); };
+  Splits now = splits_of(0), next = splits_of(1), after = splits_of(2);
+  LayerArc r[kRecs];
+  // the records of the lane's state, `other` replaced by where the value is
+  auto take_records = [&](int32_t step) {
+    const int32_t lanes = 1 << now.log_lanes, k = now.k0 + (lane & (lanes - 1));
+    const LayerArc *from = recs + (step & 1) * (kRecs * nc);
+    CpAsyncWait<0>();
+#pragma unroll
+    for (int u = 0; u < kRecs; ++u)
+      if (k + u * lanes < now.k1) {
+        r[u] = from[u * nc];
+        r[u].other = find(r[u].other);
+      }
+  };
+  fetch_records(0, now);
+  take_records(0);
+  fetch_records(1, next);
+  int32_t b, e;  // the layer's states
+  auto begin = [&](int32_t step) {
+    const int32_t l = layer_of(step);
+    b = lvl[l];
+    e = lvl[l + 1];
+    if (tid == 0)
+      MbarArriveExpectTx(&bars[step & 1],
+                         (unsigned)(team * kWideWarps * 4 +
+                                    (e - b > p.cells ? 0 : (e - b) * (int)sizeof(Val))));
+  };
+  begin(0);
+  bool ok = true;
+  for (int32_t step = 0; step < nl && ok; ++step) {
+    const int32_t log_lanes = now.log_lanes, lanes = 1 << log_lanes, g = lane & (lanes - 1);
+    const bool far = e - b > p.cells;
+    const uint32_t to = (uint32_t)((step & 1) * p.cells) * (uint32_t)sizeof(Val),
+                   to_bar = bars0 - vals0 + 8u * (step & 1);
+    sc.mul = 1.0;
+    if (kLog && step % kRescale == 0 && step > 0) {
+      int32_t hm = 0;
+      for (int32_t k = lane; k < team * kWideWarps; k += 32) hm = max(hm, words[(step - 1) & 1][k]);
+      sc.Rescale(__reduce_max_sync(kAll, hm));
+    }
+    StateSum<Val, kLog> q;
+    auto store = [&](int32_t s) {  // what global memory gets
+      if (!kLog && entering != nullptr && dir == 0) entering[s] = q.best;
+      __stcg(out + s, q.acc);
+    };
+    q.Clear();
+    const int32_t last = b + (max(e - b - 1, 0) & -nt);  // (nt: a power of two)
+    // warps beyond the layer's last state have nothing to add
+    const int32_t end = e - ((at & ~31) >> log_lanes);
+    for (int32_t s0 = b; s0 < end; s0 += nt) {  // (more than once only with a lane per state)
+      const int32_t s = s0 + (at >> log_lanes);
       if (s0 > b) {
         now.k0 = now.k1 = 0;
         if (s < e) {
           now.k0 = __ldg(gsplits + s);
           now.k1 = __ldg(gsplits + s + 1);
         }
-        fetch_records(now);
+#pragma unroll
+        for (int u = 0; u < kRecs; ++u)
+          if (now.k0 + u < now.k1) {
+            r[u] = garcs[now.k0 + u];
+            r[u].other = find(r[u].other);
+          }
       }
-      StateSum<Val, kLog> q;
       q.Clear();
       const int32_t k0 = now.k0, k1 = now.k1;
       // states of many arcs are left to the whole warp
@@ -1165,34 +1288,60 @@ LayerChainWide(k2b200_fsa_view v, const LayerArc *__restrict__ fwd_arcs,
         Val x[kRecs];
 #pragma unroll
         for (int u = 0; u < kRecs; ++u)
-          if (k0 + g + u * lanes < k1) x[u] = val(now.r[u]);
+          if (k0 + g + u * lanes < k1) x[u] = found(r[u].other);
 #pragma unroll
         for (int u = 0; u < kRecs; ++u)
-          if (k0 + g + u * lanes < k1) q.Add(now.r[u], x[u]);
+          if (k0 + g + u * lanes < k1) q.Add(r[u], x[u]);
         q.Walk(k0 + g + kRecs * lanes, k1, lanes, rec, val);
       }
       const unsigned heavy = __ballot_sync(kAll, many && g == 0);
       if (heavy) q.Heavy(heavy, lane, k0, k1, rec, val);
       q.Across(lanes);
-      if (s < e && g == 0) {
+      if (s < e) {
         if (kLog) {
           q.acc = q.acc * (Val)sc.mul;
           if (q.acc == (Val)0 && s == root) q.acc = (Val)1;
           sc.Note((double)q.acc);
-        } else {
-          if (q.acc == (Val)-INFINITY && s == root) q.acc = (Val)0;
-          if (entering != nullptr && dir == 0) entering[s] = q.best;
+        } else if (q.acc == (Val)-INFINITY && s == root) {
+          q.acc = (Val)0;
         }
-        __stcg(out + s, q.acc);
+        // the state's lanes share the CTAs out among them
+        if (!far) {
+          const uint32_t cell = to + (uint32_t)(s - b) * (uint32_t)sizeof(Val);
+          for (int32_t r = g; r < team; r += lanes) {
+            const uint32_t there = InRank(vals0, r);
+            StoreAsync(there + cell, q.acc, there + to_bar);
+          }
+        }
+        if (g == 0 && s0 < last) store(s);
       }
     }
-    sc.EndLayer(step, my_hi, lane, status);
-    if (kLog && rank == 0 && tid == 0) my_scale[l] = sc.K;
-    layer_sync();
+    const int32_t s = last + (at >> log_lanes);
+    if (far && s < e && g == 0) store(s);
+    const int32_t word = kLog && step % kRescale == kRescale - 1 ? sc.TakeMax(lane, status) : 0;
+    __syncwarp();
+    if (lane < team)
+      StoreAsync(InRank(SmemAddr(&words[step & 1][at >> 5]), lane), word,
+                 InRank(vals0, lane) + to_bar);
+    if (!far && s < e && g == 0) store(s);
+    if (kLog && rank == 0 && tid == 0) my_scale[layer_of(step)] = sc.K;
+    was_far = far;
+    was_vals = vals0 + to;
+    was_b = b;
+    was_last = max(e - b, 1) - 1;
     now = next;
     next = after;
+    take_records(step + 1);
+    fetch_records(step + 2, next);
+    after = splits_of(step + 3);
+    if (step + 1 < nl) begin(step + 1);
+    if (far) ClusterSync();
+    ok = __all_sync(kAll, MbarWaitBounded(&bars[step & 1], (unsigned)(step >> 1) & 1u));
   }
+  if (!ok && lane == 0) atomicOr(status, 2);
   sc.End(lane, status);
+  CpAsyncWait<0>();
+  ClusterSync();  // no CTA leaves while another may store into it
 }
 
 // out[s] = log(m[s]) + scale of its layer * ln 2.  grid = (layer tiles, fsas, parts of a
@@ -1216,8 +1365,8 @@ FinishLayerScores(k2b200_fsa_view v, const double *m, const int32_t *__restrict_
 
 namespace {
 struct ChainScratch {
-  // cleared together: status, the slice pool's counter, the words of ChainScale
-  int32_t *status, *hi_slots;
+  // cleared together: status, the slice pool's counter
+  int32_t *status;
   unsigned long long *pool_used;
   uint4 *pool;        // sliced layers
   SliceDesc *descs;   // [2][layers]
@@ -1240,10 +1389,9 @@ ChainScratch CarveScratch(const k2b200_fsa_view *v, const ChainPlan &p, int32_t 
   };
   const size_t na = (size_t)std::max(v->num_arcs, 1), ns = (size_t)std::max(v->num_states, 1);
   const size_t layers = (size_t)v->num_fsas * (size_t)std::max(v->max_layers, 1);
-  c.clear_bytes = sizeof(int32_t) * (4 + 4 * (size_t)v->num_fsas);
+  c.clear_bytes = sizeof(int32_t) * 4;
   c.status = reinterpret_cast<int32_t *>(take(c.clear_bytes));
   c.pool_used = reinterpret_cast<unsigned long long *>(c.status + 2);
-  c.hi_slots = c.status + 4;
   if (p.wide) {
     c.fwd_arcs = reinterpret_cast<LayerArc *>(take(sizeof(LayerArc) * na));
     c.bwd_arcs = reinterpret_cast<LayerArc *>(take(sizeof(LayerArc) * na));
@@ -1330,8 +1478,8 @@ static int32_t LaunchChain(const k2b200_fsa_view *v, const ChainScratch &c, cons
     cfg.numAttrs = 1;
     K2B_CUDA_OK(cudaLaunchKernelEx(&cfg, LayerChainWide<Val, kLog>, *v,
                                    (const LayerArc *)c.fwd_arcs, (const LayerArc *)c.bwd_arcs,
-                                   val_fwd, val_bwd, entering, c.scale, c.hi_slots, dir_base,
-                                   first, p, c.status));
+                                   val_fwd, val_bwd, entering, c.scale, dir_base, first, p,
+                                   c.status));
     NoteLaunch();
   }
   K2B_CUDA_OK(cudaGetLastError());

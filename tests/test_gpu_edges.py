@@ -57,6 +57,8 @@ def layered_lattice(rng, widths, degree, scale, hub=None):
     ([1, 1025, 1000, 1026, 1], 2.0, 1.0, 700),       # by four warps
     ([1, 500, 20000, 4097, 8, 1], 2.0, 1.0, None),   # wide: one to eight lanes per state
     ([1, 18000, 3, 18000, 1], 2.0, 1.0, 700),        # wide, with a state for the whole warp
+    ([1, 4095, 4097, 8193, 513, 1024, 2, 1], 2.0, 1.0, 90),  # turns of 4096 and their edges
+    ([1] + [5000, 12001, 10999, 11002] * 5 + [1], 1.5, 1.0, None),  # through L2 and not, in turn
 ])
 def test_lattice_scores_and_best_path(k2, widths, degree, scale, hub):
     from gpu_util import host_to_fsa
