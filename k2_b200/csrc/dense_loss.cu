@@ -595,14 +595,16 @@ GridChainMasked(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_leve
                 const float *__restrict__ vbwd, const float *__restrict__ cutoffs,
                 ProbState *__restrict__ alpha, ProbState *__restrict__ beta,
                 double *__restrict__ tot, const int32_t *__restrict__ plan,
-                int32_t *__restrict__ unfit, int32_t mask_pitch, int32_t wait_limit) {
+                int32_t *__restrict__ unfit, int32_t mask_pitch, int32_t wait_limit,
+                ChainShare share) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full[kMaskedBatches];
   __shared__ int32_t emax;
   __shared__ int32_t t_fail_sm;  // batch whose wait gave up
   constexpr int32_t kNone = INT32_MIN;
-  const int32_t i = blockIdx.y;
-  const int dir = blockIdx.x;
+  int32_t after;  // the step before the first one
+  const int32_t chain = ChainOf(share, blockIdx.x, 2 * n, &after), i = chain >> 1;
+  const int dir = chain & 1;
   // no plan, or outside the limits: the fallback kernel takes it; or of the other CTA size
   if (unfit[i] || unfit[n + i] != LaneClass(kThreads)) return;
   const FsaInfo f = infos[i];
@@ -612,6 +614,8 @@ GridChainMasked(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_leve
     if (dir == 0 && tid == 0) tot[i] = -INFINITY;
     return;
   }
+  const int32_t end = share.part == 1 ? min(share.cut, Tk) : Tk;  // the last step
+  if (after > 0 && after >= end) return;
   constexpr int kSPad = kThreads;  // a planned graph has at most that many states
   // a batch: kU packed dense rows, then kU rows of mask bytes
   const uint32_t batch_bytes = (uint32_t)kU * ((uint32_t)dp.pitch + (uint32_t)kThreads);
@@ -670,7 +674,16 @@ GridChainMasked(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_leve
     return;
   }
   ProbState *out = (dir == 0 ? alpha : beta) + f.grid_off;
-  {  // first level: 1 for the start (final) state if it survives, 0 elsewhere
+  int32_t K = 0;
+  if (after > 0) {  // the values, their exponent and the largest of them, as the chain left them
+    const ProbState *row = out + (int64_t)(dir == 0 ? after : Tk - after) * S;
+    K = row[0].e;
+    for (int32_t q = tid; q < S; q += nt) {
+      const double v = row[q].m;
+      pv[q] = v;
+      if (v != 0.0) atomicMax(&emax, (__double2hiint(v) >> 20) - 1023);
+    }
+  } else {  // first level: 1 for the start (final) state if it survives, 0 elsewhere
     const int64_t lv = dir == 0 ? 0 : Tk;
     const int32_t q1 = dir == 0 ? 0 : S - 1;
     const bool one_ok = __fadd_rn(vfwd[f.grid_off + lv * S + q1], vbwd[f.grid_off + lv * S + q1]) >
@@ -690,14 +703,14 @@ GridChainMasked(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_leve
   const unsigned char *dense_rows = dense + (int64_t)f.row0 * dp.pitch;
   const uint32_t row_bytes = (uint32_t)dp.pitch, lp_bytes = 4u * (uint32_t)dp.cols4;
   const unsigned char *mask0 = masks + ((int64_t)dir * total_levels + f.level_off) * mask_pitch;
-  const int32_t num_batches = (Tk + kU - 1) / kU;
-  // thread 0: the rows of steps b * kU + 1 .. of batch b, as two copies.  Walking forward the
+  const int32_t num_batches = (end - after + kU - 1) / kU;
+  // one thread: the rows of steps after + b * kU + 1 .. of batch b, as two copies.  Walking forward the
   // dense rows and the mask rows of consecutive steps ascend, walking backward they descend:
   // either way they are one block of memory; frame u of the batch is row u of the block
   // (forward) or row nf - 1 - u (backward).
   auto issue_batch = [&](int32_t b) {
     if (b >= num_batches) return;
-    const int32_t t_first = b * kU + 1, nf = min(kU, Tk - b * kU);
+    const int32_t t_first = after + b * kU + 1, nf = min(kU, end - t_first + 1);
     const int64_t row_lo = dir == 0 ? t_first - 1 : Tk - t_first - nf + 1;  // dense rows
     const int64_t r_lo = dir == 0 ? t_first : Tk - t_first - nf + 1;        // mask rows
     const int32_t slot = b % kMaskedBatches;
@@ -714,9 +727,8 @@ GridChainMasked(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_leve
     for (int32_t b = 0; b < kMaskedBatches - 1; ++b) issue_batch(b);
   const int32_t g_max = __reduce_max_sync(0xffffffffu, G);  // widest lane group of this warp
   const int32_t s_ld = s >= 0 ? s : 0;
-  int64_t pos = (dir == 0 ? 1 : Tk - 1) * (int64_t)S + s_ld;
+  int64_t pos = (dir == 0 ? after + 1 : Tk - 1 - after) * (int64_t)S + s_ld;
   double last = 0.0;
-  int32_t K = 0;
   bool gave_up = false;
   // the frame loop once per kind of CTA, so that the unrolled code of only one is fetched
   auto frames = [&](auto hoist_tag) {
@@ -736,7 +748,7 @@ GridChainMasked(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_leve
       }
       if (issues) issue_batch(b + kMaskedBatches - 1);
       const unsigned char *base = ring + (size_t)slot * batch_bytes;
-      const int32_t nf = min(kU, Tk - b * kU);
+      const int32_t nf = min(kU, end - after - b * kU);
       const int pb = (kU % 2 == 0) ? 0 : (b & 1);  // parity of the state buffers at the batch's start
 #pragma unroll
       for (int u = 0; u < kU; ++u) {
@@ -831,7 +843,7 @@ GridChainMasked(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_leve
     if (tid == 0) atomicOr(&unfit[i], 2);
     return;
   }
-  if (dir == 0 && s == S - 1 && g == 0)
+  if (dir == 0 && end == Tk && s == S - 1 && g == 0)
     tot[i] = last == 0.0 ? -INFINITY : log(last) + (double)K * 0.69314718055994530942;
 }
 
@@ -1784,8 +1796,9 @@ static int32_t LaunchChainMasked(const LossLayout &LL, const k2b200_intersect_ar
     else K2B_ARC_MASKS(1024)
 #undef K2B_ARC_MASKS
   }
-  {
-    dim3 grid(2, args->num_fsas);
+  ChainShare share = ShareChains(L);
+  for (share.part = share.early > 0 ? 1 : 0; share.part <= (share.early > 0 ? 2 : 0); ++share.part) {
+    const int32_t grid = share.part == 1 ? share.early : 2 * args->num_fsas;
 #define K2B_CHAIN_MASKED(KU)                                                                  \
     {                                                                                         \
       const size_t smem = MaskedSmem(LL.pack, kThreads, KU);                                  \
@@ -1797,7 +1810,7 @@ static int32_t LaunchChainMasked(const LossLayout &LL, const k2b200_intersect_ar
           args->a_in_splits, args->a_in_arcs, dense, LL.pack, masks, fwd, bwd, cutoffs,       \
           reinterpret_cast<ProbState *>(ws + LL.off_alpha),                                   \
           reinterpret_cast<ProbState *>(ws + LL.off_beta), tot, plan, unfit, LL.threads,      \
-          CopyWaitLimit());                                                                   \
+          CopyWaitLimit(), share);                                                            \
         NoteLaunch(); }                                                                       \
     }
     // frames per batch (one bulk copy of dense rows and one of mask rows each): as many as

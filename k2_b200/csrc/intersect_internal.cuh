@@ -77,6 +77,25 @@ constexpr int kLaneDeg = 8;
 // them into warps leaves unused.  (Without it a denominator graph over 80 to 100 phones
 // fell back to the kernels without plans, at three to four times the time.)
 int32_t LaneThreads(const Layout &L);
+
+// The chains (two per graph: 2 * graph + direction) of a recursion with one CTA per SM, in one
+// launch or in two.  With more chains than SMs, but not twice as many, a launch has a second
+// round that leaves SMs idle: 256 chains on 148.  Two launches then: the first `early` chains walk
+// their steps 1 .. cut, and after them the rest of those (several to an SM) runs beside the
+// others, a step's values being in global memory anyway.
+struct ChainShare {
+  int32_t cut, early;  // 0: one launch
+  int32_t part;        // of the launch: 0 all, 1 the first steps of the first chains, 2 what is left
+};
+ChainShare ShareChains(const Layout &L);
+// What CTA b of a launch does, of `chains`: which chain, and after which step it starts.
+__device__ __forceinline__ int32_t ChainOf(const ChainShare &c, int32_t b, int32_t chains,
+                                           int32_t *after) {
+  const int32_t whole = chains - c.early;  // they come first: they take longest
+  const bool rest = c.part == 2 && b >= whole;
+  *after = rest ? c.cut : 0;
+  return c.part != 2 ? b : rest ? b - whole : b + c.early;
+}
 __device__ __forceinline__ int32_t LaneClass(int32_t threads) { return threads > 768 ? 1 : 0; }
 #define K2B_LANE_THREADS(THREADS, CALL) \
   do {                                  \

@@ -435,14 +435,17 @@ LanesViterbi(const FsaInfo *__restrict__ infos, int32_t n, const Arc *__restrict
              const int32_t *__restrict__ a_row_splits2, const int32_t *__restrict__ in_splits,
              const int32_t *__restrict__ in_arcs, const float *__restrict__ scores,
              int32_t cols, int32_t cols_pad, float *__restrict__ fwd, float *__restrict__ bwd,
-             const int32_t *__restrict__ plan, const int32_t *__restrict__ unfit) {
+             const int32_t *__restrict__ plan, const int32_t *__restrict__ unfit,
+             ChainShare share) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ float buf[2][kThreads];
-  const int32_t i = blockIdx.y;
+  int32_t after;  // the step before the first one
+  const int32_t chain = ChainOf(share, blockIdx.x, 2 * n, &after), i = chain >> 1;
   if ((unfit[i] & 1) || unfit[n + i] != LaneClass(kThreads)) return;
-  const int dir = blockIdx.x;
+  const int dir = chain & 1;
   const int32_t S = infos[i].num_states, Tk = infos[i].tk;
-  if (S == 0) return;
+  const int32_t end = share.part == 1 ? min(share.cut, Tk) : Tk;  // the last step
+  if (S == 0 || (after > 0 && after >= end)) return;
   const int tid = threadIdx.x, nt = blockDim.x;
   const int32_t pitch = kPitch ? kPitch : cols_pad;
   float *ring = reinterpret_cast<float *>(smem_raw);  // [kVitRing][pitch]
@@ -491,7 +494,7 @@ LanesViterbi(const FsaInfo *__restrict__ infos, int32_t n, const Arc *__restrict
   // step t (1..Tk) consumes dense row t-1 (forward) or Tk-t (backward).  The warps that hold
   // a column copy it; the others neither copy nor wait.
   const bool copies = (tid & ~31) < cols;
-  const float *src = scores + ((int64_t)infos[i].row0 + (dir == 0 ? 0 : Tk - 1)) * cols;
+  const float *src = scores + ((int64_t)infos[i].row0 + (dir == 0 ? after : Tk - 1 - after)) * cols;
   const int64_t src_step = dir == 0 ? cols : -(int64_t)cols;
   auto issue_row = [&](bool there, int32_t slot) {
     if (there)
@@ -500,30 +503,33 @@ LanesViterbi(const FsaInfo *__restrict__ infos, int32_t n, const Arc *__restrict
     src += src_step;
   };
   if (copies)
-    for (int32_t step = 1; step <= kVitAhead; ++step) issue_row(step <= Tk, (step - 1) % kVitRing);
+    for (int32_t step = 1; step <= kVitAhead; ++step)
+      issue_row(after + step <= end, (step - 1) % kVitRing);
   const int64_t stride = dir == 0 ? (int64_t)S : -(int64_t)S;
   const bool store = s >= 0 && g == 0;
   float *gout;
   {
     float *grid = (dir == 0 ? fwd : bwd) + infos[i].grid_off;
+    float *first = grid + (int64_t)(dir == 0 ? after : Tk - after) * S;
     for (int32_t q = tid; q < S; q += nt) {
-      const float v0 = (dir == 0 ? (q == 0) : (q == S - 1)) ? 0.0f : -INFINITY;
+      float v0 = (dir == 0 ? (q == 0) : (q == S - 1)) ? 0.0f : -INFINITY;
+      if (after > 0) v0 = first[q];
+      else first[q] = v0;
       buf[0][q] = v0;
-      grid[(int64_t)(dir == 0 ? 0 : Tk) * S + q] = v0;
     }
-    gout = grid + (dir == 0 ? 1 : Tk - 1) * (int64_t)S + max(s, 0);
+    gout = first + stride + max(s, 0);
   }
   // the frame loop once per kind of CTA, so that the unrolled code of only one is fetched
   auto frames = [&](auto hoist_tag) {
     constexpr bool kHoist = decltype(hoist_tag)::value;
-    for (int32_t t0 = 1; t0 <= Tk; t0 += kVitRing) {
+    for (int32_t t0 = after + 1; t0 <= end; t0 += kVitRing) {
 #pragma unroll
       for (int u = 0; u < kVitRing; ++u) {
         const int32_t t = t0 + u;
-        if (t > Tk) break;
+        if (t > end) break;
         if (copies) CpAsyncWait<kVitAhead - 1>();  // this thread's part of row t has landed
         __syncthreads();  // ... everyone's has; the scores of step t - 1 are complete
-        if (copies) issue_row(t + kVitAhead <= Tk, (u + kVitAhead) % kVitRing);
+        if (copies) issue_row(t + kVitAhead <= end, (u + kVitAhead) % kVitRing);
         // t0 is odd: (t - 1) & 1 == u & 1
         const char *cur = reinterpret_cast<const char *>(buf[u & 1]);
         const char *row = reinterpret_cast<const char *>(ring + u * pitch);
@@ -565,17 +571,20 @@ int32_t LaunchLanesViterbi(const Layout &L, const k2b200_intersect_args *a,
                            const FsaInfo *d_infos, float *fwd, float *bwd, const int32_t *plan,
                            const int32_t *unfit, cudaStream_t stream) {
   static_assert(kLaneDeg % 2 == 0, "arcs are taken in pairs");
-  dim3 grid(2, a->num_fsas);
+  ChainShare share = ShareChains(L);
   const int32_t cols_pad = (a->cols + 3) & ~3;
   auto launch = [&](auto kernel, int32_t threads, int32_t pitch) -> int32_t {
     const size_t smem = sizeof(float) * kVitRing * (size_t)pitch;
     K2B_REQUIRE(smem <= kVitRingBytes, "too many columns for the lane Viterbi kernel");
     K2B_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem));
-    kernel<<<grid, threads, smem, stream>>>(
-        d_infos, a->num_fsas, reinterpret_cast<const Arc *>(a->a_arcs), a->a_row_splits2,
-        a->a_in_splits, a->a_in_arcs, a->scores, a->cols, cols_pad, fwd, bwd, plan, unfit);
-    NoteLaunch();
+    for (share.part = share.early > 0 ? 1 : 0; share.part <= (share.early > 0 ? 2 : 0);
+         ++share.part) {
+      kernel<<<share.part == 1 ? share.early : 2 * a->num_fsas, threads, smem, stream>>>(
+          d_infos, a->num_fsas, reinterpret_cast<const Arc *>(a->a_arcs), a->a_row_splits2,
+          a->a_in_splits, a->a_in_arcs, a->scores, a->cols, cols_pad, fwd, bwd, plan, unfit, share);
+      NoteLaunch();
+    }
     return kOk;
   };
   // graphs over phones have rows of up to 128 columns

@@ -137,6 +137,42 @@ def test_denominator_batch_of_128_against_oracle():
     assert np.abs(lp2.grad.cpu().numpy() - want_lp).max() <= 1e-4
 
 
+@pytest.mark.parametrize("utterances,longest,shortest", [
+    (75, 64, 64),     # two chains more than a B200 has SMs, lengths of whole batches of four
+    (100, 101, 70),   # some end before the cut
+    (110, 127, 1),
+    (128, 400, 400),  # four rests to an SM
+])
+def test_chains_in_two_launches_are_the_chains(utterances, longest, shortest):
+    # the batch at once (chains are cut) and in parts of at most 60 utterances (they are not): the
+    # same lattices, totals and, but for the order of additions to the graph, gradients
+    import dataclasses
+    import k2_b200 as k2
+    from k2_b200 import synthetic as syn
+    w = syn.lfmmi_den(utterances=utterances)
+    seg = w.supervision_segments.clone()
+    seg[:, 2] = torch.linspace(longest, shortest, utterances).int()
+    got = []
+    for size in (utterances, 60):
+        tots, grads, arcs = [], [], []
+        for first in range(0, utterances, size):
+            part = dataclasses.replace(w, supervision_segments=seg[first:first + size])
+            graphs = syn.build_graphs(part, DEV)
+            lp = w.log_probs.to(DEV).requires_grad_(True)
+            tot = k2.intersect_dense_tot_scores(
+                graphs, k2.DenseFsaVec(lp, part.supervision_segments), w.output_beam)
+            tot.sum().backward()
+            tots.append(tot.detach())
+            grads.append(lp.grad)
+            lat = k2.intersect_dense(graphs, k2.DenseFsaVec(lp.detach(), part.supervision_segments),
+                                     4.0)
+            arcs.append(lat.arcs.values().clone())
+        got.append((torch.cat(tots), sum(grads), torch.cat(arcs)))
+    assert torch.equal(got[0][0], got[1][0])
+    assert torch.equal(got[0][1], got[1][1])
+    assert torch.equal(got[0][2], got[1][2])
+
+
 def test_decoding_configuration_matches_the_reference_lattice_checksums():
     # hlg_decode at full size through intersect_dense_pruned; the reference's lattice
     # (tests/golden/make_pruned_full_size_golden.py) is kept as sizes and sha256 digests
