@@ -672,8 +672,9 @@ struct __align__(16) SliceEntry {  // of a layer in a slot
   int32_t blocks, tall, first_state;
 };
 
-template <typename Val, bool kLog, int K>
-__global__ void __launch_bounds__(544, 1)
+// kOne: one such warp, which has the short walk below (in the loop of several it cost 7 %).
+template <typename Val, bool kLog, int K, bool kOne>
+__global__ void __launch_bounds__(kOne ? 64 : 544, 1)
 SliceChain(k2b200_fsa_view v, const uint4 *__restrict__ pool, const SliceDesc *__restrict__ descs,
            Val *__restrict__ val_fwd, Val *__restrict__ val_bwd, int32_t *__restrict__ entering,
            int32_t *__restrict__ scale, int32_t dir_base, int32_t fsa_base, int32_t nl_total,
@@ -688,7 +689,7 @@ SliceChain(k2b200_fsa_view v, const uint4 *__restrict__ pool, const SliceDesc *_
   if (s_end == s_begin) return;
   const int32_t lv0 = v.level_offsets[i], nl = v.level_offsets[i + 1] - lv0;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nw = p.warps;
+  const int nw = kOne ? 1 : p.warps;
   Val *out = dir == 0 ? val_fwd : val_bwd;
   const uint32_t *shared_words = reinterpret_cast<const uint32_t *>(smem_raw);
   const LayerArc *shared_recs = reinterpret_cast<const LayerArc *>(smem_raw);
@@ -830,7 +831,7 @@ SliceChain(k2b200_fsa_view v, const uint4 *__restrict__ pool, const SliceDesc *_
     SliceEntry e = entries[slot][k++];
     if (e.tall == kSingle) {
       e.tall = 0;
-      if (!kLog && nw == 1 && e.at >= 0) {
+      if (kOne && !kLog && e.at >= 0) {
         Single a, b;
         int32_t at = e.at;
         read_single(at, a);
@@ -1441,10 +1442,16 @@ static int32_t LaunchChain(const k2b200_fsa_view *v, const ChainScratch &c, cons
     { slice<<<dim3(one ? CeilDiv(layers, 4) : layers, ndir), one ? 128 : 32 * warps, smem, stream>>>(
         *v, dir_base, p.rows, p.maxw, v->max_layer_arcs, buf, layers, c.pool_units, c.pool_used,
         c.pool, c.descs, c.status); NoteLaunch(); }
-    auto chain = p.rows == 2   ? SliceChain<Val, kLog, 2>
-                 : p.rows == 3 ? SliceChain<Val, kLog, 3>
-                 : p.rows == 4 ? SliceChain<Val, kLog, 4>
-                               : SliceChain<Val, kLog, 8>;
+    constexpr bool kOne = !kLog;
+    auto chain = p.rows == 2   ? SliceChain<Val, kLog, 2, false>
+                 : p.rows == 3 ? SliceChain<Val, kLog, 3, false>
+                 : p.rows == 4 ? SliceChain<Val, kLog, 4, false>
+                               : SliceChain<Val, kLog, 8, false>;
+    if (kOne && p.warps == 1)
+      chain = p.rows == 2   ? SliceChain<Val, kLog, 2, kOne>
+              : p.rows == 3 ? SliceChain<Val, kLog, 3, kOne>
+              : p.rows == 4 ? SliceChain<Val, kLog, 4, kOne>
+                            : SliceChain<Val, kLog, 8, kOne>;
     K2B_CUDA_OK(cudaFuncSetAttribute(chain, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)kLayerSmemBudget));
     for (int32_t first = 0; first < v->num_fsas; first += 65535) {
