@@ -344,7 +344,8 @@ def implementation_bytes(phase, kernel, frames, N, T, C, A, A_out, S_out, grid_s
     against, not a roofline denominator."""
     R = frames
     table = {
-        # every row by both directions, both grids written
+        # every row by both directions, both grids written (here and in BandPrep an upper bound: the
+        # cells that no path can pass are left out)
         "BandViterbi": 2 * 4 * R * C + 8 * grid_states,
         # BandPrep reads both grids (the level on either side of a chunk of 16 twice), per
         # surviving state two table entries and five grid values, and writes a list entry
@@ -711,8 +712,8 @@ def run_ours(args):
 
 
 # ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch on ctc_large (profiles/)
-NCU_TRAFFIC = {"BandViterbi": 288.2e6, "BandPrep": 267.7e6, "BandChainLists": 98.9e6,
-               "BandGradRows": 109.0e6}
+NCU_TRAFFIC = {"BandViterbi": 260.2e6, "BandPrep": 227.2e6, "BandChainLists": 96.4e6,
+               "BandGradRows": 104.7e6}
 
 
 # --------------------------------------------------------------------------- decoding
