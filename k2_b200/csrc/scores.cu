@@ -157,25 +157,46 @@ __global__ void PathFill(const int32_t *__restrict__ row_splits1, const Arc *__r
 // Best paths of a layered FsaVec (arcs go from one layer to a later one, as in lattices).  The
 // trace back is a chain of dependent loads; read from global memory a step costs two of them,
 // about half a microsecond (800 frames: 430 us, and as much again to fill the paths in once
-// their lengths are known).  Here a CTA per FSA brings the predecessors of a run of layers
-// into shared memory with all its threads, one thread follows the path through them, and
-// all of them write the arcs that it took: best[i * max_layers + k] is the k-th last arc.
+// their lengths are known).  Here Predecessors looks up where the best arc of every state comes
+// from, on all SMs; a CTA per FSA brings those of a run of layers into shared memory with all its
+// threads, one thread follows the path through them, and all of them write the arcs that it
+// took: best[i * max_layers + k] is the k-th last arc.  A step is a load and a
+// store: 22 ns.  (The look-up within the one CTA, runs of 8192 states and tests at every step: 800
+// layers of 13 states 42 us, now 18 + 2; 150 of 1 200: 87 -> 28 + 2; 32 FSAs of 100 000 states: 271 ->
+// 28 + 18.)
 // ---------------------------------------------------------------------------
-constexpr int kTraceStates = 8192;  // predecessors in shared memory
-constexpr int kTraceLayers = 512;   // layers of a run at most, one per thread and trip
-constexpr int kTraceFew = 24;       // runs of fewer layers are followed in global memory: to
-                                    // fetch 8192 predecessors takes as long as 20 steps there
+constexpr int kTraceStates = 48 * 1024;  // predecessors in shared memory
+constexpr int kTraceLayers = 512;        // layers of a run at most, one per thread and trip
+constexpr int kTraceFew = 8;             // runs of fewer layers are followed in global memory: to
+                                         // fetch a run takes as long as some seven steps there
+
+constexpr int kTraceSteps = 8;           // between looks at whether the run is left
+
+// pred[s]: the state (of its FSA) that the best arc into s comes from, -1: none enters.
+__global__ void __launch_bounds__(256)
+Predecessors(const Arc *__restrict__ arcs, const int32_t *__restrict__ entering,
+             int32_t num_states, int32_t *__restrict__ pred) {
+  const int32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= num_states) return;
+  const int32_t a = entering[s];
+  pred[s] = a >= 0 ? arcs[a].src : -1;
+}
 
 __global__ void __launch_bounds__(512)
-TraceLayers(k2b200_fsa_view v, const int32_t *__restrict__ entering, int32_t *__restrict__ best,
+TraceLayers(k2b200_fsa_view v, const int32_t *__restrict__ entering,
+            const int32_t *__restrict__ all_pred, int32_t *__restrict__ best,
             int32_t *__restrict__ lengths) {
-  __shared__ int32_t pred[kTraceStates], path[kTraceLayers];
-  __shared__ int32_t cur_sh, steps_sh;
+  // A run's predecessors, from a multiple of four states on, as offsets in this array; one outside
+  // the run, or none, is kOut, where kOut itself stands: a step then needs no test.
+  extern __shared__ int4 pred4[];
+  __shared__ int32_t path[kTraceLayers + kTraceSteps], cur_sh, steps_sh;
+  constexpr int32_t kOut = 4 * kTraceStates;
+  const char *pred = reinterpret_cast<const char *>(pred4);
   const int32_t i = blockIdx.x;
   const int tid = threadIdx.x;
   const int32_t s_begin = v.row_splits1[i], s_end = v.row_splits1[i + 1];
-  const Arc *arcs = reinterpret_cast<const Arc *>(v.arcs);
   int32_t *out = best + (int64_t)i * v.max_layers;
+  if (tid == 0) pred4[kTraceStates / 4] = make_int4(kOut, kOut, kOut, kOut);
   int32_t len = 0, cur = s_end - 1, hi = v.level_offsets[i + 1];
   const int32_t lv0 = v.level_offsets[i];
   bool alive = s_end > s_begin;
@@ -183,37 +204,64 @@ TraceLayers(k2b200_fsa_view v, const int32_t *__restrict__ entering, int32_t *__
     // as many layers below `hi` as fit
     const int32_t top = v.level_splits[hi];
     const int32_t l = hi - 1 - tid;
-    const int32_t n = __syncthreads_count(l >= lv0 && top - v.level_splits[l] <= kTraceStates);
-    const int32_t lo = hi - max(n, 1), base = v.level_splits[lo];
+    const int32_t n =
+        __syncthreads_count(l >= lv0 && top - (v.level_splits[l] & ~3) <= kTraceStates);
+    const int32_t lo = hi - max(n, 1), base = v.level_splits[lo], base4 = base & ~3;
     const bool staged = n >= min(kTraceFew, hi - lv0);
-    if (staged)
-      for (int32_t s = base + tid; s < top; s += blockDim.x) {
-        const int32_t a = entering[s];
-        pred[s - base] = a >= 0 ? s_begin + arcs[a].src : -1;
+    if (staged) {  // (what is read beyond `top` is within the array's last four)
+      const int4 *from = reinterpret_cast<const int4 *>(all_pred + base4);
+      const int32_t lowest = base - base4, to_here = s_begin - base4;
+      auto offset = [&](int32_t p) {
+        const int32_t j = p + to_here;
+        return p >= 0 && (uint32_t)(j - lowest) < (uint32_t)(top - base) ? 4 * j : kOut;
+      };
+#pragma unroll 4
+      for (int32_t k = tid; k < (top - base4 + 3) >> 2; k += 512) {
+        const int4 p = from[k];
+        pred4[k] = make_int4(offset(p.x), offset(p.y), offset(p.z), offset(p.w));
       }
+    }
     __syncthreads();
     if (tid == 0) {
+      const int32_t limit = min(kTraceLayers, v.max_layers - len);
       int32_t k = 0;
-      while (cur >= base && cur < top && k < kTraceLayers && len + k < v.max_layers) {
-        int32_t from;
-        if (staged) {
-          from = pred[cur - base];
-        } else {
-          const int32_t a = entering[cur];
-          from = a >= 0 ? s_begin + arcs[a].src : -1;
+      if (staged && cur >= base && cur < top) {
+        int32_t c = 4 * (cur - base4);
+        while (c != kOut && k < limit) {
+#pragma unroll
+          for (int u = 0; u < kTraceSteps; ++u) {
+            path[k + u] = c;
+            c = *reinterpret_cast<const int32_t *>(pred + c);
+          }
+          k += kTraceSteps;
         }
-        if (from < 0) {
-          cur = -1 - cur;  // the path begins at this state
-          break;
+        if (c == kOut) {  // to the last state of the run, and on from it
+          while (path[k - 1] == kOut) --k;
+          const int32_t last = base4 + (path[k - 1] >> 2), from = all_pred[last];
+          if (from < 0) --k;  // the path begins at this state
+          cur = from < 0 ? -1 - last : s_begin + from;
         }
-        path[k++] = cur;
-        cur = from;
+        if (k > limit || c != kOut) {
+          cur = k > limit ? base4 + (path[limit] >> 2) : base4 + (c >> 2);
+          k = limit;
+        }
+      } else if (!staged) {
+        while (cur >= base && cur < top && k < limit) {
+          const int32_t from = all_pred[cur];
+          if (from < 0) {
+            cur = -1 - cur;
+            break;
+          }
+          path[k++] = 4 * (cur - base4);
+          cur = s_begin + from;
+        }
       }
       cur_sh = cur;
       steps_sh = k;
     }
     __syncthreads();
-    for (int32_t k = tid; k < steps_sh; k += blockDim.x) out[len + k] = entering[path[k]];
+    for (int32_t k = tid; k < steps_sh; k += blockDim.x)
+      out[len + k] = entering[base4 + (path[k] >> 2)];
     cur = cur_sh;
     len += steps_sh;
     alive = cur >= 0;
@@ -612,7 +660,8 @@ int32_t k2b200_shortest_path(const int32_t *row_splits1, const void *arcs,
 size_t k2b200_best_paths_tmp_bytes(const k2b200_fsa_view *v) {
   if (v == nullptr) return 0;
   return AlignUp(sizeof(int32_t) * ((size_t)v->num_fsas + 1)) +
-         AlignUp(sizeof(int32_t) * (size_t)v->num_fsas * (size_t)v->max_layers);
+         AlignUp(sizeof(int32_t) * (size_t)v->num_fsas * (size_t)v->max_layers) +
+         AlignUp(sizeof(int32_t) * (size_t)std::max(v->num_states, 0) + 16);
 }
 
 int32_t k2b200_best_paths(const k2b200_fsa_view *v, const int32_t *entering_arcs,
@@ -627,7 +676,18 @@ int32_t k2b200_best_paths(const k2b200_fsa_view *v, const int32_t *entering_arcs
   int32_t *lengths = reinterpret_cast<int32_t *>(tmp);
   int32_t *traced = reinterpret_cast<int32_t *>(
       reinterpret_cast<char *>(tmp) + AlignUp(sizeof(int32_t) * ((size_t)v->num_fsas + 1)));
-  { TraceLayers<<<v->num_fsas, 512, 0, STREAM(stream)>>>(*v, entering_arcs, traced, lengths);
+  // (read 16 bytes at a time, whatever the alignment of `tmp`)
+  int32_t *pred = reinterpret_cast<int32_t *>(
+      (reinterpret_cast<uintptr_t>(traced) +
+       AlignUp(sizeof(int32_t) * (size_t)v->num_fsas * (size_t)v->max_layers) + 15) &
+      ~(uintptr_t)15);
+  if (v->num_states > 0)
+    { Predecessors<<<CeilDiv(v->num_states, 256), 256, 0, STREAM(stream)>>>(
+        reinterpret_cast<const Arc *>(v->arcs), entering_arcs, v->num_states, pred); NoteLaunch(); }
+  constexpr int smem = (int)sizeof(int32_t) * (kTraceStates + 4);
+  K2B_CUDA_OK(cudaFuncSetAttribute(TraceLayers, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  { TraceLayers<<<v->num_fsas, 512, smem, STREAM(stream)>>>(*v, entering_arcs, pred, traced,
+                                                            lengths);
     NoteLaunch(); }
   { WritePaths<<<v->num_fsas, 128, 0, STREAM(stream)>>>(
       reinterpret_cast<const Arc *>(v->arcs), traced, lengths, v->num_fsas, v->max_layers,

@@ -59,6 +59,9 @@ def layered_lattice(rng, widths, degree, scale, hub=None):
     ([1, 18000, 3, 18000, 1], 2.0, 1.0, 700),        # wide, with a state for the whole warp
     ([1, 4095, 4097, 8193, 513, 1024, 2, 1], 2.0, 1.0, 90),  # turns of 4096 and their edges
     ([1] + [5000, 12001, 10999, 11002] * 5 + [1], 1.5, 1.0, None),  # through L2 and not, in turn
+    ([1] + [3] * 1100 + [1], 1.2, 1.0, None),        # paths traced in runs of 512 layers
+    ([1] + [901] * 120 + [1], 1.1, 1.0, None),       # ... of 48 K states
+    ([1] + [7001] * 9 + [1], 1.1, 1.0, None),        # ... too short to be staged
 ])
 def test_lattice_scores_and_best_path(k2, widths, degree, scale, hub):
     from gpu_util import host_to_fsa
