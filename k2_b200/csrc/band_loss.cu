@@ -140,9 +140,9 @@ __device__ __forceinline__ bool WaitSlot(uint64_t *bar, unsigned parity, int32_t
 
 // Dense score of a state with `label` on dense row `row` of a sequence of T frames whose
 // frame 0 is at lp0 (the row T is the implied final row).
-__device__ __forceinline__ float BandDense(const float *__restrict__ lp0, int32_t C, int32_t T,
-                                           int32_t row, int32_t label) {
-  if (row < T) return (label >= 0 && label < C) ? __ldg(lp0 + (int64_t)row * C + label) : -INFINITY;
+__device__ __forceinline__ float BandDense(const float *lp0, int32_t C, int32_t T, int32_t row,
+                                           int32_t label) {
+  if (row < T) return (label >= 0 && label < C) ? lp0[(int64_t)row * C + label] : -INFINITY;
   return label == -1 ? 0.0f : -INFINITY;
 }
 
@@ -308,8 +308,8 @@ __device__ __forceinline__ void VitLoad(const float *p, float (&v)[K]) {
 // that it touches.
 constexpr int kGatherRows = 16;  // per CTA: two per warp
 __global__ void __launch_bounds__(256)
-BandGather(const BandInfo *__restrict__ infos, const BandState *__restrict__ tab,
-           const float *__restrict__ lp, int32_t C, float *__restrict__ by_state) {
+BandGather(const BandInfo *infos, const BandState *tab, const float *lp, int32_t C,
+           float *__restrict__ by_state) {
   __shared__ int32_t label_sh[kBandMaxStates];
   WaitForPrevious();
   const BandInfo f = infos[blockIdx.y];
@@ -326,7 +326,7 @@ BandGather(const BandInfo *__restrict__ infos, const BandState *__restrict__ tab
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
         const int32_t s = s0 + 32 * k, label = s < S ? label_sh[s] : -1;
-        x[k] = label >= 0 && label < C ? __ldg(in + label) : -INFINITY;
+        x[k] = label >= 0 && label < C ? in[label] : -INFINITY;
       }
 #pragma unroll
       for (int k = 0; k < 8; ++k)
@@ -390,10 +390,10 @@ __device__ __forceinline__ void VitFrames(int32_t n, const float *row, int32_t w
 // per batch in the other one took 5 us of 1000 frames.)
 template <bool kByState, bool kEdge>
 __global__ void __launch_bounds__(32 * (kVitMaxWarps + 1), 1)
-BandViterbi(const BandInfo *__restrict__ infos, const BandState *__restrict__ tab,
-            const float *__restrict__ lp, int64_t lp_rows, int32_t C, float *__restrict__ vf,
-            float *__restrict__ vb, int32_t F, int32_t nbatch, int32_t slot_floats,
-            int32_t xch_pad, int32_t wait_limit, int32_t *__restrict__ status) {
+BandViterbi(const BandInfo *infos, const BandState *tab, const float *lp, int64_t lp_rows,
+            int32_t C, float *__restrict__ vf, float *__restrict__ vb, int32_t F, int32_t nbatch,
+            int32_t slot_floats, int32_t xch_pad, int32_t wait_limit,
+            int32_t *__restrict__ status) {
   constexpr int K = kVitK;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full[kVitMaxBatches];
@@ -815,11 +815,10 @@ static size_t BandPrepSmem(int32_t max_states) {
 
 template <bool kDelay>
 __global__ void __launch_bounds__(32 * kPrepWarps, 3)
-BandPrep(const BandInfo *__restrict__ infos, const int32_t *__restrict__ a_row_splits2,
-         const BandState *__restrict__ tab, const BandArc *__restrict__ tabf,
-         const float *__restrict__ lp, int32_t C, const float *__restrict__ by_state,
-         const float *__restrict__ vf, const float *__restrict__ vb, float beam,
-         BandItem *__restrict__ items, BandFactor *__restrict__ factors, int2 *__restrict__ lists,
+BandPrep(const BandInfo *infos, const int32_t *a_row_splits2, const BandState *tab,
+         const BandArc *tabf, const float *lp, int32_t C, const float *by_state, const float *vf,
+         const float *vb, float beam, BandItem *__restrict__ items,
+         BandFactor *__restrict__ factors, int2 *__restrict__ lists,
          int32_t *__restrict__ chunk_r, unsigned long long *__restrict__ totals,
          int32_t *__restrict__ unfit, int32_t count_arcs, DelaySpec delay) {
   constexpr unsigned kAll = 0xffffffffu;
@@ -909,7 +908,7 @@ BandPrep(const BandInfo *__restrict__ infos, const int32_t *__restrict__ a_row_s
         if (count_arcs && l >= a && l < b) {
           for (uint32_t r = m; r; r &= r - 1) {
             const int32_t idx = f.state_off + s + __ffs(r) - 1;
-            n_cand += __ldg(a_row_splits2 + idx + 1) - __ldg(a_row_splits2 + idx);
+            n_cand += a_row_splits2[idx + 1] - a_row_splits2[idx];
           }
         }
       }
@@ -994,7 +993,7 @@ BandPrep(const BandInfo *__restrict__ infos, const int32_t *__restrict__ a_row_s
           else if (by_state != nullptr)
             x[u] = xrow[u][s[u]];
           else
-            x[u] = st[u].label >= 0 && st[u].label < C ? __ldg(xrow[u] + st[u].label) : -INFINITY;
+            x[u] = st[u].label >= 0 && st[u].label < C ? xrow[u][st[u].label] : -INFINITY;
           bc[u] = brow[u][s[u]];
 #pragma unroll
           for (int d = 0; d < 3; ++d) {
@@ -1332,13 +1331,11 @@ __device__ __forceinline__ void ChainChunk(const char *r, double *out, int32_t *
 template <int DIR>
 __device__ __forceinline__ void ChainWalk(const BandInfo &f, int32_t i, BandFactor *ring,
                                           ChainValues &vals, unsigned char *crc, uint64_t *full,
-                                          int32_t *hi_sh,
-                                          const BandFactor *__restrict__ factors,
-                                          const int32_t *__restrict__ chunk_r,
-                                          double *__restrict__ om, int32_t *__restrict__ oscale,
-                                          double *__restrict__ tot, BandTotal *__restrict__ total,
-                                          int32_t *__restrict__ unfit,
-                                          int32_t *__restrict__ status, int32_t wait_limit) {
+                                          int32_t *hi_sh, const BandFactor *factors,
+                                          const int32_t *chunk_r, double *om,
+                                          int32_t *__restrict__ oscale, double *tot,
+                                          BandTotal *__restrict__ total, int32_t *unfit,
+                                          int32_t *status, int32_t wait_limit) {
   constexpr unsigned kAll = 0xffffffffu;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int32_t T = f.frames, pitch = f.pitch, L = T + 2;
@@ -1470,12 +1467,10 @@ __device__ __forceinline__ void ChainWalk(const BandInfo &f, int32_t i, BandFact
 }
 
 __global__ void __launch_bounds__(kChainThreads + kKeepThreads)
-BandChainLists(const BandInfo *__restrict__ infos, const BandFactor *__restrict__ factors,
-               const int32_t *__restrict__ chunk_r, double *__restrict__ am,
-               double *__restrict__ bm, int32_t *__restrict__ a_scale,
-               int32_t *__restrict__ b_scale, double *__restrict__ tot,
-               BandTotal *__restrict__ total, int32_t *__restrict__ unfit,
-               int32_t *__restrict__ status, int32_t wait_limit) {
+BandChainLists(const BandInfo *infos, const BandFactor *factors, const int32_t *chunk_r,
+               double *am, double *bm, int32_t *__restrict__ a_scale,
+               int32_t *__restrict__ b_scale, double *tot, BandTotal *__restrict__ total,
+               int32_t *unfit, int32_t *status, int32_t wait_limit) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full[kChainSlots];
   __shared__ ChainValues vals;
@@ -1510,13 +1505,12 @@ constexpr int kExactThreads = 128;
 // `unfit`; every other graph returns at once.  exp(dense score) is recomputed from the
 // log-probs, the arc factors come from the graph's tables: no range limit.
 __device__ void
-ExactWalk(const BandInfo *__restrict__ infos, const BandArc *__restrict__ tabf,
-          const float *__restrict__ lp, int32_t C, const BandItem *__restrict__ items,
-          const int2 *__restrict__ lists, double *__restrict__ am, int32_t *__restrict__ ae,
-          double *__restrict__ bm, int32_t *__restrict__ be, double *__restrict__ tot,
-          BandTotal *__restrict__ total, const int32_t *__restrict__ unfit,
-          int32_t *__restrict__ status, int32_t st_pad, int32_t lv_pad, int32_t wait_limit,
-          const BandState *__restrict__ tab, const DelaySpec &delay) {
+ExactWalk(const BandInfo *infos, const BandArc *tabf, const float *lp, int32_t C,
+          const BandItem *items, const int2 *lists, double *__restrict__ am,
+          int32_t *__restrict__ ae, double *__restrict__ bm, int32_t *__restrict__ be,
+          double *tot, BandTotal *__restrict__ total, const int32_t *unfit, int32_t *status,
+          int32_t st_pad, int32_t lv_pad, int32_t wait_limit, const BandState *tab,
+          const DelaySpec &delay) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full[kChainSlots];
   const int dir = blockIdx.x;
@@ -1681,14 +1675,12 @@ __device__ __forceinline__ double LengthOf(const void *lens, int32_t type, int32
 }
 
 __global__ void __launch_bounds__(kExactThreads)
-BandChainExact(const BandInfo *__restrict__ infos, const BandArc *__restrict__ tabf,
-               const float *__restrict__ lp, int32_t C, const BandItem *__restrict__ items,
-               const int2 *__restrict__ lists, double *__restrict__ am,
+BandChainExact(const BandInfo *infos, const BandArc *tabf, const float *lp, int32_t C,
+               const BandItem *items, const int2 *lists, double *__restrict__ am,
                int32_t *__restrict__ ae, double *__restrict__ bm, int32_t *__restrict__ be,
-               double *__restrict__ tot, BandTotal *__restrict__ total,
-               const int32_t *__restrict__ unfit, int32_t *__restrict__ status, int32_t st_pad,
-               int32_t lv_pad, int32_t wait_limit, LossSpec spec, uint32_t *__restrict__ ticket,
-               const BandState *__restrict__ tab, DelaySpec delay) {
+               double *tot, BandTotal *__restrict__ total, const int32_t *unfit, int32_t *status,
+               int32_t st_pad, int32_t lv_pad, int32_t wait_limit, LossSpec spec,
+               uint32_t *ticket, const BandState *tab, DelaySpec delay) {
   WaitForPrevious();
   if (unfit[blockIdx.y] != 0)
     ExactWalk(infos, tabf, lp, C, items, lists, am, ae, bm, be, tot, total, unfit, status, st_pad,
@@ -1894,7 +1886,7 @@ BandGrad(const BandInfo *__restrict__ infos, const BandArc *__restrict__ tabf,
 // Rows whose entries a warp requests together: two, twelve CTAs to an SM, and one, sixteen, where a
 // row is read as well.  Bound by the chain list -> entries -> sums -> row of a warp beside the
 // stores (the rows alone would take 22 of the 36 us of 64 x 1000 frames, 50 of 62 of 32 x 500 x
-// 5000), so more warps with less each: with four rows and eight CTAs 37, 65 us, and 27 instead of 21
+// 5000), so more warps with less each: with four rows and eight CTAs 37, 65 us, and 27 instead of 20
 // from the logits of 32 x 600 x 501.
 __host__ __device__ constexpr int DenseRows(bool softmax) { return softmax ? 1 : 2; }
 // Columns of a range.  A warp stores its range alone, so a wide one leaves an SM few warps: 60 000
@@ -1905,13 +1897,11 @@ constexpr int kGradColumns = 6400;
 
 template <bool kSoftmax>
 __global__ void __launch_bounds__(128, kSoftmax ? 16 : 12)
-BandGradRows(const BandInfo *__restrict__ infos, const float *__restrict__ lp,
-             const BandItem *__restrict__ items, const int2 *__restrict__ lists,
-             const double *__restrict__ am, const int32_t *__restrict__ ae,
-             const double *__restrict__ bm, const int32_t *__restrict__ be,
-             const int32_t *__restrict__ a_scale, const int32_t *__restrict__ b_scale,
-             const BandTotal *__restrict__ total, const int32_t *__restrict__ unfit,
-             const GradSpec upstream, float *__restrict__ grad, int32_t C, int32_t width) {
+BandGradRows(const BandInfo *infos, const float *lp, const BandItem *items, const int2 *lists,
+             const double *am, const int32_t *ae, const double *bm, const int32_t *be,
+             const int32_t *a_scale, const int32_t *b_scale, const BandTotal *total,
+             const int32_t *unfit, const GradSpec upstream, float *__restrict__ grad, int32_t C,
+             int32_t width) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr unsigned kAll = 0xffffffffu;
   constexpr int kDenseRows = DenseRows(kSoftmax);
@@ -2016,11 +2006,19 @@ BandGradRows(const BandInfo *__restrict__ infos, const float *__restrict__ lp,
       // (the sum of a row's posteriors is at most 1, its fixed-point value fits 32 bits)
       const float total_g = value(__reduce_add_sync(kAll, added));
       const float *x = lp + (int64_t)(f.lp_row + r) * C + col0;
-#pragma unroll 4
-      for (int32_t c = lane; c < cols; c += 32) {
-        const uint32_t y = sums[c];
-        if (y) sums[c] = 0u;
-        out[c] = value(y) - expf(__ldg(x + c)) * total_g;
+      // (four loads together: the compiler does not move one past what is stored before it)
+      for (int32_t c0 = lane; c0 < cols; c0 += 128) {
+        float p[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) p[k] = c0 + 32 * k < cols ? x[c0 + 32 * k] : 0.0f;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int32_t c = c0 + 32 * k;
+          if (c >= cols) break;
+          const uint32_t y = sums[c];
+          if (y) sums[c] = 0u;
+          out[c] = value(y) - expf(p[k]) * total_g;
+        }
       }
     }
     __syncwarp();  // the row of sums is zero again
@@ -2034,7 +2032,7 @@ BandGradRows(const BandInfo *__restrict__ infos, const float *__restrict__ lp,
 // memory's).
 template <int kPer>
 __global__ void __launch_bounds__(256)
-LogSoftmaxRows(const BandInfo *__restrict__ infos, const float *__restrict__ logits, int32_t C,
+LogSoftmaxRows(const BandInfo *infos, const float *logits, int32_t C,
                float *__restrict__ log_probs) {
   WaitForPrevious();
   const BandInfo f = infos[blockIdx.y];
@@ -2045,12 +2043,12 @@ LogSoftmaxRows(const BandInfo *__restrict__ infos, const float *__restrict__ log
   float x[kPer > 0 ? kPer : 1], mx = -INFINITY, sum = 0.0f;
   if (kPer > 0) {
 #pragma unroll
-    for (int k = 0; k < kPer; ++k) x[k] = lane + 32 * k < C ? __ldg(in + lane + 32 * k) : -INFINITY;
+    for (int k = 0; k < kPer; ++k) x[k] = lane + 32 * k < C ? in[lane + 32 * k] : -INFINITY;
 #pragma unroll
     for (int k = 0; k < kPer; ++k) mx = fmaxf(mx, x[k]);
   } else {
 #pragma unroll 4
-    for (int32_t c = lane; c < C; c += 32) mx = fmaxf(mx, __ldg(in + c));
+    for (int32_t c = lane; c < C; c += 32) mx = fmaxf(mx, in[c]);
   }
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, d));
@@ -2060,7 +2058,7 @@ LogSoftmaxRows(const BandInfo *__restrict__ infos, const float *__restrict__ log
       if (lane + 32 * k < C) sum += expf(x[k] - mx);
   } else {
 #pragma unroll 4
-    for (int32_t c = lane; c < C; c += 32) sum += expf(__ldg(in + c) - mx);
+    for (int32_t c = lane; c < C; c += 32) sum += expf(in[c] - mx);
   }
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
@@ -2071,7 +2069,7 @@ LogSoftmaxRows(const BandInfo *__restrict__ infos, const float *__restrict__ log
       if (lane + 32 * k < C) out[lane + 32 * k] = (x[k] - mx) - lse;
   } else {
 #pragma unroll 4
-    for (int32_t c = lane; c < C; c += 32) out[c] = (__ldg(in + c) - mx) - lse;
+    for (int32_t c = lane; c < C; c += 32) out[c] = (in[c] - mx) - lse;
   }
 }
 

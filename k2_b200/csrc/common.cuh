@@ -116,7 +116,9 @@ struct SideReadBackScope {
 // Kernels of one stream that follow each other closely: a kernel launched with LaunchBehind may be
 // set up while the one before it still runs, from when all its CTAs have called LetNextStart() (or
 // have ended).  It calls WaitForPrevious() before it touches memory; behind that everything is as if
-// it had been launched in the usual way.
+// it had been launched in the usual way - to a load that the memory model orders.  One through a
+// pointer to const with __restrict__, or __ldg, is not: it says that nobody writes there while the
+// kernel lives, which for such a kernel begins before that call.  So what it reads has neither.
 __device__ __forceinline__ void WaitForPrevious() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }

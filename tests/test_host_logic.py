@@ -413,3 +413,27 @@ def test_what_the_lattice_free_loss_takes(degree, states, arcs, columns, support
     got = ctypes.c_int32(-1)
     _lib.check(_lib.lib.k2b200_dense_loss_supported(ctypes.byref(args), ctypes.byref(got)))
     assert bool(got.value) == supported
+
+
+def test_kernels_that_start_early_read_with_ordered_loads():
+    # a kernel that is alive while the one before it writes (WaitForPrevious) must not say that
+    # its inputs are read-only for its whole life; nor what it calls
+    csrc = os.path.join(ROOT, "k2_b200", "csrc")
+    checked = 0
+    for name in sorted(os.listdir(csrc)):
+        if not name.endswith(".cu"):
+            continue
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, name)).read())
+        if "LaunchBehind(" not in text:
+            continue
+        assert "__ldg(" not in text
+        starts = [m.start() for m in re.finditer(r"^(?:template[^\n]*\n)?__(?:global|device)__",
+                                                 text, re.M)]
+        for begin, end in zip(starts, starts[1:] + [len(text)]):
+            body = text[begin:end]
+            if "__global__" in body[:80] and "WaitForPrevious()" not in body:
+                continue  # launched in the usual way
+            signature = body[:body.index("{")]
+            assert not re.search(r"const \w+ \*\s*__restrict__", signature), signature
+            checked += "WaitForPrevious()" in body
+    assert checked >= 7
