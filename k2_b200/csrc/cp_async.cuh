@@ -59,6 +59,18 @@ __device__ __forceinline__ bool MbarTryWait(uint64_t *bar, unsigned parity) {
       : "memory");
   return ok != 0;
 }
+// The same without a suspension of the thread: a bounded number of these takes a bounded time.
+__device__ __forceinline__ bool MbarTestWait(uint64_t *bar, unsigned parity) {
+  unsigned ok;
+  asm volatile(
+      "{\n.reg .pred p;\n"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      "selp.u32 %0, 1, 0, p;\n}"
+      : "=r"(ok)
+      : "r"(SmemAddr(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 // Bounded wait: false when the phase did not complete within `max_spins` polls.
 __device__ __forceinline__ bool MbarWaitBounded(uint64_t *bar, unsigned parity,
                                                 int max_spins = 4000000) {

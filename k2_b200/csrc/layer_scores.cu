@@ -39,6 +39,7 @@ constexpr int kRangeExp = 280;        // values that are not zero stay within 2^
 constexpr int kMaxSlots = 8;
 constexpr int kWideTeam = 8, kWideWarps = 16;  // CTAs that share a layer, warps of each
 constexpr int kWideRecs = 2;                   // records of a lane ahead
+constexpr int kDrainTests = 1 << 16;           // a millisecond, for stores that take microseconds
 constexpr int kSliceMaxStates = 16384;  // states of a sliced layer
 
 struct __align__(16) LayerArc {
@@ -1130,7 +1131,7 @@ __global__ void __launch_bounds__(32 * kWideWarps, 1)
 LayerChainWide(k2b200_fsa_view v, const LayerArc *__restrict__ fwd_arcs,
                const LayerArc *__restrict__ bwd_arcs, Val *val_fwd, Val *val_bwd,
                int32_t *__restrict__ entering, int32_t *__restrict__ scale, int32_t dir_base,
-               int32_t fsa_base, ChainPlan p, int32_t *__restrict__ status) {
+               int32_t fsa_base, ChainPlan p, int32_t wait_limit, int32_t *__restrict__ status) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bars[2];
   __shared__ int32_t words[2][kWideTeam * kWideWarps];
@@ -1246,6 +1247,7 @@ LayerChainWide(k2b200_fsa_view v, const LayerArc *__restrict__ fwd_arcs,
   };
   begin(0);
   bool ok = true;
+  int32_t last_step = 0;
   for (int32_t step = 0; step < nl && ok; ++step) {
     const int32_t log_lanes = now.log_lanes, lanes = 1 << log_lanes, g = lane & (lanes - 1);
     const bool far = e - b > p.cells;
@@ -1337,12 +1339,26 @@ LayerChainWide(k2b200_fsa_view v, const LayerArc *__restrict__ fwd_arcs,
     after = splits_of(step + 3);
     if (step + 1 < nl) begin(step + 1);
     if (far) ClusterSync();
-    ok = __all_sync(kAll, MbarWaitBounded(&bars[step & 1], (unsigned)(step >> 1) & 1u));
+    ok = __all_sync(kAll,
+                    MbarWaitBounded(&bars[step & 1], (unsigned)(step >> 1) & 1u, wait_limit));
+    last_step = step;
   }
-  if (!ok && lane == 0) atomicOr(status, 2);
+  if (!ok) {
+    if (lane == 0) atomicOr(status, 2);
+    // the others still meet at the barriers of the layers that go through L2
+    for (int32_t step = last_step + 1; step < nl; ++step)
+      if (lvl[layer_of(step) + 1] - lvl[layer_of(step)] > p.cells) ClusterSync();
+  }
   sc.End(lane, status);
   CpAsyncWait<0>();
-  ClusterSync();  // no CTA leaves while another may store into it
+  // No CTA leaves while another may store into it: behind this barrier nobody does any more, and what
+  // is still on its way where a wait gave up is of that layer or the next one (nobody gets further
+  // without this CTA's words).  The bytes of the next one may never be complete.
+  ClusterSync();
+  if (!ok && tid == 0)
+    for (int32_t step = last_step; step < min(last_step + 2, nl); ++step)
+      for (int k = 0; k < kDrainTests; ++k)
+        if (MbarTestWait(&bars[step & 1], (unsigned)(step >> 1) & 1u)) break;
 }
 
 // out[s] = log(m[s]) + scale of its layer * ln 2.  grid = (layer tiles, fsas, parts of a
@@ -1486,7 +1502,7 @@ static int32_t LaunchChain(const k2b200_fsa_view *v, const ChainScratch &c, cons
     K2B_CUDA_OK(cudaLaunchKernelEx(&cfg, LayerChainWide<Val, kLog>, *v,
                                    (const LayerArc *)c.fwd_arcs, (const LayerArc *)c.bwd_arcs,
                                    val_fwd, val_bwd, entering, c.scale, dir_base, first, p,
-                                   c.status));
+                                   CopyWaitLimit(), c.status));
     NoteLaunch();
   }
   K2B_CUDA_OK(cudaGetLastError());

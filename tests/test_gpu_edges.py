@@ -46,6 +46,14 @@ def layered_lattice(rng, widths, degree, scale, hub=None):
     return host, first
 
 
+def with_layers(fsa, host, widths, first):
+    arcs_per_layer = np.diff(host.row_splits2[first])
+    fsa.arcs._levels = (torch.tensor([0, len(widths)], dtype=torch.int32, device=DEV),
+                        torch.from_numpy(first.astype(np.int32)).to(DEV))
+    fsa.arcs._layer_bounds = (1, len(widths), int(max(widths)), int(arcs_per_layer.max()))
+    return fsa
+
+
 @pytest.mark.parametrize("widths,degree,scale,hub", [
     ([1, 1], 1.0, 1.0, None),                        # one arc
     ([1, 31, 32, 33, 1], 1.2, 1.0, None),            # two arcs per lane, a warp and its edges
@@ -67,11 +75,7 @@ def test_lattice_scores_and_best_path(k2, widths, degree, scale, hub):
     from gpu_util import host_to_fsa
     rng = np.random.default_rng(len(widths))
     host, first = layered_lattice(rng, widths, degree, scale, hub)
-    fsa = host_to_fsa(host)
-    arcs_per_layer = np.diff(host.row_splits2[first])
-    fsa.arcs._levels = (torch.tensor([0, len(widths)], dtype=torch.int32, device=DEV),
-                        torch.from_numpy(first.astype(np.int32)).to(DEV))
-    fsa.arcs._layer_bounds = (1, len(widths), int(max(widths)), int(arcs_per_layer.max()))
+    fsa = with_layers(host_to_fsa(host), host, widths, first)
     for log in (True, False):
         for get, want in ((fsa.get_forward_scores, oracle.forward_scores(host, log)),
                           (fsa.get_backward_scores, oracle.backward_scores(host, log))):
@@ -81,6 +85,29 @@ def test_lattice_scores_and_best_path(k2, widths, degree, scale, hub):
     tot = fsa.get_tot_scores(log_semiring=False, use_double_scores=True)
     assert best.num_arcs == (len(widths) - 1 if torch.isfinite(tot).all() else 0)
     assert close(best.scores.double().sum().item(), tot[0].item(), rtol=1e-6, atol=1e-5)
+
+
+@pytest.mark.parametrize("widths", [
+    [1, 4095, 4097, 8193, 513, 1],            # values from CTA to CTA
+    [1, 12001, 300, 12001, 11000, 12500, 1],  # some through L2, with barriers of the cluster
+])
+def test_wide_layers_whose_waits_give_up_are_redone(k2, widths):
+    # with a limit of 0 every wait of the wide chain gives up at its first layer: it ends, says so,
+    # and the scores come from the kernel behind it
+    from gpu_util import host_to_fsa
+    from k2_b200 import _lib
+    host, first = layered_lattice(np.random.default_rng(3), widths, 1.5, 1.0)
+    for log in (True, False):
+        fsa = with_layers(host_to_fsa(host), host, widths, first)
+        want = (oracle.forward_scores(host, log), oracle.backward_scores(host, log))
+        try:
+            _lib.lib.k2b200_debug_set_copy_wait_limit(0)
+            got = [get(use_double_scores=True, log_semiring=log).detach().cpu().numpy()
+                   for get in (fsa.get_forward_scores, fsa.get_backward_scores)]
+        finally:
+            _lib.lib.k2b200_debug_set_copy_wait_limit(-1)
+        for a, b in zip(got, want):
+            assert close(a, b, rtol=1e-10, atol=1e-9)
 
 
 # --------------------------------------------------------------------------- CTC loss
