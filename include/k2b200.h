@@ -738,7 +738,7 @@ int32_t k2b200_fsa_levels(const int32_t *row_splits1, const int32_t *row_splits2
                           int32_t *level_splits, int32_t *status, void *tmp, void *stream);
 
 /* Best paths of a layered view (max_layers set; row_splits1, arcs and the layering are
- * read) as linear FSAs, in two launches and without a host read: path_splits[num_fsas+1],
+ * read) as linear FSAs, in three launches and without a host read: path_splits[num_fsas+1],
  * row_splits1[num_fsas+1], row_splits2 (room for num_fsas*(max_layers+1)+1), arcs and
  * best_arcs (arc of the view; room for num_fsas*max_layers). */
 size_t k2b200_best_paths_tmp_bytes(const k2b200_fsa_view *fsas);

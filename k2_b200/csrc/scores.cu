@@ -661,7 +661,7 @@ size_t k2b200_best_paths_tmp_bytes(const k2b200_fsa_view *v) {
   if (v == nullptr) return 0;
   return AlignUp(sizeof(int32_t) * ((size_t)v->num_fsas + 1)) +
          AlignUp(sizeof(int32_t) * (size_t)v->num_fsas * (size_t)v->max_layers) +
-         AlignUp(sizeof(int32_t) * (size_t)std::max(v->num_states, 0) + 16);
+         AlignUp(16 * ((size_t)std::max(v->num_states, 0) / 4 + 1) + 12);
 }
 
 int32_t k2b200_best_paths(const k2b200_fsa_view *v, const int32_t *entering_arcs,
@@ -676,7 +676,7 @@ int32_t k2b200_best_paths(const k2b200_fsa_view *v, const int32_t *entering_arcs
   int32_t *lengths = reinterpret_cast<int32_t *>(tmp);
   int32_t *traced = reinterpret_cast<int32_t *>(
       reinterpret_cast<char *>(tmp) + AlignUp(sizeof(int32_t) * ((size_t)v->num_fsas + 1)));
-  // (read 16 bytes at a time, whatever the alignment of `tmp`)
+  // (read 16 bytes at a time, from a multiple of 16 bytes on, wherever `tmp` lies)
   int32_t *pred = reinterpret_cast<int32_t *>(
       (reinterpret_cast<uintptr_t>(traced) +
        AlignUp(sizeof(int32_t) * (size_t)v->num_fsas * (size_t)v->max_layers) + 15) &
