@@ -165,7 +165,7 @@ __global__ void PathFill(const int32_t *__restrict__ row_splits1, const Arc *__r
 // layers of 13 states 42 us, now 18 + 2; 150 of 1 200: 87 -> 28 + 2; 32 FSAs of 100 000 states: 271 ->
 // 28 + 18.)
 // ---------------------------------------------------------------------------
-constexpr int kTraceStates = 48 * 1024;  // predecessors in shared memory
+constexpr int kTraceStates = 48 * 1024;  // predecessors in shared memory, at most (TraceRoom)
 constexpr int kTraceLayers = 512;        // layers of a run at most, one per thread and trip
 constexpr int kTraceFew = 8;             // runs of fewer layers are followed in global memory: to
                                          // fetch a run takes as long as some seven steps there
@@ -184,19 +184,19 @@ Predecessors(const Arc *__restrict__ arcs, const int32_t *__restrict__ entering,
 
 __global__ void __launch_bounds__(512)
 TraceLayers(k2b200_fsa_view v, const int32_t *__restrict__ entering,
-            const int32_t *__restrict__ all_pred, int32_t *__restrict__ best,
+            const int32_t *__restrict__ all_pred, int32_t room, int32_t *__restrict__ best,
             int32_t *__restrict__ lengths) {
-  // A run's predecessors, from a multiple of four states on, as offsets in this array; one outside
-  // the run, or none, is kOut, where kOut itself stands: a step then needs no test.
+  // A run's predecessors, from a multiple of four states on, as offsets in this array of `room`; one
+  // outside the run, or none, is kOut, where kOut itself stands: a step then needs no test.
   extern __shared__ int4 pred4[];
   __shared__ int32_t path[kTraceLayers + kTraceSteps], cur_sh, steps_sh;
-  constexpr int32_t kOut = 4 * kTraceStates;
+  const int32_t kOut = 4 * room;
   const char *pred = reinterpret_cast<const char *>(pred4);
   const int32_t i = blockIdx.x;
   const int tid = threadIdx.x;
   const int32_t s_begin = v.row_splits1[i], s_end = v.row_splits1[i + 1];
   int32_t *out = best + (int64_t)i * v.max_layers;
-  if (tid == 0) pred4[kTraceStates / 4] = make_int4(kOut, kOut, kOut, kOut);
+  if (tid == 0) pred4[room / 4] = make_int4(kOut, kOut, kOut, kOut);
   int32_t len = 0, cur = s_end - 1, hi = v.level_offsets[i + 1];
   const int32_t lv0 = v.level_offsets[i];
   bool alive = s_end > s_begin;
@@ -205,7 +205,7 @@ TraceLayers(k2b200_fsa_view v, const int32_t *__restrict__ entering,
     const int32_t top = v.level_splits[hi];
     const int32_t l = hi - 1 - tid;
     const int32_t n =
-        __syncthreads_count(l >= lv0 && top - (v.level_splits[l] & ~3) <= kTraceStates);
+        __syncthreads_count(l >= lv0 && top - (v.level_splits[l] & ~3) <= room);
     const int32_t lo = hi - max(n, 1), base = v.level_splits[lo], base4 = base & ~3;
     const bool staged = n >= min(kTraceFew, hi - lv0);
     if (staged) {  // (what is read beyond `top` is within the array's last four)
@@ -270,6 +270,19 @@ TraceLayers(k2b200_fsa_view v, const int32_t *__restrict__ entering,
   }
   // (a path ends where no arc enters: only at the start state is it complete)
   if (tid == 0) lengths[i] = cur == -1 - s_begin && s_end > s_begin ? len : 0;
+}
+
+// States of a run: no more than an FSA can have, and where there are more FSAs than SMs no more
+// than lets two, three or four CTAs (its threads allow no more) share one.  512 alignments of up to
+// 100 layers: 14.0 us with the most for all, 5.4 so; 600 of 300: 28.3 and 9.9; 2000 of 50: 38.7 and
+// 13.1; 32 of 800: 17.2 both.
+static int32_t TraceRoom(const k2b200_fsa_view *v) {
+  const int32_t ctas = std::max(1, std::min(4, CeilDiv(v->num_fsas, NumSms())));
+  int64_t states = v->num_states;
+  if (v->max_layer_states > 0)
+    states = std::min(states, (int64_t)v->max_layers * v->max_layer_states);
+  // (a run begins at a multiple of four states)
+  return (int32_t)std::min<int64_t>((states + 3 + 3) & ~(int64_t)3, kTraceStates / ctas);
 }
 
 // The paths as linear FSAs: arcs (states renumbered, labels and scores kept), the lattice arc
@@ -684,9 +697,11 @@ int32_t k2b200_best_paths(const k2b200_fsa_view *v, const int32_t *entering_arcs
   if (v->num_states > 0)
     { Predecessors<<<CeilDiv(v->num_states, 256), 256, 0, STREAM(stream)>>>(
         reinterpret_cast<const Arc *>(v->arcs), entering_arcs, v->num_states, pred); NoteLaunch(); }
-  constexpr int smem = (int)sizeof(int32_t) * (kTraceStates + 4);
-  K2B_CUDA_OK(cudaFuncSetAttribute(TraceLayers, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  { TraceLayers<<<v->num_fsas, 512, smem, STREAM(stream)>>>(*v, entering_arcs, pred, traced,
+  const int32_t room = TraceRoom(v);
+  const int smem = (int)sizeof(int32_t) * (room + 4);
+  K2B_CUDA_OK(cudaFuncSetAttribute(TraceLayers, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)sizeof(int32_t) * (kTraceStates + 4)));
+  { TraceLayers<<<v->num_fsas, 512, smem, STREAM(stream)>>>(*v, entering_arcs, pred, room, traced,
                                                             lengths);
     NoteLaunch(); }
   { WritePaths<<<v->num_fsas, 128, 0, STREAM(stream)>>>(

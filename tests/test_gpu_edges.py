@@ -87,6 +87,30 @@ def test_lattice_scores_and_best_path(k2, widths, degree, scale, hub):
     assert close(best.scores.double().sum().item(), tot[0].item(), rtol=1e-6, atol=1e-5)
 
 
+@pytest.mark.parametrize("copies", [2, 149, 297, 445])
+@pytest.mark.parametrize("widths", [[1] + [400] * 40 + [1], [1] + [3, 2, 3] * 9 + [1]])
+def test_best_paths_of_many_fsas(k2, copies, widths):
+    # what a CTA traces at a time shrinks from 48 K states to 12 K with the number of FSAs (one has
+    # 16 002 here, or 74, all of them in one run); copies of one FSA have the path of that FSA
+    from gpu_util import host_to_fsa
+    host, first = layered_lattice(np.random.default_rng(8), widths, 1.3, 1.0)
+    na, ns = len(host.arcs), int(first[-1])
+    every = np.arange(copies)[:, None]
+    tiled = HostFsaVec((np.arange(copies + 1) * ns).astype(np.int32),
+                       np.append((every * na + host.row_splits2[None, :-1]).reshape(-1),
+                                 copies * na).astype(np.int32),
+                       np.tile(host.arcs, (copies, 1)))
+    fsa = with_layers(host_to_fsa(tiled), host, widths, first)
+    splits = np.append((every * ns + first[None, :-1]).reshape(-1), copies * ns)
+    fsa.arcs._levels = (torch.arange(copies + 1, dtype=torch.int32, device=DEV) * len(widths),
+                        torch.from_numpy(splits.astype(np.int32)).to(DEV))
+    _, entering = oracle.forward_scores(host, False, True, want_entering_arcs=True)
+    want = oracle.shortest_path(host, entering)[1]
+    best = k2.shortest_path(fsa, use_double_scores=True)._best_arc_map.cpu().numpy()
+    assert len(want) == len(widths) - 1
+    assert np.array_equal(best.reshape(copies, -1), every * na + want[None, :])
+
+
 @pytest.mark.parametrize("widths", [
     [1, 4095, 4097, 8193, 513, 1],            # values from CTA to CTA
     [1, 12001, 300, 12001, 11000, 12500, 1],  # some through L2, with barriers of the cluster
