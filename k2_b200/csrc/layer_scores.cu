@@ -213,7 +213,7 @@ struct ChainPlan {
   bool ok;
 };
 
-static ChainPlan PlanChain(const k2b200_fsa_view *v, int32_t ndir) {
+static ChainPlan PlanChain(const k2b200_fsa_view *v, int32_t ndir, bool log_semiring) {
   ChainPlan p = {};
   if (!v->strict_layers || v->max_layer_states <= 0 || v->max_layer_arcs < 0 ||
       v->max_layers <= 0 || (int64_t)v->num_fsas * v->max_layers > INT32_MAX)
@@ -224,11 +224,17 @@ static ChainPlan PlanChain(const k2b200_fsa_view *v, int32_t ndir) {
   const int32_t mean_w = (int32_t)((v->num_states + layers - 1) / layers),
                 mean_a = (int32_t)((v->num_arcs + layers - 1) / layers);
   // arcs per lane (rows of a block): what most states of a lattice have, or a share of it that
-  // leaves the states of many arcs enough lanes.  Three from 1.2 arcs per state on (alignments
-  // have 1.4, at most three): then no state has two lanes, and the tropical walk is the short one
-  // (239 -> 118 us for 802 layers); two below that (decoding, 1.07).
+  // leaves the states of many arcs enough lanes.  From 1.2 to 1.6 arcs per state (alignments have 1.4,
+  // at most three) three for small layers: then hardly a state has two lanes, and the tropical walk
+  // of a single warp is the short one (SliceLayers + SliceChain, us, with two and three rows; 802
+  // layers of 2 to 5 states 262 and 141, 402 of 10 states 169 and 132, of 48 192 and 189, 502 of 60 258
+  // and 245; the log semiring 203 and 190, 229 and 229, 304 and 294).  Two beyond two blocks of lanes:
+  // the regions take longer to write and to copy (402 of 64 states 206 and 207, of 256 364 and 417;
+  // log 242 and 244, 424 and 462); and in the log semiring for layers of a few states, one lane each
+  // or two (802 of 2 to 5: 685 and 704).
   const double mean_deg = (double)v->num_arcs / std::max(v->num_states, 1);
-  p.rows = mean_deg < 1.2 ? 2 : mean_deg < 3.0 ? 3 : mean_deg < 6.0 ? 4 : 8;
+  const bool three = mean_deg >= 1.2 && mean_w <= 60 && (mean_w > 4 || !log_semiring);
+  p.rows = mean_deg < 1.6 && !three ? 2 : mean_deg < 3.0 ? 3 : mean_deg < 6.0 ? 4 : 8;
   // Warps: a block of 32 lanes each, for a layer between the mean and the largest (a warp that
   // runs alone issues an instruction in about five cycles, so more warps than blocks only
   // add to the barrier).
@@ -1426,11 +1432,13 @@ ChainScratch CarveScratch(const k2b200_fsa_view *v, const ChainPlan &p, int32_t 
 }  // namespace
 
 size_t LayerScratchBytes(const k2b200_fsa_view *v, int32_t ndir) {
-  return CarveScratch(v, PlanChain(v, ndir), ndir, nullptr).bytes;
+  // (the caller does not say in which semiring it will ask)
+  return std::max(CarveScratch(v, PlanChain(v, ndir, false), ndir, nullptr).bytes,
+                  CarveScratch(v, PlanChain(v, ndir, true), ndir, nullptr).bytes);
 }
 
 bool LayerScoresNeedIncoming(const k2b200_fsa_view *v, int32_t ndir) {
-  const ChainPlan p = PlanChain(v, ndir);
+  const ChainPlan p = PlanChain(v, ndir, true);  // (as in the other semiring)
   return !p.ok || p.wide || v->num_arcs == 0;
 }
 
@@ -1518,7 +1526,7 @@ int32_t LaunchLayerScores(const k2b200_fsa_view *v, int32_t log_semiring, Real *
   if (scratch == nullptr || v->num_arcs == 0 || v->row_ids1 == nullptr || v->row_ids2 == nullptr)
     return kOk;
   const int32_t ndir = (fwd != nullptr) + (bwd != nullptr), dir_base = fwd ? 0 : 1;
-  const ChainPlan p = PlanChain(v, ndir);
+  const ChainPlan p = PlanChain(v, ndir, log_semiring != 0);
   const ChainScratch c = CarveScratch(v, p, ndir, scratch);
   if (!p.ok || scratch_bytes < c.bytes || (reinterpret_cast<uintptr_t>(scratch) & 15)) return kOk;
   if (p.wide && fwd != nullptr && (v->in_src == nullptr || v->in_score == nullptr)) return kOk;

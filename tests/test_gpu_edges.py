@@ -57,6 +57,10 @@ def with_layers(fsa, host, widths, first):
 @pytest.mark.parametrize("widths,degree,scale,hub", [
     ([1, 1], 1.0, 1.0, None),                        # one arc
     ([1, 31, 32, 33, 1], 1.2, 1.0, None),            # two arcs per lane, a warp and its edges
+    ([1] + [4] * 40 + [1], 1.25, 1.0, None),         # ... in the log semiring, else three
+    ([1] + [6] * 40 + [1], 1.25, 1.0, None),         # three
+    ([1] + [60] * 70 + [1], 1.25, 1.0, None),        # ... the widest
+    ([1] + [64] * 70 + [1], 1.25, 1.0, None),        # two
     ([1] + [40] * 70 + [1], 2.5, 1.0, None),         # three; several slots of 32 layers
     ([1, 70, 64, 65, 1], 5.0, 1.0, 33),              # four; a state over several lanes
     ([1, 30, 40, 50, 1], 12.0, 1.0, 300),            # eight; a state of more than 32 x 8 arcs
