@@ -1346,7 +1346,7 @@ __device__ __forceinline__ void ChainWalk(const BandInfo &f, int32_t i, BandFact
   if (tid == 0) {
     for (int st = 0; st < kChainSlots; ++st) MbarInit(&full[st], 1);
     MbarInitFence();
-    hi_sh[0] = hi_sh[1] = hi_sh[2] = hi_sh[3] = hi_sh[8] = 0;
+    hi_sh[0] = hi_sh[1] = hi_sh[2] = hi_sh[3] = 0;
   }
   __syncthreads();
   const BandFactor *fac0 = factors + f.grid_off;
@@ -1394,10 +1394,10 @@ __device__ __forceinline__ void ChainWalk(const BandInfo &f, int32_t i, BandFact
   unsigned parity = 0;
   for (int32_t q = 0; q < num_chunks; ++q) {
     // the issuer's warp has seen chunk q arrive; the chunk before has been read, and its last
-    // level's values are there
-    if (tid / 32 == kChainThreads / 32 && !WaitSlot(&full[slot], parity, wait_limit)) hi_sh[8] = 1;
-    __syncthreads();
-    late = *reinterpret_cast<volatile int32_t *>(&hi_sh[8]);
+    // level's values are there.  (Whether to go on is part of the barrier: warps that disagreed
+    // would wait for one another in the levels of the chunk.)
+    late = __syncthreads_or(tid / 32 == kChainThreads / 32 &&
+                            !WaitSlot(&full[slot], parity, wait_limit));
     if (late) break;
     const int32_t c = DIR == 0 ? q : num_chunks - 1 - q;
     const BandFactor *mine = ring + (size_t)slot * kFacSlot;
@@ -1474,7 +1474,7 @@ BandChainLists(const BandInfo *infos, const BandFactor *factors, const int32_t *
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full[kChainSlots];
   __shared__ ChainValues vals;
-  __shared__ int32_t hi_sh[9];
+  __shared__ int32_t hi_sh[8];
   __shared__ unsigned char crc[kChainMaxChunks];
   const int dir = blockIdx.x;
   const int32_t i = blockIdx.y;

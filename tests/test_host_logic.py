@@ -437,3 +437,17 @@ def test_kernels_that_start_early_read_with_ordered_loads():
             assert not re.search(r"const \w+ \*\s*__restrict__", signature), signature
             checked += "WaitForPrevious()" in body
     assert checked >= 7
+
+
+def test_a_wait_that_runs_out_ends_the_walk_of_all_warps_of_a_cta():
+    # one warp may see a copy arrive in time and another not: whether a walk goes on is decided in
+    # a barrier, for all of them, or the warps that go on wait for those that left
+    csrc = os.path.join(ROOT, "k2_b200", "csrc")
+    checked = 0
+    for name in ("band_loss.cu", "dense_loss.cu"):
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, name)).read())
+        for m in re.finditer(r"if \(late\) break;|gave_up = true;", text):
+            before = text[:m.start()].rstrip()
+            assert re.search(r"__syncthreads_or\([^;{]*[;{]$", before), before[-300:]
+            checked += 1
+    assert checked >= 4
