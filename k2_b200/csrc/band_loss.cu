@@ -1489,7 +1489,9 @@ BandChainLists(const BandInfo *infos, const BandFactor *factors, const int32_t *
     z.pad = 0;
     total[i] = z;
   }
-  if (f.num_states == 0 || unfit[i] != 0) return;  // BandChainExact takes the graphs BandPrep marked
+  // BandChainExact takes the graphs BandPrep marked.  (The other direction's CTA may mark this one
+  // at any time: one answer for all warps, which wait for one another in the levels.)
+  if (f.num_states == 0 || __syncthreads_or(unfit[i] != 0)) return;
   BandFactor *ring = reinterpret_cast<BandFactor *>(smem_raw);  // [slots][kFacSlot]
   if (dir == 0)
     ChainWalk<0>(f, i, ring, vals, crc, full, hi_sh, factors, chunk_r, am, a_scale, tot, total, unfit, status,

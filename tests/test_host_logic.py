@@ -451,3 +451,13 @@ def test_a_wait_that_runs_out_ends_the_walk_of_all_warps_of_a_cta():
             assert re.search(r"__syncthreads_or\([^;{]*[;{]$", before), before[-300:]
             checked += 1
     assert checked >= 4
+
+
+def test_ctas_agree_on_marks_that_another_cta_may_set_meanwhile():
+    # `unfit` is set by the CTAs of both directions of a graph; where warps of a CTA wait for each
+    # other in barriers of a given count, they must not read it each for itself
+    csrc = os.path.join(ROOT, "k2_b200", "csrc")
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, "band_loss.cu")).read())
+    body = text[text.index("BandChainLists("):text.index("kExactThreads = 128")]
+    assert "__syncthreads_or(unfit[i] != 0)" in body
+    assert "unfit[i]" not in body.replace("__syncthreads_or(unfit[i] != 0)", "")
