@@ -826,7 +826,7 @@ SliceChain(k2b200_fsa_view v, const uint4 *__restrict__ pool, const SliceDesc *_
     if (k == m) {  // the next slot
       slot = slot + 1 == p.slots ? 0 : slot + 1;
       parity ^= (slot == 0);
-      if (!MbarWaitBounded(&full[slot], parity)) {
+      if (!__all_sync(kAll, MbarWaitBounded(&full[slot], parity))) {  // the whole warp, or none
         // nothing that the slot holds is looked at; the other warps still need the barriers
         atomicOr(status, 2);
         for (; step < nl; ++step) layer_sync();

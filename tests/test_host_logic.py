@@ -451,6 +451,10 @@ def test_a_wait_that_runs_out_ends_the_walk_of_all_warps_of_a_cta():
             assert re.search(r"__syncthreads_or\([^;{]*[;{]$", before), before[-300:]
             checked += 1
     assert checked >= 4
+    # the chains over layers, whose warps wait each for itself: no lane leaves without the others
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, "layer_scores.cu")).read())
+    for m in re.finditer(r"if \((?:[^()]|\([^()]*\))*MbarWaitBounded", text):
+        assert "__all_sync(kAll, " in m.group(), m.group()
 
 
 def test_ctas_agree_on_marks_that_another_cta_may_set_meanwhile():
