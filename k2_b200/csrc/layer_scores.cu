@@ -793,7 +793,7 @@ SliceChain(k2b200_fsa_view v, const uint4 *__restrict__ pool, const SliceDesc *_
 #pragma unroll
     for (int u = 0; u < K; ++u) l.x[u] = r[u * 32];
   };
-  auto single = [&](const Single &now, Single &next, int32_t &at, int32_t step) {
+  auto single = [&](const Single &now, Single &next, int32_t &at) {
     Val y[K];
 #pragma unroll
     for (int u = 0; u < K; ++u) y[u] = vals[prev + now.x[u].other];
@@ -811,7 +811,7 @@ SliceChain(k2b200_fsa_view v, const uint4 *__restrict__ pool, const SliceDesc *_
     for (int u = 0; u < K; ++u) q.Add(now.x[u], y[u]);
     if (now.word & kLaneHead) {
       const int32_t j = (int32_t)(now.word & kNoState), s = now.first_state + j;
-      if (step == 0 && s == root && q.acc == (Val)-INFINITY) q.acc = (Val)0;
+      if (s == root && q.acc == (Val)-INFINITY) q.acc = (Val)0;  // (empty layers may come first)
       vals[cur + j] = q.acc;
       out[s] = q.acc;
       if (entering != nullptr && dir == 0) entering[s] = q.best;
@@ -843,10 +843,10 @@ SliceChain(k2b200_fsa_view v, const uint4 *__restrict__ pool, const SliceDesc *_
         int32_t at = e.at;
         read_single(at, a);
         a.first_state = e.first_state;
-        while (single(a, b, at, step)) {
+        while (single(a, b, at)) {
           ++step;
           ++k;
-          if (!single(b, a, at, step)) break;
+          if (!single(b, a, at)) break;
           ++step;
           ++k;
         }

@@ -91,6 +91,21 @@ def test_lattice_scores_and_best_path(k2, widths, degree, scale, hub):
     assert close(best.scores.double().sum().item(), tot[0].item(), rtol=1e-6, atol=1e-5)
 
 
+def test_lattice_with_empty_layers_at_its_ends(k2):
+    # the first state of a walk is not in the walk's first layer: it scores 0 all the same
+    from gpu_util import host_to_fsa
+    widths = [1] + [5] * 70 + [1]
+    host, first = layered_lattice(np.random.default_rng(9), widths, 1.3, 1.0)
+    for before, behind in ((0, 0), (1, 0), (0, 1), (3, 40)):
+        splits = np.concatenate([np.zeros(before, np.int64), first, np.full(behind, first[-1])])
+        fsa = with_layers(host_to_fsa(host), host, [0] * before + widths + [0] * behind, splits)
+        for log in (True, False):
+            for get, want in ((fsa.get_forward_scores, oracle.forward_scores(host, log)),
+                              (fsa.get_backward_scores, oracle.backward_scores(host, log))):
+                got = get(use_double_scores=True, log_semiring=log).detach().cpu().numpy()
+                assert close(got, want, rtol=1e-10, atol=1e-9), (before, behind, log)
+
+
 @pytest.mark.parametrize("copies", [2, 149, 297, 445])
 @pytest.mark.parametrize("widths", [[1] + [400] * 40 + [1], [1] + [3, 2, 3] * 9 + [1]])
 def test_best_paths_of_many_fsas(k2, copies, widths):
