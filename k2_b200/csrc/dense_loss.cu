@@ -181,8 +181,9 @@ GridChainLanes(const FsaInfo *__restrict__ infos, int32_t n, const Arc *__restri
                LaneSmem sm, int32_t wait_limit) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full[kU];
-  __shared__ int32_t emax;
-  __shared__ int32_t t_fail_sm;  // step whose wait gave up  // largest exponent among the values of a group's last level
+  // largest exponent among the values of a group's last level: word g & 1 for group g to read
+  __shared__ int32_t emax[2];
+  __shared__ int32_t t_fail_sm;  // step whose wait gave up
   constexpr int32_t kNone = INT32_MIN;
   const int32_t i = blockIdx.y;
   const int dir = blockIdx.x;
@@ -235,7 +236,7 @@ GridChainLanes(const FsaInfo *__restrict__ infos, int32_t n, const Arc *__restri
   }
   if (tid == 0) {
     for (int st = 0; st < kU; ++st) MbarInit(&full[st], 1);
-    emax = kNone;
+    emax[0] = emax[1] = kNone;
     MbarInitFence();
   }
   if (__syncthreads_or(risky)) {  // also orders the initialisation above
@@ -259,7 +260,7 @@ GridChainLanes(const FsaInfo *__restrict__ infos, int32_t n, const Arc *__restri
       pv[q] = v.m;
       oth[q] = keep ? (dir == 0 ? fu : bu) : -INFINITY;
       out[lv * S + q] = v;
-      if (one) emax = 0;
+      if (one) emax[0] = 0;
     }
   }
   __syncthreads();
@@ -319,11 +320,11 @@ GridChainLanes(const FsaInfo *__restrict__ infos, int32_t n, const Arc *__restri
       if (producer) {
         // the slot the previous frame used takes the rows of step t + kU - 1
         issue_row(t + kU - 1, (u + kU - 1) % kU);
-        if (u == 1) emax = kNone;  // read by everyone during the frame before
+        if (u == 1) emax[parity] = kNone;  // read by everyone during the frame before
       }
       double scale = 1.0;
       if (u == 0) {  // once per group: renormalise by the exponent of the largest value
-        const int32_t e_prev = emax;
+        const int32_t e_prev = emax[parity];
         const int32_t shift = e_prev == kNone ? 0 : e_prev;
         K += shift;
         scale = __longlong_as_double((long long)(1023 - shift) << 52);
@@ -377,7 +378,7 @@ GridChainLanes(const FsaInfo *__restrict__ infos, int32_t n, const Arc *__restri
       if (u == kU - 1) {  // the next group renormalises by this level's largest value
         int32_t ex = (s >= 0 && v != 0.0) ? (vhi >> 20) - 1023 : kNone;
         ex = __reduce_max_sync(0xffffffffu, ex);
-        if ((tid & 31) == 0 && ex != kNone) atomicMax(&emax, ex);
+        if ((tid & 31) == 0 && ex != kNone) atomicMax(&emax[parity ^ 1u], ex);
       }
     }
     parity ^= 1u;
@@ -599,7 +600,9 @@ GridChainMasked(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_leve
                 ChainShare share) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full[kMaskedBatches];
-  __shared__ int32_t emax;
+  // largest exponent among the values of a batch's last level: word b % 3 for batch b to read; cleared
+  // while the batch behind it reads the next word, filled while that one reads the third
+  __shared__ int32_t emax[kMaskedBatches];
   __shared__ int32_t t_fail_sm;  // batch whose wait gave up
   constexpr int32_t kNone = INT32_MIN;
   int32_t after;  // the step before the first one
@@ -665,8 +668,10 @@ GridChainMasked(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_leve
   const bool hoist = __syncthreads_and(same);  // uniform over the CTA
   const uint32_t col0_off = 8u * (uint32_t)(col0 < 0 ? 0 : col0);  // no arc: the sum is 0
   if (tid == 0) {
-    for (int st = 0; st < kMaskedBatches; ++st) MbarInit(&full[st], 1);
-    emax = kNone;
+    for (int st = 0; st < kMaskedBatches; ++st) {
+      MbarInit(&full[st], 1);
+      emax[st] = kNone;
+    }
     MbarInitFence();
   }
   if (__syncthreads_or(risky)) {
@@ -681,7 +686,7 @@ GridChainMasked(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_leve
     for (int32_t q = tid; q < S; q += nt) {
       const double v = row[q].m;
       pv[q] = v;
-      if (v != 0.0) atomicMax(&emax, (__double2hiint(v) >> 20) - 1023);
+      if (v != 0.0) atomicMax(&emax[0], (__double2hiint(v) >> 20) - 1023);
     }
   } else {  // first level: 1 for the start (final) state if it survives, 0 elsewhere
     const int64_t lv = dir == 0 ? 0 : Tk;
@@ -696,7 +701,7 @@ GridChainMasked(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_leve
       pv[q] = v.m;
       out[lv * S + q] = v;
     }
-    if (tid == 0 && one_ok) emax = 0;
+    if (tid == 0 && one_ok) emax[0] = 0;
   }
   __syncthreads();
   const int64_t step_stride = dir == 0 ? (int64_t)S : -(int64_t)S;
@@ -754,10 +759,10 @@ GridChainMasked(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_leve
       for (int u = 0; u < kU; ++u) {
         if (u >= nf) break;
         if (u > 0) __syncthreads();  // the values of the frame before are complete
-        if (tid == 0 && u == (kU > 1 ? 1 : 0) && kU > 1) emax = kNone;  // read during frame 0
         double scale = 1.0;
         if (u == 0) {
-          const int32_t e_prev = emax;
+          if (tid == 0) emax[slot == 0 ? kMaskedBatches - 1 : slot - 1] = kNone;
+          const int32_t e_prev = emax[slot];
           const int32_t shift = e_prev == kNone ? 0 : e_prev;
           K += shift;
           scale = __longlong_as_double((long long)(1023 - shift) << 52);
@@ -813,14 +818,10 @@ GridChainMasked(const FsaInfo *__restrict__ infos, int32_t n, int64_t total_leve
         }
         pos += step_stride;
         if (u == kU - 1) {  // the next batch renormalises by this level's largest value
-          if (kU == 1) {    // no frame in between in which to reset the maximum
-            __syncthreads();
-            if (tid == 0) emax = kNone;
-            __syncthreads();
-          }
           int32_t ex = (s >= 0 && g == 0 && v != 0.0) ? (vhi >> 20) - 1023 : kNone;
           ex = __reduce_max_sync(0xffffffffu, ex);
-          if ((tid & 31) == 0 && ex != kNone) atomicMax(&emax, ex);
+          if ((tid & 31) == 0 && ex != kNone)
+            atomicMax(&emax[slot == kMaskedBatches - 1 ? 0 : slot + 1], ex);
         }
       }
     }

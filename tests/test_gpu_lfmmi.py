@@ -137,19 +137,28 @@ def test_denominator_batch_of_128_against_oracle():
     assert np.abs(lp2.grad.cpu().numpy() - want_lp).max() <= 1e-4
 
 
-@pytest.mark.parametrize("utterances,longest,shortest", [
-    (75, 64, 64),     # two chains more than a B200 has SMs, lengths of whole batches of four
-    (100, 101, 70),   # some end before the cut
-    (110, 127, 1),
-    (128, 400, 400),  # four rests to an SM
+@pytest.mark.parametrize("utterances,longest,shortest,classes,phones", [
+    (75, 64, 64, 72, 71),     # two chains more than a B200 has SMs, lengths of whole batches of four
+    (100, 101, 70, 72, 71),   # some end before the cut
+    (110, 127, 1, 72, 71),
+    (128, 400, 400, 72, 71),  # four rests to an SM
+    (80, 83, 60, 1500, 71),   # rows of which a batch holds two
+    (80, 83, 60, 3000, 71),   # ... and one
+    (80, 83, 60, 88, 84),     # graphs on 1024 lanes
 ])
-def test_chains_in_two_launches_are_the_chains(utterances, longest, shortest):
+def test_chains_in_two_launches_are_the_chains(utterances, longest, shortest, classes, phones):
     # the batch at once (chains are cut) and in parts of at most 60 utterances (they are not): the
     # same lattices, totals and, but for the order of additions to the graph, gradients
     import dataclasses
     import k2_b200 as k2
     from k2_b200 import synthetic as syn
     w = syn.lfmmi_den(utterances=utterances)
+    if classes != 72:
+        gen = torch.Generator().manual_seed(classes)
+        x = torch.randn(utterances, longest, classes, generator=gen)
+        rs2, graph = syn.den_graph(0, phones)
+        w = dataclasses.replace(w, log_probs=torch.log_softmax(x, -1), graph_row_splits2=rs2,
+                                graph_arcs=graph)
     seg = w.supervision_segments.clone()
     seg[:, 2] = torch.linspace(longest, shortest, utterances).int()
     got = []
