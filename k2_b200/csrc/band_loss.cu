@@ -846,7 +846,10 @@ BandPrep(const BandInfo *infos, const int32_t *a_row_splits2, const BandState *t
   }
   float cutoff;
   {
-    const float start = bg[0], end = fg[(int64_t)(T + 1) * pitch + (S - 1)];
+    // (without a path BandViterbi stored neither)
+    const bool path = S - 1 <= 2 * (T + 1);
+    const float start = path ? bg[0] : -INFINITY,
+                end = path ? fg[(int64_t)(T + 1) * pitch + (S - 1)] : -INFINITY;
     cutoff = __fsub_rn(start < end ? start : end, beam);
   }
   __syncthreads();

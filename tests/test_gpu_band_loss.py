@@ -224,7 +224,7 @@ def test_graphs_that_alternate_and_graphs_that_nearly_do(tokens, frames, classes
         arcs[in_second + 1, 3] = np.float32(-0.25).view(np.int32)
     elif change == "label":
         arcs[in_second:, 2][arcs[in_second:, 1] == 2 * (tokens // 2)] = classes - 1
-    elif change == "skip" and tokens > 1:
+    elif change == "skip":
         # an arc from the blank in state 0 to the blank in state 2 instead of its own loop
         assert arcs[in_second, 1] == 0 and arcs[in_second + 1, 1] == 1
         blank = int(arcs[in_second, 2])
@@ -235,6 +235,49 @@ def test_graphs_that_alternate_and_graphs_that_nearly_do(tokens, frames, classes
     lp = torch.from_numpy((x - np.log(np.exp(x).sum(-1, keepdims=True))).astype(np.float32))
     seg = torch.tensor([[0, 0, frames], [1, 0, max(tokens + 1, frames - 1)]], dtype=torch.int32)
     compare(a, lp, seg, 8.0, tag=change)
+
+
+@pytest.mark.parametrize("fill", [float("nan"), 3e38, -3e38])
+@pytest.mark.parametrize("alternates", [True, False])
+def test_transcripts_too_long_for_their_frames(monkeypatch, fill, alternates):
+    # arcs advance by at most two states: with more than 2 (T + 1) + 1 states no path is left, and
+    # cells that no path can pass are not stored, whatever the workspace held before
+    from k2_b200 import _lib
+    from k2_b200 import autograd as ag
+    from k2_b200.fsa_algo import ctc_graph
+    from gpu_util import fsa_to_host
+    rng = np.random.default_rng(5)
+    frames, classes = 21, 9
+    if alternates:  # S - 1 is 1, -1, 3, 5, 51 and -33 more than 2 (T + 1)
+        symbols = [[1 + k % 8 for k in range(tokens)] for tokens in (22, 21, 23, 24, 47, 5)]
+        a = fsa_to_host(ctc_graph(symbols, device=DEV))
+    else:
+        rs1, rs2, rows = [0], [0], []
+        for states in [2 * (frames + 1) + 1 + k for k in (0, 1, 2, 3, 4, 5, 90, 500)]:
+            labels = np.append(rng.integers(0, classes, size=states - 1), -1)
+            for s in range(states):
+                rows += [(s, s + d, labels[s + d], 0) for d in (0, 1, 2)
+                         if s + d < states and s < states - 1]
+                rs2.append(len(rows))
+            rs1.append(rs1[-1] + states)
+        a = HostFsaVec(np.asarray(rs1, np.int32), np.asarray(rs2, np.int32),
+                       make_arcs(*np.array(rows, np.int32).T[:3],
+                                 rng.normal(size=len(rows)).astype(np.float32)))
+    n = a.num_fsas
+    x = rng.normal(size=(n, frames, classes))
+    lp = torch.from_numpy((x - np.log(np.exp(x).sum(-1, keepdims=True))).astype(np.float32))
+    seg = torch.tensor([[i, 0, frames] for i in range(n)], dtype=torch.int32)
+
+    class Filled:
+        def __init__(self, nbytes, device):
+            self.tensor = torch.full(((nbytes + 3) // 4,), fill, device=device).view(torch.uint8)
+
+    monkeypatch.setattr(_lib, "workspace", Filled)
+    monkeypatch.setattr(ag, "BAND_VERIFY", True)
+    want, tot, _, gb = compare(a, lp, seg, 8.0)
+    reached = (np.diff(a.row_splits1) - 1) <= 2 * (frames + 1)
+    assert np.array_equal(np.isfinite(tot), reached) and reached.any() and not reached.all()
+    assert not gb[~reached].any()
 
 
 @pytest.mark.parametrize("classes", [3, 128, 129, 256, 257, 512, 513, 1024, 1025])
