@@ -254,9 +254,9 @@ __global__ void BandIncoming(const BandState *__restrict__ tab, const BandArc *_
 // requests by a thread that walks more).
 // A graph that alternates (VitForm) takes 17 instructions per frame and warp: three shared-memory
 // reads, a shuffle (backward: two), ten adds and maxima, a 16-byte store; any other takes 45.
-// Bound by the latency of a frame where the batch is small (36 ns with the three warps of 240
-// states, 53 on average with the nine of 801) and by DRAM where it is large: 64 x 1000 frames of
-// 500 classes are 204 MB read and 140 MB written in 62 us.  Cells that no path can pass, a quarter of
+// Bound by the latency of a frame: 36 ns with the three warps of 240 states, 53 on average with the
+// nine of 801, 62 with six and 64 x 1000 frames of 500 classes, whose 174 MB from DRAM and 86 MB to it
+// are two thirds of what the memory does in that time.  Cells that no path can pass, a quarter of
 // these grids, are neither stored nor read, and a warp without others sits out (67 and 99 us for
 // 16 x 1500 frames with all of them; 86 and 124 with all arcs by the general expressions and rows
 // requested and waited for by the warps that walk).  Two states per thread: slower; eight: 99 us.
@@ -1096,8 +1096,8 @@ BandPrep(const BandInfo *infos, const int32_t *a_row_splits2, const BandState *t
 }
 
 // ---------------------------------------------------------------------------
-// alpha (dir 0) and beta (dir 1) over the lists.  grid = (2, pairs), kMaxRegs warps per CTA:
-// thread j holds entry j of the current level's list, which says at which POSITIONS of the
+// alpha (dir 0) and beta (dir 1) over the lists.  grid = (2, pairs), up to kMaxRegs warps of a CTA
+// walk: thread j holds entry j of the current level's list, which says at which POSITIONS of the
 // previous list its neighbours are:
 //   alpha_l[j] = sum_d pw_l[j][d] * alpha_{l-1}[src_l[j][d]]
 //   beta_l[j]  = sum_d (pw_{l+1}[.][d] * beta_{l+1}[.]) at position dst_l[j][d]
@@ -1356,7 +1356,7 @@ __device__ __forceinline__ void ChainWalk(const BandInfo &f, int32_t i, BandFact
   om += f.grid_off;
   oscale += f.level_off;
   int32_t issued = 0;
-  // thread 0: the next chunk (in walking order) into the next slot; a chunk is
+  // the issuer: the next chunk (in walking order) into the next slot; a chunk is
   // levels * 32 * (warps it needs) entries, a multiple of 1 KB
   auto issue = [&]() {
     if (issued >= num_chunks) return;
@@ -2279,13 +2279,13 @@ static int32_t LaunchBandChains(const BandLayout &L, const k2b200_band_loss_args
   BandTotal *total = reinterpret_cast<BandTotal *>(ws + L.off_total);
   int32_t *unfit = reinterpret_cast<int32_t *>(ws + L.off_unfit);
   int32_t *status = reinterpret_cast<int32_t *>(ws + L.off_status);
-  { K2B_CUDA_OK(LaunchBehind(BandChainLists, grid, kChainThreads + kKeepThreads, L.chain_smem, stream, 
+  { K2B_CUDA_OK(LaunchBehind(BandChainLists, grid, kChainThreads + kKeepThreads, L.chain_smem, stream,
       infos, reinterpret_cast<const BandFactor *>(ws + L.off_factors),
       reinterpret_cast<const int32_t *>(ws + L.off_chunk_r), am, bm,
       reinterpret_cast<int32_t *>(ws + L.off_a_scale),
       reinterpret_cast<int32_t *>(ws + L.off_b_scale), tot_scores, total, unfit, status,
       CopyWaitLimit())); NoteLaunch(); }
-  { K2B_CUDA_OK(LaunchBehind(BandChainExact, grid, kExactThreads, L.exact_smem, stream, 
+  { K2B_CUDA_OK(LaunchBehind(BandChainExact, grid, kExactThreads, L.exact_smem, stream,
       infos, reinterpret_cast<const BandArc *>(args->band_arcs), args->log_probs,
       args->num_classes, items, lists, am, reinterpret_cast<int32_t *>(ws + L.off_ae), bm,
       reinterpret_cast<int32_t *>(ws + L.off_be), tot_scores, total, unfit, status, L.st_pad,
@@ -2438,7 +2438,7 @@ int32_t k2b200_band_loss_forward_reduce(const k2b200_band_loss_args *args, void 
                   : C <= 512  ? LogSoftmaxRows<16>
                   : C <= 1024 ? LogSoftmaxRows<32>
                               : LogSoftmaxRows<0>;
-    { K2B_CUDA_OK(LaunchBehind(kernel, grid, 256, 0, stream, 
+    { K2B_CUDA_OK(LaunchBehind(kernel, grid, 256, 0, stream,
         reinterpret_cast<const BandInfo *>(ws + L.off_infos), logits, args->num_classes,
         const_cast<float *>(args->log_probs))); NoteLaunch(); }
   }
@@ -2465,7 +2465,7 @@ int32_t k2b200_band_loss_forward_reduce(const k2b200_band_loss_args *args, void 
     K2B_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)L.viterbi_smem));
     dim3 grid(2, args->num_fsas);
-    { K2B_CUDA_OK(LaunchBehind(kernel, grid, L.vit_threads, L.viterbi_smem, stream, 
+    { K2B_CUDA_OK(LaunchBehind(kernel, grid, L.vit_threads, L.viterbi_smem, stream,
         infos, tab,
         L.by_state ? reinterpret_cast<const float *>(ws + L.off_by_state) : args->log_probs,
         args->log_prob_rows, args->num_classes, reinterpret_cast<float *>(ws + L.off_vf),
@@ -2500,7 +2500,7 @@ int32_t k2b200_band_loss_forward_reduce(const k2b200_band_loss_args *args, void 
       NotePhaseKernel(kPhasePrune, "BandPrep");
       dim3 grid(CeilDiv(L.max_frames + 2, kPrepLevels), args->num_fsas);
       auto prep = delay.penalty != 0.0f ? BandPrep<true> : BandPrep<false>;
-      { K2B_CUDA_OK(LaunchBehind(prep, grid, 32 * kPrepWarps, L.prep_smem, stream, 
+      { K2B_CUDA_OK(LaunchBehind(prep, grid, 32 * kPrepWarps, L.prep_smem, stream,
           reinterpret_cast<const BandInfo *>(ws + L.off_infos), args->a_row_splits2,
           reinterpret_cast<const BandState *>(args->band_states),
           reinterpret_cast<const BandArc *>(args->band_arcs), args->log_probs,
@@ -2647,7 +2647,7 @@ int32_t k2b200_band_loss_backward_dense(const k2b200_band_loss_args *args, void 
                                      (int)kBandSmemBudget));
     dim3 grid(CeilDiv(std::max(L.max_rows, 1), warps * DenseRows(softmax)), args->num_fsas,
               CeilDiv(C, width));
-    { K2B_CUDA_OK(LaunchBehind(kernel, grid, 32 * warps, row_bytes * warps, stream, 
+    { K2B_CUDA_OK(LaunchBehind(kernel, grid, 32 * warps, row_bytes * warps, stream,
         reinterpret_cast<const BandInfo *>(ws + L.off_infos), args->log_probs,
         reinterpret_cast<const BandItem *>(ws + L.off_items),
         reinterpret_cast<const int2 *>(ws + L.off_lists),
