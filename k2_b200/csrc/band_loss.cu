@@ -2173,7 +2173,9 @@ static int32_t MakeBandLayout(const k2b200_band_loss_args *a, BandLayout *L) {
   // than to walk, and a row by state is read twice instead of the row of the log-probs.  Also
   // where two batches of two rows do not fit.
   // Else frames per batch (even, at most 16) so that at least two batches of rows fit in
-  // shared memory, up to three within ~100 KB so that two CTAs share an SM.
+  // shared memory, up to three within ~100 KB so that two CTAs of up to eight warps share an SM.
+  // (Of more warps one fills an SM's registers: 76, 128, 256 x 1000 frames of 802 states and 500
+  // classes take 162, 183, 351 us, 223, 259, 461 with the general step in 80 registers.)
   {
     const size_t max_pitch = 32 * ((size_t)L->max_states / 32 + 1);
     const size_t C = (size_t)a->num_classes;

@@ -551,6 +551,22 @@ ChainShare ShareChains(const Layout &L) {
   const ChainShare one = {0, 0, 0};
   const int32_t sms = NumSms(), chains = 2 * (int32_t)L.infos.size(), whole = chains - sms;
   if (whole <= 0 || whole >= sms) return one;
+  // Not with unlike graphs: of 768 lanes, of 1024 (as far as the host can tell) or without a plan, as
+  // the CTAs of a launch whose graphs are another's return at once (55 pairs of a numerator and a
+  // denominator of 182 states: 1838 us a step, 2468 if cut); of half the lanes, whose chains are
+  // short (pairs with one of 144 states, 38: 1406, 1450; 55: 1558, 1560).
+  auto lanes = [](const FsaInfo &f) { return f.num_states + f.num_arcs / kLaneDeg; };
+  auto kind = [&](const FsaInfo &f) {
+    if (f.num_arcs > kLaneDeg * L.lane_threads) return 2;
+    return L.lane_threads > 768 && lanes(f) > kLaneRoom768 ? 1 : 0;
+  };
+  int32_t least = INT32_MAX, most = 0;
+  for (const FsaInfo &f : L.infos) {
+    if (kind(f) != kind(L.infos[0])) return one;
+    least = std::min(least, lanes(f));
+    most = std::max(most, lanes(f));
+  }
+  if (most / 2 > least) return one;
   constexpr int32_t kStart = 10;  // steps that pass before a CTA takes its first: 5 us
   // as many rests on each SM that has no whole chain as are walked in the time of a chain
   const int32_t rests = CeilDiv(sms, sms - whole);

@@ -71,6 +71,8 @@ int32_t LaunchPersistentViterbi(const Layout &L, const k2b200_intersect_args *a,
 // Lane plans: the most lanes a graph may need, and arcs per lane.
 constexpr int kLaneThreads = 1024;
 constexpr int kLaneDeg = 8;
+// Graphs of at most so many states plus eighths of an arc are sure of a place on 768 lanes.
+constexpr int kLaneRoom768 = 736;
 // The kernels that use plans have CTAs of 768 threads, with 80 registers each, and again of 1024
 // with 64 for the graphs that need more lanes: the plan says which (LaneClass).  The second
 // launch is left out when no graph can need it - states + arcs / kLaneDeg, and what packing

@@ -381,7 +381,7 @@ PlanLanes(const FsaInfo *__restrict__ infos, int32_t n,
 
 
 int32_t LaneThreads(const Layout &L) {
-  return L.max_states + L.max_arcs / kLaneDeg <= 736 ? 768 : 1024;
+  return L.max_states + L.max_arcs / kLaneDeg <= kLaneRoom768 ? 768 : 1024;
 }
 
 constexpr int kVitRing = 4;   // slots of LanesViterbi's row ring = frames per unrolled group

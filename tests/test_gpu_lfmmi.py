@@ -182,6 +182,46 @@ def test_chains_in_two_launches_are_the_chains(utterances, longest, shortest, cl
     assert torch.equal(got[0][2], got[1][2])
 
 
+def test_chains_of_unlike_graphs_are_not_cut():
+    # graphs on 768 lanes and on 1024 go through launches of their own, the CTAs of the others
+    # returning at once: 160 chains of which a launch walks 80 need no second one; nor do chains
+    # half of which are of small graphs
+    import k2_b200 as k2
+    from k2_b200 import _lib
+    from k2_b200 import synthetic as syn
+    from k2_b200.fsa_algo import _fsa_vec_from_numpy
+    kinds = [syn.den_graph(0, 71), syn.den_graph(0, 84), syn.den_graph(0, 30, 20)]
+    gen = torch.Generator().manual_seed(2)
+    n, frames, classes = 80, 60, 85
+    x = torch.log_softmax(torch.randn(n, frames, classes, generator=gen), -1).to(DEV)
+    seg = torch.tensor([[i, 0, frames] for i in range(n)], dtype=torch.int32)
+
+    def totals(which):
+        graphs = [kinds[k] for k in which]
+        states = np.cumsum([0] + [len(rs2) - 1 for rs2, _ in graphs])
+        first_arc = np.cumsum([0] + [len(arcs) for _, arcs in graphs])
+        rs2 = np.concatenate([rs2[:-1] + a for (rs2, _), a in zip(graphs, first_arc)] +
+                             [first_arc[-1:]])
+        fsa = _fsa_vec_from_numpy(states, rs2, np.concatenate([arcs for _, arcs in graphs]), DEV)
+        dense = k2.DenseFsaVec(x[:len(which)].contiguous(), seg[:len(which)])
+        out = []
+        for _ in range(2):  # (the first call makes what a graph keeps)
+            before = _lib.launch_count()
+            out.append(k2.intersect_dense_tot_scores(fsa, dense, 8.0))
+        assert torch.equal(out[0], out[1])
+        return out[0], _lib.launch_count() - before
+
+    mixed, launches = totals([0, 1] * 40)
+    assert launches == totals([0, 1] * 30)[1]
+    small, of_one_size = totals([0, 2] * 40)
+    assert of_one_size == totals([0, 2] * 30)[1]
+    for kind in (0, 1):
+        alike, cut = totals([kind] * 80)
+        assert cut > (of_one_size, launches)[kind]
+        assert torch.equal(mixed[kind::2], alike[kind::2])
+        assert kind == 1 or torch.equal(small[0::2], alike[0::2])
+
+
 def test_decoding_configuration_matches_the_reference_lattice_checksums():
     # hlg_decode at full size through intersect_dense_pruned; the reference's lattice
     # (tests/golden/make_pruned_full_size_golden.py) is kept as sizes and sha256 digests
