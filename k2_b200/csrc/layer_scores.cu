@@ -780,6 +780,7 @@ SliceChain(k2b200_fsa_view v, const uint4 *__restrict__ pool, const SliceDesc *_
   // What a warp that runs alone issues per layer bounds such a walk: 290 cycles, against 590 of the
   // general loop below.
   // (Its region then lies right behind: it is read before it is known whether it is of that kind.)
+  // The first layer with states has the one that scores 0 without an arc: it takes the general loop.
   constexpr int32_t kSingleUnits = SliceRowsAt(1, 0) + K * 32;
   struct Single {
     uint32_t word;
@@ -811,7 +812,6 @@ SliceChain(k2b200_fsa_view v, const uint4 *__restrict__ pool, const SliceDesc *_
     for (int u = 0; u < K; ++u) q.Add(now.x[u], y[u]);
     if (now.word & kLaneHead) {
       const int32_t j = (int32_t)(now.word & kNoState), s = now.first_state + j;
-      if (s == root && q.acc == (Val)-INFINITY) q.acc = (Val)0;  // (empty layers may come first)
       vals[cur + j] = q.acc;
       out[s] = q.acc;
       if (entering != nullptr && dir == 0) entering[s] = q.best;
@@ -822,6 +822,7 @@ SliceChain(k2b200_fsa_view v, const uint4 *__restrict__ pool, const SliceDesc *_
     __syncwarp();
     return more;
   };
+  bool begun = false;
   for (int32_t step = 0; step < nl; ++step) {
     if (k == m) {  // the next slot
       slot = slot + 1 == p.slots ? 0 : slot + 1;
@@ -838,7 +839,7 @@ SliceChain(k2b200_fsa_view v, const uint4 *__restrict__ pool, const SliceDesc *_
     SliceEntry e = entries[slot][k++];
     if (e.tall == kSingle) {
       e.tall = 0;
-      if (kOne && !kLog && e.at >= 0) {
+      if (kOne && !kLog && e.at >= 0 && begun) {
         Single a, b;
         int32_t at = e.at;
         read_single(at, a);
@@ -856,6 +857,7 @@ SliceChain(k2b200_fsa_view v, const uint4 *__restrict__ pool, const SliceDesc *_
         continue;
       }
     }
+    begun |= e.blocks != 0;
     sc.BeginLayer(step, hi_shared, tid == 0);
     auto finish = [&](int32_t j, StateSum<Val, kLog> &q) {
       const int32_t s = e.first_state + j;
